@@ -214,6 +214,24 @@ def test_weight_layout_round_trip(device):
     assert torch.equal(convert_layout(ts, BlackwellMXScaleLayout()).storage.data.cpu(), g_s)
 
 
+@pytest.mark.parametrize("E, K, N", [(1, 32, 2), (2, 2880, 200), (3, 160, 130)])
+def test_weight_layouts_from_strided_storage(E, K, N, device):
+    """The tiled layouts written straight from K-packed storage (rows 16-byte aligned, and a pitch that is not) equal those
+    made through the canonical row-major form."""
+    from triton_b200.tensor_details.layout import B200BlockScaledScaleLayout, B200BlockScaledValueLayout, StridedLayout
+    g = torch.Generator(device=device).manual_seed(K + N)
+    for pitch in (K // 2, K // 2 + 4):
+        q = torch.randint(0, 256, (E, N, pitch), dtype=torch.uint8, device=device, generator=g)[:, :, : K // 2].transpose(1, 2)
+        s = torch.randint(0, 255, (E, N, K // 32), dtype=torch.uint8, device=device, generator=g).transpose(1, 2)
+        tq, ts = wrap_torch_tensor(q, dtype=FP4), wrap_torch_tensor(s)
+        rq, rs = convert_layout(tq, StridedLayout()), convert_layout(ts, StridedLayout())
+        for t, r, layouts in ((tq, rq, (B200MXValueLayout(), B200BlockScaledValueLayout())),
+                              (ts, rs, (B200MXScaleLayout(), B200BlockScaledScaleLayout()))):
+            for lay in layouts:
+                via = lay.make_transformation(list(r.shape), r.dtype == FP4).swizzle_data(r.storage.data)
+                assert torch.equal(convert_layout(t, lay).storage.data, via)
+
+
 @pytest.fixture(scope="module")
 def layer_20b():
     """gpt-oss-20b-shaped expert weights (32 experts, d_model 2880, fused gate+up 5760) and their CPU dequantisation."""

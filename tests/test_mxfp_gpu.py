@@ -114,6 +114,23 @@ def test_random_shapes_against_oracle(shape, axis, mode, dt, device):
     assert torch.equal(bits(d.cpu()), bits(do.contiguous()))
 
 
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("shape", [(1, 32, 2), (1, 288, 66), (3, 320, 130), (2, 256, 64)])
+def test_strided_axis_tile_edges(shape, dt, device):
+    """Quantised axis strided: one column pair, remainders of the 64-column x 8-group tile, several batches, a whole tile."""
+    g = torch.Generator().manual_seed(sum(shape))
+    x = torch.randn(shape, generator=g).to(dt)
+    q, s = downcast_to_mxfp(x.to(device), torch.uint8, 1)
+    qo, so = oracle.downcast_to_mxfp_oracle(x, 1)
+    assert torch.equal(q.cpu(), qo) and torch.equal(s.cpu(), so)
+    for bias in (0, 100):                                  # ordinary scales, and scale bytes up to the NaN byte
+        s2 = (s.int() + bias).clamp_max(255).to(torch.uint8)
+        want = oracle.upcast_from_mxfp_oracle(qo, s2.cpu(), dt, 1)
+        got, nan = upcast_from_mxfp(q, s2, dt, axis=1).cpu(), torch.isnan(want.float())
+        assert torch.equal(torch.isnan(got.float()), nan)
+        assert torch.equal(bits(want.contiguous())[~nan], bits(got)[~nan])
+
+
 def test_full_size_properties(device):
     """bf16 [8192, 8192], N(0,1) with 1 % of entries x100: checked through size-independent properties --
     a sample of rows against the oracle, idempotence of quantise(dequantise(.)), scales never clip."""

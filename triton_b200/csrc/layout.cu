@@ -17,13 +17,10 @@ namespace {
 constexpr int TN = 128, TK = 128;
 
 __device__ __forceinline__ uint32_t nibble_interleave(uint32_t w) {   // natural -> (evens | odds << 16)
-  uint32_t r = 0;
-#pragma unroll
-  for (int a = 0; a < 4; ++a) {
-    r |= ((w >> (8 * a)) & 0xFu) << (4 * a);             // k = 2a
-    r |= ((w >> (8 * a + 4)) & 0xFu) << (16 + 4 * a);    // k = 2a + 1
-  }
-  return r;
+  uint32_t ev = w & 0x0F0F0F0Fu, od = (w >> 4) & 0x0F0F0F0Fu;          // k = 2a and k = 2a + 1 in byte a
+  ev = (ev | (ev >> 4)) & 0x00FF00FFu;
+  od = (od | (od >> 4)) & 0x00FF00FFu;
+  return ((ev | (ev >> 8)) & 0xFFFFu) | ((od | (od >> 8)) << 16);
 }
 __device__ __forceinline__ uint32_t nibble_deinterleave(uint32_t r) {
   uint32_t w = 0;
@@ -35,27 +32,42 @@ __device__ __forceinline__ uint32_t nibble_deinterleave(uint32_t r) {
   return w;
 }
 
-__global__ void __launch_bounds__(256) to_b200_values(const uint8_t* __restrict__ q, int64_t q_stride_e,
-                                                      int64_t q_stride_n, int E, int K, int N, int NT, int KT,
-                                                      uint32_t* __restrict__ out) {
-  const int64_t total = (int64_t)E * NT * KT * TN * 16;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int qw = (int)(i & 3);                       // word inside the 16-byte group chunk
-    const int r = (int)((i >> 2) & (TN - 1));
-    const int g = (int)((i >> 9) & 3);
-    const int j = g * 4 + qw;                          // word of the row: k = 8 j .. 8 j + 7
-    int64_t t = i >> 11;
-    const int kt = (int)(t % KT); t /= KT;
-    const int nt = (int)(t % NT);
-    const int e = (int)(t / NT);
-    const int n = nt * TN + r, k = kt * TK + j * 8;
-    uint32_t w = 0;
-    if (n < N && k < K) {
-      const uint8_t* src = q + (int64_t)e * q_stride_e + (int64_t)n * q_stride_n + (k >> 1);
-      // K is a multiple of 32, so the four bytes are all in range
-      w = (uint32_t)src[0] | ((uint32_t)src[1] << 8) | ((uint32_t)src[2] << 16) | ((uint32_t)src[3] << 24);
+// 16 bytes (the 32 k of one scale group) of a source row; VEC: rows are 16-byte aligned
+template <bool VEC> __device__ __forceinline__ uint4 load_group(const uint8_t* src) {
+  if constexpr (VEC) {
+    return *reinterpret_cast<const uint4*>(src);
+  } else {
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      w[i] = (uint32_t)src[4 * i] | ((uint32_t)src[4 * i + 1] << 8) | ((uint32_t)src[4 * i + 2] << 16) | ((uint32_t)src[4 * i + 3] << 24);
+    return make_uint4(w[0], w[1], w[2], w[3]);
+  }
+}
+
+// Value tiles of both layouts.  HBM-bound copy: a block takes a tile, a thread two of its 512 16-byte pieces (row, scale
+// group), four neighbouring lanes the 64 bytes of a row.  SCALED: the block-scaled layout (tiles [E][k_tile][n_block],
+// rows of 64 bytes as they are), else [E][n_tile][k_tile] with the [group][row] order and interleaved nibbles described above.
+template <bool SCALED, bool VEC>
+__global__ void __launch_bounds__(256) to_tiles_values(const uint8_t* __restrict__ q, int64_t q_stride_e, int64_t q_stride_n,
+                                                       int E, int K, int N, int NT, int KT, uint4* __restrict__ out) {
+  const int64_t tiles = (int64_t)E * NT * KT;
+  for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const int kt = SCALED ? (int)(tile / NT % KT) : (int)(tile % KT);
+    const int nt = SCALED ? (int)(tile % NT) : (int)(tile / KT % NT);
+    const int64_t e = tile / ((int64_t)NT * KT);
+    uint4* dst = out + tile * (TN * 4);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int p = threadIdx.x + i * 256, r = p >> 2, g = p & 3;
+      const int n = nt * TN + r, k = kt * TK + g * 32;             // K is a multiple of 32: a group is in or out as a whole
+      uint4 v = make_uint4(0, 0, 0, 0);
+      if (n < N && k < K) v = load_group<VEC>(q + e * q_stride_e + (int64_t)n * q_stride_n + (k >> 1));
+      if constexpr (SCALED)
+        dst[p] = v;
+      else
+        dst[g * TN + r] = make_uint4(nibble_interleave(v.x), nibble_interleave(v.y), nibble_interleave(v.z), nibble_interleave(v.w));
     }
-    out[i] = nibble_interleave(w);
   }
 }
 
@@ -106,6 +118,17 @@ __global__ void __launch_bounds__(256) from_b200_kernel(const uint32_t* __restri
   }
 }
 
+template <bool SCALED>
+void launch_to_tiles(const uint8_t* q, int64_t q_stride_e, int64_t q_stride_n, int E, int K, int N, int NT, int KT, uint8_t* out,
+                     cudaStream_t st) {
+  const int64_t tiles = (int64_t)E * NT * KT, cap = (int64_t)moe_sm_count() * 32;
+  const int grid = (int)(tiles < cap ? tiles : cap);
+  if ((uintptr_t)q % 16 == 0 && q_stride_e % 16 == 0 && q_stride_n % 16 == 0)
+    to_tiles_values<SCALED, true><<<grid, 256, 0, st>>>(q, q_stride_e, q_stride_n, E, K, N, NT, KT, (uint4*)out);
+  else
+    to_tiles_values<SCALED, false><<<grid, 256, 0, st>>>(q, q_stride_e, q_stride_n, E, K, N, NT, KT, (uint4*)out);
+}
+
 int grid_for(int64_t total) {
   int64_t blocks = cdiv64(total, 256);
   int64_t cap = (int64_t)moe_sm_count() * 16;
@@ -134,8 +157,7 @@ extern "C" __attribute__((visibility("default"))) int moe_weight_layout_to_b200(
   const int NT = (int)cdiv64(N, TN), KT = (int)cdiv64(K, TK);
   cudaStream_t st = (cudaStream_t)stream;
   if (q) {
-    to_b200_values<<<grid_for((int64_t)E * NT * KT * TN * 16), 256, 0, st>>>(q, q_stride_e, q_stride_n, E, K, N, NT, KT,
-                                                                            (uint32_t*)out_values);
+    launch_to_tiles<false>(q, q_stride_e, q_stride_n, E, K, N, NT, KT, out_values, st);
     MOE_CHECK_LAUNCH();
   }
   if (scale) {
@@ -167,27 +189,6 @@ extern "C" __attribute__((visibility("default"))) int moe_weight_layout_from_b20
 //               the reference (tensor_details/layout_details/blackwell_scale.py:165-175).
 // Out-of-range n or k is zero (value 0, scale byte 0 = 2^-127).
 namespace {
-
-__global__ void __launch_bounds__(256) to_b200mx_values(const uint8_t* __restrict__ q, int64_t q_stride_e,
-                                                        int64_t q_stride_n, int E, int K, int N, int NB, int KT,
-                                                        uint32_t* __restrict__ out) {
-  const int64_t total = (int64_t)E * KT * NB * TN * 16;             // 32-bit words
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int j = (int)(i & 15);                       // word of the row: k = 8 j .. 8 j + 7
-    const int r = (int)((i >> 4) & (TN - 1));
-    int64_t t = i >> 11;
-    const int nb = (int)(t % NB); t /= NB;
-    const int kt = (int)(t % KT);
-    const int e = (int)(t / KT);
-    const int n = nb * TN + r, k = kt * TK + j * 8;
-    uint32_t w = 0;
-    if (n < N && k < K) {
-      const uint8_t* src = q + (int64_t)e * q_stride_e + (int64_t)n * q_stride_n + (k >> 1);
-      w = (uint32_t)src[0] | ((uint32_t)src[1] << 8) | ((uint32_t)src[2] << 16) | ((uint32_t)src[3] << 24);
-    }
-    out[i] = w;
-  }
-}
 
 __global__ void __launch_bounds__(256) to_b200mx_scales(const uint8_t* __restrict__ s, int64_t s_stride_e,
                                                         int64_t s_stride_k, int64_t s_stride_n, int E, int K, int N,
@@ -251,8 +252,7 @@ extern "C" __attribute__((visibility("default"))) int moe_weight_layout_to_b200m
   const int NB = (int)cdiv64(N, TN), KT = (int)cdiv64(K, TK);
   cudaStream_t st = (cudaStream_t)stream;
   if (q) {
-    to_b200mx_values<<<grid_for((int64_t)E * NB * KT * TN * 16), 256, 0, st>>>(q, q_stride_e, q_stride_n, E, K, N, NB, KT,
-                                                                              (uint32_t*)out_values);
+    launch_to_tiles<true>(q, q_stride_e, q_stride_n, E, K, N, NB, KT, out_values, st);
     MOE_CHECK_LAUNCH();
   }
   if (scale) {

@@ -52,11 +52,6 @@ __device__ __forceinline__ uint32_t e2m1x2(float lo, float hi) {
   return (uint32_t)__nv_cvt_float2_to_fp4x2(make_float2(lo, hi), __NV_E2M1, cudaRoundNearest);
 }
 
-template <typename T> struct Vec16;  // 16-byte vector of T
-template <> struct Vec16<__nv_bfloat16> { static constexpr int N = 8; };
-template <> struct Vec16<__half> { static constexpr int N = 8; };
-template <> struct Vec16<float> { static constexpr int N = 4; };
-
 // ---- contiguous path: quant axis has unit stride, rows 16-byte aligned ------------------------------
 // One thread owns whole 32-groups: 64 (or 128) contiguous input bytes as 16-byte loads, one division and one scale
 // per group, one 16-byte store of the 32 codes and one byte of scale.  GROUPS_UNROLL groups are loaded before the first
@@ -124,23 +119,6 @@ __device__ __forceinline__ uint4 quantise_raw(const uint4 (&raw)[VPG], int mode,
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// 32 fp32 values -> scale bits and 16 bytes of codes
-__device__ __forceinline__ uint4 quantise_group(const float (&v)[32], int mode, uint32_t& sc) {
-  float m = 0.0f;
-#pragma unroll
-  for (int j = 0; j < 32; ++j) m = fmaxf(m, fabsf(v[j]));
-  sc = scale_bits(m, mode);
-  const float inv = inv_scale(sc);
-  uint32_t w[4];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const uint32_t b0 = e2m1x2(v[8 * k] * inv, v[8 * k + 1] * inv), b1 = e2m1x2(v[8 * k + 2] * inv, v[8 * k + 3] * inv);
-    const uint32_t b2 = e2m1x2(v[8 * k + 4] * inv, v[8 * k + 5] * inv), b3 = e2m1x2(v[8 * k + 6] * inv, v[8 * k + 7] * inv);
-    w[k] = __byte_perm(b0 | (b1 << 8), b2 | (b3 << 8), 0x5410);
-  }
-  return make_uint4(w[0], w[1], w[2], w[3]);
-}
-
 template <typename T, typename I>
 __global__ void __launch_bounds__(256, sizeof(T) == 2 ? 3 : 2) downcast_rows_kernel(const T* __restrict__ x, int64_t n_rows, int64_t quant,
                                                             int64_t outer, int64_t sx_batch, int64_t sx_outer,
@@ -184,49 +162,99 @@ __global__ void __launch_bounds__(256, sizeof(T) == 2 ? 3 : 2) downcast_rows_ker
   }
 }
 
-// ---- quantised axis strided, the other axis contiguous (axis 0 of a row-major matrix): a thread owns the 32-groups of
-// two neighbouring columns, so that a warp load covers 128 (bf16 / fp16) contiguous bytes; each column's codes are 16
-// contiguous bytes of the output.
-template <typename T>
-__global__ void __launch_bounds__(128) downcast_cols2_kernel(const T* __restrict__ x, int64_t batch, int64_t outer,
-                                                             int64_t quant, int64_t sx_batch, int64_t sx_quant,
-                                                             uint8_t* __restrict__ q, uint8_t* __restrict__ scale, int mode) {
-  const int64_t groups = quant >> 5;
-  const int64_t pairs = outer >> 1;
-  const int64_t total = batch * groups * pairs;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-    const int64_t op = i % pairs;
-    const int64_t t = i / pairs;
-    const int64_t g = t % groups;
-    const int64_t b = t / groups;
-    const T* src = x + b * sx_batch + g * 32 * sx_quant + op * 2;
-    float v0[32], v1[32];
+// ---- quantised axis strided, the other axis contiguous (expert weights quantised along K, axis 0 of a row-major matrix) --
+// HBM-bound.  A block takes 64 columns x 8 groups (256 elements of the quantised axis): warp = group, lane = two
+// neighbouring columns, so a warp load is 128 (bf16 / fp16) contiguous bytes and all 32 of a thread are in flight at once;
+// the raw pairs stay packed in registers (two columns' maxima by one packed max) and are unpacked only for the conversion.
+// Codes and scales meet in shared memory and leave as 128-byte runs of codes and 8-byte runs of scales per column:
+// stored from registers they were lone 16-byte and single-byte writes at the pitch of an output row (16 x 2880 x 5760
+// bf16, 671 MB moved: 221 us).
+constexpr int CT_COLS = 64, CT_GROUPS = 8;
+constexpr int CT_PITCH = CT_COLS * 16 + 16;          // bytes of one group's codes [column][16 B]; padded: a column's 8 groups on distinct banks
+
+template <typename T> struct Pair { using Raw = uint32_t; };
+template <> struct Pair<float> { using Raw = float2; };
+template <typename T> __device__ __forceinline__ float2 unpack_pair(typename Pair<T>::Raw w);
+template <> __device__ __forceinline__ float2 unpack_pair<__nv_bfloat16>(uint32_t w) {
+  return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xFFFF0000u));
+}
+template <> __device__ __forceinline__ float2 unpack_pair<__half>(uint32_t w) {
+  return __half22float2(*reinterpret_cast<const __half2*>(&w));
+}
+template <> __device__ __forceinline__ float2 unpack_pair<float>(float2 w) { return w; }
+// running |max| of both columns; NaN operands lose, as with fmaxf
+template <typename T> __device__ __forceinline__ float2 pair_absmax(const typename Pair<T>::Raw (&raw)[32]);
+template <> __device__ __forceinline__ float2 pair_absmax<__nv_bfloat16>(const uint32_t (&raw)[32]) {
+  __nv_bfloat162 m = __float2bfloat162_rn(0.0f);
 #pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      if constexpr (sizeof(T) == 2) {
-        const uint32_t w = *reinterpret_cast<const uint32_t*>(src + j * sx_quant);
-        if constexpr (std::is_same<T, __nv_bfloat16>::value) {
-          v0[j] = __uint_as_float(w << 16);
-          v1[j] = __uint_as_float(w & 0xFFFF0000u);
-        } else {
-          const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w));
-          v0[j] = f.x;
-          v1[j] = f.y;
-        }
-      } else {
-        const float2 f = *reinterpret_cast<const float2*>(src + j * sx_quant);
-        v0[j] = f.x;
-        v1[j] = f.y;
+  for (int j = 0; j < 32; ++j) m = __hmax2(m, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&raw[j])));
+  return make_float2(__low2float(m), __high2float(m));
+}
+template <> __device__ __forceinline__ float2 pair_absmax<__half>(const uint32_t (&raw)[32]) {
+  __half2 m = __float2half2_rn(0.0f);
+#pragma unroll
+  for (int j = 0; j < 32; ++j) m = __hmax2(m, __habs2(*reinterpret_cast<const __half2*>(&raw[j])));
+  return make_float2(__low2float(m), __high2float(m));
+}
+template <> __device__ __forceinline__ float2 pair_absmax<float>(const float2 (&raw)[32]) {
+  float2 m = make_float2(0.0f, 0.0f);
+#pragma unroll
+  for (int j = 0; j < 32; ++j) m = make_float2(fmaxf(m.x, fabsf(raw[j].x)), fmaxf(m.y, fabsf(raw[j].y)));
+  return m;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256, sizeof(T) == 2 ? 4 : 2) downcast_cols_kernel(
+    const T* __restrict__ x, int64_t outer, int groups, int col_blocks, int group_blocks, int64_t sx_batch, int64_t sx_quant,
+    uint8_t* __restrict__ q, uint8_t* __restrict__ scale, int mode) {
+  using Raw = typename Pair<T>::Raw;
+  __shared__ __align__(16) uint8_t s_q[CT_GROUPS * CT_PITCH];
+  __shared__ uint8_t s_s[CT_COLS * CT_GROUPS];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int cb = (int)(blockIdx.x % (unsigned)col_blocks);
+  const unsigned t = blockIdx.x / (unsigned)col_blocks;
+  const int gb = (int)(t % (unsigned)group_blocks);
+  const int64_t b = t / (unsigned)group_blocks;
+  const int64_t c0 = (int64_t)cb * CT_COLS;
+  const int g0 = gb * CT_GROUPS, g = g0 + warp;
+  const int64_t col = c0 + lane * 2;
+  if (g < groups && col < outer) {
+    const T* src = x + b * sx_batch + (int64_t)g * 32 * sx_quant + col;
+    Raw raw[32];
+#pragma unroll
+    for (int j = 0; j < 32; ++j) raw[j] = __ldcs(reinterpret_cast<const Raw*>(src + j * sx_quant));
+    const float2 m = pair_absmax<T>(raw);
+    const uint32_t u0 = scale_bits(m.x, mode), u1 = scale_bits(m.y, mode);
+    const float i0 = inv_scale(u0), i1 = inv_scale(u1);
+    uint32_t w0[4], w1[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      uint32_t b0[4], b1[4];
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        const float2 v = unpack_pair<T>(raw[8 * k + 2 * h]), n = unpack_pair<T>(raw[8 * k + 2 * h + 1]);
+        b0[h] = e2m1x2(v.x * i0, n.x * i0);
+        b1[h] = e2m1x2(v.y * i1, n.y * i1);
       }
+      w0[k] = __byte_perm(b0[0] | (b0[1] << 8), b0[2] | (b0[3] << 8), 0x5410);
+      w1[k] = __byte_perm(b1[0] | (b1[1] << 8), b1[2] | (b1[3] << 8), 0x5410);
     }
-    uint32_t s0, s1;
-    const uint4 c0 = quantise_group(v0, mode, s0), c1 = quantise_group(v1, mode, s1);
-    const int64_t row = b * outer + op * 2;
-    *reinterpret_cast<uint4*>(q + row * (quant >> 1) + g * 16) = c0;
-    *reinterpret_cast<uint4*>(q + (row + 1) * (quant >> 1) + g * 16) = c1;
-    scale[row * groups + g] = (uint8_t)(s0 >> 23);
-    scale[(row + 1) * groups + g] = (uint8_t)(s1 >> 23);
+    uint8_t* dst = s_q + warp * CT_PITCH + lane * 32;
+    *reinterpret_cast<uint4*>(dst) = make_uint4(w0[0], w0[1], w0[2], w0[3]);
+    *reinterpret_cast<uint4*>(dst + 16) = make_uint4(w1[0], w1[1], w1[2], w1[3]);
+    s_s[lane * 16 + warp] = (uint8_t)(u0 >> 23);
+    s_s[lane * 16 + 8 + warp] = (uint8_t)(u1 >> 23);
+  }
+  __syncthreads();
+  const int64_t row_bytes = (int64_t)groups * 16;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int p = threadIdx.x + i * 256, c = p >> 3, gi = p & 7;
+    if (c0 + c < outer && g0 + gi < groups) {
+      const int64_t row = b * outer + c0 + c;
+      *reinterpret_cast<uint4*>(q + row * row_bytes + (int64_t)(g0 + gi) * 16) = *reinterpret_cast<const uint4*>(s_q + gi * CT_PITCH + c * 16);
+      scale[row * groups + g0 + gi] = s_s[c * 8 + gi];
+    }
   }
 }
 
@@ -374,6 +402,64 @@ __global__ void __launch_bounds__(256) upcast_rows_kernel(const uint8_t* __restr
   }
 }
 
+// The inverse of downcast_cols_kernel: output contiguous along the other axis.  A block reads 64 columns x 8 groups of codes
+// (128-byte runs) through shared memory; warp = group, lane = two neighbouring columns, every store of a warp is 128
+// contiguous bytes (fp32: 256).  A thread per column and group stored 64-byte runs from loads at the pitch of a row.
+template <typename T>
+__global__ void __launch_bounds__(256) upcast_cols_kernel(const uint8_t* __restrict__ q, const uint8_t* __restrict__ scale,
+                                                          T* __restrict__ out, int64_t outer, int groups, int col_blocks,
+                                                          int group_blocks, int64_t so_batch, int64_t so_quant) {
+  __shared__ __align__(16) uint8_t s_q[CT_GROUPS * CT_PITCH];
+  __shared__ uint8_t s_s[CT_COLS * CT_GROUPS];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int cb = (int)(blockIdx.x % (unsigned)col_blocks);
+  const unsigned t = blockIdx.x / (unsigned)col_blocks;
+  const int gb = (int)(t % (unsigned)group_blocks);
+  const int64_t b = t / (unsigned)group_blocks;
+  const int64_t c0 = (int64_t)cb * CT_COLS;
+  const int g0 = gb * CT_GROUPS, g = g0 + warp;
+  const int64_t row_bytes = (int64_t)groups * 16;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int p = threadIdx.x + i * 256, c = p >> 3, gi = p & 7;
+    if (c0 + c < outer && g0 + gi < groups) {
+      const int64_t row = b * outer + c0 + c;
+      *reinterpret_cast<uint4*>(s_q + gi * CT_PITCH + c * 16) = *reinterpret_cast<const uint4*>(q + row * row_bytes + (int64_t)(g0 + gi) * 16);
+      s_s[c * 8 + gi] = scale[row * groups + g0 + gi];
+    }
+  }
+  __syncthreads();
+  const int64_t col = c0 + lane * 2;
+  if (g >= groups || col >= outer) return;
+  const uint4 a0 = *reinterpret_cast<const uint4*>(s_q + warp * CT_PITCH + lane * 32);
+  const uint4 a1 = *reinterpret_cast<const uint4*>(s_q + warp * CT_PITCH + lane * 32 + 16);
+  const uint32_t sb0 = s_s[lane * 16 + warp], sb1 = s_s[lane * 16 + 8 + warp];
+  const uint32_t w0[4] = {a0.x, a0.y, a0.z, a0.w}, w1[4] = {a1.x, a1.y, a1.z, a1.w};
+  T* dst = out + b * so_batch + (int64_t)g * 32 * so_quant + col;
+  if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+    if (sb0 < 253u && sb1 < 253u) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const uint4 v0 = upcast8_bf16(w0[k], sb0), v1 = upcast8_bf16(w1[k], sb1);       // pairs of elements of one column
+        const uint32_t p0[4] = {v0.x, v0.y, v0.z, v0.w}, p1[4] = {v1.x, v1.y, v1.z, v1.w};
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          *reinterpret_cast<uint32_t*>(dst + (8 * k + 2 * h) * so_quant) = __byte_perm(p0[h], p1[h], 0x5410);
+          *reinterpret_cast<uint32_t*>(dst + (8 * k + 2 * h + 1) * so_quant) = __byte_perm(p0[h], p1[h], 0x7632);
+        }
+      }
+      return;
+    }
+  }
+  const float f0 = __uint_as_float(sb0 << 23), f1 = __uint_as_float(sb1 << 23);
+  const bool n0 = sb0 == 0xFFu, n1 = sb1 == 0xFFu;
+#pragma unroll
+  for (int j = 0; j < 32; ++j) {
+    T e[2] = {dequant_one<T>((w0[j >> 3] >> (4 * (j & 7))) & 0xFu, f0, n0), dequant_one<T>((w1[j >> 3] >> (4 * (j & 7))) & 0xFu, f1, n1)};
+    *reinterpret_cast<typename Pair<T>::Raw*>(dst + j * so_quant) = *reinterpret_cast<const typename Pair<T>::Raw*>(e);
+  }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256) upcast_strided_kernel(const uint8_t* __restrict__ q,
                                                              const uint8_t* __restrict__ scale, T* __restrict__ out,
@@ -399,6 +485,10 @@ __global__ void __launch_bounds__(256) upcast_strided_kernel(const uint8_t* __re
   }
 }
 
+int64_t col_tiles(int64_t batch, int64_t outer, int64_t quant) {       // blocks of the column kernels
+  return batch * cdiv64(outer, CT_COLS) * cdiv64(quant >> 5, CT_GROUPS);
+}
+
 int grid_for(int64_t total, int threads) {
   int64_t blocks = cdiv64(total, threads);
   int64_t cap = (int64_t)moe_sm_count() * 16;
@@ -422,9 +512,10 @@ extern "C" __attribute__((visibility("default"))) int moe_downcast_mxfp4(const v
     const int64_t align = 16 / (int64_t)sizeof(T);
     const bool rows_ok = sx_quant == 1 && ((uintptr_t)x % 16 == 0) && (sx_outer % align == 0) &&
                          (sx_batch % align == 0) && ((uintptr_t)q % 4 == 0);
-    const int64_t align2 = 2;                                         // two columns per thread: 4- or 8-byte loads
-    const bool cols2_ok = sx_outer == 1 && sx_quant != 1 && outer % 2 == 0 && ((uintptr_t)x % (2 * sizeof(T)) == 0) &&
-                          (sx_quant % align2 == 0) && (sx_batch % align2 == 0) && ((uintptr_t)q % 16 == 0);
+    // two columns per thread: 4- or 8-byte loads
+    const bool cols_ok = sx_outer == 1 && sx_quant != 1 && outer % 2 == 0 && ((uintptr_t)x % (2 * sizeof(T)) == 0) &&
+                         (sx_quant % 2 == 0) && (sx_batch % 2 == 0) && ((uintptr_t)q % 16 == 0) &&
+                         col_tiles(batch, outer, quant) < 2147483647LL;
     if (rows_ok && (uintptr_t)q % 16 == 0) {
       const int64_t total = batch * outer * (quant >> 5);
       if (total + (int64_t)GROUPS_UNROLL * 256 * moe_sm_count() * 16 < 2147483647LL)       // 32-bit row / group counters
@@ -433,10 +524,11 @@ extern "C" __attribute__((visibility("default"))) int moe_downcast_mxfp4(const v
       else
         downcast_rows_kernel<T, int64_t><<<grid_for(total, GROUPS_UNROLL * 256), 256, 0, st>>>(
             (const T*)x, batch * outer, quant, outer, sx_batch, sx_outer, q, scale, rounding_mode);
-    } else if (cols2_ok) {
-      const int64_t total = batch * (outer >> 1) * (quant >> 5);
-      downcast_cols2_kernel<T><<<grid_for(total, 128), 128, 0, st>>>((const T*)x, batch, outer, quant, sx_batch, sx_quant, q,
-                                                                     scale, rounding_mode);
+    } else if (cols_ok) {
+      const int groups = (int)(quant >> 5);
+      downcast_cols_kernel<T><<<(unsigned)col_tiles(batch, outer, quant), 256, 0, st>>>(
+          (const T*)x, outer, groups, (int)cdiv64(outer, CT_COLS), (int)cdiv64(groups, CT_GROUPS), sx_batch, sx_quant, q, scale,
+          rounding_mode);
     } else {
       MOE_CHECK_ARG((uintptr_t)q % 16 == 0, "moe_downcast_mxfp4: q must be 16-byte aligned");
       const int64_t total = batch * outer * (quant >> 5);
@@ -464,6 +556,11 @@ extern "C" __attribute__((visibility("default"))) int moe_upcast_mxfp4(const uin
       const int64_t total = batch * outer * (quant >> 3);
       upcast_rows_kernel<T><<<grid_for(total, ROWS_UNROLL * 256), 256, 0, st>>>(q, scale, (T*)out, batch * outer, quant, outer,
                                                                   so_batch, so_outer);
+    } else if (so_outer == 1 && so_quant % 2 == 0 && so_batch % 2 == 0 && outer % 2 == 0 && (uintptr_t)q % 16 == 0 &&
+               (uintptr_t)out % (2 * sizeof(T)) == 0 && col_tiles(batch, outer, quant) < 2147483647LL) {
+      const int groups = (int)(quant >> 5);
+      upcast_cols_kernel<T><<<(unsigned)col_tiles(batch, outer, quant), 256, 0, st>>>(
+          q, scale, (T*)out, outer, groups, (int)cdiv64(outer, CT_COLS), (int)cdiv64(groups, CT_GROUPS), so_batch, so_quant);
     } else {
       MOE_CHECK_ARG((uintptr_t)q % 16 == 0, "moe_upcast_mxfp4: q must be 16-byte aligned");
       const int64_t total = batch * outer * (quant >> 5);

@@ -145,14 +145,18 @@ def wrap_torch_tensor(torch_tensor, dtype=None, shape=None, shape_max=None, layo
 
 
 def convert_layout(tensor: Tensor, layout: Layout, **kwargs):
-    """Re-encode `tensor` storage as `layout` (through the canonical row-major form).  Returns `tensor`
-    unchanged when its storage already is a valid encoding of `layout`."""
+    """Re-encode `tensor` storage as `layout` (through the canonical row-major form, unless `layout` can be written straight
+    from the strided storage).  Returns `tensor` unchanged when its storage already is a valid encoding of `layout`."""
     shape = list(tensor.shape)
     if not kwargs and tensor.storage.layout.can_preserve_storage_as(layout, len(shape)):
         return tensor
     is_fp4 = tensor.dtype == FP4
-    canonical = tensor.storage.layout.make_transformation(shape, is_fp4).unswizzle_data(tensor.storage.data)
-    new_data = layout.make_transformation(shape, is_fp4, **kwargs).swizzle_data(canonical)
+    old, new = tensor.storage.layout.make_transformation(shape, is_fp4), layout.make_transformation(shape, is_fp4, **kwargs)
+    new_data = None
+    if isinstance(tensor.storage.layout, StridedLayout) and hasattr(new, "swizzle_strided"):
+        new_data = new.swizzle_strided(tensor.storage.data, old.order)
+    if new_data is None:
+        new_data = new.swizzle_data(old.unswizzle_data(tensor.storage.data))
     return Tensor(Storage(new_data, layout), shape=shape, dtype=tensor.dtype)
 
 

@@ -33,6 +33,15 @@ def _tiles(shape):
     return E, K, N, (N + TILE - 1) // TILE, (K + TILE - 1) // TILE
 
 
+def _strided3(data, lead):
+    """`data` as [E, rows, cols] without a copy, or None when the leading dimensions do not collapse."""
+    if len(lead) == 1:
+        return data
+    if len(lead) == 0:
+        return data.unsqueeze(0)
+    return None
+
+
 @dataclass(frozen=True)
 class B200MXValueLayout(Layout):
 
@@ -65,17 +74,30 @@ class B200MXValueLayoutTransformation(LayoutTransformation):
         E, K, N, NT, KT = _tiles(self.shape)
         return [E * NT * KT * TILE * (TILE // 2)]
 
+    _to_tiles = "moe_weight_layout_to_b200"
+
+    def _tile(self, q, stride_e, stride_n):
+        E, K, N, NT, KT = _tiles(self.shape)
+        assert K % 32 == 0, "MXFP4 weights need K % 32 == 0"
+        out = torch.empty(self.storage_shape, dtype=torch.uint8, device=q.device)
+        _lib.check(getattr(_lib.load(), self._to_tiles)(_lib.ptr(q), stride_e, stride_n, None, 0, 0, 0, E, K, N, _lib.ptr(out),
+                                                        None, _lib.stream()), self._to_tiles)
+        return out
+
     def swizzle_data(self, data):
         from .strided import repack
         E, K, N, NT, KT = _tiles(self.shape)
-        assert K % 32 == 0, "MXFP4 weights need K % 32 == 0"
         q = repack(data.reshape(E, K, N // 2), -1, -2, True)            # [E, K/2, N]
         q = q.transpose(-1, -2).contiguous()                            # [E, N, K/2], K contiguous
-        out = torch.empty(self.storage_shape, dtype=torch.uint8, device=data.device)
-        lib = _lib.load()
-        _lib.check(lib.moe_weight_layout_to_b200(_lib.ptr(q), N * (K // 2), K // 2, None, 0, 0, 0, E, K, N,
-                                                 _lib.ptr(out), None, _lib.stream()), "moe_weight_layout_to_b200")
-        return out
+        return self._tile(q, N * (K // 2), K // 2)
+
+    def swizzle_strided(self, data, order):
+        """From strided storage packed along K (what `downcast_to_mxfp(w, axis=-2)` returns): the tiling kernel reads it in
+        place.  -> tiles, or None when the storage is packed otherwise."""
+        q = _strided3(data, self.shape[:-2])
+        if q is None or order[0] != len(self.shape) - 2 or q.stride(1) != 1 or self.shape[-2] % 32 != 0:
+            return None
+        return self._tile(q, q.stride(0), q.stride(2))
 
     def unswizzle_data(self, data):
         from .strided import repack
@@ -99,15 +121,24 @@ class B200MXScaleLayoutTransformation(LayoutTransformation):
         E, K, N, NT, KT = _tiles([*lead, KG * 32, N])
         return [E * NT * KT * TILE * 4]
 
-    def swizzle_data(self, data):
+    _to_tiles = "moe_weight_layout_to_b200"
+
+    def _tile(self, s):
         *lead, KG, N = self.shape
         E, K, N, NT, KT = _tiles([*lead, KG * 32, N])
-        s = data.reshape(E, KG, N).contiguous()
-        out = torch.empty(self.storage_shape, dtype=torch.uint8, device=data.device)
-        lib = _lib.load()
-        _lib.check(lib.moe_weight_layout_to_b200(None, 0, 0, _lib.ptr(s), KG * N, N, 1, E, K, N, None, _lib.ptr(out),
-                                                 _lib.stream()), "moe_weight_layout_to_b200")
+        out = torch.empty(self.storage_shape, dtype=torch.uint8, device=s.device)
+        _lib.check(getattr(_lib.load(), self._to_tiles)(None, 0, 0, _lib.ptr(s), s.stride(0), s.stride(1), s.stride(2), E, K, N,
+                                                        None, _lib.ptr(out), _lib.stream()), self._to_tiles)
         return out
+
+    def swizzle_data(self, data):
+        *lead, KG, N = self.shape
+        return self._tile(data.reshape(-1, KG, N).contiguous())
+
+    def swizzle_strided(self, data, order):
+        """From any strided storage, read in place; None when the leading dimensions do not collapse."""
+        s = _strided3(data, self.shape[:-2])
+        return None if s is None else self._tile(s)
 
     def unswizzle_data(self, data):
         *lead, KG, N = self.shape
@@ -147,16 +178,7 @@ class B200BlockScaledScaleLayout(Layout):
 class B200BlockScaledValueLayoutTransformation(B200MXValueLayoutTransformation):
     """Same sizes as B200MXValueLayoutTransformation; tiles ordered [E][k_tile][n_block], nibbles in natural order."""
 
-    def swizzle_data(self, data):
-        from .strided import repack
-        E, K, N, NT, KT = _tiles(self.shape)
-        assert K % 32 == 0, "MXFP4 weights need K % 32 == 0"
-        q = repack(data.reshape(E, K, N // 2), -1, -2, True).transpose(-1, -2).contiguous()     # [E, N, K/2]
-        out = torch.empty(self.storage_shape, dtype=torch.uint8, device=data.device)
-        lib = _lib.load()
-        _lib.check(lib.moe_weight_layout_to_b200mx(_lib.ptr(q), N * (K // 2), K // 2, None, 0, 0, 0, E, K, N,
-                                                   _lib.ptr(out), None, _lib.stream()), "moe_weight_layout_to_b200mx")
-        return out
+    _to_tiles = "moe_weight_layout_to_b200mx"
 
     def unswizzle_data(self, data):
         from .strided import repack
@@ -172,15 +194,7 @@ class B200BlockScaledValueLayoutTransformation(B200MXValueLayoutTransformation):
 @dataclass(frozen=True)
 class B200BlockScaledScaleLayoutTransformation(B200MXScaleLayoutTransformation):
 
-    def swizzle_data(self, data):
-        *lead, KG, N = self.shape
-        E, K, N, NT, KT = _tiles([*lead, KG * 32, N])
-        s = data.reshape(E, KG, N).contiguous()
-        out = torch.empty(self.storage_shape, dtype=torch.uint8, device=data.device)
-        lib = _lib.load()
-        _lib.check(lib.moe_weight_layout_to_b200mx(None, 0, 0, _lib.ptr(s), KG * N, N, 1, E, K, N, None, _lib.ptr(out),
-                                                   _lib.stream()), "moe_weight_layout_to_b200mx")
-        return out
+    _to_tiles = "moe_weight_layout_to_b200mx"
 
     def unswizzle_data(self, data):
         *lead, KG, N = self.shape

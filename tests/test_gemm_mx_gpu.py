@@ -296,3 +296,42 @@ def test_block_scaled_few_tiles_k_step_stages(K, sizes, act, device):
     y = run_mx(x, wq, ws, sizes_t, device, bias=bias, scatter=scatter, gammas=gammas, act=a, out_dtype=torch.float32,
                kernel="mx-f4", block_m=16)
     assert oracle.rel_l2(out, y) < 5e-4
+
+
+@pytest.mark.parametrize("acts", ["bf16", "fp8", "mxfp8"])
+@pytest.mark.parametrize("K, N, sizes", [
+    (32, 2, [1, 0, 33]),                            # one group of k, one column pair
+    (128, 256, [192, 193, 224, 225]),               # one whole k step, one 256-row block, around the tile of either form
+    (160, 129, [31, 32, 5, 449]),                   # k tail, odd width (scalar stores), an expert of several tiles
+    (416, 514, [64, 1, 0, 97]),                     # ring longer than the k loop, a second tile of weight blocks
+    (1024, 768, [300]),                             # three 256-row blocks: the last tile has one unit
+])
+@pytest.mark.parametrize("act", [False, True])
+def test_pair_kernel_tile_edges(K, N, sizes, acts, act, device):
+    """The pair form at the edges of its tiles, fp32 outputs.  e4m3 products and the two e4m3 terms of a bf16 value are
+    exact, so only the order of an fp32 sum of K terms differs: 2e-5 of the norm is far above its error."""
+    if act and N % 2:
+        pytest.skip("SwiGLU needs an even width")
+    g = torch.Generator().manual_seed(K + N + len(sizes))
+    E, M = len(sizes), sum(sizes)
+    sizes_t = torch.tensor(sizes, dtype=torch.int32)
+    wq, ws, wdeq = quantised_weights(E, K, N, g)
+    T = M + 7
+    x = torch.randn(T, K, generator=g).bfloat16()
+    a_scale = None
+    if acts != "bf16":
+        x = x.to(torch.float8_e4m3fn)
+        if acts == "mxfp8":
+            a_scale = torch.randint(122, 131, (T, K // 32), generator=g, dtype=torch.uint8)
+    xref = x.float() if acts == "bf16" else dequant_act(x, a_scale)
+    gather = torch.randint(0, T, (M,), generator=g, dtype=torch.int32)
+    scatter, gammas, betas = torch.randperm(M, generator=g).int(), torch.rand(M, generator=g), torch.rand(M, generator=g)
+    bias = torch.randn(E, N, generator=g) * 0.1
+    ref = oracle.matmul_oracle(xref[gather.long()], wdeq, bias, sizes_t, None, None, betas=betas, out_dtype=torch.float32)
+    if act:
+        ref = oracle.swiglu_oracle(ref, 1.702, 7.0)
+    out = torch.zeros_like(ref)
+    out[scatter.long()] = ref * gammas[:, None]
+    y = run_mx(x, wq, ws, sizes_t, device, a_scale=a_scale, bias=bias, gather=gather, scatter=scatter, gammas=gammas, betas=betas,
+               act=(1.702, 7.0) if act else None, out_dtype=torch.float32, block_m=256)
+    assert oracle.rel_l2(out, y) < 2e-5

@@ -33,16 +33,8 @@
 //   scales -> tensor memory through registers (tcgen05.st by four loader warps), then MB x 4 MMAs of K = 32.
 // Warps: 0 producer (one thread), 1 MMA issue + tensor-memory owner, 2-5 epilogue, 6-9 scale loaders.  Every mbarrier
 // wait is bounded.
-#include "gemm_tc_common.cuh"
-#include <cuda_fp8.h>
+#include "gemm_mx_common.cuh"
 #include <utility>
-
-// e4m3 output (the next GEMM's activations): round to nearest, saturating at +-448 like the MMA's own conversions
-template <> __device__ __forceinline__ __nv_fp8_e4m3 from_f32<__nv_fp8_e4m3>(float v) {
-  __nv_fp8_e4m3 r;
-  r.__x = __nv_cvt_float_to_fp8(v, __NV_SATFINITE, __NV_E4M3);
-  return r;
-}
 
 namespace {
 
@@ -142,27 +134,6 @@ struct PackParams {
   int64_t chunk_bytes;
   uint8_t* out;
 };
-
-__device__ __forceinline__ uint32_t f32x2_to_e4m3x2(float lo, float hi) {       // low byte <- lo, high byte <- hi
-  uint16_t r;
-  asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(r) : "f"(hi), "f"(lo));
-  return r;
-}
-__device__ __forceinline__ float2 e4m3x2_to_f32x2(uint32_t v) {
-  uint32_t h2;
-  asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(h2) : "h"((uint16_t)v));
-  return __half22float2(*reinterpret_cast<__half2*>(&h2));
-}
-// e8m0 byte s with 2^(s-127) >= amax / 448 (smallest such power of two), and the exact factors 2^(s-127), 2^(127-s)
-__device__ __forceinline__ void mx8_scale(float amax, uint32_t& sb, float& scale, float& inv) {
-  const float ds = amax * (1.0f / 448.0f);
-  uint32_t u = (__float_as_uint(ds) + 0x007FFFFFu) & 0x7F800000u;
-  sb = u >> 23;
-  if (amax == 0.0f) sb = 127u;
-  sb = min(max(sb, 1u), 253u);
-  scale = __uint_as_float(sb << 23);
-  inv = __uint_as_float((254u - sb) << 23);
-}
 
 template <bool SPLIT>
 __global__ void __launch_bounds__(256) mx_pack_x_kernel(const GemmParams p, const PackParams a) {
@@ -306,13 +277,6 @@ __global__ void __launch_bounds__(256) mx_pack_x4_kernel(const GemmParams p, con
 // ============================================================================================================
 // PTX pieces of the block-scaled path
 // ============================================================================================================
-// 3-D tile copy: box (128 elements, 128 rows, MB tiles) of the weight tensor map, starting at tile `z`
-__device__ __forceinline__ void tma_tile_3d(uint32_t dst, const CUtensorMap* tmap, int x, int y, int z, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
-      "l"(tmap), "r"(x), "r"(y), "r"(z), "r"(bar)
-      : "memory");
-}
 // instruction descriptor of kind::mxf8f6f4: A = e2m1 (code 5), B = e4m3 (code 0), both K-major, e8m0 scales,
 // M = 128, N = n; sf selects the byte (k group) of the scale words for A and B
 __device__ __forceinline__ uint32_t mx_idesc(int n, uint32_t sf) {
@@ -752,42 +716,6 @@ MxPlan mx_plan(const MoeGemmArgs& a) {
   return pl;
 }
 
-int make_w_map(const MoeGemmArgs& a, const MxPlan& pl, int n_blocks, CUtensorMap* map) {
-  static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
-  static std::mutex mu;
-  {
-    std::lock_guard<std::mutex> lk(mu);
-    if (!encode) {
-      void* fn = nullptr;
-      cudaDriverEntryPointQueryResult qr;
-      MOE_CHECK_CUDA(cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &qr));
-      if (qr != cudaDriverEntryPointSuccess || !fn) {
-        moe_set_error("moe_grouped_gemm: the driver does not provide cuTensorMapEncodeTiled");
-        return MOE_ERR_UNSUPPORTED;
-      }
-      encode = (PFN_cuTensorMapEncodeTiled_v12000)fn;
-    }
-  }
-  // [tile][128 rows][128 e2m1 = 64 bytes].  Byte-per-element form: the TMA unit writes 16 elements per 16 bytes of
-  // shared memory (128-byte rows, 128-byte swizzle); packed form: the 64-byte rows as they are, 64-byte swizzle.
-  const cuuint64_t tiles = (cuuint64_t)a.E * (cuuint64_t)pl.KT * (cuuint64_t)pl.NB;
-  const cuuint64_t inner = pl.f4 ? 64 : 128;
-  const cuuint64_t dims[3] = {inner, 128, tiles};
-  const cuuint64_t strides[2] = {64, 64 * 128};
-  const cuuint32_t box[3] = {(cuuint32_t)inner, 128, (cuuint32_t)n_blocks};
-  const cuuint32_t estr[3] = {1, 1, 1};
-  const CUresult r = encode(map, pl.f4 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_16U4_ALIGN16B, 3,
-                            const_cast<void*>(a.w), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                            pl.f4 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    moe_set_error("moe_grouped_gemm: cuTensorMapEncodeTiled (packed e2m1 weights) failed with code %d (%llu tiles)", (int)r,
-                  (unsigned long long)tiles);
-    return MOE_ERR_CUDA;
-  }
-  return MOE_OK;
-}
-
 // launch with the programmatic-stream-serialization attribute (see pdl_wait above)
 template <typename... KArgs, typename... Args>
 cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
@@ -826,6 +754,10 @@ int launch_mx_ty(const GemmParams& p, const MxParams& q, const MxPlan& pl, const
 
 }  // namespace
 
+bool moe_gemm_mx_pair_wanted(const MoeGemmArgs& a);
+int64_t moe_gemm_mx_pair_workspace(const MoeGemmArgs& a);
+int moe_gemm_mx_pair_launch(const GemmParams& p, const MoeGemmArgs& a, cudaStream_t st);
+
 bool moe_gemm_mx_supported(const MoeGemmArgs& a, const char** why) {
   if (a.w_kind != MOE_W_MX4_B200MX) { *why = "weights are not in the block-scaled B200 layout"; return false; }
   if (a.x_dtype != MOE_BF16 && a.x_dtype != MOE_F8E4M3) { *why = "activations are neither bf16 nor e4m3"; return false; }
@@ -844,10 +776,11 @@ bool moe_gemm_mx_supported(const MoeGemmArgs& a, const char** why) {
 
 extern "C" __attribute__((visibility("default"))) size_t moe_gemm_mx_workspace_bytes(const MoeGemmArgs* a) {
   if (!a || a->M <= 0 || a->E <= 0) return 0;
-  return (size_t)mx_plan(*a).ws_bytes;
+  return (size_t)(moe_gemm_mx_pair_wanted(*a) ? moe_gemm_mx_pair_workspace(*a) : mx_plan(*a).ws_bytes);
 }
 
 int moe_gemm_mx_launch(const GemmParams& p_in, const MoeGemmArgs& a, cudaStream_t st) {
+  if (moe_gemm_mx_pair_wanted(a)) return moe_gemm_mx_pair_launch(p_in, a, st);
   const MxPlan pl = mx_plan(a);
   if (pl.grid_m == 0) return MOE_OK;
   MOE_CHECK_ARG(a.mx_workspace != nullptr && a.mx_workspace_bytes >= pl.ws_bytes && (uintptr_t)a.mx_workspace % 1024 == 0,
@@ -882,7 +815,7 @@ int moe_gemm_mx_launch(const GemmParams& p_in, const MoeGemmArgs& a, cudaStream_
   q.n_groups = pl.n_groups; q.grid_m = pl.grid_m;
   MxMaps w_map;
   for (int nb = 1; nb <= 3; ++nb)
-    if (int rc = make_w_map(a, pl, nb <= pl.mb ? nb : pl.mb, &w_map.m[nb - 1])) return rc;
+    if (int rc = make_w_map(a, pl.KT, pl.NB, pl.f4 != 0, nb <= pl.mb ? nb : pl.mb, &w_map.m[nb - 1])) return rc;
   const int idle = a.idle_sms > 0 ? a.idle_sms : 0;
   if (a.y_dtype == MOE_F8E4M3) return launch_mx_ty<__nv_fp8_e4m3>(p, q, pl, w_map, idle, st);
   if (a.y_dtype == MOE_BF16) return launch_mx_ty<__nv_bfloat16>(p, q, pl, w_map, idle, st);

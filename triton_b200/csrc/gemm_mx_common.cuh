@@ -1,0 +1,81 @@
+// Pieces shared by the block-scaled GEMM kernels: e4m3 conversions and their e8m0 scales, the weight tensor map.
+#pragma once
+#include "gemm_tc_common.cuh"
+#include <cuda_fp8.h>
+
+// e4m3 output (the next GEMM's activations): round to nearest, saturating at +-448 like the MMA's own conversions
+template <> __device__ __forceinline__ __nv_fp8_e4m3 from_f32<__nv_fp8_e4m3>(float v) {
+  __nv_fp8_e4m3 r;
+  r.__x = __nv_cvt_float_to_fp8(v, __NV_SATFINITE, __NV_E4M3);
+  return r;
+}
+
+namespace {
+
+__device__ __forceinline__ uint32_t f32x2_to_e4m3x2(float lo, float hi) {       // low byte <- lo, high byte <- hi
+  uint16_t r;
+  asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(r) : "f"(hi), "f"(lo));
+  return r;
+}
+__device__ __forceinline__ float2 e4m3x2_to_f32x2(uint32_t v) {
+  uint32_t h2;
+  asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(h2) : "h"((uint16_t)v));
+  return __half22float2(*reinterpret_cast<__half2*>(&h2));
+}
+// e8m0 byte s with 2^(s-127) >= amax / 448 (smallest such power of two), and the exact factors 2^(s-127), 2^(127-s)
+__device__ __forceinline__ void mx8_scale(float amax, uint32_t& sb, float& scale, float& inv) {
+  const float ds = amax * (1.0f / 448.0f);
+  uint32_t u = (__float_as_uint(ds) + 0x007FFFFFu) & 0x7F800000u;
+  sb = u >> 23;
+  if (amax == 0.0f) sb = 127u;
+  sb = min(max(sb, 1u), 253u);
+  scale = __uint_as_float(sb << 23);
+  inv = __uint_as_float((254u - sb) << 23);
+}
+
+// 3-D tile copy: box (128 elements, 128 rows, MB tiles) of the weight tensor map, starting at tile `z`
+__device__ __forceinline__ void tma_tile_3d(uint32_t dst, const CUtensorMap* tmap, int x, int y, int z, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
+      "l"(tmap), "r"(x), "r"(y), "r"(z), "r"(bar)
+      : "memory");
+}
+// Tensor map over the value tiles of the block-scaled layout, boxes of n_blocks tiles; `packed`: 64-byte rows as they are,
+// else expanded by the TMA unit for kind::mxf8f6f4.
+inline int make_w_map(const MoeGemmArgs& a, int KT, int NB, bool packed, int n_blocks, CUtensorMap* map) {
+  static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
+  static std::mutex mu;
+  {
+    std::lock_guard<std::mutex> lk(mu);
+    if (!encode) {
+      void* fn = nullptr;
+      cudaDriverEntryPointQueryResult qr;
+      MOE_CHECK_CUDA(cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &qr));
+      if (qr != cudaDriverEntryPointSuccess || !fn) {
+        moe_set_error("moe_grouped_gemm: the driver does not provide cuTensorMapEncodeTiled");
+        return MOE_ERR_UNSUPPORTED;
+      }
+      encode = (PFN_cuTensorMapEncodeTiled_v12000)fn;
+    }
+  }
+  // [tile][128 rows][128 e2m1 = 64 bytes].  Byte-per-element form: the TMA unit writes 16 elements per 16 bytes of
+  // shared memory (128-byte rows, 128-byte swizzle); packed form: the 64-byte rows as they are, 64-byte swizzle.
+  const cuuint64_t tiles = (cuuint64_t)a.E * (cuuint64_t)KT * (cuuint64_t)NB;
+  const cuuint64_t inner = packed ? 64 : 128;
+  const cuuint64_t dims[3] = {inner, 128, tiles};
+  const cuuint64_t strides[2] = {64, 64 * 128};
+  const cuuint32_t box[3] = {(cuuint32_t)inner, 128, (cuuint32_t)n_blocks};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult r = encode(map, packed ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_16U4_ALIGN16B, 3,
+                            const_cast<void*>(a.w), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                            packed ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    moe_set_error("moe_grouped_gemm: cuTensorMapEncodeTiled (packed e2m1 weights) failed with code %d (%llu tiles)", (int)r,
+                  (unsigned long long)tiles);
+    return MOE_ERR_CUDA;
+  }
+  return MOE_OK;
+}
+
+}  // namespace

@@ -20,8 +20,7 @@
 // the commit after a tile's last MMA; ACC_EMPTY lives in the even CTA and collects the eight epilogue warps of the
 // pair.  Every wait is bounded like in the single-SM kernel; both CTAs meet at a cluster barrier before tensor
 // memory is released.
-#include "gemm_tc_common.cuh"
-#include <mutex>
+#include "gemm_pair_common.cuh"
 
 namespace {
 
@@ -49,52 +48,6 @@ struct PairSmem {
   static_assert(ALLOC <= 232448, "shared memory budget");
 };
 
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// Arrive on the barrier at the same shared-memory offset in CTA `cta` of the cluster.  Default (CTA-scope release)
-// semantics: a cluster-scope release costs about a thousand cycles per arrival while copies are in flight, and what
-// the arrival publishes here is either a go-ahead for the tensor core of the SM that already holds the data (stage
-// full) or the end of tensor-memory reads that were fenced by tcgen05.fence (accumulator drained).
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar, uint32_t cta) {
-  asm volatile(
-      "{\n\t.reg .b32 ra;\n\t"
-      "mapa.shared::cluster.u32 ra, %0, %1;\n\t"
-      "mbarrier.arrive.shared::cluster.b64 _, [ra];\n\t}" ::"r"(bar),
-      "r"(cta)
-      : "memory");
-}
-__device__ __forceinline__ bool mbar_try_cluster(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// bounded wait on a barrier that threads of the other CTA arrive on
-__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, const Ctl& ctl, int code) {
-  if (mbar_try_cluster(bar, parity)) return true;
-  const unsigned long long t0 = global_ns();
-  for (;;) {
-    if (mbar_try_cluster(bar, parity)) return true;
-    if (*ctl.abort_flag) return false;
-    if (global_ns() - t0 > WAIT_LIMIT_NS) {
-      *ctl.abort_flag = 1;
-      if (ctl.status) atomicExch(ctl.status, code);
-      return false;
-    }
-  }
-}
-
 // instruction descriptor of the pair MMA: D fp32, A/B bf16, both K-major, M = 256 over the two CTAs
 __device__ __forceinline__ constexpr uint32_t make_idesc_pair(int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
@@ -108,17 +61,6 @@ __device__ __forceinline__ void mma_bf16_pair(uint32_t d_tmem, uint64_t adesc, u
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// arrive on the barrier at this offset in both CTAs of the pair once every MMA issued so far has completed
-__device__ __forceinline__ void mma_commit_pair(uint32_t bar) {
-  asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
-      "h"((uint16_t)3)
-      : "memory");
-}
-__device__ __forceinline__ void mma_commit_pair_local(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-
 template <typename TY>
 __global__ void __launch_bounds__(PAIR_THREADS, 1)
 gemm_tc_pair_kernel(const GemmParams p, const int64_t grid_m_static, const __grid_constant__ CUtensorMap x_map) {

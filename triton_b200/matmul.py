@@ -115,6 +115,9 @@ _STATUS_TEXT = {
     603: "block-scaled kernel: the MMA thread waited for a free accumulator", 604: "block-scaled kernel: the epilogue waited for an accumulator",
     605: "block-scaled kernel: the final MMA drain", 606: "block-scaled kernel: the MMA thread waited for scales",
     607: "block-scaled kernel: a scale loader waited for a stage",
+    611: "block-scaled pair kernel: the producer waited for a free stage", 612: "block-scaled pair kernel: the MMA warp waited for scales",
+    613: "block-scaled pair kernel: the MMA warp waited for a free accumulator", 614: "block-scaled pair kernel: the final MMA drain",
+    615: "block-scaled pair kernel: a scale loader waited for a stage", 616: "block-scaled pair kernel: the epilogue waited for an accumulator",
     801: "router kernel: the producer waited for a free stage", 802: "router kernel: the MMA thread waited for a stage",
     803: "router kernel: the final MMA drain", 804: "router kernel: the selection waited for the accumulator",
     901: "expert-parallel peer barrier: a rank did not arrive within the limit; the step after it read stale peer buffers",

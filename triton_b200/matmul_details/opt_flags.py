@@ -1,8 +1,8 @@
 """User-visible tuning overrides for `matmul` (triton_kernels/matmul_details/opt_flags.py:482-532).
 
 The constraint dictionary is context-local.  Keys understood here: ``kernel`` ("auto", "simt", "tcgen05", "tcgen05-pair",
-"stream", "mx", "mx-f8", "mx-f4"), ``block_m`` (token rows per tile: 16 / 32 / 64 / 128 for the block-scaled kernel, 128 / 256 for the bf16
-tensor-core kernel, whose 128-row tile spans only the rows present in steps of 16), ``block_n`` (128 / 256 / 384),
+"stream", "mx", "mx-f8", "mx-f4"), ``block_m`` (token rows per tile: 16 / 32 / 64 / 128 for the block-scaled kernel, 256 for its form on
+pairs of SMs; 128 / 256 for the bf16 tensor-core kernel, whose 128-row tile spans only the rows present in steps of 16), ``block_n`` (128 / 256 / 384),
 ``idle_sms``.  Every other tile-shape key of the reference may be given only the value the CUDA kernels are built with
 (``block_k`` 64 or 128, ``split_k`` 1, ``is_persistent`` True, the rest None); anything else raises
 InapplicableConstraint, which the reference's tests treat as "skip"."""
@@ -66,7 +66,7 @@ def scoped_opt_flags_constraints(constraints):
 
 def resolve_tile_m() -> int:
     """`block_m` constraint -> token rows per tile (0 = heuristic).  The bf16 tensor-core kernel knows 128 and 256,
-    the block-scaled kernel 16, 32, 64 and 128; each kernel ignores a value it does not have."""
+    the block-scaled kernel 16, 32, 64, 128 and (pairs of SMs) 256; each kernel ignores a value it does not have."""
     bm = get_opt_flags_constraints().get("block_m")
     return bm if bm in (16, 32, 64, 128, 256) else 0
 

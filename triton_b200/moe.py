@@ -43,22 +43,30 @@ class MoeLayerWeights:
     w1_bs_scale: Tensor | None = None
     w2_bs: Tensor | None = None
     w2_bs_scale: Tensor | None = None
-    block_scaled_max_rows_per_expert: int = 48       # measured crossover: 32 rows per expert 1.3-1.45 x faster on the
-                                                      # block-scaled kernel, 64 rows per expert 1.1 x slower
+    block_scaled_max_rows_per_expert: int = 48       # up to here the block-scaled kernels are faster whatever the shape
 
     @property
     def n_expts(self):
         return self.b1.shape[0]
 
-    def use_block_scaled(self, n_rows: int) -> bool:
-        """Few rows per expert (decode): the block-scaled kernel streams the packed weights straight into the MMA and
-        is bound by HBM; with many rows per expert the bf16 kernel's larger token tiles win."""
-        return self.w1_bs is not None and n_rows <= self.block_scaled_max_rows_per_expert * self.n_expts
+    def use_block_scaled(self, n_rows: int, n_out: int | None = None) -> bool:
+        """Whether a product of `n_rows` routed rows with `n_out` weight rows per expert (default: fc1's) takes the
+        block-scaled copy.  Few rows per expert (decode) stream the packed weights straight into the MMA, bound by HBM.
+        With more rows the block-scaled pair kernel first re-lays the tokens out (4 bytes per element written and read
+        against 2 n_out operations), which a wide product repays and a narrow one does not; measured against the bf16
+        kernel: 64 rows per expert 1.3-1.7 x faster for n_out >= 2000 and 0.9 x at 512-1024; 1024 rows per expert
+        1.05-1.2 x faster from 2880 on, 0.9 x at 2048."""
+        if self.w1_bs is None:
+            return False
+        if n_rows <= self.block_scaled_max_rows_per_expert * self.n_expts:
+            return True
+        n_out = self.b1.shape[1] if n_out is None else n_out
+        return n_out >= (1280 if n_rows < 512 * self.n_expts else 2560)
 
     def fc_weights(self, n_rows: int):
-        if self.use_block_scaled(n_rows):
-            return self.w1_bs, self.w1_bs_scale, self.w2_bs, self.w2_bs_scale
-        return self.w1, self.w1_scale, self.w2, self.w2_scale
+        one = (self.w1_bs, self.w1_bs_scale) if self.use_block_scaled(n_rows, self.b1.shape[1]) else (self.w1, self.w1_scale)
+        two = (self.w2_bs, self.w2_bs_scale) if self.use_block_scaled(n_rows, self.b2.shape[1]) else (self.w2, self.w2_scale)
+        return (*one, *two)
 
     def weight_bytes(self):
         return sum(t.storage.data.numel() for t in (self.w1, self.w1_scale, self.w2, self.w2_scale)) + \
@@ -259,7 +267,7 @@ def _forward_ep_peer(x_local, sparse, lw_local, k, expt_assignment, pool, gemm_t
     chunks = int(getattr(pool, "overlap_chunks", 1))
     w1, w1_scale, w2, w2_scale = lw_local.fc_weights(n // W)            # rows this rank multiplies, on average
     E_loc = lw_local.n_expts
-    if lw_local.use_block_scaled(n // W) or E_loc < 2:
+    if (lw_local.use_block_scaled(n // W) and n // W <= lw_local.block_scaled_max_rows_per_expert * E_loc) or E_loc < 2:
         chunks = 1
     chunks = max(1, min(chunks, E_loc))
     plan = None

@@ -77,14 +77,15 @@ struct MxMaps {
 // correct and 20-35 % slower at 4 to 64 tokens: 48 scalar reductions per thread and slice, their fence and the counter
 // round trip take longer than a slice of a few k steps, and the epilogue warps become the bottleneck.)
 struct MxSched {
-  int64_t useful_m, cur, end;
+  uint32_t useful_m, cur, end;
   int NB, MB;
-  __device__ __forceinline__ MxSched(int64_t useful_m_, int NB_, int NG, int MB_)
-      : useful_m(useful_m_), cur(blockIdx.x), end(useful_m_ * NG), NB(NB_), MB(MB_) {}
+  __device__ __forceinline__ MxSched(uint32_t useful_m_, int NB_, int NG, int MB_)
+      : useful_m(useful_m_), cur(blockIdx.x), end(useful_m_ * (uint32_t)NG), NB(NB_), MB(MB_) {}
   __device__ __forceinline__ bool next(int64_t& pid_m, int& nb0, int& mb_live) {
     if (cur >= end) return false;
-    pid_m = cur % useful_m;
-    nb0 = (int)(cur / useful_m) * MB;
+    const uint32_t grp = cur / useful_m;
+    pid_m = cur - grp * useful_m;
+    nb0 = (int)grp * MB;
     mb_live = min(MB, NB - nb0);
     cur += gridDim.x;
     return true;
@@ -286,33 +287,32 @@ __device__ __forceinline__ uint32_t mx_idesc(int n, uint32_t sf) {
 __device__ __forceinline__ uint32_t mx4_idesc(int n, uint32_t sf) {
   return (sf << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | (1u << 23) | (1u << 27) | (sf << 29);
 }
-// shared-memory descriptor of a K-major operand with 64-byte rows and 64-byte swizzle (8-row groups 512 B apart)
-__device__ __forceinline__ uint64_t make_desc_sw64(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);
-  d |= (uint64_t)1 << 16;
-  d |= (uint64_t)(512 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)4 << 61;
-  return d;
-}
-__device__ __forceinline__ void mma_mxf4(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t sfa, uint32_t sfb,
-                                         uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %6, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], %1, %2, %3, [%4], [%5], p;\n\t}" ::"r"(d_tmem),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void mma_mxf8f6f4(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t sfa,
-                                             uint32_t sfb, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %6, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale.scale_vec::1X [%0], %1, %2, %3, [%4], [%5], p;\n\t}" ::"r"(d_tmem),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate)
-      : "memory");
+// One block-scaled MMA of either kind, issued by the lane whose `leader` is set while the whole warp runs the loop: the
+// operands of tcgen05.mma live in uniform registers, and computed by a single thread of a divergent branch each of them took a
+// move from a vector register first (87-95 cycles per instruction; a block-scaled MMA of up to 64 columns runs 45).  Of a
+// shared-memory descriptor only the low word varies.
+constexpr uint32_t MX_DESC_LO = 1u << 16;                                              // leading byte offset (unused)
+constexpr uint32_t MX_DESC_HI_SW128 = (1024u >> 4) | (1u << 14) | (2u << 29);          // 8-row groups 1024 B apart, 128-byte swizzle
+constexpr uint32_t MX_DESC_HI_SW64 = (512u >> 4) | (1u << 14) | (4u << 29);            // 64-byte rows and swizzle
+template <bool F4>
+__device__ __forceinline__ void mma_mx(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t sfa, uint32_t sfb,
+                                       uint32_t accumulate, uint32_t leader) {
+  if constexpr (F4)
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
+        "mov.b64 da, {%1, %8};\n\tmov.b64 db, {%2, %8};\n\t"
+        "setp.ne.b32 p, %6, 0;\n\tsetp.ne.b32 q, %7, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], da, db, %3, [%4], [%5], p;\n\t}" ::"r"(d_tmem),
+        "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate), "r"(leader), "n"(MX_DESC_HI_SW64)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
+        "mov.b64 da, {%1, %8};\n\tmov.b64 db, {%2, %8};\n\t"
+        "setp.ne.b32 p, %6, 0;\n\tsetp.ne.b32 q, %7, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale.scale_vec::1X [%0], da, db, %3, [%4], [%5], p;\n\t}" ::"r"(d_tmem),
+        "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate), "r"(leader), "n"(MX_DESC_HI_SW128)
+        : "memory");
 }
 
 // ============================================================================================================
@@ -334,7 +334,7 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const uint32_t sbase = smem_u32(smem);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;     // warp-uniform for the compiler
   const int STAGES = q.stages;
   // per stage: [MB weight tiles][token rows + 1024 B scale area (KM: three such chunks)][MB x 512 B weight scales]
   const uint32_t OFF_X = MB * W_TILE;
@@ -376,13 +376,13 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *s_tmem;
+  const uint32_t tmem_base = __shfl_sync(0xFFFFFFFFu, *s_tmem, 0);
   pdl_launch_dependents();
   pdl_wait();
 
   const int KT = q.KT, NB = q.NB, NG = q.n_groups;
-  int64_t useful_m = q.grid_m;
-  if (p.slice_sizes) useful_m = (int64_t)p.block_offs[p.E];
+  uint32_t useful_m = (uint32_t)q.grid_m;
+  if (p.slice_sizes) useful_m = (uint32_t)__shfl_sync(0xFFFFFFFFu, p.block_offs[p.E], 0);
   const int acc_stride = NACC * q.n_mma;            // accumulator columns of one buffer
   MxSched sched(useful_m, NB, NG, NACC);
   const int KS = KM ? (KT + 2) / 3 : KT;            // stages of a tile
@@ -432,70 +432,67 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
     __syncwarp();
   } else if (warp == 1) {
     // ================================= MMA issuer =====================================================
-    if (lane == 0) {
-      uint32_t it = 0, tc = 0;
-      bool ok = true;
-      for (; ok && sched.next(pid_m, nb0, mb_live); ++tc) {
-        const uint32_t ab = tc % (uint32_t)q.acc_bufs;
-        ok = mbar_wait(BAR_ACC_EMPTY(ab), ((tc / (uint32_t)q.acc_bufs) & 1u) ^ 1u, ctl, 603);
+    const uint32_t leader = elect_one();
+    const uint32_t idesc = F4 ? mx4_idesc(q.n_mma, 0) : mx_idesc(q.n_mma, 0);
+    uint32_t s = 0, ph = 0, tc = 0;                    // stage and parity of the next k step
+    bool ok = true;
+    for (; ok && sched.next(pid_m, nb0, mb_live); ++tc) {
+      const uint32_t ab = tc % (uint32_t)q.acc_bufs;
+      ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_ACC_EMPTY(ab), ((tc / (uint32_t)q.acc_bufs) & 1u) ^ 1u, ctl, 603));
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t d_tmem = tmem_base + ab * (uint32_t)acc_stride;
+      for (int kt = 0; kt < KS; ++kt) {
+        ok = mbar_wait(BAR_FULL(s), ph, ctl, 602);
+        ok = ok && mbar_wait(BAR_SF(s), ph, ctl, 606);
+        ok = __all_sync(0xFFFFFFFFu, ok);
         if (!ok) break;
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + ab * (uint32_t)acc_stride;
-        for (int kt = 0; kt < KS; ++kt, ++it) {
-          const int s = it % STAGES;
-          ok = mbar_wait(BAR_FULL(s), (it / STAGES) & 1u, ctl, 602);
-          ok = ok && mbar_wait(BAR_SF(s), (it / STAGES) & 1u, ctl, 606);
-          if (!ok) break;
-          tc_fence_after();
-          const uint32_t st = sbase + (uint32_t)s * (uint32_t)q.stage_bytes;
-          const uint32_t sf = tmem_base + SF_BASE + (uint32_t)(s * SF_COLS);
-          // k group outermost: consecutive MMAs go to different accumulators
-          if constexpr (KM) {
-            const int k_live = min(3, KT - 3 * kt);
+        const uint32_t st = sbase + s * (uint32_t)q.stage_bytes;
+        const uint32_t sf = tmem_base + SF_BASE + s * SF_COLS;
+        const uint32_t a_lo = MX_DESC_LO | (st >> 4), b_lo = MX_DESC_LO | ((st + OFF_X) >> 4);
+        const uint32_t more = (uint32_t)(kt > 0);
+        // k group outermost: consecutive MMAs go to different accumulators
+        if constexpr (KM) {
+          const uint32_t bstep = (uint32_t)q.chunk_bytes >> 4;
+          const int k_live = min(3, KT - 3 * kt);
 #pragma unroll
-            for (int i = 0; i < 3; ++i) {
-              if (i < k_live) {
-                const uint64_t adesc = make_desc_sw64(st + (uint32_t)i * W_TILE);
-                const uint64_t bdesc = make_desc_sw64(st + OFF_X + (uint32_t)i * (uint32_t)q.chunk_bytes);
+          for (int i = 0; i < 3; ++i) {
+            if (i < k_live) {
 #pragma unroll
-                for (int kk = 0; kk < 2; ++kk)
-                  mma_mxf4(d_tmem, adesc + (uint64_t)(kk * 2), bdesc + (uint64_t)(kk * 2), mx4_idesc(q.n_mma, (uint32_t)(kk * 2)),
-                           sf + 4u * (uint32_t)i, sf + 12u + 4u * (uint32_t)i, (kt | i | kk) ? 1u : 0u);
-              }
-            }
-          } else if constexpr (F4) {
-            const uint64_t bdesc = make_desc_sw64(st + OFF_X);
-#pragma unroll
-            for (int kk = 0; kk < 2; ++kk) {
-#pragma unroll
-              for (int mb = 0; mb < MB; ++mb) {
-                if (mb < mb_live)
-                  mma_mxf4(d_tmem + (uint32_t)(mb * q.n_mma), make_desc_sw64(st + (uint32_t)mb * W_TILE) + (uint64_t)(kk * 2),
-                           bdesc + (uint64_t)(kk * 2), mx4_idesc(q.n_mma, (uint32_t)(kk * 2)), sf + 4u * (uint32_t)mb, sf + 4u * MB,
-                           (kt | kk) ? 1u : 0u);
-              }
-            }
-          } else {
-            const uint64_t bdesc = make_desc(st + OFF_X);
-#pragma unroll
-            for (int kk = 0; kk < 4; ++kk) {
-#pragma unroll
-              for (int mb = 0; mb < MB; ++mb) {
-                if (mb < mb_live)
-                  mma_mxf8f6f4(d_tmem + (uint32_t)(mb * q.n_mma), make_desc(st + (uint32_t)mb * W_TILE) + (uint64_t)(kk * 2),
-                               bdesc + (uint64_t)(kk * 2), mx_idesc(q.n_mma, (uint32_t)kk), sf + 4u * (uint32_t)mb, sf + 4u * MB,
-                               (kt | kk) ? 1u : 0u);
-              }
+              for (int kk = 0; kk < 2; ++kk)
+                mma_mx<true>(d_tmem, a_lo + i * (W_TILE >> 4) + kk * 2, b_lo + i * bstep + kk * 2, idesc + (uint32_t)kk * ((2u << 4) + (2u << 29)),
+                             sf + 4 * i, sf + 12 + 4 * i, (i | kk) ? 1u : more, leader);
             }
           }
-          mma_commit(BAR_EMPTY(s));
+        } else {
+          constexpr int KK = F4 ? 2 : 4;
+          constexpr uint32_t SFK = F4 ? (2u << 4) + (2u << 29) : (1u << 4) + (1u << 29);       // next scale byte (pair)
+          if (mb_live == MB) {
+#pragma unroll
+            for (int kk = 0; kk < KK; ++kk)
+#pragma unroll
+              for (int mb = 0; mb < MB; ++mb)
+                mma_mx<F4>(d_tmem + (uint32_t)(mb * q.n_mma), a_lo + mb * (W_TILE >> 4) + kk * 2, b_lo + kk * 2, idesc + kk * SFK, sf + 4 * mb,
+                           sf + 4 * MB, kk ? 1u : more, leader);
+          } else {
+#pragma unroll
+            for (int kk = 0; kk < KK; ++kk)
+#pragma unroll
+              for (int mb = 0; mb < MB; ++mb)
+                if (mb < mb_live)
+                  mma_mx<F4>(d_tmem + (uint32_t)(mb * q.n_mma), a_lo + mb * (W_TILE >> 4) + kk * 2, b_lo + kk * 2, idesc + kk * SFK, sf + 4 * mb,
+                             sf + 4 * MB, kk ? 1u : more, leader);
+          }
         }
-        if (ok) mma_commit(BAR_ACC_FULL(ab));
+        mma_commit(BAR_EMPTY(s), leader);
+        if (++s == (uint32_t)STAGES) { s = 0; ph ^= 1u; }
       }
-      // every MMA issued by this thread has retired before tensor memory is freed
-      mma_commit(BAR_DRAIN);
-      mbar_wait(BAR_DRAIN, 0, ctl, 605);
+      if (ok) mma_commit(BAR_ACC_FULL(ab), leader);
     }
+    // every MMA issued by this warp has retired before tensor memory is freed
+    mma_commit(BAR_DRAIN, leader);
+    mbar_wait(BAR_DRAIN, 0, ctl, 605);
     __syncwarp();
   } else if (warp >= 6) {
     // ================================= scale loaders ==================================================
@@ -674,11 +671,10 @@ MxPlan mx_plan(const MoeGemmArgs& a) {
   if (a.tile_m == 16 || a.tile_m == 32 || a.tile_m == 64 || a.tile_m == 128) {
     tb = a.tile_m;
   } else {
-    // bf16 tokens: 16 rows up to 8 rows per expert on average, 32 beyond (64-row blocks were slower than two 32-row
-    // blocks at every size measured: 32 rows per expert 294 against 226 us on a 32-expert layer, 911 against 698 us on
-    // a 128-expert one); fp8 tokens grow to 128
+    // 16 rows up to 8 rows per expert on average, 32 beyond (64-row blocks were slower than two 32-row blocks at every size
+    // measured, with bf16 and with fp8 tokens: 32 experts, 8 rows, fp8: 102 us with 32-row blocks, 125 with 64, 153 with 128)
     const int64_t per = a.slice_sizes ? (a.M + a.E - 1) / a.E : a.M;      // mean rows per expert
-    const int tb_auto = bf16 ? (tb_max < 32 ? tb_max : 32) : tb_max;
+    const int tb_auto = tb_max < 32 ? tb_max : 32;
     while (tb < tb_auto && tb < 2 * per) tb *= 2;
   }
   if (tb > tb_max) tb = tb_max;
@@ -802,7 +798,7 @@ int moe_gemm_mx_launch(const GemmParams& p_in, const MoeGemmArgs& a, cudaStream_
   pk.chunk_bytes = pl.chunk_bytes;
   pk.out = (uint8_t*)a.mx_workspace;
   const dim3 pgrid((unsigned)pl.grid_m, (unsigned)pl.KT);
-  MOE_CHECK_ARG(pl.grid_m < 2147483647LL, "moe_grouped_gemm: too many token blocks");
+  MOE_CHECK_ARG(pl.grid_m * pl.n_groups < 2147483647LL - 65536, "moe_grouped_gemm: too many token blocks");
   if (pl.f4) MOE_CHECK_CUDA(launch_pdl(mx_pack_x4_kernel, pgrid, dim3(256), 0, st, p, pk));
   else if (pl.split > 1) MOE_CHECK_CUDA(launch_pdl(mx_pack_x_kernel<true>, pgrid, dim3(256), 0, st, p, pk));
   else MOE_CHECK_CUDA(launch_pdl(mx_pack_x_kernel<false>, pgrid, dim3(256), 0, st, p, pk));

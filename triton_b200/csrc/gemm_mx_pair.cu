@@ -760,19 +760,18 @@ int launch_mx_pair_terms(const GemmParams& p, const PairParams& q, int terms, in
 
 }  // namespace
 
-// The pair form against the decode forms of gemm_mx.cu, by mean rows per expert: from 48 on it wins everywhere (32 experts of
-// 2880 x 5760, 48 rows: fc1 + fc2 285 -> 200 us, 128 rows 550 -> 296), from 16 on where a product is wide enough to repay its
-// larger tiles (128 experts, 16 rows: 448 -> 398 us; 8 experts of 512 x 2048: 35 -> 40).  e4m3 tokens: at every size (32
-// experts, 8 rows: 149 -> 113 us, 512 rows 1500 -> 446), since one term needs no second pass over the operands.
-// tile_m = 256 asks for it.
+// The pair form against the decode forms of gemm_mx.cu, by mean rows per expert (fc1 + fc2).  bf16 tokens, from 40 on: 32
+// experts of 2880 x 5760, 32 rows 172 us there and 189 here, 48 rows 219 and 216; 128 experts, 32 rows 530 and 486; narrow
+// products repay the larger tiles later (8 experts of 512 x 2048, 64 rows: 41 and 48).  e4m3 tokens, one term, from 16 on
+// (32 experts, 8 rows: 102 and 114; 64 rows: 320 and 167).  tile_m = 256 asks for it.
 bool moe_gemm_mx_pair_wanted(const MoeGemmArgs& a) {
   if (a.slice_sizes && a.E > MAX_PREFIX_EXPERTS) return false;
   if (a.M >= (1ll << 31) - (1 << 20) || a.kernel == MOE_GEMM_MX_F4 || a.tile_n != 0) return false;
   if (a.tile_m == 256) return true;
   if (a.tile_m != 0 || a.kernel == MOE_GEMM_MX_F8) return false;
   const int64_t per = a.slice_sizes ? a.M / a.E : a.M;
-  if (a.x_dtype != MOE_BF16) return true;
-  return per >= 48 || (per >= 16 && a.N >= 1280);
+  if (a.x_dtype != MOE_BF16) return per >= 16;
+  return per >= (a.N >= 1280 ? 40 : 96);
 }
 
 int64_t moe_gemm_mx_pair_workspace(const MoeGemmArgs& a) { return pair_plan(a).ws_bytes; }

@@ -62,12 +62,7 @@ __device__ __forceinline__ void mma_commit_pair_local(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
-// the same with a lane's predicate, for a warp that runs the issue loop as a whole
-__device__ __forceinline__ uint32_t elect_one() {
-  uint32_t r;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
-  return r;
-}
+// the same for a warp that runs its issue loop as a whole (see elect_one)
 __device__ __forceinline__ void mma_commit_pair(uint32_t bar, uint32_t leader) {
   asm volatile(
       "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t"

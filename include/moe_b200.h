@@ -101,6 +101,17 @@ int moe_route(const void* logits, int dtype, int64_t T, int E, int k, int apply_
               int32_t* block_sched, int64_t ld_sched, int64_t n_sched,
               void* workspace, size_t workspace_bytes, void* stream);
 
+/* moe_route on fp32 logits that also writes, for every expert-sorted position, its token row and its routing weight (the
+ * gather index and the gammas of the layer's two products), in the same launches.                                  */
+int moe_route_positions(const float* logits, int64_t T, int E, int k, int apply_softmax, int64_t ld_logits,
+                        float* vals, int64_t ld_vals, int16_t* indx, int64_t ld_indx,
+                        uint32_t* bitmatrix, int64_t bm_stride_row, int64_t bm_stride_word,
+                        int32_t* col_sum, int32_t* col_sorted, int32_t* row_sorted,
+                        int32_t* slice_offs, int32_t* block_offs, int64_t ld_block_offs,
+                        int32_t* block_sched, int64_t ld_sched, int64_t n_sched,
+                        int32_t* token_of_position, float* weight_of_position,
+                        void* workspace, size_t workspace_bytes, void* stream);
+
 /* The router product and the top-k selection in one kernel: logits = x @ Wg + bg on the tensor cores, then what
  * moe_topk_fwd does, in the epilogue (the reference runs `matmul(x, wg, bg)` and `topk` apart:
  * triton_kernels bench/bench_mlp.py:70, topk.py:25-141).

@@ -387,3 +387,24 @@ def test_weight_file_and_block_checkpoint_reader(tmp_path, device):
                                lw.w2_s.transpose(1, 2).contiguous(), lw.b2, block_scaled=True)
     for name in ("w1", "w1_scale", "w2", "w2_scale", "w1_bs", "w1_bs_scale", "w2_bs", "w2_bs_scale"):
         assert torch.equal(getattr(ck, name).storage.data, getattr(lw, name).storage.data), name
+
+
+@pytest.mark.parametrize("tokens, E, k, dtype", [(1, 5, 1, "bf16"), (7, 33, 4, "bf16"), (256, 8, 6, "bf16"), (257, 8, 2, "bf16"),
+                                                 (1100, 8, 2, "bf16"), (1, 5, 1, "e4m3"), (300, 33, 4, "e4m3")])
+def test_layer_in_one_call_equals_the_operators(tokens, E, k, dtype, device):
+    """The step as one native call runs the kernels of the step composed from the operators on the same operands: the results
+    are the same bits.  (Sizes: either side of the single-launch routing, k the quad top-k does and does not take, 2048 gathered
+    rows and fewer.)"""
+    from triton_b200.moe import _NoTimer, _one_call, moe_layer_forward
+    from triton_b200.testing import make_synthetic_layer
+    lw = make_synthetic_layer(E, 512, 736, device, seed=3, block_scaled=True)
+    for weights in ((lw,) if dtype == "e4m3" else (lw, make_synthetic_layer(E, 512, 736, device, seed=3))):
+        g = torch.Generator(device=device).manual_seed(tokens + E)
+        x = torch.randn(tokens, 512, device=device, generator=g).bfloat16()
+        x = x.to(torch.float8_e4m3fn) if dtype == "e4m3" else x
+        logits = torch.randn(tokens, E, device=device, generator=g)
+        assert _one_call(x, logits, weights, k)
+        one = moe_layer_forward(x, logits, weights, k)
+        many = moe_layer_forward(x, logits, weights, k, gemm_timer=_NoTimer)
+        tb.matmul_check_status()
+        assert torch.equal(one, many)

@@ -67,6 +67,8 @@ PROTOTYPES = {
     "moe_route_workspace": (sz, [i64, i32, i32]),
     "moe_route": (i32, [vp, i32, i64, i32, i32, i32, i64, vp, i64, vp, i64, vp, i64, i64, vp, vp, vp, vp, vp, i64, vp, i64,
                         i64, vp, sz, vp]),
+    "moe_route_positions": (i32, [vp, i64, i32, i32, i32, i64, vp, i64, vp, i64, vp, i64, i64, vp, vp, vp, vp, vp, i64, vp, i64,
+                                  i64, vp, vp, vp, sz, vp]),
     "moe_router_topk_workspace_bytes": (sz, [i64, i64, i32]),
     "moe_router_topk": (i32, [vp, i64, i64, i64, vp, i64, vp, i32, i32, i32, i32, i32, vp, i64, vp, i32, i64, vp, i64, vp, i64,
                               i64, vp, sz, vp, vp]),
@@ -123,6 +125,24 @@ def load():
         fn.restype, fn.argtypes = res, args
     _lib = lib
     return lib
+
+
+_host_mod = None
+
+
+def host():
+    """The native host path (csrc/host.cpp), bound to the loaded library.  Like the library it has no substitute."""
+    global _host_mod
+    if _host_mod is None:
+        lib = load()
+        try:
+            from . import _host
+        except ImportError as e:
+            raise MoeLibraryError(f"{_HERE / '_host.so'} cannot be loaded ({e}): build it with `python -m triton_b200.build`") from e
+        from .matmul_details.opt_flags import InapplicableConstraint
+        _host.bind(lib._handle, InapplicableConstraint)
+        _host_mod = _host
+    return _host_mod
 
 
 def check(status: int, what: str = ""):

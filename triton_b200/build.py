@@ -20,6 +20,27 @@ NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", 
               "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden"]
 
 
+HOST_SRC = CSRC / "host.cpp"
+HOST_LIB = HERE / "_host.so"
+
+
+def build_host():
+    """The native host path (csrc/host.cpp, a Python extension against torch); the library itself has no torch in it."""
+    import sysconfig
+    import torch
+    from torch.utils import cpp_extension
+    cuda = Path(_nvcc()).resolve().parent.parent
+    inc = [*cpp_extension.include_paths(), str(cuda / "include"), sysconfig.get_paths()["include"]]
+    tmp = HOST_LIB.with_suffix(".so.tmp")
+    subprocess.check_call([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-w",
+                           "-DTORCH_EXTENSION_NAME=_host", "-DTORCH_API_INCLUDE_EXTENSION_H",
+                           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[f"-isystem{i}" for i in inc],
+                           str(HOST_SRC), "-o", str(tmp), f"-L{cpp_extension.library_paths()[0]}", "-lc10", "-lc10_cuda",
+                           "-ltorch_cpu", "-ltorch", "-ltorch_python", "-ldl"])
+    os.replace(tmp, HOST_LIB)
+    return HOST_LIB
+
+
 def _nvcc():
     for cand in (os.environ.get("NVCC"), shutil.which("nvcc"), "/usr/local/cuda/bin/nvcc"):
         if cand and Path(cand).exists():
@@ -40,6 +61,20 @@ def needs_build():
 
 
 def build(force=False, verbose=False):
+    host = None
+    deps = [HOST_SRC, HERE.parent / "include" / "moe_b200.h"]
+    if force or not HOST_LIB.exists() or any(d.stat().st_mtime > HOST_LIB.stat().st_mtime for d in deps):
+        # in a process of its own, beside nvcc: importing torch here would load libraries that the compilers do not need
+        host = subprocess.Popen([sys.executable, "-c", f"import sys; sys.path.insert(0, {str(HERE.parent)!r}); "
+                                 "import triton_b200.build as b; b.build_host()"])
+    try:
+        return _build_kernels(force, verbose)
+    finally:
+        if host is not None and host.wait() != 0:
+            raise RuntimeError("_host.so: compilation failed")
+
+
+def _build_kernels(force, verbose):
     if not force and not needs_build():
         return LIB
     objdir = HERE / "build"

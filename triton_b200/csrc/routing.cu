@@ -314,11 +314,20 @@ __global__ void __launch_bounds__(1024) bm_scan_kernel(int32_t* __restrict__ par
   }
 }
 
+// What the layer wants per expert-sorted position beside the permutation: token row and routing weight (token NULL: nothing).
+struct PerPosition {
+  int32_t* token = nullptr;
+  float* weight = nullptr;
+  const float* vals = nullptr;
+  int64_t ld_vals = 0;
+};
+
 // Positions of the entries of one block of blockDim.x tokens starting at token `tok_base`: `base[e]` is where the
 // block's entries of expert e start (expert offset + entries of earlier blocks); s_cnt holds [warps][E] counters.
 __device__ __forceinline__ void rank_block(const int16_t* __restrict__ indx, int64_t ld_indx, int64_t T_rows, int E, int k,
                                            int64_t n_rows, const int32_t* base_a, const int32_t* base_b, int64_t tok_base,
-                                           int32_t* __restrict__ col_sorted, int32_t* __restrict__ row_sorted, int32_t* s_cnt) {
+                                           int32_t* __restrict__ col_sorted, int32_t* __restrict__ row_sorted, int32_t* s_cnt,
+                                           const PerPosition& out = PerPosition()) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   int32_t* my = s_cnt + (int64_t)warp * E;
   for (int i = threadIdx.x; i < nwarps * E; i += blockDim.x) s_cnt[i] = 0;
@@ -359,6 +368,10 @@ __device__ __forceinline__ void rank_block(const int16_t* __restrict__ indx, int
       const int64_t flat = token * k + slot;
       row_sorted[flat] = pos;
       col_sorted[pos] = (int32_t)flat;
+      if (out.token) {
+        out.token[pos] = (int32_t)token;
+        out.weight[pos] = out.vals[token * out.ld_vals + slot];
+      }
     }
   }
 }
@@ -367,11 +380,12 @@ __global__ void __launch_bounds__(256) bm_rank_kernel(const int16_t* __restrict_
                                                       int E, int k, const int32_t* __restrict__ n_rows_dev,
                                                       const int32_t* __restrict__ partial,
                                                       const int32_t* __restrict__ col_offs,
-                                                      int32_t* __restrict__ col_sorted, int32_t* __restrict__ row_sorted) {
+                                                      int32_t* __restrict__ col_sorted, int32_t* __restrict__ row_sorted,
+                                                      const PerPosition out) {
   extern __shared__ int32_t s_cnt[];  // [warps][E]; a block covers blockDim.x tokens, the blocks of `partial`
   const int64_t n_rows = n_rows_dev ? min((int64_t)*n_rows_dev, T_rows) : T_rows;
   rank_block(indx, ld_indx, T_rows, E, k, n_rows, partial + (int64_t)blockIdx.x * E, col_offs, (int64_t)blockIdx.x * blockDim.x,
-             col_sorted, row_sorted, s_cnt);
+             col_sorted, row_sorted, s_cnt, out);
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -547,7 +561,7 @@ extern "C" __attribute__((visibility("default"))) int moe_bitmatrix_metadata(con
   if (smem_rank > 48 * 1024)
     MOE_CHECK_CUDA(cudaFuncSetAttribute(bm_rank_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_rank));
   bm_rank_kernel<<<(int)nb, 256, smem_rank, st>>>(indx, ld_indx, T, E, k, n_rows_dev, partial, col_offs, col_sorted,
-                                                  row_sorted);
+                                                  row_sorted, PerPosition());
   MOE_CHECK_LAUNCH();
   return MOE_OK;
 }
@@ -811,7 +825,7 @@ __global__ void __launch_bounds__(1024) route_small_kernel(
     int64_t ld_vals, int16_t* __restrict__ indx, int64_t ld_indx, uint32_t* __restrict__ bitmatrix, int64_t bm_stride_row,
     int64_t bm_stride_word, int32_t* __restrict__ col_sum, int32_t* __restrict__ col_sorted, int32_t* __restrict__ row_sorted,
     int32_t* __restrict__ slice_offs, int32_t* __restrict__ block_offs, int64_t ld_block_offs, int32_t* __restrict__ block_sched,
-    int64_t ld_sched, int64_t n_sched) {
+    int64_t ld_sched, int64_t n_sched, const PerPosition out) {
   extern __shared__ int32_t s_mem[];            // [E + 1] sizes, [E + 1] scan input, [E + 1] offsets, [E] expert offsets, [32][E] counters
   __shared__ int32_t s_warp[33];
   int32_t* s_size = s_mem;
@@ -847,7 +861,7 @@ __global__ void __launch_bounds__(1024) route_small_kernel(
   ragged_row(0, s_size, E, s_nb, s_offs, s_warp, slice_offs, nullptr, block_offs, ld_block_offs, block_sched, ld_sched, n_sched);
   for (int e = threadIdx.x; e < E; e += blockDim.x) s_col[e] = s_offs[e];
   __syncthreads();
-  rank_block(indx, ld_indx, T_rows, E, K, T_rows, nullptr, s_col, 0, col_sorted, row_sorted, s_cnt);
+  rank_block(indx, ld_indx, T_rows, E, K, T_rows, nullptr, s_col, 0, col_sorted, row_sorted, s_cnt, out);
 }
 
 constexpr int kRouteSmallTokens = 256;
@@ -860,11 +874,12 @@ extern "C" __attribute__((visibility("default"))) size_t moe_route_workspace(int
   return (size_t)((2 * nb * E + E) * (int64_t)sizeof(int32_t));
 }
 
-extern "C" __attribute__((visibility("default"))) int moe_route(
+static int route_launch(
     const void* logits, int dtype, int64_t T, int E, int k, int apply_softmax, int64_t ld_logits, void* vals, int64_t ld_vals,
     int16_t* indx, int64_t ld_indx, uint32_t* bitmatrix, int64_t bm_stride_row, int64_t bm_stride_word, int32_t* col_sum,
     int32_t* col_sorted, int32_t* row_sorted, int32_t* slice_offs, int32_t* block_offs, int64_t ld_block_offs,
-    int32_t* block_sched, int64_t ld_sched, int64_t n_sched, void* workspace, size_t workspace_bytes, void* stream) {
+    int32_t* block_sched, int64_t ld_sched, int64_t n_sched, void* workspace, size_t workspace_bytes, const PerPosition& out,
+    void* stream) {
   MOE_CHECK_ARG(T > 0 && E > 0 && k > 0 && k <= kMaxTopK && k <= E, "moe_route: bad extents T=%lld E=%d k=%d", (long long)T, E, k);
   if (E > 256) {
     moe_set_error("moe_route: the fused routing handles up to 256 experts (got %d); use the separate entry points", E);
@@ -884,7 +899,7 @@ extern "C" __attribute__((visibility("default"))) int moe_route(
     route_small_kernel<Tv, KK><<<5, 1024, smem_s, st>>>((const Tv*)logits, ld_logits, T, E, apply_softmax, (Tv*)vals, ld_vals, \
                                                          indx, ld_indx, bitmatrix, bm_stride_row, bm_stride_word, col_sum,  \
                                                          col_sorted, row_sorted, slice_offs, block_offs, ld_block_offs,     \
-                                                         block_sched, ld_sched, n_sched);                                   \
+                                                         block_sched, ld_sched, n_sched, out);                              \
   })
     switch (k) {
       case 1: MOE_ROUTE_SMALL(1); break;
@@ -928,9 +943,33 @@ extern "C" __attribute__((visibility("default"))) int moe_route(
   MOE_CHECK_LAUNCH();
   const size_t smem_rank = (size_t)(kRouteTokPerBlock / 32) * E * sizeof(int32_t);
   bm_rank_kernel<<<(int)nb, kRouteTokPerBlock, smem_rank, st>>>(indx, ld_indx, T, E, k, nullptr, scanned, col_offs, col_sorted,
-                                                                row_sorted);
+                                                                row_sorted, out);
   MOE_CHECK_LAUNCH();
   return MOE_OK;
+}
+
+extern "C" __attribute__((visibility("default"))) int moe_route(
+    const void* logits, int dtype, int64_t T, int E, int k, int apply_softmax, int64_t ld_logits, void* vals, int64_t ld_vals,
+    int16_t* indx, int64_t ld_indx, uint32_t* bitmatrix, int64_t bm_stride_row, int64_t bm_stride_word, int32_t* col_sum,
+    int32_t* col_sorted, int32_t* row_sorted, int32_t* slice_offs, int32_t* block_offs, int64_t ld_block_offs,
+    int32_t* block_sched, int64_t ld_sched, int64_t n_sched, void* workspace, size_t workspace_bytes, void* stream) {
+  return route_launch(logits, dtype, T, E, k, apply_softmax, ld_logits, vals, ld_vals, indx, ld_indx, bitmatrix, bm_stride_row,
+                      bm_stride_word, col_sum, col_sorted, row_sorted, slice_offs, block_offs, ld_block_offs, block_sched, ld_sched,
+                      n_sched, workspace, workspace_bytes, PerPosition(), stream);
+}
+
+extern "C" __attribute__((visibility("default"))) int moe_route_positions(
+    const float* logits, int64_t T, int E, int k, int apply_softmax, int64_t ld_logits, float* vals, int64_t ld_vals,
+    int16_t* indx, int64_t ld_indx, uint32_t* bitmatrix, int64_t bm_stride_row, int64_t bm_stride_word, int32_t* col_sum,
+    int32_t* col_sorted, int32_t* row_sorted, int32_t* slice_offs, int32_t* block_offs, int64_t ld_block_offs,
+    int32_t* block_sched, int64_t ld_sched, int64_t n_sched, int32_t* token_of_position, float* weight_of_position, void* workspace,
+    size_t workspace_bytes, void* stream) {
+  MOE_CHECK_ARG(token_of_position && weight_of_position, "moe_route_positions: NULL pointer");
+  PerPosition out;
+  out.token = token_of_position; out.weight = weight_of_position; out.vals = vals; out.ld_vals = ld_vals;
+  return route_launch(logits, MOE_F32, T, E, k, apply_softmax, ld_logits, vals, ld_vals, indx, ld_indx, bitmatrix, bm_stride_row,
+                      bm_stride_word, col_sum, col_sorted, row_sorted, slice_offs, block_offs, ld_block_offs, block_sched, ld_sched,
+                      n_sched, workspace, workspace_bytes, out, stream);
 }
 
 // ---------------------------------------------------------------------------------------------------------

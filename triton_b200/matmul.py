@@ -13,7 +13,7 @@ import torch
 
 from . import _lib
 from .matmul_details.opt_flags import (InapplicableConstraint, get_idle_sms, reset_opt_flags_constraints,  # noqa: F401
-                                       resolve_kernel_choice, resolve_tile_m, resolve_tile_n,
+                                       gemm_tuning,
                                        scoped_opt_flags_constraints, set_idle_sms,
                                        update_opt_flags_constraints)
 from .numerics import InFlexData, OutFlexData
@@ -27,6 +27,9 @@ from .tensor_details.layout import (B200BlockScaledScaleLayout, B200BlockScaledV
 class FusedActivation:
     specs: FnSpecs = FnSpecs.default()
     fn_args: tuple = tuple()
+
+
+_NO_ACTIVATION = FusedActivation()
 
 
 @dataclass
@@ -68,11 +71,14 @@ class FlexCtx:
     acc_data: InFlexData = InFlexData()
 
 
+_NO_FLEX = FlexCtx()
+
+
 @dataclass
 class PrecisionConfig:
     max_num_imprecise_acc: int | None = None
     allow_tf32: bool = True
-    flex_ctx: FlexCtx = FlexCtx()
+    flex_ctx: FlexCtx = _NO_FLEX
     acc_scale: float = 1.0
     flexpoint_saturate_inf: bool = False
     report_quantization_err_fn: Callable | None = None
@@ -99,7 +105,7 @@ _scale_cache = {}
 
 
 def _status_word(device):
-    key = torch.device(device).index
+    key = device.index if isinstance(device, torch.device) else torch.device(device).index
     if key not in _status_words:
         _status_words[key] = torch.zeros(1, dtype=torch.int32, device=device)
     return _status_words[key]
@@ -193,7 +199,7 @@ def matmul(a, b, bias,
     if precision_config is None:
         precision_config = PrecisionConfig()
     if fused_activation is None:
-        fused_activation = FusedActivation(FnSpecs.default(), tuple())
+        fused_activation = _NO_ACTIVATION
     if epilogue is not None and epilogue.specs.name != "dflt":
         raise NotImplementedError("quantising epilogues are not implemented")
     pc = precision_config
@@ -207,18 +213,17 @@ def matmul(a, b, bias,
                 raise NotImplementedError("a_mx_scale must be a plain [M, K/32] tensor")
             a_scale = a_scale.storage.data
     fc = pc.flex_ctx
-    if any(s is not None for s in (fc.lhs_data.scale, fc.rhs_data.scale, fc.out_data.expected_scale, fc.acc_data.scale)):
+    if fc is not _NO_FLEX and any(s is not None for s in (fc.lhs_data.scale, fc.rhs_data.scale, fc.out_data.expected_scale,
+                                                          fc.acc_data.scale)):
         raise NotImplementedError("flexpoint scales are not implemented")
-    kernel_choice = resolve_kernel_choice()
+    tuning = gemm_tuning()
     if isinstance(a, Tensor):
         a = a.storage.data
     assert a.ndim == 2
     if a.stride(-1) != 1:
         a = a.contiguous()
-    lib = _lib.load()
     dev = a.device
-    args = _lib.MoeGemmArgs()
-    keep = []                                           # temporaries that must outlive the launch call
+    w_scale = None
 
     # ---- weights --------------------------------------------------------------------------------------
     b_scale = pc.b_mx_scale
@@ -239,14 +244,11 @@ def matmul(a, b, bias,
                 (type(sl) in (B200MXScaleLayout, B200BlockScaledScaleLayout)) or \
                 isinstance(vl, B200BlockScaledValueLayout) != isinstance(sl, B200BlockScaledScaleLayout):
             raise ValueError("B200 tiled weights need values and scales in the matching pair of B200 layouts")
-        if isinstance(vl, B200BlockScaledValueLayout):
-            args.w_kind = _lib.MOE_W_MX4_B200MX
-            args.w, args.w_scale = b.storage.data.data_ptr(), b_scale.storage.data.data_ptr()
-        elif isinstance(vl, B200MXValueLayout):
-            args.w_kind = _lib.MOE_W_MX4_B200
-            args.w, args.w_scale = b.storage.data.data_ptr(), b_scale.storage.data.data_ptr()
+        wd = b.storage.data
+        if isinstance(vl, (B200BlockScaledValueLayout, B200MXValueLayout)):
+            w_kind = _lib.MOE_W_MX4_B200MX if isinstance(vl, B200BlockScaledValueLayout) else _lib.MOE_W_MX4_B200
+            w_scale = b_scale.storage.data
         else:
-            wd = b.storage.data
             if wd.ndim == 2:
                 wd = wd.unsqueeze(0)
             if isinstance(vl, (StridedLayout, BlackwellMXValueLayout)):
@@ -264,27 +266,20 @@ def matmul(a, b, bias,
             else:
                 raise NotImplementedError(f"weight scale layout {sl} is not supported")
             assert tuple(sd.shape) == (E, K // 32, N), f"scale shape {tuple(sd.shape)} != {(E, K // 32, N)}"
-            keep += [wd, sd]
-            args.w_kind = _lib.MOE_W_MX4_CANONICAL
-            args.w, args.w_scale = wd.data_ptr(), sd.data_ptr()
-            args.w_stride_e, args.w_stride_k, args.w_stride_n = wd.stride(0), 1, wd.stride(2)
-            args.ws_stride_e, args.ws_stride_k, args.ws_stride_n = sd.stride(0), sd.stride(1), sd.stride(2)
+            w_kind, w_scale = _lib.MOE_W_MX4_CANONICAL, sd
     else:
         if isinstance(b, Tensor):
             b = b.storage.data
         assert b.dtype == a.dtype, "dense weights must have the activation dtype"
         wd = b if b.ndim == 3 else b.unsqueeze(0)
         E, K, N = wd.shape
-        keep.append(wd)
-        args.w_kind = _lib.MOE_W_DENSE
-        args.w = wd.data_ptr()
-        args.w_stride_e, args.w_stride_k, args.w_stride_n = wd.stride(0), wd.stride(1), wd.stride(2)
+        w_kind = _lib.MOE_W_DENSE
     assert a.shape[-1] == K, f"inner dimensions differ: {a.shape[-1]} vs {K}"
     if a.dtype == torch.float8_e4m3fn or a_scale is not None:
         # e4m3 / MXFP8 activations exist on the block-scaled tensor-core path only
         if a.dtype != torch.float8_e4m3fn:
             raise NotImplementedError("a_mx_scale is implemented for e4m3 activations (MXFP8)")
-        if args.w_kind != _lib.MOE_W_MX4_B200MX:
+        if w_kind != _lib.MOE_W_MX4_B200MX:
             raise NotImplementedError("e4m3 / MXFP8 activations need MXFP4 weights in B200BlockScaledValueLayout / "
                                       "B200BlockScaledScaleLayout")
         if pc.out_dtype is None:
@@ -294,8 +289,6 @@ def matmul(a, b, bias,
                 f"a_mx_scale must be uint8 [M, K/32], got {a_scale.dtype} {tuple(a_scale.shape)}"
             if a_scale.stride(-1) != 1:
                 a_scale = a_scale.contiguous()
-            keep.append(a_scale)
-            args.x_scale, args.ld_x_scale = a_scale.data_ptr(), a_scale.stride(0)
 
     # ---- shapes / output ------------------------------------------------------------------------------
     M = a.shape[0] if gather_indx is None else gather_indx.shape[0]
@@ -309,23 +302,23 @@ def matmul(a, b, bias,
     out_rows = M if scatter_indx is None else scatter_indx.shape[0]
     out_dtype = pc.out_dtype or a.dtype
     out_shape = (out_rows, N // red_n)
+    peers = None
     if fused_comm is not None:
         c = fused_comm.local
+        peers = (list(fused_comm.out_handles), int(fused_comm.rows_per_shard))
         assert c.ndim == 2 and c.shape[1] == N // red_n and c.stride(-1) == 1 and c.dtype == out_dtype
         assert c.shape[0] == fused_comm.rows_per_shard
-    elif c is None:
-        c = torch.empty(out_shape, dtype=out_dtype, device=dev)
-    else:
+    elif c is not None:
         if c.ndim == 3 and c.shape[0] == 1:
             c = c[0]
         assert tuple(c.shape) == out_shape and c.stride(-1) == 1 and c.dtype == out_dtype
     if M == 0 or N == 0:
-        return c
+        return torch.empty(out_shape, dtype=out_dtype, device=dev) if c is None else c
     if a_ragged_metadata is None:
         assert E == 1, "several weight matrices need a_ragged_metadata"
     # A plain dense product (the router's logits = x @ Wg + bg, bench/bench_mlp.py:70 of the reference) is a library
     # GEMM: cuBLAS through torch, fp32 accumulation, with the epilogue terms that apply to it.
-    if (args.w_kind == _lib.MOE_W_DENSE and kernel_choice == "auto" and a_ragged_metadata is None and gather_indx is None
+    if (w_kind == _lib.MOE_W_DENSE and tuning[0] == _lib.MOE_GEMM_AUTO and a_ragged_metadata is None and gather_indx is None
             and scatter_indx is None and fused_comm is None and act_name == "dflt" and betas is None and gammas is None
             and a.dtype in (torch.bfloat16, torch.float16) and a.is_cuda):
         try:
@@ -336,72 +329,21 @@ def matmul(a, b, bias,
             y = y + bias.reshape(1, -1).float()
         if out_alpha is not None:
             y = y * float(out_alpha)
+        if c is None:
+            return y.to(out_dtype)
         c.copy_(y)
         return c
-
-    def i32(t):
-        if t is None:
-            return None
-        t = t if t.dtype == torch.int32 else t.to(torch.int32)
-        t = t if t.is_contiguous() else t.contiguous()
-        keep.append(t)
-        return t.data_ptr()
-
-    def f32v(t):
-        if t is None:
-            return None
-        t = t if t.dtype == torch.float32 else t.float()
-        t = t if t.is_contiguous() else t.contiguous()
-        keep.append(t)
-        return t.data_ptr()
-
-    args.x, args.x_dtype, args.ld_x, args.rows_x = a.data_ptr(), _lib.dtype_code(a.dtype), a.stride(0), a.shape[0]
-    args.E, args.K, args.N, args.M = E, K, N, M
+    ragged = None
     if a_ragged_metadata is not None:
         md = a_ragged_metadata
-        assert md.block_offs_data.stride(1) == 1 and md.block_schedule_data.stride(1) == 1
-        args.slice_sizes, args.slice_offs = md.slice_sizes.data_ptr(), md.slice_offs.data_ptr()
-        args.block_offs_16, args.block_sched_16 = md.block_offs_data.data_ptr(), md.block_schedule_data.data_ptr()
-        args.ld_block_offs, args.ld_block_sched = md.block_offs_data.stride(0), md.block_schedule_data.stride(0)
+        ragged = (md.slice_sizes, md.slice_offs, md.block_offs_data, md.block_schedule_data)
     if bias is not None:
         if bias.ndim == 1:
             bias = bias.view(1, -1)
         assert bias.shape[-1] == N and bias.stride(-1) == 1
-        args.bias, args.bias_dtype, args.ld_bias = bias.data_ptr(), _lib.dtype_code(bias.dtype), bias.stride(0)
-    args.gather_indx, args.scatter_indx = i32(gather_indx), i32(scatter_indx)
-    args.betas, args.gammas = f32v(betas), f32v(gammas)
-    if out_alpha is not None:
-        args.out_alpha, args.has_out_alpha = float(out_alpha), 1
-    if act_name == "swiglu":
-        alpha, limit = fused_activation.fn_args
-        args.activation, args.act_alpha = _lib.MOE_ACT_SWIGLU, float(alpha)
-        args.act_limit, args.act_has_limit = (float(limit), 1) if limit is not None else (0.0, 0)
-    args.y, args.y_dtype, args.ld_y = c.data_ptr(), _lib.dtype_code(c.dtype), c.stride(0)
-    if fused_comm is not None:
-        args.n_y_peers, args.y_rows_per_peer = len(fused_comm.out_handles), int(fused_comm.rows_per_shard)
-        for i, h in enumerate(fused_comm.out_handles):
-            args.y_peers[i] = int(h)
-    args.kernel = {"auto": _lib.MOE_GEMM_AUTO, "simt": _lib.MOE_GEMM_SIMT, "tcgen05": _lib.MOE_GEMM_TCGEN05,
-                   "tcgen05-pair": _lib.MOE_GEMM_TCGEN05_PAIR, "stream": _lib.MOE_GEMM_STREAM,
-                   "mx": _lib.MOE_GEMM_MX, "mx-f8": _lib.MOE_GEMM_MX_F8, "mx-f4": _lib.MOE_GEMM_MX_F4}[kernel_choice]
-    args.tile_m, args.tile_n = resolve_tile_m(), resolve_tile_n()
-    args.idle_sms = get_idle_sms()
-    args.status = _status_word(dev).data_ptr()
-    if args.w_kind == _lib.MOE_W_MX4_B200MX:
-        ws_bytes = lib.moe_gemm_mx_workspace_bytes(args)
-        ws = torch.empty(ws_bytes + 1024, dtype=torch.uint8, device=dev)        # token blocks in the MMA's operand layout
-        keep.append(ws)
-        args.mx_workspace = (ws.data_ptr() + 1023) // 1024 * 1024
-        args.mx_workspace_bytes = ws_bytes
-    if gather_indx is not None and args.w_kind == _lib.MOE_W_MX4_B200 and a.dtype == torch.bfloat16 and M >= 2048:
-        scratch = torch.empty(M * K, dtype=torch.bfloat16, device=dev)   # the library decides whether to use it
-        keep.append(scratch)
-        args.gather_scratch, args.gather_scratch_bytes = scratch.data_ptr(), scratch.numel() * 2
-    st = lib.moe_grouped_gemm(args, _lib.stream())
-    if st == 3:
-        raise InapplicableConstraint(lib.moe_last_error().decode(errors="replace"))
-    _lib.check(st, "moe_grouped_gemm")
-    return c
+    return _lib.host().gemm(a, w_kind, wd, w_scale, E, K, N, ragged, bias, gather_indx, scatter_indx, betas, gammas, out_alpha,
+                            fused_activation.fn_args if act_name == "swiglu" else None, c, out_dtype, a_scale, tuning,
+                            _status_word(dev), peers)
 
 
 matmul_ogs = matmul          # the name this operator had in earlier releases of the reference

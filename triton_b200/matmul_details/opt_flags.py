@@ -94,3 +94,13 @@ def resolve_kernel_choice() -> str:
         else:
             raise InapplicableConstraint(f"unsupported opt_flags constraint {k!r}")
     return c.get("kernel", "auto")
+
+
+_KERNEL_CODE = {"auto": 0, "simt": 1, "tcgen05": 2, "tcgen05-pair": 3, "stream": 4, "mx": 5, "mx-f8": 6, "mx-f4": 7}   # MOE_GEMM_*
+
+
+def gemm_tuning() -> tuple:
+    """(kernel, tile_m, tile_n, idle_sms) of the current constraints, as the C argument block takes them."""
+    if not get_opt_flags_constraints():
+        return (0, 0, 0, _idle_sms)
+    return (_KERNEL_CODE[resolve_kernel_choice()], resolve_tile_m(), resolve_tile_n(), get_idle_sms())

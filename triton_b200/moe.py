@@ -10,15 +10,18 @@ from dataclasses import dataclass
 
 import torch
 
-from .matmul import FusedActivation, PrecisionConfig, matmul
+from . import _lib
+from .matmul import FusedActivation, PrecisionConfig, _status_word, matmul
+from .matmul_details.opt_flags import gemm_tuning
 from .numerics_details.mxfp import downcast_to_mxfp
 from .reduce import reduce
-from .routing import route, routing  # noqa: F401
+from .routing import FUSED_MAX_TOKENS, route, routing  # noqa: F401
 from .specialize import FnSpecs
 from .swiglu import swiglu_fn
 from .tensor import (FP4, Tensor, convert_layout, make_ragged_tensor_metadata, remap_ragged_tensor_metadata,
                      wrap_torch_tensor)
-from .tensor_details.layout import make_default_matmul_mxfp4_w_layout, make_default_matmul_mxfp4_w_scale_layout
+from .tensor_details.layout import (B200BlockScaledValueLayout, B200MXValueLayout, make_default_matmul_mxfp4_w_layout,
+                                    make_default_matmul_mxfp4_w_scale_layout)
 from .topk import topk
 
 
@@ -99,6 +102,25 @@ def _activation(lw):
     return FusedActivation(FnSpecs("swiglu", swiglu_fn, ("alpha", "limit"), reduction_n=2), (lw.alpha, lw.limit))
 
 
+_LAYER_KIND = {B200MXValueLayout: _lib.MOE_W_MX4_B200, B200BlockScaledValueLayout: _lib.MOE_W_MX4_B200MX}
+
+
+def _product(w: Tensor, scale: Tensor):
+    return _LAYER_KIND[type(w.storage.layout)], w.storage.data, scale.storage.data
+
+
+def _one_call(x, logits, lw: MoeLayerWeights, k: int) -> bool:
+    """Whether the step is one the native host path takes as a whole: fp32 logits, bf16 or e4m3 rows, weights and biases in
+    the forms this package prepares.  Anything else goes through the operators one by one."""
+    fp8 = x.dtype == torch.float8_e4m3fn
+    E = logits.shape[1] if logits.ndim == 2 else 0
+    return ((fp8 or x.dtype == torch.bfloat16) and logits.dtype == torch.float32 and 0 < E <= 256 and E == lw.n_expts
+            and 0 < k <= E and x.ndim == 2 and x.stride(1) == 1 and logits.stride(1) == 1 and 0 < x.shape[0] <= FUSED_MAX_TOKENS
+            and logits.shape[0] == x.shape[0] and x.shape[1] == lw.w1.shape[1] and (not fp8 or lw.w1_bs is not None)
+            and type(lw.w1.storage.layout) is B200MXValueLayout and type(lw.w2.storage.layout) is B200MXValueLayout
+            and lw.b1.stride(1) == 1 and lw.b2.stride(1) == 1 and lw.w1.shape[2] == 2 * lw.w2.shape[1])
+
+
 def moe_layer_forward(x, logits, lw: MoeLayerWeights, k: int, gemm_timer=None):
     """x [T, d_model] bf16, logits [T, E] -> [T, d_model]: sum over the k selected experts of
     softmax-weight * (SwiGLU(x W1 + b1) W2 + b2).
@@ -106,12 +128,19 @@ def moe_layer_forward(x, logits, lw: MoeLayerWeights, k: int, gemm_timer=None):
     e4m3 activations (`x.dtype == torch.float8_e4m3fn`, the reference's fp8 mode: bench/bench_mlp.py `x_dtype="fp8"`) run
     both GEMMs on the block-scaled kernel at every size: fc1 writes e4m3 rows, fc2 reads them and writes bf16."""
     T = x.shape[0]
+    if gemm_timer is None and _one_call(x, logits, lw, k):
+        if x.dtype == torch.float8_e4m3fn:
+            w1, w1_scale, w2, w2_scale = lw.w1_bs, lw.w1_bs_scale, lw.w2_bs, lw.w2_bs_scale
+        else:
+            w1, w1_scale, w2, w2_scale = lw.fc_weights(T * k)
+        return _lib.host().layer(x, logits, k, (*_product(w1, w1_scale), lw.b1, *w1.shape[1:]),
+                                 (*_product(w2, w2_scale), lw.b2, *w2.shape[1:]), lw.alpha, lw.limit, gemm_tuning(),
+                                 _status_word(x.device))
     ragged, sparse = route(logits, k, apply_softmax=True)
     md = sparse.mask_metadata
     n = T * k
     scatter_idx = md.col_sorted_indx                                    # sorted position -> flat (token, slot) row
     # token row and routing weight of every expert-sorted position, by one kernel (padding positions read no row)
-    from . import _lib
     gather_idx = torch.empty(n, dtype=torch.int32, device=x.device)
     gammas = torch.empty(n, dtype=torch.float32, device=x.device)
     indx16 = sparse.indx if sparse.indx.dtype == torch.int16 else sparse.indx.to(torch.int16)
@@ -242,7 +271,6 @@ def _forward_ep_peer(x_local, sparse, lw_local, k, expt_assignment, pool, gemm_t
     16 bytes from the GEMM epilogue into peer memory ran at a seventh of that) and stream-ordered barriers replace the
     two all-to-alls: one before the dispatch (shared with the all-gather of the routing outputs when the caller put the
     tokens into the pool's buffer ahead of it: `tokens_published`) and one before the combine."""
-    from . import _lib
     lib = _lib.load()
     mesh = pool.mesh
     W, rank = mesh.world_size, mesh.local_rank

@@ -17,27 +17,6 @@ class DequantScaleRoundingMode(Enum):
     ROUND_DOWN = 1    # scale = 2^floor(log2(max / 4)): the OCP rule, may clip
 
 
-def _collapse3(t, axis):
-    """View `t` (axis moved last) as [batch, outer, quant] with element strides, copying only when the
-    leading dimensions cannot be merged into two."""
-    tt = t.transpose(axis, -1)
-    lead = [(s, st) for s, st in zip(tt.shape[:-1], tt.stride()[:-1]) if s != 1]
-    merged = []
-    for s, st in lead:                       # merge adjacent dims that are contiguous with each other
-        if merged and merged[-1][1] == st * s:
-            merged[-1] = (merged[-1][0] * s, st)
-        else:
-            merged.append((s, st))
-    if len(merged) > 2:
-        tt = tt.contiguous()
-        outer = tt.numel() // max(tt.shape[-1], 1)
-        return tt, 1, outer, 0, tt.shape[-1], 1
-    while len(merged) < 2:
-        merged.insert(0, (1, 0))
-    (b, sb), (o, so) = merged
-    return tt, b, o, sb, so, tt.stride(-1)
-
-
 def downcast_to_mxfp(x, out_dtype, axis: int, scale_dtype: torch.dtype = torch.uint8,
                      microblock_size: int = MXFP_BLOCK_SIZE,
                      DEQUANT_SCALE_ROUNDING_MODE: DequantScaleRoundingMode = DequantScaleRoundingMode.ROUND_UP):
@@ -53,17 +32,8 @@ def downcast_to_mxfp(x, out_dtype, axis: int, scale_dtype: torch.dtype = torch.u
     axis %= x.ndim
     L = x.shape[axis]
     assert L % microblock_size == 0, f"axis dim must be divisible by {microblock_size}. Got {L}"
-    lib = _lib.load()
     # outputs: quantised axis innermost in memory, the other axes as in x.transpose(axis, -1)
-    lead = x.transpose(axis, -1).shape[:-1]
-    q = torch.empty((*lead, L // 2), dtype=torch.uint8, device=x.device)
-    s = torch.empty((*lead, L // 32), dtype=torch.uint8, device=x.device)
-    if x.numel() > 0:
-        xt, b, o, sb, so, sq = _collapse3(x, axis)
-        _lib.check(lib.moe_downcast_mxfp4(_lib.ptr(xt), _lib.dtype_code(x.dtype), b, o, L, sb, so, sq, _lib.ptr(q),
-                                          _lib.ptr(s), DEQUANT_SCALE_ROUNDING_MODE.value, _lib.stream()),
-                   "moe_downcast_mxfp4")
-    return q.transpose(axis, -1), s.transpose(axis, -1)
+    return _lib.host().downcast(x, axis, DEQUANT_SCALE_ROUNDING_MODE.value)
 
 
 def upcast_from_mxfp(tensor: torch.Tensor, scale: torch.Tensor, target_dtype: torch.dtype, axis: int,
@@ -77,18 +47,4 @@ def upcast_from_mxfp(tensor: torch.Tensor, scale: torch.Tensor, target_dtype: to
     ndim = tensor.ndim
     assert -ndim <= axis < ndim and tensor.ndim == scale.ndim
     axis %= ndim
-    lib = _lib.load()
-    q = tensor.transpose(axis, -1).contiguous()
-    s = scale.transpose(axis, -1).contiguous()
-    L = q.shape[-1] * 2
-    assert s.shape[-1] * 32 == L, "scale shape does not match the packed values"
-    out_shape = list(tensor.shape)
-    out_shape[axis] = L
-    out = torch.empty(out_shape, dtype=target_dtype, device=tensor.device)
-    if out.numel() > 0:
-        ot, b, o, sb, so, sq = _collapse3(out, axis)
-        _lib.check(lib.moe_upcast_mxfp4(_lib.ptr(q), _lib.ptr(s), _lib.ptr(ot), _lib.dtype_code(target_dtype), b, o, L,
-                                        sb, so, sq, _lib.stream()), "moe_upcast_mxfp4")
-        if ot.data_ptr() != out.data_ptr():      # more than two non-mergeable leading axes: written to a copy
-            out.transpose(axis, -1).copy_(ot)
-    return out
+    return _lib.host().upcast(tensor, scale, target_dtype, axis)

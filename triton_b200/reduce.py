@@ -39,10 +39,13 @@ def reduce(x: torch.Tensor, dim: int, mask: Optional[torch.Tensor] = None, scale
     if y_has_mx or (x_flex is not None and x_flex.scale is not None) or \
             (y_flex is not None and y_flex.expected_scale is not None):
         raise NotImplementedError("reduce: mx / flexpoint outputs are not supported")
-    lib = _lib.load()
     nonred = [d for d in range(3) if d != dim]
     S0, S1, R = x.shape[nonred[0]], x.shape[nonred[1]], x.shape[dim]
     y_dtype = y_dtype or x.dtype
+    if mask is None and scale is None:
+        assert y is None or tuple(y.shape) == (S0, S1)
+        return _lib.host().reduce(x, dim, y, y_dtype), None
+    lib = _lib.load()
     if y is None:
         y = torch.empty((S0, S1), device=x.device, dtype=y_dtype)
     assert tuple(y.shape) == (S0, S1)

@@ -7,7 +7,7 @@ import torch
 
 from . import _lib
 from .matmul import _status_word
-from .tensor import BIT, SparseMatrix, wrap_torch_tensor
+from .tensor import SparseMatrix, bit_tensor
 from .topk import topk
 
 
@@ -51,11 +51,6 @@ def router_topk(x: torch.Tensor, wg: torch.Tensor, bg, k: int, apply_softmax: bo
     T, K = x.shape
     E = wg.shape[1]
     dev = x.device
-    vals = torch.empty((T, k), dtype=logits_dtype, device=dev)
-    indx = torch.empty((T, k), dtype=torch.int16, device=dev)
-    words, t_pad = (E + 31) // 32, (T + 31) // 32 * 32
-    bm_store = torch.empty((words, t_pad), dtype=torch.int32, device=dev)
-    bm = bm_store.transpose(0, 1)[:T]
     logits = torch.empty((T, E), dtype=torch.float32, device=dev) if return_logits else None
     ws_bytes = lib.moe_router_topk_workspace_bytes(T, K, E)
     ws = _lib.zero_scratch(dev, ws_bytes) if ws_bytes > 0 else None
@@ -65,14 +60,7 @@ def router_topk(x: torch.Tensor, wg: torch.Tensor, bg, k: int, apply_softmax: bo
         return _two_steps(logits.to(logits_dtype), k, apply_softmax, return_logits)
     if bg is not None and bg.dtype not in (torch.float32, torch.bfloat16):
         bg = bg.float()
-    if T > 0:
-        _lib.check(lib.moe_router_topk(_lib.ptr(x), T, K, x.stride(0), _lib.ptr(wg), wg.stride(1), _lib.ptr(bg),
-                                       _lib.dtype_code(bg.dtype) if bg is not None else 0, E, k, int(bool(apply_softmax)),
-                                       int(logits_dtype == torch.bfloat16), _lib.ptr(logits), E, _lib.ptr(vals),
-                                       _lib.dtype_code(vals.dtype), vals.stride(0), _lib.ptr(indx), indx.stride(0), _lib.ptr(bm),
-                                       bm.stride(0), bm.stride(1), _lib.ptr(ws), ws_bytes if ws is not None else 0,
-                                       _status_word(dev).data_ptr(),
-                                       _lib.stream()), "moe_router_topk")
-    bitmatrix = wrap_torch_tensor(bm, dtype=BIT, shape=[T, E], shape_max=[T, None])
-    sp = SparseMatrix(indx=indx, vals=vals, mask=bitmatrix)
+    vals, indx, bm = _lib.host().router(x, wg, bg, k, bool(apply_softmax), logits_dtype == torch.bfloat16, logits, ws, ws_bytes,
+                                        _status_word(dev))
+    sp = SparseMatrix(indx=indx, vals=vals, mask=bit_tensor(bm, T, E))
     return (sp, logits) if return_logits else sp

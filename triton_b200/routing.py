@@ -3,8 +3,8 @@ its tests today (python/triton_kernels/tests/test_distributed.py:203-210)."""
 import torch
 
 from . import _lib
-from .tensor import BIT, BitmatrixMetadata, RaggedTensorMetadata, SparseMatrix, make_ragged_tensor_metadata, wrap_torch_tensor
-from .tensor_details.ragged_tensor import _empty_aligned
+from .tensor import BitmatrixMetadata, SparseMatrix, bit_tensor, make_ragged_tensor_metadata
+from .tensor_details.ragged_tensor import ragged_from_kernel
 from .topk import topk
 
 
@@ -21,33 +21,12 @@ def route(logits, n_expts_act, apply_softmax=True):
         sparse = topk(logits, n_expts_act, apply_softmax=apply_softmax)
         md = sparse.mask_metadata
         return make_ragged_tensor_metadata(md.col_sum, md.row_sorted_indx.shape[0]), sparse
-    lib = _lib.load()
     T, E = logits.shape
-    k = n_expts_act
-    dev = logits.device
-    vals = torch.empty((T, k), dtype=logits.dtype, device=dev)
-    indx = torch.empty((T, k), dtype=torch.int16, device=dev)
-    words, t_pad = (E + 31) // 32, (T + 31) // 32 * 32
-    bm_store = torch.empty((words, t_pad), dtype=torch.int32, device=dev)
-    bm = bm_store.transpose(0, 1)[:T]
-    col_sum = torch.empty(E, dtype=torch.int32, device=dev)
-    combined = torch.empty(2 * T * k, dtype=torch.int32, device=dev)
-    col_sorted, row_sorted = combined[: T * k], combined[T * k:]
-    mnb = RaggedTensorMetadata.max_n_blocks(E, T * k)
-    offs = _empty_aligned((5, E + 1), dev)
-    sched = _empty_aligned((4, mnb), dev)
-    slice_offs, block_offs = offs[0], offs[1:]
-    ws_bytes = lib.moe_route_workspace(T, E, k)
-    ws = torch.empty(max(ws_bytes, 4), dtype=torch.uint8, device=dev)
-    _lib.check(lib.moe_route(_lib.ptr(logits), _lib.dtype_code(logits.dtype), T, E, k, int(bool(apply_softmax)), logits.stride(0),
-                             _lib.ptr(vals), vals.stride(0), _lib.ptr(indx), indx.stride(0), _lib.ptr(bm), bm.stride(0),
-                             bm.stride(1), _lib.ptr(col_sum), _lib.ptr(col_sorted), _lib.ptr(row_sorted), _lib.ptr(slice_offs),
-                             _lib.ptr(block_offs), block_offs.stride(0), _lib.ptr(sched), sched.stride(0), mnb, _lib.ptr(ws),
-                             ws_bytes, _lib.stream()), "moe_route")
-    bitmatrix = wrap_torch_tensor(bm, dtype=BIT, shape=[T, E], shape_max=[T, None])
-    sparse = SparseMatrix(indx=indx, vals=vals, mask=bitmatrix,
+    vals, indx, bm, col_sum, col_sorted, row_sorted, slice_offs, block_offs, sched = \
+        _lib.host().route(logits, n_expts_act, bool(apply_softmax))
+    sparse = SparseMatrix(indx=indx, vals=vals, mask=bit_tensor(bm, T, E),
                           mask_metadata=BitmatrixMetadata(col_sum=col_sum, col_sorted_indx=col_sorted, row_sorted_indx=row_sorted))
-    return RaggedTensorMetadata(col_sum, slice_offs, block_offs, sched), sparse
+    return ragged_from_kernel(col_sum, slice_offs, block_offs, sched), sparse
 
 
 def routing(logits, n_expts_act, all_gather=False, y_indx=None, symm_mem_pool=None, apply_softmax=True):

@@ -81,6 +81,17 @@ class Tensor:
         return self.shape if i is None else self.shape[i]
 
 
+_BIT_LAYOUT = StridedLayout(major_dim=-2)
+
+
+def bit_tensor(bm, T, E):
+    """BIT tensor [T, E] over the top-k kernels' bitmatrix view: what `wrap_torch_tensor(bm, dtype=BIT, shape=[T, E],
+    shape_max=[T, None])` returns, without its checks (it is made on every routing call)."""
+    t = Tensor.__new__(Tensor)
+    t.storage, t.dtype, t.shape, t.shape_max = Storage(bm, _BIT_LAYOUT), BIT, [T, E], [T, bm.shape[1]]
+    return t
+
+
 make_bitmatrix_metadata = bitmatrix_details.make_bitmatrix_metadata
 make_ragged_tensor_metadata = ragged_tensor_details.make_ragged_tensor_metadata
 remap_ragged_tensor_metadata = ragged_tensor_details.remap_ragged_tensor_metadata

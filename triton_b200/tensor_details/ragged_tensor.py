@@ -58,6 +58,13 @@ class RaggedTensorMetadata:
         return [2**x for x in RaggedTensorMetadata.block_sizes_log2()]
 
 
+def ragged_from_kernel(slice_sizes, slice_offs, block_offs_data, block_schedule_data):
+    """Metadata whose arrays a kernel of this library has just laid out (nothing to check)."""
+    md = RaggedTensorMetadata.__new__(RaggedTensorMetadata)
+    md.slice_sizes, md.slice_offs, md.block_offs_data, md.block_schedule_data = slice_sizes, slice_offs, block_offs_data, block_schedule_data
+    return md
+
+
 def ragged_metadata_fields(metadata, block_size):
     return (metadata.slice_sizes, metadata.slice_offs, metadata.block_offs(block_size),
             metadata.block_schedule(block_size), metadata.expected_slice_size, metadata.slice_sizes_divisibility or 1)

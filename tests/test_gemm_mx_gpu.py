@@ -305,6 +305,9 @@ def test_block_scaled_few_tiles_k_step_stages(K, sizes, act, device):
     (160, 129, [31, 32, 5, 449]),                   # k tail, odd width (scalar stores), an expert of several tiles
     (416, 514, [64, 1, 0, 97]),                     # ring longer than the k loop, a second tile of weight blocks
     (1024, 768, [300]),                             # three 256-row blocks: the last tile has one unit
+    (160, 5129, [31, 32, 95, 449]),                 # enough tiles for two 256-row blocks each, the last has one row
+    (96, 4866, [300, 2, 2, 700]),                   # the same with more rows per expert
+    (96, 514, [225, 385]),                          # more rows per expert, one 256-row block each
 ])
 @pytest.mark.parametrize("act", [False, True])
 def test_pair_kernel_tile_edges(K, N, sizes, acts, act, device):
@@ -335,3 +338,69 @@ def test_pair_kernel_tile_edges(K, N, sizes, acts, act, device):
     y = run_mx(x, wq, ws, sizes_t, device, a_scale=a_scale, bias=bias, gather=gather, scatter=scatter, gammas=gammas, betas=betas,
                act=(1.702, 7.0) if act else None, out_dtype=torch.float32, block_m=256)
     assert oracle.rel_l2(out, y) < 2e-5
+
+
+@pytest.mark.parametrize("K, N, sizes", [
+    (32, 2, [1, 0, 33]),                            # one group of k, one column pair
+    (128, 256, [192, 193, 224, 225]),               # one whole k step, one 256-row block
+    (160, 129, [31, 32, 5, 449]),                   # k tail, odd width, an expert of several tiles
+    (416, 514, [64, 1, 0, 97]),                     # a second tile of weight blocks
+    (1024, 768, [300, 2, 2]),                       # three 256-row blocks: the last tile has one
+    (160, 5129, [31, 32, 95, 449]),                 # enough tiles for two 256-row blocks each, the last has one row
+    (96, 4866, [300, 2, 2, 700]),                   # the same with more rows per expert
+    (96, 514, [225, 385]),                          # more rows per expert, one 256-row block each
+])
+@pytest.mark.parametrize("act", [False, True])
+def test_pair_kernel_on_default_weight_tiles(K, N, sizes, act, device):
+    """The pair kernel fed from the default layout (rows of a weight block permuted, k permuted inside eight).  As above, only
+    the order of an fp32 sum of exact products differs."""
+    from triton_b200.tensor_details.layout import B200MXScaleLayout, B200MXValueLayout
+    if act and N % 2:
+        pytest.skip("SwiGLU needs an even width")
+    g = torch.Generator().manual_seed(K + N + len(sizes))
+    E, M = len(sizes), sum(sizes)
+    sizes_t = torch.tensor(sizes, dtype=torch.int32)
+    wq, ws, wdeq = quantised_weights(E, K, N, g)
+    T = M + 7
+    x = torch.randn(T, K, generator=g).bfloat16()
+    gather = torch.randint(0, T, (M,), generator=g, dtype=torch.int32)
+    scatter, gammas, betas = torch.randperm(M, generator=g).int(), torch.rand(M, generator=g), torch.rand(M, generator=g)
+    bias = torch.randn(E, N, generator=g) * 0.1
+    ref = oracle.matmul_oracle(x.float()[gather.long()], wdeq, bias, sizes_t, None, None, betas=betas, out_dtype=torch.float32)
+    if act:
+        ref = oracle.swiglu_oracle(ref, 1.702, 7.0)
+    out = torch.zeros_like(ref)
+    out[scatter.long()] = ref * gammas[:, None]
+    dev = lambda t: t.to(device)
+    pc = tb.PrecisionConfig(b_mx_scale=convert_layout(wrap_torch_tensor(dev(ws)), B200MXScaleLayout()), b_microblock_size=32,
+                            out_dtype=torch.float32)
+    fa = tb.FusedActivation(tb.FnSpecs("swiglu", tb.swiglu_fn, ("alpha", "limit"), reduction_n=2), (1.702, 7.0)) if act else None
+    with tb.scoped_opt_flags_constraints({"kernel": "mx"}):
+        y = tb.matmul(dev(x), convert_layout(wrap_torch_tensor(dev(wq), dtype=FP4), B200MXValueLayout()), dev(bias),
+                      tb.make_ragged_tensor_metadata(dev(sizes_t), M), None, dev(gather), dev(scatter), pc, betas=dev(betas),
+                      gammas=dev(gammas), fused_activation=fa)
+    tb.matmul_check_status()
+    assert oracle.rel_l2(out, y.cpu()) < 2e-5
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("tiled", [False, True])
+def test_pair_kernel_non_finite_tokens(value, tiled, device):
+    """A token row with a NaN or an infinity gives a row without finite values; the other rows are untouched."""
+    from triton_b200.tensor_details.layout import B200MXScaleLayout, B200MXValueLayout
+    g = torch.Generator().manual_seed(4)
+    wq, ws, wdeq = quantised_weights(1, 256, 256, g)
+    x = torch.randn(64, 256, generator=g).bfloat16()
+    x[5, 77] = value
+    sizes = torch.tensor([64], dtype=torch.int32)
+    if tiled:
+        pc = tb.PrecisionConfig(b_mx_scale=convert_layout(wrap_torch_tensor(ws.to(device)), B200MXScaleLayout()), b_microblock_size=32)
+        with tb.scoped_opt_flags_constraints({"kernel": "mx"}):
+            y = tb.matmul(x.to(device), convert_layout(wrap_torch_tensor(wq.to(device), dtype=FP4), B200MXValueLayout()), None,
+                          tb.make_ragged_tensor_metadata(sizes.to(device), 64), precision_config=pc).cpu()
+    else:
+        y = run_mx(x, wq, ws, sizes, device, block_m=256)
+    assert not torch.isfinite(y[5]).any()
+    keep = torch.arange(64) != 5
+    ref = oracle.matmul_oracle(x[keep].float(), wdeq, None, torch.tensor([63], dtype=torch.int32), out_dtype=torch.float32)
+    assert oracle.rel_l2(ref, y[keep].float()) < 1e-2

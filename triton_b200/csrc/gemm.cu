@@ -10,6 +10,9 @@ int moe_gemm_stream_launch(const GemmParams& p, const MoeGemmArgs& a, cudaStream
 bool moe_gemm_stream_supported(const MoeGemmArgs& a, const char** why);
 int moe_gemm_mx_launch(const GemmParams& p, const MoeGemmArgs& a, cudaStream_t st);
 bool moe_gemm_mx_supported(const MoeGemmArgs& a, const char** why);
+bool moe_gemm_mx_pair_wanted(const MoeGemmArgs& a);
+int64_t moe_gemm_mx_pair_workspace(const MoeGemmArgs& a);
+int moe_gemm_mx_pair_launch(const GemmParams& p, const MoeGemmArgs& a, cudaStream_t st);
 
 // upper bound on the number of row blocks (triton_kernels tensor_details/ragged_tensor.py:73-77)
 static int64_t n_blocks_bound(int64_t n_slices, int64_t n_rows, int64_t block) {
@@ -64,6 +67,10 @@ extern "C" __attribute__((visibility("default"))) int moe_grouped_gemm(const Moe
 
   const char* why = "";
   const bool mx_asked = a->kernel == MOE_GEMM_MX || a->kernel == MOE_GEMM_MX_F8 || a->kernel == MOE_GEMM_MX_F4;
+  // default tiles on the block-scaled pair kernel; without its workspace they stay with the kernels below
+  if (a->w_kind == MOE_W_MX4_B200 && moe_gemm_mx_pair_wanted(*a) &&
+      (mx_asked || (a->mx_workspace && a->mx_workspace_bytes >= moe_gemm_mx_pair_workspace(*a))))
+    return moe_gemm_mx_pair_launch(p, *a, st);
   if (a->w_kind == MOE_W_MX4_B200MX || mx_asked) {
     // weights laid out for the block-scaled MMA: that kernel or nothing
     if (!moe_gemm_mx_supported(*a, &why) || (a->kernel != MOE_GEMM_AUTO && !mx_asked)) {
@@ -90,8 +97,7 @@ extern "C" __attribute__((visibility("default"))) int moe_grouped_gemm(const Moe
     else if (a->kernel != MOE_GEMM_STREAM)
       streaming = false;
     if (streaming) return moe_gemm_stream_launch(p, *a, st);
-    // Large problems run on pairs of SMs (256 x 256 tiles, cta_group::2); small ones and explicit tile requests on
-    // the single-SM kernel.
+    // (the bf16 kernel on pairs of SMs, 256 x 256 tiles, runs on request only)
     bool pair = moe_gemm_tc_pair_supported(*a, &why);
     if (a->kernel == MOE_GEMM_TCGEN05_PAIR && !pair) {
       moe_set_error("moe_grouped_gemm: SM-pair tcgen05 kernel not applicable: %s", why);

@@ -287,7 +287,7 @@ __device__ __forceinline__ uint32_t mx_idesc(int n, uint32_t sf) {
 __device__ __forceinline__ uint32_t mx4_idesc(int n, uint32_t sf) {
   return (sf << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | (1u << 23) | (1u << 27) | (sf << 29);
 }
-// One block-scaled MMA of either kind, issued by the lane whose `leader` is set while the whole warp runs the loop: the
+// One block-scaled MMA of either kind, issued by an elected lane while the whole warp runs the loop: the
 // operands of tcgen05.mma live in uniform registers, and computed by a single thread of a divergent branch each of them took a
 // move from a vector register first (87-95 cycles per instruction; a block-scaled MMA of up to 64 columns runs 45).  Of a
 // shared-memory descriptor only the low word varies.
@@ -296,22 +296,22 @@ constexpr uint32_t MX_DESC_HI_SW128 = (1024u >> 4) | (1u << 14) | (2u << 29);   
 constexpr uint32_t MX_DESC_HI_SW64 = (512u >> 4) | (1u << 14) | (4u << 29);            // 64-byte rows and swizzle
 template <bool F4>
 __device__ __forceinline__ void mma_mx(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t sfa, uint32_t sfb,
-                                       uint32_t accumulate, uint32_t leader) {
+                                       uint32_t accumulate) {
   if constexpr (F4)
     asm volatile(
         "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
-        "mov.b64 da, {%1, %8};\n\tmov.b64 db, {%2, %8};\n\t"
-        "setp.ne.b32 p, %6, 0;\n\tsetp.ne.b32 q, %7, 0;\n\t"
+        "mov.b64 da, {%1, %7};\n\tmov.b64 db, {%2, %7};\n\t"
+        "setp.ne.b32 p, %6, 0;\n\telect.sync _|q, 0xFFFFFFFF;\n\t"
         "@q tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], da, db, %3, [%4], [%5], p;\n\t}" ::"r"(d_tmem),
-        "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate), "r"(leader), "n"(MX_DESC_HI_SW64)
+        "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate), "n"(MX_DESC_HI_SW64)
         : "memory");
   else
     asm volatile(
         "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
-        "mov.b64 da, {%1, %8};\n\tmov.b64 db, {%2, %8};\n\t"
-        "setp.ne.b32 p, %6, 0;\n\tsetp.ne.b32 q, %7, 0;\n\t"
+        "mov.b64 da, {%1, %7};\n\tmov.b64 db, {%2, %7};\n\t"
+        "setp.ne.b32 p, %6, 0;\n\telect.sync _|q, 0xFFFFFFFF;\n\t"
         "@q tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale.scale_vec::1X [%0], da, db, %3, [%4], [%5], p;\n\t}" ::"r"(d_tmem),
-        "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate), "r"(leader), "n"(MX_DESC_HI_SW128)
+        "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate), "n"(MX_DESC_HI_SW128)
         : "memory");
 }
 
@@ -391,51 +391,49 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
 
   if (warp == 0) {
     // ================================= producer =======================================================
-    if (lane == 0) {
-      uint32_t it = 0;
-      bool ok = true;
-      while (ok && sched.next(pid_m, nb0, mb_live)) {
-        int e; int64_t row0; int rows;
-        mx_map_block(p, q.tb, pid_m, e, row0, rows);
-        const uint8_t* xsrc = q.xq + pid_m * KT * q.chunk_bytes;
-        const CUtensorMap* w_map = &w_maps.m[mb_live - 1];
-        for (int kt = 0; kt < KS; ++kt, ++it) {
-          const int s = it % STAGES;
-          ok = mbar_wait(BAR_EMPTY(s), ((it / STAGES) & 1u) ^ 1u, ctl, 601);
-          if (!ok) break;
-          const uint32_t st = sbase + (uint32_t)s * (uint32_t)q.stage_bytes;
-          if constexpr (KM) {
-            const int k_live = min(3, KT - 3 * kt);
-            mbar_expect_tx(BAR_FULL(s), (uint32_t)k_live * ((uint32_t)(MX_W_TILE_TX + MX_WS_TILE) + (uint32_t)q.chunk_bytes));
-            for (int i = 0; i < k_live; ++i) {
-              const int64_t tile = ((int64_t)e * KT + 3 * kt + i) * NB + nb0;
-              tma_tile_3d(st + (uint32_t)i * W_TILE, &w_maps.m[0], 0, 0, (int)tile, BAR_FULL(s));
-              bulk_g2s(st + OFF_WS + (uint32_t)i * MX_WS_TILE, p.w_scale + tile * MX_WS_TILE, (uint32_t)MX_WS_TILE, BAR_FULL(s));
-            }
-            bulk_g2s(st + OFF_X, xsrc + (int64_t)(3 * kt) * q.chunk_bytes, (uint32_t)k_live * (uint32_t)q.chunk_bytes, BAR_FULL(s));
-          } else {
-            const int64_t tile = ((int64_t)e * KT + kt) * NB + nb0;
-            mbar_expect_tx(BAR_FULL(s), (uint32_t)(mb_live * (MX_W_TILE_TX + MX_WS_TILE)) + (uint32_t)q.chunk_bytes);
-            tma_tile_3d(st, w_map, 0, 0, (int)tile, BAR_FULL(s));
-            bulk_g2s(st + OFF_WS, p.w_scale + tile * MX_WS_TILE, (uint32_t)(mb_live * MX_WS_TILE), BAR_FULL(s));
-            bulk_g2s(st + OFF_X, xsrc + (int64_t)kt * q.chunk_bytes, (uint32_t)q.chunk_bytes, BAR_FULL(s));
+    uint32_t s = 0, ph = 1, issued = 0;
+    bool ok = true;
+    while (ok && sched.next(pid_m, nb0, mb_live)) {
+      int e; int64_t row0; int rows;
+      mx_map_block(p, q.tb, pid_m, e, row0, rows);
+      const uint32_t chunk = (uint32_t)q.chunk_bytes;
+      const uint8_t* xsrc = q.xq + pid_m * KT * chunk;
+      const CUtensorMap* w_map = &w_maps.m[KM ? 0 : mb_live - 1];
+      int tile = __shfl_sync(0xFFFFFFFFu, e, 0) * KT * NB + nb0;             // weight tile of the stage's first k step
+      for (int kt = 0; kt < KS; ++kt, ++issued) {
+        ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_EMPTY(s), ph, ctl, 601));
+        if (!ok) break;
+        const uint32_t st = sbase + s * (uint32_t)q.stage_bytes, bar = BAR_FULL(s);
+        if constexpr (KM) {
+          const int k_live = min(3, KT - 3 * kt);
+          elect_expect_tx(bar, (uint32_t)k_live * ((uint32_t)(MX_W_TILE_TX + MX_WS_TILE) + chunk));
+          for (int i = 0; i < k_live; ++i, tile += NB) {
+            elect_tile_3d(st + (uint32_t)i * W_TILE, w_map, 0, 0, tile, bar);
+            elect_bulk_g2s(st + OFF_WS + (uint32_t)i * MX_WS_TILE, p.w_scale + (int64_t)tile * MX_WS_TILE, (uint32_t)MX_WS_TILE, bar);
           }
+          elect_bulk_g2s(st + OFF_X, xsrc, (uint32_t)k_live * chunk, bar);
+          xsrc += 3 * chunk;
+        } else {
+          elect_expect_tx(bar, (uint32_t)(mb_live * (MX_W_TILE_TX + MX_WS_TILE)) + chunk);
+          elect_tile_3d(st, w_map, 0, 0, tile, bar);
+          elect_bulk_g2s(st + OFF_WS, p.w_scale + (int64_t)tile * MX_WS_TILE, (uint32_t)(mb_live * MX_WS_TILE), bar);
+          elect_bulk_g2s(st + OFF_X, xsrc, chunk, bar);
+          xsrc += chunk; tile += NB;
         }
+        if (++s == (uint32_t)STAGES) { s = 0; ph ^= 1u; }
       }
-      if (!ok) {
-        // aborting: let the copies that were already issued land before the CTA leaves
-        const uint32_t lo = it > (uint32_t)STAGES ? it - STAGES : 0;
-        for (uint32_t j = lo; j < it; ++j)
-          for (uint32_t i = 0; i < (1u << 16) && !mbar_test(BAR_FULL(j % STAGES), (j / STAGES) & 1u); ++i) __nanosleep(64);
-      }
+    }
+    if (!ok && lane == 0) {
+      // aborting: let the copies that were already issued land before the CTA leaves
+      for (uint32_t j = issued > (uint32_t)STAGES ? issued - STAGES : 0; j < issued; ++j)
+        for (uint32_t i = 0; i < (1u << 16) && !mbar_test(BAR_FULL(j % STAGES), (j / STAGES) & 1u); ++i) __nanosleep(64);
     }
     __syncwarp();
   } else if (warp == 1) {
     // ================================= MMA issuer =====================================================
-    const uint32_t leader = elect_one();
     const uint32_t idesc = F4 ? mx4_idesc(q.n_mma, 0) : mx_idesc(q.n_mma, 0);
     uint32_t s = 0, ph = 0, tc = 0;                    // stage and parity of the next k step
-    bool ok = true;
+    bool ok = true, ready = false;                     // ready: the next step was complete when the last one was issued
     for (; ok && sched.next(pid_m, nb0, mb_live); ++tc) {
       const uint32_t ab = tc % (uint32_t)q.acc_bufs;
       ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_ACC_EMPTY(ab), ((tc / (uint32_t)q.acc_bufs) & 1u) ^ 1u, ctl, 603));
@@ -443,9 +441,8 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
       tc_fence_after();
       const uint32_t d_tmem = tmem_base + ab * (uint32_t)acc_stride;
       for (int kt = 0; kt < KS; ++kt) {
-        ok = mbar_wait(BAR_FULL(s), ph, ctl, 602);
-        ok = ok && mbar_wait(BAR_SF(s), ph, ctl, 606);
-        ok = __all_sync(0xFFFFFFFFu, ok);
+        // (the scale loaders have seen the stage's copies land)
+        if (!__all_sync(0xFFFFFFFFu, ready)) ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_SF(s), ph, ctl, 602));
         if (!ok) break;
         tc_fence_after();
         const uint32_t st = sbase + s * (uint32_t)q.stage_bytes;
@@ -462,7 +459,7 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
 #pragma unroll
               for (int kk = 0; kk < 2; ++kk)
                 mma_mx<true>(d_tmem, a_lo + i * (W_TILE >> 4) + kk * 2, b_lo + i * bstep + kk * 2, idesc + (uint32_t)kk * ((2u << 4) + (2u << 29)),
-                             sf + 4 * i, sf + 12 + 4 * i, (i | kk) ? 1u : more, leader);
+                             sf + 4 * i, sf + 12 + 4 * i, (i | kk) ? 1u : more);
             }
           }
         } else {
@@ -474,7 +471,7 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
 #pragma unroll
               for (int mb = 0; mb < MB; ++mb)
                 mma_mx<F4>(d_tmem + (uint32_t)(mb * q.n_mma), a_lo + mb * (W_TILE >> 4) + kk * 2, b_lo + kk * 2, idesc + kk * SFK, sf + 4 * mb,
-                           sf + 4 * MB, kk ? 1u : more, leader);
+                           sf + 4 * MB, kk ? 1u : more);
           } else {
 #pragma unroll
             for (int kk = 0; kk < KK; ++kk)
@@ -482,16 +479,17 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
               for (int mb = 0; mb < MB; ++mb)
                 if (mb < mb_live)
                   mma_mx<F4>(d_tmem + (uint32_t)(mb * q.n_mma), a_lo + mb * (W_TILE >> 4) + kk * 2, b_lo + kk * 2, idesc + kk * SFK, sf + 4 * mb,
-                             sf + 4 * MB, kk ? 1u : more, leader);
+                             sf + 4 * MB, kk ? 1u : more);
           }
         }
-        mma_commit(BAR_EMPTY(s), leader);
+        elect_commit(BAR_EMPTY(s));
         if (++s == (uint32_t)STAGES) { s = 0; ph ^= 1u; }
+        ready = mbar_test(BAR_SF(s), ph);
       }
-      if (ok) mma_commit(BAR_ACC_FULL(ab), leader);
+      if (ok) elect_commit(BAR_ACC_FULL(ab));
     }
     // every MMA issued by this warp has retired before tensor memory is freed
-    mma_commit(BAR_DRAIN, leader);
+    elect_commit(BAR_DRAIN);
     mbar_wait(BAR_DRAIN, 0, ctl, 605);
     __syncwarp();
   } else if (warp >= 6) {
@@ -772,7 +770,8 @@ bool moe_gemm_mx_supported(const MoeGemmArgs& a, const char** why) {
 
 extern "C" __attribute__((visibility("default"))) size_t moe_gemm_mx_workspace_bytes(const MoeGemmArgs* a) {
   if (!a || a->M <= 0 || a->E <= 0) return 0;
-  return (size_t)(moe_gemm_mx_pair_wanted(*a) ? moe_gemm_mx_pair_workspace(*a) : mx_plan(*a).ws_bytes);
+  if (moe_gemm_mx_pair_wanted(*a)) return (size_t)moe_gemm_mx_pair_workspace(*a);
+  return a->w_kind == MOE_W_MX4_B200MX ? (size_t)mx_plan(*a).ws_bytes : 0;
 }
 
 int moe_gemm_mx_launch(const GemmParams& p_in, const MoeGemmArgs& a, cudaStream_t st) {

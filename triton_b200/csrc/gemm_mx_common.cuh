@@ -33,16 +33,9 @@ __device__ __forceinline__ void mx8_scale(float amax, uint32_t& sb, float& scale
   inv = __uint_as_float((254u - sb) << 23);
 }
 
-// 3-D tile copy: box (128 elements, 128 rows, MB tiles) of the weight tensor map, starting at tile `z`
-__device__ __forceinline__ void tma_tile_3d(uint32_t dst, const CUtensorMap* tmap, int x, int y, int z, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
-      "l"(tmap), "r"(x), "r"(y), "r"(z), "r"(bar)
-      : "memory");
-}
-// Tensor map over the value tiles of the block-scaled layout, boxes of n_blocks tiles; `packed`: 64-byte rows as they are,
-// else expanded by the TMA unit for kind::mxf8f6f4.
-inline int make_w_map(const MoeGemmArgs& a, int KT, int NB, bool packed, int n_blocks, CUtensorMap* map) {
+// cuTensorMapEncodeTiled with the defaults of these kernels
+inline int encode_map(CUtensorMap* map, CUtensorMapDataType type, int rank, const void* base, const cuuint64_t* dims, const cuuint64_t* strides,
+                      const cuuint32_t* box, CUtensorMapSwizzle swizzle, const char* what) {
   static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
   static std::mutex mu;
   {
@@ -58,24 +51,55 @@ inline int make_w_map(const MoeGemmArgs& a, int KT, int NB, bool packed, int n_b
       encode = (PFN_cuTensorMapEncodeTiled_v12000)fn;
     }
   }
-  // [tile][128 rows][128 e2m1 = 64 bytes].  Byte-per-element form: the TMA unit writes 16 elements per 16 bytes of
-  // shared memory (128-byte rows, 128-byte swizzle); packed form: the 64-byte rows as they are, 64-byte swizzle.
-  const cuuint64_t tiles = (cuuint64_t)a.E * (cuuint64_t)KT * (cuuint64_t)NB;
-  const cuuint64_t inner = packed ? 64 : 128;
-  const cuuint64_t dims[3] = {inner, 128, tiles};
-  const cuuint64_t strides[2] = {64, 64 * 128};
-  const cuuint32_t box[3] = {(cuuint32_t)inner, 128, (cuuint32_t)n_blocks};
-  const cuuint32_t estr[3] = {1, 1, 1};
-  const CUresult r = encode(map, packed ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_16U4_ALIGN16B, 3,
-                            const_cast<void*>(a.w), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                            packed ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  const cuuint32_t estr[4] = {1, 1, 1, 1};
+  const CUresult r = encode(map, type, rank, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
-    moe_set_error("moe_grouped_gemm: cuTensorMapEncodeTiled (packed e2m1 weights) failed with code %d (%llu tiles)", (int)r,
-                  (unsigned long long)tiles);
+    moe_set_error("moe_grouped_gemm: cuTensorMapEncodeTiled (%s) failed with code %d", what, (int)r);
     return MOE_ERR_CUDA;
   }
   return MOE_OK;
+}
+
+// Tensor map over the value tiles of the block-scaled layout, boxes of n_blocks tiles.  [tile][128 rows][128 e2m1 = 64 bytes];
+// `packed`: the 64-byte rows as they are, 64-byte swizzle; else the TMA unit writes 16 elements per 16 bytes of shared memory
+// (128-byte rows, 128-byte swizzle), the operand form of kind::mxf8f6f4.
+inline int make_w_map(const MoeGemmArgs& a, int KT, int NB, bool packed, int n_blocks, CUtensorMap* map) {
+  const cuuint64_t inner = packed ? 64 : 128;
+  const cuuint64_t dims[3] = {inner, 128, (cuuint64_t)a.E * (cuuint64_t)KT * (cuuint64_t)NB};
+  const cuuint64_t strides[2] = {64, 64 * 128};
+  const cuuint32_t box[3] = {(cuuint32_t)inner, 128, (cuuint32_t)n_blocks};
+  return encode_map(map, packed ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_16U4_ALIGN16B, 3, a.w, dims, strides, box,
+                    packed ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, "packed e2m1 weights");
+}
+
+// ---- copies issued by a warp that runs its loop as a whole: the instruction is guarded by an election next to it and its operands
+// live in uniform registers (issued by a single thread of a divergent branch, a copy cost about 150 cycles)
+__device__ __forceinline__ void elect_expect_tx(uint32_t bar, uint32_t bytes) {
+  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xFFFFFFFF;\n\t@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(bar),
+               "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ void elect_bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\telect.sync _|q, 0xFFFFFFFF;\n\t"
+      "@q cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n\t}" ::"r"(dst),
+      "l"(src), "r"(bytes), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void elect_tile_3d(uint32_t dst, const CUtensorMap* tmap, int x, int y, int z, uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\telect.sync _|q, 0xFFFFFFFF;\n\t"
+      "@q cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];\n\t}" ::"r"(dst),
+      "l"(tmap), "r"(x), "r"(y), "r"(z), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void elect_tile_4d(uint32_t dst, const CUtensorMap* tmap, int x, int y, int z, int w, uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\telect.sync _|q, 0xFFFFFFFF;\n\t"
+      "@q cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];\n\t}" ::"r"(dst),
+      "l"(tmap), "r"(x), "r"(y), "r"(z), "r"(w), "r"(bar)
+      : "memory");
 }
 
 }  // namespace

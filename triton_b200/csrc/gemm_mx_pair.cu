@@ -6,21 +6,26 @@
 // e4m3 / MXFP8 tokens are one term.  Nothing is dequantised in software, and the MMA pipe does K = 32 per instruction in the
 // time kind::f16 does K = 16 (measured: 4.4 PFLOP/s for N >= 128 on 148 SMs, so two terms run at 2.2 -- the bf16 rate).
 //
+// (Elements far below their group of 32's largest lose what lies below 2^-23 of it, as much as an fp32 sum rounds away.)
+//
 // What bounds it.  An SM takes in at most about 26 B per cycle from L2, and the MMA of a 128-k step is 64 cycles per 128
 // token columns, weight block and K = 32: the tile has to be large.  A cluster of two CTAs computes (2 x 256 weight rows) x
-// (up to 224 tokens; 192 with two terms): the weights are the M operand (every CTA loads its own 128 rows of each of the
-// two 256-row blocks, packed in global memory: 16 KB per step), the tokens the N operand (every CTA loads half of them:
-// 14 or 24 KB), 26-34 B per MMA cycle.  Tokens on N also make a ragged tail cost what it holds, in steps of 32 rows, where
-// tokens on M padded every expert to a multiple of 128 or 256 (31 % of the rows of a skewed 128-expert batch of 16384
-// tokens).
+// (up to 192 tokens): the weights are the M operand (every CTA loads its own 128 rows of each of the two 256-row blocks,
+// packed in global memory: 16 KB per step), the tokens the N operand (every CTA loads half of them: 12 or 24 KB), 26-34 B per
+// MMA cycle.  Tokens on N also make a ragged tail cost what it holds, in steps of 32 rows, where tokens on M padded every
+// expert to a multiple of 128 or 256 (31 % of the rows of a skewed 128-expert batch of 16384 tokens).  With few rows per
+// expert it is the packed weights: 128 experts of 2880 x 5760, 300 tokens, 1.1 GB in 189 us.
 //
-// A tile's accumulator is two units (its 256-row weight blocks), and each is handed to the epilogue and back by itself: the
-// next tile starts on the unit that is drained while the other still is (the MMA warp lets a unit lag by at most the stages
-// of the ring).  One accumulator of 448 columns drained as a whole would leave the tensor pipe idle for the time of an
-// epilogue on every tile; two buffers of it do not fit tensor memory.  (Four units, halves of the columns each, drain in
-// finer steps but read the weight operand twice: 59 cycles for an MMA of 96 columns against 96 for one of 192.)
+// A k step of a small tile is eight MMAs of 64 cycles, so what the issuing warp does around them counts: operands in uniform
+// registers, the election inside the instruction's own asm block (with a leader flag kept in a register a step took 1150 cycles, so
+// 900), the next step's barrier asked for ahead.
 //
-// Warps of a CTA: 0 producer (one thread), 1 MMA issue (even CTA) and tensor-memory owner, 4-7 scale loaders (shared memory ->
+// The accumulators of a tile's 256-row blocks are regions of a ring in tensor memory; each is handed to the epilogue and back by
+// itself: the next tile starts in regions that are drained while others still are (the MMA warp lets a block lag by at most
+// the stages of the operand ring).  One accumulator of all columns drained as a whole would leave the tensor pipe idle for the
+// time of an epilogue on every tile.
+//
+// Warps of a CTA: 0 producer, 1 MMA issue (even CTA) and tensor-memory owner, 4-7 scale loaders (shared memory ->
 // registers -> tensor memory; the token scales of all columns in both CTAs, the weight scales of the own rows), 8-19 epilogue.
 // Every wait is bounded; both CTAs meet at a cluster barrier before tensor memory is freed.
 #include "gemm_mx_common.cuh"
@@ -35,34 +40,36 @@ constexpr int REGS_ISSUE = 56, REGS_SF = 64, REGS_EPI = 120;
 static_assert(128 * (REGS_ISSUE + REGS_SF) + PP_EPI_WARPS * 32 * REGS_EPI <= 96 * 640, "register split");
 constexpr int PP_THREADS = (PP_EPI_WARP0 + PP_EPI_WARPS) * 32;
 
-template <int TERMS> struct PCfg {
-  static constexpr int NMAX = TERMS == 1 ? 224 : 192;        // token columns of a tile
-  static constexpr int STAGES = TERMS == 1 ? 4 : 3;
-  static constexpr int X_TERM = NMAX / 2 * 128;              // bytes of a CTA's half of the tokens, one term
-  static constexpr int OFF_X = 2 * 128 * 128;                // two weight blocks, byte per element
-  static constexpr int OFF_WS = OFF_X + TERMS * X_TERM;      // their scales
-  static constexpr int OFF_XS = OFF_WS + 1024;               // token scales of all columns (256 words per term)
-  static constexpr int STAGE = OFF_XS + TERMS * 1024;
-  static constexpr int SF_BASE = 2 * NMAX, SF_COLS = 8 + 8 * TERMS;
-  static constexpr int TAB = 256 * 16;                       // token table of a tile: row address [256], gamma [256], beta [256]
-  static constexpr int OFF_TAB = STAGES * STAGE;             // two of them
-  static constexpr int OFF_BAR = OFF_TAB + 2 * TAB;
-  static constexpr int NUM_BARS = 3 * STAGES + 4 + 1;
-  static constexpr int EPI_CHUNKS = (NMAX / 16 + 2) / 3;      //  16-token chunks of a unit per epilogue warp (three warps share a lane quarter)
-  static constexpr int OFF_MISC = OFF_BAR + NUM_BARS * 8 + (NUM_BARS % 2) * 8;
-  static constexpr int OFF_COLS = OFF_MISC + 16;             // columns of the next tiles, for the MMA warp
-  static constexpr int OFF_PREFIX = OFF_COLS + 8 * 4;        // int32 tile prefix over experts, their row counts and offsets
-  static constexpr int ALLOC = OFF_PREFIX + (3 * MAX_PREFIX_EXPERTS + 1) * 4 + 1024;
-  static_assert(STAGE % 1024 == 0 && X_TERM % 1024 == 0, "operand tiles start on swizzle atoms");
-  static_assert(SF_BASE + STAGES * SF_COLS <= TMEM_COLS && ALLOC <= 232448, "budgets");
-};
+constexpr int PP_MAX_STAGES = 6, PP_MAX_REGIONS = 12;
+constexpr int PP_NUM_BARS = 3 * PP_MAX_STAGES + 2 * PP_MAX_REGIONS + 1;
+// shared memory behind the stages: [token tables x 2][barriers][tensor-memory base, abort flag][columns of the next tiles][prefix]
+constexpr int PP_OFF_BAR = 2 * PAIR_TAB, PP_OFF_MISC = PP_OFF_BAR + (PP_NUM_BARS * 8 + 15) / 16 * 16, PP_OFF_COLS = PP_OFF_MISC + 16,
+              PP_OFF_PREFIX = PP_OFF_COLS + 8 * 4, PP_CTL = (PP_OFF_PREFIX + PAIR_PREFIX_INTS * 4 + 15) / 16 * 16;
+constexpr int PP_SMEM = 227 * 1024;
+// How tokens enter the MMA.  ONE: e4m3 rows, one term.  TWO: two terms, two MMAs into the same columns.  SIDE: the terms as
+// neighbouring columns of one MMA (eight hi, eight lo, ...), added in the epilogue.  An MMA takes 45-59 cycles however few
+// columns it has: with up to 96 tokens a tile SIDE issues half of them (32 tokens: 45 cycles per 32 k of a weight block
+// against 118).
+enum { PP_ONE = 1, PP_TWO = 2, PP_SIDE = 3 };
+template <int FORM> constexpr int TERMS_OF = FORM == PP_ONE ? 1 : 2;
+template <int FORM> constexpr int SF_COLS = FORM == PP_TWO ? 24 : 16;      // tensor-memory columns of scales per stage: 8 of two blocks, 8 per MMA of a k group
 
 struct PairParams {
-  const uint8_t* xq;            // [term][k step][padded row][128 B], 16-byte pieces swizzled with (row & 7)
-  const uint8_t* xs;            // [term][k step][padded row][4 B]: e8m0 of the four 32-groups
+  const uint8_t* xq;            // [k step][padded row / 8][term][8 rows][128 B], 16-byte pieces swizzled with (row & 7)
+  const uint8_t* xs;            // [k step][padded row / 8][term][8 rows][4 B]: e8m0 of the four 32-groups
   int64_t prows;                // padded rows: expert e's rows start at (slice_offs[e] & ~31) + 32 e
   int KT, NB;                   // 128-k steps, 128-row weight blocks
+  int nmax;                     // token columns of a tile at most, a multiple of 32
+  int upt;                      // weight blocks of 256 rows per tile: 1 or 2
+  int stages, stage_bytes, regions, reg_cols;      // accumulator regions of reg_cols tensor-memory columns
 };
+
+struct PairMaps { CUtensorMap w[2], s[2]; };        // weight tiles and their scales in boxes of one and two blocks
+
+// line (128 bytes of values, 4 of scales) of a token's term
+template <int TERMS> __device__ __forceinline__ int64_t token_line(int64_t kt, int64_t prows, int64_t prow, int term) {
+  return TERMS * (kt * prows + (prow & ~(int64_t)7)) + term * 8 + (prow & 7);
+}
 
 // first padded row of an expert: a multiple of 32, and never before the end of the previous expert's last group of 32
 __device__ __forceinline__ int64_t padded_base(int e, int off) { return (int64_t)(off & ~31) + 32 * (int64_t)e; }
@@ -103,11 +110,12 @@ __device__ __forceinline__ float amax4(float a) {          // maximum over the f
   return fmaxf(a, __shfl_xor_sync(0xFFFFFFFFu, a, 2));
 }
 
+// TILED: k inside eight in the order of the default weight tiles (0, 2, 4, 6, 1, 3, 5, 7)
+template <bool TILED>
 __global__ void __launch_bounds__(256) mx_pair_pack2_kernel(const GemmParams p, const PairPackParams a) {
   int e; int64_t row0, prow0; int rows;
   if (!pack_block(p, blockIdx.x, e, row0, rows, prow0)) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t q_term = (int64_t)a.KT * a.prows * 128, s_term = (int64_t)a.KT * a.prows * 4;
   const int K128 = a.KT * 128;
   for (int r = warp; r < rows; r += 8) {
     int64_t src = a.gather ? (int64_t)a.gather[row0 + r] : row0 + r;
@@ -135,8 +143,18 @@ __global__ void __launch_bounds__(256) mx_pair_pack2_kernel(const GemmParams p, 
           v[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
           m = fmaxf(m, fmaxf(fabsf(v[2 * i]), fabsf(v[2 * i + 1])));
         }
+        if constexpr (TILED) {
+          const float o[8] = {v[0], v[2], v[4], v[6], v[1], v[3], v[5], v[7]};
+#pragma unroll
+          for (int i = 0; i < 8; ++i) v[i] = o[i];
+        }
         m = amax4(m);
-        if (!(m < 3.0e38f)) m = 3.0e38f;                           // Inf / NaN in the group: keep the scale finite
+        if (!(m < 3.0e38f)) {                                      // Inf / NaN in the group: keep the scale finite; e4m3 has no Inf,
+          m = 3.0e38f;                                             // a NaN makes the row's results NaN
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            if (!(fabsf(v[i]) < 3.4e38f)) v[i] = __uint_as_float(0x7FC00000u);
+        }
         uint32_t sh; float s_hi, i_hi;
         mx8_scale(m, sh, s_hi, i_hi);
         uint32_t h[4], l[4];
@@ -156,14 +174,14 @@ __global__ void __launch_bounds__(256) mx_pair_pack2_kernel(const GemmParams p, 
 #pragma unroll
         for (int i = 0; i < 4; ++i) l[i] = f32x2_to_e4m3x2(v[2 * i] * i_lo, v[2 * i + 1] * i_lo);
         if (k < K128) {
-          const int64_t line = (int64_t)(k >> 7) * a.prows + prow;
+          const int64_t line = token_line<2>(k >> 7, a.prows, prow, 0);
           uint8_t* dst = a.xq + line * 128 + ((((uint32_t)(k & 127) >> 4) ^ x7) << 4) + (k & 8);
           *reinterpret_cast<uint2*>(dst) = make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16));
-          *reinterpret_cast<uint2*>(dst + q_term) = make_uint2(l[0] | (l[1] << 16), l[2] | (l[3] << 16));
+          *reinterpret_cast<uint2*>(dst + 1024) = make_uint2(l[0] | (l[1] << 16), l[2] | (l[3] << 16));
           if ((lane & 3) == 0) {
             uint8_t* sd = a.xs + line * 4 + ((k >> 5) & 3);
             sd[0] = (uint8_t)sh;
-            sd[s_term] = (uint8_t)sl;
+            sd[32] = (uint8_t)sl;
           }
         }
       }
@@ -212,122 +230,84 @@ __global__ void __launch_bounds__(256) mx_pair_pack1_kernel(const GemmParams p, 
 // ============================================================================================================
 // The GEMM kernel
 // ============================================================================================================
-// The whole MMA warp runs the issue loop and one lane's predicate guards the instruction.  The operands of tcgen05.mma live in
-// uniform registers: computed by a single thread of a divergent branch, each takes a move from a vector register first, and
-// an MMA cost 170-190 cycles to issue.  Of a shared-memory descriptor only the low word varies (start address, 16-byte units).
-constexpr uint32_t DESC_LO = 1u << 16;                               // leading byte offset (unused for swizzled K-major)
-constexpr uint32_t DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29); // 8-row groups 1024 B apart, sm_100, 128-byte swizzle
+// A_HI, B_HI: high words of the descriptors (swizzle, distance of 8-row groups)
+template <uint32_t A_HI, uint32_t B_HI>
 __device__ __forceinline__ void mma_mxf8f6f4_pair(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t sfa,
-                                                  uint32_t sfb, uint32_t accumulate, uint32_t leader) {
+                                                  uint32_t sfb, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"
-      "mov.b64 da, {%1, %8};\n\t"
+      "mov.b64 da, {%1, %7};\n\t"
       "mov.b64 db, {%2, %8};\n\t"
       "setp.ne.b32 p, %6, 0;\n\t"
-      "setp.ne.b32 q, %7, 0;\n\t"
+      "elect.sync _|q, 0xFFFFFFFF;\n\t"
       "@q tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale.scale_vec::1X [%0], da, db, %3, [%4], [%5], p;\n\t}" ::"r"(d_tmem),
-      "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate), "r"(leader), "n"(DESC_HI)
+      "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate), "n"(A_HI), "n"(B_HI)
       : "memory");
 }
+// Weights in the default tiles ([group of 32 k][128 rows][16 B], see layout.cu).  The TMA unit reads 64 bytes = four rows of
+// one group per 128-byte line and swizzles 16-byte pieces with the line (address bits 4-6 ^= bits 7-9).  Read as rows of 32
+// bytes with the 32-byte swizzle (bit 4 ^= bit 7) those lines are one K = 32 operand of 128 rows in which row r sits at
+// r ^ ((r >> 3) & 3): the other two swizzled bits are row bits.  The order of k inside eight (even, then odd) is taken up by the
+// token pack kernel.  So the tiles of the bf16 kernels feed the block-scaled MMA as they are stored.
+constexpr uint32_t DESC_HI_SW32 = (256u >> 4) | (1u << 14) | (6u << 29);      // 8-row groups 256 B apart, 32-byte swizzle
+__device__ __forceinline__ int tiled_row(int pos) { return pos ^ ((pos >> 3) & 3); }       // its own inverse
 // A = e2m1 (code 5), B = e4m3 (code 0), both K-major, e8m0 scales, M = 256 over the two CTAs; sf: byte of the scale words
 __device__ __forceinline__ uint32_t pair_idesc(int n, uint32_t sf) {
   return (sf << 4) | (5u << 7) | ((uint32_t)(n >> 3) << 17) | (1u << 23) | (2u << 27) | (sf << 29);
 }
 
-// Token tile tt: rows of one expert, in groups of 32 dealt evenly over the expert's tiles (a tail of a few rows does not
-// become a tile of its own).
-struct PTile { int e, rows, cols; int64_t row0, prow0; };
-template <int NMAX> __device__ __forceinline__ PTile map_ptile(const GemmParams& p, const int32_t* prefix, int tt) {
-  PTile t;
-  int lo = 0, hi = p.slice_sizes ? p.E : 1;                          // largest e with prefix[e] <= tt
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (prefix[mid] <= tt) lo = mid; else hi = mid;
-  }
-  const int size = prefix[MAX_PREFIX_EXPERTS + 1 + lo], off = prefix[2 * MAX_PREFIX_EXPERTS + 1 + lo];
-  const int nt = prefix[lo + 1] - prefix[lo], j = tt - prefix[lo];
-  const int64_t q = (size + 31) >> 5;
-  const int u0 = (int)(j * q / nt), u1 = (int)((j + 1) * q / nt);
-  t.e = lo;
-  t.row0 = (int64_t)off + 32 * u0;
-  t.prow0 = padded_base(lo, off) + 32 * u0;
-  t.cols = 32 * (u1 - u0);
-  t.rows = min(t.cols, size - 32 * u0);
-  return t;
-}
-
-// two fp32 operations in one instruction
-__device__ __forceinline__ void add_f32x2(float& o0, float& o1, float a0, float a1, float b0, float b1) {
-  asm("{\n\t.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tadd.rn.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;\n\t}"
-      : "=f"(o0), "=f"(o1) : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
-}
-__device__ __forceinline__ void mul_f32x2(float& o0, float& o1, float a0, float a1, float b0, float b1) {
-  asm("{\n\t.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmul.rn.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;\n\t}"
-      : "=f"(o0), "=f"(o1) : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
-}
-
-template <typename TY, int TERMS>
+// TILED: weights in the default tiles [E][n_tile][k_tile], else in the block-scaled ones [E][k_tile][n_block]
+template <typename TY, int FORM, bool TILED>
 __global__ void __launch_bounds__(PP_THREADS, 1)
-gemm_mx_pair_kernel(const GemmParams p, const PairParams a, const __grid_constant__ CUtensorMap w_map) {
-  using C = PCfg<TERMS>;
-  constexpr int STAGES = C::STAGES;
+gemm_mx_pair_kernel(const GemmParams p, const PairParams a, const __grid_constant__ PairMaps maps) {
+  constexpr int TERMS = TERMS_OF<FORM>, MMAS = FORM == PP_TWO ? 2 : 1;
+  constexpr uint32_t B_HI = FORM == PP_TWO ? (2048u >> 4) | (DESC_HI & 0xFFFFC000u) : DESC_HI;      // TWO: 8 hi rows, 8 lo rows, ...
+  constexpr uint32_t A_HI = TILED ? DESC_HI_SW32 : DESC_HI, A_KK = TILED ? 4096 >> 4 : 2;      // next 32 k of A: 16-byte units
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const uint32_t sbase = smem_u32(smem);
   const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;     // warp-uniform for the compiler
   const uint32_t rank = cluster_ctarank();
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
-  const uint32_t bar0 = sbase + C::OFF_BAR;
+  const int STAGES = a.stages, UPT = a.upt;
+  // stage: [UPT x 16 KB weights, byte per element][TERMS x nmax / 2 token rows x 128 B][weight scales][token scales of all columns:
+  // TERMS x 256 words]
+  const uint32_t OFF_X = (uint32_t)UPT * (128 * 128), OFF_WS = OFF_X + TERMS * (uint32_t)a.nmax * 64u, OFF_XS = OFF_WS + 1024u;
+  const uint32_t SF_BASE = (uint32_t)(TMEM_COLS - STAGES * SF_COLS<FORM>);
+  uint8_t* ctl_ptr = smem + (size_t)STAGES * a.stage_bytes;
+  const uint32_t ctl0 = smem_u32(ctl_ptr), bar0 = ctl0 + PP_OFF_BAR;
   auto BAR_FULL = [&](int s) { return bar0 + 8u * (uint32_t)s; };                       // own copies have landed
-  auto BAR_EMPTY = [&](int s) { return bar0 + 8u * (uint32_t)(STAGES + s); };
-  auto BAR_SF = [&](int s) { return bar0 + 8u * (uint32_t)(2 * STAGES + s); };           // even CTA: scales (and operands) of both CTAs
-  auto BAR_ACC_FULL = [&](int u) { return bar0 + 8u * (uint32_t)(3 * STAGES + u); };
-  auto BAR_ACC_EMPTY = [&](int u) { return bar0 + 8u * (uint32_t)(3 * STAGES + 2 + u); };   // even CTA
-  const uint32_t BAR_DRAIN = bar0 + 8u * (uint32_t)(3 * STAGES + 4);
-  volatile uint32_t* s_tmem = reinterpret_cast<volatile uint32_t*>(smem + C::OFF_MISC);
-  volatile int* s_abort = reinterpret_cast<volatile int*>(smem + C::OFF_MISC + 4);
-  volatile int* s_cols = reinterpret_cast<volatile int*>(smem + C::OFF_COLS);
-  int32_t* s_prefix = reinterpret_cast<int32_t*>(smem + C::OFF_PREFIX);
+  auto BAR_EMPTY = [&](int s) { return bar0 + 8u * (uint32_t)(PP_MAX_STAGES + s); };
+  auto BAR_SF = [&](int s) { return bar0 + 8u * (uint32_t)(2 * PP_MAX_STAGES + s); };    // even CTA: scales (and operands) of both CTAs
+  auto BAR_ACC_FULL = [&](int r) { return bar0 + 8u * (uint32_t)(3 * PP_MAX_STAGES + r); };
+  auto BAR_ACC_EMPTY = [&](int r) { return bar0 + 8u * (uint32_t)(3 * PP_MAX_STAGES + PP_MAX_REGIONS + r); };   // even CTA
+  const uint32_t BAR_DRAIN = bar0 + 8u * (uint32_t)(PP_NUM_BARS - 1);
+  volatile uint32_t* s_tmem = reinterpret_cast<volatile uint32_t*>(ctl_ptr + PP_OFF_MISC);
+  volatile int* s_abort = reinterpret_cast<volatile int*>(ctl_ptr + PP_OFF_MISC + 4);
+  volatile int* s_cols = reinterpret_cast<volatile int*>(ctl_ptr + PP_OFF_COLS);
+  int32_t* s_prefix = reinterpret_cast<int32_t*>(ctl_ptr + PP_OFF_PREFIX);
   Ctl ctl{s_abort, p.status};
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
+    for (int s = 0; s < PP_MAX_STAGES; ++s) {
       mbar_init(BAR_FULL(s), 1);
       mbar_init(BAR_EMPTY(s), 1);
       mbar_init(BAR_SF(s), 8);                         // four scale warps in each CTA
     }
-    for (int u = 0; u < 2; ++u) {
-      mbar_init(BAR_ACC_FULL(u), 1);
-      mbar_init(BAR_ACC_EMPTY(u), 2 * PP_EPI_WARPS);
+    for (int r = 0; r < PP_MAX_REGIONS; ++r) {
+      mbar_init(BAR_ACC_FULL(r), 1);
+      mbar_init(BAR_ACC_EMPTY(r), 2 * PP_EPI_WARPS);
     }
     mbar_init(BAR_DRAIN, 1);
     *s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sbase + C::OFF_MISC), "r"((uint32_t)TMEM_COLS) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(ctl0 + PP_OFF_MISC), "r"((uint32_t)TMEM_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   if (warp == PP_SF_WARP0) {                           // tile prefix over experts
-    const int n = p.slice_sizes ? p.E : 1;
-    int run = 0;
-    for (int e0 = 0; e0 < n; e0 += 32) {
-      const int e = e0 + lane;
-      const int size = e < n ? max(p.slice_sizes ? p.slice_sizes[e] : (int)p.M, 0) : 0;
-      int v = (size + C::NMAX - 1) / C::NMAX;
-      if (e < n) {
-        s_prefix[MAX_PREFIX_EXPERTS + 1 + e] = size;
-        s_prefix[2 * MAX_PREFIX_EXPERTS + 1 + e] = p.slice_sizes ? p.slice_offs[e] : 0;
-      }
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(0xFFFFFFFFu, v, o);
-        if (lane >= o) v += t;
-      }
-      if (e < n) s_prefix[e + 1] = run + v;
-      run += __shfl_sync(0xFFFFFFFFu, v, 31);
-    }
-    if (lane == 0) s_prefix[0] = 0;
+    pair_prefix(p, s_prefix, a.nmax, lane);
   }
   tc_fence_before();
   __syncthreads();
@@ -336,152 +316,167 @@ gemm_mx_pair_kernel(const GemmParams p, const PairParams a, const __grid_constan
   const uint32_t tmem_base = __shfl_sync(0xFFFFFFFFu, *s_tmem, 0);
 
   const int KT = a.KT, NB = a.NB;
-  const int MB = (NB + 1) >> 1, MT = (MB + 1) >> 1;     // 256-row weight blocks, tiles of two of them
+  const int MB = (NB + 1) >> 1, MT = (MB + UPT - 1) / UPT;      // 256-row weight blocks, tiles of UPT of them
+  // The blocks of a tile: CTA r takes the neighbouring blocks 4 t + 2 r and + 1 (one copy each stage), a block of the MMA is one
+  // block of either CTA; with at most two blocks left (or UPT = 1), block + r.  -> own first block, own blocks, MMA blocks.
+  struct Blocks { int first, own, units; };
+  auto blocks_of = [&](int tile) {
+    const int b0 = (tile % MT) * UPT * 2, left = NB - b0;
+    Blocks b;
+    const bool wide = UPT == 2 && left > 2;
+    b.first = b0 + (wide ? 2 : 1) * (int)rank;
+    b.own = wide ? min(2, max(0, NB - b.first)) : (int)((int)rank < left);
+    b.units = wide ? 2 : 1;
+    return b;
+  };
   const int n_tiles = __shfl_sync(0xFFFFFFFFu, s_prefix[p.slice_sizes ? p.E : 1], 0) * MT;
 
   if (warp < PP_SF_WARP0) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_ISSUE));
   if (warp == 0) {
     // ================================= producer =======================================================
-    if (lane == 0) {
-      uint32_t it = 0;
-      bool ok = true;
-      PTile t, nxt;                                    // the next tile is looked up while this one streams
-      if (pair < n_tiles) nxt = map_ptile<C::NMAX>(p, s_prefix, pair / MT);
-      for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
-        t = nxt;
-        const int blk0 = (tile % MT) * 4 + (int)rank;                 // own block of the first 256-row block; the second's is + 2
-        const int n_w = (blk0 < NB) + (blk0 + 2 < NB);                // (an absent block's stage keeps stale data)
-        const uint32_t bx = (uint32_t)t.cols * 64u, bs = (uint32_t)t.cols * 4u;       // own half of the rows, all scales
-        const uint32_t tx = (uint32_t)n_w * (128 * 64 + 512) + TERMS * (bx + bs);
-        for (int kt = 0; kt < KT; ++kt, ++it) {
-          const int s = it % STAGES;
-          ok = mbar_wait(BAR_EMPTY(s), ((it / STAGES) & 1u) ^ 1u, ctl, 611);
-          if (!ok) break;
-          const uint32_t st = sbase + (uint32_t)s * C::STAGE;
-          mbar_expect_tx(BAR_FULL(s), tx);
-          const int64_t wt = ((int64_t)t.e * KT + kt) * NB + blk0;
-#pragma unroll
-          for (int m = 0; m < 2; ++m)
-            if (m < n_w) {
-              tma_tile_3d(st + m * 128 * 128, &w_map, 0, 0, (int)(wt + 2 * m), BAR_FULL(s));
-              bulk_g2s(st + C::OFF_WS + m * 512, p.w_scale + (wt + 2 * m) * 512, 512u, BAR_FULL(s));
-            }
-#pragma unroll
-          for (int c = 0; c < TERMS; ++c) {
-            const int64_t line = ((int64_t)c * KT + kt) * a.prows + t.prow0;
-            bulk_g2s(st + C::OFF_X + c * C::X_TERM, a.xq + line * 128 + rank * bx, bx, BAR_FULL(s));
-            bulk_g2s(st + C::OFF_XS + c * 1024, a.xs + line * 4, bs, BAR_FULL(s));
-          }
-          if (kt == 0 && tile + n_pairs < n_tiles) nxt = map_ptile<C::NMAX>(p, s_prefix, (tile + n_pairs) / MT);
+    uint32_t s = 0, ph = 1, issued = 0;
+    bool ok = true;
+    PTile nxt;                                         // the next tile is looked up while this one streams
+    if (pair < n_tiles) nxt = map_ptile(p, s_prefix, pair / MT);
+    for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
+      const int e = __shfl_sync(0xFFFFFFFFu, nxt.e, 0), cols = __shfl_sync(0xFFFFFFFFu, nxt.cols, 0);
+      const int prow0 = __shfl_sync(0xFFFFFFFFu, (int)padded_base(nxt.e, nxt.off) + nxt.first, 0);
+      const Blocks b = blocks_of(tile);
+      const uint32_t bx = (uint32_t)(TERMS * cols) * 64u, bs = (uint32_t)(TERMS * cols) * 4u;        // own half of the rows, all scales
+      const uint32_t tx = (uint32_t)b.own * (128 * 64 + 512) + bx + bs;
+      const CUtensorMap* wm = &maps.w[b.own == 2];
+      const CUtensorMap* sm = &maps.s[b.own == 2];
+      const uint8_t* xq = a.xq + TERMS * ((int64_t)prow0 * 128) + rank * bx;
+      const uint8_t* xs = a.xs + TERMS * ((int64_t)prow0 * 4);
+      const int64_t q_step = TERMS * a.prows * 128, s_step = TERMS * a.prows * 4;
+      int c2 = TILED ? 0 : b.first, c3 = TILED ? e * NB + b.first : e * KT;
+      for (int kt = 0; kt < KT; ++kt, ++issued) {
+        ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_EMPTY(s), ph, ctl, 611));
+        if (!ok) break;
+        const uint32_t st = sbase + s * (uint32_t)a.stage_bytes, bar = BAR_FULL(s);
+        elect_expect_tx(bar, tx);
+        if (b.own > 0) {
+          elect_tile_4d(st, wm, 0, 0, c2, c3, bar);
+          elect_tile_3d(st + OFF_WS, sm, 0, c2, c3, bar);
         }
+        elect_bulk_g2s(st + OFF_X, xq, bx, bar);
+        elect_bulk_g2s(st + OFF_XS, xs, bs, bar);
+        xq += q_step; xs += s_step;
+        if (TILED) ++c2; else ++c3;
+        if (++s == (uint32_t)STAGES) { s = 0; ph ^= 1u; }
+        if (kt == 0 && tile + n_pairs < n_tiles) nxt = map_ptile(p, s_prefix, (tile + n_pairs) / MT);
       }
-      if (!ok) {
-        // aborting: let the copies that were already issued land before the CTA leaves
-        const uint32_t lo = it > (uint32_t)STAGES ? it - STAGES : 0;
-        for (uint32_t j = lo; j < it; ++j)
-          for (uint32_t i = 0; i < (1u << 16) && !mbar_test(BAR_FULL(j % STAGES), (j / STAGES) & 1u); ++i) __nanosleep(64);
-      }
+    }
+    if (!ok && lane == 0) {
+      // aborting: let the copies that were already issued land before the CTA leaves
+      for (uint32_t j = issued > (uint32_t)STAGES ? issued - STAGES : 0; j < issued; ++j)
+        for (uint32_t i = 0; i < (1u << 16) && !mbar_test(BAR_FULL(j % STAGES), (j / STAGES) & 1u); ++i) __nanosleep(64);
     }
     __syncwarp();
   } else if (warp == 1) {
     // ================================= MMA issuer (even CTA) ==========================================
     if (rank == 0) {
-      const uint32_t leader = elect_one();
       const int k_whole = p.K >> 7;                    // steps of 128 k; the last may hold less
       uint32_t s = 0, ph = 0;                          // stage and parity of the next k step
-      uint32_t acc_ph = 3u;                          // parity to wait for, per unit
-      uint32_t tc = 0;
+      uint32_t acc_ph = 0xFFFFu;                       // parity to wait for, per region
+      uint32_t r0 = 0, tc = 0;                         // region of the tile's first block
       bool ok = true;
       for (int tile = pair; tile < n_tiles && ok; tile += n_pairs, ++tc) {
-        ok = __all_sync(0xFFFFFFFFu, mbar_wait_cluster(BAR_SF(s), ph, ctl, 612));         // first k step; the scale loader left the columns
+        ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_SF(s), ph, ctl, 612));         // first k step; the scale loader left the columns
         if (!ok) break;
-        const uint32_t id0 = pair_idesc(__shfl_sync(0xFFFFFFFFu, s_cols[tc & 7u], 0), 0);
-        const uint32_t live = (tile % MT) * 2 + 1 < MB ? 3u : 1u;      // units of the tile: 256-row weight blocks
-        auto issue = [&](int u, int k, uint32_t s) {   // k step `k` of unit u, operands in stage s
-          const uint32_t st = sbase + s * C::STAGE;
-          const uint32_t sf = tmem_base + C::SF_BASE + s * C::SF_COLS;
+        const uint32_t id0 = pair_idesc(__shfl_sync(0xFFFFFFFFu, s_cols[tc & 7u], 0) * (FORM == PP_SIDE ? 2 : 1), 0);
+        const uint32_t live = blocks_of(tile).units == 2 ? 3u : 1u;
+        const uint32_t reg[2] = {r0, r0 + 1 < (uint32_t)a.regions ? r0 + 1 : 0u};
+        auto issue = [&](int u, int k, uint32_t s) {   // k step `k` of block u, operands in stage s
+          const uint32_t st = sbase + s * (uint32_t)a.stage_bytes;
+          const uint32_t sf = tmem_base + SF_BASE + s * SF_COLS<FORM>;
           const uint32_t a_lo = DESC_LO | ((st + (uint32_t)u * (128 * 128)) >> 4);
-          const uint32_t b_lo = DESC_LO | ((st + C::OFF_X) >> 4);
-          const uint32_t d = tmem_base + (uint32_t)(u * C::NMAX);
+          const uint32_t b_lo = DESC_LO | ((st + OFF_X) >> 4);
+          const uint32_t d = tmem_base + reg[u] * (uint32_t)a.reg_cols;
           // (a step that is whole has no test between its instructions: they must issue in less than the 45-64 cycles that
           // one of them runs)
           if (k < k_whole) {
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk)
 #pragma unroll
-              for (int c = 0; c < TERMS; ++c)
-                mma_mxf8f6f4_pair(d, a_lo + kk * 2, b_lo + c * (C::X_TERM >> 4) + kk * 2, id0 + ((uint32_t)kk << 4) + ((uint32_t)kk << 29),
-                                  sf + 4 * u, sf + 8 + 8 * c, (kk | c) ? 1u : (uint32_t)(k > 0), leader);
+              for (int c = 0; c < MMAS; ++c)
+                mma_mxf8f6f4_pair<A_HI, B_HI>(d, a_lo + kk * A_KK, b_lo + c * (1024 >> 4) + kk * 2, id0 + ((uint32_t)kk << 4) + ((uint32_t)kk << 29),
+                                        sf + 4 * u, sf + 8 + 8 * c, (kk | c) ? 1u : (uint32_t)(k > 0));
           } else {
             const int kk_live = (p.K - k * 128 + 31) >> 5;
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk)
               if (kk < kk_live) {
 #pragma unroll
-                for (int c = 0; c < TERMS; ++c)
-                  mma_mxf8f6f4_pair(d, a_lo + kk * 2, b_lo + c * (C::X_TERM >> 4) + kk * 2, id0 + ((uint32_t)kk << 4) + ((uint32_t)kk << 29),
-                                    sf + 4 * u, sf + 8 + 8 * c, (k | kk | c) ? 1u : 0u, leader);
+                for (int c = 0; c < MMAS; ++c)
+                  mma_mxf8f6f4_pair<A_HI, B_HI>(d, a_lo + kk * A_KK, b_lo + c * (1024 >> 4) + kk * 2, id0 + ((uint32_t)kk << 4) + ((uint32_t)kk << 29),
+                                          sf + 4 * u, sf + 8 + 8 * c, (k | kk | c) ? 1u : 0u);
               }
           }
         };
-        // ---- ramp: units join as the epilogue hands them back; those that have joined run ahead by up to the ring ------
+        // ---- ramp: blocks join as the epilogue hands back their regions; those that have joined run ahead by up to the ring ----
         uint32_t joined = 0;
-        int kt = 0, base = 0;                          // next k step of the joined units, of the others
-        uint32_t s_base = s;
+        int kt = 0;                                    // next k step of the joined blocks; the others have issued none
+        const uint32_t s_base = s;
         while (ok && (joined != live || kt == 0)) {
-          if (kt - base < STAGES && kt < KT) {
-            ok = __all_sync(0xFFFFFFFFu, mbar_wait_cluster(BAR_SF(s), ph, ctl, 612));
+          if (joined && kt < STAGES && kt < KT) {
+            ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_SF(s), ph, ctl, 612));
             if (!ok) break;
             tc_fence_after();
 #pragma unroll
             for (int u = 0; u < 2; ++u)
               if ((joined >> u) & 1u) issue(u, kt, s);
+            if (joined == live) elect_commit_pair(BAR_EMPTY(s));
             ++kt;
-            if (++s == STAGES) { s = 0; ph ^= 1u; }
+            if (++s == (uint32_t)STAGES) { s = 0; ph ^= 1u; }
           }
-          const bool full = kt - base >= STAGES || kt >= KT;           // nothing to do for the joined units: wait for the next one
+          const bool full = kt >= STAGES || kt >= KT;  // nothing to do for the joined blocks: wait for the next one
 #pragma unroll
           for (int u = 0; u < 2; ++u) {
             if (!((live >> u) & 1u) || ((joined >> u) & 1u)) continue;
-            const uint32_t par = (acc_ph >> u) & 1u;
+            const uint32_t par = (acc_ph >> reg[u]) & 1u;
             bool got;
-            if (full || joined == 0) got = ok = __all_sync(0xFFFFFFFFu, mbar_wait_cluster(BAR_ACC_EMPTY(u), par, ctl, 613));
-            else got = __all_sync(0xFFFFFFFFu, mbar_test(BAR_ACC_EMPTY(u), par));                  // (try_wait would sleep)
+            if (full || joined == 0) got = ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_ACC_EMPTY(reg[u]), par, ctl, 613));
+            else got = __all_sync(0xFFFFFFFFu, mbar_test(BAR_ACC_EMPTY(reg[u]), par));             // (try_wait would sleep)
             if (!got) break;
             tc_fence_after();
             joined |= 1u << u;
-            acc_ph ^= 1u << u;
+            acc_ph ^= 1u << reg[u];
             uint32_t sk = s_base;
-            for (int k = base; k < kt; ++k) {                          // catch up with the others
+            for (int k = 0; k < kt; ++k) {             // catch up with the others
               issue(u, k, sk);
-              if (joined == live) mma_commit_pair(BAR_EMPTY(sk), leader);
-              if (++sk == STAGES) sk = 0;
+              if (joined == live) elect_commit_pair(BAR_EMPTY(sk));
+              if (++sk == (uint32_t)STAGES) sk = 0;
             }
             if (full) break;
           }
         }
         // ---- steady state ---------------------------------------------------------------------------------------
-        const bool all_in_ramp = kt == KT;
+        const bool in_ramp = kt == KT;
+        bool ready = false;                            // the next step was complete when the last one was issued
         for (; ok && kt < KT; ++kt) {
-          ok = __all_sync(0xFFFFFFFFu, mbar_wait_cluster(BAR_SF(s), ph, ctl, 612));
+          if (!__all_sync(0xFFFFFFFFu, ready)) ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_SF(s), ph, ctl, 612));
           if (!ok) break;
           tc_fence_after();
 #pragma unroll
           for (int u = 0; u < 2; ++u)
             if ((live >> u) & 1u) {
               issue(u, kt, s);
-              if (kt == KT - 1) mma_commit_pair(BAR_ACC_FULL(u), leader);
+              if (kt == KT - 1) elect_commit_pair(BAR_ACC_FULL(reg[u]));
             }
-          mma_commit_pair(BAR_EMPTY(s), leader);
-          if (++s == STAGES) { s = 0; ph ^= 1u; }
+          elect_commit_pair(BAR_EMPTY(s));
+          if (++s == (uint32_t)STAGES) { s = 0; ph ^= 1u; }
+          ready = mbar_test(BAR_SF(s), ph);
         }
-        if (ok && all_in_ramp)
+        if (ok && in_ramp)
 #pragma unroll
           for (int u = 0; u < 2; ++u)
-            if ((live >> u) & 1u) mma_commit_pair(BAR_ACC_FULL(u), leader);
+            if ((live >> u) & 1u) elect_commit_pair(BAR_ACC_FULL(reg[u]));
+        const uint32_t last = live == 3u ? reg[1] : reg[0];
+        r0 = last + 1 < (uint32_t)a.regions ? last + 1 : 0u;
       }
       // every MMA issued by this warp has retired before tensor memory is freed
-      mma_commit_pair_local(BAR_DRAIN, leader);
+      elect_commit_pair_local(BAR_DRAIN);
       mbar_wait(BAR_DRAIN, 0, ctl, 614);
     }
     __syncwarp();
@@ -493,31 +488,43 @@ gemm_mx_pair_kernel(const GemmParams p, const PairParams a, const __grid_constan
     // lane l of every lane quarter holds rows l, l + 32, ... of each block of scales: four columns per weight block, one per
     // 32 tokens and term (words are one row's four k groups, rows in order).
     const int qd = warp & 3;
-    uint32_t it = 0, tc = 0;
+    uint32_t s = 0, ph = 0, tc = 0;
     bool ok = true;
     PTile t, nxt;
-    if (pair < n_tiles) nxt = map_ptile<C::NMAX>(p, s_prefix, pair / MT);
+    if (pair < n_tiles) nxt = map_ptile(p, s_prefix, pair / MT);
     for (int tile = pair; tile < n_tiles && ok; tile += n_pairs, ++tc) {
       t = nxt;
       if (warp == PP_SF_WARP0 && lane == 0) s_cols[tc & 7u] = t.cols;     // read by the MMA warp after the first SF wait
-      for (int kt = 0; kt < KT; ++kt, ++it) {
-        const int s = it % STAGES;
-        ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_FULL(s), (it / STAGES) & 1u, ctl, 615));
+      for (int kt = 0; kt < KT; ++kt) {
+        ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_FULL(s), ph, ctl, 615));
         if (!ok) break;
-        const uint32_t st = sbase + (uint32_t)s * C::STAGE;
-        const uint32_t taddr = tmem_base + ((uint32_t)(qd * 32) << 16) + (uint32_t)(C::SF_BASE + s * C::SF_COLS);
-        const uint4 w0 = lds128(st + C::OFF_WS + (uint32_t)lane * 16u), w1 = lds128(st + C::OFF_WS + 512u + (uint32_t)lane * 16u);
-        uint32_t x[TERMS][8];
+        const uint32_t st = sbase + s * (uint32_t)a.stage_bytes;
+        const uint32_t taddr = tmem_base + ((uint32_t)(qd * 32) << 16) + SF_BASE + s * SF_COLS<FORM>;
+        uint4 w0, w1;
+        if constexpr (TILED) {                         // [row][4 groups], rows in the order the operand has them
+          const uint32_t ws = st + OFF_WS + (uint32_t)tiled_row(lane) * 4u;
+          w0 = make_uint4(lds32(ws), lds32(ws + 128u), lds32(ws + 256u), lds32(ws + 384u));
+          w1 = make_uint4(lds32(ws + 512u), lds32(ws + 640u), lds32(ws + 768u), lds32(ws + 896u));
+        } else {
+          w0 = lds128(st + OFF_WS + (uint32_t)lane * 16u);
+          w1 = lds128(st + OFF_WS + 512u + (uint32_t)lane * 16u);
+        }
+        uint32_t x[MMAS][8];
+        const int n_cols = FORM == PP_SIDE ? 2 * t.cols : t.cols;
 #pragma unroll
-        for (int c = 0; c < TERMS; ++c)
+        for (int c = 0; c < MMAS; ++c)
 #pragma unroll
-          for (int i = 0; i < 8; ++i) x[c][i] = lds32(st + C::OFF_XS + (uint32_t)(c * 1024 + (32 * i + lane) * 4));
+          for (int i = 0; i < 8; ++i) {
+            const int n = 32 * i + lane;               // column; TWO: eight hi words, eight lo words, ...
+            x[c][i] = 0;
+            if (32 * i < n_cols) x[c][i] = lds32(st + OFF_XS + (uint32_t)(FORM == PP_TWO ? (n >> 3) * 64 + c * 32 + (n & 7) * 4 : n * 4));
+          }
         asm volatile(
             "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
             "r"(w0.x), "r"(w0.y), "r"(w0.z), "r"(w0.w), "r"(w1.x), "r"(w1.y), "r"(w1.z), "r"(w1.w), "r"(x[0][0]), "r"(x[0][1]),
             "r"(x[0][2]), "r"(x[0][3]), "r"(x[0][4]), "r"(x[0][5]), "r"(x[0][6]), "r"(x[0][7])
             : "memory");
-        if constexpr (TERMS == 2)
+        if constexpr (FORM == PP_TWO)
           asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr + 16u), "r"(x[1][0]),
                        "r"(x[1][1]), "r"(x[1][2]), "r"(x[1][3]), "r"(x[1][4]), "r"(x[1][5]), "r"(x[1][6]), "r"(x[1][7])
                        : "memory");
@@ -525,158 +532,84 @@ gemm_mx_pair_kernel(const GemmParams p, const PairParams a, const __grid_constan
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(BAR_SF(s), 0);
-        if (kt == 0 && tile + n_pairs < n_tiles) nxt = map_ptile<C::NMAX>(p, s_prefix, (tile + n_pairs) / MT);
+        if (++s == (uint32_t)STAGES) { s = 0; ph ^= 1u; }
+        if (kt == 0 && tile + n_pairs < n_tiles) nxt = map_ptile(p, s_prefix, (tile + n_pairs) / MT);
       }
     }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS_EPI));
     // ================================= epilogue =======================================================
-    // Accumulator [weight row = lane][token = column].  The warps of a lane quarter take the 16-token chunks of a unit in turn.
-    // Neighbouring lanes hold neighbouring outputs of a row (or gate and linear): they swap halves of a chunk, after which the
-    // even lane has both values of tokens 0-7 and the odd lane those of tokens 8-15.  Row addresses and routing weights come
-    // from a table in shared memory, filled once per tile.
+    // The warps of a lane quarter take the 16-token chunks of a unit in turn.
     const int ew = warp - PP_EPI_WARP0, qd = warp & 3, grp = ew >> 2;
     const int tid = threadIdx.x - PP_EPI_WARP0 * 32;
-    const int odd = lane & 1;
+    const int own = TILED ? tiled_row(lane) : lane;    // weight row of this lane inside its quarter
+    const int odd = own & 1;
     const uint32_t sel = odd ? 0x3276u : 0x5410u;
     const bool swiglu = p.activation == MOE_ACT_SWIGLU;
     const bool vec = p.ld_y % 2 == 0 && (uintptr_t)p.y % (2 * sizeof(TY)) == 0;
     uint32_t tc = 0;
-    uint32_t acc_ph = 0;                               // parity to wait for, per unit
+    uint32_t acc_ph = 0, reg = 0;                      // parity to wait for, per region; region of the next block
     bool ok = true;
     for (int tile = pair; tile < n_tiles && ok; tile += n_pairs, ++tc) {
-      const PTile t = map_ptile<C::NMAX>(p, s_prefix, tile / MT);
-      const int mt = tile % MT;
-      const uint32_t tab = sbase + C::OFF_TAB + (tc & 1u) * C::TAB;
-      if (tid < t.cols) {                                         // at most 224 of the 256 or more threads
-        unsigned long long row = 0;
-        float beta = 1.0f, gamma = 1.0f;
-        if (tid < t.rows) {
-          const int64_t m = t.row0 + tid;
-          const int64_t d = p.scatter_indx ? (int64_t)p.scatter_indx[m] : m;
-          if (d >= 0) row = (unsigned long long)gemm_out_row<TY>(p, d);
-          if (p.betas) beta = p.betas[m];
-          if (p.gammas) gamma = p.gammas[m];
-        }
-        asm volatile("st.shared.u64 [%0], %1;" ::"r"(tab + (uint32_t)tid * 8u), "l"(row) : "memory");
-        asm volatile("st.shared.f32 [%0], %1;" ::"r"(tab + 2048u + (uint32_t)tid * 4u), "f"(gamma) : "memory");
-        asm volatile("st.shared.f32 [%0], %1;" ::"r"(tab + 3072u + (uint32_t)tid * 4u), "f"(beta) : "memory");
-      }
+      const PTile t = map_ptile(p, s_prefix, tile / MT);
+      const Blocks b = blocks_of(tile);
+      const uint32_t tab = ctl0 + (tc & 1u) * PAIR_TAB;
+      if (tid < t.cols) pair_table_entry<TY>(p, t, tid, tab);
       float bias_m[2];
 #pragma unroll
       for (int m = 0; m < 2; ++m) {
-        const int n = ((mt * 2 + m) * 2 + (int)rank) * 128 + qd * 32 + lane;     // own weight row
+        const int n = (b.first + m) * 128 + qd * 32 + own;
         bias_m[m] = (p.bias && n < p.N) ? load_bias(p.bias, p.bias_dtype, (int64_t)t.e * p.ld_bias + n) : 0.0f;
       }
       asm volatile("bar.sync 1, %0;" ::"n"(PP_EPI_WARPS * 32) : "memory");
 #pragma unroll 1
-      for (int u = 0; u < 2; ++u) {
-        if (mt * 2 + u >= MB) break;
-        const int ne = ((mt * 2 + u) * 2 + (int)rank) * 128 + qd * 32 + (lane & ~1);      // first of the lane pair's two columns
+      for (int u = 0; u < b.units; ++u) {
+        const int ne = (b.first + u) * 128 + qd * 32 + (own & ~1);      // first of the lane pair's two columns
         const bool first = ne < p.N, both = ne + 1 < p.N;
-        const float bias_n = u ? bias_m[1] : bias_m[0];
-        ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_ACC_FULL(u), (acc_ph >> u) & 1u, ctl, 616));
+        const PairOut out{ne, first, both, __all_sync(0xFFFFFFFFu, both && (swiglu || vec)) != 0, odd, sel, u ? bias_m[1] : bias_m[0]};
+        ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_ACC_FULL(reg), (acc_ph >> reg) & 1u, ctl, 616));
         if (!ok) break;
-        acc_ph ^= 1u << u;
+        acc_ph ^= 1u << reg;
         tc_fence_after();
-        const uint32_t taddr = tmem_base + ((uint32_t)(qd * 32) << 16) + (uint32_t)(u * C::NMAX);
-        // No branch inside a chunk but the stores' own predicates: exchanges, table loads and arithmetic of its tokens
-        // overlap (token by token behind a branch each, a chunk took 1700 cycles).
-        const bool fast = __all_sync(0xFFFFFFFFu, both && (swiglu || vec));
-        auto emit = [&](const uint32_t (&raw)[16], int c) {
-          const uint32_t tb = tab + (uint32_t)(c) * 8u, tg = tab + 2048u + (uint32_t)(c) * 4u;
-          float v[16];
-#pragma unroll
-          for (int j = 0; j < 16; j += 2) add_f32x2(v[j], v[j + 1], __uint_as_float(raw[j]), __uint_as_float(raw[j + 1]), bias_n, bias_n);
-          if (p.betas) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(raw[j]) + bias_n * __uint_as_float(lds32(tg + 1024u + (uint32_t)j * 4u));
-          }
-          if (p.has_out_alpha) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] *= p.out_alpha;
-          }
-          unsigned long long row[8];                                   // output rows of this lane's eight tokens
-#pragma unroll
-          for (int j = 0; j < 8; j += 2) {
-            const uint4 e = lds128(tb + (uint32_t)(j + 8 * odd) * 8u);
-            row[j] = ((unsigned long long)e.y << 32) | e.x;
-            row[j + 1] = ((unsigned long long)e.w << 32) | e.z;
-          }
-          if (!swiglu && sizeof(TY) == 2 && fast) {
-            // weights applied and rounded before the exchange: one shuffle and one byte permute per pair of outputs
-#pragma unroll
-            for (int j = 0; j < 16; j += 4) {
-              const uint4 g = lds128(tg + (uint32_t)j * 4u);
-              mul_f32x2(v[j], v[j + 1], v[j], v[j + 1], __uint_as_float(g.x), __uint_as_float(g.y));
-              mul_f32x2(v[j + 2], v[j + 3], v[j + 2], v[j + 3], __uint_as_float(g.z), __uint_as_float(g.w));
-            }
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              TY h[2] = {from_f32<TY>(v[j]), from_f32<TY>(v[8 + j])};
-              const uint32_t own = *reinterpret_cast<const uint32_t*>(h);
-              const uint32_t out = __byte_perm(own, __shfl_xor_sync(0xFFFFFFFFu, own, 1), sel);
-              if (row[j]) *reinterpret_cast<uint32_t*>((TY*)row[j] + ne) = out;
-            }
-            return;
-          }
-          float v0[8], v1[8], g[8];
-#pragma unroll
-          for (int j = 0; j < 8; j += 4) {
-            const uint4 e = lds128(tg + (uint32_t)(j + 8 * odd) * 4u);
-            g[j] = __uint_as_float(e.x); g[j + 1] = __uint_as_float(e.y); g[j + 2] = __uint_as_float(e.z); g[j + 3] = __uint_as_float(e.w);
-          }
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float recv = __shfl_xor_sync(0xFFFFFFFFu, odd ? v[j] : v[8 + j], 1);
-            v0[j] = odd ? recv : v[j];
-            v1[j] = odd ? v[8 + j] : recv;
-          }
-          if (swiglu) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) v0[j] = gemm_swiglu(v0[j], v1[j], p.act_alpha, p.act_limit, p.act_has_limit) * g[j];
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-              if (row[j] && both) ((TY*)row[j])[ne >> 1] = from_f32<TY>(v0[j]);
-          } else {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              if (row[j] && first) ((TY*)row[j])[ne] = from_f32<TY>(v0[j] * g[j]);
-              if (row[j] && both) ((TY*)row[j])[ne + 1] = from_f32<TY>(v1[j] * g[j]);
-            }
-          }
-        };
-        if constexpr (TERMS == 2) {
-          // The warp's whole share of the unit goes to registers and the unit back to the MMA warp before any of it is worked
-          // on: drained chunk by chunk, the tensor pipe waited 3000-4600 cycles for the first unit of every tile.  (The wider
-          // one-term tile does not fit the registers that way.)
-          uint32_t raw[C::EPI_CHUNKS][16];
-#pragma unroll
-          for (int i = 0; i < C::EPI_CHUNKS; ++i) {
-            const int c = (grp + i * (PP_EPI_WARPS / 4)) * 16;
-            if (c < t.rows) tmem_ld16(taddr + (uint32_t)c, raw[i]);
-          }
-          tmem_ld_wait();
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive_cluster(BAR_ACC_EMPTY(u), 0);
-#pragma unroll
-          for (int i = 0; i < C::EPI_CHUNKS; ++i) {
-            const int c = (grp + i * (PP_EPI_WARPS / 4)) * 16;
-            if (c < t.rows) emit(raw[i], c);
-          }
-        } else {
-          uint32_t raw[16];
+        const uint32_t taddr = tmem_base + ((uint32_t)(qd * 32) << 16) + reg * (uint32_t)a.reg_cols;
+        // The warp's share of the region (up to four chunks at a time) goes to registers and the region back to the MMA warp
+        // before any of it is worked on: drained chunk by chunk, the tensor pipe waited 3000-4600 cycles for the first region of
+        // every tile.
+        constexpr int STEP = 4 * PP_EPI_WARPS;         // columns from one chunk of a warp to its next
+        constexpr int BATCH = FORM == PP_SIDE ? 2 : 4;
 #pragma unroll 1
-          for (int c = grp * 16; c < t.rows; c += 4 * PP_EPI_WARPS) {
-            tmem_ld16(taddr + (uint32_t)c, raw);
-            tmem_ld_wait();
-            emit(raw, c);
+        for (int c0 = grp * 16; c0 < t.rows || c0 == grp * 16; c0 += BATCH * STEP) {
+          constexpr int W = FORM == PP_SIDE ? 32 : 16;
+          uint32_t raw[BATCH][W];
+#pragma unroll
+          for (int i = 0; i < BATCH; ++i)
+            if (c0 + STEP * i < t.rows) {
+              if constexpr (FORM == PP_SIDE) tmem_ld32(taddr + (uint32_t)(2 * (c0 + STEP * i)), raw[i]);
+              else tmem_ld16(taddr + (uint32_t)(c0 + STEP * i), raw[i]);
+            }
+          tmem_ld_wait();
+          if (c0 + BATCH * STEP >= t.rows) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(BAR_ACC_EMPTY(reg), 0);
           }
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive_cluster(BAR_ACC_EMPTY(u), 0);
+#pragma unroll
+          for (int i = 0; i < BATCH; ++i)
+            if (c0 + STEP * i < t.rows) {
+              if constexpr (FORM == PP_SIDE) {
+                uint32_t v[16];
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                  const int at = (j >> 3) * 16 + (j & 7);
+                  v[j] = __float_as_uint(__uint_as_float(raw[i][at]) + __uint_as_float(raw[i][at + 8]));
+                }
+                pair_emit<TY>(p, out, v, tab, c0 + STEP * i);
+              } else {
+                pair_emit<TY>(p, out, raw[i], tab, c0 + STEP * i);
+              }
+            }
         }
+        if (++reg == (uint32_t)a.regions) reg = 0;
       }
     }
     // aborting: a warp that is a tile ahead may be at the table barrier
@@ -711,12 +644,43 @@ PairPlan pair_plan(const MoeGemmArgs& a) {
   return pl;
 }
 
-template <typename TY, int TERMS>
-int launch_mx_pair(const GemmParams& p, const PairParams& q, int64_t tiles, const CUtensorMap& w_map, int idle_sms, cudaStream_t st) {
-  auto kernel = gemm_mx_pair_kernel<TY, TERMS>;
+// Token columns and weight blocks of a tile, and the form of two-term tokens.  fc1 + fc2, us:
+// - SIDE with 96 columns of tokens up to 224 rows per expert, where TWO with 192 takes over (32 experts of 2880 x 5760: 16 rows
+//   156 and 192, 64 rows 207 and 231, 150 rows 321 and 327, 300 rows 506 and 481; 128 experts, 64 rows: 608 and 659).  SIDE with
+//   64 or 32 columns gains 2 % below 16 rows and loses 3-30 % from 32 on.
+// - One weight block per tile where twice the tiles still run at a time (8 experts of 512 x 2048, 16 rows: 19 -> 17); beyond, a
+//   tile of two blocks reads the tokens once for both (32 experts, 64 rows: 91 against 105).
+struct PairShape { int nmax, upt, form; };
+PairShape pair_shape(const MoeGemmArgs& a, int terms) {
+  const int64_t experts = a.slice_sizes ? a.E : 1, per = a.M / experts;
+  PairShape s;
+  s.form = terms == 1 ? PP_ONE : (per < 224 ? PP_SIDE : PP_TWO);
+  s.nmax = s.form == PP_SIDE ? 96 : 192;
+  const int64_t active = experts < a.M ? experts : a.M;
+  s.upt = active * (per / s.nmax + 1) * cdiv64(a.N, 256) <= moe_sm_count() / 2 ? 1 : 2;
+  return s;
+}
+
+template <typename TY, int FORM, bool TILED>
+int launch_mx_pair(const GemmParams& p, PairParams q, const PairShape& shape, const MoeGemmArgs& args, const PairMaps& maps,
+                   cudaStream_t st) {
+  auto kernel = gemm_mx_pair_kernel<TY, FORM, TILED>;
+  q.nmax = shape.nmax; q.upt = shape.upt;
+  q.reg_cols = q.nmax * (FORM == PP_SIDE ? 2 : 1);
+  q.stage_bytes = q.upt * 128 * 128 + TERMS_OF<FORM> * (q.nmax * 64 + 1024) + 1024;
+  q.stages = (PP_SMEM - 1024 - PP_CTL) / q.stage_bytes;
+  if (q.stages > PP_MAX_STAGES) q.stages = PP_MAX_STAGES;
+  while ((TMEM_COLS - q.stages * SF_COLS<FORM>) / q.reg_cols < 2) --q.stages;
+  q.regions = (TMEM_COLS - q.stages * SF_COLS<FORM>) / q.reg_cols;
+  if (q.regions > PP_MAX_REGIONS) q.regions = PP_MAX_REGIONS;
+  MOE_CHECK_ARG(q.stages >= 2, "moe_grouped_gemm: block-scaled pair tile does not fit shared memory");
+  // every expert has at most ceil(rows / nmax) token tiles
+  const int64_t experts = args.slice_sizes ? (args.E < args.M ? args.E : args.M) : 0;
+  const int64_t tiles = (experts + cdiv64(args.M, q.nmax)) * cdiv64(cdiv64(q.NB, 2), q.upt);
+  const int idle_sms = args.idle_sms > 0 ? args.idle_sms : 0;
   cudaLaunchConfig_t cfg = {};
   cfg.blockDim = dim3(PP_THREADS, 1, 1);
-  cfg.dynamicSmemBytes = PCfg<TERMS>::ALLOC;
+  cfg.dynamicSmemBytes = PP_SMEM;
   cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -732,7 +696,7 @@ int launch_mx_pair(const GemmParams& p, const PairParams& q, int64_t tiles, cons
   {
     std::lock_guard<std::mutex> lk(mu);
     if (max_pairs[dev] == 0) {
-      MOE_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PCfg<TERMS>::ALLOC));
+      MOE_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PP_SMEM));
       cfg.gridDim = dim3(2 * (unsigned)(moe_sm_count() / 2), 1, 1);
       int n = 0;
       MOE_CHECK_CUDA(cudaOccupancyMaxActiveClusters(&n, kernel, &cfg));
@@ -749,29 +713,56 @@ int launch_mx_pair(const GemmParams& p, const PairParams& q, int64_t tiles, cons
   if (tiles < pairs) pairs = tiles;
   cfg.gridDim = dim3((unsigned)(2 * pairs), 1, 1);
   moe_count_launch();
-  MOE_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kernel, p, q, w_map));
+  MOE_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kernel, p, q, maps));
   return MOE_OK;
 }
 
 template <typename TY>
-int launch_mx_pair_terms(const GemmParams& p, const PairParams& q, int terms, int64_t tiles, const CUtensorMap& m, int idle, cudaStream_t st) {
-  return terms == 2 ? launch_mx_pair<TY, 2>(p, q, tiles, m, idle, st) : launch_mx_pair<TY, 1>(p, q, tiles, m, idle, st);
+int launch_mx_pair_ty(const GemmParams& p, const PairParams& q, const MoeGemmArgs& a, const PairMaps& m, cudaStream_t st) {
+  const PairShape shape = pair_shape(a, a.x_dtype == MOE_BF16 ? 2 : 1);
+  if constexpr (sizeof(TY) > 1) {
+    if (a.w_kind == MOE_W_MX4_B200)
+      return shape.form == PP_SIDE ? launch_mx_pair<TY, PP_SIDE, true>(p, q, shape, a, m, st) : launch_mx_pair<TY, PP_TWO, true>(p, q, shape, a, m, st);
+  }
+  if (shape.form == PP_SIDE) return launch_mx_pair<TY, PP_SIDE, false>(p, q, shape, a, m, st);
+  if (shape.form == PP_TWO) return launch_mx_pair<TY, PP_TWO, false>(p, q, shape, a, m, st);
+  return launch_mx_pair<TY, PP_ONE, false>(p, q, shape, a, m, st);
 }
 
 }  // namespace
 
-// The pair form against the decode forms of gemm_mx.cu, by mean rows per expert (fc1 + fc2).  bf16 tokens, from 40 on: 32
-// experts of 2880 x 5760, 32 rows 172 us there and 189 here, 48 rows 219 and 216; 128 experts, 32 rows 530 and 486; narrow
-// products repay the larger tiles later (8 experts of 512 x 2048, 64 rows: 41 and 48).  e4m3 tokens, one term, from 16 on
-// (32 experts, 8 rows: 102 and 114; 64 rows: 320 and 167).  tile_m = 256 asks for it.
+// Where the pair form is the faster one (us, fc1 + fc2 unless said).  `load` is what one pass over the weights of the experts in
+// use costs, in elements.
+// Default tiles (against the bf16 tensor-core kernel, above ten or so rows also against the streaming one), kernel "mx" asks
+// for it: the pack pass and the cluster launch want 2^24 elements and 2^28 products a token row to be repaid, and a product
+// over fewer than 2560 weight rows stays ahead up to 512 rows per expert only.
+//   32 experts of 2880 x 5760:  1 row 96 (streaming: 112), 8 rows 152 (243), 64 rows 207 (332), 150 rows 321 (457)
+//   64 experts of 1024 x 1536:  4 rows 53 (59), 16 rows 63 (100), 64 rows 88 (106)
+//   16 experts of 1440 x 1472:  8 rows 49 (45), 32 rows 53 (55), 64 rows 59 (66), 256 rows 80 (102), 1024 rows 167 (156)
+//   8 experts of 512 x 2048:    16 rows 37 (33), 64 rows 45 (41), 256 rows 53 (49), 1024 rows 84 (66)
+// Block-scaled tiles (against the decode forms of gemm_mx.cu), tile_m = 256 asks for it: bf16 tokens from 20 rows on (32 experts
+// of 2880 x 5760, 16 rows: 139 there, 156 here, 32 rows 178 and 162; 64 experts of 1024 x 1536, 16 rows: 76 and 63), small ones from
+// 96 on (8 experts of 512 x 2048, 32 rows: 40 and 43); e4m3 tokens, one term, from 16 on (32 experts, 8 rows: 102 and 114;
+// 64 rows: 320 and 167).
 bool moe_gemm_mx_pair_wanted(const MoeGemmArgs& a) {
   if (a.slice_sizes && a.E > MAX_PREFIX_EXPERTS) return false;
   if (a.M >= (1ll << 31) - (1 << 20) || a.kernel == MOE_GEMM_MX_F4 || a.tile_n != 0) return false;
+  const int64_t experts = a.slice_sizes ? a.E : 1, per = a.M / experts;
+  const int64_t load = (experts < a.M ? experts : a.M) * a.N * a.K;
+  if (a.w_kind == MOE_W_MX4_B200) {
+    // default tiles, bf16 tokens
+    if (a.x_dtype != MOE_BF16 || (a.y_dtype != MOE_BF16 && a.y_dtype != MOE_F32) || (uintptr_t)a.w % 32 != 0 ||
+        (uintptr_t)a.w_scale % 16 != 0 || (uintptr_t)a.x % 16 != 0 || a.ld_x % 8 != 0 ||
+        (int64_t)a.E * cdiv64(a.K, 128) * cdiv64(a.N, 128) >= 2147483647LL)
+      return false;
+    if (a.kernel == MOE_GEMM_MX) return true;
+    if (a.kernel != MOE_GEMM_AUTO || a.tile_m != 0) return false;
+    return load >= (1 << 24) && (per > 0 ? per : 1) * load >= (1 << 28) && (a.N >= 2560 || per < 512);
+  }
   if (a.tile_m == 256) return true;
   if (a.tile_m != 0 || a.kernel == MOE_GEMM_MX_F8) return false;
-  const int64_t per = a.slice_sizes ? a.M / a.E : a.M;
   if (a.x_dtype != MOE_BF16) return per >= 16;
-  return per >= (a.N >= 1280 ? 40 : 96);
+  return per >= (load >= (1 << 24) ? 20 : 96);
 }
 
 int64_t moe_gemm_mx_pair_workspace(const MoeGemmArgs& a) { return pair_plan(a).ws_bytes; }
@@ -796,17 +787,31 @@ int moe_gemm_mx_pair_launch(const GemmParams& p_in, const MoeGemmArgs& a, cudaSt
   pk.gather = a.gather_indx;
   pk.K = a.K; pk.KT = pl.KT; pk.prows = pl.prows;
   pk.xq = (uint8_t*)a.mx_workspace; pk.xs = pk.xq + pl.xs_off;
-  if (pl.terms == 2) mx_pair_pack2_kernel<<<(unsigned)blocks16, 256, 0, st>>>(p, pk);
+  const bool tiled = a.w_kind == MOE_W_MX4_B200;
+  if (pl.terms == 2 && tiled) mx_pair_pack2_kernel<true><<<(unsigned)blocks16, 256, 0, st>>>(p, pk);
+  else if (pl.terms == 2) mx_pair_pack2_kernel<false><<<(unsigned)blocks16, 256, 0, st>>>(p, pk);
   else mx_pair_pack1_kernel<<<(unsigned)blocks16, 256, 0, st>>>(p, pk);
   MOE_CHECK_LAUNCH();
   PairParams q;
   q.xq = pk.xq; q.xs = pk.xs; q.prows = pl.prows; q.KT = pl.KT; q.NB = pl.NB;
-  CUtensorMap w_map;
-  if (int rc = make_w_map(a, pl.KT, pl.NB, false, 1, &w_map)) return rc;
-  // every expert has at most ceil(rows / 192) token tiles
-  const int64_t tiles = ((a.slice_sizes ? a.E : 0) + cdiv64(a.M, PCfg<2>::NMAX)) * cdiv64(pl.NB, 4);
-  const int idle = a.idle_sms > 0 ? a.idle_sms : 0;
-  if (a.y_dtype == MOE_F8E4M3) return launch_mx_pair_terms<__nv_fp8_e4m3>(p, q, pl.terms, tiles, w_map, idle, st);
-  if (a.y_dtype == MOE_BF16) return launch_mx_pair_terms<__nv_bfloat16>(p, q, pl.terms, tiles, w_map, idle, st);
-  return launch_mx_pair_terms<float>(p, q, pl.terms, tiles, w_map, idle, st);
+  PairMaps maps;
+  for (int n = 1; n <= 2; ++n) {
+    // values as the TMA unit expands them (a row of a box: 64 bytes -> 128), scales as words; blocks along the slowest dimension
+    // (default tiles) or the one before (block-scaled tiles)
+    const cuuint64_t d2 = tiled ? pl.KT : pl.NB, d3 = (cuuint64_t)a.E * (tiled ? pl.NB : pl.KT);
+    const cuuint32_t b2 = tiled ? 1 : n, b3 = tiled ? n : 1;
+    const cuuint64_t wd[4] = {128, 128, d2, d3}, wst[3] = {64, 8192, 8192 * d2};
+    const cuuint32_t wb[4] = {128, 128, b2, b3};
+    if (int rc = encode_map(&maps.w[n - 1], CU_TENSOR_MAP_DATA_TYPE_16U4_ALIGN16B, 4, a.w, wd, wst, wb, CU_TENSOR_MAP_SWIZZLE_128B,
+                            "packed e2m1 weights"))
+      return rc;
+    const cuuint64_t sd[3] = {128, d2, d3}, sst[2] = {512, 512 * d2};
+    const cuuint32_t sb[3] = {128, b2, b3};
+    if (int rc = encode_map(&maps.s[n - 1], CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, a.w_scale, sd, sst, sb, CU_TENSOR_MAP_SWIZZLE_NONE, "weight scales"))
+      return rc;
+  }
+  if (a.y_dtype == MOE_BF16) return launch_mx_pair_ty<__nv_bfloat16>(p, q, a, maps, st);
+  if (a.y_dtype == MOE_F32) return launch_mx_pair_ty<float>(p, q, a, maps, st);
+  MOE_CHECK_ARG(!tiled, "moe_grouped_gemm: e4m3 output needs weights in the block-scaled layout");
+  return launch_mx_pair_ty<__nv_fp8_e4m3>(p, q, a, maps, st);
 }

@@ -20,7 +20,7 @@ constexpr int RAWS_BYTES = HALF_N * 4;                  // 512 B: the scale tile
 constexpr int TMEM_COLS = 512;                           // two accumulator buffers of MH x 128 columns (256 used when MH = 1)
 constexpr int MAX_PREFIX_EXPERTS = 512;                  // experts the 256-row tile schedule can index
 
-constexpr unsigned long long WAIT_LIMIT_NS = 2000000000ull;      // a wait that lasts 2 s aborts the CTA
+constexpr long long WAIT_LIMIT_CYCLES = 4000000000ll;            // a wait that lasts 2 s (at 2 GHz) aborts the CTA
 
 // ---- PTX wrappers -------------------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -57,25 +57,20 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-__device__ __forceinline__ unsigned long long global_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
 struct Ctl {
   volatile int* abort_flag;   // shared memory
   int32_t* status;            // global, may be null
 };
 
-// Bounded wait.  Returns false when the CTA is aborting (this wait expired, or another one did).
+// Bounded wait.  Returns false when the CTA is aborting (this wait expired, or another one did).  The limit is counted in SM
+// cycles and looked at every 256 tries: a read of %globaltimer per wait took longer than most waits.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const Ctl& ctl, int code) {
   if (mbar_try(bar, parity)) return true;
-  const unsigned long long t0 = global_ns();
-  for (;;) {
+  const long long t0 = clock64();
+  for (uint32_t i = 0;; ++i) {
     if (mbar_try(bar, parity)) return true;
-    if (*ctl.abort_flag) return false;
-    if (global_ns() - t0 > WAIT_LIMIT_NS) {
+    if ((i & 7u) == 7u && *ctl.abort_flag) return false;
+    if ((i & 255u) == 255u && clock64() - t0 > WAIT_LIMIT_CYCLES) {
       *ctl.abort_flag = 1;
       if (ctl.status) atomicExch(ctl.status, code);
       return false;
@@ -133,15 +128,10 @@ __device__ __forceinline__ void mma_commit(uint32_t bar) {
 }
 
 // the same for a warp that runs its issue loop as a whole: one elected lane's predicate guards the instruction
-__device__ __forceinline__ uint32_t elect_one() {
-  uint32_t r;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void mma_commit(uint32_t bar, uint32_t leader) {
+__device__ __forceinline__ void elect_commit(uint32_t bar) {
   asm volatile(
-      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
-      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar), "r"(leader)
+      "{\n\t.reg .pred q;\n\telect.sync _|q, 0xFFFFFFFF;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar)
       : "memory");
 }
 

@@ -150,7 +150,7 @@ gemm_tc_pair_kernel(const GemmParams p, const int64_t grid_m_static, const __gri
       const uint32_t idesc = make_idesc_pair(P_TILE_N);
       for (int64_t tile = pair; tile < n_tiles && ok; tile += n_pairs, ++tc) {
         const uint32_t ab = tc & 1u;
-        ok = mbar_wait_cluster(BAR_ACC_EMPTY(ab), ((tc >> 1) & 1u) ^ 1u, ctl, 101);
+        ok = mbar_wait(BAR_ACC_EMPTY(ab), ((tc >> 1) & 1u) ^ 1u, ctl, 101);
         if (!ok) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + ab * P_ACC_COLS;
@@ -159,7 +159,7 @@ gemm_tc_pair_kernel(const GemmParams p, const int64_t grid_m_static, const __gri
           const uint32_t ph = (it / P_STAGES) & 1u;
           ok = mbar_wait(BAR_A_FULL(s), ph, ctl, 102);
           ok = ok && mbar_wait(BAR_B_FULL(s), ph, ctl, 103);
-          ok = ok && mbar_wait_cluster(BAR_PEER_FULL(s), ph, ctl, 105);
+          ok = ok && mbar_wait(BAR_PEER_FULL(s), ph, ctl, 105);
           if (!ok) break;
           fence_proxy_async();          // the A stage was written by cp.async (generic proxy) of other threads
           tc_fence_after();

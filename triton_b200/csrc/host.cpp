@@ -112,18 +112,28 @@ py::tuple bitmatrix_metadata(const Tensor& indx, int64_t E, const OptTensor& n_r
 }
 
 // ---- grouped GEMM ------------------------------------------------------------------------------------------------
-// temporaries of one call: the block-scaled kernels' token workspace or the bf16 kernel's gathered rows
+// Temporary bytes of one call: the block-scaled kernels' token workspace, else the bf16 kernel's gathered rows (2048 and more:
+// the library decides whether to use them), else none.
+int64_t temp_bytes(MoeGemmArgs& g, bool gathers, bool& workspace) {
+  const bool tiles = g.w_kind == MOE_W_MX4_B200 || g.w_kind == MOE_W_MX4_B200MX;
+  const int64_t ws = tiles ? (int64_t)lib.moe_gemm_mx_workspace_bytes(&g) : 0;
+  workspace = ws > 0;
+  if (workspace) return ws;
+  return gathers && g.w_kind == MOE_W_MX4_B200 && g.x_dtype == MOE_BF16 && g.M >= 2048 ? g.M * g.K * 2 : 0;
+}
+void set_temp(MoeGemmArgs& g, void* at, int64_t bytes, bool workspace) {
+  if (bytes == 0) return;
+  if (workspace) { g.mx_workspace = at; g.mx_workspace_bytes = bytes; }
+  else { g.gather_scratch = at; g.gather_scratch_bytes = bytes; }
+}
+
 int run_gemm(MoeGemmArgs& g, const Tensor& like) {
-  Tensor scratch;
-  if (g.w_kind == MOE_W_MX4_B200MX) {
-    const int64_t bytes = (int64_t)lib.moe_gemm_mx_workspace_bytes(&g);
-    scratch = empty({bytes + 1024}, at::kByte, like);
-    g.mx_workspace = (void*)(((uintptr_t)scratch.data_ptr() + 1023) / 1024 * 1024);
-    g.mx_workspace_bytes = bytes;
-  } else if (g.gather_indx && g.w_kind == MOE_W_MX4_B200 && g.x_dtype == MOE_BF16 && g.M >= 2048) {
-    scratch = empty({g.M * g.K}, at::kBFloat16, like);       // the library decides whether to use it
-    g.gather_scratch = scratch.data_ptr();
-    g.gather_scratch_bytes = g.M * g.K * 2;
+  bool workspace;
+  const int64_t bytes = temp_bytes(g, g.gather_indx != nullptr, workspace);
+  Tensor temp;
+  if (bytes > 0) {
+    temp = empty({bytes + 1024}, at::kByte, like);
+    set_temp(g, (void*)(((uintptr_t)temp.data_ptr() + 1023) / 1024 * 1024), bytes, workspace);
   }
   return lib.moe_grouped_gemm(&g, stream());
 }
@@ -237,11 +247,10 @@ Tensor layer(const Tensor& x, const Tensor& logits, int64_t k, const py::tuple& 
   g1.slice_sizes = g2.slice_sizes = &present;
   const int64_t lo = pad512(E + 1), mnb = max_blocks16(E, n), ls = pad512(mnb), words = cdiv(E, 32), t_pad = cdiv(T, 32) * 32;
   const int64_t route_ws = (int64_t)lib.moe_route_workspace(T, (int)E, (int)k);
-  auto temp_bytes = [&](MoeGemmArgs& g, bool gathers) -> int64_t {
-    if (g.w_kind == MOE_W_MX4_B200MX) return (int64_t)lib.moe_gemm_mx_workspace_bytes(&g);
-    return gathers && n >= 2048 ? n * g.K * 2 : 0;
-  };
-  const int64_t t1 = temp_bytes(g1, true), t2 = temp_bytes(g2, false);
+  g1.ld_x = x.stride(0); g2.ld_x = ff;   // (the size query looks at types and pitches too)
+  g1.y_dtype = fp8 ? MOE_F8E4M3 : MOE_BF16; g2.y_dtype = MOE_BF16;
+  bool ws1, ws2;
+  const int64_t t1 = temp_bytes(g1, true, ws1), t2 = temp_bytes(g2, false, ws2);
   Carver c;
   const int64_t o_vals = c.take(n * 4), o_indx = c.take(n * 2), o_bm = c.take(words * t_pad * 4), o_sum = c.take(E * 4), o_col = c.take(n * 4),
                 o_row = c.take(n * 4), o_offs = c.take(5 * lo * 4), o_sched = c.take(4 * ls * 4), o_rws = c.take(route_ws), o_tok = c.take(n * 4),
@@ -260,18 +269,17 @@ Tensor layer(const Tensor& x, const Tensor& logits, int64_t k, const py::tuple& 
     g->slice_sizes = (int32_t*)(base + o_sum); g->slice_offs = offs;
     g->block_offs_16 = offs + lo; g->block_sched_16 = sched;
     g->ld_block_offs = lo; g->ld_block_sched = ls;
-    const int64_t t = g == &g1 ? t1 : t2;
-    if (g->w_kind == MOE_W_MX4_B200MX) { g->mx_workspace = base + o_tmp; g->mx_workspace_bytes = t; }
-    else if (t > 0) { g->gather_scratch = base + o_tmp; g->gather_scratch_bytes = t; }
   }
+  set_temp(g1, base + o_tmp, t1, ws1);
+  set_temp(g2, base + o_tmp, t2, ws2);
   g1.gather_indx = (int32_t*)(base + o_tok);
   g1.activation = MOE_ACT_SWIGLU; g1.act_alpha = (float)alpha;
   if (limit) { g1.act_limit = (float)*limit; g1.act_has_limit = 1; }
-  g1.y = base + o_h; g1.y_dtype = fp8 ? MOE_F8E4M3 : MOE_BF16; g1.ld_y = ff;
+  g1.y = base + o_h; g1.ld_y = ff;
   check(lib.moe_grouped_gemm(&g1, st), "moe_grouped_gemm", true);
-  g2.x = base + o_h; g2.ld_x = ff; g2.rows_x = n;
+  g2.x = base + o_h; g2.rows_x = n;
   g2.scatter_indx = (int32_t*)(base + o_col); g2.gammas = (float*)(base + o_gam);
-  g2.y = base + o_y; g2.y_dtype = MOE_BF16; g2.ld_y = d;
+  g2.y = base + o_y; g2.ld_y = d;
   check(lib.moe_grouped_gemm(&g2, st), "moe_grouped_gemm", true);
   check(lib.moe_reduce(base + o_y, MOE_BF16, k, T, d, d, k * d, 1, nullptr, 0, 0, 0, 0, nullptr, 0, 0, 0, z.data_ptr(), MOE_BF16, d, 1, st),
         "moe_reduce");

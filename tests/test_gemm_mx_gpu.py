@@ -305,7 +305,7 @@ def test_block_scaled_few_tiles_k_step_stages(K, sizes, act, device):
     (160, 129, [31, 32, 5, 449]),                   # k tail, odd width (scalar stores), an expert of several tiles
     (416, 514, [64, 1, 0, 97]),                     # ring longer than the k loop, a second tile of weight blocks
     (1024, 768, [300]),                             # three 256-row blocks: the last tile has one unit
-    (160, 5129, [31, 32, 95, 449]),                 # enough tiles for two 256-row blocks each, the last has one row
+    (160, 5129, [31, 32, 95, 40]),                  # enough tiles for two 256-row blocks each, the last has one row
     (96, 4866, [300, 2, 2, 700]),                   # the same with more rows per expert
     (96, 514, [225, 385]),                          # more rows per expert, one 256-row block each
 ])
@@ -346,7 +346,7 @@ def test_pair_kernel_tile_edges(K, N, sizes, acts, act, device):
     (160, 129, [31, 32, 5, 449]),                   # k tail, odd width, an expert of several tiles
     (416, 514, [64, 1, 0, 97]),                     # a second tile of weight blocks
     (1024, 768, [300, 2, 2]),                       # three 256-row blocks: the last tile has one
-    (160, 5129, [31, 32, 95, 449]),                 # enough tiles for two 256-row blocks each, the last has one row
+    (160, 5129, [31, 32, 95, 40]),                  # enough tiles for two 256-row blocks each, the last has one row
     (96, 4866, [300, 2, 2, 700]),                   # the same with more rows per expert
     (96, 514, [225, 385]),                          # more rows per expert, one 256-row block each
 ])

@@ -8,24 +8,25 @@
 //
 // (Elements far below their group of 32's largest lose what lies below 2^-23 of it, as much as an fp32 sum rounds away.)
 //
-// What bounds it.  An SM takes in at most about 26 B per cycle from L2, and the MMA of a 128-k step is 64 cycles per 128
-// token columns, weight block and K = 32: the tile has to be large.  A cluster of two CTAs computes (2 x 256 weight rows) x
-// (up to 192 tokens): the weights are the M operand (every CTA loads its own 128 rows of each of the two 256-row blocks,
-// packed in global memory: 16 KB per step), the tokens the N operand (every CTA loads half of them: 12 or 24 KB), 26-34 B per
-// MMA cycle.  Tokens on N also make a ragged tail cost what it holds, in steps of 32 rows, where tokens on M padded every
-// expert to a multiple of 128 or 256 (31 % of the rows of a skewed 128-expert batch of 16384 tokens).  With few rows per
-// expert it is the packed weights: 128 experts of 2880 x 5760, 300 tokens, 1.1 GB in 189 us.
+// What bounds it.  Shared memory, 128 B per cycle and SM: every operand byte is written once and read once per MMA, and an
+// e2m1 value takes a byte there.  A cluster of two CTAs computes (2 x 256 weight rows) x (up to 128 tokens of two terms, 192 of
+// one): the weights are the M operand (every CTA loads its own 128 rows of each of the two 256-row blocks: 32 KB per 128 k,
+// packed in global memory), the tokens the N operand (every CTA loads half of them).  128 tokens of two terms: 49 KB written and
+// 97 KB read per step, 1140 cycles, against 1024 of MMA; as two tiles of 64 tokens the weights alone would be written and
+// read twice.  Large prefill runs into the power limit first (1.5 GHz).  Tokens on N
+// also make a ragged tail cost what it holds, in steps of 32 rows, where tokens on M padded every expert to a multiple of 128
+// or 256 (31 % of the rows of a skewed 128-expert batch of 16384 tokens).  With few rows per expert the packed weights bound it:
+// 128 experts of 2880 x 5760, 300 tokens, 1.1 GB in 165 us.
 //
 // A k step of a small tile is eight MMAs of 64 cycles, so what the issuing warp does around them counts: operands in uniform
-// registers, the election inside the instruction's own asm block (with a leader flag kept in a register a step took 1150 cycles, so
-// 900), the next step's barrier asked for ahead.
+// registers, the election inside the instruction's own asm block (a step took 1150 cycles with a leader flag kept in a register,
+// 840 so), and a warp for either block, whose waits the other's MMAs cover (32 experts, 1200 tokens: 319 -> 305 us).
 //
-// The accumulators of a tile's 256-row blocks are regions of a ring in tensor memory; each is handed to the epilogue and back by
-// itself: the next tile starts in regions that are drained while others still are (the MMA warp lets a block lag by at most
-// the stages of the operand ring).  One accumulator of all columns drained as a whole would leave the tensor pipe idle for the
-// time of an epilogue on every tile.
+// The accumulators of a tile's 256-row blocks are regions of a ring in tensor memory, each handed to the epilogue and back by
+// itself.  A warp whose block has a region goes on while the other block still waits for one, up to the stages of the operand
+// ring ahead.  With two regions in all the pipe waited 10000 of 37000 cycles of a tile for the epilogue.
 //
-// Warps of a CTA: 0 producer, 1 MMA issue (even CTA) and tensor-memory owner, 4-7 scale loaders (shared memory ->
+// Warps of a CTA: 0 producer, 1 and 2 MMA issue (even CTA; 1 owns tensor memory), 4-7 scale loaders (shared memory ->
 // registers -> tensor memory; the token scales of all columns in both CTAs, the weight scales of the own rows), 8-19 epilogue.
 // Every wait is bounded; both CTAs meet at a cluster barrier before tensor memory is freed.
 #include "gemm_mx_common.cuh"
@@ -291,14 +292,14 @@ gemm_mx_pair_kernel(const GemmParams p, const PairParams a, const __grid_constan
   if (threadIdx.x == 0) {
     for (int s = 0; s < PP_MAX_STAGES; ++s) {
       mbar_init(BAR_FULL(s), 1);
-      mbar_init(BAR_EMPTY(s), 1);
+      mbar_init(BAR_EMPTY(s), 2);                      // both MMA warps
       mbar_init(BAR_SF(s), 8);                         // four scale warps in each CTA
     }
     for (int r = 0; r < PP_MAX_REGIONS; ++r) {
       mbar_init(BAR_ACC_FULL(r), 1);
       mbar_init(BAR_ACC_EMPTY(r), 2 * PP_EPI_WARPS);
     }
-    mbar_init(BAR_DRAIN, 1);
+    mbar_init(BAR_DRAIN, 2);
     *s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -373,109 +374,65 @@ gemm_mx_pair_kernel(const GemmParams p, const PairParams a, const __grid_constan
         for (uint32_t i = 0; i < (1u << 16) && !mbar_test(BAR_FULL(j % STAGES), (j / STAGES) & 1u); ++i) __nanosleep(64);
     }
     __syncwarp();
-  } else if (warp == 1) {
-    // ================================= MMA issuer (even CTA) ==========================================
+  } else if (warp <= 2) {
+    // ================================= MMA issuers (even CTA) =========================================
+    // One warp per block of the tile: what a warp does between its k steps is covered by the other's MMAs, and a block whose
+    // region is free starts while the other still waits for the epilogue, up to the stages of the ring ahead.
     if (rank == 0) {
-      const int k_whole = p.K >> 7;                    // steps of 128 k; the last may hold less
+      const int u = warp - 1, k_whole = p.K >> 7;      // steps of 128 k; the last may hold less
       uint32_t s = 0, ph = 0;                          // stage and parity of the next k step
-      uint32_t acc_ph = 0xFFFFu;                       // parity to wait for, per region
-      uint32_t r0 = 0, tc = 0;                         // region of the tile's first block
+      uint32_t tc = 0, blk = 0;                        // tiles and blocks of this CTA so far: block b is use b / regions of region b % regions
       bool ok = true;
       for (int tile = pair; tile < n_tiles && ok; tile += n_pairs, ++tc) {
-        ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_SF(s), ph, ctl, 612));         // first k step; the scale loader left the columns
-        if (!ok) break;
-        const uint32_t id0 = pair_idesc(__shfl_sync(0xFFFFFFFFu, s_cols[tc & 7u], 0) * (FORM == PP_SIDE ? 2 : 1), 0);
-        const uint32_t live = blocks_of(tile).units == 2 ? 3u : 1u;
-        const uint32_t reg[2] = {r0, r0 + 1 < (uint32_t)a.regions ? r0 + 1 : 0u};
-        auto issue = [&](int u, int k, uint32_t s) {   // k step `k` of block u, operands in stage s
-          const uint32_t st = sbase + s * (uint32_t)a.stage_bytes;
-          const uint32_t sf = tmem_base + SF_BASE + s * SF_COLS<FORM>;
-          const uint32_t a_lo = DESC_LO | ((st + (uint32_t)u * (128 * 128)) >> 4);
-          const uint32_t b_lo = DESC_LO | ((st + OFF_X) >> 4);
-          const uint32_t d = tmem_base + reg[u] * (uint32_t)a.reg_cols;
-          // (a step that is whole has no test between its instructions: they must issue in less than the 45-64 cycles that
-          // one of them runs)
-          if (k < k_whole) {
-#pragma unroll
-            for (int kk = 0; kk < 4; ++kk)
-#pragma unroll
-              for (int c = 0; c < MMAS; ++c)
-                mma_mxf8f6f4_pair<A_HI, B_HI>(d, a_lo + kk * A_KK, b_lo + c * (1024 >> 4) + kk * 2, id0 + ((uint32_t)kk << 4) + ((uint32_t)kk << 29),
-                                        sf + 4 * u, sf + 8 + 8 * c, (kk | c) ? 1u : (uint32_t)(k > 0));
-          } else {
-            const int kk_live = (p.K - k * 128 + 31) >> 5;
-#pragma unroll
-            for (int kk = 0; kk < 4; ++kk)
-              if (kk < kk_live) {
-#pragma unroll
-                for (int c = 0; c < MMAS; ++c)
-                  mma_mxf8f6f4_pair<A_HI, B_HI>(d, a_lo + kk * A_KK, b_lo + c * (1024 >> 4) + kk * 2, id0 + ((uint32_t)kk << 4) + ((uint32_t)kk << 29),
-                                          sf + 4 * u, sf + 8 + 8 * c, (k | kk | c) ? 1u : 0u);
-              }
-          }
-        };
-        // ---- ramp: blocks join as the epilogue hands back their regions; those that have joined run ahead by up to the ring ----
-        uint32_t joined = 0;
-        int kt = 0;                                    // next k step of the joined blocks; the others have issued none
-        const uint32_t s_base = s;
-        while (ok && (joined != live || kt == 0)) {
-          if (joined && kt < STAGES && kt < KT) {
-            ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_SF(s), ph, ctl, 612));
-            if (!ok) break;
-            tc_fence_after();
-#pragma unroll
-            for (int u = 0; u < 2; ++u)
-              if ((joined >> u) & 1u) issue(u, kt, s);
-            if (joined == live) elect_commit_pair(BAR_EMPTY(s));
-            ++kt;
-            if (++s == (uint32_t)STAGES) { s = 0; ph ^= 1u; }
-          }
-          const bool full = kt >= STAGES || kt >= KT;  // nothing to do for the joined blocks: wait for the next one
-#pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            if (!((live >> u) & 1u) || ((joined >> u) & 1u)) continue;
-            const uint32_t par = (acc_ph >> reg[u]) & 1u;
-            bool got;
-            if (full || joined == 0) got = ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_ACC_EMPTY(reg[u]), par, ctl, 613));
-            else got = __all_sync(0xFFFFFFFFu, mbar_test(BAR_ACC_EMPTY(reg[u]), par));             // (try_wait would sleep)
-            if (!got) break;
-            tc_fence_after();
-            joined |= 1u << u;
-            acc_ph ^= 1u << reg[u];
-            uint32_t sk = s_base;
-            for (int k = 0; k < kt; ++k) {             // catch up with the others
-              issue(u, k, sk);
-              if (joined == live) elect_commit_pair(BAR_EMPTY(sk));
-              if (++sk == (uint32_t)STAGES) sk = 0;
-            }
-            if (full) break;
-          }
-        }
-        // ---- steady state ---------------------------------------------------------------------------------------
-        const bool in_ramp = kt == KT;
-        bool ready = false;                            // the next step was complete when the last one was issued
-        for (; ok && kt < KT; ++kt) {
-          if (!__all_sync(0xFFFFFFFFu, ready)) ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_SF(s), ph, ctl, 612));
+        const int units = blocks_of(tile).units;
+        const bool mine = u < units;
+        // (The ring has at most as many stages as a tile k steps: when one warp starts a tile the other is past its wait for a
+        // region of the tile before, so a region's barrier is never two uses behind.)
+        const uint32_t use = (blk + (uint32_t)u) / (uint32_t)a.regions, reg = blk + (uint32_t)u - use * (uint32_t)a.regions;
+        const uint32_t d = tmem_base + reg * (uint32_t)a.reg_cols;
+        blk += (uint32_t)units;
+        uint32_t id0 = 0;
+        for (int kt = 0; kt < KT; ++kt) {
+          ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_SF(s), ph, ctl, 612));
           if (!ok) break;
-          tc_fence_after();
-#pragma unroll
-          for (int u = 0; u < 2; ++u)
-            if ((live >> u) & 1u) {
-              issue(u, kt, s);
-              if (kt == KT - 1) elect_commit_pair(BAR_ACC_FULL(reg[u]));
+          if (mine) {
+            if (kt == 0) {
+              id0 = pair_idesc(__shfl_sync(0xFFFFFFFFu, s_cols[tc & 7u], 0) * (FORM == PP_SIDE ? 2 : 1), 0);     // left by the scale loader
+              ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_ACC_EMPTY(reg), (use & 1u) ^ 1u, ctl, 613));
+              if (!ok) break;
             }
+            tc_fence_after();
+            const uint32_t st = sbase + s * (uint32_t)a.stage_bytes;
+            const uint32_t sf = tmem_base + SF_BASE + s * SF_COLS<FORM>;
+            const uint32_t a_lo = DESC_LO | ((st + (uint32_t)u * (128 * 128)) >> 4);
+            const uint32_t b_lo = DESC_LO | ((st + OFF_X) >> 4);
+            const int kk_live = kt < k_whole ? 4 : (p.K - kt * 128 + 31) >> 5;
+            auto mma = [&](int kk, int c) {
+              mma_mxf8f6f4_pair<A_HI, B_HI>(d, a_lo + kk * A_KK, b_lo + c * (1024 >> 4) + kk * 2, id0 + ((uint32_t)kk << 4) + ((uint32_t)kk << 29),
+                                            sf + 4 * u, sf + 8 + 8 * c, (kk | c) ? 1u : (uint32_t)(kt > 0));
+            };
+            // (a step that is whole has no test between its instructions: they must issue in less than the 45-64 cycles that
+            // one of them runs)
+            if (kk_live == 4) {
+#pragma unroll
+              for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+                for (int c = 0; c < MMAS; ++c) mma(kk, c);
+            } else {
+#pragma unroll
+              for (int kk = 0; kk < 4; ++kk)
+                if (kk < kk_live) {
+#pragma unroll
+                  for (int c = 0; c < MMAS; ++c) mma(kk, c);
+                }
+            }
+          }
           elect_commit_pair(BAR_EMPTY(s));
           if (++s == (uint32_t)STAGES) { s = 0; ph ^= 1u; }
-          ready = mbar_test(BAR_SF(s), ph);
         }
-        if (ok && in_ramp)
-#pragma unroll
-          for (int u = 0; u < 2; ++u)
-            if ((live >> u) & 1u) elect_commit_pair(BAR_ACC_FULL(reg[u]));
-        const uint32_t last = live == 3u ? reg[1] : reg[0];
-        r0 = last + 1 < (uint32_t)a.regions ? last + 1 : 0u;
+        if (ok && mine) elect_commit_pair(BAR_ACC_FULL(reg));
       }
-      // every MMA issued by this warp has retired before tensor memory is freed
+      // every MMA issued by these warps has retired before tensor memory is freed
       elect_commit_pair_local(BAR_DRAIN);
       mbar_wait(BAR_DRAIN, 0, ctl, 614);
     }
@@ -645,17 +602,18 @@ PairPlan pair_plan(const MoeGemmArgs& a) {
 }
 
 // Token columns and weight blocks of a tile, and the form of two-term tokens.  fc1 + fc2, us:
-// - SIDE with 96 columns of tokens up to 224 rows per expert, where TWO with 192 takes over (32 experts of 2880 x 5760: 16 rows
-//   156 and 192, 64 rows 207 and 231, 150 rows 321 and 327, 300 rows 506 and 481; 128 experts, 64 rows: 608 and 659).  SIDE with
-//   64 or 32 columns gains 2 % below 16 rows and loses 3-30 % from 32 on.
+// - SIDE with 96 columns of tokens below 56 rows per expert, TWO with 128 from there on (32 experts of 2880 x 5760: 50 rows 176
+//   and 180, 80 rows 219 and 197, 150 rows 305 and 293, 300 rows 489 and 457; 128 experts, 512 rows: 3157 and 2978).  SIDE with 64
+//   columns reads the weight operand more often and is 0-20 % slower from 32 rows on; TWO with 192 has no third region to go on in
+//   while a tile is drained (150 rows: 336, 512 rows: 3349).
 // - One weight block per tile where twice the tiles still run at a time (8 experts of 512 x 2048, 16 rows: 19 -> 17); beyond, a
 //   tile of two blocks reads the tokens once for both (32 experts, 64 rows: 91 against 105).
 struct PairShape { int nmax, upt, form; };
 PairShape pair_shape(const MoeGemmArgs& a, int terms) {
   const int64_t experts = a.slice_sizes ? a.E : 1, per = a.M / experts;
   PairShape s;
-  s.form = terms == 1 ? PP_ONE : (per < 224 ? PP_SIDE : PP_TWO);
-  s.nmax = s.form == PP_SIDE ? 96 : 192;
+  s.form = terms == 1 ? PP_ONE : (per < 56 ? PP_SIDE : PP_TWO);
+  s.nmax = s.form == PP_SIDE ? 96 : s.form == PP_TWO ? 128 : 192;
   const int64_t active = experts < a.M ? experts : a.M;
   s.upt = active * (per / s.nmax + 1) * cdiv64(a.N, 256) <= moe_sm_count() / 2 ? 1 : 2;
   return s;
@@ -671,9 +629,10 @@ int launch_mx_pair(const GemmParams& p, PairParams q, const PairShape& shape, co
   q.stages = (PP_SMEM - 1024 - PP_CTL) / q.stage_bytes;
   if (q.stages > PP_MAX_STAGES) q.stages = PP_MAX_STAGES;
   while ((TMEM_COLS - q.stages * SF_COLS<FORM>) / q.reg_cols < 2) --q.stages;
+  if (q.stages > q.KT) q.stages = q.KT;               // see the MMA warps
   q.regions = (TMEM_COLS - q.stages * SF_COLS<FORM>) / q.reg_cols;
   if (q.regions > PP_MAX_REGIONS) q.regions = PP_MAX_REGIONS;
-  MOE_CHECK_ARG(q.stages >= 2, "moe_grouped_gemm: block-scaled pair tile does not fit shared memory");
+  MOE_CHECK_ARG(q.stages >= 1, "moe_grouped_gemm: block-scaled pair tile does not fit shared memory");
   // every expert has at most ceil(rows / nmax) token tiles
   const int64_t experts = args.slice_sizes ? (args.E < args.M ? args.E : args.M) : 0;
   const int64_t tiles = (experts + cdiv64(args.M, q.nmax)) * cdiv64(cdiv64(q.NB, 2), q.upt);

@@ -102,7 +102,7 @@ int moe_route(const void* logits, int dtype, int64_t T, int E, int k, int apply_
               void* workspace, size_t workspace_bytes, void* stream);
 
 /* moe_route on fp32 logits that also writes, for every expert-sorted position, its token row and its routing weight (the
- * gather index and the gammas of the layer's two products), in the same launches.                                  */
+ * gather index and the gammas of the layer's two products), in the same launches; weight_of_position may be NULL.    */
 int moe_route_positions(const float* logits, int64_t T, int E, int k, int apply_softmax, int64_t ld_logits,
                         float* vals, int64_t ld_vals, int16_t* indx, int64_t ld_indx,
                         uint32_t* bitmatrix, int64_t bm_stride_row, int64_t bm_stride_word,

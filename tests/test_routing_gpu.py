@@ -183,3 +183,24 @@ def test_fused_route_equals_separate_entry_points(T, E, k, dtype, device, monkey
     assert torch.equal(md.col_sum.cpu().long(), col_sum_o.long())
     assert torch.equal(md.col_sorted_indx.cpu().long(), col_sorted_o.long())
     assert torch.equal(md.row_sorted_indx.cpu().long(), row_sorted_o.long())
+
+
+@pytest.mark.parametrize("T", [2, 32, 33, 64, 65, 128, 129, 256])
+@pytest.mark.parametrize("E, k", [(8, 8), (20, 1), (100, 2), (256, 16)])
+def test_small_batch_routing_at_its_lane_splits(T, E, k, device):
+    """Up to 256 tokens route in one launch with 32, 16, 8 or 4 lanes per token; whole numbers, so equal to the oracle."""
+    g = torch.Generator().manual_seed(T * 1000 + E + k)
+    # ties; + 0.0 leaves no negative zeros, which the selection has always ordered below zero and the oracle equal to it
+    logits = (torch.randn(T, E, generator=g) * 4).round() / 4 + 0.0
+    ragged, gather_idx, scatter_idx, sp = routing(logits.to(device), k)
+    vals_o, indx_o, _ = oracle.topk_oracle(logits, k, apply_softmax=True)
+    col_sum_o, col_sorted_o, row_sorted_o = oracle.bitmatrix_metadata_oracle(indx_o, E)
+    assert torch.equal(sp.indx.cpu().long(), indx_o.long())
+    # exps of 2 ulp, a sum of k terms, a division
+    torch.testing.assert_close(sp.vals.cpu(), vals_o.float(), rtol=(k + 6) * 2 ** -23, atol=0)
+    assert torch.equal(ragged.slice_sizes.cpu().long(), col_sum_o.long())
+    assert torch.equal(scatter_idx.cpu().long(), col_sorted_o.long())
+    assert torch.equal(sp.mask_metadata.row_sorted_indx.cpu().long(), row_sorted_o.long())
+    assert torch.equal(gather_idx.cpu().long(), col_sorted_o.long() // k)
+    ref = make_ragged_tensor_metadata(ragged.slice_sizes, T * k)
+    assert torch.equal(ragged.block_offs_data, ref.block_offs_data) and torch.equal(ragged.block_schedule_data, ref.block_schedule_data)

@@ -73,7 +73,8 @@ int64_t pad512(int64_t n) { return std::max<int64_t>(cdiv(n, 512) * 512, 512); }
 int64_t max_blocks16(int64_t E, int64_t n) { return n <= E ? n : E - 1 + cdiv(n + 1 - E, 16); }
 
 // ---- routing -----------------------------------------------------------------------------------------------------
-// -> vals, indx, bitmatrix view [T, words], col_sum, col_sorted, row_sorted, slice_offs, block_offs, block_schedule
+// -> vals, indx, bitmatrix view [T, words], col_sum, col_sorted, row_sorted, slice_offs, block_offs, block_schedule, token of
+// every position (float logits; else None)
 py::tuple route(const Tensor& logits, int64_t k, bool softmax) {
   need_cuda(logits);
   const int64_t T = logits.size(0), E = logits.size(1), n = T * k;
@@ -83,18 +84,27 @@ py::tuple route(const Tensor& logits, int64_t k, bool softmax) {
   const int64_t mnb = max_blocks16(E, n), lo = pad512(E + 1), ls = pad512(mnb);
   // the index arrays and the metadata rows are parts of one buffer; every row of the metadata starts on 2 KB
   const size_t ws = lib.moe_route_workspace(T, (int)E, (int)k);
-  Tensor buf = empty({5 * lo + 4 * ls + 2 * n + E}, at::kInt, logits), work = empty({(int64_t)std::max<size_t>(ws, 4)}, at::kByte, logits);
+  Tensor buf = empty({5 * lo + 4 * ls + 3 * n + E}, at::kInt, logits), work = empty({(int64_t)std::max<size_t>(ws, 4)}, at::kByte, logits);
   Tensor offs = buf.narrow(0, 0, 5 * lo).view({5, lo}).narrow(1, 0, E + 1);
   Tensor sched = buf.narrow(0, 5 * lo, 4 * ls).view({4, ls}).narrow(1, 0, mnb);
   Tensor col_sorted = buf.narrow(0, 5 * lo + 4 * ls, n), row_sorted = buf.narrow(0, 5 * lo + 4 * ls + n, n);
-  Tensor col_sum = buf.narrow(0, 5 * lo + 4 * ls + 2 * n, E);
+  Tensor tokens = buf.narrow(0, 5 * lo + 4 * ls + 2 * n, n), col_sum = buf.narrow(0, 5 * lo + 4 * ls + 3 * n, E);
   int32_t* b = buf.data_ptr<int32_t>();
-  check(lib.moe_route(logits.data_ptr(), code, T, (int)E, (int)k, softmax, logits.stride(0), vals.data_ptr(), k,
+  const bool positions = code == MOE_F32;
+  if (positions)
+    check(lib.moe_route_positions(logits.data_ptr<float>(), T, (int)E, (int)k, softmax, logits.stride(0), vals.data_ptr<float>(), k,
+                                  indx.data_ptr<int16_t>(), k, (uint32_t*)bm.data_ptr(), bm.stride(0), bm.stride(1),
+                                  col_sum.data_ptr<int32_t>(), col_sorted.data_ptr<int32_t>(), row_sorted.data_ptr<int32_t>(), b, b + lo,
+                                  lo, b + 5 * lo, ls, mnb, tokens.data_ptr<int32_t>(), nullptr, work.data_ptr(), ws, stream()),
+          "moe_route_positions");
+  else
+    check(lib.moe_route(logits.data_ptr(), code, T, (int)E, (int)k, softmax, logits.stride(0), vals.data_ptr(), k,
                       indx.data_ptr<int16_t>(), k, (uint32_t*)bm.data_ptr(), bm.stride(0), bm.stride(1), col_sum.data_ptr<int32_t>(),
                       col_sorted.data_ptr<int32_t>(), row_sorted.data_ptr<int32_t>(), b, b + lo, lo, b + 5 * lo, ls, mnb, work.data_ptr(),
                       ws, stream()),
         "moe_route");
-  return py::make_tuple(vals, indx, bm, col_sum, col_sorted, row_sorted, offs.select(0, 0), offs.narrow(0, 1, 4), sched);
+  return py::make_tuple(vals, indx, bm, col_sum, col_sorted, row_sorted, offs.select(0, 0), offs.narrow(0, 1, 4), sched,
+                        positions ? py::cast(tokens) : py::none());
 }
 
 // -> col_sum, col_sorted, row_sorted

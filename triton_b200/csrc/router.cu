@@ -266,10 +266,7 @@ router_topk_kernel(const RouterParams p, const __grid_constant__ CUtensorMap x_m
       }
       TopK<K> tk = sub[0];
 #pragma unroll
-      for (int u = 1; u < NSUB; ++u) {
-#pragma unroll
-        for (int i = 0; i < K; ++i) tk.push_any(sub[u].key[i], sub[u].idx[i]);
-      }
+      for (int u = 1; u < NSUB; ++u) tk.merge(sub[u].key, sub[u].idx);
       tk.merge_lanes(P);
       if (live && part == 0) rt_store_row<K>(p, row, tk);
     }

@@ -113,48 +113,56 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) topk_kernel(
   }
 }
 
-// Four lanes per token row (k in {1, 2, 4, 8, 16}, every row valid, no provided indices).  Lane `part` of a row's four
-// walks the chunks of four experts c = part, part + 4, ... with best-k lists in registers (two lists side by side for
-// k <= 4: independent insertion chains), the four lanes' lists meet by shuffles, lane 0 writes values and indices and the
-// four lanes share the bitmatrix words.  With HIST the block (256 rows) also counts its picks per expert into
+// Four lanes per token row (k in {1, 2, 4, 8, 16}, every row valid, no provided indices; `parts` lanes for small batches).
+// Lane `part` of a row's four walks the chunks of four experts c = part, part + 4, ... with best-k lists in registers (two
+// lists side by side for k <= 4: independent insertion chains), the four lanes' lists meet by shuffles, lane 0 writes values
+// and indices and the four lanes share the bitmatrix words.  With HIST the block (256 rows) also counts its picks per expert into
 // partial[block][e], the first pass of the expert sort.  The warp-per-row kernel above spends its time in k rounds of
 // 64-bit warp reductions per row: 19.6 us for 16384 x 128 logits against about 5 us here.
 template <typename T, int K>
-__device__ __forceinline__ TopK<K> quad_select(const T* __restrict__ x, int E, int part) {
+__device__ __forceinline__ TopK<K> quad_select(const T* __restrict__ x, int E, int part, int parts = 4) {
   constexpr int NL = K <= 4 ? 2 : 1;
   TopK<K> sub[NL];
-  for (int c0 = part; c0 * 4 < E; c0 += 4 * NL) {
-    float v[NL][4];
+  float v[NL][4];
+  auto load = [&](int c0, float (&to)[NL][4]) {
 #pragma unroll
     for (int u = 0; u < NL; ++u)
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const int e = (c0 + 4 * u) * 4 + i;
-        v[u][i] = e < E ? to_f32<T>(x[e]) : 0.0f;
+        const int e = (c0 + parts * u) * 4 + i;
+        to[u][i] = e < E ? to_f32<T>(x[e]) : 0.0f;
       }
+  };
+  load(part, v);
+  for (int c0 = part; c0 * 4 < E; c0 += parts * NL) {
+    float next[NL][4];                             // in flight while this chunk is inserted
+    load(c0 + parts * NL, next);
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int u = 0; u < NL; ++u) {               // the lists alternate; each takes its experts in ascending order
-        const int e = (c0 + 4 * u) * 4 + i;
+        const int e = (c0 + parts * u) * 4 + i;
         if (e < E) sub[u].push(v[u][i], e);
       }
+#pragma unroll
+    for (int u = 0; u < NL; ++u)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[u][i] = next[u][i];
   }
   TopK<K> tk = sub[0];
 #pragma unroll
-  for (int u = 1; u < NL; ++u)
-#pragma unroll
-    for (int i = 0; i < K; ++i) tk.push_any(sub[u].key[i], sub[u].idx[i]);
-  tk.merge_lanes(4);
+  for (int u = 1; u < NL; ++u) tk.merge(sub[u].key, sub[u].idx);
+  tk.merge_lanes(parts);
   return tk;
 }
 
-// values (softmax over the picks), indices, bitmatrix words of one row; `hist` (shared memory, may be NULL) counts the picks
+// values (softmax over the picks), indices, bitmatrix words of one row; `hist` (shared memory, may be NULL) counts the picks,
+// s_pick and s_val (shared memory, may be NULL) keep the row's picks and values for the block
 template <typename T, int K>
 __device__ __forceinline__ void quad_store(const TopK<K>& tk, int part, int64_t row, int E, int apply_softmax, T* __restrict__ vals,
                                            int64_t ld_vals, int16_t* __restrict__ indx, int64_t ld_indx,
                                            uint32_t* __restrict__ bitmatrix, int64_t bm_stride_row, int64_t bm_stride_word,
-                                           int32_t* hist) {
+                                           int32_t* hist, int parts = 4, int16_t* s_pick = nullptr, float* s_val = nullptr) {
   if (part == 0) {
     float v[K];
 #pragma unroll
@@ -174,10 +182,14 @@ __device__ __forceinline__ void quad_store(const TopK<K>& tk, int part, int64_t 
       vals[row * ld_vals + i] = from_f32<T>(v[i]);
       indx[row * ld_indx + i] = (int16_t)tk.idx[i];
       if (hist) atomicAdd(&hist[tk.idx[i]], 1);
+      if (s_pick) {
+        s_pick[i] = (int16_t)tk.idx[i];
+        s_val[i] = to_f32<T>(from_f32<T>(v[i]));
+      }
     }
   }
   const int words = (E + 31) >> 5;
-  for (int w = part; w < words; w += 4) {
+  for (int w = part; w < words; w += parts) {
     uint32_t bits = 0;
 #pragma unroll
     for (int i = 0; i < K; ++i)
@@ -370,7 +382,7 @@ __device__ __forceinline__ void rank_block(const int16_t* __restrict__ indx, int
       col_sorted[pos] = (int32_t)flat;
       if (out.token) {
         out.token[pos] = (int32_t)token;
-        out.weight[pos] = out.vals[token * out.ld_vals + slot];
+        if (out.weight) out.weight[pos] = out.vals[token * out.ld_vals + slot];
       }
     }
   }
@@ -815,53 +827,101 @@ __global__ void __launch_bounds__(1024) route_scan_ragged_kernel(const int32_t* 
 
 // The whole routing step of a small batch (at most 256 tokens, at most 256 experts, k in {1, 2, 4, 8, 16}) in ONE launch
 // of five blocks of 1024 threads that do not wait on one another: every block selects the top-k of every row for itself
-// (four lanes per row; 128 KB of logits at most) and counts the picks; block 0 stores the selection, the expert offsets
-// (ragged row 0) and the positions of the entries, blocks 1..4 each build the block_offs row and the schedule of one
-// block size.  Repeating the selection five times costs less than what it replaces: a chain of kernel boundaries
-// (three launches) or of block barriers (one block doing all five rows took 20 us at 64 tokens).
+// (`parts` lanes per row: all that 1024 threads can give a row, up to a warp; 128 KB of logits at most) and counts the picks;
+// block 0 stores the selection, the expert offsets (ragged row 0) and the positions of the entries, blocks 1..4 each build
+// the block_offs row and the schedule of one block size.  Repeating the selection five times costs less than what it
+// replaces: a chain of kernel boundaries (three launches) or of block barriers (one block doing all five rows took 20 us at
+// 64 tokens).  What is left is a chain of latencies: with four lanes per row whatever their number and the picks read back
+// from global memory by one warp per 32 tokens, 1 and 64 tokens of 128 experts took 11.6 and 12.7 us in a graph, so 4.3 and 8.3.
 template <typename T, int K>
 __global__ void __launch_bounds__(1024) route_small_kernel(
-    const T* __restrict__ logits, int64_t ld_logits, int64_t T_rows, int E, int apply_softmax, T* __restrict__ vals,
+    const T* __restrict__ logits, int64_t ld_logits, int T_rows, int E, int parts, int apply_softmax, T* __restrict__ vals,
     int64_t ld_vals, int16_t* __restrict__ indx, int64_t ld_indx, uint32_t* __restrict__ bitmatrix, int64_t bm_stride_row,
     int64_t bm_stride_word, int32_t* __restrict__ col_sum, int32_t* __restrict__ col_sorted, int32_t* __restrict__ row_sorted,
     int32_t* __restrict__ slice_offs, int32_t* __restrict__ block_offs, int64_t ld_block_offs, int32_t* __restrict__ block_sched,
     int64_t ld_sched, int64_t n_sched, const PerPosition out) {
-  extern __shared__ int32_t s_mem[];            // [E + 1] sizes, [E + 1] scan input, [E + 1] offsets, [E] expert offsets, [32][E] counters
+  // [E + 1] sizes, [E + 1] scan input, [E + 1] offsets, [n] values, [n] picks (int16), [warps in use][E] counters (uint16)
+  extern __shared__ int32_t s_mem[];
   __shared__ int32_t s_warp[33];
+  const int n = T_rows * K;
   int32_t* s_size = s_mem;
   int32_t* s_nb = s_size + (E + 1);
   int32_t* s_offs = s_nb + (E + 1);
-  int32_t* s_col = s_offs + (E + 1);
-  int32_t* s_cnt = s_col + E;
-  const int role = blockIdx.x;
+  float* s_val = reinterpret_cast<float*>(s_offs + (E + 1));
+  int16_t* s_pick = reinterpret_cast<int16_t*>(s_val + n);
+  uint16_t* s_cnt = reinterpret_cast<uint16_t*>(s_pick + n);
+  const int role = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rounds = (n + 1023) >> 10, per = rounds * 32, warps = (n + per - 1) / per;      // entries of a warp, warps with entries
   for (int e = threadIdx.x; e <= E; e += blockDim.x) s_size[e] = 0;
+  if (role == 0)
+    for (int i = threadIdx.x; i < warps * E; i += blockDim.x) s_cnt[i] = 0;
   __syncthreads();
   {
-    const int part = threadIdx.x & 3;
-    const int64_t row = threadIdx.x >> 2;
+    const int part = threadIdx.x & (parts - 1), row = threadIdx.x / parts;
     const bool live = row < T_rows;
-    const T* x = logits + (live ? row : 0) * ld_logits;
-    const TopK<K> tk = quad_select<T, K>(x, E, part);
-    if (live) {
-      if (role == 0) {
-        quad_store<T, K>(tk, part, row, E, apply_softmax, vals, ld_vals, indx, ld_indx, bitmatrix, bm_stride_row,
-                         bm_stride_word, s_size);
-      } else if (part == 0) {
+    if (__any_sync(0xFFFFFFFFu, live)) {
+      const T* x = logits + (live ? row : 0) * ld_logits;
+      const TopK<K> tk = quad_select<T, K>(x, E, part, parts);
+      if (live) {
+        if (role == 0) {
+          quad_store<T, K>(tk, part, row, E, apply_softmax, vals, ld_vals, indx, ld_indx, bitmatrix, bm_stride_row,
+                           bm_stride_word, s_size, parts, s_pick + row * K, s_val + row * K);
+        } else if (part == 0) {
 #pragma unroll
-        for (int i = 0; i < K; ++i) atomicAdd(&s_size[tk.idx[i]], 1);
+          for (int i = 0; i < K; ++i) atomicAdd(&s_size[tk.idx[i]], 1);
+        }
       }
     }
   }
-  __syncthreads();                               // the picks are counted (block 0: and in global memory)
+  __syncthreads();                               // the picks are counted (block 0: and stored)
   if (role > 0) {
     ragged_row(role, s_size, E, s_nb, s_offs, s_warp, slice_offs, nullptr, block_offs, ld_block_offs, block_sched, ld_sched, n_sched);
     return;
   }
   for (int e = threadIdx.x; e < E; e += blockDim.x) col_sum[e] = s_size[e];
+  // stable expert-major positions: a warp ranks `per` entries in order, on top of the counts of the warps before it
+  uint16_t* my = s_cnt + warp * E;
+  if (warp < warps)
+    for (int r = 0; r < rounds; ++r) {
+      const int j = warp * per + r * 32 + lane, c = j < n ? s_pick[j] : -1;
+      const unsigned peers = __match_any_sync(0xFFFFFFFFu, c);
+      if (c >= 0 && (peers & ((1u << lane) - 1u)) == 0) my[c] += (uint16_t)__popc(peers);
+      __syncwarp();
+    }
   ragged_row(0, s_size, E, s_nb, s_offs, s_warp, slice_offs, nullptr, block_offs, ld_block_offs, block_sched, ld_sched, n_sched);
-  for (int e = threadIdx.x; e < E; e += blockDim.x) s_col[e] = s_offs[e];
+  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+    int run = s_offs[e];
+    for (int w0 = 0; w0 < warps; w0 += 8) {
+      int v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = w0 + u < warps ? s_cnt[(w0 + u) * E + e] : 0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        if (w0 + u < warps) s_cnt[(w0 + u) * E + e] = (uint16_t)run;
+        run += v[u];
+      }
+    }
+  }
   __syncthreads();
-  rank_block(indx, ld_indx, T_rows, E, K, T_rows, nullptr, s_col, 0, col_sorted, row_sorted, s_cnt, out);
+  if (warp >= warps) return;
+  for (int r = 0; r < rounds; ++r) {
+    const int j = warp * per + r * 32 + lane, c = j < n ? s_pick[j] : -1;
+    const unsigned peers = __match_any_sync(0xFFFFFFFFu, c);
+    const int before = __popc(peers & ((1u << lane) - 1u));
+    const int base = c >= 0 ? my[c] : 0;
+    __syncwarp();
+    if (c >= 0 && before == 0) my[c] = (uint16_t)(base + __popc(peers));
+    __syncwarp();
+    if (c >= 0) {
+      const int pos = base + before;
+      row_sorted[j] = pos;
+      col_sorted[pos] = j;
+      if (out.token) {
+        out.token[pos] = j / K;
+        if (out.weight) out.weight[pos] = s_val[j];
+      }
+    }
+  }
 }
 
 constexpr int kRouteSmallTokens = 256;
@@ -893,13 +953,15 @@ static int route_launch(
                 moe_route_workspace(T, E, k));
   cudaStream_t st = (cudaStream_t)stream;
   if (T <= kRouteSmallTokens && (k == 1 || k == 2 || k == 4 || k == 8 || k == 16)) {
-    const size_t smem_s = (size_t)(3 * (E + 1) + E + 32 * E) * sizeof(int32_t);
+    const int n = (int)T * k, warps = (n + 31) / 32 < 32 ? (n + 31) / 32 : 32;
+    const size_t smem_s = (size_t)(3 * (E + 1) + n) * sizeof(int32_t) + (size_t)(n + warps * E) * sizeof(int16_t);   // < 48 KB
+    const int parts = T <= 32 ? 32 : T <= 64 ? 16 : T <= 128 ? 8 : 4;
 #define MOE_ROUTE_SMALL(KK)                                                                                              \
   MOE_DISPATCH_FLOAT(dtype, Tv, {                                                                                         \
-    route_small_kernel<Tv, KK><<<5, 1024, smem_s, st>>>((const Tv*)logits, ld_logits, T, E, apply_softmax, (Tv*)vals, ld_vals, \
-                                                         indx, ld_indx, bitmatrix, bm_stride_row, bm_stride_word, col_sum,  \
-                                                         col_sorted, row_sorted, slice_offs, block_offs, ld_block_offs,     \
-                                                         block_sched, ld_sched, n_sched, out);                              \
+    route_small_kernel<Tv, KK><<<5, 1024, smem_s, st>>>((const Tv*)logits, ld_logits, (int)T, E, parts, apply_softmax,       \
+                                                         (Tv*)vals, ld_vals, indx, ld_indx, bitmatrix, bm_stride_row,       \
+                                                         bm_stride_word, col_sum, col_sorted, row_sorted, slice_offs,       \
+                                                         block_offs, ld_block_offs, block_sched, ld_sched, n_sched, out);   \
   })
     switch (k) {
       case 1: MOE_ROUTE_SMALL(1); break;
@@ -964,7 +1026,7 @@ extern "C" __attribute__((visibility("default"))) int moe_route_positions(
     int32_t* col_sorted, int32_t* row_sorted, int32_t* slice_offs, int32_t* block_offs, int64_t ld_block_offs,
     int32_t* block_sched, int64_t ld_sched, int64_t n_sched, int32_t* token_of_position, float* weight_of_position, void* workspace,
     size_t workspace_bytes, void* stream) {
-  MOE_CHECK_ARG(token_of_position && weight_of_position, "moe_route_positions: NULL pointer");
+  MOE_CHECK_ARG(token_of_position, "moe_route_positions: NULL pointer");
   PerPosition out;
   out.token = token_of_position; out.weight = weight_of_position; out.vals = vals; out.ld_vals = ld_vals;
   return route_launch(logits, MOE_F32, T, E, k, apply_softmax, ld_logits, vals, ld_vals, indx, ld_indx, bitmatrix, bm_stride_row,

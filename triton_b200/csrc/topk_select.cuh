@@ -17,8 +17,8 @@ __device__ __forceinline__ float sel_key_float(uint32_t k) {
 // The K best (value key, expert) pairs, best first.  An insertion compares the candidate with all K places at once
 // (independent compares, then two selects per place) instead of bubbling it down: a thread walks its share of a row
 // alone, so the length of the dependent chain is what the selection costs.  `push` takes experts in ascending order
-// and keeps the earlier of two equal values ahead with a strict compare; `push_any` takes them in any order and
-// compares the expert index too.
+// and keeps the earlier of two equal values ahead with a strict compare; `merge` joins two lists of any experts and
+// compares the expert index too (a third of the instructions of inserting one list into the other).
 template <int K>
 struct TopK {
   uint32_t key[K];
@@ -43,11 +43,27 @@ struct TopK {
     for (int i = 0; i < K; ++i) gt[i] = c > key[i];
     place(c, e, gt);
   }
-  __device__ __forceinline__ void push_any(uint32_t c, int ci) {
-    bool gt[K];
+  __device__ __forceinline__ static bool ahead(uint32_t a, int ai, uint32_t b, int bi) { return a > b || (a == b && ai < bi); }
+  // the best K of this list and another, both best first: place by place the better of one list's i-th and the other's
+  // (K - 1 - i)-th, which leaves a bitonic list to sort (K a power of two)
+  __device__ __forceinline__ void merge(const uint32_t (&k2)[K], const int (&i2)[K]) {
 #pragma unroll
-    for (int i = 0; i < K; ++i) gt[i] = c > key[i] || (c == key[i] && ci < idx[i]);
-    place(c, ci, gt);
+    for (int i = 0; i < K; ++i) {
+      const bool other = ahead(k2[K - 1 - i], i2[K - 1 - i], key[i], idx[i]);
+      key[i] = other ? k2[K - 1 - i] : key[i];
+      idx[i] = other ? i2[K - 1 - i] : idx[i];
+    }
+#pragma unroll
+    for (int s = K / 2; s > 0; s >>= 1)
+#pragma unroll
+      for (int i = 0; i < K; ++i)
+        if ((i & s) == 0) {
+          const bool swap = ahead(key[i + s], idx[i + s], key[i], idx[i]);
+          const uint32_t ka = key[i], kb = key[i + s];
+          const int ia = idx[i], ib = idx[i + s];
+          key[i] = swap ? kb : ka; key[i + s] = swap ? ka : kb;
+          idx[i] = swap ? ib : ia; idx[i + s] = swap ? ia : ib;
+        }
   }
   // the lists of the lanes lane ^ 1, lane ^ 2, ... lane ^ (parts - 1) meet: afterwards every lane of the group holds
   // the best K of the group (parts a power of two, groups aligned in the warp; all 32 lanes must call)
@@ -60,8 +76,7 @@ struct TopK {
         ok_[i] = __shfl_xor_sync(0xFFFFFFFFu, key[i], m);
         oi[i] = __shfl_xor_sync(0xFFFFFFFFu, idx[i], m);
       }
-#pragma unroll
-      for (int i = 0; i < K; ++i) push_any(ok_[i], oi[i]);
+      merge(ok_, oi);
     }
   }
 };

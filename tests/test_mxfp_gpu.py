@@ -131,6 +131,26 @@ def test_strided_axis_tile_edges(shape, dt, device):
         assert torch.equal(bits(want.contiguous())[~nan], bits(got)[~nan])
 
 
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("rows, quant, skip", [(1, 32, 0), (3, 96, 8), (5, 8224, 16), (257, 1024, 0)])
+def test_upcast_store_widths(rows, quant, skip, dt, device):
+    """Stores of 32 bytes where the output allows them, else of 16: outputs that start `skip` elements into rows of a wider
+    matrix; whole bytes, so equal to the oracle."""
+    from triton_b200 import _lib
+    g = torch.Generator().manual_seed(rows + quant)
+    q = torch.randint(0, 256, (rows, quant // 2), generator=g, dtype=torch.uint8)
+    s = torch.randint(100, 150, (rows, quant // 32), generator=g, dtype=torch.uint8)
+    want = oracle.upcast_from_mxfp_oracle(q, s, dt, 1).contiguous()
+    wide = torch.zeros((rows, quant + 32), dtype=dt, device=device)
+    out = wide[:, skip:skip + quant]
+    code = {torch.float32: 0, torch.float16: 1, torch.bfloat16: 2}[dt]
+    qd, sd = q.to(device), s.to(device)
+    _lib.check(_lib.load().moe_upcast_mxfp4(_lib.ptr(qd), _lib.ptr(sd), _lib.ptr(out), code, 1, rows, quant, 0, out.stride(0), 1,
+                                            _lib.stream()), "moe_upcast_mxfp4")
+    assert torch.equal(bits(out.contiguous().cpu()), bits(want))
+    assert not wide[:, :skip].any() and not wide[:, skip + quant:].any()
+
+
 def test_full_size_properties(device):
     """bf16 [8192, 8192], N(0,1) with 1 % of entries x100: checked through size-independent properties --
     a sample of rows against the oracle, idempotence of quantise(dequantise(.)), scales never clip."""

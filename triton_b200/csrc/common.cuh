@@ -56,3 +56,10 @@ template <> __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(flo
     case MOE_BF16: { using T = __nv_bfloat16; __VA_ARGS__; break; }         \
     default: moe_set_error("unsupported dtype %d", (int)(dtype)); return MOE_ERR_ARG; \
   }
+
+// 32 contiguous bytes (aligned to 32), a whole sector, in one store
+__device__ __forceinline__ void st_v8(void* p, const uint4& a, const uint4& b) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b.x),
+               "r"(b.y), "r"(b.z), "r"(b.w)
+               : "memory");
+}

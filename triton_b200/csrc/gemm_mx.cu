@@ -34,6 +34,7 @@
 // Warps: 0 producer (one thread), 1 MMA issue + tensor-memory owner, 2-5 epilogue, 6-9 scale loaders.  Every mbarrier
 // wait is bounded.
 #include "gemm_mx_common.cuh"
+#include <cuda_fp4.h>
 #include <utility>
 
 namespace {
@@ -201,17 +202,15 @@ __global__ void __launch_bounds__(256) mx_pack_x_kernel(const GemmParams p, cons
 // ---- four e2m1 terms -----------------------------------------------------------------------------------------
 // Chunk of the four-term form: row r (r < 4 tb; term t of token j is row t * tb + j) is 64 bytes = 128 e2m1 values, low
 // nibble first, its 16-byte pieces XOR-swizzled with ((r >> 1) & 3) like a 64-byte-swizzled TMA tile; scales as above.
-__device__ __forceinline__ uint32_t f32_to_e2m1(float q) {           // round to nearest, ties to the even code; |q| <= 6
-  const float a = fabsf(q);
-  const uint32_t c = (uint32_t)(a > 0.25f) + (uint32_t)(a >= 0.75f) + (uint32_t)(a > 1.25f) + (uint32_t)(a >= 1.75f) +
-                     (uint32_t)(a > 2.5f) + (uint32_t)(a >= 3.5f) + (uint32_t)(a > 5.0f);
-  return c | ((__float_as_uint(q) >> 28) & 8u);
+// Two values at a time by the conversion instructions (round to nearest, ties to the even code; |q| <= 6 but for Inf, which
+// saturates): with compares and selects per value, and a warp reduction under four masks, the pack of 64 tokens for 128 experts
+// took 13.6-14.4 us, so 10.5-11.1.
+__device__ __forceinline__ uint32_t f32x2_to_e2m1x2(float lo, float hi) {       // `lo` in bits 0..3
+  return (uint32_t)__nv_cvt_float2_to_fp4x2(make_float2(lo, hi), __NV_E2M1, cudaRoundNearest);
 }
-__device__ __forceinline__ float e2m1_to_f32(uint32_t c) {
-  const uint32_t m = c & 7u;
-  // 0, 0.5 | (1 + 0.5 (m & 1)) * 2^((m >> 1) - 1)
-  float v = m < 2u ? 0.5f * (float)m : __uint_as_float(((126u + (m >> 1)) << 23) | ((m & 1u) << 22));
-  return (c & 8u) ? -v : v;
+__device__ __forceinline__ float2 e2m1x2_to_f32x2(uint32_t c) {
+  const __half2_raw h = __nv_cvt_fp4x2_to_halfraw2((__nv_fp4x2_storage_t)c, __NV_E2M1);
+  return __half22float2(__half2(h));
 }
 // e8m0 byte s with 2^(s-127) >= amax / 6, and the exact factors 2^(s-127), 2^(127-s)
 __device__ __forceinline__ void mx4_scale(float amax, uint32_t& sb, float& scale, float& inv) {
@@ -227,7 +226,8 @@ __device__ __forceinline__ void mx4_scale(float amax, uint32_t& sb, float& scale
   inv = __uint_as_float((254u - sb) << 23);
 }
 
-// (A warp per (token block, k step, four rows) with the rows' chains side by side, and dead warps grouped into whole
+// (16 warps over the rows of eight k steps, for a third of the blocks: 2.6 x slower at 64 tokens, the blocks of 16 rows decide;
+// four warps instead of eight: 8 % slower.)  (A warp per (token block, k step, four rows) with the rows' chains side by side, and dead warps grouped into whole
 // CTAs, was tried in place of the loop over rows below: 2.3 x slower.  A row's four-term chain is latency, and four of
 // them in one warp add up where eight warps of a CTA overlap them.)
 __global__ void __launch_bounds__(256) mx_pack_x4_kernel(const GemmParams p, const PackParams a) {
@@ -252,21 +252,25 @@ __global__ void __launch_bounds__(256) mx_pack_x4_kernel(const GemmParams p, con
       v[0] = __uint_as_float(raw.x << 16); v[1] = __uint_as_float(raw.x & 0xFFFF0000u);
       v[2] = __uint_as_float(raw.y << 16); v[3] = __uint_as_float(raw.y & 0xFFFF0000u);
     }
+    const bool nan[4] = {v[0] != v[0], v[1] != v[1], v[2] != v[2], v[3] != v[3]};      // e2m1 has no NaN: such a value counts as 0
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
-      // maximum of the 32-group: the 8 lanes that hold it reduce the bit patterns of their |values| (non-negative floats
-      // order like unsigned integers; NaN patterns rank above Inf and are caught below)
-      float amax = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
-      amax = __uint_as_float(__reduce_max_sync(0xFFu << (lane & 24), __float_as_uint(amax)));
+      // maximum of the 32-group over the 8 lanes that hold it (NaN ranks above Inf where all four values are NaN, and is caught below)
+      uint32_t top = __float_as_uint(fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))));
+#pragma unroll
+      for (int o = 1; o <= 4; o <<= 1) top = max(top, __shfl_xor_sync(0xFFFFFFFFu, top, o));
+      float amax = __uint_as_float(top);
       if (!(amax < 3.0e38f)) amax = t == 0 ? 3.0e38f : 0.0f;       // Inf / NaN in the group: keep the scales finite
       uint32_t sb; float s, inv;
       mx4_scale(amax, sb, s, inv);
       uint32_t codes = 0;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const uint32_t c = f32_to_e2m1(v[i] * inv);
+      for (int i = 0; i < 4; i += 2) {
+        const uint32_t c = f32x2_to_e2m1x2(nan[i] ? 0.0f : v[i] * inv, nan[i + 1] ? 0.0f : v[i + 1] * inv);
         codes |= c << (4 * i);
-        v[i] -= e2m1_to_f32(c) * s;
+        const float2 f = e2m1x2_to_f32x2(c);
+        v[i] -= f.x * s;
+        v[i + 1] -= f.y * s;
       }
       const int rt = t * a.tb + r;
       *reinterpret_cast<uint16_t*>(chunk + rt * 64 + ((g ^ (uint32_t)((rt >> 1) & 3)) << 4) + within) = (uint16_t)codes;

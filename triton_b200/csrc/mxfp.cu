@@ -347,14 +347,18 @@ __device__ __forceinline__ uint4 upcast8_bf16(uint32_t w, uint32_t sb) {
                     __byte_perm(r[2], r[3], 0x7632));
 }
 
+// HBM-bound on its writes: with 16-byte stores (a sector in two) 8192 x 8192 to bf16 took 41.3 us, with a sector per lane 31.7
+// (5.4 TB/s over all 172 MB; a fill of the output alone takes 37.9).
 constexpr int ROWS_UNROLL = 4;
-// contiguous output: thread owns 8 elements (4 input bytes) of each of ROWS_UNROLL chunks per iteration
-template <typename T>
+// contiguous output: thread owns U units of 8 elements (4 input bytes each) of each of ROWS_UNROLL chunks per iteration; a
+// chunk of two units of a 2-byte type, or of one of fp32, leaves as one 32-byte store (WIDE)
+template <typename T, bool WIDE>
 __global__ void __launch_bounds__(256) upcast_rows_kernel(const uint8_t* __restrict__ q,
                                                           const uint8_t* __restrict__ scale, T* __restrict__ out,
                                                           int64_t n_rows, int64_t quant, int64_t outer,
                                                           int64_t so_batch, int64_t so_outer) {
-  const int64_t chunks_per_row = quant >> 3;
+  constexpr int U = WIDE && sizeof(T) == 2 ? 2 : 1;
+  const int64_t chunks_per_row = quant / (8 * U);
   const int64_t total = n_rows * chunks_per_row;
   const int64_t stride = (int64_t)gridDim.x * (ROWS_UNROLL * 256);
   const int64_t tile0 = (int64_t)blockIdx.x * (ROWS_UNROLL * 256);
@@ -364,13 +368,19 @@ __global__ void __launch_bounds__(256) upcast_rows_kernel(const uint8_t* __restr
                                 RowCursor(tile0 + 768 + threadIdx.x, stride, chunks_per_row)};
   const bool one_batch = outer == n_rows;
   for (int64_t tile = tile0; tile < total; tile += stride) {
-    uint32_t w[ROWS_UNROLL], sb[ROWS_UNROLL];
+    uint32_t w[ROWS_UNROLL][U], sb[ROWS_UNROLL];
 #pragma unroll
     for (int u = 0; u < ROWS_UNROLL; ++u) {
       const bool live = tile + u * 256 + threadIdx.x < total;
       const int64_t row = live ? cur[u].row : 0, c = live ? cur[u].c : 0;
-      w[u] = *reinterpret_cast<const uint32_t*>(q + row * (quant >> 1) + c * 4);
-      sb[u] = scale[row * (quant >> 5) + (c >> 2)];
+      const uint8_t* src = q + row * (quant >> 1) + c * (4 * U);
+      if constexpr (U == 2) {
+        const uint2 two = *reinterpret_cast<const uint2*>(src);
+        w[u][0] = two.x; w[u][1] = two.y;
+      } else {
+        w[u][0] = *reinterpret_cast<const uint32_t*>(src);
+      }
+      sb[u] = scale[row * (quant >> 5) + c * U / 4];
     }
 #pragma unroll
     for (int u = 0; u < ROWS_UNROLL; ++u) {
@@ -380,23 +390,30 @@ __global__ void __launch_bounds__(256) upcast_rows_kernel(const uint8_t* __restr
       if (!live) continue;
       int64_t b = 0, o = row;
       if (!one_batch) { b = row / outer; o = row - b * outer; }
-      T* dst = out + b * so_batch + o * so_outer + c * 8;
+      T* dst = out + b * so_batch + o * so_outer + c * (8 * U);
+      uint4 v[U * 8 * sizeof(T) / 16];
+      bool done = false;
       if constexpr (std::is_same<T, __nv_bfloat16>::value) {
         if (sb[u] < 253u) {
-          *reinterpret_cast<uint4*>(dst) = upcast8_bf16(w[u], sb[u]);
-          continue;
+#pragma unroll
+          for (int i = 0; i < U; ++i) v[i] = upcast8_bf16(w[u][i], sb[u]);
+          done = true;
         }
       }
-      const float s = __uint_as_float(sb[u] << 23);
-      const bool nan_scale = sb[u] == 0xFFu;
-      T e[8];
+      if (!done) {
+        const float s = __uint_as_float(sb[u] << 23);
+        const bool nan_scale = sb[u] == 0xFFu;
+        alignas(16) T e[8 * U];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) e[j] = dequant_one<T>((w[u] >> (4 * j)) & 0xFu, s, nan_scale);
-      if constexpr (sizeof(T) == 2) {
-        *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(e);
+        for (int j = 0; j < 8 * U; ++j) e[j] = dequant_one<T>((w[u][j / 8] >> (4 * (j % 8))) & 0xFu, s, nan_scale);
+#pragma unroll
+        for (int i = 0; i < (int)(sizeof(v) / 16); ++i) v[i] = reinterpret_cast<const uint4*>(e)[i];
+      }
+      if constexpr (WIDE) {
+        st_v8(dst, v[0], v[1]);
       } else {
-        *reinterpret_cast<float4*>(dst) = *reinterpret_cast<const float4*>(e);
-        *reinterpret_cast<float4*>(dst + 4) = *reinterpret_cast<const float4*>(e + 4);
+#pragma unroll
+        for (int i = 0; i < (int)(sizeof(v) / 16); ++i) reinterpret_cast<uint4*>(dst)[i] = v[i];
       }
     }
   }
@@ -552,10 +569,16 @@ extern "C" __attribute__((visibility("default"))) int moe_upcast_mxfp4(const uin
     const int64_t align = 16 / (int64_t)sizeof(T);
     const bool rows_ok = so_quant == 1 && ((uintptr_t)out % 16 == 0) && (so_outer % align == 0) &&
                          (so_batch % align == 0) && ((uintptr_t)q % 4 == 0);
-    if (rows_ok) {
+    const bool wide = rows_ok && (uintptr_t)out % 32 == 0 && so_outer % (2 * align) == 0 && so_batch % (2 * align) == 0 &&
+                      (uintptr_t)q % 8 == 0;
+    if (wide) {
+      const int64_t total = batch * outer * (quant * (int64_t)sizeof(T) >> 5);
+      upcast_rows_kernel<T, true><<<grid_for(total, ROWS_UNROLL * 256), 256, 0, st>>>(q, scale, (T*)out, batch * outer, quant, outer,
+                                                                                      so_batch, so_outer);
+    } else if (rows_ok) {
       const int64_t total = batch * outer * (quant >> 3);
-      upcast_rows_kernel<T><<<grid_for(total, ROWS_UNROLL * 256), 256, 0, st>>>(q, scale, (T*)out, batch * outer, quant, outer,
-                                                                  so_batch, so_outer);
+      upcast_rows_kernel<T, false><<<grid_for(total, ROWS_UNROLL * 256), 256, 0, st>>>(q, scale, (T*)out, batch * outer, quant, outer,
+                                                                                       so_batch, so_outer);
     } else if (so_outer == 1 && so_quant % 2 == 0 && so_batch % 2 == 0 && outer % 2 == 0 && (uintptr_t)q % 16 == 0 &&
                (uintptr_t)out % (2 * sizeof(T)) == 0 && col_tiles(batch, outer, quant) < 2147483647LL) {
       const int groups = (int)(quant >> 5);

@@ -296,6 +296,8 @@ int moe_ep_pull_index(const int32_t* col_sorted, const int16_t* expt_indx, const
  * output buffers that moe_gather_reduce_rows_peers reads.  Replaces the index arithmetic of distributed.py:256-283. */
 int moe_ep_combine_index(const int32_t* row_sorted, const int16_t* expt_indx, const int32_t* owner, int64_t lo,
                          int64_t n_local, int64_t rows_per_peer, int32_t* out, void* stream);
+/* Two copies of device memory in one launch (16-byte aligned pointers, any sizes; the second may be empty). */
+int moe_copy2(void* dst0, const void* src0, int64_t bytes0, void* dst1, const void* src1, int64_t bytes1, void* stream);
 int moe_gather_rows(const void* src, int64_t ld_src, const int32_t* row_indx, int64_t n_rows_out, int64_t row_bytes,
                     void* dst, int64_t ld_dst, void* stream);
 /* moe_gather_rows over rows that live on several devices: global row g = row_indx[r] is row g % rows_per_peer of

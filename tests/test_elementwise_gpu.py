@@ -142,3 +142,27 @@ def test_gather_reduce_over_peer_buffers(device):
     for j in range(1, k):
         want = want + picked[:, j]                    # same order of fp32 additions as the kernel
     assert torch.equal(out, want.bfloat16())
+
+
+@pytest.mark.parametrize("n0, n1", [(1, 0), (16, 15), (33, 16), (4096 * 16 + 5, 7), (0, 1 << 20)])
+def test_copy2(n0, n1, device):
+    """Two copies in one launch: whole 16-byte pieces and the bytes after them; what lies behind stays."""
+    from triton_b200 import _lib
+    src = [torch.randint(0, 255, (n + 64,), dtype=torch.uint8, device=device) for n in (n0, n1)]
+    dst = [torch.full((n + 64,), 255, dtype=torch.uint8, device=device) for n in (n0, n1)]
+    _lib.check(_lib.load().moe_copy2(_lib.ptr(dst[0]), _lib.ptr(src[0]), n0, _lib.ptr(dst[1]), _lib.ptr(src[1]), n1, _lib.stream()))
+    for d, s, n in zip(dst, src, (n0, n1)):
+        assert torch.equal(d[:n], s[:n]) and (d[n:] == 255).all()
+
+
+@pytest.mark.parametrize("E, K, N", [(1, 32, 1), (2, 96, 129), (3, 2880, 300), (2, 12320, 130)])
+def test_scale_layouts_from_either_storage_order(E, K, N, device):
+    """Scales stored K-innermost go through shared memory (up to 12288 of K), others word by word: the same bytes."""
+    from triton_b200.tensor import convert_layout, wrap_torch_tensor
+    from triton_b200.tensor_details.layout import B200BlockScaledScaleLayout, B200MXScaleLayout
+    rows = torch.randint(0, 255, (E, N, K // 32), dtype=torch.uint8, device=device)
+    for layout in (B200MXScaleLayout, B200BlockScaledScaleLayout):
+        a = convert_layout(wrap_torch_tensor(rows.transpose(1, 2)), layout())
+        b = convert_layout(wrap_torch_tensor(rows.transpose(1, 2).contiguous()), layout())
+        assert torch.equal(a.storage.data, b.storage.data)
+

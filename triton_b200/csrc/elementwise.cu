@@ -314,6 +314,36 @@ extern "C" __attribute__((visibility("default"))) int moe_reduce(const void* x, 
   return MOE_ERR_UNSUPPORTED;
 }
 
+// Two device-to-device copies in one launch (the inputs of a replayed step: two copies were two launches of 2 us each).
+namespace {
+__global__ void __launch_bounds__(256) copy2_kernel(uint8_t* __restrict__ d0, const uint8_t* __restrict__ s0, int64_t n0,
+                                                    uint8_t* __restrict__ d1, const uint8_t* __restrict__ s1, int64_t n1) {
+  const int64_t v0 = n0 >> 4, total = v0 + (n1 >> 4);
+  for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < total; i += (int64_t)gridDim.x * 256) {
+    if (i < v0) reinterpret_cast<uint4*>(d0)[i] = reinterpret_cast<const uint4*>(s0)[i];
+    else reinterpret_cast<uint4*>(d1)[i - v0] = reinterpret_cast<const uint4*>(s1)[i - v0];
+  }
+  if (blockIdx.x == 0 && threadIdx.x < 32) {           // the last n % 16 bytes
+    const int64_t t = threadIdx.x & 15;
+    if (threadIdx.x < 16) { if (t < (n0 & 15)) d0[v0 * 16 + t] = s0[v0 * 16 + t]; }
+    else if (t < (n1 & 15)) d1[(n1 & ~(int64_t)15) + t] = s1[(n1 & ~(int64_t)15) + t];
+  }
+}
+}  // namespace
+
+extern "C" __attribute__((visibility("default"))) int moe_copy2(void* dst0, const void* src0, int64_t bytes0, void* dst1, const void* src1,
+                                                                int64_t bytes1, void* stream) {
+  MOE_CHECK_ARG(bytes0 >= 0 && bytes1 >= 0, "moe_copy2: negative extent");
+  MOE_CHECK_ARG((bytes0 == 0 || (dst0 && src0)) && (bytes1 == 0 || (dst1 && src1)), "moe_copy2: NULL pointer");
+  MOE_CHECK_ARG((((uintptr_t)dst0 | (uintptr_t)src0 | (uintptr_t)dst1 | (uintptr_t)src1) & 15) == 0,
+                "moe_copy2: pointers must be 16-byte aligned");
+  if (bytes0 + bytes1 == 0) return MOE_OK;
+  copy2_kernel<<<grid_for(bytes0 / 16 + bytes1 / 16 + 1, 256), 256, 0, (cudaStream_t)stream>>>(
+      (uint8_t*)dst0, (const uint8_t*)src0, bytes0, (uint8_t*)dst1, (const uint8_t*)src1, bytes1);
+  MOE_CHECK_LAUNCH();
+  return MOE_OK;
+}
+
 extern "C" __attribute__((visibility("default"))) int moe_gather_rows(const void* src, int64_t ld_src, const int32_t* row_indx, int64_t n_rows_out,
                                int64_t row_bytes, void* dst, int64_t ld_dst, void* stream) {
   MOE_CHECK_ARG(n_rows_out >= 0 && row_bytes >= 0, "moe_gather_rows: negative extent");

@@ -17,7 +17,7 @@ struct Lib {
 #define MOE_HOST_FUNCTIONS(X)                                                                                            \
   X(moe_last_error) X(moe_route) X(moe_route_positions) X(moe_route_workspace) X(moe_grouped_gemm) X(moe_gemm_mx_workspace_bytes) \
   X(moe_reduce) X(moe_downcast_mxfp4) X(moe_upcast_mxfp4) X(moe_bitmatrix_metadata) X(moe_bitmatrix_metadata_workspace) \
-  X(moe_router_topk) X(moe_router_topk_workspace_bytes)
+  X(moe_router_topk) X(moe_router_topk_workspace_bytes) X(moe_copy2)
 #define X(name) decltype(&::name) name = nullptr;
   MOE_HOST_FUNCTIONS(X)
 #undef X
@@ -390,9 +390,39 @@ py::tuple router(const Tensor& x, const Tensor& wg, const OptTensor& bg, int64_t
   return py::make_tuple(vals, indx, bm);
 }
 
+// ---- inputs and result of a replayed step --------------------------------------------------------------------------
+bool plain_copy(const Tensor& dst, const Tensor& src) {
+  return src.is_cuda() && src.device() == dst.device() && src.scalar_type() == dst.scalar_type() && src.sizes() == dst.sizes() &&
+         src.is_contiguous() && dst.is_contiguous() && (uintptr_t)src.data_ptr() % 16 == 0 && (uintptr_t)dst.data_ptr() % 16 == 0;
+}
+
+// src -> dst of both pairs: one launch where they are plain copies on the current device, else what copy_ does
+void copy2(const Tensor& dst0, const Tensor& src0, const Tensor& dst1, const Tensor& src1) {
+  if (plain_copy(dst0, src0) && plain_copy(dst1, src1) && dst0.device() == dst1.device() &&
+      dst0.device().index() == c10::cuda::current_device()) {
+    check(lib.moe_copy2(dst0.data_ptr(), src0.data_ptr(), (int64_t)src0.nbytes(), dst1.data_ptr(), src1.data_ptr(), (int64_t)src1.nbytes(),
+                        stream()),
+          "moe_copy2");
+    return;
+  }
+  Tensor d0 = dst0, d1 = dst1;
+  d0.copy_(src0, true);
+  d1.copy_(src1, true);
+}
+
+Tensor copy_of(const Tensor& src) {
+  if (!src.is_contiguous() || !src.is_cuda() || (uintptr_t)src.data_ptr() % 16 != 0 || src.device().index() != c10::cuda::current_device())
+    return src.clone();
+  Tensor out = at::empty(src.sizes(), src.options());
+  check(lib.moe_copy2(out.data_ptr(), src.data_ptr(), (int64_t)src.nbytes(), nullptr, nullptr, 0, stream()), "moe_copy2");
+  return out;
+}
+
 }  // namespace
 
 PYBIND11_MODULE(_host, m) {
+  m.def("copy2", &copy2);
+  m.def("copy_of", &copy_of);
   m.def("bind", &bind);
   m.def("route", &route);
   m.def("bitmatrix_metadata", &bitmatrix_metadata);

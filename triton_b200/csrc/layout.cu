@@ -71,6 +71,46 @@ __global__ void __launch_bounds__(256) to_tiles_values(const uint8_t* __restrict
   }
 }
 
+// Scales stored K-innermost and dense ([E][N][K / 32], what the quantiser returns along K), either layout: a block takes the rows of
+// one weight block, contiguous in memory, through shared memory and writes their tiles of all k steps.  A word per thread read four
+// lone bytes at the pitch of a row (16 x 2880 x 5760: 15.5 us, so 8.5).  MX: the block-scaled order [E][k step][block].
+constexpr int SCALE_ROWS_SMEM = 48 * 1024;
+template <bool MX>
+__global__ void __launch_bounds__(256) scales_from_rows(const uint8_t* __restrict__ s, int64_t s_stride_e, int groups, int N, int NB, int KT,
+                                                        uint32_t* __restrict__ out) {
+  extern __shared__ uint32_t s_words[];              // [rows][groups] bytes
+  const int nb = blockIdx.x % NB, e = blockIdx.x / NB, rows = min(TN, N - nb * TN);
+  const uint8_t* src = s + (int64_t)e * s_stride_e + (int64_t)nb * TN * groups;       // 4-byte aligned: TN is a multiple of 4
+  const int bytes = rows * groups;
+  for (int i = threadIdx.x; i < bytes >> 2; i += 256) s_words[i] = reinterpret_cast<const uint32_t*>(src)[i];
+  uint8_t* s_bytes = reinterpret_cast<uint8_t*>(s_words);
+  if ((int)threadIdx.x < (bytes & 3)) s_bytes[(bytes & ~3) + threadIdx.x] = src[(bytes & ~3) + threadIdx.x];
+  __syncthreads();
+  for (int i = threadIdx.x; i < KT * TN; i += 256) {
+    const int c = i & (TN - 1), kt = i >> 7;
+    const int r = MX ? (c >> 2) + 32 * (c & 3) : c;  // block-scaled word: (r % 32) * 4 + r / 32
+    uint32_t w = 0;
+    if (r < rows) {
+#pragma unroll
+      for (int g = 0; g < 4; ++g)
+        if (kt * 4 + g < groups) w |= (uint32_t)s_bytes[r * groups + kt * 4 + g] << (8 * g);
+    }
+    const int64_t tile = MX ? ((int64_t)e * KT + kt) * NB + nb : ((int64_t)e * NB + nb) * KT + kt;
+    out[tile * TN + c] = w;
+  }
+}
+// false: the scales are laid out in some other way
+template <bool MX>
+bool launch_scales_from_rows(const uint8_t* s, int64_t s_stride_e, int64_t s_stride_k, int64_t s_stride_n, int E, int K, int N, int NB, int KT,
+                             uint32_t* out, cudaStream_t st) {
+  const int groups = K / 32, smem = TN * groups;
+  if (K % 32 || s_stride_k != 1 || s_stride_n != groups || s_stride_e % 4 || (uintptr_t)s % 4 || smem > SCALE_ROWS_SMEM ||
+      (int64_t)E * NB >= 2147483647LL)
+    return false;
+  scales_from_rows<MX><<<(unsigned)(E * NB), 256, smem, st>>>(s, s_stride_e, groups, N, NB, KT, out);
+  return true;
+}
+
 __global__ void __launch_bounds__(256) to_b200_scales(const uint8_t* __restrict__ s, int64_t s_stride_e,
                                                       int64_t s_stride_k, int64_t s_stride_n, int E, int K, int N,
                                                       int NT, int KT, uint32_t* __restrict__ out) {
@@ -161,8 +201,9 @@ extern "C" __attribute__((visibility("default"))) int moe_weight_layout_to_b200(
     MOE_CHECK_LAUNCH();
   }
   if (scale) {
-    to_b200_scales<<<grid_for((int64_t)E * NT * KT * TN), 256, 0, st>>>(scale, s_stride_e, s_stride_k, s_stride_n, E, K,
-                                                                       N, NT, KT, (uint32_t*)out_scales);
+    if (!launch_scales_from_rows<false>(scale, s_stride_e, s_stride_k, s_stride_n, E, K, N, NT, KT, (uint32_t*)out_scales, st))
+      to_b200_scales<<<grid_for((int64_t)E * NT * KT * TN), 256, 0, st>>>(scale, s_stride_e, s_stride_k, s_stride_n, E, K,
+                                                                         N, NT, KT, (uint32_t*)out_scales);
     MOE_CHECK_LAUNCH();
   }
   return MOE_OK;
@@ -256,8 +297,9 @@ extern "C" __attribute__((visibility("default"))) int moe_weight_layout_to_b200m
     MOE_CHECK_LAUNCH();
   }
   if (scale) {
-    to_b200mx_scales<<<grid_for((int64_t)E * NB * KT * TN), 256, 0, st>>>(scale, s_stride_e, s_stride_k, s_stride_n, E, K,
-                                                                         N, NB, KT, (uint32_t*)out_scales);
+    if (!launch_scales_from_rows<true>(scale, s_stride_e, s_stride_k, s_stride_n, E, K, N, NB, KT, (uint32_t*)out_scales, st))
+      to_b200mx_scales<<<grid_for((int64_t)E * NB * KT * TN), 256, 0, st>>>(scale, s_stride_e, s_stride_k, s_stride_n, E, K,
+                                                                           N, NB, KT, (uint32_t*)out_scales);
     MOE_CHECK_LAUNCH();
   }
   return MOE_OK;

@@ -57,14 +57,14 @@ class MoeLayerWeights:
         block-scaled copy.  Few rows per expert (decode) stream the packed weights straight into the MMA, bound by HBM.
         With more rows the block-scaled pair kernel first re-lays the tokens out (4 bytes per element written and read
         against 2 n_out operations), which a wide product repays and a narrow one does not; measured against the bf16
-        kernel: 64 rows per expert 1.3-1.7 x faster for n_out >= 2000 and 0.9 x at 512-1024; 1024 rows per expert
-        1.05-1.2 x faster from 2880 on, 0.9 x at 2048."""
+        kernel: 64 rows per expert 1.3-1.7 x faster for n_out >= 2000 and 1.0-1.2 x at 512-1440; 256 rows 0.8 x at 512;
+        1024 rows per expert 1.05-1.2 x faster from 2880 on, 0.9 x at 2048."""
         if self.w1_bs is None:
             return False
         if n_rows <= self.block_scaled_max_rows_per_expert * self.n_expts:
             return True
         n_out = self.b1.shape[1] if n_out is None else n_out
-        return n_out >= (1280 if n_rows < 512 * self.n_expts else 2560)
+        return n_rows <= 80 * self.n_expts or n_out >= (1280 if n_rows < 512 * self.n_expts else 2560)
 
     def fc_weights(self, n_rows: int):
         one = (self.w1_bs, self.w1_bs_scale) if self.use_block_scaled(n_rows, self.b1.shape[1]) else (self.w1, self.w1_scale)
@@ -207,11 +207,12 @@ class GraphedMoeLayer:
         return self.z
 
     def __call__(self, x, logits):
-        self.x.copy_(x, non_blocking=True)
-        self.logits.copy_(logits, non_blocking=True)
+        # both inputs in one native call and launch: as two copy_ and a clone around the replay they took 19 us of a step
+        host = _lib.host()
+        host.copy2(self.x, x, self.logits, logits)
         self.graph.replay()
         # a copy, so that the caller may still be reading one result (a download, say) while the next step replays
-        return self.z.clone()
+        return host.copy_of(self.z) if isinstance(self.z, torch.Tensor) else self.z.clone()
 
 
 class HostStreamingLayer:

@@ -75,11 +75,6 @@ inline int make_w_map(const MoeGemmArgs& a, int KT, int NB, bool packed, int n_b
 
 // ---- copies issued by a warp that runs its loop as a whole: the instruction is guarded by an election next to it and its operands
 // live in uniform registers (issued by a single thread of a divergent branch, a copy cost about 150 cycles)
-__device__ __forceinline__ void elect_expect_tx(uint32_t bar, uint32_t bytes) {
-  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xFFFFFFFF;\n\t@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(bar),
-               "r"(bytes)
-               : "memory");
-}
 __device__ __forceinline__ void elect_bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile(
       "{\n\t.reg .pred q;\n\telect.sync _|q, 0xFFFFFFFF;\n\t"

@@ -51,12 +51,6 @@ __device__ __forceinline__ void elect_commit_pair_local(uint32_t bar) {
       : "memory");
 }
 
-// The whole MMA warp runs the issue loop and one lane's predicate guards the instruction.  The operands of tcgen05.mma live in
-// uniform registers: computed by a single thread of a divergent branch, each takes a move from a vector register first, and
-// an MMA cost 170-190 cycles to issue.  Of a shared-memory descriptor only the low word varies (start address, 16-byte units).
-constexpr uint32_t DESC_LO = 1u << 16;                               // leading byte offset (unused for swizzled K-major)
-constexpr uint32_t DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29); // 8-row groups 1024 B apart, sm_100, 128-byte swizzle
-
 // ---- token tiles -------------------------------------------------------------------------------------------------
 // prefix (shared memory): [E + 1] tiles of the experts before, [E] rows at MAX_PREFIX_EXPERTS + 1, [E] first rows after them
 constexpr int PAIR_PREFIX_INTS = 3 * MAX_PREFIX_EXPERTS + 1;

@@ -85,7 +85,7 @@ gemm_tc_kernel(const GemmParams p, const int64_t grid_m_static, const __grid_con
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const uint32_t sbase = smem_u32(smem);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;     // warp-uniform for the compiler
   // 256-row tiles of consecutive token rows are fetched by TMA tile copies (x_map), everything else by cp.async
   const bool use_tma = MH == 2 && p.gather_indx == nullptr;
   // second epilogue group (see the epilogue role): only where the loader warps are free and the epilogue is heavy
@@ -151,7 +151,7 @@ gemm_tc_kernel(const GemmParams p, const int64_t grid_m_static, const __grid_con
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *s_tmem;
+  const uint32_t tmem_base = __shfl_sync(0xFFFFFFFFu, *s_tmem, 0);
 
   // ---- tile schedule shared by every role -----------------------------------------------------------
   const int NT128 = (p.N + HALF_N - 1) / HALF_N;        // weight tiles along n in memory
@@ -164,55 +164,53 @@ gemm_tc_kernel(const GemmParams p, const int64_t grid_m_static, const __grid_con
 
   if (warp == 0) {
     // ================================= MMA issuer ===================================================
-    if (lane == 0) {
-      uint32_t it = 0, tc = 0;
-      bool ok = true;
-      for (int64_t tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, ++tc) {
-        int halves = 1, rows_cur = HALF_M;
-        {
-          int e; int64_t row0;
-          map_tile<MH>(p, s_prefix, tile / NT, e, row0, rows_cur);
-          halves = (MH == 2 && rows_cur > HALF_M) ? 2 : 1;
-        }
-        const int nh_live = min(NH, NT128 - (int)(tile % NT) * NH);
-        // MH == 1 swaps the operands: the dequantised weight tile is the M = 128 operand and the token tile the
-        // N operand, with N = the tile's rows rounded up to 16, so that a tile of a few tokens costs a few columns
-        // of MMA time instead of a full 128 x 128 product.  The accumulator is then [weight row][token].
-        const int n_tok = max(16, (min(rows_cur, HALF_M) + 15) & ~15);
-        const uint32_t idesc = make_idesc(MH == 1 ? n_tok : nh_live * HALF_N);
-        const uint32_t ab = tc % ACC_BUFS;
-        ok = mbar_wait(BAR_ACC_EMPTY(ab), ((tc / ACC_BUFS) & 1u) ^ 1u, ctl, 101);
-        if (!ok) break;
-        tc_fence_after();
-        const uint32_t d_tmem = tmem_base + ab * C::ACC_COLS;
-        for (int kt = 0; kt < KT; ++kt, ++it) {
-          const int s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1u;
-          ok = mbar_wait(BAR_A_FULL(s), ph, ctl, 102);
-          ok = ok && mbar_wait(BAR_B_FULL(s), ph, ctl, 103);
-          if (!ok) break;
-          fence_proxy_async();          // the A tile was written by cp.async (generic proxy) of other threads
-          tc_fence_after();
-          const uint64_t adesc = make_desc(sbase + C::OFF_A + s * C::A_STAGE_BYTES);
-          const uint64_t bdesc = make_desc(sbase + C::OFF_B + s * B_STAGE_BYTES);
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk) {
-            if constexpr (MH == 1)
-              mma_bf16(d_tmem, bdesc + (uint64_t)(kk * 2), adesc + (uint64_t)(kk * 2), idesc, (kt | kk) ? 1u : 0u);
-            else
-              mma_bf16(d_tmem, adesc + (uint64_t)(kk * 2), bdesc + (uint64_t)(kk * 2), idesc, (kt | kk) ? 1u : 0u);
-            if (MH == 2 && halves == 2)
-              mma_bf16(d_tmem + NH * HALF_N, adesc + (uint64_t)((SUBTILE_BYTES >> 4) + kk * 2),
-                       bdesc + (uint64_t)(kk * 2), idesc, (kt | kk) ? 1u : 0u);
-          }
-          mma_commit(BAR_AB_EMPTY(s));
-        }
-        if (ok) mma_commit(BAR_ACC_FULL(ab));
+    uint32_t it = 0, tc = 0;
+    bool ok = true;
+    for (int64_t tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, ++tc) {
+      int halves = 1, rows_cur = HALF_M;
+      {
+        int e; int64_t row0;
+        map_tile<MH>(p, s_prefix, tile / NT, e, row0, rows_cur);
+        rows_cur = __shfl_sync(0xFFFFFFFFu, rows_cur, 0);
+        halves = (MH == 2 && rows_cur > HALF_M) ? 2 : 1;
       }
-      // make sure every MMA issued by this thread has retired before tensor memory is freed
-      mma_commit(BAR_DRAIN);
-      mbar_wait(BAR_DRAIN, 0, ctl, 104);
+      const int nh_live = min(NH, NT128 - (int)(tile % NT) * NH);
+      // MH == 1 swaps the operands: the dequantised weight tile is the M = 128 operand and the token tile the
+      // N operand, with N = the tile's rows rounded up to 16, so that a tile of a few tokens costs a few columns
+      // of MMA time instead of a full 128 x 128 product.  The accumulator is then [weight row][token].
+      const int n_tok = max(16, (min(rows_cur, HALF_M) + 15) & ~15);
+      const uint32_t idesc = make_idesc(MH == 1 ? n_tok : nh_live * HALF_N);
+      const uint32_t ab = tc % ACC_BUFS;
+      ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_ACC_EMPTY(ab), ((tc / ACC_BUFS) & 1u) ^ 1u, ctl, 101));
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t d_tmem = tmem_base + ab * C::ACC_COLS;
+      for (int kt = 0; kt < KT; ++kt, ++it) {
+        const int s = it % STAGES;
+        const uint32_t ph = (it / STAGES) & 1u;
+        ok = mbar_wait(BAR_A_FULL(s), ph, ctl, 102);
+        ok = __all_sync(0xFFFFFFFFu, ok && mbar_wait(BAR_B_FULL(s), ph, ctl, 103));
+        if (!ok) break;
+        fence_proxy_async();          // the A tile was written by cp.async (generic proxy) of other threads
+        tc_fence_after();
+        const uint32_t a_lo = DESC_LO | ((sbase + C::OFF_A + s * C::A_STAGE_BYTES) >> 4);
+        const uint32_t b_lo = DESC_LO | ((sbase + C::OFF_B + s * B_STAGE_BYTES) >> 4);
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+          if constexpr (MH == 1)
+            elect_mma_bf16(d_tmem, b_lo + kk * 2, a_lo + kk * 2, idesc, (kt | kk) ? 1u : 0u);
+          else
+            elect_mma_bf16(d_tmem, a_lo + kk * 2, b_lo + kk * 2, idesc, (kt | kk) ? 1u : 0u);
+          if (MH == 2 && halves == 2)
+            elect_mma_bf16(d_tmem + NH * HALF_N, a_lo + (SUBTILE_BYTES >> 4) + kk * 2, b_lo + kk * 2, idesc, (kt | kk) ? 1u : 0u);
+        }
+        elect_commit(BAR_AB_EMPTY(s));
+      }
+      if (ok) elect_commit(BAR_ACC_FULL(ab));
     }
+    // make sure every MMA issued by this warp has retired before tensor memory is freed
+    elect_commit(BAR_DRAIN);
+    mbar_wait(BAR_DRAIN, 0, ctl, 104);
     __syncwarp();
   } else if (warp == 1) {
     // ================================= weight producer =================================================

@@ -83,7 +83,7 @@ router_topk_kernel(const RouterParams p, const __grid_constant__ CUtensorMap x_m
   __shared__ int s_abort;
   __shared__ int s_last;
   __shared__ float s_bias[256];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;     // warp-uniform for the compiler
   const int STAGES = p.stages;
   const uint32_t X_BYTES = RT_BLOCK_T * 128u, W_BYTES = (uint32_t)p.n_mma * 128u;
   const uint32_t stage_bytes = X_BYTES + ((W_BYTES + 1023u) & ~1023u);
@@ -114,7 +114,7 @@ router_topk_kernel(const RouterParams p, const __grid_constant__ CUtensorMap x_m
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = s_tmem;
+  const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, s_tmem, 0);
 
   const int64_t blk = blockIdx.x;
   const int split = blockIdx.y;
@@ -122,46 +122,41 @@ router_topk_kernel(const RouterParams p, const __grid_constant__ CUtensorMap x_m
   const int n_steps = kt1 - kt0;
 
   if (warp == 0) {
-    if (lane == 0) {
-      bool ok = true;
-      int it = 0;
-      for (; it < n_steps && ok; ++it) {
-        const int s = it % STAGES;
-        ok = mbar_wait(BAR_EMPTY(s), ((it / STAGES) & 1u) ^ 1u, ctl, 801);
-        if (!ok) break;
-        const uint32_t st = sbase + (uint32_t)s * stage_bytes;
-        mbar_expect_tx(BAR_FULL(s), X_BYTES + W_BYTES);
-        // token blocks start at different k steps: CTAs that run side by side do not all ask for the same Wg tile
-        const int kt = kt0 + (int)((it + blk * 5) % n_steps);
-        tma_tile_2d(st, &x_map, kt * 64, (int)(blk * RT_BLOCK_T), BAR_FULL(s));
-        tma_tile_2d(st + X_BYTES, &w_map, kt * 64, 0, BAR_FULL(s));
-      }
-      if (!ok) {
-        const int lo = it > STAGES ? it - STAGES : 0;
-        for (int j = lo; j < it; ++j)
-          for (uint32_t i = 0; i < (1u << 16) && !mbar_test(BAR_FULL(j % STAGES), (j / STAGES) & 1u); ++i) __nanosleep(64);
-      }
+    bool ok = true;
+    int it = 0;
+    for (; it < n_steps && ok; ++it) {
+      const int s = it % STAGES;
+      ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_EMPTY(s), ((it / STAGES) & 1u) ^ 1u, ctl, 801));
+      if (!ok) break;
+      const uint32_t st = sbase + (uint32_t)s * stage_bytes;
+      elect_expect_tx(BAR_FULL(s), X_BYTES + W_BYTES);
+      // token blocks start at different k steps: CTAs that run side by side do not all ask for the same Wg tile
+      const int kt = kt0 + (int)((it + blk * 5) % n_steps);
+      elect_tile_2d(st, &x_map, kt * 64, (int)(blk * RT_BLOCK_T), BAR_FULL(s));
+      elect_tile_2d(st + X_BYTES, &w_map, kt * 64, 0, BAR_FULL(s));
+    }
+    if (!ok && lane == 0) {
+      const int lo = it > STAGES ? it - STAGES : 0;
+      for (int j = lo; j < it; ++j)
+        for (uint32_t i = 0; i < (1u << 16) && !mbar_test(BAR_FULL(j % STAGES), (j / STAGES) & 1u); ++i) __nanosleep(64);
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      bool ok = true;
-      const uint32_t idesc = make_idesc(p.n_mma);
-      for (int it = 0; it < n_steps && ok; ++it) {
-        const int s = it % STAGES;
-        ok = mbar_wait(BAR_FULL(s), (it / STAGES) & 1u, ctl, 802);
-        if (!ok) break;
-        tc_fence_after();
-        const uint32_t st = sbase + (uint32_t)s * stage_bytes;
-        const uint64_t adesc = make_desc(st), bdesc = make_desc(st + X_BYTES);
+    bool ok = true;
+    const uint32_t idesc = make_idesc(p.n_mma);
+    for (int it = 0; it < n_steps && ok; ++it) {
+      const int s = it % STAGES;
+      ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_FULL(s), (it / STAGES) & 1u, ctl, 802));
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t st = sbase + (uint32_t)s * stage_bytes;
+      const uint32_t a_lo = DESC_LO | (st >> 4), b_lo = DESC_LO | ((st + X_BYTES) >> 4);
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk)
-          mma_bf16(tmem, adesc + (uint64_t)(kk * 2), bdesc + (uint64_t)(kk * 2), idesc, (it | kk) ? 1u : 0u);
-        mma_commit(BAR_EMPTY(s));
-      }
-      mma_commit(BAR_ACC);              // arrives when every MMA above has retired
-      if (!ok) mbar_wait(BAR_ACC, 0, ctl, 803);
+      for (int kk = 0; kk < 4; ++kk) elect_mma_bf16(tmem, a_lo + kk * 2, b_lo + kk * 2, idesc, (it | kk) ? 1u : 0u);
+      elect_commit(BAR_EMPTY(s));
     }
+    elect_commit(BAR_ACC);              // arrives when every MMA above has retired
+    if (!ok) mbar_wait(BAR_ACC, 0, ctl, 803);
     __syncwarp();
   } else {
     // ---- selection: 16 warps ------------------------------------------------------------------------------

@@ -31,7 +31,7 @@
 //   tokens      one bulk copy of a chunk the pack kernel below prepared per (token block, k step): the e4m3 rows in
 //               the swizzled operand layout followed by their 512 B of scales;
 //   scales -> tensor memory through registers (tcgen05.st by four loader warps), then MB x 4 MMAs of K = 32.
-// Warps: 0 producer (one thread), 1 MMA issue + tensor-memory owner, 2-5 epilogue, 6-9 scale loaders.  Every mbarrier
+// Warps: 0 producer, 1 MMA issue + tensor-memory owner, 2-5 epilogue, 6-9 scale loaders.  Every mbarrier
 // wait is bounded.
 #include "gemm_mx_common.cuh"
 #include <cuda_fp4.h>
@@ -73,7 +73,8 @@ struct MxMaps {
 // blocks; tile = (weight group, token block) with token blocks varying fastest, dealt out round robin, so that CTAs
 // running at the same time share a weight group (large problems: the group is read from HBM once).  (Equal contiguous
 // ranges of weight blocks per CTA, which leave no partly filled last wave, were measured 5-12 % slower at 16 and 64
-// tokens: they cut more tiles short of MB blocks, and a k step costs about the same whatever it carries.  Slices of K per
+// tokens and, after the issuing warps got cheaper, 0-10 %: they cut more tiles short of MB blocks, and a k step costs about the same
+// whatever it carries.  Slices of K per
 // tile with fp32 partial sums in global memory -- red.global.add, the slice that arrives last runs the epilogue -- were
 // correct and 20-35 % slower at 4 to 64 tokens: 48 scalar reductions per thread and slice, their fence and the counter
 // round trip take longer than a slice of a few k steps, and the epilogue warps become the bottleneck.)

@@ -404,3 +404,32 @@ def test_pair_kernel_non_finite_tokens(value, tiled, device):
     keep = torch.arange(64) != 5
     ref = oracle.matmul_oracle(x[keep].float(), wdeq, None, torch.tensor([63], dtype=torch.int32), out_dtype=torch.float32)
     assert oracle.rel_l2(ref, y[keep].float()) < 1e-2
+
+
+@pytest.mark.parametrize("tiled", [True, False])
+def test_pair_kernel_expert_of_more_rows_than_a_schedule_entry_counts(tiled, device):
+    """An entry of the block schedule counts 65536 blocks of 16 rows inside an expert; the rows beyond are packed too.  (Two
+    turns of the counter, with experts before and after; one group of k, so that the case is small.)"""
+    from triton_b200.tensor_details.layout import B200MXScaleLayout, B200MXValueLayout
+    g = torch.Generator().manual_seed(11)
+    sizes = [40, 2 * 65536 * 16 + 50, 0, 33]
+    E, K, N, M = len(sizes), 32, 64, sum(sizes)
+    wq, ws, wdeq = quantised_weights(E, K, N, g)
+    gd = torch.Generator(device=device).manual_seed(11)
+    x = torch.randn(M, K, device=device, generator=gd).bfloat16()
+    md = tb.make_ragged_tensor_metadata(torch.tensor(sizes, dtype=torch.int32, device=device), M)
+    if tiled:
+        w, s = (convert_layout(wrap_torch_tensor(wq.to(device), dtype=FP4), B200MXValueLayout()),
+                convert_layout(wrap_torch_tensor(ws.to(device)), B200MXScaleLayout()))
+    else:
+        w, s = to_block_scaled(wq, ws, device)
+    with tb.scoped_opt_flags_constraints({"kernel": "mx"} if tiled else {"block_m": 256}):
+        y = tb.matmul(x, w, None, md, precision_config=tb.PrecisionConfig(b_mx_scale=s, b_microblock_size=32, out_dtype=torch.float32))
+    tb.matmul_check_status()
+    row = 0
+    for e, n in enumerate(sizes):
+        ref = x[row:row + n].double() @ wdeq[e].to(device).double()
+        if n:
+            # an fp32 sum of 32 exact products, the second term's underflow 2^-23 of the group's maximum
+            assert ((y[row:row + n] - ref).norm(dim=1) <= 2e-5 * ref.norm(dim=1) + 1e-6).all(), e
+        row += n

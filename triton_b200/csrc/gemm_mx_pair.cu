@@ -99,7 +99,11 @@ __device__ __forceinline__ bool pack_block(const GemmParams& p, int64_t pid, int
   const uint32_t ent = (uint32_t)p.block_sched[pid];
   if (ent == 0xFFFFFFFFu) return false;
   e = (int)(ent & 0xFFFFu);
-  const int first = (int)(ent >> 16) * 16, off = p.slice_offs[e];
+  // An entry holds 16 bits of the block's place inside its expert.  The blocks of an expert are neighbours in the schedule, so
+  // every entry of the same expert 65536 places (2^20 rows) further back is one more turn of the counter.
+  int first = (int)(ent >> 16) * 16;
+  for (int64_t back = pid - 65536; back >= 0 && (p.block_sched[back] & 0xFFFF) == e; back -= 65536) first += 65536 * 16;
+  const int off = p.slice_offs[e];
   row0 = (int64_t)off + first;
   prow0 = padded_base(e, off) + first;
   rows = min(16, p.slice_sizes[e] - first);

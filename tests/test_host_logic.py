@@ -274,3 +274,14 @@ def test_weight_file_round_trip_on_cpu(tmp_path):
     bad.write_bytes(b"not a weight file at all")
     with pytest.raises(ValueError):
         read_header(bad)
+
+
+@pytest.mark.parametrize("T, E", [(50, 128), (1, 5), (33, 40), (32, 32)])
+def test_bit_tensor_equals_the_checked_construction(T, E):
+    """The mask every routing call makes without checks is the one `wrap_torch_tensor` returns."""
+    from triton_b200.tensor import BIT, bit_tensor
+    words, t_pad = (E + 31) // 32, (T + 31) // 32 * 32
+    bm = torch.zeros(words, t_pad, dtype=torch.int32).transpose(0, 1)[:T]
+    got, want = bit_tensor(bm, T, E), wrap_torch_tensor(bm, dtype=BIT, shape=[T, E], shape_max=[T, None])
+    assert (got.shape, got.shape_max, got.dtype, got.storage.layout) == (want.shape, want.shape_max, want.dtype, want.storage.layout)
+    assert got.storage.data is bm

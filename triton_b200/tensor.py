@@ -88,7 +88,7 @@ def bit_tensor(bm, T, E):
     """BIT tensor [T, E] over the top-k kernels' bitmatrix view: what `wrap_torch_tensor(bm, dtype=BIT, shape=[T, E],
     shape_max=[T, None])` returns, without its checks (it is made on every routing call)."""
     t = Tensor.__new__(Tensor)
-    t.storage, t.dtype, t.shape, t.shape_max = Storage(bm, _BIT_LAYOUT), BIT, [T, E], [T, bm.shape[1]]
+    t.storage, t.dtype, t.shape, t.shape_max = Storage(bm, _BIT_LAYOUT), BIT, [T, E], [T, E]
     return t
 
 

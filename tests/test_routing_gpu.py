@@ -204,3 +204,22 @@ def test_small_batch_routing_at_its_lane_splits(T, E, k, device):
     assert torch.equal(gather_idx.cpu().long(), col_sorted_o.long() // k)
     ref = make_ragged_tensor_metadata(ragged.slice_sizes, T * k)
     assert torch.equal(ragged.block_offs_data, ref.block_offs_data) and torch.equal(ragged.block_schedule_data, ref.block_schedule_data)
+
+
+@pytest.mark.parametrize("call", ["row count", "reduce output", "router weight", "router bias"])
+def test_host_tensors_are_refused(call, device):
+    """A tensor in host memory beside device tensors is refused, not handed to a kernel."""
+    from triton_b200 import reduce, router_topk
+    x = torch.randn(64, 64, device=device).bfloat16()
+    wg = torch.randn(8, 64).bfloat16().t()
+    with pytest.raises(ValueError, match="CUDA tensors only"):
+        if call == "row count":
+            sp = topk(torch.randn(64, 8, device=device), 2)
+            mask = wrap_torch_tensor(sp.mask.storage.data, dtype=BIT, shape=[torch.tensor(40, dtype=torch.int32), 8], shape_max=[64, 8])
+            make_bitmatrix_metadata(sp.indx, mask)
+        elif call == "reduce output":
+            reduce(x.view(8, 8, 64), 1, y=torch.empty(8, 64, dtype=torch.bfloat16))
+        elif call == "router weight":
+            router_topk(x, wg, None, 2)
+        else:
+            router_topk(x, wg.to(device), torch.zeros(8), 2)

@@ -120,6 +120,7 @@ py::tuple route(const Tensor& logits, int64_t k, bool softmax) {
 // -> col_sum, col_sorted, row_sorted
 py::tuple bitmatrix_metadata(const Tensor& indx, int64_t E, const OptTensor& n_rows) {
   need_cuda(indx);
+  if (n_rows) need_cuda(*n_rows);
   const int64_t T = indx.size(0), k = indx.size(1), n = T * k;
   const size_t ws = lib.moe_bitmatrix_metadata_workspace(T, (int)E, (int)k);
   const int64_t at_work = cdiv(2 * n + E, 64) * 64;
@@ -375,6 +376,7 @@ Tensor upcast(const Tensor& q_, const Tensor& s_, py::object dtype, int64_t axis
 // sum over `dim` without mask or scale; y is the caller's output or None
 Tensor reduce(const Tensor& x, int64_t dim, const OptTensor& y_, py::object y_dtype) {
   need_cuda(x);
+  if (y_) need_cuda(*y_);
   const int64_t a = dim == 0 ? 1 : 0, b = dim == 2 ? 1 : 2;
   Tensor y = y_ ? *y_ : empty({x.size(a), x.size(b)}, torch::python::detail::py_object_to_dtype(y_dtype), x);
   if (y.numel() > 0)
@@ -388,6 +390,8 @@ Tensor reduce(const Tensor& x, int64_t dim, const OptTensor& y_, py::object y_dt
 // -> vals, indx, bitmatrix view; wg in the kernel's memory order, `scratch` zero and large enough (or None)
 py::tuple router(const Tensor& x, const Tensor& wg, const OptTensor& bg, int64_t k, bool softmax, bool round_bf16, const OptTensor& logits,
                  const OptTensor& scratch, int64_t scratch_bytes, const Tensor& status) {
+  need_cuda(x); need_cuda(wg);
+  if (bg) need_cuda(*bg);
   const int64_t T = x.size(0), K = x.size(1), E = wg.size(1);
   Tensor vals = empty({T, k}, round_bf16 ? at::kBFloat16 : at::kFloat, x), indx = empty({T, k}, at::kShort, x);
   const int64_t t_pad = cdiv(T, 32) * 32, words = cdiv(E, 32);

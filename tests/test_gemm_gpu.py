@@ -408,3 +408,15 @@ def test_layer_in_one_call_equals_the_operators(tokens, E, k, dtype, device):
         many = moe_layer_forward(x, logits, weights, k, gemm_timer=_NoTimer)
         tb.matmul_check_status()
         assert torch.equal(one, many)
+
+
+def test_layer_with_a_bias_of_the_wrong_width_is_refused(device):
+    """As the operators refuse it: nothing reads past the end of a bias row."""
+    from triton_b200.moe import moe_layer_forward
+    from triton_b200.testing import make_synthetic_layer
+    x, logits = torch.randn(9, 512, device=device).bfloat16(), torch.randn(9, 8, device=device)
+    for name in ("b1", "b2"):
+        lw = make_synthetic_layer(8, 512, 256, device, seed=3, block_scaled=True)
+        setattr(lw, name, getattr(lw, name)[:, :-32].contiguous())
+        with pytest.raises(AssertionError):
+            moe_layer_forward(x, logits, lw, 2)

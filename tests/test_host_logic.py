@@ -285,3 +285,56 @@ def test_bit_tensor_equals_the_checked_construction(T, E):
     got, want = bit_tensor(bm, T, E), wrap_torch_tensor(bm, dtype=BIT, shape=[T, E], shape_max=[T, None])
     assert (got.shape, got.shape_max, got.dtype, got.storage.layout) == (want.shape, want.shape_max, want.dtype, want.storage.layout)
     assert got.storage.data is bm
+
+
+def _layer_on_cpu(E=3, d=64, ff=96, block_scaled=True):
+    from triton_b200.moe import MoeLayerWeights
+    from triton_b200.tensor import UINT8, Storage, Tensor
+    from triton_b200.tensor_details.layout import (B200BlockScaledScaleLayout, B200BlockScaledValueLayout, B200MXScaleLayout,
+                                                   B200MXValueLayout)
+
+    def pair(K, N, value, scale):
+        n = E * ((K + 127) // 128) * ((N + 127) // 128)
+        return (Tensor(Storage(torch.zeros(n * 8192, dtype=torch.uint8), value), dtype=FP4, shape=[E, K, N]),
+                Tensor(Storage(torch.zeros(n * 512, dtype=torch.uint8), scale), dtype=UINT8, shape=[E, K // 32, N]))
+
+    w1, s1 = pair(d, 2 * ff, B200MXValueLayout(), B200MXScaleLayout())
+    w2, s2 = pair(ff, d, B200MXValueLayout(), B200MXScaleLayout())
+    lw = MoeLayerWeights(w1, s1, torch.zeros(E, 2 * ff), w2, s2, torch.zeros(E, d))
+    if block_scaled:
+        lw.w1_bs, lw.w1_bs_scale = pair(d, 2 * ff, B200BlockScaledValueLayout(), B200BlockScaledScaleLayout())
+        lw.w2_bs, lw.w2_bs_scale = pair(ff, d, B200BlockScaledValueLayout(), B200BlockScaledScaleLayout())
+    return lw
+
+
+@pytest.mark.parametrize("block_scaled", [False, True])
+@pytest.mark.parametrize("fault", ["narrow b1", "narrow b2", "short b2", "width of w1", "depth of w2", "scale layout", "second scale layout"])
+def test_layer_in_one_call_leaves_unfitting_weights_to_the_operators(block_scaled, fault):
+    """The native layer step takes extents and layouts on trust, so only weights whose parts fit one another reach it; the
+    operators, which check them, take the rest."""
+    from triton_b200.moe import _one_call
+    from triton_b200.tensor import Storage, Tensor
+    from triton_b200.tensor_details.layout import StridedLayout
+    lw, x, logits = _layer_on_cpu(block_scaled=block_scaled), torch.zeros(5, 64, dtype=torch.bfloat16), torch.zeros(5, 3)
+    assert _one_call(x, logits, lw, 2)
+    if block_scaled:
+        assert _one_call(x.to(torch.float8_e4m3fn), logits, lw, 2)
+    else:
+        assert not _one_call(x.to(torch.float8_e4m3fn), logits, lw, 2)
+    end = "_bs" if block_scaled else ""
+    reshaped = lambda t, shape: Tensor(t.storage, dtype=t.dtype, shape=shape)
+    if fault == "narrow b1":
+        lw.b1 = lw.b1[:, :-1].contiguous()
+    elif fault == "narrow b2":
+        lw.b2 = lw.b2[:, :-1].contiguous()
+    elif fault == "short b2":
+        lw.b2 = lw.b2[:-1]
+    elif fault == "width of w1":
+        setattr(lw, "w1" + end, reshaped(getattr(lw, "w1" + end), [3, 64, 2 * 96 - 2]))
+    elif fault == "depth of w2":
+        setattr(lw, "w2" + end, reshaped(getattr(lw, "w2" + end), [3, 64, 64]))
+    else:
+        name = ("w1" if fault == "scale layout" else "w2") + end + "_scale"
+        t = getattr(lw, name)
+        setattr(lw, name, Tensor(Storage(t.storage.data, StridedLayout()), dtype=t.dtype, shape=t.shape))
+    assert not _one_call(x, logits, lw, 2)

@@ -20,8 +20,8 @@ from .specialize import FnSpecs
 from .swiglu import swiglu_fn
 from .tensor import (FP4, Tensor, convert_layout, make_ragged_tensor_metadata, remap_ragged_tensor_metadata,
                      wrap_torch_tensor)
-from .tensor_details.layout import (B200BlockScaledValueLayout, B200MXValueLayout, make_default_matmul_mxfp4_w_layout,
-                                    make_default_matmul_mxfp4_w_scale_layout)
+from .tensor_details.layout import (B200BlockScaledScaleLayout, B200BlockScaledValueLayout, B200MXScaleLayout, B200MXValueLayout,
+                                    make_default_matmul_mxfp4_w_layout, make_default_matmul_mxfp4_w_scale_layout)
 from .topk import topk
 
 
@@ -102,23 +102,43 @@ def _activation(lw):
     return FusedActivation(FnSpecs("swiglu", swiglu_fn, ("alpha", "limit"), reduction_n=2), (lw.alpha, lw.limit))
 
 
-_LAYER_KIND = {B200MXValueLayout: _lib.MOE_W_MX4_B200, B200BlockScaledValueLayout: _lib.MOE_W_MX4_B200MX}
+_LAYER_KIND = {B200MXValueLayout: (_lib.MOE_W_MX4_B200, B200MXScaleLayout),
+               B200BlockScaledValueLayout: (_lib.MOE_W_MX4_B200MX, B200BlockScaledScaleLayout)}
+
+
+def _step_weights(x, lw: MoeLayerWeights, n_rows: int):
+    """(w1, scales, w2, scales) of a step of `n_rows` routed rows: e4m3 tokens are multiplied on the block-scaled copy only."""
+    if x.dtype == torch.float8_e4m3fn:
+        return lw.w1_bs, lw.w1_bs_scale, lw.w2_bs, lw.w2_bs_scale
+    return lw.fc_weights(n_rows)
 
 
 def _product(w: Tensor, scale: Tensor):
-    return _LAYER_KIND[type(w.storage.layout)], w.storage.data, scale.storage.data
+    return _LAYER_KIND[type(w.storage.layout)][0], w.storage.data, scale.storage.data
 
 
-def _one_call(x, logits, lw: MoeLayerWeights, k: int) -> bool:
+def _product_fits(w, scale, bias, E: int, K: int) -> bool:
+    """What `matmul` checks of one product: matching pair of tiled layouts, extents of weights and bias."""
+    if w is None or scale is None:
+        return False
+    kind = _LAYER_KIND.get(type(w.storage.layout))
+    return (kind is not None and type(scale.storage.layout) is kind[1] and w.dtype == FP4 and len(w.shape) == 3
+            and w.shape[0] >= E and w.shape[1] == K and bias.ndim == 2 and bias.shape[0] >= E and bias.shape[1] == w.shape[2]
+            and bias.stride(1) == 1)
+
+
+def _one_call(x, logits, lw: MoeLayerWeights, k: int, weights=None) -> bool:
     """Whether the step is one the native host path takes as a whole: fp32 logits, bf16 or e4m3 rows, weights and biases in
-    the forms this package prepares.  Anything else goes through the operators one by one."""
-    fp8 = x.dtype == torch.float8_e4m3fn
+    the forms this package prepares, extents that fit one another.  Anything else goes through the operators one by one,
+    which run it or say what is wrong with it."""
     E = logits.shape[1] if logits.ndim == 2 else 0
-    return ((fp8 or x.dtype == torch.bfloat16) and logits.dtype == torch.float32 and 0 < E <= 256 and E == lw.n_expts
-            and 0 < k <= E and x.ndim == 2 and x.stride(1) == 1 and logits.stride(1) == 1 and 0 < x.shape[0] <= FUSED_MAX_TOKENS
-            and logits.shape[0] == x.shape[0] and x.shape[1] == lw.w1.shape[1] and (not fp8 or lw.w1_bs is not None)
-            and type(lw.w1.storage.layout) is B200MXValueLayout and type(lw.w2.storage.layout) is B200MXValueLayout
-            and lw.b1.stride(1) == 1 and lw.b2.stride(1) == 1 and lw.w1.shape[2] == 2 * lw.w2.shape[1])
+    if not ((x.dtype == torch.float8_e4m3fn or x.dtype == torch.bfloat16) and logits.dtype == torch.float32 and 0 < E <= 256
+            and E == lw.n_expts and 0 < k <= E and x.ndim == 2 and x.stride(1) == 1 and logits.stride(1) == 1
+            and 0 < x.shape[0] <= FUSED_MAX_TOKENS and logits.shape[0] == x.shape[0]):
+        return False
+    w1, w1_scale, w2, w2_scale = _step_weights(x, lw, x.shape[0] * k) if weights is None else weights
+    return (_product_fits(w1, w1_scale, lw.b1, E, x.shape[1]) and w1.shape[2] % 2 == 0
+            and _product_fits(w2, w2_scale, lw.b2, E, w1.shape[2] // 2))
 
 
 def moe_layer_forward(x, logits, lw: MoeLayerWeights, k: int, gemm_timer=None):
@@ -128,11 +148,9 @@ def moe_layer_forward(x, logits, lw: MoeLayerWeights, k: int, gemm_timer=None):
     e4m3 activations (`x.dtype == torch.float8_e4m3fn`, the reference's fp8 mode: bench/bench_mlp.py `x_dtype="fp8"`) run
     both GEMMs on the block-scaled kernel at every size: fc1 writes e4m3 rows, fc2 reads them and writes bf16."""
     T = x.shape[0]
-    if gemm_timer is None and _one_call(x, logits, lw, k):
-        if x.dtype == torch.float8_e4m3fn:
-            w1, w1_scale, w2, w2_scale = lw.w1_bs, lw.w1_bs_scale, lw.w2_bs, lw.w2_bs_scale
-        else:
-            w1, w1_scale, w2, w2_scale = lw.fc_weights(T * k)
+    weights = _step_weights(x, lw, T * k)
+    if gemm_timer is None and _one_call(x, logits, lw, k, weights):
+        w1, w1_scale, w2, w2_scale = weights
         return _lib.host().layer(x, logits, k, (*_product(w1, w1_scale), lw.b1, *w1.shape[1:]),
                                  (*_product(w2, w2_scale), lw.b2, *w2.shape[1:]), lw.alpha, lw.limit, gemm_tuning(),
                                  _status_word(x.device))
@@ -147,13 +165,12 @@ def moe_layer_forward(x, logits, lw: MoeLayerWeights, k: int, gemm_timer=None):
     _lib.check(_lib.load().moe_ep_pull_index(_lib.ptr(scatter_idx.reshape(-1)), _lib.ptr(indx16.contiguous()),
                                              _lib.ptr(sparse.vals.contiguous()), _lib.ptr(_all_local(logits.shape[1], x.device)),
                                              n, k, _lib.ptr(gather_idx), _lib.ptr(gammas), _lib.stream()), "moe_ep_pull_index")
+    w1, w1_scale, w2, w2_scale = weights
     if x.dtype == torch.float8_e4m3fn:
         assert lw.w1_bs is not None, "e4m3 activations need the block-scaled copy of the weights"
-        w1, w1_scale, w2, w2_scale = lw.w1_bs, lw.w1_bs_scale, lw.w2_bs, lw.w2_bs_scale
         pc1 = PrecisionConfig(b_mx_scale=w1_scale, b_microblock_size=32, out_dtype=torch.float8_e4m3fn)
         pc2 = PrecisionConfig(b_mx_scale=w2_scale, b_microblock_size=32, out_dtype=torch.bfloat16)
     else:
-        w1, w1_scale, w2, w2_scale = lw.fc_weights(T * k)
         pc1 = PrecisionConfig(b_mx_scale=w1_scale, b_microblock_size=32)
         pc2 = PrecisionConfig(b_mx_scale=w2_scale, b_microblock_size=32)
     with _span(gemm_timer):

@@ -338,3 +338,24 @@ def test_layer_in_one_call_leaves_unfitting_weights_to_the_operators(block_scale
         t = getattr(lw, name)
         setattr(lw, name, Tensor(Storage(t.storage.data, StridedLayout()), dtype=t.dtype, shape=t.shape))
     assert not _one_call(x, logits, lw, 2)
+
+
+@pytest.mark.parametrize("block_scaled", [False, True])
+def test_tiling_reads_storage_in_place_only_where_it_has_the_stated_shape(block_scaled):
+    """A tensor may be stated larger than its storage (one expert's bytes standing for several): the kernel that reads the storage
+    in place must not take it, the canonical form that broadcasts it does."""
+    from triton_b200.tensor_details.layout import (B200BlockScaledScaleLayout, B200BlockScaledValueLayout, B200MXScaleLayout,
+                                                   B200MXValueLayout)
+    E, K, N = 3, 64, 40
+    value, scale = (B200BlockScaledValueLayout(), B200BlockScaledScaleLayout()) if block_scaled else (B200MXValueLayout(), B200MXScaleLayout())
+    tv, ts = value.make_transformation([E, K, N], True), scale.make_transformation([E, K // 32, N], False)
+    q = torch.zeros(E, N, K // 2, dtype=torch.uint8).transpose(1, 2)
+    s = torch.zeros(E, N, K // 32, dtype=torch.uint8).transpose(1, 2)
+    order = StridedLayout(major_dim=-2).order(3)
+    for bad in (q[:1], q[0], q[:, :16], q[:, :, :-1], q.to(torch.int16)):
+        assert tv.swizzle_strided(bad, order) is None
+    for bad in (s[:1], s[0], s[:, :1], s[:, :, :-1], s.float()):
+        assert ts.swizzle_strided(bad, order) is None
+    for good, t in ((q, tv), (s, ts)):
+        with pytest.raises(ValueError, match="CUDA tensors only"):      # goes to the kernel
+            t.swizzle_strided(good, order)

@@ -171,3 +171,20 @@ def test_full_size_properties(device):
     assert (dq <= blk * 1.2001).all() and (dq >= blk * 0.7999).all()
     err = (d.float() - x.float()).abs().view(8192, -1, 32) / blk.clamp_min(1e-30).unsqueeze(-1)
     assert err.max() <= 1.0 / 3 + 1e-6                           # half the coarsest e2m1 step (4 -> 6), block max > 3
+
+
+@pytest.mark.parametrize("block_scaled", [False, True])
+def test_tiles_of_storage_that_stands_for_several_experts(block_scaled, device):
+    """One expert's bytes stated as three: the tiles are those of the three written out."""
+    from triton_b200.tensor import FP4, UINT8, Storage, Tensor, convert_layout
+    from triton_b200.tensor_details.layout import (B200BlockScaledScaleLayout, B200BlockScaledValueLayout, B200MXScaleLayout,
+                                                   B200MXValueLayout, StridedLayout)
+    g = torch.Generator().manual_seed(5)
+    E, K, N = 3, 96, 130
+    q = torch.randint(0, 256, (1, N, K // 2), generator=g, dtype=torch.uint8).to(device).transpose(1, 2)
+    s = torch.randint(0, 255, (1, N, K // 32), generator=g, dtype=torch.uint8).to(device).transpose(1, 2)
+    layouts = (B200BlockScaledValueLayout(), B200BlockScaledScaleLayout()) if block_scaled else (B200MXValueLayout(), B200MXScaleLayout())
+    for t, dtype, shape, layout in ((q, FP4, [E, K, N], layouts[0]), (s, UINT8, [E, K // 32, N], layouts[1])):
+        three = t.transpose(1, 2).repeat(E, 1, 1).transpose(1, 2)
+        got, want = (convert_layout(Tensor(Storage(d, StridedLayout(major_dim=-2)), dtype=dtype, shape=shape), layout) for d in (t, three))
+        assert torch.equal(got.storage.data, want.storage.data)

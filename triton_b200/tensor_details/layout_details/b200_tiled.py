@@ -33,13 +33,12 @@ def _tiles(shape):
     return E, K, N, (N + TILE - 1) // TILE, (K + TILE - 1) // TILE
 
 
-def _strided3(data, lead):
-    """`data` as [E, rows, cols] without a copy, or None when the leading dimensions do not collapse."""
-    if len(lead) == 1:
-        return data
-    if len(lead) == 0:
-        return data.unsqueeze(0)
-    return None
+def _strided3(data, shape):
+    """`data` as [E, rows, cols] without a copy, or None where the tiling kernel cannot read it as a tensor of `shape` bytes:
+    another shape or type, or leading dimensions that do not collapse."""
+    if list(data.shape) != list(shape) or data.element_size() != 1 or not 2 <= data.ndim <= 3:
+        return None
+    return data if data.ndim == 3 else data.unsqueeze(0)
 
 
 @dataclass(frozen=True)
@@ -94,8 +93,9 @@ class B200MXValueLayoutTransformation(LayoutTransformation):
     def swizzle_strided(self, data, order):
         """From strided storage packed along K (what `downcast_to_mxfp(w, axis=-2)` returns): the tiling kernel reads it in
         place.  -> tiles, or None when the storage is packed otherwise."""
-        q = _strided3(data, self.shape[:-2])
-        if q is None or order[0] != len(self.shape) - 2 or q.stride(1) != 1 or self.shape[-2] % 32 != 0:
+        *lead, K, N = self.shape
+        q = _strided3(data, [*lead, K // 2, N])
+        if q is None or order[0] != len(self.shape) - 2 or q.stride(1) != 1 or K % 32 != 0:
             return None
         return self._tile(q, q.stride(0), q.stride(2))
 
@@ -136,8 +136,8 @@ class B200MXScaleLayoutTransformation(LayoutTransformation):
         return self._tile(data.reshape(-1, KG, N).contiguous())
 
     def swizzle_strided(self, data, order):
-        """From any strided storage, read in place; None when the leading dimensions do not collapse."""
-        s = _strided3(data, self.shape[:-2])
+        """From any strided storage, read in place; None when it cannot be (see `_strided3`)."""
+        s = _strided3(data, self.shape)
         return None if s is None else self._tile(s)
 
     def unswizzle_data(self, data):

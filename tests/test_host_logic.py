@@ -359,3 +359,16 @@ def test_tiling_reads_storage_in_place_only_where_it_has_the_stated_shape(block_
     for good, t in ((q, tv), (s, ts)):
         with pytest.raises(ValueError, match="CUDA tensors only"):      # goes to the kernel
             t.swizzle_strided(good, order)
+
+
+@pytest.mark.parametrize("limit", [0, 16, 47, 49, 100, 10000])
+def test_block_scaled_row_limit_is_the_callers(limit):
+    """A limit the caller sets decides alone, at any width; the default goes on by shape beyond its 48 rows per expert."""
+    for ff, d in ((96, 64), (2880, 2880)):
+        lw = _layer_on_cpu(E=3, d=d, ff=ff)
+        for rows in (1, 48, 49, 64, 80, 81, 100, 300, 5000):
+            assert lw.use_block_scaled(rows * 3) == (rows <= 80 or (ff == 2880 and rows >= 81))
+        lw.block_scaled_max_rows_per_expert = limit
+        for rows in (1, 16, 17, 47, 48, 49, 64, 80, 81, 100, 101, 300, 5000):
+            assert lw.use_block_scaled(rows * 3) == (rows <= limit)
+            assert (lw.fc_weights(rows * 3)[0] is lw.w1_bs) == (lw.fc_weights(rows * 3)[2] is lw.w2_bs) == (rows <= limit)

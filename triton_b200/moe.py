@@ -25,6 +25,9 @@ from .tensor_details.layout import (B200BlockScaledScaleLayout, B200BlockScaledV
 from .topk import topk
 
 
+BLOCK_SCALED_ROWS = 48
+
+
 @dataclass
 class MoeLayerWeights:
     w1: Tensor                 # FP4 [E, d_model, 2 * d_ff] (gate / linear columns interleaved)
@@ -46,7 +49,9 @@ class MoeLayerWeights:
     w1_bs_scale: Tensor | None = None
     w2_bs: Tensor | None = None
     w2_bs_scale: Tensor | None = None
-    block_scaled_max_rows_per_expert: int = 48       # up to here the block-scaled kernels are faster whatever the shape
+    # rows per expert up to which a step runs on the block-scaled copy.  A caller's own figure is the limit (0: never, e4m3 tokens
+    # apart); with the default, up to which those kernels are faster whatever the shape, `use_block_scaled` goes on by shape.
+    block_scaled_max_rows_per_expert: int = BLOCK_SCALED_ROWS
 
     @property
     def n_expts(self):
@@ -63,6 +68,8 @@ class MoeLayerWeights:
             return False
         if n_rows <= self.block_scaled_max_rows_per_expert * self.n_expts:
             return True
+        if self.block_scaled_max_rows_per_expert != BLOCK_SCALED_ROWS:
+            return False
         n_out = self.b1.shape[1] if n_out is None else n_out
         return n_rows <= 80 * self.n_expts or n_out >= (1280 if n_rows < 512 * self.n_expts else 2560)
 

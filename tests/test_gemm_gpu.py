@@ -420,3 +420,30 @@ def test_layer_with_a_bias_of_the_wrong_width_is_refused(device):
         setattr(lw, name, getattr(lw, name)[:, :-32].contiguous())
         with pytest.raises(AssertionError):
             moe_layer_forward(x, logits, lw, 2)
+
+
+@pytest.mark.parametrize("rows_per_expert", [40, 64])
+@pytest.mark.parametrize("constraint", [{"kernel": "tcgen05"}, {"kernel": "tcgen05-pair"}, {"kernel": "stream"}, {"block_m": 128}, {"block_n": 256},
+                                        {"kernel": "mx"}])
+def test_layer_with_both_weight_copies_under_a_constraint(constraint, rows_per_expert, device):
+    """Beyond 48 rows per expert a layer with both weight copies runs the kernel or tile that a constraint names: the same bits
+    as without the second copy.  Up to there it stays on the block-scaled copy, which refuses a bf16 kernel."""
+    from triton_b200.moe import moe_layer_forward
+    from triton_b200.testing import make_synthetic_layer
+    E, k = 8, 2
+    T = rows_per_expert * E // k
+    g = torch.Generator(device=device).manual_seed(1)
+    x = torch.randn(T, 512, device=device, generator=g).bfloat16()
+    logits = torch.randn(T, E, device=device, generator=g)
+    both, default = make_synthetic_layer(E, 512, 736, device, seed=3, block_scaled=True), make_synthetic_layer(E, 512, 736, device, seed=3)
+    free = moe_layer_forward(x, logits, both, k)
+    with tb.scoped_opt_flags_constraints(constraint):
+        if rows_per_expert <= 48 and constraint.get("kernel", "mx") != "mx":
+            with pytest.raises(tb.InapplicableConstraint):
+                moe_layer_forward(x, logits, both, k)
+            return
+        y = moe_layer_forward(x, logits, both, k)
+        tb.matmul_check_status()
+        assert oracle.rel_l2(free.cpu(), y.cpu()) < 1e-2
+        if rows_per_expert > 48 and "mx" not in constraint.values():
+            assert torch.equal(y, moe_layer_forward(x, logits, default, k))

@@ -372,3 +372,15 @@ def test_block_scaled_row_limit_is_the_callers(limit):
         for rows in (1, 16, 17, 47, 48, 49, 64, 80, 81, 100, 101, 300, 5000):
             assert lw.use_block_scaled(rows * 3) == (rows <= limit)
             assert (lw.fc_weights(rows * 3)[0] is lw.w1_bs) == (lw.fc_weights(rows * 3)[2] is lw.w2_bs) == (rows <= limit)
+
+
+def test_weights_of_a_step_under_a_tuning_constraint():
+    """Beyond the row limit a constraint that names a bf16 kernel or a tile keeps a step on the default copy; up to the limit, and
+    under any other constraint, the choice is the one without it."""
+    lw = _layer_on_cpu(E=3, d=2880, ff=2880)
+    pinned = [{"kernel": k} for k in ("tcgen05", "tcgen05-pair", "stream", "simt")] + [{"block_m": 128}, {"block_m": 256}, {"block_n": 256}]
+    free = [{}, {"kernel": "auto"}, {"idle_sms": 8}, {"kernel": "mx"}, {"block_m": None}]
+    for cons in pinned + free:
+        with triton_b200.scoped_opt_flags_constraints(cons):
+            for rows in (1, 48, 49, 64, 300, 2048):
+                assert lw.use_block_scaled(rows * 3) == (rows <= 48 or cons in free), (cons, rows)

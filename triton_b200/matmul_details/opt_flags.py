@@ -104,3 +104,10 @@ def gemm_tuning() -> tuple:
     if not get_opt_flags_constraints():
         return (0, 0, 0, _idle_sms)
     return (_KERNEL_CODE[resolve_kernel_choice()], resolve_tile_m(), resolve_tile_n(), get_idle_sms())
+
+
+def bf16_kernel_or_tile_named() -> bool:
+    """Whether the current constraints name a kernel that multiplies bf16 tokens (default weight tiles), or a tile shape."""
+    c = get_opt_flags_constraints()
+    return bool(c) and (c.get("kernel") in ("simt", "tcgen05", "tcgen05-pair", "stream")
+                        or c.get("block_m") is not None or c.get("block_n") is not None)

@@ -12,7 +12,7 @@ import torch
 
 from . import _lib
 from .matmul import FusedActivation, PrecisionConfig, _status_word, matmul
-from .matmul_details.opt_flags import gemm_tuning
+from .matmul_details.opt_flags import bf16_kernel_or_tile_named, gemm_tuning
 from .numerics_details.mxfp import downcast_to_mxfp
 from .reduce import reduce
 from .routing import FUSED_MAX_TOKENS, route, routing  # noqa: F401
@@ -63,12 +63,13 @@ class MoeLayerWeights:
         With more rows the block-scaled pair kernel first re-lays the tokens out (4 bytes per element written and read
         against 2 n_out operations), which a wide product repays and a narrow one does not; measured against the bf16
         kernel: 64 rows per expert 1.3-1.7 x faster for n_out >= 2000 and 1.0-1.2 x at 512-1440; 256 rows 0.8 x at 512;
-        1024 rows per expert 1.05-1.2 x faster from 2880 on, 0.9 x at 2048."""
+        1024 rows per expert 1.05-1.2 x faster from 2880 on, 0.9 x at 2048.  A tuning constraint that names a kernel of the
+        default copy, or a tile, keeps steps beyond the row limit on that copy, whose kernels have it."""
         if self.w1_bs is None:
             return False
         if n_rows <= self.block_scaled_max_rows_per_expert * self.n_expts:
             return True
-        if self.block_scaled_max_rows_per_expert != BLOCK_SCALED_ROWS:
+        if self.block_scaled_max_rows_per_expert != BLOCK_SCALED_ROWS or bf16_kernel_or_tile_named():
             return False
         n_out = self.b1.shape[1] if n_out is None else n_out
         return n_rows <= 80 * self.n_expts or n_out >= (1280 if n_rows < 512 * self.n_expts else 2560)

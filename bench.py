@@ -258,9 +258,15 @@ def measured_peaks():
     return {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0, "bf16_tflops_sustained": 1400.0, "source": "fallback"}
 
 
-def gemm_traffic_note(tokens, n_expts, world):
-    """DRAM bytes per step of the grouped-GEMM launches from the committed ncu summary; only for the configuration the
-    summary was scaled to."""
+def kernel_names(lw, n_rows, dtype=torch.bfloat16):
+    """The kernels that the library runs fc1 and fc2 of a step of `n_rows` routed rows on."""
+    fc1, fc2 = lw.kernels(n_rows, dtype)
+    return fc1 if fc1 == fc2 else f"{fc1} (fc1), {fc2} (fc2)"
+
+
+def gemm_traffic_note(tokens, n_expts, world, kernels):
+    """DRAM bytes per step of the grouped-GEMM launches from the committed ncu summary; only for the configuration and the kernel
+    that the summary was taken of."""
     p = ROOT / "profiles" / "gemm_tc_traffic.json"
     if not p.exists():
         return None
@@ -268,7 +274,7 @@ def gemm_traffic_note(tokens, n_expts, world):
         d = json.loads(p.read_text())
     except Exception:
         return None
-    if world == 1 and d.get("tokens") == tokens and d.get("experts") == n_expts:
+    if world == 1 and d.get("tokens") == tokens and d.get("experts") == n_expts and kernels == "gemm_tc_kernel":
         return d.get("dram_bytes_per_step")
     return None
 
@@ -444,7 +450,7 @@ def decode_point(lw, n_expts, T, dev, expert_bias, peaks, n_batches=6, rounds=5)
     act = sum(n_act) / len(n_act)
     wbytes = act * BYTES_PER_EXPERT
     return {"tokens": T, "active_experts": act, "weight_mb": wbytes / 1e6,
-            "kernel": "gemm_mx_kernel (block-scaled)" if lw.use_block_scaled(T * TOP_K) else "bf16 kernels",
+            "kernel": kernel_names(lw, T * TOP_K),
             "gemm_ms": ms_gemm, "gemm_gbs": wbytes / ms_gemm / 1e6, "gemm_frac_hbm": wbytes / ms_gemm / 1e6 / peaks["hbm_gbs"],
             "step_ms": ms_step, "step_gbs": wbytes / ms_step / 1e6, "step_frac_hbm": wbytes / ms_step / 1e6 / peaks["hbm_gbs"],
             "tokens_per_s": T / (ms_step * 1e-3)}
@@ -491,7 +497,7 @@ def sweep_20b_record(lw20, dev, expert_bias, peaks):
             gm = median(per_step)
             tf = T * TOP_K * (FLOP_PER_ROW_FC1 + FLOP_PER_ROW_FC2) / (gm * 1e-3) / 1e12
             rec = {"tokens": T, "ms_per_step": ms, "tokens_per_s": T / (ms * 1e-3), "cuda_graph": False, "gemm_ms": gm,
-                   "gemm_tflops": tf, "gemm_frac_bf16_burst": tf / peaks["bf16_tflops"], "kernel": "gemm_tc_kernel (bf16)"}
+                   "gemm_tflops": tf, "gemm_frac_bf16_burst": tf / peaks["bf16_tflops"], "kernel": kernel_names(lw20, T * TOP_K)}
         pts.append(rec)
     tb.matmul_check_status()
     return {"what": "gpt-oss-20b layer shape (E=32 top-4, d_model 2880, fused gate+up 5760), 1 GPU, whole layer step",
@@ -560,7 +566,8 @@ def act_fp8_record(lw, dev, expert_bias, peaks, T, n_steps, roofs):
     rel = oracle.rel_l2(ref, got)
     mx, _ = oracle.rel_errors(ref, got)
     roof = roofs["tflops"].get("e2m1 x e4m3 block-scaled kind::mxf8f6f4") if roofs else None
-    return {"what": "e4m3 activations x MXFP4 weights, gemm_mx_kernel (kind::mxf8f6f4) for fc1 and fc2, eager steps",
+    return {"what": "e4m3 activations x MXFP4 weights (kind::mxf8f6f4), eager steps",
+            "kernel": kernel_names(lw, T * TOP_K, torch.float8_e4m3fn),
             "tokens": T, "ms_per_step": ms, "tokens_per_s": T / (ms * 1e-3), "gemm_ms_per_step": gm, "gemm_tflops": tf,
             "frac_of_measured_mxf8f6f4_roof": None if not roof else tf / roof,
             "parity": {"tokens": len(rows), "rel_l2": float(rel), "max_rel": float(mx), "ok": bool(rel < 1e-2 and mx <= 3e-2),
@@ -597,22 +604,9 @@ def micro_record(dev, peaks, steps=5):
             ts.append(e0.elapsed_time(e1) / len(fns))
         return median(ts), launches
 
-    # a write-dominated kernel cannot reach the copy bandwidth (half reads, half writes): measure the pure-write rate too
-    big = torch.empty(1 << 30, dtype=torch.uint8, device=dev)
-    fill_ms = []
-    for _ in range(6):
-        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        e0.record()
-        big.zero_()
-        e1.record()
-        torch.cuda.synchronize()
-        fill_ms.append(e0.elapsed_time(e1))
-    write_gbs = (1 << 30) / (min(fill_ms[2:]) * 1e-3) / 1e9
-    del big
     out = {"l2": "flushed by a 512 MB write before every timed span; a span is the same call on 4 distinct inputs, back to back",
            "peak_gbs": peaks["hbm_gbs"],
-           "peak_source": f"{peaks['source']} copy bandwidth", "write_only_gbs": write_gbs,
-           "write_only_source": "torch zero_ of 1 GiB, best of 4, measured in this run", "kernels": {}}
+           "peak_source": f"{peaks['source']} copy bandwidth", "kernels": {}}
 
     def add(name, res, nbytes):
         ms, launches = res
@@ -655,10 +649,6 @@ def micro_record(dev, peaks, steps=5):
     add("downcast_to_mxfp bf16 [8192,8192] axis 1", timed([lambda x=x: downcast_to_mxfp(x, torch.uint8, axis=1) for x in xs]), nb)
     add("upcast_from_mxfp -> bf16 [8192,8192] axis 1",
         timed([lambda q=q, sc=sc: upcast_from_mxfp(q, sc, torch.bfloat16, axis=1) for q, sc in qs]), nb)
-    up = out["kernels"]["upcast_from_mxfp -> bf16 [8192,8192] axis 1"]
-    # 79 % of the dequantiser's bytes are writes: its bound is the time to write R * C * 2 bytes at the write-only rate
-    up["write_bound_ms"] = R * C * 2 / write_gbs / 1e6
-    up["frac_of_write_bound"] = up["write_bound_ms"] / up["ms"]
     add("downcast_to_mxfp bf16 [8192,8192] axis 0 (strided)",
         timed([lambda x=x: downcast_to_mxfp(x, torch.uint8, axis=0) for x in xs]), nb)
     return out
@@ -876,17 +866,17 @@ def main():
 
     act_bytes = rows_local * (D_MODEL * 2 + D_FF * 2 * 2 + D_MODEL * 2)
     stream_gbs = (n_active * BYTES_PER_EXPERT + act_bytes) / (gemm_ms_per_step * 1e-3) / 1e9
-    decode_kernel = lw.use_block_scaled(T * TOP_K if world == 1 else rows_local)
+    kernels = kernel_names(lw, T * TOP_K if world == 1 else rows_local)
     roofline = {
         "bound": "tensor",
-        "kernel": "gemm_tc_kernel (fc1 + fc2 launches of a step incl. fc1's row gather, bf16 kind::f16 after in-SM dequant)",
+        "kernel": kernels, "timed": "the fc1 + fc2 calls of a step composed from the operators, token pack or row gather included",
         "achieved": achieved_tflops, "peak": peaks["bf16_tflops"], "unit": "TFLOP/s",
         "frac": achieved_tflops / peaks["bf16_tflops"],
         "peak_source": f"{peaks['source']} bf16 cuBLAS, burst (the timed block is short and runs at full clocks)",
         "frac_burst": achieved_tflops / peaks["bf16_tflops"],
         "frac_sustained": None if sustained is None else sustained["tflops"] / peaks["bf16_tflops_sustained"],
         "peak_sustained": peaks["bf16_tflops_sustained"],
-        "traffic": gemm_traffic_note(T, N_EXPTS, world),
+        "traffic": gemm_traffic_note(T, N_EXPTS, world, kernels),
         "ms_per_step_in_kernel": gemm_ms_per_step, "launches_per_step": calls_per_step,
         "rows_this_rank": rows_local, "per_rank": per_rank,
         "hbm": {"active_experts": n_active, "algorithmic_gbs": stream_gbs, "peak_gbs": peaks["hbm_gbs"],
@@ -901,8 +891,7 @@ def main():
         roofline.update({"bound": "hbm", "achieved": stream_gbs, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                          "frac": stream_gbs / peaks["hbm_gbs"], "peak_source": f"{peaks['source']} copy bandwidth",
                          "tflops": achieved_tflops, "frac_burst": None, "frac_sustained": None,
-                         "kernel": ("gemm_mx_kernel (block-scaled, fc1 + fc2)" if decode_kernel else "gemm_stream_kernel (fc1 + fc2)") +
-                                   ", timed as the whole replayed step"})
+                         "timed": "the whole replayed step"})
 
     # ---- per-phase breakdown of the expert-parallel step (untimed pass, eager) -----------------------------------
     phases = None

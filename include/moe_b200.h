@@ -265,6 +265,9 @@ typedef struct {
 } MoeGemmArgs;
 int moe_grouped_gemm(const MoeGemmArgs* args_host, void* stream);
 size_t moe_gemm_mx_workspace_bytes(const MoeGemmArgs* args_host);
+/* Name of the kernel that moe_grouped_gemm launches for these arguments (with the workspace of the size above given), "" for an
+ * empty product; NULL, with the reason in moe_last_error(), where it refuses them.  Launches nothing and reads no device memory. */
+const char* moe_gemm_kernel_name(const MoeGemmArgs* args_host);
 
 /* Tensor-pipe roof of one MMA kind on this device, for the benchmark's roofline: one CTA per SM issues `iters` x 4
  * back-to-back tcgen05.mma (M 128, N 256) over operand tiles resident in shared memory.  kind 0: bf16 (kind::f16),

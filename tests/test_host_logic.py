@@ -384,3 +384,21 @@ def test_weights_of_a_step_under_a_tuning_constraint():
         with triton_b200.scoped_opt_flags_constraints(cons):
             for rows in (1, 48, 49, 64, 300, 2048):
                 assert lw.use_block_scaled(rows * 3) == (rows <= 48 or cons in free), (cons, rows)
+
+
+def test_kernels_of_a_step():
+    """The library names the kernel its dispatch takes: the figures beside the rules, on either weight copy."""
+    both, default = _layer_on_cpu(E=3, d=2880, ff=2880), _layer_on_cpu(E=3, d=2880, ff=2880, block_scaled=False)
+    decode, pair, tc = "gemm_mx_kernel", "gemm_mx_pair_kernel", "gemm_tc_kernel"
+    assert both.kernels(3 * 8) == (decode,) * 2 and both.kernels(3 * 19) == (decode,) * 2
+    assert both.kernels(3 * 20) == (pair,) * 2 and both.kernels(3 * 1000) == (pair,) * 2
+    assert both.kernels(3 * 15, torch.float8_e4m3fn) == (decode,) * 2 and both.kernels(3 * 16, torch.float8_e4m3fn) == (pair,) * 2
+    assert default.kernels(3 * 20) == (pair,) * 2 and default.kernels(3 * 1000) == (pair,) * 2
+    small = _layer_on_cpu(E=3, d=512, ff=512, block_scaled=False)
+    assert small.kernels(3 * 10) == ("gemm_stream_kernel",) * 2 and small.kernels(3 * 64) == (tc,) * 2
+    narrow = _layer_on_cpu(E=3, d=2048, ff=2880, block_scaled=False)
+    assert narrow.kernels(3 * 511) == (pair,) * 2 and narrow.kernels(3 * 512) == (pair, tc)
+    with triton_b200.scoped_opt_flags_constraints({"kernel": "tcgen05"}):
+        assert both.kernels(3 * 100) == (tc,) * 2
+        with pytest.raises(triton_b200.InapplicableConstraint):
+            both.kernels(3 * 8)

@@ -22,7 +22,13 @@ static int64_t n_blocks_bound(int64_t n_slices, int64_t n_rows, int64_t block) {
   return n_slices - 1 - fl;
 }
 
-extern "C" __attribute__((visibility("default"))) int moe_grouped_gemm(const MoeGemmArgs* a, void* stream) {
+namespace {
+
+enum Kernel { K_MX_PAIR, K_MX, K_STREAM, K_TC, K_TC_PAIR, K_SIMT };
+const char* const KERNEL_NAME[] = {"gemm_mx_pair_kernel", "gemm_mx_kernel", "gemm_stream_kernel", "gemm_tc_kernel", "gemm_tc_pair_kernel",
+                                   "gemm_simt_kernel"};
+
+int check_args(const MoeGemmArgs* a) {
   MOE_CHECK_ARG(a != nullptr, "moe_grouped_gemm: args is NULL");
   MOE_CHECK_ARG(a->E > 0 && a->K >= 0 && a->N >= 0 && a->M >= 0, "moe_grouped_gemm: bad extents E=%d K=%d N=%d M=%lld",
                 a->E, a->K, a->N, (long long)a->M);
@@ -37,7 +43,81 @@ extern "C" __attribute__((visibility("default"))) int moe_grouped_gemm(const Moe
   } else {
     MOE_CHECK_ARG(a->E == 1, "moe_grouped_gemm: without ragged metadata there must be one weight matrix");
   }
+  MOE_CHECK_ARG(a->n_y_peers >= 0 && a->n_y_peers <= MOE_MAX_PEERS, "moe_grouped_gemm: n_y_peers must be 0..%d", MOE_MAX_PEERS);
+  if (a->n_y_peers > 0) {
+    MOE_CHECK_ARG(a->y_rows_per_peer > 0, "moe_grouped_gemm: y_rows_per_peer must be positive with y_peers");
+    for (int i = 0; i < a->n_y_peers; ++i)
+      MOE_CHECK_ARG(a->y_peers[i] != nullptr && (uintptr_t)a->y_peers[i] % 16 == 0,
+                    "moe_grouped_gemm: y_peers[%d] is NULL or not 16-byte aligned", i);
+  }
+  return MOE_OK;
+}
+
+// The kernel of a call, or the status (and error) of a refused one.  `workspace`: the block-scaled kernels' workspace is there.
+int choose_kernel(const MoeGemmArgs& a, bool workspace, Kernel& out) {
+  const char* why = "";
+  const bool mx_asked = a.kernel == MOE_GEMM_MX || a.kernel == MOE_GEMM_MX_F8 || a.kernel == MOE_GEMM_MX_F4;
+  // default tiles on the block-scaled pair kernel; without its workspace they stay with the kernels below
+  if (a.w_kind == MOE_W_MX4_B200 && (mx_asked || workspace) && moe_gemm_mx_pair_wanted(a)) {
+    out = K_MX_PAIR;
+    return MOE_OK;
+  }
+  if (a.w_kind == MOE_W_MX4_B200MX || mx_asked) {
+    // weights laid out for the block-scaled MMA: that kernel or nothing
+    if (!moe_gemm_mx_supported(a, &why) || (a.kernel != MOE_GEMM_AUTO && !mx_asked)) {
+      moe_set_error("moe_grouped_gemm: block-scaled kernel not applicable: %s", *why ? why : "another kernel was requested");
+      return MOE_ERR_UNSUPPORTED;
+    }
+    out = moe_gemm_mx_pair_wanted(a) ? K_MX_PAIR : K_MX;
+    return MOE_OK;
+  }
+  const bool tc = moe_gemm_tc_supported(a, &why);
+  if ((a.kernel == MOE_GEMM_TCGEN05 || a.kernel == MOE_GEMM_TCGEN05_PAIR || a.kernel == MOE_GEMM_STREAM) && !tc) {
+    moe_set_error("moe_grouped_gemm: tcgen05 kernel not applicable: %s", why);
+    return MOE_ERR_UNSUPPORTED;
+  }
+  if (!tc || a.kernel == MOE_GEMM_SIMT) {
+    MOE_CHECK_ARG(a.w_kind == MOE_W_DENSE || a.w_kind == MOE_W_MX4_CANONICAL,
+                  "moe_grouped_gemm: the SIMT kernel takes dense or canonical MXFP4 weights (%s)", why);
+    out = K_SIMT;
+    return MOE_OK;
+  }
+  // A few rows per expert (decode): the weight-streaming kernel, bound by HBM rather than by pipeline hand-offs.
+  const bool streams = moe_gemm_stream_supported(a, &why);
+  if (a.kernel == MOE_GEMM_STREAM && !streams) {
+    moe_set_error("moe_grouped_gemm: streaming kernel not applicable: %s", why);
+    return MOE_ERR_UNSUPPORTED;
+  }
+  if (a.kernel == MOE_GEMM_STREAM ||
+      (a.kernel == MOE_GEMM_AUTO && streams && a.tile_m == 0 && a.tile_n == 0 && a.M <= 10 * (int64_t)a.E)) {
+    out = K_STREAM;
+    return MOE_OK;
+  }
+  // (the bf16 kernel on pairs of SMs, 256 x 256 tiles, runs on request only)
+  if (a.kernel == MOE_GEMM_TCGEN05_PAIR && !moe_gemm_tc_pair_supported(a, &why)) {
+    moe_set_error("moe_grouped_gemm: SM-pair tcgen05 kernel not applicable: %s", why);
+    return MOE_ERR_UNSUPPORTED;
+  }
+  out = a.kernel == MOE_GEMM_TCGEN05_PAIR ? K_TC_PAIR : K_TC;
+  return MOE_OK;
+}
+
+}  // namespace
+
+extern "C" __attribute__((visibility("default"))) const char* moe_gemm_kernel_name(const MoeGemmArgs* a) {
+  if (check_args(a) != MOE_OK) return nullptr;
+  if (a->M == 0 || a->N == 0) return "";
+  Kernel k;
+  return choose_kernel(*a, true, k) == MOE_OK ? KERNEL_NAME[k] : nullptr;
+}
+
+extern "C" __attribute__((visibility("default"))) int moe_grouped_gemm(const MoeGemmArgs* a, void* stream) {
+  if (const int rc = check_args(a)) return rc;
+  if (a->M == 0 || a->N == 0) return MOE_OK;
   cudaStream_t st = (cudaStream_t)stream;
+  Kernel kernel;
+  const bool workspace = a->mx_workspace && a->mx_workspace_bytes >= moe_gemm_mx_pair_workspace(*a);
+  if (const int rc = choose_kernel(*a, workspace, kernel)) return rc;
 
   GemmParams p;
   p.x = a->x; p.ld_x = a->ld_x; p.rows_x = a->rows_x;
@@ -52,72 +132,26 @@ extern "C" __attribute__((visibility("default"))) int moe_grouped_gemm(const Moe
   p.betas = a->betas; p.gammas = a->gammas;
   p.out_alpha = a->out_alpha; p.has_out_alpha = a->has_out_alpha;
   p.activation = a->activation; p.act_alpha = a->act_alpha; p.act_limit = a->act_limit; p.act_has_limit = a->act_has_limit;
-  p.y = a->y; p.ld_y = a->ld_y;
+  p.y = a->n_y_peers > 0 ? a->y_peers[0] : a->y; p.ld_y = a->ld_y;
   p.status = a->status;
-  MOE_CHECK_ARG(a->n_y_peers >= 0 && a->n_y_peers <= MOE_MAX_PEERS, "moe_grouped_gemm: n_y_peers must be 0..%d", MOE_MAX_PEERS);
   p.n_y_peers = a->n_y_peers; p.y_rows_per_peer = a->y_rows_per_peer;
   for (int i = 0; i < MOE_MAX_PEERS; ++i) p.y_peers[i] = i < a->n_y_peers ? a->y_peers[i] : nullptr;
-  if (a->n_y_peers > 0) {
-    MOE_CHECK_ARG(a->y_rows_per_peer > 0, "moe_grouped_gemm: y_rows_per_peer must be positive with y_peers");
-    for (int i = 0; i < a->n_y_peers; ++i)
-      MOE_CHECK_ARG(a->y_peers[i] != nullptr && (uintptr_t)a->y_peers[i] % 16 == 0,
-                    "moe_grouped_gemm: y_peers[%d] is NULL or not 16-byte aligned", i);
-    p.y = a->y_peers[0];
-  }
 
-  const char* why = "";
-  const bool mx_asked = a->kernel == MOE_GEMM_MX || a->kernel == MOE_GEMM_MX_F8 || a->kernel == MOE_GEMM_MX_F4;
-  // default tiles on the block-scaled pair kernel; without its workspace they stay with the kernels below
-  if (a->w_kind == MOE_W_MX4_B200 && moe_gemm_mx_pair_wanted(*a) &&
-      (mx_asked || (a->mx_workspace && a->mx_workspace_bytes >= moe_gemm_mx_pair_workspace(*a))))
-    return moe_gemm_mx_pair_launch(p, *a, st);
-  if (a->w_kind == MOE_W_MX4_B200MX || mx_asked) {
-    // weights laid out for the block-scaled MMA: that kernel or nothing
-    if (!moe_gemm_mx_supported(*a, &why) || (a->kernel != MOE_GEMM_AUTO && !mx_asked)) {
-      moe_set_error("moe_grouped_gemm: block-scaled kernel not applicable: %s", *why ? why : "another kernel was requested");
-      return MOE_ERR_UNSUPPORTED;
-    }
-    return moe_gemm_mx_launch(p, *a, st);
-  }
-  bool tc = moe_gemm_tc_supported(*a, &why);
-  if ((a->kernel == MOE_GEMM_TCGEN05 || a->kernel == MOE_GEMM_TCGEN05_PAIR || a->kernel == MOE_GEMM_STREAM) && !tc) {
-    moe_set_error("moe_grouped_gemm: tcgen05 kernel not applicable: %s", why);
-    return MOE_ERR_UNSUPPORTED;
-  }
-  if (a->kernel == MOE_GEMM_SIMT) tc = false;
-  if (tc) {
-    // A few rows per expert (decode): the weight-streaming kernel, bound by HBM rather than by pipeline hand-offs.
-    bool streaming = moe_gemm_stream_supported(*a, &why);
-    if (a->kernel == MOE_GEMM_STREAM && !streaming) {
-      moe_set_error("moe_grouped_gemm: streaming kernel not applicable: %s", why);
-      return MOE_ERR_UNSUPPORTED;
-    }
-    if (a->kernel == MOE_GEMM_AUTO)
-      streaming = streaming && a->tile_m == 0 && a->tile_n == 0 && a->M <= 10 * (int64_t)(a->E > 0 ? a->E : 1);
-    else if (a->kernel != MOE_GEMM_STREAM)
-      streaming = false;
-    if (streaming) return moe_gemm_stream_launch(p, *a, st);
-    // (the bf16 kernel on pairs of SMs, 256 x 256 tiles, runs on request only)
-    bool pair = moe_gemm_tc_pair_supported(*a, &why);
-    if (a->kernel == MOE_GEMM_TCGEN05_PAIR && !pair) {
-      moe_set_error("moe_grouped_gemm: SM-pair tcgen05 kernel not applicable: %s", why);
-      return MOE_ERR_UNSUPPORTED;
-    }
-    if (a->kernel != MOE_GEMM_TCGEN05_PAIR) pair = false;
+  if (kernel == K_MX_PAIR) return moe_gemm_mx_pair_launch(p, *a, st);
+  if (kernel == K_MX) return moe_gemm_mx_launch(p, *a, st);
+  if (kernel == K_STREAM) return moe_gemm_stream_launch(p, *a, st);
+  if (kernel == K_TC || kernel == K_TC_PAIR) {
     // Large gathered problems: copy the gathered rows once into the caller's scratch, then stream them by TMA.
-    const bool big = (a->tile_m == 0 || a->tile_m == 256) && (a->tile_m == 256 || a->M / (a->E > 0 ? a->E : 1) >= 12);
+    const bool big = (a->tile_m == 0 || a->tile_m == 256) && (a->tile_m == 256 || a->M / a->E >= 12);
     if (a->gather_indx && a->gather_scratch && big && a->gather_scratch_bytes >= (int64_t)a->M * a->K * 2) {
       const int rc = moe_gather_rows(a->x, a->ld_x * 2, a->gather_indx, a->M, (int64_t)a->K * 2, a->gather_scratch,
                                      (int64_t)a->K * 2, stream);
       if (rc != MOE_OK) return rc;
       p.x = a->gather_scratch; p.ld_x = a->K; p.rows_x = a->M; p.gather_indx = nullptr;
     }
-    if (pair) return moe_gemm_tc_pair_launch(p, *a, st);
-    return moe_gemm_tc_launch(p, *a, st);
+    return kernel == K_TC_PAIR ? moe_gemm_tc_pair_launch(p, *a, st) : moe_gemm_tc_launch(p, *a, st);
   }
 
-  MOE_CHECK_ARG(a->w_kind == MOE_W_DENSE || a->w_kind == MOE_W_MX4_CANONICAL,
-                "moe_grouped_gemm: the SIMT kernel takes dense or canonical MXFP4 weights (%s)", why);
   int64_t grid_m;
   if (a->slice_sizes) {
     p.block_offs = a->block_offs_16 + 2 * a->ld_block_offs;     // block size 64

@@ -755,7 +755,6 @@ int launch_mx_ty(const GemmParams& p, const MxParams& q, const MxPlan& pl, const
 
 bool moe_gemm_mx_pair_wanted(const MoeGemmArgs& a);
 int64_t moe_gemm_mx_pair_workspace(const MoeGemmArgs& a);
-int moe_gemm_mx_pair_launch(const GemmParams& p, const MoeGemmArgs& a, cudaStream_t st);
 
 bool moe_gemm_mx_supported(const MoeGemmArgs& a, const char** why) {
   if (a.w_kind != MOE_W_MX4_B200MX) { *why = "weights are not in the block-scaled B200 layout"; return false; }
@@ -780,7 +779,6 @@ extern "C" __attribute__((visibility("default"))) size_t moe_gemm_mx_workspace_b
 }
 
 int moe_gemm_mx_launch(const GemmParams& p_in, const MoeGemmArgs& a, cudaStream_t st) {
-  if (moe_gemm_mx_pair_wanted(a)) return moe_gemm_mx_pair_launch(p_in, a, st);
   const MxPlan pl = mx_plan(a);
   if (pl.grid_m == 0) return MOE_OK;
   MOE_CHECK_ARG(a.mx_workspace != nullptr && a.mx_workspace_bytes >= pl.ws_bytes && (uintptr_t)a.mx_workspace % 1024 == 0,

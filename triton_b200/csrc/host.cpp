@@ -17,7 +17,8 @@ struct Lib {
 #define MOE_HOST_FUNCTIONS(X)                                                                                            \
   X(moe_last_error) X(moe_route) X(moe_route_positions) X(moe_route_workspace) X(moe_grouped_gemm) X(moe_gemm_mx_workspace_bytes) \
   X(moe_reduce) X(moe_downcast_mxfp4) X(moe_upcast_mxfp4) X(moe_bitmatrix_metadata) X(moe_bitmatrix_metadata_workspace) \
-  X(moe_router_topk) X(moe_router_topk_workspace_bytes) X(moe_copy2)
+  X(moe_router_topk) X(moe_router_topk_workspace_bytes) X(moe_copy2) \
+  X(moe_gemm_kernel_name)
 #define X(name) decltype(&::name) name = nullptr;
   MOE_HOST_FUNCTIONS(X)
 #undef X
@@ -49,15 +50,16 @@ void check(int status, const char* what, bool tuning = false) {
 
 void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 
-int dtype_code(const Tensor& t) {
-  switch (t.scalar_type()) {
+int dtype_code(at::ScalarType t) {
+  switch (t) {
     case at::kFloat: return MOE_F32;
     case at::kHalf: return MOE_F16;
     case at::kBFloat16: return MOE_BF16;
     case at::kFloat8_e4m3fn: return MOE_F8E4M3;
-    default: raise(PyExc_ValueError, std::string("unsupported dtype ") + c10::toString(t.scalar_type()));
+    default: raise(PyExc_ValueError, std::string("unsupported dtype ") + c10::toString(t));
   }
 }
+int dtype_code(const Tensor& t) { return dtype_code(t.scalar_type()); }
 
 void need_cuda(const Tensor& t) {
   if (!t.is_cuda()) raise(PyExc_ValueError, "triton_b200 operators take CUDA tensors only (no CPU path)");
@@ -234,6 +236,21 @@ Tensor gemm(const Tensor& a, int kind, const Tensor& w, const OptTensor& ws, int
   g.status = status.data_ptr<int32_t>();
   check(run_gemm(g, a), "moe_grouped_gemm", true);
   return out;
+}
+
+// name of the kernel of a ragged product of M rows on aligned operands in weight tiles `kind` (no tensors: a question to the dispatch)
+std::string gemm_kernel(int kind, int64_t E, int64_t K, int64_t N, int64_t M, py::object x_dtype, py::object y_dtype, const py::tuple& tuning) {
+  MoeGemmArgs g{};
+  void* const some = (void*)(uintptr_t)4096;
+  g.x = g.y = some; g.w = some; g.w_scale = (const uint8_t*)some; g.w_kind = kind;
+  g.slice_sizes = g.slice_offs = g.block_offs_16 = g.block_sched_16 = (const int32_t*)some;
+  g.E = (int)E; g.K = (int)K; g.N = (int)N; g.M = g.rows_x = M; g.ld_x = K; g.ld_y = N;
+  g.x_dtype = dtype_code(torch::python::detail::py_object_to_dtype(x_dtype));
+  g.y_dtype = dtype_code(torch::python::detail::py_object_to_dtype(y_dtype));
+  set_tuning(g, tuning);
+  const char* name = lib.moe_gemm_kernel_name(&g);
+  if (!name) raise(inapplicable, lib.moe_last_error());
+  return name;
 }
 
 // ---- one layer step ------------------------------------------------------------------------------------------------
@@ -443,6 +460,7 @@ PYBIND11_MODULE(_host, m) {
   m.def("route", &route);
   m.def("bitmatrix_metadata", &bitmatrix_metadata);
   m.def("gemm", &gemm);
+  m.def("gemm_kernel", &gemm_kernel);
   m.def("layer", &layer);
   m.def("downcast", &downcast);
   m.def("upcast", &upcast);

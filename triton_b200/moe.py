@@ -79,6 +79,12 @@ class MoeLayerWeights:
         two = (self.w2_bs, self.w2_bs_scale) if self.use_block_scaled(n_rows, self.b2.shape[1]) else (self.w2, self.w2_scale)
         return (*one, *two)
 
+    def kernels(self, n_rows: int, dtype: torch.dtype = torch.bfloat16) -> tuple[str, str]:
+        """Names of the kernels that fc1 and fc2 of a step of `n_rows` routed rows run on under the current tuning constraints."""
+        w1, s1, w2, s2 = _step_weights(dtype, self, n_rows)
+        return tuple(_lib.host().gemm_kernel(_product(w, s)[0], *w.shape, n_rows, dtype, out, gemm_tuning())
+                     for w, s, out in ((w1, s1, dtype), (w2, s2, torch.bfloat16)))
+
     def weight_bytes(self):
         return sum(t.storage.data.numel() for t in (self.w1, self.w1_scale, self.w2, self.w2_scale)) + \
             self.b1.numel() * self.b1.element_size() + self.b2.numel() * self.b2.element_size()
@@ -114,9 +120,9 @@ _LAYER_KIND = {B200MXValueLayout: (_lib.MOE_W_MX4_B200, B200MXScaleLayout),
                B200BlockScaledValueLayout: (_lib.MOE_W_MX4_B200MX, B200BlockScaledScaleLayout)}
 
 
-def _step_weights(x, lw: MoeLayerWeights, n_rows: int):
+def _step_weights(dtype, lw: MoeLayerWeights, n_rows: int):
     """(w1, scales, w2, scales) of a step of `n_rows` routed rows: e4m3 tokens are multiplied on the block-scaled copy only."""
-    if x.dtype == torch.float8_e4m3fn:
+    if dtype == torch.float8_e4m3fn:
         return lw.w1_bs, lw.w1_bs_scale, lw.w2_bs, lw.w2_bs_scale
     return lw.fc_weights(n_rows)
 
@@ -144,7 +150,7 @@ def _one_call(x, logits, lw: MoeLayerWeights, k: int, weights=None) -> bool:
             and E == lw.n_expts and 0 < k <= E and x.ndim == 2 and x.stride(1) == 1 and logits.stride(1) == 1
             and 0 < x.shape[0] <= FUSED_MAX_TOKENS and logits.shape[0] == x.shape[0]):
         return False
-    w1, w1_scale, w2, w2_scale = _step_weights(x, lw, x.shape[0] * k) if weights is None else weights
+    w1, w1_scale, w2, w2_scale = _step_weights(x.dtype, lw, x.shape[0] * k) if weights is None else weights
     return (_product_fits(w1, w1_scale, lw.b1, E, x.shape[1]) and w1.shape[2] % 2 == 0
             and _product_fits(w2, w2_scale, lw.b2, E, w1.shape[2] // 2))
 
@@ -156,7 +162,7 @@ def moe_layer_forward(x, logits, lw: MoeLayerWeights, k: int, gemm_timer=None):
     e4m3 activations (`x.dtype == torch.float8_e4m3fn`, the reference's fp8 mode: bench/bench_mlp.py `x_dtype="fp8"`) run
     both GEMMs on the block-scaled kernel at every size: fc1 writes e4m3 rows, fc2 reads them and writes bf16."""
     T = x.shape[0]
-    weights = _step_weights(x, lw, T * k)
+    weights = _step_weights(x.dtype, lw, T * k)
     if gemm_timer is None and _one_call(x, logits, lw, k, weights):
         w1, w1_scale, w2, w2_scale = weights
         return _lib.host().layer(x, logits, k, (*_product(w1, w1_scale), lw.b1, *w1.shape[1:]),

@@ -262,6 +262,9 @@ typedef struct {
   void* mx_workspace; int64_t mx_workspace_bytes;
   int idle_sms;                                    /* persistent kernels leave this many SMs without a CTA
                                                       (matmul.py:239-243 matmul_set_idle_sms of the reference) */
+  int rows_per_expert;                             /* mean rows per expert to expect where M is far above them (a shard that
+                                                      holds the rows of its own experts only); 0: M / E.  Steers the choice
+                                                      of the block-scaled kernel, never a bound. */
 } MoeGemmArgs;
 int moe_grouped_gemm(const MoeGemmArgs* args_host, void* stream);
 size_t moe_gemm_mx_workspace_bytes(const MoeGemmArgs* args_host);

@@ -433,3 +433,24 @@ def test_pair_kernel_expert_of_more_rows_than_a_schedule_entry_counts(tiled, dev
             # an fp32 sum of 32 exact products, the second term's underflow 2^-23 of the group's maximum
             assert ((y[row:row + n] - ref).norm(dim=1) <= 2e-5 * ref.norm(dim=1) + 1e-6).all(), e
         row += n
+
+
+def test_expected_rows_choose_the_kernel(device):
+    """A shard's metadata bounds its rows by those of all ranks; the rows it says to expect decide between the decode and the pair
+    kernel (same bits as that kernel asked for by its block)."""
+    g = torch.Generator().manual_seed(3)
+    E, K, N, sizes = 16, 1024, 1536, [4, 3, 0, 5] * 4
+    M = 512
+    wq, ws, _ = quantised_weights(E, K, N, g)
+    tq, ts = to_block_scaled(wq, ws, device)
+    x = torch.randn(M, K, generator=g).bfloat16().to(device)
+    y = {}
+    for expected, cons in ((None, {}), (None, {"block_m": 256}), (4, {}), (None, {"block_m": 32})):
+        md = tb.make_ragged_tensor_metadata(torch.tensor(sizes, dtype=torch.int32, device=device), M)
+        md.expected_slice_size = expected
+        with tb.scoped_opt_flags_constraints(cons):
+            y[expected, tuple(cons.values())] = tb.matmul(x, tq, None, md, precision_config=tb.PrecisionConfig(b_mx_scale=ts, b_microblock_size=32),
+                                                          c=torch.zeros(M, N, dtype=torch.bfloat16, device=device))
+    tb.matmul_check_status()
+    assert torch.equal(y[None, ()], y[None, (256,)]) and torch.equal(y[4, ()], y[None, (32,)])
+    assert oracle.rel_l2(y[None, ()].cpu(), y[4, ()].cpu()) < 1e-2

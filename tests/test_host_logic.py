@@ -402,3 +402,17 @@ def test_kernels_of_a_step():
         assert both.kernels(3 * 100) == (tc,) * 2
         with pytest.raises(triton_b200.InapplicableConstraint):
             both.kernels(3 * 8)
+
+
+def test_kernel_of_a_shard_goes_by_its_own_rows(monkeypatch):
+    """Eight ranks, 16 experts each, 512 routed rows in all: four rows per expert, not the 32 that the bound on the rows suggests."""
+    from triton_b200 import _lib, moe
+    kernel = lambda kind, M, rows: _lib.host().gemm_kernel(kind, 16, 2880, 5760, M, torch.bfloat16, torch.bfloat16, (0, 0, 0, 0), rows)
+    mx, default = _lib.MOE_W_MX4_B200MX, _lib.MOE_W_MX4_B200
+    assert kernel(mx, 512, 0) == "gemm_mx_pair_kernel" and kernel(mx, 512, 4) == kernel(mx, 64, 0) == "gemm_mx_kernel"
+    assert kernel(mx, 512, 1000) == kernel(mx, 512, 0)                  # never above what the bound allows
+    assert kernel(default, 8 * 512 * 16, 512) == kernel(default, 512 * 16, 0) == "gemm_mx_pair_kernel"
+    md = triton_b200.RaggedTensorMetadata(*(torch.zeros(s, dtype=torch.int32) for s in ((2,), (3,), (4, 3), (4, 3))))
+    monkeypatch.setattr(moe, "remap_ragged_tensor_metadata", lambda meta, table: md)
+    assert moe._local_metadata(None, None, 512 // 8, 16).expected_slice_size == 4
+    assert moe._local_metadata(None, None, 1, 16).expected_slice_size == 1

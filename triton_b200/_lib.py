@@ -49,7 +49,7 @@ class MoeGemmArgs(C.Structure):
         ("kernel", i32), ("tile_m", i32), ("tile_n", i32), ("status", vp),
         ("y_peers", vp * 16), ("n_y_peers", i32), ("y_rows_per_peer", i64),
         ("gather_scratch", vp), ("gather_scratch_bytes", i64),
-        ("x_scale", vp), ("ld_x_scale", i64), ("mx_workspace", vp), ("mx_workspace_bytes", i64), ("idle_sms", i32),
+        ("x_scale", vp), ("ld_x_scale", i64), ("mx_workspace", vp), ("mx_workspace_bytes", i64), ("idle_sms", i32), ("rows_per_expert", i32),
     ]
 
 

@@ -598,8 +598,14 @@ PairPlan pair_plan(const MoeGemmArgs& a) {
 // - One weight block per tile where twice the tiles still run at a time (8 experts of 512 x 2048, 16 rows: 19 -> 17); beyond, a
 //   tile of two blocks reads the tokens once for both (32 experts, 64 rows: 91 against 105).
 struct PairShape { int nmax, upt, form; };
+// mean rows per expert: what the caller expects, else the bound on the rows over the experts
+int64_t mean_rows(const MoeGemmArgs& a) {
+  const int64_t mean = a.M / (a.slice_sizes ? a.E : 1);
+  return a.rows_per_expert > 0 && a.rows_per_expert < mean ? a.rows_per_expert : mean;
+}
+
 PairShape pair_shape(const MoeGemmArgs& a, int terms) {
-  const int64_t experts = a.slice_sizes ? a.E : 1, per = a.M / experts;
+  const int64_t experts = a.slice_sizes ? a.E : 1, per = mean_rows(a);
   PairShape s;
   s.form = terms == 1 ? PP_ONE : (per < 56 ? PP_SIDE : PP_TWO);
   s.nmax = s.form == PP_SIDE ? 96 : s.form == PP_TWO ? 128 : 192;
@@ -695,7 +701,7 @@ int launch_mx_pair_ty(const GemmParams& p, const PairParams& q, const MoeGemmArg
 bool moe_gemm_mx_pair_wanted(const MoeGemmArgs& a) {
   if (a.slice_sizes && a.E > MAX_PREFIX_EXPERTS) return false;
   if (a.M >= (1ll << 31) - (1 << 20) || a.kernel == MOE_GEMM_MX_F4 || a.tile_n != 0) return false;
-  const int64_t experts = a.slice_sizes ? a.E : 1, per = a.M / experts;
+  const int64_t experts = a.slice_sizes ? a.E : 1, per = mean_rows(a);
   const int64_t load = (experts < a.M ? experts : a.M) * a.N * a.K;
   if (a.w_kind == MOE_W_MX4_B200) {
     // default tiles, bf16 tokens

@@ -192,7 +192,8 @@ void set_weights(MoeGemmArgs& g, int kind, const Tensor& w, const OptTensor& ws)
   }
 }
 
-// y is the caller's output tensor or None (allocated here); `ragged` is (slice_sizes, slice_offs, block_offs, schedule) or None;
+// y is the caller's output tensor or None (allocated here); `ragged` is (slice_sizes, slice_offs, block_offs, schedule, expected
+// rows per expert or 0) or None;
 // `peers` is (device addresses, rows per peer) or None.
 Tensor gemm(const Tensor& a, int kind, const Tensor& w, const OptTensor& ws, int64_t E, int64_t K, int64_t N, const py::object& ragged,
             const OptTensor& bias, const OptTensor& gather, const OptTensor& scatter, const OptTensor& betas, const OptTensor& gammas,
@@ -213,6 +214,7 @@ Tensor gemm(const Tensor& a, int kind, const Tensor& w, const OptTensor& ws, int
     g.slice_sizes = sizes.data_ptr<int32_t>(); g.slice_offs = offs.data_ptr<int32_t>();
     g.block_offs_16 = boffs.data_ptr<int32_t>(); g.block_sched_16 = sched.data_ptr<int32_t>();
     g.ld_block_offs = boffs.stride(0); g.ld_block_sched = sched.stride(0);
+    g.rows_per_expert = r[4].cast<int>();
   }
   if (bias) { g.bias = bias->data_ptr(); g.bias_dtype = dtype_code(*bias); g.ld_bias = bias->stride(0); }
   g.gather_indx = i32(gather, keep); g.scatter_indx = i32(scatter, keep);
@@ -239,7 +241,8 @@ Tensor gemm(const Tensor& a, int kind, const Tensor& w, const OptTensor& ws, int
 }
 
 // name of the kernel of a ragged product of M rows on aligned operands in weight tiles `kind` (no tensors: a question to the dispatch)
-std::string gemm_kernel(int kind, int64_t E, int64_t K, int64_t N, int64_t M, py::object x_dtype, py::object y_dtype, const py::tuple& tuning) {
+std::string gemm_kernel(int kind, int64_t E, int64_t K, int64_t N, int64_t M, py::object x_dtype, py::object y_dtype, const py::tuple& tuning,
+                        int rows_per_expert) {
   MoeGemmArgs g{};
   void* const some = (void*)(uintptr_t)4096;
   g.x = g.y = some; g.w = some; g.w_scale = (const uint8_t*)some; g.w_kind = kind;
@@ -248,6 +251,7 @@ std::string gemm_kernel(int kind, int64_t E, int64_t K, int64_t N, int64_t M, py
   g.x_dtype = dtype_code(torch::python::detail::py_object_to_dtype(x_dtype));
   g.y_dtype = dtype_code(torch::python::detail::py_object_to_dtype(y_dtype));
   set_tuning(g, tuning);
+  g.rows_per_expert = rows_per_expert;
   const char* name = lib.moe_gemm_kernel_name(&g);
   if (!name) raise(inapplicable, lib.moe_last_error());
   return name;
@@ -460,7 +464,8 @@ PYBIND11_MODULE(_host, m) {
   m.def("route", &route);
   m.def("bitmatrix_metadata", &bitmatrix_metadata);
   m.def("gemm", &gemm);
-  m.def("gemm_kernel", &gemm_kernel);
+  m.def("gemm_kernel", &gemm_kernel, py::arg("kind"), py::arg("E"), py::arg("K"), py::arg("N"), py::arg("M"), py::arg("x_dtype"),
+        py::arg("y_dtype"), py::arg("tuning"), py::arg("rows_per_expert") = 0);
   m.def("layer", &layer);
   m.def("downcast", &downcast);
   m.def("upcast", &upcast);

@@ -336,7 +336,8 @@ def matmul(a, b, bias,
     ragged = None
     if a_ragged_metadata is not None:
         md = a_ragged_metadata
-        ragged = (md.slice_sizes, md.slice_offs, md.block_offs_data, md.block_schedule_data)
+        ragged = (md.slice_sizes, md.slice_offs, md.block_offs_data, md.block_schedule_data,
+                  min(max(int(md.expected_slice_size or 0), 0), 2**31 - 1))
     if bias is not None:
         if bias.ndim == 1:
             bias = bias.view(1, -1)

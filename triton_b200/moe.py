@@ -310,8 +310,9 @@ def _forward_ep_peer(x_local, sparse, lw_local, k, expt_assignment, pool, gemm_t
     md = sparse.mask_metadata
     n = md.row_sorted_indx.shape[0]
     dev = x_local.device
+    E_loc = lw_local.n_expts
     meta_global = make_ragged_tensor_metadata(md.col_sum, n)
-    meta_local = remap_ragged_tensor_metadata(meta_global, expt_assignment.expt_map[rank, :])
+    meta_local = _local_metadata(meta_global, expt_assignment.expt_map[rank, :], n // W, E_loc)
     col = md.col_sorted_indx.reshape(-1)                               # flat (token * k + slot) of every position
     # positions whose expert lives here pull their token's row; all others are skipped (and never read by the GEMMs)
     src_row = torch.empty(n, dtype=torch.int32, device=dev)
@@ -326,7 +327,6 @@ def _forward_ep_peer(x_local, sparse, lw_local, k, expt_assignment, pool, gemm_t
                "moe_ep_pull_index")
     chunks = int(getattr(pool, "overlap_chunks", 1))
     w1, w1_scale, w2, w2_scale = lw_local.fc_weights(n // W)            # rows this rank multiplies, on average
-    E_loc = lw_local.n_expts
     if (lw_local.use_block_scaled(n // W) and n // W <= lw_local.block_scaled_max_rows_per_expert * E_loc) or E_loc < 2:
         chunks = 1
     chunks = max(1, min(chunks, E_loc))
@@ -344,7 +344,7 @@ def _forward_ep_peer(x_local, sparse, lw_local, k, expt_assignment, pool, gemm_t
             _lib.check(lib.moe_ep_pull_index(_lib.ptr(col), _lib.ptr(indx16), _lib.ptr(sparse.vals.contiguous()),
                                              _lib.ptr(table), n, k, _lib.ptr(rows_c), _lib.ptr(gammas), _lib.stream()),
                        "moe_ep_pull_index")
-            plan.append((rows_c, remap_ragged_tensor_metadata(meta_global, table), lo_e, hi_e))
+            plan.append((rows_c, _local_metadata(meta_global, table, n // W, E_loc), lo_e, hi_e))
     if not tokens_published:                                           # (the caller did both ahead of the routing barrier)
         if x_local.data_ptr() != pool.xbuf.data_ptr():                 # a caller may keep its tokens in the pool's buffer
             pool.xbuf.copy_(x_local)
@@ -407,6 +407,14 @@ def _forward_ep_peer(x_local, sparse, lw_local, k, expt_assignment, pool, gemm_t
                                                 _lib.ptr(z), z.stride(0), _lib.stream()), "moe_gather_reduce_rows_peers")
     mark("output barrier + combine")
     return z
+
+
+def _local_metadata(meta_global, expt_map, n_rows: int, n_expts: int):
+    """Ragged metadata of one rank's experts.  Its arrays keep the global row count as their bound; `n_rows` is what the rank is
+    to expect of them on average, which the library's choice of kernel goes by."""
+    md = remap_ragged_tensor_metadata(meta_global, expt_map)
+    md.expected_slice_size = max(1, n_rows // n_expts)
+    return md
 
 
 def _expert_range(t: Tensor, lo: int, hi: int) -> Tensor:
@@ -478,7 +486,7 @@ def moe_layer_forward_ep(x_local, logits_local, lw_local: MoeLayerWeights, k: in
     n_entries = md.row_sorted_indx.shape[0]
     meta_global = make_ragged_tensor_metadata(md.col_sum, n_entries)
     plan = make_exchange_plan_cuda(sparse.indx, md.col_sorted_indx, expt_assignment, pool.mesh.world_size, T_local)
-    meta_local = remap_ragged_tensor_metadata(meta_global, expt_assignment.expt_map[rank, :])
+    meta_local = _local_metadata(meta_global, expt_assignment.expt_map[rank, :], n_entries // pool.mesh.world_size, lw_local.n_expts)
     gammas = sparse.vals.reshape(-1)[md.col_sorted_indx.long().clamp_min(0)]
     pc1 = PrecisionConfig(b_mx_scale=lw_local.w1_scale, b_microblock_size=32)
     pc2 = PrecisionConfig(b_mx_scale=lw_local.w2_scale, b_microblock_size=32)

@@ -454,3 +454,65 @@ def test_expected_rows_choose_the_kernel(device):
     tb.matmul_check_status()
     assert torch.equal(y[None, ()], y[None, (256,)]) and torch.equal(y[4, ()], y[None, (32,)])
     assert oracle.rel_l2(y[None, ()].cpu(), y[4, ()].cpu()) < 1e-2
+
+
+@pytest.mark.parametrize("tiled", [True, False])
+@pytest.mark.parametrize("sizes", [[20, 1, 0, 33], [70, 128, 0, 257]])       # terms side by side, and in two MMAs
+@pytest.mark.parametrize("mode", ["plain", "scatter", "swiglu", "bf16 out"])
+def test_pair_kernel_values_beyond_two_terms(tiled, sizes, mode, device):
+    """Rows with an infinity, or a finite value that e4m3 rounds to 2^128, come out as the product of bf16 values gives them: infinite
+    with the weight's sign, NaN where the weight is zero or infinities cancel, finite for the finite ones; other rows as ever.
+    Against the exact sums in 64 bits, and under SwiGLU (whose limit makes infinities finite) against the bf16 kernel."""
+    from triton_b200.tensor_details.layout import B200MXScaleLayout, B200MXValueLayout
+    g = torch.Generator().manual_seed(sum(sizes))
+    E, K, N, M = len(sizes), 416, 514, sum(sizes)
+    sizes_t = torch.tensor(sizes, dtype=torch.int32)
+    wq, ws, wdeq = quantised_weights(E, K, N, g)
+    T = M + 5
+    x = torch.randn(T, K, generator=g).bfloat16()
+    gather = torch.randperm(T, generator=g)[:M].int()
+    odd = {0: [(7, float("inf"))], sizes[0] - 1: [(415, float("-inf"))], sizes[0]: [(0, 3.3895e38)], M - 1: [(64, float("inf")), (65, float("-inf"))],
+           M - 2: [(100, -3.3e38), (300, 1.0)], 3: [(5, float("nan")), (200, float("inf"))]}
+    for m, values in odd.items():
+        for k, v in values:
+            x[gather[m].long(), k] = v
+    scatter = torch.randperm(M, generator=g).int() if mode == "scatter" else None
+    gammas, betas = (torch.rand(M, generator=g) + 0.5, torch.rand(M, generator=g)) if mode == "scatter" else (None, None)
+    if mode == "scatter":
+        scatter[0] = -1                                     # a dropped row, one of those with an infinity
+    bias = torch.randn(E, N, generator=g) * 0.1
+    dev = lambda t: None if t is None else t.to(device)
+    dw = convert_layout(wrap_torch_tensor(dev(wq), dtype=FP4), B200MXValueLayout()), convert_layout(wrap_torch_tensor(dev(ws)), B200MXScaleLayout())
+    bs = to_block_scaled(wq, ws, device)
+    fa = tb.FusedActivation(tb.FnSpecs("swiglu", tb.swiglu_fn, ("alpha", "limit"), reduction_n=2), (1.702, 7.0)) if mode == "swiglu" else None
+    out_dtype = torch.bfloat16 if mode == "bf16 out" else torch.float32
+
+    def run(w, s, cons):
+        with tb.scoped_opt_flags_constraints(cons):
+            y = tb.matmul(dev(x), w, dev(bias), tb.make_ragged_tensor_metadata(dev(sizes_t), M), None, dev(gather), dev(scatter),
+                          tb.PrecisionConfig(b_mx_scale=s, b_microblock_size=32, out_dtype=out_dtype), gammas=dev(gammas), betas=dev(betas),
+                          fused_activation=fa, c=torch.zeros(M, N // 2 if fa else N, dtype=out_dtype, device=device))
+        tb.matmul_check_status()
+        return y.cpu()
+
+    y = run(*dw, {"kernel": "mx"}) if tiled else run(*bs, {"block_m": 256})
+    if mode == "swiglu":
+        want = run(*dw, {"kernel": "tcgen05"}).double()
+    else:
+        want, row = torch.empty(M, N, dtype=torch.float64), 0
+        for e, n in enumerate(sizes):
+            beta = 1.0 if betas is None else betas[row:row + n, None].double()
+            want[row:row + n] = x[gather[row:row + n].long()].double() @ wdeq[e].double() + bias[e].double() * beta
+            row += n
+        if mode == "scatter":
+            out = torch.zeros_like(want)
+            out[scatter[1:].long()] = (want * gammas[:, None].double())[1:]
+            want = out
+        assert torch.isinf(want).any() and torch.isnan(want).any()
+    assert torch.equal(torch.isnan(y), torch.isnan(want)) and torch.equal(torch.isposinf(y), torch.isposinf(want))
+    assert torch.equal(torch.isneginf(y), torch.isneginf(want))
+    # rows without such values, and those with large finite ones: fp32 sums of exact products (SwiGLU passes them on), relative to
+    # the row; 1e-4 leaves room for a gate at the edge of the limit, 2^-8 is bf16's rounding
+    for got, ref in zip(y, want):
+        keep = torch.isfinite(ref)
+        assert (got.double() - ref)[keep].norm() <= (2.0 ** -8 if mode == "bf16 out" else 1e-4) * ref[keep].norm() + 1e-6

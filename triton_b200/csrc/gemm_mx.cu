@@ -34,7 +34,6 @@
 // Warps: 0 producer, 1 MMA issue + tensor-memory owner, 2-5 epilogue, 6-9 scale loaders.  Every mbarrier
 // wait is bounded.
 #include "gemm_mx_common.cuh"
-#include <cuda_fp4.h>
 #include <utility>
 
 namespace {
@@ -208,10 +207,6 @@ __global__ void __launch_bounds__(256) mx_pack_x_kernel(const GemmParams p, cons
 // took 13.6-14.4 us, so 10.5-11.1.
 __device__ __forceinline__ uint32_t f32x2_to_e2m1x2(float lo, float hi) {       // `lo` in bits 0..3
   return (uint32_t)__nv_cvt_float2_to_fp4x2(make_float2(lo, hi), __NV_E2M1, cudaRoundNearest);
-}
-__device__ __forceinline__ float2 e2m1x2_to_f32x2(uint32_t c) {
-  const __half2_raw h = __nv_cvt_fp4x2_to_halfraw2((__nv_fp4x2_storage_t)c, __NV_E2M1);
-  return __half22float2(__half2(h));
 }
 // e8m0 byte s with 2^(s-127) >= amax / 6, and the exact factors 2^(s-127), 2^(127-s)
 __device__ __forceinline__ void mx4_scale(float amax, uint32_t& sb, float& scale, float& inv) {

@@ -1,6 +1,7 @@
 // Pieces shared by the block-scaled GEMM kernels: e4m3 conversions and their e8m0 scales, the weight tensor map.
 #pragma once
 #include "gemm_tc_common.cuh"
+#include <cuda_fp4.h>
 #include <cuda_fp8.h>
 
 // e4m3 output (the next GEMM's activations): round to nearest, saturating at +-448 like the MMA's own conversions
@@ -21,6 +22,10 @@ __device__ __forceinline__ float2 e4m3x2_to_f32x2(uint32_t v) {
   uint32_t h2;
   asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(h2) : "h"((uint16_t)v));
   return __half22float2(*reinterpret_cast<__half2*>(&h2));
+}
+__device__ __forceinline__ float2 e2m1x2_to_f32x2(uint32_t c) {
+  const __half2_raw h = __nv_cvt_fp4x2_to_halfraw2((__nv_fp4x2_storage_t)c, __NV_E2M1);
+  return __half22float2(__half2(h));
 }
 // e8m0 byte s with 2^(s-127) >= amax / 448 (smallest such power of two), and the exact factors 2^(s-127), 2^(127-s)
 __device__ __forceinline__ void mx8_scale(float amax, uint32_t& sb, float& scale, float& inv) {

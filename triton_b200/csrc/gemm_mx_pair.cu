@@ -7,6 +7,9 @@
 // time kind::f16 does K = 16 (measured: 4.4 PFLOP/s for N >= 128 on 148 SMs, so two terms run at 2.2 -- the bf16 rate).
 //
 // (Elements far below their group of 32's largest lose what lies below 2^-23 of it, as much as an fp32 sum rounds away.)
+// A row with a value beyond e4m3's scales (infinite, or near the end of bf16's range) is computed by the pack kernel in fp32, and
+// the GEMM kernel does not store it.  (The pack kernel's word per 16 rows and its look-up cost about 1 us of 183 for fc1 + fc2 of 32
+// experts, 300 tokens; the same recomputation called from this kernel's epilogue took 7, by the code the call made of the rest.)
 //
 // What bounds it.  Shared memory, 128 B per cycle and SM: every operand byte is written once and read once per MMA, and an
 // e2m1 value takes a byte there.  A cluster of two CTAs computes (2 x 256 weight rows) x (up to 128 tokens of two terms, 192 of
@@ -58,6 +61,7 @@ template <int FORM> constexpr int SF_COLS = FORM == PP_TWO ? 24 : 16;      // te
 struct PairParams {
   const uint8_t* xq;            // [k step][padded row / 8][term][8 rows][128 B], 16-byte pieces swizzled with (row & 7)
   const uint8_t* xs;            // [k step][padded row / 8][term][8 rows][4 B]: e8m0 of the four 32-groups
+  const uint32_t* done;         // [padded row / 16]: bit of each row whose outputs the pack kernel has written itself (two-term tokens)
   int64_t prows;                // padded rows: expert e's rows start at (slice_offs[e] & ~31) + 32 e
   int KT, NB;                   // 128-k steps, 128-row weight blocks
   int nmax;                     // token columns of a tile at most, a multiple of 32
@@ -84,9 +88,10 @@ struct PairPackParams {
   const void* x; int64_t ld_x; int64_t rows_x;
   const uint8_t* x_scale; int64_t ld_xs;
   const int32_t* gather;
-  int K, KT;
+  int K, KT, NB, y_dtype;
   int64_t prows;
   uint8_t* xq; uint8_t* xs;
+  uint32_t* done;
 };
 
 __device__ __forceinline__ bool pack_block(const GemmParams& p, int64_t pid, int& e, int64_t& row0, int& rows, int64_t& prow0) {
@@ -110,14 +115,81 @@ __device__ __forceinline__ bool pack_block(const GemmParams& p, int64_t pid, int
   return rows > 0;
 }
 
+// Magnitude from which on two e4m3 terms do not hold a token's value: infinities, and finite values that round to 2^128.
+constexpr float BEYOND = 3.0e38f;
+
+// Output of a row with such a value, in fp32 on the CUDA cores by one warp, 32 weight rows at a time: what the product of bf16 values
+// gives (an infinite token value times a weight is infinite, or NaN for a zero weight).
+template <typename TY, bool TILED>
+__device__ void exact_row(const GemmParams& p, const PairPackParams& a, int e, int64_t m, int64_t dst, const __nv_bfloat16* x, int lane) {
+  TY* y = gemm_out_row<TY>(p, dst);
+  for (int n = lane; n - lane < p.N; n += 32) {
+    const int b = n >> 7, row = n & 127;
+    float acc = 0.0f;
+    for (int kg = 0; kg < p.K >> 5; ++kg) {                        // scale groups of 32 k
+      const int kt = kg >> 2, g = kg & 3;
+      const int64_t at = TILED ? ((int64_t)e * a.NB + b) * a.KT + kt : ((int64_t)e * a.KT + kt) * a.NB + b;
+      const uint8_t* q = (const uint8_t*)p.w + at * 8192 + (TILED ? (g * 128 + row) * 16 : row * 64 + g * 16);
+      const uint32_t sb = p.w_scale[at * 512 + (TILED ? row * 4 + g : (row & 31) * 16 + (row >> 5) * 4 + g)];
+      const float s = __uint_as_float(sb ? (sb == 255u ? 0x7FC00000u : sb << 23) : 0x00400000u);
+      for (int i = 0; i < 4; ++i) {                                // words of eight values
+        uint32_t w = reinterpret_cast<const uint32_t*>(q)[i];
+        if (TILED) {                                               // evens, then odds: back to pairs
+          uint32_t pairs = 0;
+          for (int j = 0; j < 4; ++j) pairs |= (((w >> (4 * j)) & 0xFu) | (((w >> (16 + 4 * j)) & 0xFu) << 4)) << (8 * j);
+          w = pairs;
+        }
+        for (int j = 0; j < 4; ++j) {
+          const float2 f = e2m1x2_to_f32x2((w >> (8 * j)) & 0xFFu);
+          const int k = kg * 32 + 8 * i + 2 * j;
+          acc = fmaf(__bfloat162float(x[k]), f.x * s, acc);
+          acc = fmaf(__bfloat162float(x[k + 1]), f.y * s, acc);
+        }
+      }
+    }
+    if (p.bias && n < p.N) acc += load_bias(p.bias, p.bias_dtype, (int64_t)e * p.ld_bias + n) * (p.betas ? p.betas[m] : 1.0f);
+    if (p.has_out_alpha) acc *= p.out_alpha;
+    const float gamma = p.gammas ? p.gammas[m] : 1.0f, other = __shfl_xor_sync(0xFFFFFFFFu, acc, 1);
+    if (p.activation == MOE_ACT_SWIGLU) {
+      if (!(lane & 1) && n + 1 < p.N) y[n >> 1] = from_f32<TY>(gemm_swiglu(acc, other, p.act_alpha, p.act_limit, p.act_has_limit) * gamma);
+    } else if (n < p.N) {
+      y[n] = from_f32<TY>(acc * gamma);
+    }
+  }
+}
+
+// The rows with such a value among a block's; all of its threads call.  -> their bits
+template <bool TILED>
+__device__ __noinline__ uint32_t exact_rows(const GemmParams& p, const PairPackParams& a, int e, int64_t row0, int rows) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint32_t mine = 0;
+  for (int r = warp; r < rows; r += 8) {
+    const int64_t m = row0 + r, src = p.gather_indx ? (int64_t)p.gather_indx[m] : m, d = p.scatter_indx ? (int64_t)p.scatter_indx[m] : m;
+    if (src < 0 || src >= a.rows_x) continue;
+    const __nv_bfloat16* x = (const __nv_bfloat16*)a.x + src * a.ld_x;
+    bool is = false;
+    for (int k = lane; k < a.K; k += 32) is |= fabsf(__bfloat162float(x[k])) >= BEYOND;
+    if (!__any_sync(0xFFFFFFFFu, is)) continue;
+    mine |= 1u << r;
+    if (d < 0) continue;
+    if (a.y_dtype == MOE_BF16) exact_row<__nv_bfloat16, TILED>(p, a, e, m, d, x, lane);
+    else if (a.y_dtype == MOE_F32) exact_row<float, TILED>(p, a, e, m, d, x, lane);
+    else exact_row<__nv_fp8_e4m3, TILED>(p, a, e, m, d, x, lane);
+  }
+  uint32_t all = 0;
+  for (int r = 0; r < 16; ++r) all |= __syncthreads_or((mine >> r) & 1u) ? 1u << r : 0u;
+  return all;
+}
+
 // TILED: k inside eight in the order of the default weight tiles (0, 2, 4, 6, 1, 3, 5, 7).  A thread takes a whole group of 32 k:
 // no exchange between lanes, 64 bytes in, a 32-byte sector out per term.  With eight k per lane and four lanes to a group, 65536
 // rows of 2880 took 153 us and 4800 rows 20.3, so 141 and 16.8.
 template <bool TILED>
-__global__ void __launch_bounds__(256) mx_pair_pack2_kernel(const GemmParams p, const PairPackParams a) {
+__global__ void __launch_bounds__(256) mx_pair_pack2_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ PairPackParams a) {
   int e; int64_t row0, prow0; int rows;
   if (!pack_block(p, blockIdx.x, e, row0, rows, prow0)) return;
   const int G = a.KT * 4;
+  bool beyond = false;
   for (int t = threadIdx.x; t < rows * G; t += 256) {
     const int r = t / G, g = t - r * G;
     int64_t src = a.gather ? (int64_t)a.gather[row0 + r] : row0 + r;
@@ -141,12 +213,7 @@ __global__ void __launch_bounds__(256) mx_pair_pack2_kernel(const GemmParams p, 
         m = fmaxf(m, fmaxf(fabsf(lo), fabsf(hi)));
       }
     }
-    if (!(m < 3.0e38f)) {                              // Inf in the group: keep the scale finite; e4m3 has no Inf, a NaN makes
-      m = 3.0e38f;                                     // the row's results NaN
-#pragma unroll
-      for (int i = 0; i < 32; ++i)
-        if (!(fabsf(v[i]) < 3.4e38f)) v[i] = __uint_as_float(0x7FC00000u);
-    }
+    beyond |= !(m < BEYOND);                           // (what is packed of such a row is not used; a NaN makes its results NaN)
     uint32_t sh; float s_hi, i_hi;
     mx8_scale(m, sh, s_hi, i_hi);
     uint32_t h[8], l[8];
@@ -177,6 +244,9 @@ __global__ void __launch_bounds__(256) mx_pair_pack2_kernel(const GemmParams p, 
     sd[0] = (uint8_t)sh;
     sd[32] = (uint8_t)sl;
   }
+  uint32_t done = 0;
+  if (__syncthreads_or(beyond)) done = exact_rows<TILED>(p, a, e, row0, rows);
+  if (threadIdx.x == 0) a.done[prow0 >> 4] = done;
 }
 
 __global__ void __launch_bounds__(256) mx_pair_pack1_kernel(const GemmParams p, const PairPackParams a) {
@@ -500,7 +570,11 @@ gemm_mx_pair_kernel(const GemmParams p, const PairParams a, const __grid_constan
       const PTile t = map_ptile(p, s_prefix, tile / MT);
       const Blocks b = blocks_of(tile);
       const uint32_t tab = ctl0 + (tc & 1u) * PAIR_TAB;
-      if (tid < t.cols) pair_table_entry<TY>(p, t, tid, tab);
+      if (tid < t.cols) {
+        bool stored = tid < t.rows;                    // not by the pack kernel
+        if (TERMS == 2 && stored) stored = !((a.done[(padded_base(t.e, t.off) + t.first + tid) >> 4] >> (tid & 15)) & 1u);
+        pair_table_entry<TY>(p, t, tid, stored, tab);
+      }
       float bias_m[2];
 #pragma unroll
       for (int m = 0; m < 2; ++m) {
@@ -575,7 +649,7 @@ gemm_mx_pair_kernel(const GemmParams p, const PairParams a, const __grid_constan
 // ---- host side -----------------------------------------------------------------------------------------------
 struct PairPlan {
   int KT, NB, terms;
-  int64_t prows, xs_off, ws_bytes;
+  int64_t prows, xs_off, done_off, ws_bytes;
 };
 
 PairPlan pair_plan(const MoeGemmArgs& a) {
@@ -586,7 +660,8 @@ PairPlan pair_plan(const MoeGemmArgs& a) {
   const int64_t E = a.slice_sizes ? a.E : 1;
   pl.prows = cdiv64(a.M, 32) * 32 + 32 * (E + 1);
   pl.xs_off = pl.terms * pl.KT * pl.prows * 128;
-  pl.ws_bytes = pl.xs_off + pl.terms * pl.KT * pl.prows * 4;
+  pl.done_off = pl.xs_off + pl.terms * pl.KT * pl.prows * 4;
+  pl.ws_bytes = pl.done_off + pl.prows / 16 * 4;
   return pl;
 }
 
@@ -739,15 +814,15 @@ int moe_gemm_mx_pair_launch(const GemmParams& p_in, const MoeGemmArgs& a, cudaSt
   pk.x = a.x; pk.ld_x = a.ld_x; pk.rows_x = a.rows_x;
   pk.x_scale = a.x_scale; pk.ld_xs = a.ld_x_scale;
   pk.gather = a.gather_indx;
-  pk.K = a.K; pk.KT = pl.KT; pk.prows = pl.prows;
-  pk.xq = (uint8_t*)a.mx_workspace; pk.xs = pk.xq + pl.xs_off;
+  pk.K = a.K; pk.KT = pl.KT; pk.NB = pl.NB; pk.y_dtype = a.y_dtype; pk.prows = pl.prows;
+  pk.xq = (uint8_t*)a.mx_workspace; pk.xs = pk.xq + pl.xs_off; pk.done = (uint32_t*)(pk.xq + pl.done_off);
   const bool tiled = a.w_kind == MOE_W_MX4_B200;
   if (pl.terms == 2 && tiled) mx_pair_pack2_kernel<true><<<(unsigned)blocks16, 256, 0, st>>>(p, pk);
   else if (pl.terms == 2) mx_pair_pack2_kernel<false><<<(unsigned)blocks16, 256, 0, st>>>(p, pk);
   else mx_pair_pack1_kernel<<<(unsigned)blocks16, 256, 0, st>>>(p, pk);
   MOE_CHECK_LAUNCH();
   PairParams q;
-  q.xq = pk.xq; q.xs = pk.xs; q.prows = pl.prows; q.KT = pl.KT; q.NB = pl.NB;
+  q.xq = pk.xq; q.xs = pk.xs; q.done = pk.done; q.prows = pl.prows; q.KT = pl.KT; q.NB = pl.NB;
   PairMaps maps;
   for (int n = 1; n <= 2; ++n) {
     // values as the TMA unit expands them (a row of a box: 64 bytes -> 128), scales as words; blocks along the slowest dimension

@@ -115,10 +115,10 @@ __device__ __forceinline__ void mul_f32x2(float& o0, float& o1, float a0, float 
 // tokens 8-15.  Row addresses and routing weights come from a table in shared memory, filled once per tile:
 // row address [256], gamma [256], beta [256].
 constexpr int PAIR_TAB = 256 * 16;
-template <typename TY> __device__ __forceinline__ void pair_table_entry(const GemmParams& p, const PTile& t, int tid, uint32_t tab) {
+template <typename TY> __device__ __forceinline__ void pair_table_entry(const GemmParams& p, const PTile& t, int tid, bool stored, uint32_t tab) {
   unsigned long long row = 0;
   float beta = 1.0f, gamma = 1.0f;
-  if (tid < t.rows) {
+  if (stored) {
     const int64_t m = t.row0 + tid;
     const int64_t d = p.scatter_indx ? (int64_t)p.scatter_indx[m] : m;
     if (d >= 0) row = (unsigned long long)gemm_out_row<TY>(p, d);

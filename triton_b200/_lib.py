@@ -33,27 +33,8 @@ class MoeDeviceInfo(C.Structure):
                 ("l2_bytes", sz), ("total_mem", sz)]
 
 
-class MoeGemmArgs(C.Structure):
-    _fields_ = [
-        ("x", vp), ("x_dtype", i32), ("ld_x", i64), ("rows_x", i64),
-        ("w_kind", i32), ("w", vp), ("w_stride_e", i64), ("w_stride_k", i64), ("w_stride_n", i64),
-        ("w_scale", vp), ("ws_stride_e", i64), ("ws_stride_k", i64), ("ws_stride_n", i64),
-        ("E", i32), ("K", i32), ("N", i32),
-        ("slice_sizes", vp), ("slice_offs", vp), ("block_offs_16", vp), ("block_sched_16", vp),
-        ("ld_block_offs", i64), ("ld_block_sched", i64), ("M", i64),
-        ("bias", vp), ("bias_dtype", i32), ("ld_bias", i64),
-        ("gather_indx", vp), ("scatter_indx", vp), ("betas", vp), ("gammas", vp),
-        ("out_alpha", f32), ("has_out_alpha", i32),
-        ("activation", i32), ("act_alpha", f32), ("act_limit", f32), ("act_has_limit", i32),
-        ("y", vp), ("y_dtype", i32), ("ld_y", i64),
-        ("kernel", i32), ("tile_m", i32), ("tile_n", i32), ("status", vp),
-        ("y_peers", vp * 16), ("n_y_peers", i32), ("y_rows_per_peer", i64),
-        ("gather_scratch", vp), ("gather_scratch_bytes", i64),
-        ("x_scale", vp), ("ld_x_scale", i64), ("mx_workspace", vp), ("mx_workspace_bytes", i64), ("idle_sms", i32), ("rows_per_expert", i32),
-    ]
-
-
-# name -> (restype, argtypes); must list every symbol declared in include/moe_b200.h
+# name -> (restype, argtypes); must list every symbol declared in include/moe_b200.h.  MoeGemmArgs goes by address: csrc/host.cpp
+# builds it from the header.
 PROTOTYPES = {
     "moe_last_error": (C.c_char_p, []),
     "moe_abi_version": (i32, []),
@@ -85,9 +66,9 @@ PROTOTYPES = {
     "moe_weight_layout_from_b200": (i32, [vp, vp, i32, i32, i32, vp, vp, vp]),
     "moe_weight_layout_to_b200mx": (i32, [vp, i64, i64, vp, i64, i64, i64, i32, i32, i32, vp, vp, vp]),
     "moe_weight_layout_from_b200mx": (i32, [vp, vp, i32, i32, i32, vp, vp, vp]),
-    "moe_grouped_gemm": (i32, [C.POINTER(MoeGemmArgs), vp]),
-    "moe_gemm_mx_workspace_bytes": (sz, [C.POINTER(MoeGemmArgs)]),
-    "moe_gemm_kernel_name": (C.c_char_p, [C.POINTER(MoeGemmArgs)]),
+    "moe_grouped_gemm": (i32, [vp, vp]),
+    "moe_gemm_mx_workspace_bytes": (sz, [vp]),
+    "moe_gemm_kernel_name": (C.c_char_p, [vp]),
     "moe_tensor_roof": (i32, [i32, i32, C.POINTER(C.c_double), vp, vp]),
     "moe_ep_keys": (i32, [vp, vp, vp, i64, i32, i32, vp, vp]),
     "moe_ep_pull_index": (i32, [vp, vp, vp, vp, i64, i32, vp, vp, vp]),

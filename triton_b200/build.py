@@ -32,7 +32,7 @@ def build_host():
     cuda = Path(_nvcc()).resolve().parent.parent
     inc = [*cpp_extension.include_paths(), str(cuda / "include"), sysconfig.get_paths()["include"]]
     tmp = HOST_LIB.with_suffix(".so.tmp")
-    subprocess.check_call([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-w",
+    subprocess.check_call([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-Wall", "-Wextra",
                            "-DTORCH_EXTENSION_NAME=_host", "-DTORCH_API_INCLUDE_EXTENSION_H",
                            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[f"-isystem{i}" for i in inc],
                            str(HOST_SRC), "-o", str(tmp), f"-L{cpp_extension.library_paths()[0]}", "-lc10", "-lc10_cuda",

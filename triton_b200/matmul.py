@@ -117,9 +117,9 @@ _STATUS_TEXT = {
     201: "tcgen05 kernel: the weight producer waited for a free stage", 301: "tcgen05 kernel: the activation loader waited for a free stage",
     401: "tcgen05 kernel: the dequantiser waited for packed weights", 402: "tcgen05 kernel: the dequantiser waited for a free stage",
     501: "tcgen05 kernel: the epilogue waited for an accumulator",
-    601: "block-scaled kernel: the producer waited for a free stage", 602: "block-scaled kernel: the MMA thread waited for a stage",
-    603: "block-scaled kernel: the MMA thread waited for a free accumulator", 604: "block-scaled kernel: the epilogue waited for an accumulator",
-    605: "block-scaled kernel: the final MMA drain", 606: "block-scaled kernel: the MMA thread waited for scales",
+    601: "block-scaled kernel: the producer waited for a free stage", 602: "block-scaled kernel: the MMA warp waited for a stage's scales",
+    603: "block-scaled kernel: the MMA warp waited for a free accumulator", 604: "block-scaled kernel: the epilogue waited for an accumulator",
+    605: "block-scaled kernel: the final MMA drain",
     607: "block-scaled kernel: a scale loader waited for a stage",
     611: "block-scaled pair kernel: the producer waited for a free stage", 612: "block-scaled pair kernel: the MMA warp waited for scales",
     613: "block-scaled pair kernel: the MMA warp waited for a free accumulator", 614: "block-scaled pair kernel: the final MMA drain",

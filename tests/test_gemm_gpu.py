@@ -345,21 +345,41 @@ def _sampled_layer_check(lw, n_expts, tokens, device, seed, skew, n_sample=8):
 
 
 def test_gpt_oss_120b_layer_benchmark_configuration_against_oracle(device):
-    """The benchmarked configuration itself -- 128 experts, 16384 tokens, skewed router: 256 x 256 tiles, TMA activation
-    loads, row-gather scratch -- against the CPU oracle on sampled tokens."""
+    """The benchmarked configuration itself -- 128 experts, 16384 tokens, skewed router: the pair kernel on the default weight
+    tiles, bf16 tokens as two e4m3 terms -- against the CPU oracle on sampled tokens."""
     from triton_b200.testing import make_synthetic_layer
     lw = make_synthetic_layer(128, 2880, 2880, device, seed=1000, keep_canonical=True)
+    assert lw.kernels(4 * 16384) == ("gemm_mx_pair_kernel",) * 2
+    _sampled_layer_check(lw, 128, 16384, device, seed=0, skew=True)
+
+
+def test_gpt_oss_120b_layer_on_the_bf16_kernel_against_oracle(device):
+    """The same on the bf16 kernel, which narrow products of many rows take by themselves: 256 x 256 tiles, TMA activation loads,
+    row-gather scratch."""
+    from triton_b200.testing import make_synthetic_layer
+    lw = make_synthetic_layer(128, 2880, 2880, device, seed=1000, keep_canonical=True)
+    with tb.scoped_opt_flags_constraints({"kernel": "tcgen05"}):
+        assert lw.kernels(4 * 16384) == ("gemm_tc_kernel",) * 2
+        _sampled_layer_check(lw, 128, 16384, device, seed=0, skew=True)
+
+
+def test_gpt_oss_120b_layer_prefill_on_the_block_scaled_copy_against_oracle(device):
+    """The same with both weight copies: the pair kernel on the block-scaled tiles."""
+    from triton_b200.testing import make_synthetic_layer
+    lw = make_synthetic_layer(128, 2880, 2880, device, seed=1000, keep_canonical=True, block_scaled=True)
+    assert lw.use_block_scaled(4 * 16384) and lw.kernels(4 * 16384) == ("gemm_mx_pair_kernel",) * 2
     _sampled_layer_check(lw, 128, 16384, device, seed=0, skew=True)
 
 
 @pytest.mark.parametrize("tokens", [1, 16, 64, 300, 1200])
 def test_gpt_oss_120b_layer_decode_path_against_oracle(tokens, device):
-    """Steps of the 128-expert layer with up to 48 rows per expert on average take the block-scaled kernel (its own copy of
-    the weights): 1 to 64 tokens in 16-row token blocks (four e2m1 terms), 300 and 1200 tokens (9 and 38 rows per expert) in
-    32-row blocks (two e4m3 terms)."""
+    """Steps of the 128-expert layer with up to 48 rows per expert on average take the block-scaled copy of the weights: 1 to 64
+    tokens on the decode kernel in 16-row token blocks (four e2m1 terms), 300 (9 rows per expert) in 32-row blocks (two e4m3
+    terms), 1200 (38 rows per expert) on the pair kernel."""
     from triton_b200.testing import make_synthetic_layer
     lw = make_synthetic_layer(128, 2880, 2880, device, seed=1000, keep_canonical=True, block_scaled=True)
     assert lw.use_block_scaled(tokens * 4)
+    assert lw.kernels(tokens * 4) == ("gemm_mx_kernel" if tokens <= 300 else "gemm_mx_pair_kernel",) * 2
     _sampled_layer_check(lw, 128, tokens, device, seed=tokens, skew=True, n_sample=min(tokens, 6))
 
 

@@ -245,16 +245,19 @@ def test_block_scaled_e4m3_output(device):
     assert (diff > 0).float().mean() < 0.02
 
 
-@pytest.mark.parametrize("tokens", [64, 2048])
-def test_layer_with_e4m3_activations_against_oracle(tokens, device):
-    """The layer in fp8 mode (e4m3 tokens in, e4m3 between the GEMMs) against the oracle fed the same quantised rows."""
+@pytest.mark.parametrize("tokens, E, kernel", [(64, 16, "gemm_mx_pair_kernel"), (2048, 16, "gemm_mx_pair_kernel"), (48, 16, "gemm_mx_kernel"),
+                                               (8192, 32, "gemm_mx_pair_kernel")])
+def test_layer_with_e4m3_activations_against_oracle(tokens, E, kernel, device):
+    """The layer in fp8 mode (e4m3 tokens in, e4m3 between the GEMMs) against the oracle fed the same quantised rows: 16 rows per
+    expert and prefill sizes on the pair kernel, fewer on the decode kernel."""
     from triton_b200.moe import moe_layer_forward
     from triton_b200.testing import make_synthetic_layer
-    E, k = 16, 4
+    k = 4
     lw = make_synthetic_layer(E, 2880, 2880, device, seed=5, keep_canonical=True, block_scaled=True)
     g = torch.Generator(device=device).manual_seed(tokens)
     x8 = torch.randn(tokens, 2880, device=device, generator=g).to(torch.float8_e4m3fn)
     logits = torch.randn(tokens, E, device=device, generator=g)
+    assert lw.kernels(tokens * k, torch.float8_e4m3fn) == (kernel,) * 2
     z = moe_layer_forward(x8, logits, lw, k)
     tb.matmul_check_status()
     assert z.dtype == torch.bfloat16

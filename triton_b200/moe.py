@@ -136,22 +136,25 @@ def _product_fits(w, scale, bias, E: int, K: int) -> bool:
     if w is None or scale is None:
         return False
     kind = _LAYER_KIND.get(type(w.storage.layout))
-    return (kind is not None and type(scale.storage.layout) is kind[1] and w.dtype == FP4 and len(w.shape) == 3
-            and w.shape[0] >= E and w.shape[1] == K and bias.ndim == 2 and bias.shape[0] >= E and bias.shape[1] == w.shape[2]
-            and bias.stride(1) == 1)
+    if kind is None or type(scale.storage.layout) is not kind[1] or len(w.shape) != 3:
+        return False
+    e, k, n = w.shape
+    b = bias.shape
+    return e >= E and k == K and len(b) == 2 and b[0] >= E and b[1] == n and bias.stride(1) == 1
 
 
 def _one_call(x, logits, lw: MoeLayerWeights, k: int, weights=None) -> bool:
     """Whether the step is one the native host path takes as a whole: fp32 logits, bf16 or e4m3 rows, weights and biases in
     the forms this package prepares, extents that fit one another.  Anything else goes through the operators one by one,
     which run it or say what is wrong with it."""
-    E = logits.shape[1] if logits.ndim == 2 else 0
-    if not ((x.dtype == torch.float8_e4m3fn or x.dtype == torch.bfloat16) and logits.dtype == torch.float32 and 0 < E <= 256
-            and E == lw.n_expts and 0 < k <= E and x.ndim == 2 and x.stride(1) == 1 and logits.stride(1) == 1
-            and 0 < x.shape[0] <= FUSED_MAX_TOKENS and logits.shape[0] == x.shape[0]):
+    if x.ndim != 2 or logits.ndim != 2 or x.dtype not in (torch.bfloat16, torch.float8_e4m3fn) or logits.dtype != torch.float32:
         return False
-    w1, w1_scale, w2, w2_scale = _step_weights(x.dtype, lw, x.shape[0] * k) if weights is None else weights
-    return (_product_fits(w1, w1_scale, lw.b1, E, x.shape[1]) and w1.shape[2] % 2 == 0
+    (T, K), (rows, E) = x.shape, logits.shape
+    if not (0 < T <= FUSED_MAX_TOKENS and rows == T and 0 < E <= 256 and E == lw.n_expts and 0 < k <= E
+            and x.stride(1) == 1 and logits.stride(1) == 1):
+        return False
+    w1, w1_scale, w2, w2_scale = _step_weights(x.dtype, lw, T * k) if weights is None else weights
+    return (_product_fits(w1, w1_scale, lw.b1, E, K) and w1.shape[2] % 2 == 0
             and _product_fits(w2, w2_scale, lw.b2, E, w1.shape[2] // 2))
 
 

@@ -416,3 +416,17 @@ def test_kernel_of_a_shard_goes_by_its_own_rows(monkeypatch):
     monkeypatch.setattr(moe, "remap_ragged_tensor_metadata", lambda meta, table: md)
     assert moe._local_metadata(None, None, 512 // 8, 16).expected_slice_size == 4
     assert moe._local_metadata(None, None, 1, 16).expected_slice_size == 1
+
+
+def test_small_block_scaled_products_leave_the_decode_kernel_after_one_wave():
+    """Below 2^24 elements the decode kernel keeps a product while its 32 x 128 tiles fit the SMs (148 of them where no GPU says
+    otherwise): 32 experts of 512 x 512 up to some 16 rows per expert, 8 experts of 2048 x 512 to well beyond 96."""
+    from triton_b200 import _lib
+    if torch.cuda.is_available() and torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("sizes are those of 148 SMs")
+    kernel = lambda E, K, N, per: _lib.host().gemm_kernel(_lib.MOE_W_MX4_B200MX, E, K, N, E * per, torch.bfloat16, torch.bfloat16, (0, 0, 0, 0))
+    decode, pair = "gemm_mx_kernel", "gemm_mx_pair_kernel"
+    assert kernel(32, 512, 512, 16) == decode and kernel(32, 512, 512, 32) == kernel(32, 512, 512, 64) == pair
+    assert kernel(8, 512, 2048, 16) == decode and kernel(8, 512, 2048, 32) == kernel(8, 512, 2048, 80) == pair
+    assert kernel(8, 2048, 512, 96) == kernel(8, 2048, 512, 128) == decode and kernel(8, 2048, 512, 160) == pair
+    assert kernel(1, 512, 512, 1000) == decode and kernel(1, 512, 512, 1200) == pair

@@ -770,8 +770,10 @@ int launch_mx_pair_ty(const GemmParams& p, const PairParams& q, const MoeGemmArg
 //   16 experts of 1440 x 1472:  8 rows 49 (45), 32 rows 53 (55), 64 rows 59 (66), 256 rows 80 (102), 1024 rows 167 (156)
 //   8 experts of 512 x 2048:    16 rows 37 (33), 64 rows 45 (41), 256 rows 53 (49), 1024 rows 84 (66)
 // Block-scaled tiles (against the decode forms of gemm_mx.cu), tile_m = 256 asks for it: bf16 tokens from 20 rows on (32 experts
-// of 2880 x 5760, 16 rows: 139 there, 156 here, 32 rows 178 and 162; 64 experts of 1024 x 1536, 16 rows: 76 and 63), small ones from
-// 96 on (8 experts of 512 x 2048, 32 rows: 40 and 43); e4m3 tokens, one term, from 16 on (32 experts, 8 rows: 102 and 114;
+// of 2880 x 5760, 16 rows: 139 there, 156 here, 32 rows 178 and 162; 64 experts of 1024 x 1536, 16 rows: 76 and 63), small ones
+// once the decode kernel's tiles of 32 rows x 128 weight rows (half a block lost per expert) are more than a wave, up to which it
+// takes one tile's time (a product of 32 experts of 512 x 512, 16 rows: 10 there, 11 here, 64 rows 21 and 13; 8 experts of
+// 512 x 2048, 16 rows 9 and 11, 80 rows 20 and 13; of 2048 x 512, 96 rows 17 and 21); e4m3 tokens, one term, from 16 on (32 experts, 8 rows: 102 and 114;
 // 64 rows: 320 and 167).
 bool moe_gemm_mx_pair_wanted(const MoeGemmArgs& a) {
   if (a.slice_sizes && a.E > MAX_PREFIX_EXPERTS) return false;
@@ -791,7 +793,8 @@ bool moe_gemm_mx_pair_wanted(const MoeGemmArgs& a) {
   if (a.tile_m == 256) return true;
   if (a.tile_m != 0 || a.kernel == MOE_GEMM_MX_F8) return false;
   if (a.x_dtype != MOE_BF16) return per >= 16;
-  return per >= (load >= (1 << 24) ? 20 : 96);
+  if (load >= (1 << 24)) return per >= 20;
+  return experts * (per + 16) / 32 * cdiv64(a.N, 128) > moe_sm_count();
 }
 
 int64_t moe_gemm_mx_pair_workspace(const MoeGemmArgs& a) { return pair_plan(a).ws_bytes; }

@@ -467,3 +467,19 @@ def test_layer_with_both_weight_copies_under_a_constraint(constraint, rows_per_e
         assert oracle.rel_l2(free.cpu(), y.cpu()) < 1e-2
         if rows_per_expert > 48 and "mx" not in constraint.values():
             assert torch.equal(y, moe_layer_forward(x, logits, default, k))
+
+
+@pytest.mark.parametrize("block_scaled", [False, True])
+def test_layer_in_one_call_sizes_its_workspace_for_the_activation(block_scaled, device):
+    """fc1 over few k behind SwiGLU takes the bf16 kernel from 512 rows per expert on: the one call asks for its temporaries with the
+    activation set, so that it runs what the operators run."""
+    from triton_b200.moe import _NoTimer, moe_layer_forward
+    from triton_b200.testing import make_synthetic_layer
+    E, d, ff, k, T = 8, 512, 2176, 2, 2100
+    lw = make_synthetic_layer(E, d, ff, device, seed=3, block_scaled=block_scaled)
+    assert lw.kernels(T * k)[0] == "gemm_tc_kernel" and lw.kernels(500 * E)[0] == "gemm_mx_pair_kernel"
+    g = torch.Generator(device=device).manual_seed(1)
+    x, logits = torch.randn(T, d, device=device, generator=g).bfloat16(), torch.randn(T, E, device=device, generator=g)
+    one, many = moe_layer_forward(x, logits, lw, k), moe_layer_forward(x, logits, lw, k, gemm_timer=_NoTimer)
+    tb.matmul_check_status()
+    assert torch.equal(one, many)

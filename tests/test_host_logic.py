@@ -430,3 +430,14 @@ def test_small_block_scaled_products_leave_the_decode_kernel_after_one_wave():
     assert kernel(8, 512, 2048, 16) == decode and kernel(8, 512, 2048, 32) == kernel(8, 512, 2048, 80) == pair
     assert kernel(8, 2048, 512, 96) == kernel(8, 2048, 512, 128) == decode and kernel(8, 2048, 512, 160) == pair
     assert kernel(1, 512, 512, 1000) == decode and kernel(1, 512, 512, 1200) == pair
+
+
+def test_wide_swiglu_product_over_few_k_stays_with_the_bf16_kernel():
+    """From 512 rows per expert on, and only behind SwiGLU (fc1): a layer of 512 x 4096 with either weight copy."""
+    for lw in (_layer_on_cpu(E=16, d=512, ff=2048, block_scaled=False), _layer_on_cpu(E=16, d=512, ff=2048)):
+        assert lw.kernels(16 * 511)[0] == "gemm_mx_pair_kernel" and lw.kernels(16 * 512)[0] == "gemm_tc_kernel"
+    wide = _layer_on_cpu(E=4, d=1024, ff=2048)
+    assert wide.kernels(4 * 1024)[0] == "gemm_mx_pair_kernel"
+    from triton_b200 import _lib
+    plain = _lib.host().gemm_kernel(_lib.MOE_W_MX4_B200, 16, 512, 4096, 16 * 1024, torch.bfloat16, torch.bfloat16, (0, 0, 0, 0))
+    assert plain == "gemm_mx_pair_kernel"

@@ -769,6 +769,10 @@ int launch_mx_pair_ty(const GemmParams& p, const PairParams& q, const MoeGemmArg
 //   64 experts of 1024 x 1536:  4 rows 53 (59), 16 rows 63 (100), 64 rows 88 (106)
 //   16 experts of 1440 x 1472:  8 rows 49 (45), 32 rows 53 (55), 64 rows 59 (66), 256 rows 80 (102), 1024 rows 167 (156)
 //   8 experts of 512 x 2048:    16 rows 37 (33), 64 rows 45 (41), 256 rows 53 (49), 1024 rows 84 (66)
+// Wide SwiGLU products over few k are bound by this kernel's epilogue and stay with the bf16 kernel from 512 rows on (512 x 4096, 8
+// experts of 1024 rows: 72 here, 57 there; 16 experts 132 and 109; without the activation 64 and 61, 114 and 116).
+// (Both kernels lose up to a third of a wave, so no line in these sizes is right everywhere: over 500 products of 48 to 1024 rows
+// this one is 2 % from the better kernel on average, most of it at 100-400 balanced rows of K <= 1024.)
 // Block-scaled tiles (against the decode forms of gemm_mx.cu), tile_m = 256 asks for it: bf16 tokens from 20 rows on (32 experts
 // of 2880 x 5760, 16 rows: 139 there, 156 here, 32 rows 178 and 162; 64 experts of 1024 x 1536, 16 rows: 76 and 63), small ones
 // once the decode kernel's tiles of 32 rows x 128 weight rows (half a block lost per expert) are more than a wave, up to which it
@@ -788,7 +792,8 @@ bool moe_gemm_mx_pair_wanted(const MoeGemmArgs& a) {
       return false;
     if (a.kernel == MOE_GEMM_MX) return true;
     if (a.kernel != MOE_GEMM_AUTO || a.tile_m != 0) return false;
-    return load >= (1 << 24) && (per > 0 ? per : 1) * load >= (1 << 28) && (a.N >= 2560 || per < 512);
+    const bool wide = a.N >= 2560 && !(a.activation == MOE_ACT_SWIGLU && a.K < 1024);
+    return load >= (1 << 24) && (per > 0 ? per : 1) * load >= (1 << 28) && (wide || per < 512);
   }
   if (a.tile_m == 256) return true;
   if (a.tile_m != 0 || a.kernel == MOE_GEMM_MX_F8) return false;

@@ -242,7 +242,7 @@ Tensor gemm(const Tensor& a, int kind, const Tensor& w, const OptTensor& ws, int
 
 // name of the kernel of a ragged product of M rows on aligned operands in weight tiles `kind` (no tensors: a question to the dispatch)
 std::string gemm_kernel(int kind, int64_t E, int64_t K, int64_t N, int64_t M, py::object x_dtype, py::object y_dtype, const py::tuple& tuning,
-                        int rows_per_expert) {
+                        int rows_per_expert, bool swiglu) {
   MoeGemmArgs g{};
   void* const some = (void*)(uintptr_t)4096;
   g.x = g.y = some; g.w = some; g.w_scale = (const uint8_t*)some; g.w_kind = kind;
@@ -252,6 +252,7 @@ std::string gemm_kernel(int kind, int64_t E, int64_t K, int64_t N, int64_t M, py
   g.y_dtype = dtype_code(torch::python::detail::py_object_to_dtype(y_dtype));
   set_tuning(g, tuning);
   g.rows_per_expert = rows_per_expert;
+  g.activation = swiglu ? MOE_ACT_SWIGLU : MOE_ACT_NONE;
   const char* name = lib.moe_gemm_kernel_name(&g);
   if (!name) raise(inapplicable, lib.moe_last_error());
   return name;
@@ -290,8 +291,9 @@ Tensor layer(const Tensor& x, const Tensor& logits, int64_t k, const py::tuple& 
   g1.slice_sizes = g2.slice_sizes = &present;
   const int64_t lo = pad512(E + 1), mnb = max_blocks16(E, n), ls = pad512(mnb), words = cdiv(E, 32), t_pad = cdiv(T, 32) * 32;
   const int64_t route_ws = (int64_t)lib.moe_route_workspace(T, (int)E, (int)k);
-  g1.ld_x = x.stride(0); g2.ld_x = ff;   // (the size query looks at types and pitches too)
+  g1.ld_x = x.stride(0); g2.ld_x = ff;   // (the size query looks at types, pitches and the activation too)
   g1.y_dtype = fp8 ? MOE_F8E4M3 : MOE_BF16; g2.y_dtype = MOE_BF16;
+  g1.activation = MOE_ACT_SWIGLU; g1.act_alpha = (float)alpha;
   bool ws1, ws2;
   const int64_t t1 = temp_bytes(g1, true, ws1), t2 = temp_bytes(g2, false, ws2);
   Carver c;
@@ -316,7 +318,6 @@ Tensor layer(const Tensor& x, const Tensor& logits, int64_t k, const py::tuple& 
   set_temp(g1, base + o_tmp, t1, ws1);
   set_temp(g2, base + o_tmp, t2, ws2);
   g1.gather_indx = (int32_t*)(base + o_tok);
-  g1.activation = MOE_ACT_SWIGLU; g1.act_alpha = (float)alpha;
   if (limit) { g1.act_limit = (float)*limit; g1.act_has_limit = 1; }
   g1.y = base + o_h; g1.ld_y = ff;
   check(lib.moe_grouped_gemm(&g1, st), "moe_grouped_gemm", true);
@@ -465,7 +466,7 @@ PYBIND11_MODULE(_host, m) {
   m.def("bitmatrix_metadata", &bitmatrix_metadata);
   m.def("gemm", &gemm);
   m.def("gemm_kernel", &gemm_kernel, py::arg("kind"), py::arg("E"), py::arg("K"), py::arg("N"), py::arg("M"), py::arg("x_dtype"),
-        py::arg("y_dtype"), py::arg("tuning"), py::arg("rows_per_expert") = 0);
+        py::arg("y_dtype"), py::arg("tuning"), py::arg("rows_per_expert") = 0, py::arg("swiglu") = false);
   m.def("layer", &layer);
   m.def("downcast", &downcast);
   m.def("upcast", &upcast);

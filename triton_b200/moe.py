@@ -57,32 +57,37 @@ class MoeLayerWeights:
     def n_expts(self):
         return self.b1.shape[0]
 
-    def use_block_scaled(self, n_rows: int, n_out: int | None = None) -> bool:
-        """Whether a product of `n_rows` routed rows with `n_out` weight rows per expert (default: fc1's) takes the
-        block-scaled copy.  Few rows per expert (decode) stream the packed weights straight into the MMA, bound by HBM.
-        With more rows the block-scaled pair kernel first re-lays the tokens out (4 bytes per element written and read
-        against 2 n_out operations), which a wide product repays and a narrow one does not; measured against the bf16
-        kernel: 64 rows per expert 1.3-1.7 x faster for n_out >= 2000 and 1.0-1.2 x at 512-1440; 256 rows 0.8 x at 512;
-        1024 rows per expert 1.05-1.2 x faster from 2880 on, 0.9 x at 2048.  A tuning constraint that names a kernel of the
-        default copy, or a tile, keeps steps beyond the row limit on that copy, whose kernels have it."""
+    def use_block_scaled(self, n_rows: int, n_out: int | None = None, swiglu_k: int | None = None) -> bool:
+        """Whether a product of `n_rows` routed rows with `n_out` weight rows per expert (default: fc1's; `swiglu_k`: k of a product
+        behind SwiGLU) takes the block-scaled copy.  Few rows per expert (decode) stream the packed weights straight into the MMA,
+        bound by HBM.  With more rows either copy runs on the pair kernel where that pays, at the same speed; what is decided here
+        is where the other would not: up to 80 rows per expert small products take the block-scaled copy (8 experts of 512 x 2048, 80
+        rows: 13 us against 14 balanced and 20 skewed), beyond them wide ones (1280; from 512 rows per expert on 2560, and with SwiGLU
+        not over few k), the rest the bf16 kernel.  (At 512 rows 512-1472 wide products would be 1.1-1.4 x faster on the copy, at
+        1024 up to 1.2 x slower.)  A tuning constraint that names a kernel of the default copy, or a tile, keeps steps beyond the
+        row limit on that copy, whose kernels have it."""
         if self.w1_bs is None:
             return False
         if n_rows <= self.block_scaled_max_rows_per_expert * self.n_expts:
             return True
         if self.block_scaled_max_rows_per_expert != BLOCK_SCALED_ROWS or bf16_kernel_or_tile_named():
             return False
-        n_out = self.b1.shape[1] if n_out is None else n_out
-        return n_rows <= 80 * self.n_expts or n_out >= (1280 if n_rows < 512 * self.n_expts else 2560)
+        if n_out is None:
+            n_out, swiglu_k = self.b1.shape[1], self.w1.shape[1]
+        if n_rows < 512 * self.n_expts:
+            return n_rows <= 80 * self.n_expts or n_out >= 1280
+        return n_out >= 2560 and (swiglu_k is None or swiglu_k >= 1024)
 
     def fc_weights(self, n_rows: int):
-        one = (self.w1_bs, self.w1_bs_scale) if self.use_block_scaled(n_rows, self.b1.shape[1]) else (self.w1, self.w1_scale)
-        two = (self.w2_bs, self.w2_bs_scale) if self.use_block_scaled(n_rows, self.b2.shape[1]) else (self.w2, self.w2_scale)
-        return (*one, *two)
+        one = self.use_block_scaled(n_rows, self.b1.shape[1], self.w1.shape[1])
+        two = self.use_block_scaled(n_rows, self.b2.shape[1])
+        return (*((self.w1_bs, self.w1_bs_scale) if one else (self.w1, self.w1_scale)),
+                *((self.w2_bs, self.w2_bs_scale) if two else (self.w2, self.w2_scale)))
 
     def kernels(self, n_rows: int, dtype: torch.dtype = torch.bfloat16) -> tuple[str, str]:
         """Names of the kernels that fc1 and fc2 of a step of `n_rows` routed rows run on under the current tuning constraints."""
         w1, s1, w2, s2 = _step_weights(dtype, self, n_rows)
-        return tuple(_lib.host().gemm_kernel(_product(w, s)[0], *w.shape, n_rows, dtype, out, gemm_tuning())
+        return tuple(_lib.host().gemm_kernel(_product(w, s)[0], *w.shape, n_rows, dtype, out, gemm_tuning(), swiglu=w is w1)
                      for w, s, out in ((w1, s1, dtype), (w2, s2, torch.bfloat16)))
 
     def weight_bytes(self):

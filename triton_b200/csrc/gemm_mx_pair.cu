@@ -18,8 +18,9 @@
 // 97 KB read per step, 1140 cycles, against 1024 of MMA; as two tiles of 64 tokens the weights alone would be written and
 // read twice.  Large prefill runs into the power limit first (1.5 GHz).  Tokens on N
 // also make a ragged tail cost what it holds, in steps of 32 rows, where tokens on M padded every expert to a multiple of 128
-// or 256 (31 % of the rows of a skewed 128-expert batch of 16384 tokens).  With few rows per expert the packed weights bound it:
-// 128 experts of 2880 x 5760, 300 tokens, 1.1 GB in 165 us.
+// or 256 (31 % of the rows of a skewed 128-expert batch of 16384 tokens).  With few rows per expert it streams the packed weights at 3
+// to 4 TB/s (128 experts of 2880 x 5760 and 2880 x 2880, eight rows each: 1.7 GB in 406 us): an MMA takes 45-59 cycles however few
+// columns it has.
 //
 // A k step of a small tile is eight MMAs of 64 cycles, so what the issuing warp does around them counts: operands in uniform
 // registers, the election inside the instruction's own asm block (a step took 1150 cycles with a leader flag kept in a register,
@@ -760,25 +761,27 @@ int launch_mx_pair_ty(const GemmParams& p, const PairParams& q, const MoeGemmArg
 
 }  // namespace
 
-// Where the pair form is the faster one (us, fc1 + fc2 unless said).  `load` is what one pass over the weights of the experts in
-// use costs, in elements.
+// Where the pair form is the faster one (us, fc1 + fc2 unless said; balanced routing unless said).  `load` is what one pass over the
+// weights of the experts in use costs, in elements.
 // Default tiles (against the bf16 tensor-core kernel, above ten or so rows also against the streaming one), kernel "mx" asks
 // for it: the pack pass and the cluster launch want 2^24 elements and 2^28 products a token row to be repaid, and a product
 // over fewer than 2560 weight rows stays ahead up to 512 rows per expert only.
-//   32 experts of 2880 x 5760:  1 row 96 (streaming: 112), 8 rows 152 (243), 64 rows 207 (332), 150 rows 321 (457)
-//   64 experts of 1024 x 1536:  4 rows 53 (59), 16 rows 63 (100), 64 rows 88 (106)
-//   16 experts of 1440 x 1472:  8 rows 49 (45), 32 rows 53 (55), 64 rows 59 (66), 256 rows 80 (102), 1024 rows 167 (156)
-//   8 experts of 512 x 2048:    16 rows 37 (33), 64 rows 45 (41), 256 rows 53 (49), 1024 rows 84 (66)
+//   32 experts of 2880 x 5760:  8 rows 141 (streaming: 235), 64 rows 170 (272), 150 rows 289 (379), 1024 rows 1515 (1564)
+//   64 experts of 1024 x 1536:  4 rows 55 (75), 16 rows 53 (86), 64 rows 69 (82), 256 rows 144 (146)
+//   16 experts of 1440 x 1472:  64 rows 38 (43), 256 rows 61 (53), logits biased by N(0, 1) per expert 62 (79), 1024 rows 151 (135)
 // Wide SwiGLU products over few k are bound by this kernel's epilogue and stay with the bf16 kernel from 512 rows on (512 x 4096, 8
 // experts of 1024 rows: 72 here, 57 there; 16 experts 132 and 109; without the activation 64 and 61, 114 and 116).
 // (Both kernels lose up to a third of a wave, so no line in these sizes is right everywhere: over 500 products of 48 to 1024 rows
 // this one is 2 % from the better kernel on average, most of it at 100-400 balanced rows of K <= 1024.)
-// Block-scaled tiles (against the decode forms of gemm_mx.cu), tile_m = 256 asks for it: bf16 tokens from 20 rows on (32 experts
-// of 2880 x 5760, 16 rows: 139 there, 156 here, 32 rows 178 and 162; 64 experts of 1024 x 1536, 16 rows: 76 and 63), small ones
-// once the decode kernel's tiles of 32 rows x 128 weight rows (half a block lost per expert) are more than a wave, up to which it
-// takes one tile's time (a product of 32 experts of 512 x 512, 16 rows: 10 there, 11 here, 64 rows 21 and 13; 8 experts of
-// 512 x 2048, 16 rows 9 and 11, 80 rows 20 and 13; of 2048 x 512, 96 rows 17 and 21); e4m3 tokens, one term, from 16 on (32 experts, 8 rows: 102 and 114;
-// 64 rows: 320 and 167).
+// Block-scaled tiles (against the decode forms of gemm_mx.cu), tile_m = 256 asks for it.  bf16 tokens from 20 rows on: 32 experts of
+// 2880 x 5760, 16 rows 126 there, 144 here, 24 rows 135 and 145, 32 rows 165 and 150; 128 experts, 16 rows 416 and 427, 24 rows 467
+// and 437, but with logits biased by N(0, 1) per expert 12 rows on average 326 and 309, 16 rows 360 and 306 (what an expert has
+// decides, not the mean); 64 experts of 1024 x 1536, 12 rows 52 and 53, 16 rows 61 and 53.
+// Small ones once the decode kernel's tiles of 32 rows x 128 weight rows (half a block lost per expert) are more than a wave, up to
+// which it takes one tile's time: a product of 32 experts of 512 x 512, 16 rows 10 there, 11 here, 64 rows 21 and 13; 8 experts of
+// 512 x 2048, 16 rows 9 and 11, 80 rows 20 and 13; of 2048 x 512, 96 rows 17 and 21.
+// e4m3 tokens, one term, from 16 on: 32 experts of 2880 x 5760, 16 rows 113 and 136, 32 rows 149 and 140; 128 experts, 16 rows 366 and
+// 403, biased 301 and 256, 32 rows 514 and 435; 64 experts of 1024 x 1536, 16 rows 57 and 52.
 bool moe_gemm_mx_pair_wanted(const MoeGemmArgs& a) {
   if (a.slice_sizes && a.E > MAX_PREFIX_EXPERTS) return false;
   if (a.M >= (1ll << 31) - (1 << 20) || a.kernel == MOE_GEMM_MX_F4 || a.tile_n != 0) return false;

@@ -119,22 +119,29 @@ __device__ __forceinline__ bool pack_block(const GemmParams& p, int64_t pid, int
 // Magnitude from which on two e4m3 terms do not hold a token's value: infinities, and finite values that round to 2^128.
 constexpr float BEYOND = 3.0e38f;
 
-// Output of a row with such a value, in fp32 on the CUDA cores by one warp, 32 weight rows at a time: what the product of bf16 values
-// gives (an infinite token value times a weight is infinite, or NaN for a zero weight).
+// Output of a row with such a value, in fp32 on the CUDA cores by the whole block, a thread per weight row: what the product of bf16
+// values gives (an infinite token value times a weight is infinite, or NaN for a zero weight).  `groups`: bits of the groups of 32 k
+// that decide it (those with an infinity or NaN, if there is an infinity), NULL for all.
+constexpr int EXACT_WORDS = 64;
 template <typename TY, bool TILED>
-__device__ void exact_row(const GemmParams& p, const PairPackParams& a, int e, int64_t m, int64_t dst, const __nv_bfloat16* x, int lane) {
+__device__ void exact_row(const GemmParams& p, const PairPackParams& a, int e, int64_t m, int64_t dst, const __nv_bfloat16* x,
+                          const uint32_t* groups) {
   TY* y = gemm_out_row<TY>(p, dst);
-  for (int n = lane; n - lane < p.N; n += 32) {
+  const int lane = threadIdx.x & 31;
+  for (int n = threadIdx.x; n - lane < p.N; n += 256) {
     const int b = n >> 7, row = n & 127;
     float acc = 0.0f;
     for (int kg = 0; kg < p.K >> 5; ++kg) {                        // scale groups of 32 k
+      if (groups && !((groups[kg >> 5] >> (kg & 31)) & 1u)) continue;
       const int kt = kg >> 2, g = kg & 3;
       const int64_t at = TILED ? ((int64_t)e * a.NB + b) * a.KT + kt : ((int64_t)e * a.KT + kt) * a.NB + b;
       const uint8_t* q = (const uint8_t*)p.w + at * 8192 + (TILED ? (g * 128 + row) * 16 : row * 64 + g * 16);
       const uint32_t sb = p.w_scale[at * 512 + (TILED ? row * 4 + g : (row & 31) * 16 + (row >> 5) * 4 + g)];
       const float s = __uint_as_float(sb ? (sb == 255u ? 0x7FC00000u : sb << 23) : 0x00400000u);
+      const uint4 q4 = *reinterpret_cast<const uint4*>(q);
+#pragma unroll
       for (int i = 0; i < 4; ++i) {                                // words of eight values
-        uint32_t w = reinterpret_cast<const uint32_t*>(q)[i];
+        uint32_t w = i == 0 ? q4.x : i == 1 ? q4.y : i == 2 ? q4.z : q4.w;
         if (TILED) {                                               // evens, then odds: back to pairs
           uint32_t pairs = 0;
           for (int j = 0; j < 4; ++j) pairs |= (((w >> (4 * j)) & 0xFu) | (((w >> (16 + 4 * j)) & 0xFu) << 4)) << (8 * j);
@@ -163,22 +170,40 @@ __device__ void exact_row(const GemmParams& p, const PairPackParams& a, int e, i
 template <bool TILED>
 __device__ __noinline__ uint32_t exact_rows(const GemmParams& p, const PairPackParams& a, int e, int64_t row0, int rows) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  uint32_t mine = 0;
+  __shared__ uint32_t s_groups[EXACT_WORDS];
+  uint32_t mine = 0, all = 0;
   for (int r = warp; r < rows; r += 8) {
-    const int64_t m = row0 + r, src = p.gather_indx ? (int64_t)p.gather_indx[m] : m, d = p.scatter_indx ? (int64_t)p.scatter_indx[m] : m;
+    const int64_t src = p.gather_indx ? (int64_t)p.gather_indx[row0 + r] : row0 + r;
     if (src < 0 || src >= a.rows_x) continue;
     const __nv_bfloat16* x = (const __nv_bfloat16*)a.x + src * a.ld_x;
     bool is = false;
     for (int k = lane; k < a.K; k += 32) is |= fabsf(__bfloat162float(x[k])) >= BEYOND;
-    if (!__any_sync(0xFFFFFFFFu, is)) continue;
-    mine |= 1u << r;
-    if (d < 0) continue;
-    if (a.y_dtype == MOE_BF16) exact_row<__nv_bfloat16, TILED>(p, a, e, m, d, x, lane);
-    else if (a.y_dtype == MOE_F32) exact_row<float, TILED>(p, a, e, m, d, x, lane);
-    else exact_row<__nv_fp8_e4m3, TILED>(p, a, e, m, d, x, lane);
+    if (__any_sync(0xFFFFFFFFu, is)) mine |= 1u << r;
   }
-  uint32_t all = 0;
-  for (int r = 0; r < 16; ++r) all |= __syncthreads_or((mine >> r) & 1u) ? 1u << r : 0u;
+  for (int r = 0; r < rows; ++r) {
+    if (!__syncthreads_or((mine >> r) & 1u)) continue;
+    all |= 1u << r;
+    const int64_t m = row0 + r, d = p.scatter_indx ? (int64_t)p.scatter_indx[m] : m;
+    if (d < 0) continue;
+    const __nv_bfloat16* x = (const __nv_bfloat16*)a.x + (p.gather_indx ? (int64_t)p.gather_indx[m] : m) * a.ld_x;
+    for (int i = threadIdx.x; i < EXACT_WORDS; i += 256) s_groups[i] = 0;
+    __syncthreads();
+    bool inf = false;
+    for (int kg = threadIdx.x; kg < a.K >> 5; kg += 256) {
+      bool odd = false;
+      for (int k = kg * 32; k < kg * 32 + 32; ++k) {
+        const float v = fabsf(__bfloat162float(x[k]));
+        odd |= !(v < BEYOND);
+        inf |= v > 3.4e38f;
+      }
+      if (odd && kg < 32 * EXACT_WORDS) atomicOr(&s_groups[kg >> 5], 1u << (kg & 31));
+    }
+    const uint32_t* groups = __syncthreads_or(inf) && a.K <= 1024 * EXACT_WORDS ? s_groups : nullptr;
+    if (a.y_dtype == MOE_BF16) exact_row<__nv_bfloat16, TILED>(p, a, e, m, d, x, groups);
+    else if (a.y_dtype == MOE_F32) exact_row<float, TILED>(p, a, e, m, d, x, groups);
+    else exact_row<__nv_fp8_e4m3, TILED>(p, a, e, m, d, x, groups);
+    __syncthreads();
+  }
   return all;
 }
 

@@ -223,3 +223,17 @@ def test_host_tensors_are_refused(call, device):
             router_topk(x, wg, None, 2)
         else:
             router_topk(x, wg.to(device), torch.zeros(8), 2)
+
+
+@pytest.mark.parametrize("T, E, k", [(3, 5, 4), (300, 128, 4), (40, 8, 6), (70, 32, 8)])
+def test_rows_of_all_ones_bits_pick_experts_in_range(T, E, k, device):
+    """Logits whose bytes are all 0xFF (memory that was never written, say) are NaN of the lowest order: their rows pick k different
+    experts all the same, and nothing is counted outside the histogram."""
+    logits = torch.randn(T, E, device=device)
+    logits.view(torch.int32)[::2] = -1
+    ragged, gather, scatter, sp = routing(logits, k)
+    indx = sp.indx.cpu().long()
+    assert (indx >= 0).all() and (indx < E).all()
+    assert all(len(set(r.tolist())) == k for r in indx)
+    assert torch.equal(sp.mask_metadata.col_sum.cpu(), torch.bincount(indx.reshape(-1), minlength=E).int())
+    assert torch.equal(topk(logits, k).indx.cpu().long(), indx)

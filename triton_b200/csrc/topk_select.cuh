@@ -5,10 +5,11 @@
 #pragma once
 #include <cstdint>
 
-// order-preserving map float -> uint32 (larger float <=> larger key)
+// order-preserving map float -> uint32 (larger float <=> larger key), never 0: that is an empty place's key, and the NaN whose bits
+// are all ones must fill one like any other value
 __device__ __forceinline__ uint32_t sel_float_key(float f) {
   const uint32_t b = __float_as_uint(f);
-  return b ^ ((b & 0x80000000u) ? 0xFFFFFFFFu : 0x80000000u);
+  return max(b ^ ((b & 0x80000000u) ? 0xFFFFFFFFu : 0x80000000u), 1u);
 }
 __device__ __forceinline__ float sel_key_float(uint32_t k) {
   return __uint_as_float(k ^ ((k & 0x80000000u) ? 0x80000000u : 0xFFFFFFFFu));

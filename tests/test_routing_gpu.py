@@ -4,6 +4,7 @@ import pytest
 import torch
 
 import oracle
+from triton_b200 import _lib
 from triton_b200 import (make_bitmatrix_metadata, make_ragged_tensor_metadata, remap_ragged_tensor_metadata, routing,
                          topk)
 from triton_b200.tensor import BIT, RaggedTensorMetadata, wrap_torch_tensor
@@ -91,6 +92,16 @@ def test_bitmatrix_metadata_grid(T, E, k, device):
     assert torch.equal(md.col_sum.cpu(), cs)
     assert torch.equal(md.row_sorted_indx.cpu(), row)
     assert torch.equal(md.col_sorted_indx.cpu(), col)
+
+
+@pytest.mark.parametrize("T, E, k", [(1, 1, 1), (600, 1024, 2), (300, 1025, 2), (700, 2500, 1), (33000, 128, 1), (20000, 3, 2)])
+def test_expert_sort_at_the_segments_of_its_scan(T, E, k, device):
+    # one block scans: experts 1024 at a time, the blocks of tokens in 1024 / E segments of up to (and past) sixteen
+    torch.manual_seed(T + E)
+    indx = torch.stack([torch.randperm(E)[:k] for _ in range(T)]).short()
+    col_sum, col, row = _lib.host().bitmatrix_metadata(indx.to(device), E, None)
+    o_sum, o_col, o_row = oracle.bitmatrix_metadata_oracle(indx, E)
+    assert torch.equal(col_sum.cpu(), o_sum.int()) and torch.equal(col.cpu(), o_col.int()) and torch.equal(row.cpu(), o_row.int())
 
 
 @pytest.mark.parametrize("n_slices", [1, 7, 33, 911, 1025])

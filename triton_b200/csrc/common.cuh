@@ -5,6 +5,7 @@
 #include <cuda_fp16.h>
 #include <stdint.h>
 #include <stdio.h>
+#include <utility>
 #include "../../include/moe_b200.h"
 
 // per-thread error message, set by every failing entry point
@@ -33,6 +34,32 @@ void moe_count_launch();   // one kernel launch (api.cu keeps the process-wide c
     moe_count_launch();                 \
     MOE_CHECK_CUDA(cudaGetLastError()); \
   } while (0)
+
+// ---- programmatic dependent launch ---------------------------------------------------------------------------
+// Kernels of the short chains (routing, layer step) are launched with the programmatic-stream-serialization attribute: the
+// next kernel of the stream may start once every block of this one has passed pdl_launch_dependents() or left, and whatever it
+// reads or writes comes after its own pdl_wait(), which returns when its predecessors have completed and their writes are
+// visible (so those kernels take their pointers without __restrict__: a load through such a pointer may move ahead of the
+// wait).  Launch and prologue of a kernel then overlap the tail of the one before.  A kernel waits before it lets its
+// dependents go, so at most one kernel is ahead of a running one, and every grid before that one has completed.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_begin() { pdl_wait(); pdl_launch_dependents(); }
+
+template <typename... KArgs, typename... Args>
+cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
 
 static inline int64_t cdiv64(int64_t a, int64_t b) { return (a + b - 1) / b; }
 

@@ -69,11 +69,12 @@ __device__ __forceinline__ bool mask_nonzero(const void* m, int bytes, int64_t o
 
 // y[s0, s1] = sum_r mask * scale * x[r, s0, s1]; thread = V consecutive s1 (V = 8 on the vector path)
 template <typename TX, typename TY, bool VEC>
-__global__ void __launch_bounds__(256) reduce_kernel(const TX* __restrict__ x, int64_t R, int64_t S0, int64_t S1,
-                                                     int64_t sx_r, int64_t sx_0, int64_t sx_1, const void* __restrict__ mask,
+__global__ void __launch_bounds__(256) reduce_kernel(const TX* x, int64_t R, int64_t S0, int64_t S1,
+                                                     int64_t sx_r, int64_t sx_0, int64_t sx_1, const void* mask,
                                                      int mask_bytes, int64_t sm_r, int64_t sm_0, int64_t sm_1,
-                                                     const float* __restrict__ scale, int64_t ss_r, int64_t ss_0,
-                                                     int64_t ss_1, TY* __restrict__ y, int64_t sy_0, int64_t sy_1) {
+                                                     const float* scale, int64_t ss_r, int64_t ss_0, int64_t ss_1, TY* y,
+                                                     int64_t sy_0, int64_t sy_1) {
+  pdl_begin();
   constexpr int V = VEC ? 8 : 1;
   const int64_t per_row = (S1 + V - 1) / V;
   const int64_t total = S0 * per_row;
@@ -275,15 +276,14 @@ static int launch_reduce(const void* x, int64_t R, int64_t S0, int64_t S1, int64
     const bool vec = sx_1 == 1 && sy_1 == 1 && S1 % 8 == 0 && sx_r % 8 == 0 && sx_0 % 8 == 0 && sy_0 % 8 == 0 &&
                      (uintptr_t)x % 16 == 0 && (uintptr_t)y % 16 == 0 && (!mask || sm_1 == 0) && (!scale || ss_1 == 0);
     if (vec) {
-      reduce_kernel<TX, TY, true><<<grid_for(S0 * (S1 / 8), 256), 256, 0, st>>>(
-          (const TX*)x, R, S0, S1, sx_r, sx_0, sx_1, mask, mb, sm_r, sm_0, sm_1, scale, ss_r, ss_0, ss_1, (TY*)y, sy_0,
-          sy_1);
+      MOE_CHECK_CUDA(launch_pdl(reduce_kernel<TX, TY, true>, dim3(grid_for(S0 * (S1 / 8), 256)), dim3(256), 0, st, (const TX*)x, R, S0, S1,
+                                sx_r, sx_0, sx_1, mask, mb, sm_r, sm_0, sm_1, scale, ss_r, ss_0, ss_1, (TY*)y, sy_0, sy_1));
       MOE_CHECK_LAUNCH();
       return MOE_OK;
     }
   }
-  reduce_kernel<TX, TY, false><<<grid_for(S0 * S1, 256), 256, 0, st>>>(
-      (const TX*)x, R, S0, S1, sx_r, sx_0, sx_1, mask, mb, sm_r, sm_0, sm_1, scale, ss_r, ss_0, ss_1, (TY*)y, sy_0, sy_1);
+  MOE_CHECK_CUDA(launch_pdl(reduce_kernel<TX, TY, false>, dim3(grid_for(S0 * S1, 256)), dim3(256), 0, st, (const TX*)x, R, S0, S1, sx_r,
+                            sx_0, sx_1, mask, mb, sm_r, sm_0, sm_1, scale, ss_r, ss_0, ss_1, (TY*)y, sy_0, sy_1));
   MOE_CHECK_LAUNCH();
   return MOE_OK;
 }
@@ -316,8 +316,9 @@ extern "C" __attribute__((visibility("default"))) int moe_reduce(const void* x, 
 
 // Two device-to-device copies in one launch (the inputs of a replayed step: two copies were two launches of 2 us each).
 namespace {
-__global__ void __launch_bounds__(256) copy2_kernel(uint8_t* __restrict__ d0, const uint8_t* __restrict__ s0, int64_t n0,
-                                                    uint8_t* __restrict__ d1, const uint8_t* __restrict__ s1, int64_t n1) {
+__global__ void __launch_bounds__(256) copy2_kernel(uint8_t* d0, const uint8_t* s0, int64_t n0, uint8_t* d1, const uint8_t* s1,
+                                                    int64_t n1) {
+  pdl_begin();
   const int64_t v0 = n0 >> 4, total = v0 + (n1 >> 4);
   for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < total; i += (int64_t)gridDim.x * 256) {
     if (i < v0) reinterpret_cast<uint4*>(d0)[i] = reinterpret_cast<const uint4*>(s0)[i];
@@ -338,8 +339,8 @@ extern "C" __attribute__((visibility("default"))) int moe_copy2(void* dst0, cons
   MOE_CHECK_ARG((((uintptr_t)dst0 | (uintptr_t)src0 | (uintptr_t)dst1 | (uintptr_t)src1) & 15) == 0,
                 "moe_copy2: pointers must be 16-byte aligned");
   if (bytes0 + bytes1 == 0) return MOE_OK;
-  copy2_kernel<<<grid_for(bytes0 / 16 + bytes1 / 16 + 1, 256), 256, 0, (cudaStream_t)stream>>>(
-      (uint8_t*)dst0, (const uint8_t*)src0, bytes0, (uint8_t*)dst1, (const uint8_t*)src1, bytes1);
+  MOE_CHECK_CUDA(launch_pdl(copy2_kernel, dim3(grid_for(bytes0 / 16 + bytes1 / 16 + 1, 256)), dim3(256), 0, (cudaStream_t)stream,
+                            (uint8_t*)dst0, (const uint8_t*)src0, bytes0, (uint8_t*)dst1, (const uint8_t*)src1, bytes1));
   MOE_CHECK_LAUNCH();
   return MOE_OK;
 }

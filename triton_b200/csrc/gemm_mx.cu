@@ -34,7 +34,6 @@
 // Warps: 0 producer, 1 MMA issue + tensor-memory owner, 2-5 epilogue, 6-9 scale loaders.  Every mbarrier
 // wait is bounded.
 #include "gemm_mx_common.cuh"
-#include <utility>
 
 namespace {
 
@@ -111,16 +110,6 @@ __device__ __forceinline__ bool mx_map_block(const GemmParams& p, int tb, int64_
   return rows > 0;
 }
 
-// ---- programmatic dependent launch ---------------------------------------------------------------------------
-// The pack kernel and the GEMM are launched with the programmatic-stream-serialization attribute: the next kernel of the
-// stream may start while this one still runs, and whatever it reads from a predecessor comes after its own
-// griddepcontrol.wait, which returns once the predecessors have completed and their writes are visible.  A decode step is
-// short launches back to back; this way a kernel's launch and prologue overlap the tail of its predecessor.  (Inside a
-// replayed CUDA graph the gain is within the noise: launches are back to back there anyway.  Requesting the first weight
-// tiles ahead of the wait changed nothing either.)
-__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // ============================================================================================================
 // Pack kernel: token rows -> per (token block, k step) chunks in the operand layout of the MMA.
 //   row r of the chunk (r < n_mma) is 128 bytes = 128 e4m3 values of k = 128 kt .. +127, its 16-byte pieces XOR-
@@ -139,8 +128,7 @@ struct PackParams {
 
 template <bool SPLIT>
 __global__ void __launch_bounds__(256) mx_pack_x_kernel(const GemmParams p, const PackParams a) {
-  pdl_launch_dependents();
-  pdl_wait();
+  pdl_begin();
   const int64_t slot = blockIdx.x;
   const int kt = blockIdx.y;
   int e; int64_t row0; int rows;
@@ -227,8 +215,7 @@ __device__ __forceinline__ void mx4_scale(float amax, uint32_t& sb, float& scale
 // CTAs, was tried in place of the loop over rows below: 2.3 x slower.  A row's four-term chain is latency, and four of
 // them in one warp add up where eight warps of a CTA overlap them.)
 __global__ void __launch_bounds__(256) mx_pack_x4_kernel(const GemmParams p, const PackParams a) {
-  pdl_launch_dependents();
-  pdl_wait();
+  pdl_begin();
   const int64_t slot = blockIdx.x;
   const int kt = blockIdx.y;
   int e; int64_t row0; int rows;
@@ -377,8 +364,7 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xFFFFFFFFu, *s_tmem, 0);
-  pdl_launch_dependents();
-  pdl_wait();
+  pdl_begin();
 
   const int KT = q.KT, NB = q.NB, NG = q.n_groups;
   uint32_t useful_m = (uint32_t)q.grid_m;
@@ -708,22 +694,6 @@ MxPlan mx_plan(const MoeGemmArgs& a) {
   }
   pl.ws_bytes = pl.grid_m * pl.KT * pl.chunk_bytes;
   return pl;
-}
-
-// launch with the programmatic-stream-serialization attribute (see pdl_wait above)
-template <typename... KArgs, typename... Args>
-cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
 template <typename TY, int MB, bool F4, bool KM = false>

@@ -212,6 +212,7 @@ __device__ __noinline__ uint32_t exact_rows(const GemmParams& p, const PairPackP
 // rows of 2880 took 153 us and 4800 rows 20.3, so 141 and 16.8.
 template <bool TILED>
 __global__ void __launch_bounds__(256) mx_pair_pack2_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ PairPackParams a) {
+  pdl_begin();
   int e; int64_t row0, prow0; int rows;
   if (!pack_block(p, blockIdx.x, e, row0, rows, prow0)) return;
   const int G = a.KT * 4;
@@ -275,7 +276,8 @@ __global__ void __launch_bounds__(256) mx_pair_pack2_kernel(const __grid_constan
   if (threadIdx.x == 0) a.done[prow0 >> 4] = done;
 }
 
-__global__ void __launch_bounds__(256) mx_pair_pack1_kernel(const GemmParams p, const PairPackParams a) {
+__global__ void __launch_bounds__(256) mx_pair_pack1_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ PairPackParams a) {
+  pdl_begin();
   int e; int64_t row0, prow0; int rows;
   if (!pack_block(p, blockIdx.x, e, row0, rows, prow0)) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -392,6 +394,7 @@ gemm_mx_pair_kernel(const GemmParams p, const PairParams a, const __grid_constan
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(ctl0 + PP_OFF_MISC), "r"((uint32_t)TMEM_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
+  pdl_begin();
   if (warp == PP_SF_WARP0) {                           // tile prefix over experts
     pair_prefix(p, s_prefix, a.nmax, lane);
   }
@@ -737,10 +740,12 @@ int launch_mx_pair(const GemmParams& p, PairParams q, const PairShape& shape, co
   cfg.blockDim = dim3(PP_THREADS, 1, 1);
   cfg.dynamicSmemBytes = PP_SMEM;
   cfg.stream = st;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-  cfg.attrs = at; cfg.numAttrs = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at; cfg.numAttrs = 1;                    // (the occupancy query has no use for the second)
   // per device: opt in to the shared-memory size once, and ask how many pairs can be resident at a time
   static std::mutex mu;
   static int max_pairs[64] = {0};
@@ -767,6 +772,7 @@ int launch_mx_pair(const GemmParams& p, PairParams q, const PairShape& shape, co
   if (pairs < 1) pairs = 1;
   if (tiles < pairs) pairs = tiles;
   cfg.gridDim = dim3((unsigned)(2 * pairs), 1, 1);
+  cfg.numAttrs = 2;
   moe_count_launch();
   MOE_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kernel, p, q, maps));
   return MOE_OK;
@@ -853,9 +859,8 @@ int moe_gemm_mx_pair_launch(const GemmParams& p_in, const MoeGemmArgs& a, cudaSt
   pk.K = a.K; pk.KT = pl.KT; pk.NB = pl.NB; pk.y_dtype = a.y_dtype; pk.prows = pl.prows;
   pk.xq = (uint8_t*)a.mx_workspace; pk.xs = pk.xq + pl.xs_off; pk.done = (uint32_t*)(pk.xq + pl.done_off);
   const bool tiled = a.w_kind == MOE_W_MX4_B200;
-  if (pl.terms == 2 && tiled) mx_pair_pack2_kernel<true><<<(unsigned)blocks16, 256, 0, st>>>(p, pk);
-  else if (pl.terms == 2) mx_pair_pack2_kernel<false><<<(unsigned)blocks16, 256, 0, st>>>(p, pk);
-  else mx_pair_pack1_kernel<<<(unsigned)blocks16, 256, 0, st>>>(p, pk);
+  auto pack = pl.terms == 1 ? mx_pair_pack1_kernel : tiled ? mx_pair_pack2_kernel<true> : mx_pair_pack2_kernel<false>;
+  MOE_CHECK_CUDA(launch_pdl(pack, dim3((unsigned)blocks16), dim3(256), 0, st, p, pk));
   MOE_CHECK_LAUNCH();
   PairParams q;
   q.xq = pk.xq; q.xs = pk.xs; q.done = pk.done; q.prows = pl.prows; q.KT = pl.KT; q.NB = pl.NB;

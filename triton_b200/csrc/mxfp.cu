@@ -120,10 +120,11 @@ __device__ __forceinline__ uint4 quantise_raw(const uint4 (&raw)[VPG], int mode,
 }
 
 template <typename T, typename I>
-__global__ void __launch_bounds__(256, sizeof(T) == 2 ? 3 : 2) downcast_rows_kernel(const T* __restrict__ x, int64_t n_rows, int64_t quant,
+__global__ void __launch_bounds__(256, sizeof(T) == 2 ? 3 : 2) downcast_rows_kernel(const T* x, int64_t n_rows, int64_t quant,
                                                             int64_t outer, int64_t sx_batch, int64_t sx_outer,
-                                                            uint8_t* __restrict__ q, uint8_t* __restrict__ scale,
+                                                            uint8_t* q, uint8_t* scale,
                                                             int mode) {
+  pdl_begin();
   constexpr int EPV = 16 / (int)sizeof(T);               // elements per 16-byte vector
   constexpr int VPG = 32 / EPV;                          // vectors per group
   const int64_t groups_per_row = quant >> 5;
@@ -205,8 +206,9 @@ template <> __device__ __forceinline__ float2 pair_absmax<float>(const float2 (&
 
 template <typename T>
 __global__ void __launch_bounds__(256, sizeof(T) == 2 ? 4 : 2) downcast_cols_kernel(
-    const T* __restrict__ x, int64_t outer, int groups, int col_blocks, int group_blocks, int64_t sx_batch, int64_t sx_quant,
-    uint8_t* __restrict__ q, uint8_t* __restrict__ scale, int mode) {
+    const T* x, int64_t outer, int groups, int col_blocks, int group_blocks, int64_t sx_batch, int64_t sx_quant,
+    uint8_t* q, uint8_t* scale, int mode) {
+  pdl_begin();
   using Raw = typename Pair<T>::Raw;
   __shared__ __align__(16) uint8_t s_q[CT_GROUPS * CT_PITCH];
   __shared__ uint8_t s_s[CT_COLS * CT_GROUPS];
@@ -260,10 +262,11 @@ __global__ void __launch_bounds__(256, sizeof(T) == 2 ? 4 : 2) downcast_cols_ker
 
 // ---- strided path: any strides; consecutive threads walk the `outer` axis ---------------------------
 template <typename T>
-__global__ void __launch_bounds__(256) downcast_strided_kernel(const T* __restrict__ x, int64_t batch, int64_t outer,
+__global__ void __launch_bounds__(256) downcast_strided_kernel(const T* x, int64_t batch, int64_t outer,
                                                                int64_t quant, int64_t sx_batch, int64_t sx_outer,
-                                                               int64_t sx_quant, uint8_t* __restrict__ q,
-                                                               uint8_t* __restrict__ scale, int mode) {
+                                                               int64_t sx_quant, uint8_t* q,
+                                                               uint8_t* scale, int mode) {
+  pdl_begin();
   const int64_t groups = quant >> 5;
   const int64_t total = batch * outer * groups;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -353,10 +356,11 @@ constexpr int ROWS_UNROLL = 4;
 // contiguous output: thread owns U units of 8 elements (4 input bytes each) of each of ROWS_UNROLL chunks per iteration; a
 // chunk of two units of a 2-byte type, or of one of fp32, leaves as one 32-byte store (WIDE)
 template <typename T, bool WIDE>
-__global__ void __launch_bounds__(256) upcast_rows_kernel(const uint8_t* __restrict__ q,
-                                                          const uint8_t* __restrict__ scale, T* __restrict__ out,
+__global__ void __launch_bounds__(256) upcast_rows_kernel(const uint8_t* q,
+                                                          const uint8_t* scale, T* out,
                                                           int64_t n_rows, int64_t quant, int64_t outer,
                                                           int64_t so_batch, int64_t so_outer) {
+  pdl_begin();
   constexpr int U = WIDE && sizeof(T) == 2 ? 2 : 1;
   const int64_t chunks_per_row = quant / (8 * U);
   const int64_t total = n_rows * chunks_per_row;
@@ -423,9 +427,10 @@ __global__ void __launch_bounds__(256) upcast_rows_kernel(const uint8_t* __restr
 // (128-byte runs) through shared memory; warp = group, lane = two neighbouring columns, every store of a warp is 128
 // contiguous bytes (fp32: 256).  A thread per column and group stored 64-byte runs from loads at the pitch of a row.
 template <typename T>
-__global__ void __launch_bounds__(256) upcast_cols_kernel(const uint8_t* __restrict__ q, const uint8_t* __restrict__ scale,
-                                                          T* __restrict__ out, int64_t outer, int groups, int col_blocks,
+__global__ void __launch_bounds__(256) upcast_cols_kernel(const uint8_t* q, const uint8_t* scale,
+                                                          T* out, int64_t outer, int groups, int col_blocks,
                                                           int group_blocks, int64_t so_batch, int64_t so_quant) {
+  pdl_begin();
   __shared__ __align__(16) uint8_t s_q[CT_GROUPS * CT_PITCH];
   __shared__ uint8_t s_s[CT_COLS * CT_GROUPS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -478,10 +483,11 @@ __global__ void __launch_bounds__(256) upcast_cols_kernel(const uint8_t* __restr
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) upcast_strided_kernel(const uint8_t* __restrict__ q,
-                                                             const uint8_t* __restrict__ scale, T* __restrict__ out,
+__global__ void __launch_bounds__(256) upcast_strided_kernel(const uint8_t* q,
+                                                             const uint8_t* scale, T* out,
                                                              int64_t batch, int64_t outer, int64_t quant,
                                                              int64_t so_batch, int64_t so_outer, int64_t so_quant) {
+  pdl_begin();
   const int64_t groups = quant >> 5;
   const int64_t total = batch * outer * groups;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -536,21 +542,21 @@ extern "C" __attribute__((visibility("default"))) int moe_downcast_mxfp4(const v
     if (rows_ok && (uintptr_t)q % 16 == 0) {
       const int64_t total = batch * outer * (quant >> 5);
       if (total + (int64_t)GROUPS_UNROLL * 256 * moe_sm_count() * 16 < 2147483647LL)       // 32-bit row / group counters
-        downcast_rows_kernel<T, int32_t><<<grid_for(total, GROUPS_UNROLL * 256), 256, 0, st>>>(
-            (const T*)x, batch * outer, quant, outer, sx_batch, sx_outer, q, scale, rounding_mode);
+        MOE_CHECK_CUDA(launch_pdl(downcast_rows_kernel<T, int32_t>, dim3(grid_for(total, GROUPS_UNROLL * 256)), dim3(256), 0, st,
+                                  (const T*)x, batch * outer, quant, outer, sx_batch, sx_outer, q, scale, rounding_mode));
       else
-        downcast_rows_kernel<T, int64_t><<<grid_for(total, GROUPS_UNROLL * 256), 256, 0, st>>>(
-            (const T*)x, batch * outer, quant, outer, sx_batch, sx_outer, q, scale, rounding_mode);
+        MOE_CHECK_CUDA(launch_pdl(downcast_rows_kernel<T, int64_t>, dim3(grid_for(total, GROUPS_UNROLL * 256)), dim3(256), 0, st,
+                                  (const T*)x, batch * outer, quant, outer, sx_batch, sx_outer, q, scale, rounding_mode));
     } else if (cols_ok) {
       const int groups = (int)(quant >> 5);
-      downcast_cols_kernel<T><<<(unsigned)col_tiles(batch, outer, quant), 256, 0, st>>>(
-          (const T*)x, outer, groups, (int)cdiv64(outer, CT_COLS), (int)cdiv64(groups, CT_GROUPS), sx_batch, sx_quant, q, scale,
-          rounding_mode);
+      MOE_CHECK_CUDA(launch_pdl(downcast_cols_kernel<T>, dim3((unsigned)col_tiles(batch, outer, quant)), dim3(256), 0, st, (const T*)x,
+                                outer, groups, (int)cdiv64(outer, CT_COLS), (int)cdiv64(groups, CT_GROUPS), sx_batch, sx_quant, q,
+                                scale, rounding_mode));
     } else {
       MOE_CHECK_ARG((uintptr_t)q % 16 == 0, "moe_downcast_mxfp4: q must be 16-byte aligned");
       const int64_t total = batch * outer * (quant >> 5);
-      downcast_strided_kernel<T><<<grid_for(total, 256), 256, 0, st>>>((const T*)x, batch, outer, quant, sx_batch,
-                                                                       sx_outer, sx_quant, q, scale, rounding_mode);
+      MOE_CHECK_CUDA(launch_pdl(downcast_strided_kernel<T>, dim3(grid_for(total, 256)), dim3(256), 0, st, (const T*)x, batch, outer,
+                                quant, sx_batch, sx_outer, sx_quant, q, scale, rounding_mode));
     }
   });
   MOE_CHECK_LAUNCH();
@@ -573,22 +579,22 @@ extern "C" __attribute__((visibility("default"))) int moe_upcast_mxfp4(const uin
                       (uintptr_t)q % 8 == 0;
     if (wide) {
       const int64_t total = batch * outer * (quant * (int64_t)sizeof(T) >> 5);
-      upcast_rows_kernel<T, true><<<grid_for(total, ROWS_UNROLL * 256), 256, 0, st>>>(q, scale, (T*)out, batch * outer, quant, outer,
-                                                                                      so_batch, so_outer);
+      MOE_CHECK_CUDA(launch_pdl(upcast_rows_kernel<T, true>, dim3(grid_for(total, ROWS_UNROLL * 256)), dim3(256), 0, st, q, scale,
+                                (T*)out, batch * outer, quant, outer, so_batch, so_outer));
     } else if (rows_ok) {
       const int64_t total = batch * outer * (quant >> 3);
-      upcast_rows_kernel<T, false><<<grid_for(total, ROWS_UNROLL * 256), 256, 0, st>>>(q, scale, (T*)out, batch * outer, quant, outer,
-                                                                                       so_batch, so_outer);
+      MOE_CHECK_CUDA(launch_pdl(upcast_rows_kernel<T, false>, dim3(grid_for(total, ROWS_UNROLL * 256)), dim3(256), 0, st, q, scale,
+                                (T*)out, batch * outer, quant, outer, so_batch, so_outer));
     } else if (so_outer == 1 && so_quant % 2 == 0 && so_batch % 2 == 0 && outer % 2 == 0 && (uintptr_t)q % 16 == 0 &&
                (uintptr_t)out % (2 * sizeof(T)) == 0 && col_tiles(batch, outer, quant) < 2147483647LL) {
       const int groups = (int)(quant >> 5);
-      upcast_cols_kernel<T><<<(unsigned)col_tiles(batch, outer, quant), 256, 0, st>>>(
-          q, scale, (T*)out, outer, groups, (int)cdiv64(outer, CT_COLS), (int)cdiv64(groups, CT_GROUPS), so_batch, so_quant);
+      MOE_CHECK_CUDA(launch_pdl(upcast_cols_kernel<T>, dim3((unsigned)col_tiles(batch, outer, quant)), dim3(256), 0, st, q, scale,
+                                (T*)out, outer, groups, (int)cdiv64(outer, CT_COLS), (int)cdiv64(groups, CT_GROUPS), so_batch, so_quant));
     } else {
       MOE_CHECK_ARG((uintptr_t)q % 16 == 0, "moe_upcast_mxfp4: q must be 16-byte aligned");
       const int64_t total = batch * outer * (quant >> 5);
-      upcast_strided_kernel<T><<<grid_for(total, 256), 256, 0, st>>>(q, scale, (T*)out, batch, outer, quant, so_batch,
-                                                                     so_outer, so_quant);
+      MOE_CHECK_CUDA(launch_pdl(upcast_strided_kernel<T>, dim3(grid_for(total, 256)), dim3(256), 0, st, q, scale, (T*)out, batch, outer,
+                                quant, so_batch, so_outer, so_quant));
     }
   });
   MOE_CHECK_LAUNCH();

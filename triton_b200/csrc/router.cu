@@ -115,6 +115,7 @@ router_topk_kernel(const RouterParams p, const __grid_constant__ CUtensorMap x_m
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, s_tmem, 0);
+  pdl_begin();
 
   const int64_t blk = blockIdx.x;
   const int split = blockIdx.y;
@@ -385,7 +386,7 @@ extern "C" __attribute__((visibility("default"))) int moe_router_topk(
 #define RT_LAUNCH(KK)                                                                                                    \
   do {                                                                                                                   \
     MOE_CHECK_CUDA(cudaFuncSetAttribute(router_topk_kernel<KK>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));     \
-    router_topk_kernel<KK><<<grid, RT_THREADS, smem, st>>>(p, x_map, w_map);                                             \
+    MOE_CHECK_CUDA(launch_pdl(router_topk_kernel<KK>, grid, dim3(RT_THREADS), smem, st, p, x_map, w_map));               \
   } while (0)
   switch (k) {
     case 1: RT_LAUNCH(1); break;

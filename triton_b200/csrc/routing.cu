@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) topk_kernel(
 // partial[block][e], the first pass of the expert sort.  The warp-per-row kernel above spends its time in k rounds of
 // 64-bit warp reductions per row: 19.6 us for 16384 x 128 logits against about 5 us here.
 template <typename T, int K>
-__device__ __forceinline__ TopK<K> quad_select(const T* __restrict__ x, int E, int part, int parts = 4) {
+__device__ __forceinline__ TopK<K> quad_select(const T* x, int E, int part, int parts = 4) {
   constexpr int NL = K <= 4 ? 2 : 1;
   TopK<K> sub[NL];
   float v[NL][4];
@@ -200,10 +200,10 @@ __device__ __forceinline__ void quad_store(const TopK<K>& tk, int part, int64_t 
 
 template <typename T, int K, bool HIST>
 __global__ void __launch_bounds__(HIST ? 1024 : 256) topk_quad_kernel(
-    const T* __restrict__ logits, int64_t ld_logits, int64_t T_rows, int E, int apply_softmax, T* __restrict__ vals,
-    int64_t ld_vals, int16_t* __restrict__ indx, int64_t ld_indx, uint32_t* __restrict__ bitmatrix, int64_t bm_stride_row,
-    int64_t bm_stride_word, int32_t* __restrict__ partial) {
+    const T* logits, int64_t ld_logits, int64_t T_rows, int E, int apply_softmax, T* vals, int64_t ld_vals, int16_t* indx,
+    int64_t ld_indx, uint32_t* bitmatrix, int64_t bm_stride_row, int64_t bm_stride_word, int32_t* partial) {
   extern __shared__ int32_t s_hist[];                     // [E] with HIST
+  pdl_begin();
   if constexpr (HIST) {
     for (int e = threadIdx.x; e < E; e += blockDim.x) s_hist[e] = 0;
     __syncthreads();
@@ -226,9 +226,9 @@ __global__ void __launch_bounds__(HIST ? 1024 : 256) topk_quad_kernel(
 // Expert histogram + stable expert-major sort.  Flat entry i = token * k + slot, expert c = indx[i]
 // (negative, or token >= n_rows: dropped).  row_sorted[i] = col_offs[c] + #{j < i : indx[j] == c},
 // col_sorted = inverse permutation; both -1 padded.
-//   pass 1: per block of kTokPerBlock tokens, a shared-memory histogram -> partial[blk][e]; global
-//           histogram by atomics; both index arrays pre-filled with -1.
-//   pass 2: exclusive scan of partial[.][e] over blocks, exclusive scan of col_sum -> col_offs.
+//   pass 1: per block of kTokPerBlock tokens, a shared-memory histogram -> partial[blk][e]; both index arrays
+//           pre-filled with -1.
+//   pass 2: exclusive scan of partial[.][e] over blocks, totals -> col_sum, their exclusive scan -> col_offs.
 //   pass 3: rank inside the block: each warp owns 32 consecutive tokens and ranks them in order with
 //           warp match, on top of the counts of the warps before it.
 constexpr int kTokPerBlock = 256;
@@ -240,10 +240,10 @@ __device__ __forceinline__ int entry_expert(const int16_t* indx, int64_t ld_indx
   return (c < 0 || c >= E) ? -1 : c;
 }
 
-__global__ void __launch_bounds__(256) bm_hist_kernel(const int16_t* __restrict__ indx, int64_t ld_indx, int64_t T_rows,
-                                                      int E, int k, const int32_t* __restrict__ n_rows_dev,
-                                                      int32_t* __restrict__ col_sum, int32_t* __restrict__ partial,
-                                                      int32_t* __restrict__ col_sorted, int32_t* __restrict__ row_sorted) {
+__global__ void __launch_bounds__(256) bm_hist_kernel(const int16_t* indx, int64_t ld_indx, int64_t T_rows,
+                                                      int E, int k, const int32_t* n_rows_dev,
+                                                      int32_t* partial, int32_t* col_sorted, int32_t* row_sorted) {
+  pdl_begin();
   extern __shared__ int32_t s_cnt[];
   const int64_t n_rows = n_rows_dev ? min((int64_t)*n_rows_dev, T_rows) : T_rows;
   for (int e = threadIdx.x; e < E; e += blockDim.x) s_cnt[e] = 0;
@@ -271,9 +271,7 @@ __global__ void __launch_bounds__(256) bm_hist_kernel(const int16_t* __restrict_
   }
   __syncthreads();
   for (int e = threadIdx.x; e < E; e += blockDim.x) {
-    int v = s_cnt[e];
-    partial[(int64_t)blockIdx.x * E + e] = v;
-    if (v) atomicAdd(&col_sum[e], v);
+    partial[(int64_t)blockIdx.x * E + e] = s_cnt[e];
   }
 }
 
@@ -310,29 +308,48 @@ __device__ void block_exclusive_scan(const int32_t* in, int32_t* out, int n, int
   }
 }
 
-__global__ void __launch_bounds__(1024) bm_scan_kernel(int32_t* __restrict__ partial, int64_t n_blocks, int E,
-                                                       const int32_t* __restrict__ col_sum,
-                                                       int32_t* __restrict__ col_offs) {
+// One block: exclusive scan of partial[.][e] over the blocks of tokens, by S segments of blocks per expert (1024 experts at a time),
+// the expert totals (col_sum) and their exclusive scan (col_offs).  Totals added up by atomics in the pass before would want a cleared
+// array, a launch of its own.
+__global__ void __launch_bounds__(1024) bm_scan_kernel(int32_t* partial, int64_t n_blocks, int E, int32_t* col_sum, int32_t* col_offs) {
+  pdl_begin();
+  __shared__ int32_t s_seg[1024];
   __shared__ int32_t s_warp[33];
-  if (blockIdx.x == 0) {
-    block_exclusive_scan(col_sum, col_offs, E, s_warp);
-    return;
-  }
-  // remaining blocks: one thread per expert walks the blocks of tokens
-  const int e = (blockIdx.x - 1) * blockDim.x + threadIdx.x;
-  if (e >= E) return;
-  // sixteen loads in flight per thread: the walk is a chain of L2 round trips otherwise
-  int run = 0;
-  for (int64_t b0 = 0; b0 < n_blocks; b0 += 16) {
-    int v[16];
+  int Ep = 1;
+  while (Ep < E && Ep < 1024) Ep <<= 1;
+  const int S = 1024 / Ep, seg = threadIdx.x / Ep;
+  const int64_t per = (n_blocks + S - 1) / S;
+  const int64_t b_lo = min((int64_t)seg * per, n_blocks), b_hi = min(b_lo + per, n_blocks);
+  for (int e0 = 0; e0 < E; e0 += Ep) {
+    const int e = e0 + (int)(threadIdx.x % Ep);
+    // sixteen loads in flight per thread: the walk is a chain of L2 round trips otherwise
+    auto walk = [&](int run, bool store) {
+      if (e < E)
+        for (int64_t b0 = b_lo; b0 < b_hi; b0 += 16) {
+          int v[16];
 #pragma unroll
-    for (int u = 0; u < 16; ++u) v[u] = b0 + u < n_blocks ? partial[(b0 + u) * E + e] : 0;
+          for (int u = 0; u < 16; ++u) v[u] = b0 + u < b_hi ? partial[(b0 + u) * E + e] : 0;
 #pragma unroll
-    for (int u = 0; u < 16; ++u) {
-      if (b0 + u < n_blocks) partial[(b0 + u) * E + e] = run;
-      run += v[u];
+          for (int u = 0; u < 16; ++u) {
+            if (store && b0 + u < b_hi) partial[(b0 + u) * E + e] = run;
+            run += v[u];
+          }
+        }
+      return run;
+    };
+    s_seg[threadIdx.x] = walk(0, false);
+    __syncthreads();
+    int run = 0, total = 0;
+    for (int i = 0; i < S; ++i) {
+      const int v = s_seg[i * Ep + (int)(threadIdx.x % Ep)];
+      if (i < seg) run += v;
+      total += v;
     }
+    walk(run, true);
+    if (seg == 0 && e < E) col_sum[e] = total;
+    __syncthreads();
   }
+  block_exclusive_scan(col_sum, col_offs, E, s_warp);
 }
 
 // What the layer wants per expert-sorted position beside the permutation: token row and routing weight (token NULL: nothing).
@@ -345,7 +362,7 @@ struct PerPosition {
 
 // Positions of the entries of one block of blockDim.x tokens starting at token `tok_base`: `base[e]` is where the
 // block's entries of expert e start (expert offset + entries of earlier blocks); s_cnt holds [warps][E] counters.
-__device__ __forceinline__ void rank_block(const int16_t* __restrict__ indx, int64_t ld_indx, int64_t T_rows, int E, int k,
+__device__ __forceinline__ void rank_block(const int16_t* indx, int64_t ld_indx, int64_t T_rows, int E, int k,
                                            int64_t n_rows, const int32_t* base_a, const int32_t* base_b, int64_t tok_base,
                                            int32_t* __restrict__ col_sorted, int32_t* __restrict__ row_sorted, int32_t* s_cnt,
                                            const PerPosition& out = PerPosition()) {
@@ -397,13 +414,12 @@ __device__ __forceinline__ void rank_block(const int16_t* __restrict__ indx, int
   }
 }
 
-__global__ void __launch_bounds__(256) bm_rank_kernel(const int16_t* __restrict__ indx, int64_t ld_indx, int64_t T_rows,
-                                                      int E, int k, const int32_t* __restrict__ n_rows_dev,
-                                                      const int32_t* __restrict__ partial,
-                                                      const int32_t* __restrict__ col_offs,
-                                                      int32_t* __restrict__ col_sorted, int32_t* __restrict__ row_sorted,
+__global__ void __launch_bounds__(256) bm_rank_kernel(const int16_t* indx, int64_t ld_indx, int64_t T_rows, int E, int k,
+                                                      const int32_t* n_rows_dev, const int32_t* partial,
+                                                      const int32_t* col_offs, int32_t* col_sorted, int32_t* row_sorted,
                                                       const PerPosition out) {
   extern __shared__ int32_t s_cnt[];  // [warps][E]; a block covers blockDim.x tokens, the blocks of `partial`
+  pdl_begin();
   const int64_t n_rows = n_rows_dev ? min((int64_t)*n_rows_dev, T_rows) : T_rows;
   rank_block(indx, ld_indx, T_rows, E, k, n_rows, partial + (int64_t)blockIdx.x * E, col_offs, (int64_t)blockIdx.x * blockDim.x,
              col_sorted, row_sorted, s_cnt, out);
@@ -526,9 +542,9 @@ extern "C" __attribute__((visibility("default"))) int moe_topk_fwd(const void* l
     const int qgrid = (int)cdiv64(T, 64);
 #define MOE_TOPK_QUAD(KK)                                                                                                 \
   MOE_DISPATCH_FLOAT(dtype, Tv, {                                                                                         \
-    topk_quad_kernel<Tv, KK, false><<<qgrid, 256, 0, st>>>((const Tv*)logits, ld_logits, T, E, apply_softmax, (Tv*)vals,   \
-                                                           ld_vals, indx, ld_indx, bitmatrix, bm_stride_row,               \
-                                                           bm_stride_word, nullptr);                                       \
+    MOE_CHECK_CUDA(launch_pdl(topk_quad_kernel<Tv, KK, false>, dim3(qgrid), dim3(256), 0, st, (const Tv*)logits, ld_logits, \
+                              T, E, apply_softmax, (Tv*)vals, ld_vals, indx, ld_indx, bitmatrix, bm_stride_row,             \
+                              bm_stride_word, nullptr));                                                                    \
   })
     switch (k) {
       case 1: MOE_TOPK_QUAD(1); break;
@@ -563,8 +579,10 @@ extern "C" __attribute__((visibility("default"))) int moe_bitmatrix_metadata(con
   MOE_CHECK_ARG(T >= 0 && E > 0 && k > 0, "moe_bitmatrix_metadata: bad extents T=%lld E=%d k=%d", (long long)T, E, k);
   MOE_CHECK_ARG(col_sum, "moe_bitmatrix_metadata: col_sum is NULL");
   cudaStream_t st = (cudaStream_t)stream;
-  MOE_CHECK_CUDA(cudaMemsetAsync(col_sum, 0, sizeof(int32_t) * (size_t)E, st));
-  if (T == 0) return MOE_OK;
+  if (T == 0) {
+    MOE_CHECK_CUDA(cudaMemsetAsync(col_sum, 0, sizeof(int32_t) * (size_t)E, st));
+    return MOE_OK;
+  }
   MOE_CHECK_ARG(indx && col_sorted && row_sorted && workspace, "moe_bitmatrix_metadata: NULL pointer");
   MOE_CHECK_ARG(workspace_bytes >= moe_bitmatrix_metadata_workspace(T, E, k),
                 "moe_bitmatrix_metadata: workspace too small (%zu < %zu)", workspace_bytes,
@@ -574,15 +592,15 @@ extern "C" __attribute__((visibility("default"))) int moe_bitmatrix_metadata(con
   const int64_t nb = cdiv64(T, kTokPerBlock);
   int32_t* partial = (int32_t*)workspace;
   int32_t* col_offs = partial + nb * E;
-  bm_hist_kernel<<<(int)nb, 256, (size_t)E * sizeof(int32_t), st>>>(indx, ld_indx, T, E, k, n_rows_dev, col_sum, partial,
-                                                                  col_sorted, row_sorted);
+  MOE_CHECK_CUDA(launch_pdl(bm_hist_kernel, dim3((unsigned)nb), dim3(256), (size_t)E * sizeof(int32_t), st, indx, ld_indx, T, E, k,
+                            n_rows_dev, partial, col_sorted, row_sorted));
   MOE_CHECK_LAUNCH();
-  bm_scan_kernel<<<1 + (int)cdiv64(E, 1024), 1024, 0, st>>>(partial, nb, E, col_sum, col_offs);
+  MOE_CHECK_CUDA(launch_pdl(bm_scan_kernel, dim3(1), dim3(1024), 0, st, partial, nb, E, col_sum, col_offs));
   MOE_CHECK_LAUNCH();
   if (smem_rank > 48 * 1024)
     MOE_CHECK_CUDA(cudaFuncSetAttribute(bm_rank_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_rank));
-  bm_rank_kernel<<<(int)nb, 256, smem_rank, st>>>(indx, ld_indx, T, E, k, n_rows_dev, partial, col_offs, col_sorted,
-                                                  row_sorted, PerPosition());
+  MOE_CHECK_CUDA(launch_pdl(bm_rank_kernel, dim3((unsigned)nb), dim3(256), smem_rank, st, indx, ld_indx, T, E, k, n_rows_dev, partial,
+                            col_offs, col_sorted, row_sorted, PerPosition()));
   MOE_CHECK_LAUNCH();
   return MOE_OK;
 }
@@ -643,10 +661,11 @@ constexpr int kRowsPerWarp = kRouteTokPerBlock / kRouteWarps;
 // reductions (redux.sync): the largest value key, then the smallest expert index among the lanes that hold it.
 template <typename T>
 __global__ void __launch_bounds__(kRouteWarps * 32) route_topk_hist_kernel(
-    const T* __restrict__ logits, int64_t ld_logits, int64_t T_rows, int E, int k, int apply_softmax,
-    T* __restrict__ vals, int64_t ld_vals, int16_t* __restrict__ indx, int64_t ld_indx,
-    uint32_t* __restrict__ bitmatrix, int64_t bm_stride_row, int64_t bm_stride_word, int32_t* __restrict__ partial) {
+    const T* logits, int64_t ld_logits, int64_t T_rows, int E, int k, int apply_softmax,
+    T* vals, int64_t ld_vals, int16_t* indx, int64_t ld_indx,
+    uint32_t* bitmatrix, int64_t bm_stride_row, int64_t bm_stride_word, int32_t* partial) {
   extern __shared__ int32_t s_hist[];                     // [E]
+  pdl_begin();
   __shared__ float s_val[kRouteWarps][kMaxTopK];
   __shared__ int s_idx[kRouteWarps][kMaxTopK];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -757,14 +776,15 @@ __device__ void ragged_row(int row, const int32_t* s_size, int E, int32_t* s_nb,
 }
 
 // Six blocks of 1024 threads.  n_experts <= 1024.
-__global__ void __launch_bounds__(1024) route_scan_ragged_kernel(const int32_t* __restrict__ partial_in,
-                                                                 int32_t* __restrict__ partial_out, int64_t n_blocks, int E,
-                                                                 int32_t* __restrict__ col_sum, int32_t* __restrict__ col_offs,
-                                                                 int32_t* __restrict__ slice_offs, int32_t* __restrict__ block_offs,
-                                                                 int64_t ld_block_offs, int32_t* __restrict__ block_sched,
+__global__ void __launch_bounds__(1024) route_scan_ragged_kernel(const int32_t* partial_in,
+                                                                 int32_t* partial_out, int64_t n_blocks, int E,
+                                                                 int32_t* col_sum, int32_t* col_offs,
+                                                                 int32_t* slice_offs, int32_t* block_offs,
+                                                                 int64_t ld_block_offs, int32_t* block_sched,
                                                                  int64_t ld_sched, int64_t n_sched) {
   extern __shared__ int32_t s_mem[];             // [1024] segment sums, then [E + 1] sizes, [E + 1] scan input, [E + 1] offsets
   __shared__ int32_t s_warp[33];
+  pdl_begin();
   int32_t* s_seg = s_mem;
   int32_t* s_size = s_mem + 1024;
   int32_t* s_nb = s_size + (E + 1);
@@ -844,14 +864,15 @@ __global__ void __launch_bounds__(1024) route_scan_ragged_kernel(const int32_t* 
 // from global memory by one warp per 32 tokens, 1 and 64 tokens of 128 experts took 11.6 and 12.7 us in a graph, so 4.3 and 8.3.
 template <typename T, int K>
 __global__ void __launch_bounds__(1024) route_small_kernel(
-    const T* __restrict__ logits, int64_t ld_logits, int T_rows, int E, int parts, int apply_softmax, T* __restrict__ vals,
-    int64_t ld_vals, int16_t* __restrict__ indx, int64_t ld_indx, uint32_t* __restrict__ bitmatrix, int64_t bm_stride_row,
-    int64_t bm_stride_word, int32_t* __restrict__ col_sum, int32_t* __restrict__ col_sorted, int32_t* __restrict__ row_sorted,
-    int32_t* __restrict__ slice_offs, int32_t* __restrict__ block_offs, int64_t ld_block_offs, int32_t* __restrict__ block_sched,
+    const T* logits, int64_t ld_logits, int T_rows, int E, int parts, int apply_softmax, T* vals,
+    int64_t ld_vals, int16_t* indx, int64_t ld_indx, uint32_t* bitmatrix, int64_t bm_stride_row,
+    int64_t bm_stride_word, int32_t* col_sum, int32_t* col_sorted, int32_t* row_sorted,
+    int32_t* slice_offs, int32_t* block_offs, int64_t ld_block_offs, int32_t* block_sched,
     int64_t ld_sched, int64_t n_sched, const PerPosition out) {
   // [E + 1] sizes, [E + 1] scan input, [E + 1] offsets, [n] values, [n] picks (int16), [warps in use][E] counters (uint16)
   extern __shared__ int32_t s_mem[];
   __shared__ int32_t s_warp[33];
+  pdl_begin();
   const int n = T_rows * K;
   int32_t* s_size = s_mem;
   int32_t* s_nb = s_size + (E + 1);
@@ -967,10 +988,10 @@ static int route_launch(
     const int parts = T <= 32 ? 32 : T <= 64 ? 16 : T <= 128 ? 8 : 4;
 #define MOE_ROUTE_SMALL(KK)                                                                                              \
   MOE_DISPATCH_FLOAT(dtype, Tv, {                                                                                         \
-    route_small_kernel<Tv, KK><<<5, 1024, smem_s, st>>>((const Tv*)logits, ld_logits, (int)T, E, parts, apply_softmax,       \
-                                                         (Tv*)vals, ld_vals, indx, ld_indx, bitmatrix, bm_stride_row,       \
-                                                         bm_stride_word, col_sum, col_sorted, row_sorted, slice_offs,       \
-                                                         block_offs, ld_block_offs, block_sched, ld_sched, n_sched, out);   \
+    MOE_CHECK_CUDA(launch_pdl(route_small_kernel<Tv, KK>, dim3(5), dim3(1024), smem_s, st, (const Tv*)logits, ld_logits,    \
+                              (int)T, E, parts, apply_softmax, (Tv*)vals, ld_vals, indx, ld_indx, bitmatrix, bm_stride_row, \
+                              bm_stride_word, col_sum, col_sorted, row_sorted, slice_offs, block_offs, ld_block_offs,       \
+                              block_sched, ld_sched, n_sched, out));                                                        \
   })
     switch (k) {
       case 1: MOE_ROUTE_SMALL(1); break;
@@ -989,9 +1010,9 @@ static int route_launch(
   int32_t* col_offs = scanned + nb * E;
 #define MOE_ROUTE_QUAD(KK)                                                                                               \
   MOE_DISPATCH_FLOAT(dtype, Tv, {                                                                                         \
-    topk_quad_kernel<Tv, KK, true><<<(int)nb, 4 * kRouteTokPerBlock, (size_t)E * sizeof(int32_t), st>>>(                                   \
-        (const Tv*)logits, ld_logits, T, E, apply_softmax, (Tv*)vals, ld_vals, indx, ld_indx, bitmatrix, bm_stride_row,    \
-        bm_stride_word, partial);                                                                                          \
+    MOE_CHECK_CUDA(launch_pdl(topk_quad_kernel<Tv, KK, true>, dim3((unsigned)nb), dim3(4 * kRouteTokPerBlock),              \
+                              (size_t)E * sizeof(int32_t), st, (const Tv*)logits, ld_logits, T, E, apply_softmax,           \
+                              (Tv*)vals, ld_vals, indx, ld_indx, bitmatrix, bm_stride_row, bm_stride_word, partial));       \
   })
   switch (k) {
     case 1: MOE_ROUTE_QUAD(1); break;
@@ -1001,20 +1022,20 @@ static int route_launch(
     case 16: MOE_ROUTE_QUAD(16); break;
     default:
       MOE_DISPATCH_FLOAT(dtype, Tv, {
-        route_topk_hist_kernel<Tv><<<(int)nb, kRouteWarps * 32, (size_t)E * sizeof(int32_t), st>>>(
-            (const Tv*)logits, ld_logits, T, E, k, apply_softmax, (Tv*)vals, ld_vals, indx, ld_indx, bitmatrix, bm_stride_row,
-            bm_stride_word, partial);
+        MOE_CHECK_CUDA(launch_pdl(route_topk_hist_kernel<Tv>, dim3((unsigned)nb), dim3(kRouteWarps * 32), (size_t)E * sizeof(int32_t),
+                                  st, (const Tv*)logits, ld_logits, T, E, k, apply_softmax, (Tv*)vals, ld_vals, indx, ld_indx,
+                                  bitmatrix, bm_stride_row, bm_stride_word, partial));
       });
   }
 #undef MOE_ROUTE_QUAD
   MOE_CHECK_LAUNCH();
   const size_t smem_b = (size_t)(1024 + 3 * (E + 1)) * sizeof(int32_t);
-  route_scan_ragged_kernel<<<6, 1024, smem_b, st>>>(partial, scanned, nb, E, col_sum, col_offs, slice_offs, block_offs,
-                                                    ld_block_offs, block_sched, ld_sched, n_sched);
+  MOE_CHECK_CUDA(launch_pdl(route_scan_ragged_kernel, dim3(6), dim3(1024), smem_b, st, partial, scanned, nb, E, col_sum, col_offs,
+                            slice_offs, block_offs, ld_block_offs, block_sched, ld_sched, n_sched));
   MOE_CHECK_LAUNCH();
   const size_t smem_rank = (size_t)(kRouteTokPerBlock / 32) * E * sizeof(int32_t);
-  bm_rank_kernel<<<(int)nb, kRouteTokPerBlock, smem_rank, st>>>(indx, ld_indx, T, E, k, nullptr, scanned, col_offs, col_sorted,
-                                                                row_sorted, out);
+  MOE_CHECK_CUDA(launch_pdl(bm_rank_kernel, dim3((unsigned)nb), dim3(kRouteTokPerBlock), smem_rank, st, indx, ld_indx, T, E, k, nullptr,
+                            scanned, col_offs, col_sorted, row_sorted, out));
   MOE_CHECK_LAUNCH();
   return MOE_OK;
 }
@@ -1083,7 +1104,7 @@ extern "C" __attribute__((visibility("default"))) int moe_bitmatrix_metadata_noa
     g_bm_scratch_addr[dev] = p;
   }
   // Nothing in the scratch has to start at zero: pass 1 writes every partial[block][expert] and pass 2 every
-  // col_offs[expert] before they are read.  col_sum, which must, is cleared by the call below.
+  // col_offs[expert] before they are read.
   return moe_bitmatrix_metadata(indx, ld_indx, T, E, k, n_rows_dev, col_sum, col_sorted, row_sorted,
                                 g_bm_scratch_addr[dev], kNoAllocScratchBytes, stream);
 }

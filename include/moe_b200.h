@@ -267,6 +267,10 @@ typedef struct {
                                                       of the block-scaled kernel, never a bound. */
 } MoeGemmArgs;
 int moe_grouped_gemm(const MoeGemmArgs* args_host, void* stream);
+/* Two products in a row: the same as moe_grouped_gemm of `first` and then of `second`, whose x is the first's y.  Where both run on
+ * block-scaled kernels and their workspaces do not overlap, the first product leaves its rows as the second's tokens in that
+ * workspace and y is scratch (its contents are then undefined).  The results of the second product are the same. */
+int moe_grouped_gemm_chain(const MoeGemmArgs* first_host, const MoeGemmArgs* second_host, void* stream);
 size_t moe_gemm_mx_workspace_bytes(const MoeGemmArgs* args_host);
 /* Name of the kernel that moe_grouped_gemm launches for these arguments (with the workspace of the size above given), "" for an
  * empty product; NULL, with the reason in moe_last_error(), where it refuses them.  Launches nothing and reads no device memory. */

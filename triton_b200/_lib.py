@@ -67,6 +67,7 @@ PROTOTYPES = {
     "moe_weight_layout_to_b200mx": (i32, [vp, i64, i64, vp, i64, i64, i64, i32, i32, i32, vp, vp, vp]),
     "moe_weight_layout_from_b200mx": (i32, [vp, vp, i32, i32, i32, vp, vp, vp]),
     "moe_grouped_gemm": (i32, [vp, vp]),
+    "moe_grouped_gemm_chain": (i32, [vp, vp, vp]),
     "moe_gemm_mx_workspace_bytes": (sz, [vp]),
     "moe_gemm_kernel_name": (C.c_char_p, [vp]),
     "moe_tensor_roof": (i32, [i32, i32, C.POINTER(C.c_double), vp, vp]),

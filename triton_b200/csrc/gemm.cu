@@ -8,11 +8,14 @@ int moe_gemm_tc_pair_launch(const GemmParams& p, const MoeGemmArgs& a, cudaStrea
 bool moe_gemm_tc_pair_supported(const MoeGemmArgs& a, const char** why);
 int moe_gemm_stream_launch(const GemmParams& p, const MoeGemmArgs& a, cudaStream_t st);
 bool moe_gemm_stream_supported(const MoeGemmArgs& a, const char** why);
-int moe_gemm_mx_launch(const GemmParams& p, const MoeGemmArgs& a, cudaStream_t st);
+int moe_gemm_mx_launch(const GemmParams& p, const MoeGemmArgs& a, const TokenOut& out, bool packed, cudaStream_t st);
+int moe_gemm_mx_terms(const MoeGemmArgs& a);
+bool moe_gemm_mx_token_out(const MoeGemmArgs& a, TokenOut& out);
+bool moe_gemm_mx_pair_token_out(const MoeGemmArgs& a, TokenOut& out);
 bool moe_gemm_mx_supported(const MoeGemmArgs& a, const char** why);
 bool moe_gemm_mx_pair_wanted(const MoeGemmArgs& a);
 int64_t moe_gemm_mx_pair_workspace(const MoeGemmArgs& a);
-int moe_gemm_mx_pair_launch(const GemmParams& p, const MoeGemmArgs& a, cudaStream_t st);
+int moe_gemm_mx_pair_launch(const GemmParams& p, const MoeGemmArgs& a, const TokenOut& out, bool packed, cudaStream_t st);
 
 // upper bound on the number of row blocks (triton_kernels tensor_details/ragged_tensor.py:73-77)
 static int64_t n_blocks_bound(int64_t n_slices, int64_t n_rows, int64_t block) {
@@ -111,14 +114,12 @@ extern "C" __attribute__((visibility("default"))) const char* moe_gemm_kernel_na
   return choose_kernel(*a, true, k) == MOE_OK ? KERNEL_NAME[k] : nullptr;
 }
 
-extern "C" __attribute__((visibility("default"))) int moe_grouped_gemm(const MoeGemmArgs* a, void* stream) {
-  if (const int rc = check_args(a)) return rc;
-  if (a->M == 0 || a->N == 0) return MOE_OK;
-  cudaStream_t st = (cudaStream_t)stream;
-  Kernel kernel;
-  const bool workspace = a->mx_workspace && a->mx_workspace_bytes >= moe_gemm_mx_pair_workspace(*a);
-  if (const int rc = choose_kernel(*a, workspace, kernel)) return rc;
+static bool has_workspace(const MoeGemmArgs* a) { return a->mx_workspace && a->mx_workspace_bytes >= moe_gemm_mx_pair_workspace(*a); }
 
+// The product on the kernel chosen for it.  out: its rows go there instead of y (block-scaled kernels); packed: its tokens are in
+// the workspace already.
+static int run_product(const MoeGemmArgs* a, Kernel kernel, const TokenOut& out, bool packed, void* stream) {
+  cudaStream_t st = (cudaStream_t)stream;
   GemmParams p;
   p.x = a->x; p.ld_x = a->ld_x; p.rows_x = a->rows_x;
   p.w = a->w; p.w_stride_e = a->w_stride_e; p.w_stride_k = a->w_stride_k; p.w_stride_n = a->w_stride_n;
@@ -137,8 +138,8 @@ extern "C" __attribute__((visibility("default"))) int moe_grouped_gemm(const Moe
   p.n_y_peers = a->n_y_peers; p.y_rows_per_peer = a->y_rows_per_peer;
   for (int i = 0; i < MOE_MAX_PEERS; ++i) p.y_peers[i] = i < a->n_y_peers ? a->y_peers[i] : nullptr;
 
-  if (kernel == K_MX_PAIR) return moe_gemm_mx_pair_launch(p, *a, st);
-  if (kernel == K_MX) return moe_gemm_mx_launch(p, *a, st);
+  if (kernel == K_MX_PAIR) return moe_gemm_mx_pair_launch(p, *a, out, packed, st);
+  if (kernel == K_MX) return moe_gemm_mx_launch(p, *a, out, packed, st);
   if (kernel == K_STREAM) return moe_gemm_stream_launch(p, *a, st);
   if (kernel == K_TC || kernel == K_TC_PAIR) {
     // Large gathered problems: copy the gathered rows once into the caller's scratch, then stream them by TMA.
@@ -162,4 +163,53 @@ extern "C" __attribute__((visibility("default"))) int moe_grouped_gemm(const Moe
   }
   if (grid_m == 0) return MOE_OK;
   return moe_gemm_simt_launch(p, a->x_dtype, a->y_dtype, a->w_kind, grid_m, st);
+}
+
+extern "C" __attribute__((visibility("default"))) int moe_grouped_gemm(const MoeGemmArgs* a, void* stream) {
+  if (const int rc = check_args(a)) return rc;
+  if (a->M == 0 || a->N == 0) return MOE_OK;
+  Kernel kernel;
+  if (const int rc = choose_kernel(*a, has_workspace(a), kernel)) return rc;
+  return run_product(a, kernel, TokenOut(), false, stream);
+}
+
+// Whether product a may leave its rows as the tokens of product b, and where.  Both run on block-scaled kernels; b takes exactly a's
+// rows, in the same ragged structure, from workspace of its own; nothing but bias and activation is between.  bf16 rows: a limit on the
+// activation, which bounds them far below where two terms stop holding a value (the pack kernels have a way for such rows):
+// |silu(g)| <= max(limit, 0.28 / alpha) and the factor <= limit + 1.
+static bool hands_over(const MoeGemmArgs& a, Kernel ka, const MoeGemmArgs& b, Kernel kb, TokenOut& out) {
+  if ((ka != K_MX_PAIR && ka != K_MX) || (kb != K_MX_PAIR && kb != K_MX)) return false;
+  if (a.activation != MOE_ACT_SWIGLU || a.N % 64 != 0 || a.N != 2 * b.K || a.M != b.M || a.E != b.E || b.x != a.y || b.x_dtype != a.y_dtype ||
+      b.gather_indx || b.x_scale || a.scatter_indx || a.betas || a.gammas || a.has_out_alpha || a.n_y_peers > 0)
+    return false;
+  if (!a.slice_sizes || a.slice_sizes != b.slice_sizes || a.slice_offs != b.slice_offs || a.block_offs_16 != b.block_offs_16 ||
+      a.block_sched_16 != b.block_sched_16)
+    return false;
+  const uint8_t *wa = (const uint8_t*)a.mx_workspace, *wb = (const uint8_t*)b.mx_workspace;
+  if (wa < wb + b.mx_workspace_bytes && wb < wa + a.mx_workspace_bytes) return false;
+  const bool bf16 = a.y_dtype == MOE_BF16;
+  if (bf16 && !(a.act_has_limit && a.act_limit > 0.0f && a.act_limit < 1e9f && a.act_alpha > 1e-9f)) return false;
+  if (!bf16 && a.y_dtype != MOE_F8E4M3) return false;
+  if ((uintptr_t)wb % 1024 != 0 || !(kb == K_MX_PAIR ? moe_gemm_mx_pair_token_out(b, out) : moe_gemm_mx_token_out(b, out))) return false;
+  // (a kernel has its own tokens' terms to write: the rules choose the same for both products but at the edges)
+  const int terms = ka == K_MX ? moe_gemm_mx_terms(a) : bf16 ? 2 : 1;
+  if (out.terms == terms && a.x_dtype == a.y_dtype) return true;
+  out = TokenOut();
+  return false;
+}
+
+extern "C" __attribute__((visibility("default"))) int moe_grouped_gemm_chain(const MoeGemmArgs* a, const MoeGemmArgs* b, void* stream) {
+  if (const int rc = check_args(a)) return rc;
+  if (const int rc = check_args(b)) return rc;
+  if (a->M == 0 || a->N == 0 || b->M == 0 || b->N == 0) {
+    const int rc = moe_grouped_gemm(a, stream);
+    return rc ? rc : moe_grouped_gemm(b, stream);
+  }
+  Kernel ka, kb;
+  if (const int rc = choose_kernel(*a, has_workspace(a), ka)) return rc;
+  if (const int rc = choose_kernel(*b, has_workspace(b), kb)) return rc;
+  TokenOut out;
+  const bool over = hands_over(*a, ka, *b, kb, out);
+  const int rc = run_product(a, ka, out, false, stream);
+  return rc ? rc : run_product(b, kb, TokenOut(), over, stream);
 }

@@ -23,6 +23,19 @@ struct GemmParams {
   void* y_peers[MOE_MAX_PEERS]; int n_y_peers; int64_t y_rows_per_peer;   // output rows spread over peer buffers
 };
 
+// Where a SwiGLU product leaves its rows instead of y: in the operand form of the product that follows (token_out.cuh)
+struct TokenOut {
+  uint8_t* q = nullptr; uint8_t* s = nullptr;   // values and scales of the first row at k step 0; NULL: rows go to y
+  int64_t q_step = 0, s_step = 0;               // bytes from a k step to the next
+  int64_t block_bytes = 0;                      // chunk form: bytes from a token block to the next
+  int lo_q = 0, lo_s = 0;                       // bytes from a term's line and scale to the next term's (scale: two terms only)
+  int terms = 0;                                // 1, 2: e4m3; 4: e2m1
+  int tb = 0;                                   // rows of a token block; 0: the pair kernel's lines
+  int permuted = 0;                             // k inside eight in the order of the default weight tiles
+  int KT = 0;                                   // k steps of 128
+  const int32_t* block_offs = nullptr;          // chunk form: first block of every expert
+};
+
 // first element of output row `dst`: in y, or in the peer buffer that holds that row
 template <typename TY> __device__ __forceinline__ TY* gemm_out_row(const GemmParams& p, int64_t dst) {
   if (p.n_y_peers == 0) return (TY*)p.y + dst * p.ld_y;

@@ -33,7 +33,7 @@
 //   scales -> tensor memory through registers (tcgen05.st by four loader warps), then MB x 4 MMAs of K = 32.
 // Warps: 0 producer, 1 MMA issue + tensor-memory owner, 2-5 epilogue, 6-9 scale loaders.  Every mbarrier
 // wait is bounded.
-#include "gemm_mx_common.cuh"
+#include "token_out.cuh"
 
 namespace {
 
@@ -48,6 +48,7 @@ constexpr int MX_SF_BASE = 512 - MX_MAX_STAGES * MX_SF_COLS;    // 384: accumula
 constexpr int MX_SMEM_LIMIT = 227 * 1024;
 constexpr int MX_CTL_BARS = 3 * MX_MAX_STAGES + 5;          // full, empty, scales-ready rings; 2 + 2 accumulator; drain
 constexpr int MX_CTL_BYTES = MX_CTL_BARS * 8 + 16;          // + tensor-memory base, abort flag
+constexpr int MX_TOK_BYTES = 2 * TOK_STAGE;                 // two stages of rows on their way to the next product's tokens
 
 struct MxParams {
   const uint8_t* xq;            // packed token chunks: [slot][k step][n_mma rows x 128 B | 1024 B scale area]
@@ -61,6 +62,7 @@ struct MxParams {
   int acc_bufs;
   int n_groups;                 // ceil(NB / MB)
   int64_t grid_m;               // static bound on token blocks (dense problems: exact)
+  TokenOut out;                 // the rows as the next product's tokens
 };
 
 struct MxMaps {
@@ -193,23 +195,6 @@ __global__ void __launch_bounds__(256) mx_pack_x_kernel(const GemmParams p, cons
 // Two values at a time by the conversion instructions (round to nearest, ties to the even code; |q| <= 6 but for Inf, which
 // saturates): with compares and selects per value, and a warp reduction under four masks, the pack of 64 tokens for 128 experts
 // took 13.6-14.4 us, so 10.5-11.1.
-__device__ __forceinline__ uint32_t f32x2_to_e2m1x2(float lo, float hi) {       // `lo` in bits 0..3
-  return (uint32_t)__nv_cvt_float2_to_fp4x2(make_float2(lo, hi), __NV_E2M1, cudaRoundNearest);
-}
-// e8m0 byte s with 2^(s-127) >= amax / 6, and the exact factors 2^(s-127), 2^(127-s)
-__device__ __forceinline__ void mx4_scale(float amax, uint32_t& sb, float& scale, float& inv) {
-  // amax / 6 rounded UP to a power of two; the product with a constant just above 1/6 is never below the quotient, so
-  // every value of the group still fits (it doubles the scale where amax is within an ulp of 6 * 2^e, which costs nothing
-  // that matters here) and the division is off the chain
-  const float ds = amax * 0.16666668f;
-  uint32_t u = (__float_as_uint(ds) + 0x007FFFFFu) & 0x7F800000u;
-  sb = u >> 23;
-  if (amax == 0.0f) sb = 127u;
-  sb = min(max(sb, 1u), 253u);
-  scale = __uint_as_float(sb << 23);
-  inv = __uint_as_float((254u - sb) << 23);
-}
-
 // (16 warps over the rows of eight k steps, for a third of the blocks: 2.6 x slower at 64 tokens, the blocks of 16 rows decide;
 // four warps instead of eight: 8 % slower.)  (A warp per (token block, k step, four rows) with the rows' chains side by side, and dead warps grouped into whole
 // CTAs, was tried in place of the loop over rows below: 2.3 x slower.  A row's four-term chain is latency, and four of
@@ -238,23 +223,12 @@ __global__ void __launch_bounds__(256) mx_pack_x4_kernel(const GemmParams p, con
     const bool nan[4] = {v[0] != v[0], v[1] != v[1], v[2] != v[2], v[3] != v[3]};      // e2m1 has no NaN: such a value counts as 0
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
-      // maximum of the 32-group over the 8 lanes that hold it (NaN ranks above Inf where all four values are NaN, and is caught below)
-      uint32_t top = __float_as_uint(fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))));
+      uint32_t codes;
+      const uint32_t sb = e2m1_term(t, v, nan, codes, [](uint32_t top) {       // over the 8 lanes that hold the group
 #pragma unroll
-      for (int o = 1; o <= 4; o <<= 1) top = max(top, __shfl_xor_sync(0xFFFFFFFFu, top, o));
-      float amax = __uint_as_float(top);
-      if (!(amax < 3.0e38f)) amax = t == 0 ? 3.0e38f : 0.0f;       // Inf / NaN in the group: keep the scales finite
-      uint32_t sb; float s, inv;
-      mx4_scale(amax, sb, s, inv);
-      uint32_t codes = 0;
-#pragma unroll
-      for (int i = 0; i < 4; i += 2) {
-        const uint32_t c = f32x2_to_e2m1x2(nan[i] ? 0.0f : v[i] * inv, nan[i + 1] ? 0.0f : v[i + 1] * inv);
-        codes |= c << (4 * i);
-        const float2 f = e2m1x2_to_f32x2(c);
-        v[i] -= f.x * s;
-        v[i + 1] -= f.y * s;
-      }
+        for (int o = 1; o <= 4; o <<= 1) top = max(top, __shfl_xor_sync(0xFFFFFFFFu, top, o));
+        return top;
+      });
       const int rt = t * a.tb + r;
       *reinterpret_cast<uint16_t*>(chunk + rt * 64 + ((g ^ (uint32_t)((rt >> 1) & 3)) << 4) + within) = (uint16_t)codes;
       if ((lane & 7) == 0) sc[(rt & 31) * 16 + (rt >> 5) * 4 + (int)g] = (uint8_t)sb;
@@ -300,6 +274,30 @@ __device__ __forceinline__ void mma_mx(uint32_t d_tmem, uint32_t a_lo, uint32_t 
         "@q tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale.scale_vec::1X [%0], da, db, %3, [%4], [%5], p;\n\t}" ::"r"(d_tmem),
         "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(sfa), "r"(sfb), "r"(accumulate), "n"(MX_DESC_HI_SW128)
         : "memory");
+}
+
+// sums of sixteen tokens over their terms, smallest first
+template <bool F4>
+__device__ __forceinline__ void mx_sums(uint32_t taddr, int split, int tb, uint32_t (&sum)[16]) {
+  uint32_t lo[16];
+  tmem_ld16(taddr, sum);
+  if (split > 1) tmem_ld16(taddr + (uint32_t)tb, lo);
+  tmem_ld_wait();
+  if constexpr (F4) {                                   // terms 2 and 3
+    uint32_t t2[16], t3[16];
+    tmem_ld16(taddr + 2u * (uint32_t)tb, t2);
+    tmem_ld16(taddr + 3u * (uint32_t)tb, t3);
+    tmem_ld_wait();
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      sum[j] = __float_as_uint(__uint_as_float(sum[j]) + __uint_as_float(t3[j]));
+      lo[j] = __float_as_uint(__uint_as_float(lo[j]) + __uint_as_float(t2[j]));
+    }
+  }
+  if (split > 1) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) sum[j] = __float_as_uint(__uint_as_float(sum[j]) + __uint_as_float(lo[j]));
+  }
 }
 
 // ============================================================================================================
@@ -547,6 +545,8 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
     // SwiGLU the even lane holds the gate and the odd lane the linear half of a pair.
     const int qd = warp & 3;
     const bool swiglu = p.activation == MOE_ACT_SWIGLU;
+    const int half = qd >> 1;
+    const TokStage tok{ctl0 + MX_CTL_BYTES + (uint32_t)(half * TOK_STAGE), 1 + half, (qd & 1) * 32 + lane};
     uint32_t tc = 0;
     bool ok = true;
     for (; ok && sched.next(pid_m, nb0, mb_live); ++tc) {
@@ -559,59 +559,69 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
         const int n = (nb0 + mb) * 128 + qd * 32 + lane;
         bias_n[mb] = (p.bias && n < p.N) ? load_bias(p.bias, p.bias_dtype, (int64_t)e * p.ld_bias + n) : 0.0f;
       }
+      int off = 0, first_block = 0;
+      if constexpr (TOK_TERMS<TY> != 0) {
+        off = p.slice_offs[e];
+        if (q.out.tb) first_block = q.out.block_offs[e];
+      }
       ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_ACC_FULL(ab), (tc / (uint32_t)q.acc_bufs) & 1u, ctl, 604));
+      if constexpr (TOK_TERMS<TY> != 0) ok = tok.all(ok);
       if (!ok) break;
       tc_fence_after();
       for (int c0 = 0; c0 < rows; c0 += 16) {
-        // parameters of token c0 + lane (lanes 0..15)
-        const int tj = c0 + (lane & 15);
-        TY* dst_l = nullptr;
-        float beta_l = 1.0f, gamma_l = 1.0f;
-        if (tj < rows) {
-          const int64_t m = row0 + tj;
-          const int64_t d = p.scatter_indx ? (int64_t)p.scatter_indx[m] : m;
-          if (d >= 0) dst_l = gemm_out_row<TY>(p, d);
-          if (p.betas) beta_l = p.betas[m];
-          if (p.gammas) gamma_l = p.gammas[m];
-        }
-        const int jmax = min(16, rows - c0);
+        if constexpr (TOK_TERMS<TY> != 0) {
+          uint8_t *tq = nullptr, *ts = nullptr;        // of token i >> 2 of the chunk
+          const int tr = c0 + (tok.i >> 2);
+          if (tr < rows) token_addr(q.out, e, off, first_block, (int)(row0 - off) + tr, tq, ts);
 #pragma unroll
-        for (int mb = 0; mb < NACC; ++mb) {
-          if (mb < mb_live) {
-            const int n = (nb0 + mb) * 128 + qd * 32 + lane;
-            const uint32_t taddr = tmem_base + ((uint32_t)(qd * 32) << 16) + ab * (uint32_t)acc_stride +
-                                   (uint32_t)(mb * q.n_mma + c0);
-            uint32_t hi[16], lo[16];
-            tmem_ld16(taddr, hi);
-            if (q.split > 1) tmem_ld16(taddr + (uint32_t)q.tb, lo);
-            tmem_ld_wait();
-            if constexpr (F4) {                                   // terms 2 and 3
-              uint32_t t2[16], t3[16];
-              tmem_ld16(taddr + 2u * (uint32_t)q.tb, t2);
-              tmem_ld16(taddr + 3u * (uint32_t)q.tb, t3);
-              tmem_ld_wait();
+          for (int mb = 0; mb < NACC; ++mb) {
+            if (mb < mb_live) {
+              const uint32_t taddr = tmem_base + ((uint32_t)(qd * 32) << 16) + ab * (uint32_t)acc_stride + (uint32_t)(mb * q.n_mma + c0);
+              uint32_t sum[16];
+              mx_sums<F4>(taddr, q.split, q.tb, sum);
+              float y[8];
+              swiglu_chunk(p, sum, bias_n[mb], lane & 1, y);
+              emit_tokens<TY>(q.out, tok, y, ((qd & 1) << 4) + (lane >> 1), lane & 1, 2 * (nb0 + mb) + half, tq, ts,
+                              nb0 + mb == NB - 1 && 2 * NB + half < 4 * q.out.KT);
+            }
+          }
+        } else {
+          // parameters of token c0 + lane (lanes 0..15)
+          const int tj = c0 + (lane & 15);
+          TY* dst_l = nullptr;
+          float beta_l = 1.0f, gamma_l = 1.0f;
+          if (tj < rows) {
+            const int64_t m = row0 + tj;
+            const int64_t d = p.scatter_indx ? (int64_t)p.scatter_indx[m] : m;
+            if (d >= 0) dst_l = gemm_out_row<TY>(p, d);
+            if (p.betas) beta_l = p.betas[m];
+            if (p.gammas) gamma_l = p.gammas[m];
+          }
+          const int jmax = min(16, rows - c0);
+#pragma unroll
+          for (int mb = 0; mb < NACC; ++mb) {
+            if (mb < mb_live) {
+              const int n = (nb0 + mb) * 128 + qd * 32 + lane;
+              const uint32_t taddr = tmem_base + ((uint32_t)(qd * 32) << 16) + ab * (uint32_t)acc_stride +
+                                     (uint32_t)(mb * q.n_mma + c0);
+              uint32_t sum[16];
+              mx_sums<F4>(taddr, q.split, q.tb, sum);
 #pragma unroll
               for (int j = 0; j < 16; ++j) {
-                hi[j] = __float_as_uint(__uint_as_float(hi[j]) + __uint_as_float(t3[j]));      // smallest terms first
-                lo[j] = __float_as_uint(__uint_as_float(lo[j]) + __uint_as_float(t2[j]));
-              }
-            }
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              if (j < jmax) {                                   // warp-uniform
-                TY* yrow = (TY*)__shfl_sync(0xFFFFFFFFu, (unsigned long long)dst_l, j);
-                const float beta = __shfl_sync(0xFFFFFFFFu, beta_l, j);
-                const float gamma = __shfl_sync(0xFFFFFFFFu, gamma_l, j);
-                float a = __uint_as_float(hi[j]);
-                if (q.split > 1) a += __uint_as_float(lo[j]);
-                a += bias_n[mb] * beta;
-                if (p.has_out_alpha) a *= p.out_alpha;
-                if (swiglu) {
-                  const float other = __shfl_xor_sync(0xFFFFFFFFu, a, 1);
-                  if (!(lane & 1) && yrow != nullptr && n + 1 < p.N)
-                    yrow[n >> 1] = from_f32<TY>(gemm_swiglu(a, other, p.act_alpha, p.act_limit, p.act_has_limit) * gamma);
-                } else if (yrow != nullptr && n < p.N) {
-                  yrow[n] = from_f32<TY>(a * gamma);
+                if (j < jmax) {                                   // warp-uniform
+                  TY* yrow = (TY*)__shfl_sync(0xFFFFFFFFu, (unsigned long long)dst_l, j);
+                  const float beta = __shfl_sync(0xFFFFFFFFu, beta_l, j);
+                  const float gamma = __shfl_sync(0xFFFFFFFFu, gamma_l, j);
+                  float a = __uint_as_float(sum[j]);
+                  a += bias_n[mb] * beta;
+                  if (p.has_out_alpha) a *= p.out_alpha;
+                  if (swiglu) {
+                    const float other = __shfl_xor_sync(0xFFFFFFFFu, a, 1);
+                    if (!(lane & 1) && yrow != nullptr && n + 1 < p.N)
+                      yrow[n >> 1] = from_f32<TY>(gemm_swiglu(a, other, p.act_alpha, p.act_limit, p.act_has_limit) * gamma);
+                  } else if (yrow != nullptr && n < p.N) {
+                    yrow[n] = from_f32<TY>(a * gamma);
+                  }
                 }
               }
             }
@@ -679,7 +689,7 @@ MxPlan mx_plan(const MoeGemmArgs& a) {
   pl.km = (pl.f4 && tb == 16 && pl.mb == 1 && a.tile_n == 0 && pl.KT >= 3) ? 1 : 0;
   pl.n_groups = (int)cdiv64(pl.NB, pl.mb);
   pl.chunk_bytes = (int64_t)pl.n_mma * (pl.f4 ? 64 : 128) + 1024;
-  const int ctl_bytes = MX_CTL_BYTES;
+  const int ctl_bytes = MX_CTL_BYTES + MX_TOK_BYTES;
   if (pl.km) {
     pl.mb = 3;                                       // tiles of a stage; n_groups stays the number of weight blocks
     pl.stage_bytes = 3 * MX_W_TILE_TX + 3 * (int)pl.chunk_bytes + 2048;
@@ -698,7 +708,7 @@ MxPlan mx_plan(const MoeGemmArgs& a) {
 
 template <typename TY, int MB, bool F4, bool KM = false>
 int launch_mx(const GemmParams& p, const MxParams& q, const MxPlan& pl, const MxMaps& w_map, int idle_sms, cudaStream_t st) {
-  const int smem = pl.stages * pl.stage_bytes + MX_CTL_BYTES + 1024;
+  const int smem = pl.stages * pl.stage_bytes + MX_CTL_BYTES + MX_TOK_BYTES + 1024;
   const int64_t items = pl.grid_m * pl.n_groups;
   int sms = moe_sm_count() - idle_sms;
   if (sms < 1) sms = 1;
@@ -709,11 +719,15 @@ int launch_mx(const GemmParams& p, const MxParams& q, const MxPlan& pl, const Mx
   return MOE_OK;
 }
 
+// TY: output rows, or the next product's tokens in the form this one's have
 template <typename TY>
 int launch_mx_ty(const GemmParams& p, const MxParams& q, const MxPlan& pl, const MxMaps& w_map, int idle_sms, cudaStream_t st) {
-  if (pl.km) return launch_mx<TY, 3, true, true>(p, q, pl, w_map, idle_sms, st);
-  if (pl.f4) return pl.mb == 3 ? launch_mx<TY, 3, true>(p, q, pl, w_map, idle_sms, st) : launch_mx<TY, 1, true>(p, q, pl, w_map, idle_sms, st);
-  return pl.mb == 3 ? launch_mx<TY, 3, false>(p, q, pl, w_map, idle_sms, st) : launch_mx<TY, 1, false>(p, q, pl, w_map, idle_sms, st);
+  if constexpr (TOK_TERMS<TY> == 0 || TOK_TERMS<TY> == 4) {
+    if (pl.km) return launch_mx<TY, 3, true, true>(p, q, pl, w_map, idle_sms, st);
+    if (pl.f4) return pl.mb == 3 ? launch_mx<TY, 3, true>(p, q, pl, w_map, idle_sms, st) : launch_mx<TY, 1, true>(p, q, pl, w_map, idle_sms, st);
+  }
+  if constexpr (TOK_TERMS<TY> == 4) return MOE_ERR_UNSUPPORTED;
+  else return pl.mb == 3 ? launch_mx<TY, 3, false>(p, q, pl, w_map, idle_sms, st) : launch_mx<TY, 1, false>(p, q, pl, w_map, idle_sms, st);
 }
 
 }  // namespace
@@ -743,7 +757,24 @@ extern "C" __attribute__((visibility("default"))) size_t moe_gemm_mx_workspace_b
   return a->w_kind == MOE_W_MX4_B200MX ? (size_t)mx_plan(*a).ws_bytes : 0;
 }
 
-int moe_gemm_mx_launch(const GemmParams& p_in, const MoeGemmArgs& a, cudaStream_t st) {
+int moe_gemm_mx_terms(const MoeGemmArgs& a) { return mx_plan(a).split; }
+
+bool moe_gemm_mx_token_out(const MoeGemmArgs& a, TokenOut& o) {
+  const MxPlan pl = mx_plan(a);
+  if (a.slice_sizes == nullptr || a.mx_workspace == nullptr || a.mx_workspace_bytes < pl.ws_bytes || (pl.split == 4 && pl.tb != 16)) return false;
+  const int row = pl.split == 4 ? 64 : 128;
+  int log2_tb = 4;
+  while ((1 << log2_tb) < pl.tb) ++log2_tb;
+  o.q = (uint8_t*)a.mx_workspace; o.s = o.q + (int64_t)pl.n_mma * row;
+  o.q_step = o.s_step = pl.chunk_bytes;
+  o.block_bytes = pl.KT * pl.chunk_bytes;
+  o.lo_q = pl.tb * row; o.lo_s = pl.tb == 16 ? 256 : pl.tb / 32 * 4;     // scale of row r: 16 (r % 32) + 4 (r / 32)
+  o.terms = pl.split; o.tb = pl.tb; o.KT = pl.KT;
+  o.block_offs = a.block_offs_16 + (log2_tb - 4) * a.ld_block_offs;
+  return true;
+}
+
+int moe_gemm_mx_launch(const GemmParams& p_in, const MoeGemmArgs& a, const TokenOut& out, bool packed, cudaStream_t st) {
   const MxPlan pl = mx_plan(a);
   if (pl.grid_m == 0) return MOE_OK;
   MOE_CHECK_ARG(a.mx_workspace != nullptr && a.mx_workspace_bytes >= pl.ws_bytes && (uintptr_t)a.mx_workspace % 1024 == 0,
@@ -766,12 +797,14 @@ int moe_gemm_mx_launch(const GemmParams& p_in, const MoeGemmArgs& a, cudaStream_
   pk.out = (uint8_t*)a.mx_workspace;
   const dim3 pgrid((unsigned)pl.grid_m, (unsigned)pl.KT);
   MOE_CHECK_ARG(pl.grid_m * pl.n_groups < 2147483647LL - 65536, "moe_grouped_gemm: too many token blocks");
-  if (pl.f4) MOE_CHECK_CUDA(launch_pdl(mx_pack_x4_kernel, pgrid, dim3(256), 0, st, p, pk));
-  else if (pl.split > 1) MOE_CHECK_CUDA(launch_pdl(mx_pack_x_kernel<true>, pgrid, dim3(256), 0, st, p, pk));
-  else MOE_CHECK_CUDA(launch_pdl(mx_pack_x_kernel<false>, pgrid, dim3(256), 0, st, p, pk));
-  MOE_CHECK_LAUNCH();
+  if (!packed) {
+    auto pack = pl.f4 ? mx_pack_x4_kernel : pl.split > 1 ? mx_pack_x_kernel<true> : mx_pack_x_kernel<false>;
+    MOE_CHECK_CUDA(launch_pdl(pack, pgrid, dim3(256), 0, st, p, pk));
+    MOE_CHECK_LAUNCH();
+  }
 
   MxParams q;
+  q.out = out;
   q.xq = (const uint8_t*)a.mx_workspace; q.chunk_bytes = pl.chunk_bytes;
   q.n_mma = pl.n_mma; q.tb = pl.tb; q.split = pl.split;
   q.KT = pl.KT; q.NB = pl.NB; q.stages = pl.stages; q.stage_bytes = pl.stage_bytes; q.acc_bufs = pl.acc_bufs;
@@ -780,6 +813,10 @@ int moe_gemm_mx_launch(const GemmParams& p_in, const MoeGemmArgs& a, cudaStream_
   for (int nb = 1; nb <= 3; ++nb)
     if (int rc = make_w_map(a, pl.KT, pl.NB, pl.f4 != 0, nb <= pl.mb ? nb : pl.mb, &w_map.m[nb - 1])) return rc;
   const int idle = a.idle_sms > 0 ? a.idle_sms : 0;
+  if (out.q) {
+    if (out.terms == 4) return launch_mx_ty<Tok4>(p, q, pl, w_map, idle, st);
+    return out.terms == 2 ? launch_mx_ty<Tok2>(p, q, pl, w_map, idle, st) : launch_mx_ty<Tok1>(p, q, pl, w_map, idle, st);
+  }
   if (a.y_dtype == MOE_F8E4M3) return launch_mx_ty<__nv_fp8_e4m3>(p, q, pl, w_map, idle, st);
   if (a.y_dtype == MOE_BF16) return launch_mx_ty<__nv_bfloat16>(p, q, pl, w_map, idle, st);
   return launch_mx_ty<float>(p, q, pl, w_map, idle, st);

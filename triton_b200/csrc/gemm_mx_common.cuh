@@ -38,6 +38,46 @@ __device__ __forceinline__ void mx8_scale(float amax, uint32_t& sb, float& scale
   inv = __uint_as_float((254u - sb) << 23);
 }
 
+__device__ __forceinline__ uint32_t f32x2_to_e2m1x2(float lo, float hi) {       // `lo` in bits 0..3
+  return (uint32_t)__nv_cvt_float2_to_fp4x2(make_float2(lo, hi), __NV_E2M1, cudaRoundNearest);
+}
+// e8m0 byte s with 2^(s-127) >= amax / 6, and the exact factors 2^(s-127), 2^(127-s)
+__device__ __forceinline__ void mx4_scale(float amax, uint32_t& sb, float& scale, float& inv) {
+  // amax / 6 rounded UP to a power of two; the product with a constant just above 1/6 is never below the quotient, so
+  // every value of the group still fits (it doubles the scale where amax is within an ulp of 6 * 2^e, which costs nothing
+  // that matters here) and the division is off the chain
+  const float ds = amax * 0.16666668f;
+  uint32_t u = (__float_as_uint(ds) + 0x007FFFFFu) & 0x7F800000u;
+  sb = u >> 23;
+  if (amax == 0.0f) sb = 127u;
+  sb = min(max(sb, 1u), 253u);
+  scale = __uint_as_float(sb << 23);
+  inv = __uint_as_float((254u - sb) << 23);
+}
+// Term t of N values of a 32-group (v: what the terms before left over, and leaves); its maximum comes from `all`.  -> scale byte
+template <int N, typename F>
+__device__ __forceinline__ uint32_t e2m1_term(int t, float (&v)[N], const bool (&nan)[N], uint32_t& codes, F all) {
+  // (NaN ranks above Inf where four neighbouring values are NaN, and is caught below)
+  uint32_t top = 0;
+#pragma unroll
+  for (int i = 0; i < N; i += 4)
+    top = max(top, __float_as_uint(fmaxf(fmaxf(fabsf(v[i]), fabsf(v[i + 1])), fmaxf(fabsf(v[i + 2]), fabsf(v[i + 3])))));
+  float amax = __uint_as_float(all(top));
+  if (!(amax < 3.0e38f)) amax = t == 0 ? 3.0e38f : 0.0f;           // Inf / NaN in the group: keep the scales finite
+  uint32_t sb; float s, inv;
+  mx4_scale(amax, sb, s, inv);
+  codes = 0;
+#pragma unroll
+  for (int i = 0; i < N; i += 2) {
+    const uint32_t c = f32x2_to_e2m1x2(nan[i] ? 0.0f : v[i] * inv, nan[i + 1] ? 0.0f : v[i + 1] * inv);
+    codes |= c << (4 * i);
+    const float2 f = e2m1x2_to_f32x2(c);
+    v[i] -= f.x * s;
+    v[i + 1] -= f.y * s;
+  }
+  return sb;
+}
+
 // cuTensorMapEncodeTiled with the defaults of these kernels
 inline int encode_map(CUtensorMap* map, CUtensorMapDataType type, int rank, const void* base, const cuuint64_t* dims, const cuuint64_t* strides,
                       const cuuint32_t* box, CUtensorMapSwizzle swizzle, const char* what) {

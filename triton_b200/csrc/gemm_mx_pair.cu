@@ -33,8 +33,8 @@
 // Warps of a CTA: 0 producer, 1 and 2 MMA issue (even CTA; 1 owns tensor memory), 4-7 scale loaders (shared memory ->
 // registers -> tensor memory; the token scales of all columns in both CTAs, the weight scales of the own rows), 8-19 epilogue.
 // Every wait is bounded; both CTAs meet at a cluster barrier before tensor memory is freed.
-#include "gemm_mx_common.cuh"
 #include "gemm_pair_common.cuh"
+#include "token_out.cuh"
 
 namespace {
 
@@ -49,7 +49,9 @@ constexpr int PP_MAX_STAGES = 6, PP_MAX_REGIONS = 12;
 constexpr int PP_NUM_BARS = 3 * PP_MAX_STAGES + 2 * PP_MAX_REGIONS + 1;
 // shared memory behind the stages: [token tables x 2][barriers][tensor-memory base, abort flag][columns of the next tiles][prefix]
 constexpr int PP_OFF_BAR = 2 * PAIR_TAB, PP_OFF_MISC = PP_OFF_BAR + (PP_NUM_BARS * 8 + 15) / 16 * 16, PP_OFF_COLS = PP_OFF_MISC + 16,
-              PP_OFF_PREFIX = PP_OFF_COLS + 8 * 4, PP_CTL = (PP_OFF_PREFIX + PAIR_PREFIX_INTS * 4 + 15) / 16 * 16;
+              PP_OFF_PREFIX = PP_OFF_COLS + 8 * 4, PP_CTL_BASE = (PP_OFF_PREFIX + PAIR_PREFIX_INTS * 4 + 15) / 16 * 16;
+// ... and where the rows become the next product's tokens, a stage per two epilogue warps
+template <typename TY> constexpr int PP_CTL = PP_CTL_BASE + (TOK_TERMS<TY> ? PP_EPI_WARPS / 2 * TOK_STAGE : 0);
 constexpr int PP_SMEM = 227 * 1024;
 // How tokens enter the MMA.  ONE: e4m3 rows, one term.  TWO: two terms, two MMAs into the same columns.  SIDE: the terms as
 // neighbouring columns of one MMA (eight hi, eight lo, ...), added in the epilogue.  An MMA takes 45-59 cycles however few
@@ -68,6 +70,7 @@ struct PairParams {
   int nmax;                     // token columns of a tile at most, a multiple of 32
   int upt;                      // weight blocks of 256 rows per tile: 1 or 2
   int stages, stage_bytes, regions, reg_cols;      // accumulator regions of reg_cols tensor-memory columns
+  TokenOut out;
 };
 
 struct PairMaps { CUtensorMap w[2], s[2]; };        // weight tiles and their scales in boxes of one and two blocks
@@ -76,9 +79,6 @@ struct PairMaps { CUtensorMap w[2], s[2]; };        // weight tiles and their sc
 template <int TERMS> __device__ __forceinline__ int64_t token_line(int64_t kt, int64_t prows, int64_t prow, int term) {
   return TERMS * (kt * prows + (prow & ~(int64_t)7)) + term * 8 + (prow & 7);
 }
-
-// first padded row of an expert: a multiple of 32, and never before the end of the previous expert's last group of 32
-__device__ __forceinline__ int64_t padded_base(int e, int off) { return (int64_t)(off & ~31) + 32 * (int64_t)e; }
 
 // ============================================================================================================
 // Pack kernel.  A block takes up to 16 rows of one expert (an entry of the 16-row block schedule).  bf16: a thread a group of
@@ -93,6 +93,7 @@ struct PairPackParams {
   int64_t prows;
   uint8_t* xq; uint8_t* xs;
   uint32_t* done;
+  TokenOut out;                  // the product's rows are the next one's tokens: those computed here go there too
 };
 
 __device__ __forceinline__ bool pack_block(const GemmParams& p, int64_t pid, int& e, int64_t& row0, int& rows, int64_t& prow0) {
@@ -114,6 +115,34 @@ __device__ __forceinline__ bool pack_block(const GemmParams& p, int64_t pid, int
   prow0 = padded_base(e, off) + first;
   rows = min(16, p.slice_sizes[e] - first);
   return rows > 0;
+}
+
+// One 32-group of a bf16 row as two terms; q, s: the row's line and scales at the group's k step.  -> the group's maximum
+// PERMUTED: k inside eight in the order of the default weight tiles (0, 2, 4, 6, 1, 3, 5, 7)
+template <bool PERMUTED>
+__device__ __forceinline__ float pack_group2(const uint4 (&raw)[4], int x7, int g, uint8_t* q, int lo_q, uint8_t* s, int lo_s) {
+  float v[32];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t w[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      v[8 * i + (PERMUTED ? j : 2 * j)] = __uint_as_float(w[j] << 16);
+      v[8 * i + (PERMUTED ? 4 + j : 2 * j + 1)] = __uint_as_float(w[j] & 0xFFFF0000u);
+    }
+  }
+  uint32_t h[8], l[8], sh, sl;
+  float m;
+  two_terms<32>(v, [](float own) { return own; }, h, l, sh, sl, m);
+  const uint32_t odd = (uint32_t)x7 & 1u;                          // 16-byte pieces 2 g and 2 g + 1 of the line, xor x7
+  uint8_t* dst = q + ((((uint32_t)(g & 3) << 1) ^ ((uint32_t)x7 & 6u)) << 4);
+  const uint4 h0 = make_uint4(h[0], h[1], h[2], h[3]), h1 = make_uint4(h[4], h[5], h[6], h[7]);
+  const uint4 l0 = make_uint4(l[0], l[1], l[2], l[3]), l1 = make_uint4(l[4], l[5], l[6], l[7]);
+  st_v8(dst, odd ? h1 : h0, odd ? h0 : h1);
+  st_v8(dst + lo_q, odd ? l1 : l0, odd ? l0 : l1);
+  s[g & 3] = (uint8_t)sh;
+  s[lo_s + (g & 3)] = (uint8_t)sl;
+  return m;
 }
 
 // Magnitude from which on two e4m3 terms do not hold a token's value: infinities, and finite values that round to 2^128.
@@ -203,6 +232,19 @@ __device__ __noinline__ uint32_t exact_rows(const GemmParams& p, const PairPackP
     else if (a.y_dtype == MOE_F32) exact_row<float, TILED>(p, a, e, m, d, x, groups);
     else exact_row<__nv_fp8_e4m3, TILED>(p, a, e, m, d, x, groups);
     __syncthreads();
+    if (a.out.q) {
+      const uint4* y = reinterpret_cast<const uint4*>((const __nv_bfloat16*)p.y + d * p.ld_y);
+      uint8_t *q, *s;
+      const int off = p.slice_offs[e], rr = (int)(m - off);
+      token_addr(a.out, e, off, a.out.tb ? a.out.block_offs[e] : 0, rr, q, s);
+      for (int g = threadIdx.x; g < 4 * a.out.KT; g += 256) {
+        uint4 raw[4] = {};
+        if (g < p.N >> 6)
+          for (int i = 0; i < 4; ++i) raw[i] = y[g * 4 + i];
+        if (a.out.permuted) pack_group2<true>(raw, rr & 7, g, q + (g >> 2) * a.out.q_step, a.out.lo_q, s + (g >> 2) * a.out.s_step, a.out.lo_s);
+        else pack_group2<false>(raw, rr & 7, g, q + (g >> 2) * a.out.q_step, a.out.lo_q, s + (g >> 2) * a.out.s_step, a.out.lo_s);
+      }
+    }
   }
   return all;
 }
@@ -227,49 +269,9 @@ __global__ void __launch_bounds__(256) mx_pair_pack2_kernel(const __grid_constan
 #pragma unroll
       for (int i = 0; i < 4; ++i) raw[i] = x[i];
     }
-    float v[32];
-    float m = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const uint32_t w[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float lo = __uint_as_float(w[j] << 16), hi = __uint_as_float(w[j] & 0xFFFF0000u);
-        v[8 * i + (TILED ? j : 2 * j)] = lo;
-        v[8 * i + (TILED ? 4 + j : 2 * j + 1)] = hi;
-        m = fmaxf(m, fmaxf(fabsf(lo), fabsf(hi)));
-      }
-    }
-    beyond |= !(m < BEYOND);                           // (what is packed of such a row is not used; a NaN makes its results NaN)
-    uint32_t sh; float s_hi, i_hi;
-    mx8_scale(m, sh, s_hi, i_hi);
-    uint32_t h[8], l[8];
-    float rm = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const uint32_t c = f32x2_to_e4m3x2(v[2 * i] * i_hi, v[2 * i + 1] * i_hi);
-      const float2 f = e4m3x2_to_f32x2(c);
-      v[2 * i] -= f.x * s_hi;
-      v[2 * i + 1] -= f.y * s_hi;
-      rm = fmaxf(rm, fmaxf(fabsf(v[2 * i]), fabsf(v[2 * i + 1])));
-      h[i >> 1] = (i & 1) ? (h[i >> 1] | (c << 16)) : c;
-    }
-    if (!(rm < 3.0e38f)) rm = 0.0f;
-    uint32_t sl; float s_lo, i_lo;
-    mx8_scale(rm, sl, s_lo, i_lo);
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-      l[i] = f32x2_to_e4m3x2(v[4 * i] * i_lo, v[4 * i + 1] * i_lo) | (f32x2_to_e4m3x2(v[4 * i + 2] * i_lo, v[4 * i + 3] * i_lo) << 16);
     const int64_t prow = prow0 + r, line = token_line<2>(g >> 2, a.prows, prow, 0);
-    const uint32_t x7 = (uint32_t)prow & 7u, odd = x7 & 1u;       // 16-byte pieces 2 g and 2 g + 1 of the line, xor x7
-    uint8_t* dst = a.xq + line * 128 + ((((uint32_t)(g & 3) << 1) ^ (x7 & 6u)) << 4);
-    const uint4 h0 = make_uint4(h[0], h[1], h[2], h[3]), h1 = make_uint4(h[4], h[5], h[6], h[7]);
-    const uint4 l0 = make_uint4(l[0], l[1], l[2], l[3]), l1 = make_uint4(l[4], l[5], l[6], l[7]);
-    st_v8(dst, odd ? h1 : h0, odd ? h0 : h1);
-    st_v8(dst + 1024, odd ? l1 : l0, odd ? l0 : l1);
-    uint8_t* sd = a.xs + line * 4 + (g & 3);
-    sd[0] = (uint8_t)sh;
-    sd[32] = (uint8_t)sl;
+    const float m = pack_group2<TILED>(raw, (int)prow & 7, g, a.xq + line * 128, 1024, a.xs + line * 4, 32);
+    beyond |= !(m < BEYOND);                           // (what is packed of such a row is not used; a NaN makes its results NaN)
   }
   uint32_t done = 0;
   if (__syncthreads_or(beyond)) done = exact_rows<TILED>(p, a, e, row0, rows);
@@ -594,6 +596,23 @@ gemm_mx_pair_kernel(const GemmParams p, const PairParams a, const __grid_constan
     const bool vec = p.ld_y % 2 == 0 && (uintptr_t)p.y % (2 * sizeof(TY)) == 0;
     uint32_t tc = 0;
     uint32_t acc_ph = 0, reg = 0;                      // parity to wait for, per region; region of the next block
+    // (two warps to a group of 32 outputs, see emit_tokens)
+    const int half = qd >> 1, tok_pair = grp * 2 + half;
+    const TokStage tok{ctl0 + PP_CTL_BASE + (uint32_t)(tok_pair * TOK_STAGE), 2 + tok_pair, (qd & 1) * 32 + lane};
+    // 16 tokens of block b, from the raw sums
+    auto emit = [&](const PairOut& out, const uint32_t (&sums)[16], uint32_t tab, int c, int block) {
+      if constexpr (TOK_TERMS<TY> != 0) {
+        if (block >= NB) return;                       // (both warps of the pair)
+        float y[8];
+        swiglu_chunk(p, sums, out.bias, odd, y);
+        const uint32_t at = tab + (uint32_t)(c + (tok.i >> 2)) * 8u;
+        const uint2 q = lds64(at), s = lds64(at + 2048u);
+        emit_tokens<TY>(a.out, tok, y, ((qd & 1) << 4) + (own >> 1), odd, 2 * block + half, (uint8_t*)(((uint64_t)q.y << 32) | q.x),
+                        (uint8_t*)(((uint64_t)s.y << 32) | s.x), block == NB - 1 && 2 * NB + half < 4 * a.out.KT);
+      } else {
+        pair_emit<TY>(p, out, sums, tab, c);
+      }
+    };
     bool ok = true;
     for (int tile = pair; tile < n_tiles && ok; tile += n_pairs, ++tc) {
       const PTile t = map_ptile(p, s_prefix, tile / MT);
@@ -601,8 +620,15 @@ gemm_mx_pair_kernel(const GemmParams p, const PairParams a, const __grid_constan
       const uint32_t tab = ctl0 + (tc & 1u) * PAIR_TAB;
       if (tid < t.cols) {
         bool stored = tid < t.rows;                    // not by the pack kernel
-        if (TERMS == 2 && stored) stored = !((a.done[(padded_base(t.e, t.off) + t.first + tid) >> 4] >> (tid & 15)) & 1u);
-        pair_table_entry<TY>(p, t, tid, stored, tab);
+        if (TERMS == 2 && stored && a.done) stored = !((a.done[(padded_base(t.e, t.off) + t.first + tid) >> 4] >> (tid & 15)) & 1u);
+        if constexpr (TOK_TERMS<TY> != 0) {            // line and scales of the row as the next product's token, in place of row and weights
+          uint8_t *q = nullptr, *s = nullptr;
+          if (stored) token_addr(a.out, t.e, t.off, a.out.tb ? a.out.block_offs[t.e] : 0, t.first + tid, q, s);
+          asm volatile("st.shared.u64 [%0], %1;" ::"r"(tab + (uint32_t)tid * 8u), "l"(q) : "memory");
+          asm volatile("st.shared.u64 [%0], %1;" ::"r"(tab + 2048u + (uint32_t)tid * 8u), "l"(s) : "memory");
+        } else {
+          pair_table_entry<TY>(p, t, tid, stored, tab);
+        }
       }
       float bias_m[2];
 #pragma unroll
@@ -617,6 +643,7 @@ gemm_mx_pair_kernel(const GemmParams p, const PairParams a, const __grid_constan
         const bool first = ne < p.N, both = ne + 1 < p.N;
         const PairOut out{ne, first, both, __all_sync(0xFFFFFFFFu, both && (swiglu || vec)) != 0, odd, sel, u ? bias_m[1] : bias_m[0]};
         ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_ACC_FULL(reg), (acc_ph >> reg) & 1u, ctl, 616));
+        if constexpr (TOK_TERMS<TY> != 0) ok = tok.all(ok);
         if (!ok) break;
         acc_ph ^= 1u << reg;
         tc_fence_after();
@@ -652,9 +679,9 @@ gemm_mx_pair_kernel(const GemmParams p, const PairParams a, const __grid_constan
                   const int at = (j >> 3) * 16 + (j & 7);
                   v[j] = __float_as_uint(__uint_as_float(raw[i][at]) + __uint_as_float(raw[i][at + 8]));
                 }
-                pair_emit<TY>(p, out, v, tab, c0 + STEP * i);
+                emit(out, v, tab, c0 + STEP * i, b.first + u);
               } else {
-                pair_emit<TY>(p, out, raw[i], tab, c0 + STEP * i);
+                emit(out, raw[i], tab, c0 + STEP * i, b.first + u);
               }
             }
         }
@@ -725,7 +752,7 @@ int launch_mx_pair(const GemmParams& p, PairParams q, const PairShape& shape, co
   q.nmax = shape.nmax; q.upt = shape.upt;
   q.reg_cols = q.nmax * (FORM == PP_SIDE ? 2 : 1);
   q.stage_bytes = q.upt * 128 * 128 + TERMS_OF<FORM> * (q.nmax * 64 + 1024) + 1024;
-  q.stages = (PP_SMEM - 1024 - PP_CTL) / q.stage_bytes;
+  q.stages = (PP_SMEM - 1024 - PP_CTL<TY>) / q.stage_bytes;
   if (q.stages > PP_MAX_STAGES) q.stages = PP_MAX_STAGES;
   while ((TMEM_COLS - q.stages * SF_COLS<FORM>) / q.reg_cols < 2) --q.stages;
   if (q.stages > q.KT) q.stages = q.KT;               // see the MMA warps
@@ -778,6 +805,7 @@ int launch_mx_pair(const GemmParams& p, PairParams q, const PairShape& shape, co
   return MOE_OK;
 }
 
+// TY: output rows, or the next product's tokens
 template <typename TY>
 int launch_mx_pair_ty(const GemmParams& p, const PairParams& q, const MoeGemmArgs& a, const PairMaps& m, cudaStream_t st) {
   const PairShape shape = pair_shape(a, a.x_dtype == MOE_BF16 ? 2 : 1);
@@ -785,9 +813,13 @@ int launch_mx_pair_ty(const GemmParams& p, const PairParams& q, const MoeGemmArg
     if (a.w_kind == MOE_W_MX4_B200)
       return shape.form == PP_SIDE ? launch_mx_pair<TY, PP_SIDE, true>(p, q, shape, a, m, st) : launch_mx_pair<TY, PP_TWO, true>(p, q, shape, a, m, st);
   }
-  if (shape.form == PP_SIDE) return launch_mx_pair<TY, PP_SIDE, false>(p, q, shape, a, m, st);
-  if (shape.form == PP_TWO) return launch_mx_pair<TY, PP_TWO, false>(p, q, shape, a, m, st);
-  return launch_mx_pair<TY, PP_ONE, false>(p, q, shape, a, m, st);
+  // (a product hands its rows on in the form its own tokens have)
+  if constexpr (TOK_TERMS<TY> != 1) {
+    if (shape.form == PP_SIDE) return launch_mx_pair<TY, PP_SIDE, false>(p, q, shape, a, m, st);
+    if (shape.form == PP_TWO) return launch_mx_pair<TY, PP_TWO, false>(p, q, shape, a, m, st);
+  }
+  if constexpr (TOK_TERMS<TY> != 2) return launch_mx_pair<TY, PP_ONE, false>(p, q, shape, a, m, st);
+  return MOE_ERR_UNSUPPORTED;
 }
 
 }  // namespace
@@ -838,7 +870,17 @@ bool moe_gemm_mx_pair_wanted(const MoeGemmArgs& a) {
 
 int64_t moe_gemm_mx_pair_workspace(const MoeGemmArgs& a) { return pair_plan(a).ws_bytes; }
 
-int moe_gemm_mx_pair_launch(const GemmParams& p_in, const MoeGemmArgs& a, cudaStream_t st) {
+bool moe_gemm_mx_pair_token_out(const MoeGemmArgs& a, TokenOut& o) {
+  const PairPlan pl = pair_plan(a);
+  if (a.mx_workspace == nullptr || a.mx_workspace_bytes < pl.ws_bytes) return false;
+  o.q = (uint8_t*)a.mx_workspace; o.s = o.q + pl.xs_off;
+  o.q_step = pl.terms * pl.prows * 128; o.s_step = pl.terms * pl.prows * 4;
+  o.lo_q = 1024; o.lo_s = 32;
+  o.terms = pl.terms; o.permuted = a.w_kind == MOE_W_MX4_B200; o.KT = pl.KT;
+  return true;
+}
+
+int moe_gemm_mx_pair_launch(const GemmParams& p_in, const MoeGemmArgs& a, const TokenOut& out, bool packed, cudaStream_t st) {
   const PairPlan pl = pair_plan(a);
   MOE_CHECK_ARG(a.mx_workspace != nullptr && a.mx_workspace_bytes >= pl.ws_bytes && (uintptr_t)a.mx_workspace % 1024 == 0,
                 "moe_grouped_gemm: the block-scaled kernel needs mx_workspace of moe_gemm_mx_workspace_bytes() = %lld "
@@ -859,11 +901,15 @@ int moe_gemm_mx_pair_launch(const GemmParams& p_in, const MoeGemmArgs& a, cudaSt
   pk.K = a.K; pk.KT = pl.KT; pk.NB = pl.NB; pk.y_dtype = a.y_dtype; pk.prows = pl.prows;
   pk.xq = (uint8_t*)a.mx_workspace; pk.xs = pk.xq + pl.xs_off; pk.done = (uint32_t*)(pk.xq + pl.done_off);
   const bool tiled = a.w_kind == MOE_W_MX4_B200;
-  auto pack = pl.terms == 1 ? mx_pair_pack1_kernel : tiled ? mx_pair_pack2_kernel<true> : mx_pair_pack2_kernel<false>;
-  MOE_CHECK_CUDA(launch_pdl(pack, dim3((unsigned)blocks16), dim3(256), 0, st, p, pk));
-  MOE_CHECK_LAUNCH();
+  pk.out = out;
+  if (!packed) {
+    auto pack = pl.terms == 1 ? mx_pair_pack1_kernel : tiled ? mx_pair_pack2_kernel<true> : mx_pair_pack2_kernel<false>;
+    MOE_CHECK_CUDA(launch_pdl(pack, dim3((unsigned)blocks16), dim3(256), 0, st, p, pk));
+    MOE_CHECK_LAUNCH();
+  }
   PairParams q;
-  q.xq = pk.xq; q.xs = pk.xs; q.done = pk.done; q.prows = pl.prows; q.KT = pl.KT; q.NB = pl.NB;
+  q.out = out;
+  q.xq = pk.xq; q.xs = pk.xs; q.done = packed ? nullptr : pk.done; q.prows = pl.prows; q.KT = pl.KT; q.NB = pl.NB;
   PairMaps maps;
   for (int n = 1; n <= 2; ++n) {
     // values as the TMA unit expands them (a row of a box: 64 bytes -> 128), scales as words; blocks along the slowest dimension
@@ -880,6 +926,7 @@ int moe_gemm_mx_pair_launch(const GemmParams& p_in, const MoeGemmArgs& a, cudaSt
     if (int rc = encode_map(&maps.s[n - 1], CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, a.w_scale, sd, sst, sb, CU_TENSOR_MAP_SWIZZLE_NONE, "weight scales"))
       return rc;
   }
+  if (out.q) return out.terms == 1 ? launch_mx_pair_ty<Tok1>(p, q, a, maps, st) : launch_mx_pair_ty<Tok2>(p, q, a, maps, st);
   if (a.y_dtype == MOE_BF16) return launch_mx_pair_ty<__nv_bfloat16>(p, q, a, maps, st);
   if (a.y_dtype == MOE_F32) return launch_mx_pair_ty<float>(p, q, a, maps, st);
   MOE_CHECK_ARG(!tiled, "moe_grouped_gemm: e4m3 output needs weights in the block-scaled layout");

@@ -18,7 +18,7 @@ struct Lib {
   X(moe_last_error) X(moe_route) X(moe_route_positions) X(moe_route_workspace) X(moe_grouped_gemm) X(moe_gemm_mx_workspace_bytes) \
   X(moe_reduce) X(moe_downcast_mxfp4) X(moe_upcast_mxfp4) X(moe_bitmatrix_metadata) X(moe_bitmatrix_metadata_workspace) \
   X(moe_router_topk) X(moe_router_topk_workspace_bytes) X(moe_copy2) \
-  X(moe_gemm_kernel_name)
+  X(moe_gemm_kernel_name) X(moe_grouped_gemm_chain)
 #define X(name) decltype(&::name) name = nullptr;
   MOE_HOST_FUNCTIONS(X)
 #undef X
@@ -275,7 +275,8 @@ void set_product(MoeGemmArgs& g, const py::tuple& w, int64_t E, int64_t n, const
 }
 
 // routing -> fc1 (+ bias, SwiGLU) -> fc2 (+ bias, x routing weight) -> sum over the k slots.  Every temporary is a part of one
-// buffer: two allocations per step, and the temporaries of both products share theirs.
+// buffer: two allocations per step.  fc1's temporary is over when fc2's output begins and shares its place; fc2's is apart, since fc1 may
+// write its rows there.
 Tensor layer(const Tensor& x, const Tensor& logits, int64_t k, const py::tuple& w1, const py::tuple& w2, double alpha,
              std::optional<double> limit, const py::tuple& tuning, const Tensor& status) {
   need_cuda(x); need_cuda(logits);
@@ -299,7 +300,7 @@ Tensor layer(const Tensor& x, const Tensor& logits, int64_t k, const py::tuple& 
   Carver c;
   const int64_t o_vals = c.take(n * 4), o_indx = c.take(n * 2), o_bm = c.take(words * t_pad * 4), o_sum = c.take(E * 4), o_col = c.take(n * 4),
                 o_row = c.take(n * 4), o_offs = c.take(5 * lo * 4), o_sched = c.take(4 * ls * 4), o_rws = c.take(route_ws), o_tok = c.take(n * 4),
-                o_gam = c.take(n * 4), o_h = c.take(n * ff * h_size), o_y = c.take(n * d * 2), o_tmp = c.take(std::max(t1, t2));
+                o_gam = c.take(n * 4), o_h = c.take(n * ff * h_size), o_y = c.take(std::max(n * d * 2, t1)), o_tmp = c.take(t2);
   Tensor buf = empty({c.bytes + 1024}, at::kByte, x), z = empty({T, d}, at::kBFloat16, x);
   uint8_t* base = (uint8_t*)(((uintptr_t)buf.data_ptr() + 1023) / 1024 * 1024);
   void* st = stream();
@@ -315,16 +316,15 @@ Tensor layer(const Tensor& x, const Tensor& logits, int64_t k, const py::tuple& 
     g->block_offs_16 = offs + lo; g->block_sched_16 = sched;
     g->ld_block_offs = lo; g->ld_block_sched = ls;
   }
-  set_temp(g1, base + o_tmp, t1, ws1);
+  set_temp(g1, base + o_y, t1, ws1);
   set_temp(g2, base + o_tmp, t2, ws2);
   g1.gather_indx = (int32_t*)(base + o_tok);
   if (limit) { g1.act_limit = (float)*limit; g1.act_has_limit = 1; }
   g1.y = base + o_h; g1.ld_y = ff;
-  check(lib.moe_grouped_gemm(&g1, st), "moe_grouped_gemm", true);
   g2.x = base + o_h; g2.rows_x = n;
   g2.scatter_indx = (int32_t*)(base + o_col); g2.gammas = (float*)(base + o_gam);
   g2.y = base + o_y; g2.ld_y = d;
-  check(lib.moe_grouped_gemm(&g2, st), "moe_grouped_gemm", true);
+  check(lib.moe_grouped_gemm_chain(&g1, &g2, st), "moe_grouped_gemm", true);
   check(lib.moe_reduce(base + o_y, MOE_BF16, k, T, d, d, k * d, 1, nullptr, 0, 0, 0, 0, nullptr, 0, 0, 0, z.data_ptr(), MOE_BF16, d, 1, st),
         "moe_reduce");
   return z;

@@ -102,102 +102,114 @@ __device__ __forceinline__ uint2 lds64(uint32_t a) {
   return v;
 }
 
-// y: outputs of tokens 8 odd .. + 7 in column `col` (0 .. 31) of group g; q, s: lines of token i >> 2 of the chunk at k step 0 (q
-// NULL: not stored).  zero_next: group g + 2 is past the last weight block, and zero.
-template <typename TY>
-__device__ __forceinline__ void emit_tokens(const TokenOut& o, const TokStage& st, const float (&y)[8], int col, int odd, int g, uint8_t* q,
-                                            uint8_t* s, bool zero_next) {
+// y[u]: outputs of tokens 8 odd .. + 7 in column `col` (0 .. 31) of group g + 2 u, for `live` of the U neighbouring weight blocks (a
+// stage each, their chains side by side); q, s: lines of token i >> 2 of the chunk at k step 0 (q NULL: not stored).  zero_next: the
+// group two past the last block's is past K too, and zero.
+template <typename TY, int U>
+__device__ __forceinline__ void emit_tokens(const TokenOut& o, const TokStage& st, const float (&y)[U][8], int live, int col, int odd, int g,
+                                            uint8_t* q, uint8_t* s, bool zero_next) {
   constexpr int TERMS = TOK_TERMS<TY>;
   const uint32_t w = st.at + (uint32_t)(odd * 8 * TOK_PITCH + col * (TERMS == 1 ? 1 : 2));
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    if constexpr (TERMS == 1) {
-      asm volatile("st.shared.u8 [%0], %1;" ::"r"(w + (uint32_t)(j * TOK_PITCH)), "r"((uint32_t)from_f32<__nv_fp8_e4m3>(y[j]).__x) : "memory");
-    } else {
-      const __nv_bfloat16 b = __float2bfloat16_rn(y[j]);
-      asm volatile("st.shared.u16 [%0], %1;" ::"r"(w + (uint32_t)(j * TOK_PITCH)), "h"(__bfloat16_as_ushort(b)) : "memory");
+  for (int u = 0; u < U; ++u)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const uint32_t at = w + (uint32_t)(u * TOK_STAGE + j * TOK_PITCH);
+      if constexpr (TERMS == 1)
+        asm volatile("st.shared.u8 [%0], %1;" ::"r"(at), "r"((uint32_t)from_f32<__nv_fp8_e4m3>(y[u][j]).__x) : "memory");
+      else
+        asm volatile("st.shared.u16 [%0], %1;" ::"r"(at), "h"(__bfloat16_as_ushort(__float2bfloat16_rn(y[u][j]))) : "memory");
     }
-  }
   st.sync();
   const int token = st.i >> 2, l4 = st.i & 3;
   const uint32_t r = st.at + (uint32_t)(token * TOK_PITCH + l4 * (TERMS == 1 ? 8 : 16));
-  const uint2 lo = lds64(r);
-  uint2 hi = make_uint2(0, 0);
-  if constexpr (TERMS != 1) hi = lds64(r + 8u);
+  uint2 lo[U], hi[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    lo[u] = lds64(r + (uint32_t)(u * TOK_STAGE));
+    if constexpr (TERMS != 1) hi[u] = lds64(r + (uint32_t)(u * TOK_STAGE) + 8u);
+  }
   st.sync();                                           // the stage may be written again
-  const int kt = g >> 2, gi = g & 3, x7 = token & 7;   // (chunks start at multiples of 8 rows)
-  uint8_t* sd = s + kt * o.s_step + gi;
-  if constexpr (TERMS == 4) {
-    const uint32_t raw[4] = {lo.x, lo.y, hi.x, hi.y};
-    float v[8];
-    bool nan[8];
+  const int x7 = token & 7;                            // (chunks start at multiples of 8 rows)
+  // the value bytes of these lanes in group gg, its scale
+  auto value = [&](int gg) {
+    uint8_t* line = q + (gg >> 2) * o.q_step;
+    if constexpr (TERMS == 4) return line + (((gg & 3) ^ (x7 >> 1 & 3)) << 4) + l4 * 4;
+    else return line + (((2 * (gg & 3) + (l4 >> 1)) ^ x7) << 4) + (l4 & 1) * 8;
+  };
+  auto scale = [&](int gg) { return s + (gg >> 2) * o.s_step + (gg & 3); };
+  if constexpr (TERMS == 1) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      v[2 * j] = __uint_as_float(raw[j] << 16);
-      v[2 * j + 1] = __uint_as_float(raw[j] & 0xFFFF0000u);
-    }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) nan[j] = v[j] != v[j];
-    uint8_t* qd = q + kt * o.q_step + ((gi ^ (x7 >> 1 & 3)) << 4) + l4 * 4;
-#pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      uint32_t codes;
-      const uint32_t sb = e2m1_term(t, v, nan, codes, [](uint32_t top) {
-        top = max(top, __shfl_xor_sync(0xFFFFFFFFu, top, 1));
-        return max(top, __shfl_xor_sync(0xFFFFFFFFu, top, 2));
-      });
-      if (q) {
-        *reinterpret_cast<uint32_t*>(qd + t * o.lo_q) = codes;
-        if (l4 == 0) sd[(t & 1) * 256 + (t >> 1) * 4] = (uint8_t)sb;      // row t * 16 + r of the chunk
-        if (zero_next) {
-          *reinterpret_cast<uint32_t*>(q + kt * o.q_step + (((gi + 2) ^ (x7 >> 1 & 3)) << 4) + l4 * 4 + t * o.lo_q) = 0;
-          if (l4 == 0) sd[(t & 1) * 256 + (t >> 1) * 4 + 2] = 127;
-        }
+    for (int u = 0; u < U; ++u)
+      if (q && u < live) {
+        *reinterpret_cast<uint2*>(value(g + 2 * u)) = lo[u];
+        if (l4 == 0) *scale(g + 2 * u) = 127;          // 1.0
       }
-    }
   } else {
-    uint8_t* qd = q + kt * o.q_step + (((2 * gi + (l4 >> 1)) ^ x7) << 4) + (l4 & 1) * 8;
-    uint8_t* qz = q + kt * o.q_step + (((2 * gi + 4 + (l4 >> 1)) ^ x7) << 4) + (l4 & 1) * 8;
-    if constexpr (TERMS == 1) {
-      if (q) {
-        *reinterpret_cast<uint2*>(qd) = lo;
-        if (l4 == 0) sd[0] = 127;                      // 1.0
-        if (zero_next) {
-          *reinterpret_cast<uint2*>(qz) = make_uint2(0, 0);
-          if (l4 == 0) sd[2] = 127;
-        }
-      }
-    } else {
-      const uint32_t raw[4] = {lo.x, lo.y, hi.x, hi.y};
-      float v[8], amax;
+    float v[U][8];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t raw[4] = {lo[u].x, lo[u].y, hi[u].x, hi[u].y};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        v[2 * j] = __uint_as_float(raw[j] << 16);
-        v[2 * j + 1] = __uint_as_float(raw[j] & 0xFFFF0000u);
+        v[u][2 * j] = __uint_as_float(raw[j] << 16);
+        v[u][2 * j + 1] = __uint_as_float(raw[j] & 0xFFFF0000u);
       }
-      uint32_t h[2], l[2], sh, sl;
-      two_terms<8>(v, [](float m) {
-        m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, 1));
-        return fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, 2));
-      }, h, l, sh, sl, amax);
-      if (o.permuted) {                                // k inside eight: even, then odd
-        const uint32_t h0 = __byte_perm(h[0], h[1], 0x6420), l0 = __byte_perm(l[0], l[1], 0x6420);
-        h[1] = __byte_perm(h[0], h[1], 0x7531); h[0] = h0;
-        l[1] = __byte_perm(l[0], l[1], 0x7531); l[0] = l0;
-      }
-      if (q) {
-        *reinterpret_cast<uint2*>(qd) = make_uint2(h[0], h[1]);
-        *reinterpret_cast<uint2*>(qd + o.lo_q) = make_uint2(l[0], l[1]);
-        if (l4 == 0) {
-          sd[0] = (uint8_t)sh;
-          sd[o.lo_s] = (uint8_t)sl;
+    }
+    if constexpr (TERMS == 4) {
+      bool nan[U][8];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) nan[u][j] = v[u][j] != v[u][j];
+#pragma unroll
+      for (int t = 0; t < 4; ++t)
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          uint32_t codes;
+          const uint32_t sb = e2m1_term(t, v[u], nan[u], codes, [](uint32_t top) {
+            top = max(top, __shfl_xor_sync(0xFFFFFFFFu, top, 1));
+            return max(top, __shfl_xor_sync(0xFFFFFFFFu, top, 2));
+          });
+          if (q && u < live) {
+            *reinterpret_cast<uint32_t*>(value(g + 2 * u) + t * o.lo_q) = codes;
+            if (l4 == 0) scale(g + 2 * u)[(t & 1) * 256 + (t >> 1) * 4] = (uint8_t)sb;      // row t * 16 + r of the chunk
+          }
         }
-        if (zero_next) {
-          *reinterpret_cast<uint2*>(qz) = make_uint2(0, 0);
-          *reinterpret_cast<uint2*>(qz + o.lo_q) = make_uint2(0, 0);
-          if (l4 == 0) sd[2] = sd[o.lo_s + 2] = 127;
+    } else {
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        uint32_t h[2], l[2], sh, sl;
+        float amax;
+        two_terms<8>(v[u], [](float m) {
+          m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, 1));
+          return fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, 2));
+        }, h, l, sh, sl, amax);
+        if (o.permuted) {                              // k inside eight: even, then odd
+          const uint32_t h0 = __byte_perm(h[0], h[1], 0x6420), l0 = __byte_perm(l[0], l[1], 0x6420);
+          h[1] = __byte_perm(h[0], h[1], 0x7531); h[0] = h0;
+          l[1] = __byte_perm(l[0], l[1], 0x7531); l[0] = l0;
+        }
+        if (q && u < live) {
+          uint8_t* d = value(g + 2 * u);
+          *reinterpret_cast<uint2*>(d) = make_uint2(h[0], h[1]);
+          *reinterpret_cast<uint2*>(d + o.lo_q) = make_uint2(l[0], l[1]);
+          if (l4 == 0) {
+            scale(g + 2 * u)[0] = (uint8_t)sh;
+            scale(g + 2 * u)[o.lo_s] = (uint8_t)sl;
+          }
         }
       }
+    }
+  }
+  if (zero_next && q) {
+    const int gz = g + 2 * live;
+#pragma unroll
+    for (int t = 0; t < TERMS; ++t) {
+      uint8_t* d = value(gz) + t * o.lo_q;
+      if constexpr (TERMS == 4) *reinterpret_cast<uint32_t*>(d) = 0;
+      else *reinterpret_cast<uint2*>(d) = make_uint2(0, 0);
+      if (l4 == 0) scale(gz)[TERMS == 4 ? (t & 1) * 256 + (t >> 1) * 4 : t * o.lo_s] = 127;
     }
   }
 }

@@ -301,6 +301,22 @@ def test_block_scaled_few_tiles_k_step_stages(K, sizes, act, device):
     assert oracle.rel_l2(out, y) < 5e-4
 
 
+@pytest.mark.parametrize("kernel", ["mx-f4", "mx-f8"])
+@pytest.mark.parametrize("K", [128, 640])                   # one k step, and an odd number of them
+@pytest.mark.parametrize("E, N", [(50, 1152), (50, 1280), (50, 1408), (50, 384), (7, 640)])
+def test_block_scaled_last_round_by_blocks(E, N, K, kernel, device):
+    """What does not fill a last round of the 148 CTAs is dealt out by single weight blocks, two k steps a stage: behind a whole round
+    with 0, 1 and 2 blocks left over per token block, as all there is, and not where it would take two rounds."""
+    g = torch.Generator().manual_seed(E + N + K)
+    sizes = torch.randint(1, 17, (E,), generator=g).int()
+    M = int(sizes.sum())
+    wq, ws, wdeq = quantised_weights(E, K, N, g)
+    x = torch.randn(M, K, generator=g).bfloat16()
+    ref = oracle.matmul_oracle(x.float(), wdeq, None, sizes, out_dtype=torch.float32)
+    y = run_mx(x, wq, ws, sizes, device, out_dtype=torch.float32, kernel=kernel, block_m=16, block_n=384)
+    assert oracle.rel_l2(ref, y) < 5e-4
+
+
 @pytest.mark.parametrize("acts", ["bf16", "fp8", "mxfp8"])
 @pytest.mark.parametrize("K, N, sizes", [
     (32, 2, [1, 0, 33]),                            # one group of k, one column pair

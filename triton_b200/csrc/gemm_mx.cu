@@ -34,6 +34,7 @@
 // Warps: 0 producer, 1 MMA issue + tensor-memory owner, 2-5 epilogue, 6-9 scale loaders.  Every mbarrier
 // wait is bounded.
 #include "token_out.cuh"
+#include <type_traits>
 
 namespace {
 
@@ -48,8 +49,8 @@ constexpr int MX_SF_BASE = 512 - MX_MAX_STAGES * MX_SF_COLS;    // 384: accumula
 constexpr int MX_SMEM_LIMIT = 227 * 1024;
 constexpr int MX_CTL_BARS = 3 * MX_MAX_STAGES + 5;          // full, empty, scales-ready rings; 2 + 2 accumulator; drain
 constexpr int MX_CTL_BYTES = MX_CTL_BARS * 8 + 16;          // + tensor-memory base, abort flag
-// rows on their way to the next product's tokens: a stage per two epilogue warps and, in the four-term form, weight block of the tile
-constexpr int mx_tok_bytes(bool f4) { return (f4 ? 6 : 2) * TOK_STAGE; }
+// rows on their way to the next product's tokens: a stage per two epilogue warps and weight block of the tile
+template <typename TY> constexpr int MX_TOK_BYTES = TOK_TERMS<TY> ? 6 * TOK_STAGE : 0;
 
 struct MxParams {
   const uint8_t* xq;            // packed token chunks: [slot][k step][n_mma rows x 128 B | 1024 B scale area]
@@ -61,7 +62,6 @@ struct MxParams {
   int KT, NB;                   // 128-k steps, 128-row weight blocks
   int stages, stage_bytes;
   int acc_bufs;
-  int n_groups;                 // ceil(NB / MB)
   int64_t grid_m;               // static bound on token blocks (dense problems: exact)
   TokenOut out;                 // the rows as the next product's tokens
 };
@@ -79,17 +79,39 @@ struct MxMaps {
 // tile with fp32 partial sums in global memory -- red.global.add, the slice that arrives last runs the epilogue -- were
 // correct and 20-35 % slower at 4 to 64 tokens: 48 scalar reductions per thread and slice, their fence and the counter
 // round trip take longer than a slice of a few k steps, and the epilogue warps become the bottleneck.)
+//
+// The tiles that do not fill a last round are dealt out block by block where that is one round.  A block by itself has two k steps to
+// a stage: a stage takes its way through copy, scales and MMA whatever it carries, with one k step a block took as long as
+// three do.  (fc1 of 300 tokens, 1380 tiles: 158 -> 152 us; of 4 tokens, 150 tiles, with the code of the epilogue: 24 -> 20.)
 struct MxSched {
-  uint32_t useful_m, cur, end;
+  uint32_t useful_m, cur, end, whole, wide;      // tiles dealt out whole, tiles of MB blocks; `end` counts blocks behind the whole tiles
   int NB, MB;
-  __device__ __forceinline__ MxSched(uint32_t useful_m_, int NB_, int NG, int MB_)
-      : useful_m(useful_m_), cur(blockIdx.x), end(useful_m_ * (uint32_t)NG), NB(NB_), MB(MB_) {}
+  bool narrow = false;                           // the tile is a block by itself: two k steps a stage
+  __device__ __forceinline__ MxSched(uint32_t useful_m_, int NB_, int MB_) : useful_m(useful_m_), cur(blockIdx.x), NB(NB_), MB(MB_) {
+    const uint32_t rest = (uint32_t)(NB % MB), n = useful_m * (uint32_t)((NB + MB - 1) / MB);
+    wide = useful_m * (uint32_t)(NB / MB);
+    whole = end = n;
+    const uint32_t last = n % gridDim.x, last_wide = wide + last > n ? wide + last - n : 0u;      // of the last round: tiles, wide ones
+    const uint32_t blocks = last_wide * (uint32_t)MB + (last - last_wide) * rest;
+    if (MB == 3 && last && blocks <= gridDim.x) {
+      whole = n - last;
+      end = whole + blocks;
+    }
+  }
   __device__ __forceinline__ bool next(int64_t& pid_m, int& nb0, int& mb_live) {
     if (cur >= end) return false;
-    const uint32_t grp = cur / useful_m;
-    pid_m = cur - grp * useful_m;
-    nb0 = (int)grp * MB;
-    mb_live = min(MB, NB - nb0);
+    uint32_t tile = cur, block = 0;
+    if (cur >= whole) {                          // block `block` of a tile of the last round, the wide ones first
+      const uint32_t i = cur - whole, in_wide = (wide > whole ? wide - whole : 0u) * (uint32_t)MB;
+      const uint32_t per = i < in_wide ? (uint32_t)MB : (uint32_t)(NB % MB), j = i < in_wide ? i : i - in_wide;
+      tile = (i < in_wide ? whole : max(wide, whole)) + j / per;
+      block = j % per;
+    }
+    const uint32_t grp = tile / useful_m;
+    pid_m = tile - grp * useful_m;
+    nb0 = (int)grp * MB + (int)block;
+    mb_live = cur >= whole ? 1 : min(MB, NB - nb0);
+    narrow = MB == 3 && mb_live == 1;
     cur += gridDim.x;
     return true;
   }
@@ -277,27 +299,30 @@ __device__ __forceinline__ void mma_mx(uint32_t d_tmem, uint32_t a_lo, uint32_t 
         : "memory");
 }
 
-// sums of sixteen tokens over their terms, smallest first
-template <bool F4>
-__device__ __forceinline__ void mx_sums(uint32_t taddr, int split, int tb, uint32_t (&sum)[16]) {
-  uint32_t lo[16];
-  tmem_ld16(taddr, sum);
-  if (split > 1) tmem_ld16(taddr + (uint32_t)tb, lo);
-  tmem_ld_wait();
-  if constexpr (F4) {                                   // terms 2 and 3
-    uint32_t t2[16], t3[16];
-    tmem_ld16(taddr + 2u * (uint32_t)tb, t2);
-    tmem_ld16(taddr + 3u * (uint32_t)tb, t3);
-    tmem_ld_wait();
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      sum[j] = __float_as_uint(__uint_as_float(sum[j]) + __uint_as_float(t3[j]));
-      lo[j] = __float_as_uint(__uint_as_float(lo[j]) + __uint_as_float(t2[j]));
-    }
+// sums of N tokens over their terms, smallest first
+__device__ __forceinline__ void tmem_ld_n(uint32_t taddr, uint32_t (&r)[4]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tmem_ld_n(uint32_t taddr, uint32_t (&r)[16]) { tmem_ld16(taddr, r); }
+template <bool F4, int N>
+__device__ __forceinline__ void mx_sums(uint32_t taddr, int split, int tb, uint32_t (&sum)[N]) {
+  uint32_t t1[N], t2[N], t3[N];
+  tmem_ld_n(taddr, sum);
+  if (split > 1) tmem_ld_n(taddr + (uint32_t)tb, t1);
+  if constexpr (F4) {
+    tmem_ld_n(taddr + 2u * (uint32_t)tb, t2);
+    tmem_ld_n(taddr + 3u * (uint32_t)tb, t3);
   }
-  if (split > 1) {
+  tmem_ld_wait();
 #pragma unroll
-    for (int j = 0; j < 16; ++j) sum[j] = __float_as_uint(__uint_as_float(sum[j]) + __uint_as_float(lo[j]));
+  for (int j = 0; j < N; ++j) {
+    float a = __uint_as_float(sum[j]), b = split > 1 ? __uint_as_float(t1[j]) : 0.0f;
+    if constexpr (F4) {
+      a += __uint_as_float(t3[j]);
+      b += __uint_as_float(t2[j]);
+    }
+    if (split > 1) a += b;
+    sum[j] = __float_as_uint(a);
   }
 }
 
@@ -323,9 +348,9 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
   const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;     // warp-uniform for the compiler
   const int STAGES = q.stages;
   // per stage: [MB weight tiles][token rows + 1024 B scale area (KM: three such chunks)][MB x 512 B weight scales]
-  const uint32_t OFF_X = MB * W_TILE;
-  const uint32_t OFF_XS = OFF_X + (uint32_t)q.n_mma * X_ROW;
-  const uint32_t OFF_WS = KM ? OFF_X + 3u * (uint32_t)q.chunk_bytes : OFF_XS + 1024u;
+  // where the k steps of a stage follow one another, S > 1: [S weight tiles][S such chunks][S x 512 B]
+  auto off_x = [&](int S) { return (uint32_t)(S > 1 ? S : MB) * W_TILE; };
+  auto off_ws = [&](int S) { return off_x(S) + (S > 1 ? (uint32_t)S * (uint32_t)q.chunk_bytes : (uint32_t)q.n_mma * X_ROW + 1024u); };
   const uint32_t SF_BASE = KM ? 512u - (uint32_t)(MX_MAX_STAGES > 5 ? 5 : MX_MAX_STAGES) * 24u : (uint32_t)MX_SF_BASE;
   const uint32_t ctl0 = sbase + (uint32_t)STAGES * (uint32_t)q.stage_bytes;
   auto BAR_FULL = [&](int s) { return ctl0 + 8u * (uint32_t)s; };
@@ -366,14 +391,20 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
 
   // (Whatever is read ahead of pdl_wait -- ragged metadata, weights -- is older than the kernel before this one, which let this one start
   // when its own predecessors had completed.)
-  const int KT = q.KT, NB = q.NB, NG = q.n_groups;
+  const int KT = q.KT, NB = q.NB;
   uint32_t useful_m = (uint32_t)q.grid_m;
   if (p.slice_sizes) useful_m = (uint32_t)__shfl_sync(0xFFFFFFFFu, p.block_offs[p.E], 0);
   const int acc_stride = NACC * q.n_mma;            // accumulator columns of one buffer
-  MxSched sched(useful_m, NB, NG, NACC);
-  const int KS = KM ? (KT + 2) / 3 : KT;            // stages of a tile
+  MxSched sched(useful_m, NB, NACC);
   int64_t pid_m;
   int nb0, mb_live;
+  // k steps of a stage of the current tile, as a constant of the role's loop (a loop for either form: with the choice inside, the
+  // issuing warps took 2-5 us longer over a product of 50)
+  auto with_steps = [&](auto&& loop) {
+    if constexpr (KM) loop(std::integral_constant<int, 3>());
+    else if (MB == 3 && sched.narrow) loop(std::integral_constant<int, 2>());
+    else loop(std::integral_constant<int, 1>());
+  };
 
   if (warp == 0) {
     // ================================= producer =======================================================
@@ -387,41 +418,45 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
       mx_map_block(p, q.tb, pid_m, e, row0, rows);
       const uint32_t chunk = (uint32_t)q.chunk_bytes;
       const uint8_t* xsrc = q.xq + pid_m * KT * chunk;
-      const CUtensorMap* w_map = &w_maps.m[KM ? 0 : mb_live - 1];
       int tile = __shfl_sync(0xFFFFFFFFu, e, 0) * KT * NB + nb0;             // weight tile of the stage's first k step
-      auto weights = [&](int kt, uint32_t st, uint32_t bar) {
-        if constexpr (KM) {
-          const int k_live = min(3, KT - 3 * kt);
-          elect_expect_tx(bar, (uint32_t)k_live * ((uint32_t)(MX_W_TILE_TX + MX_WS_TILE) + chunk));
-          for (int i = 0; i < k_live; ++i, tile += NB) {
-            elect_tile_3d(st + (uint32_t)i * W_TILE, w_map, 0, 0, tile, bar);
-            elect_bulk_g2s(st + OFF_WS + (uint32_t)i * MX_WS_TILE, p.w_scale + (int64_t)tile * MX_WS_TILE, (uint32_t)MX_WS_TILE, bar);
+      with_steps([&](auto steps) {
+        constexpr int S = decltype(steps)::value;
+        const int stages = (KT + S - 1) / S;
+        const CUtensorMap* w_map = &w_maps.m[S > 1 ? 0 : mb_live - 1];
+        auto weights = [&](int kt, uint32_t st, uint32_t bar) {
+          if constexpr (S > 1) {
+            const int k_live = min(S, KT - S * kt);
+            elect_expect_tx(bar, (uint32_t)k_live * ((uint32_t)(MX_W_TILE_TX + MX_WS_TILE) + chunk));
+            for (int i = 0; i < k_live; ++i, tile += NB) {
+              elect_tile_3d(st + (uint32_t)i * W_TILE, w_map, 0, 0, tile, bar);
+              elect_bulk_g2s(st + off_ws(S) + (uint32_t)i * MX_WS_TILE, p.w_scale + (int64_t)tile * MX_WS_TILE, (uint32_t)MX_WS_TILE, bar);
+            }
+          } else {
+            elect_expect_tx(bar, (uint32_t)(mb_live * (MX_W_TILE_TX + MX_WS_TILE)) + chunk);
+            elect_tile_3d(st, w_map, 0, 0, tile, bar);
+            elect_bulk_g2s(st + off_ws(1), p.w_scale + (int64_t)tile * MX_WS_TILE, (uint32_t)(mb_live * MX_WS_TILE), bar);
+            tile += NB;
           }
-        } else {
-          elect_expect_tx(bar, (uint32_t)(mb_live * (MX_W_TILE_TX + MX_WS_TILE)) + chunk);
-          elect_tile_3d(st, w_map, 0, 0, tile, bar);
-          elect_bulk_g2s(st + OFF_WS, p.w_scale + (int64_t)tile * MX_WS_TILE, (uint32_t)(mb_live * MX_WS_TILE), bar);
-          tile += NB;
+        };
+        int ahead = 0;                                 // stages that have their weights
+        if (!waited) {
+          waited = true;
+          for (; ahead < min(STAGES, stages); ++ahead) weights(ahead, sbase + (uint32_t)ahead * (uint32_t)q.stage_bytes, BAR_FULL(ahead));
+          pdl_wait();
         }
-      };
-      int ahead = 0;                                   // stages that have their weights
-      if (!waited) {
-        waited = true;
-        for (; ahead < min(STAGES, KS); ++ahead) weights(ahead, sbase + (uint32_t)ahead * (uint32_t)q.stage_bytes, BAR_FULL(ahead));
-        pdl_wait();
-      }
-      for (int kt = 0; kt < KS; ++kt, ++issued) {
-        const uint32_t st = sbase + s * (uint32_t)q.stage_bytes, bar = BAR_FULL(s);
-        if (kt >= ahead) {
-          ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_EMPTY(s), ph, ctl, 601));
-          if (!ok) break;
-          weights(kt, st, bar);
+        for (int kt = 0; kt < stages; ++kt, ++issued) {
+          const uint32_t st = sbase + s * (uint32_t)q.stage_bytes, bar = BAR_FULL(s);
+          if (kt >= ahead) {
+            ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_EMPTY(s), ph, ctl, 601));
+            if (!ok) break;
+            weights(kt, st, bar);
+          }
+          const uint32_t bytes = S > 1 ? (uint32_t)min(S, KT - S * kt) * chunk : chunk;
+          elect_bulk_g2s(st + off_x(S), xsrc, bytes, bar);
+          xsrc += bytes;
+          if (++s == (uint32_t)STAGES) { s = 0; ph ^= 1u; }
         }
-        const uint32_t bytes = KM ? (uint32_t)min(3, KT - 3 * kt) * chunk : chunk;
-        elect_bulk_g2s(st + OFF_X, xsrc, bytes, bar);
-        xsrc += bytes;
-        if (++s == (uint32_t)STAGES) { s = 0; ph ^= 1u; }
-      }
+      });
     }
     if (!ok && lane == 0) {
       // aborting: let the copies that were already issued land before the CTA leaves
@@ -441,32 +476,34 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
       if (!ok) break;
       tc_fence_after();
       const uint32_t d_tmem = tmem_base + ab * (uint32_t)acc_stride;
-      for (int kt = 0; kt < KS; ++kt) {
-        // (the scale loaders have seen the stage's copies land)
-        if (!__all_sync(0xFFFFFFFFu, ready)) ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_SF(s), ph, ctl, 602));
-        if (!ok) break;
-        tc_fence_after();
-        const uint32_t st = sbase + s * (uint32_t)q.stage_bytes;
-        const uint32_t sf = tmem_base + SF_BASE + s * SF_COLS;
-        const uint32_t a_lo = MX_DESC_LO | (st >> 4), b_lo = MX_DESC_LO | ((st + OFF_X) >> 4);
-        const uint32_t more = (uint32_t)(kt > 0);
-        // k group outermost: consecutive MMAs go to different accumulators
-        if constexpr (KM) {
-          const uint32_t bstep = (uint32_t)q.chunk_bytes >> 4;
-          const int k_live = min(3, KT - 3 * kt);
+      with_steps([&](auto steps) {
+        constexpr int S = decltype(steps)::value;
+        constexpr int KK = F4 ? 2 : 4;
+        constexpr uint32_t SFK = F4 ? (2u << 4) + (2u << 29) : (1u << 4) + (1u << 29);         // next scale byte (pair)
+        const int stages = (KT + S - 1) / S;
+        for (int kt = 0; kt < stages; ++kt) {
+          // (the scale loaders have seen the stage's copies land)
+          if (!__all_sync(0xFFFFFFFFu, ready)) ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_SF(s), ph, ctl, 602));
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t st = sbase + s * (uint32_t)q.stage_bytes;
+          const uint32_t sf = tmem_base + SF_BASE + s * SF_COLS;
+          const uint32_t a_lo = MX_DESC_LO | (st >> 4), b_lo = MX_DESC_LO | ((st + off_x(S)) >> 4);
+          const uint32_t more = (uint32_t)(kt > 0);
+          // k group outermost: consecutive MMAs go to different accumulators
+          if constexpr (S > 1) {
+            const uint32_t bstep = (uint32_t)q.chunk_bytes >> 4;
+            const int k_live = min(S, KT - S * kt);
 #pragma unroll
-          for (int i = 0; i < 3; ++i) {
-            if (i < k_live) {
+            for (int i = 0; i < S; ++i) {
+              if (i < k_live) {
 #pragma unroll
-              for (int kk = 0; kk < 2; ++kk)
-                mma_mx<true>(d_tmem, a_lo + i * (W_TILE >> 4) + kk * 2, b_lo + i * bstep + kk * 2, idesc + (uint32_t)kk * ((2u << 4) + (2u << 29)),
-                             sf + 4 * i, sf + 12 + 4 * i, (i | kk) ? 1u : more);
+                for (int kk = 0; kk < KK; ++kk)
+                  mma_mx<F4>(d_tmem, a_lo + i * (W_TILE >> 4) + kk * 2, b_lo + i * bstep + kk * 2, idesc + kk * SFK, sf + 4 * i, sf + 4 * S + 4 * i,
+                             (i | kk) ? 1u : more);
+              }
             }
-          }
-        } else {
-          constexpr int KK = F4 ? 2 : 4;
-          constexpr uint32_t SFK = F4 ? (2u << 4) + (2u << 29) : (1u << 4) + (1u << 29);       // next scale byte (pair)
-          if (mb_live == MB) {
+          } else if (mb_live == MB) {
 #pragma unroll
             for (int kk = 0; kk < KK; ++kk)
 #pragma unroll
@@ -482,11 +519,11 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
                   mma_mx<F4>(d_tmem + (uint32_t)(mb * q.n_mma), a_lo + mb * (W_TILE >> 4) + kk * 2, b_lo + kk * 2, idesc + kk * SFK, sf + 4 * mb,
                              sf + 4 * MB, kk ? 1u : more);
           }
+          elect_commit(BAR_EMPTY(s));
+          if (++s == (uint32_t)STAGES) { s = 0; ph ^= 1u; }
+          ready = mbar_test(BAR_SF(s), ph);
         }
-        elect_commit(BAR_EMPTY(s));
-        if (++s == (uint32_t)STAGES) { s = 0; ph ^= 1u; }
-        ready = mbar_test(BAR_SF(s), ph);
-      }
+      });
       if (ok) elect_commit(BAR_ACC_FULL(ab));
     }
     // every MMA issued by this warp has retired before tensor memory is freed
@@ -503,57 +540,44 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
     uint32_t it = 0;
     bool ok = true;
     while (ok && sched.next(pid_m, nb0, mb_live)) {
-      for (int kt = 0; kt < KS; ++kt, ++it) {
-        const int s = it % STAGES;
-        ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_FULL(s), (it / STAGES) & 1u, ctl, 607));
-        if (!ok) break;
-        const uint32_t st = sbase + (uint32_t)s * (uint32_t)q.stage_bytes;
-        const uint32_t taddr = tmem_base + ((uint32_t)(qd * 32) << 16) + SF_BASE + (uint32_t)(s * SF_COLS);
-        if constexpr (KM) {
-          // columns 0..11: the weight scales of the three k steps, 12..23: the token scales of the three chunks
-          const int k_live = min(3, KT - 3 * kt);
-          uint4 w[3], x[3];
+      with_steps([&](auto steps) {
+        constexpr int S = decltype(steps)::value;
+        const int stages = (KT + S - 1) / S;
+        for (int kt = 0; kt < stages; ++kt, ++it) {
+          const int s = it % STAGES;
+          ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_FULL(s), (it / STAGES) & 1u, ctl, 607));
+          if (!ok) break;
+          const uint32_t st = sbase + (uint32_t)s * (uint32_t)q.stage_bytes;
+          const uint32_t taddr = tmem_base + ((uint32_t)(qd * 32) << 16) + SF_BASE + (uint32_t)(s * SF_COLS);
+          // S > 1: the weight scales of the k steps, then the token scales of their chunks
+          constexpr int NV = S > 1 ? 2 * S : MB + 1;
+          const int live = S > 1 ? min(S, KT - S * kt) : mb_live;
+          uint4 v[NV];
 #pragma unroll
-          for (int i = 0; i < 3; ++i) {
-            w[i] = i < k_live ? lds128(st + OFF_WS + (uint32_t)i * MX_WS_TILE + (uint32_t)lane * 16u) : make_uint4(0, 0, 0, 0);
-            x[i] = i < k_live ? lds128(st + OFF_X + (uint32_t)i * (uint32_t)q.chunk_bytes + (uint32_t)q.n_mma * X_ROW + (uint32_t)lane * 16u)
-                              : make_uint4(0, 0, 0, 0);
+          for (int i = 0; i < NV; ++i) {
+            const int j = S > 1 && i >= S ? i - S : i;
+            uint32_t at = st + off_ws(S) + (uint32_t)j * MX_WS_TILE;
+            if (S > 1 ? i >= S : i == MB) at = st + off_x(S) + (S > 1 ? (uint32_t)j * (uint32_t)q.chunk_bytes : 0u) + (uint32_t)q.n_mma * X_ROW;
+            v[i] = j < live || (S == 1 && i == MB) ? lds128(at + (uint32_t)lane * 16u) : make_uint4(0, 0, 0, 0);
           }
-          asm volatile(
-              "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
-              "r"(w[0].x), "r"(w[0].y), "r"(w[0].z), "r"(w[0].w), "r"(w[1].x), "r"(w[1].y), "r"(w[1].z), "r"(w[1].w),
-              "r"(w[2].x), "r"(w[2].y), "r"(w[2].z), "r"(w[2].w), "r"(x[0].x), "r"(x[0].y), "r"(x[0].z), "r"(x[0].w)
-              : "memory");
-          asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr + 16u), "r"(x[1].x),
-                       "r"(x[1].y), "r"(x[1].z), "r"(x[1].w), "r"(x[2].x), "r"(x[2].y), "r"(x[2].z), "r"(x[2].w)
-                       : "memory");
+          if constexpr (NV >= 4)
+            asm volatile(
+                "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
+                "r"(v[0].x), "r"(v[0].y), "r"(v[0].z), "r"(v[0].w), "r"(v[1].x), "r"(v[1].y), "r"(v[1].z), "r"(v[1].w),
+                "r"(v[2].x), "r"(v[2].y), "r"(v[2].z), "r"(v[2].w), "r"(v[3].x), "r"(v[3].y), "r"(v[3].z), "r"(v[3].w)
+                : "memory");
+          if constexpr (NV != 4) {
+            constexpr int I = NV == 2 ? 0 : 4;
+            asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr + 4u * I), "r"(v[I].x),
+                         "r"(v[I].y), "r"(v[I].z), "r"(v[I].w), "r"(v[I + 1].x), "r"(v[I + 1].y), "r"(v[I + 1].z), "r"(v[I + 1].w)
+                         : "memory");
+          }
           asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(BAR_SF(s));
-          continue;
         }
-        uint4 v[MB + 1];
-#pragma unroll
-        for (int mb = 0; mb < MB; ++mb)
-          v[mb] = mb < mb_live ? lds128(st + OFF_WS + (uint32_t)mb * MX_WS_TILE + (uint32_t)lane * 16u) : make_uint4(0, 0, 0, 0);
-        v[MB] = lds128(st + OFF_XS + (uint32_t)lane * 16u);
-        if constexpr (MB == 3) {
-          asm volatile(
-              "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
-              "r"(v[0].x), "r"(v[0].y), "r"(v[0].z), "r"(v[0].w), "r"(v[1].x), "r"(v[1].y), "r"(v[1].z), "r"(v[1].w),
-              "r"(v[2].x), "r"(v[2].y), "r"(v[2].z), "r"(v[2].w), "r"(v[3].x), "r"(v[3].y), "r"(v[3].z), "r"(v[3].w)
-              : "memory");
-        } else {
-          asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(v[0].x),
-                       "r"(v[0].y), "r"(v[0].z), "r"(v[0].w), "r"(v[1].x), "r"(v[1].y), "r"(v[1].z), "r"(v[1].w)
-                       : "memory");
-        }
-        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(BAR_SF(s));
-      }
+      });
     }
   } else {
     // ================================= epilogue =======================================================
@@ -562,8 +586,9 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
     // SwiGLU the even lane holds the gate and the odd lane the linear half of a pair.
     const int qd = warp & 3;
     const bool swiglu = p.activation == MOE_ACT_SWIGLU;
+    constexpr int TG = F4 ? 4 : 16;                    // tokens at a time: a four-term block has few
     const int half = qd >> 1;
-    const TokStage tok{ctl0 + MX_CTL_BYTES + (uint32_t)(half * (F4 ? 3 : 1) * TOK_STAGE), 1 + half, (qd & 1) * 32 + lane};
+    const TokStage tok{ctl0 + MX_CTL_BYTES + (uint32_t)(half * 3 * TOK_STAGE), 1 + half, (qd & 1) * 32 + lane};
     uint32_t tc = 0;
     bool ok = true;
     for (; ok && sched.next(pid_m, nb0, mb_live); ++tc) {
@@ -576,6 +601,12 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
         const int n = (nb0 + mb) * 128 + qd * 32 + lane;
         bias_n[mb] = (p.bias && n < p.N) ? load_bias(p.bias, p.bias_dtype, (int64_t)e * p.ld_bias + n) : 0.0f;
       }
+      auto bias_of = [&](int mb) {                     // (selects: an index into registers would put them into memory)
+        float b = bias_n[0];
+#pragma unroll
+        for (int i = 1; i < NACC; ++i) b = mb == i ? bias_n[i] : b;
+        return b;
+      };
       int off = 0, first_block = 0;
       if constexpr (TOK_TERMS<TY> != 0) {
         off = p.slice_offs[e];
@@ -588,26 +619,37 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
       if (tc == 0) pdl_wait();                         // ahead of the first store
       for (int c0 = 0; c0 < rows; c0 += 16) {
         if constexpr (TOK_TERMS<TY> != 0) {
-          uint8_t *tq = nullptr, *ts = nullptr;        // of token i >> 2 of the chunk
-          const int tr = c0 + (tok.i >> 2);
-          if (tr < rows) token_addr(q.out, e, off, first_block, (int)(row0 - off) + tr, tq, ts);
-          constexpr int U = F4 ? NACC : 1;             // (stages: mx_tok_bytes)
-#pragma unroll
-          for (int m0 = 0; m0 < NACC; m0 += U) {
-            const int live = min(U, mb_live - m0);
-            if (live > 0) {
-              float y[U][8];
-#pragma unroll
-              for (int u = 0; u < U; ++u) {
-                uint32_t sum[16];
-                mx_sums<F4>(tmem_base + ((uint32_t)(qd * 32) << 16) + ab * (uint32_t)acc_stride + (uint32_t)((m0 + u) * q.n_mma + c0), q.split,
-                            q.tb, sum);
-                swiglu_chunk(p, sum, bias_n[m0 + u], lane & 1, y[u]);
-              }
-              emit_tokens<TY, U>(q.out, tok, y, live, ((qd & 1) << 4) + (lane >> 1), lane & 1, 2 * (nb0 + m0) + half, tq, ts,
-                                 nb0 + m0 + live == NB && 2 * NB + half < 4 * q.out.KT);
+          // the rows of the tile's groups into their stages, then the groups of all of them to the threads, four lanes each: with the few
+          // rows that a decode block has, one turn for the three blocks
+          const int jmax = min(16, rows - c0);
+#pragma unroll 1
+          for (int mb = 0; mb < mb_live; ++mb) {
+            const float bias = bias_of(mb);
+            const uint32_t taddr = tmem_base + ((uint32_t)(qd * 32) << 16) + ab * (uint32_t)acc_stride + (uint32_t)(mb * q.n_mma + c0);
+#pragma unroll 1
+            for (int j0 = 0; j0 < jmax; j0 += TG) {
+              uint32_t sum[TG];
+              float y[TG / 2];
+              mx_sums<F4>(taddr + (uint32_t)j0, q.split, q.tb, sum);
+              swiglu_chunk(p, sum, bias, lane & 1, y);
+              stage_tokens<TY>(tok.at + (uint32_t)(mb * TOK_STAGE), y, j0 + TG / 2 * (lane & 1), ((qd & 1) << 4) + (lane >> 1));
             }
           }
+          tok.sync();
+          const int l4 = tok.i & 3;
+#pragma unroll 1
+          for (int t0 = 0; t0 < jmax * mb_live; t0 += 16) {
+            const int t = t0 + (tok.i >> 2);
+            int mb = 0, token = t;
+            for (int i = 1; i < NACC; ++i)             // (t / jmax)
+              if (token >= jmax) { ++mb; token -= jmax; }
+            uint8_t *tq = nullptr, *ts = nullptr;
+            if (t < jmax * mb_live) token_addr(q.out, e, off, first_block, (int)(row0 - off) + c0 + token, tq, ts);
+            else mb = token = 0;
+            emit_group<TY>(q.out, staged_row<TY>(tok.at + (uint32_t)(mb * TOK_STAGE), token, l4), l4, token & 7, 2 * (nb0 + mb) + half, tq, ts,
+                           nb0 + mb == NB - 1 && 2 * NB + half < 4 * q.out.KT);
+          }
+          tok.sync();                                  // the stages may be written again
         } else {
           // parameters of token c0 + lane (lanes 0..15)
           const int tj = c0 + (lane & 15);
@@ -621,22 +663,25 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
             if (p.gammas) gamma_l = p.gammas[m];
           }
           const int jmax = min(16, rows - c0);
+          // rolled: unrolled over the blocks and sixteen tokens the code of a launch's first pass through here came from memory line by
+          // line (fc2 of 64 tokens and 128 experts 48 us, so 43.6)
+#pragma unroll 1
+          for (int mb = 0; mb < mb_live; ++mb) {
+            const int n = (nb0 + mb) * 128 + qd * 32 + lane;
+            const float bias = bias_of(mb);
+            const uint32_t taddr = tmem_base + ((uint32_t)(qd * 32) << 16) + ab * (uint32_t)acc_stride + (uint32_t)(mb * q.n_mma + c0);
+#pragma unroll 1
+            for (int j0 = 0; j0 < jmax; j0 += TG) {
+              uint32_t sum[TG];
+              mx_sums<F4>(taddr + (uint32_t)j0, q.split, q.tb, sum);
 #pragma unroll
-          for (int mb = 0; mb < NACC; ++mb) {
-            if (mb < mb_live) {
-              const int n = (nb0 + mb) * 128 + qd * 32 + lane;
-              const uint32_t taddr = tmem_base + ((uint32_t)(qd * 32) << 16) + ab * (uint32_t)acc_stride +
-                                     (uint32_t)(mb * q.n_mma + c0);
-              uint32_t sum[16];
-              mx_sums<F4>(taddr, q.split, q.tb, sum);
-#pragma unroll
-              for (int j = 0; j < 16; ++j) {
-                if (j < jmax) {                                   // warp-uniform
-                  TY* yrow = (TY*)__shfl_sync(0xFFFFFFFFu, (unsigned long long)dst_l, j);
-                  const float beta = __shfl_sync(0xFFFFFFFFu, beta_l, j);
-                  const float gamma = __shfl_sync(0xFFFFFFFFu, gamma_l, j);
+              for (int j = 0; j < TG; ++j) {
+                if (j0 + j < jmax) {                              // warp-uniform
+                  TY* yrow = (TY*)__shfl_sync(0xFFFFFFFFu, (unsigned long long)dst_l, j0 + j);
+                  const float beta = __shfl_sync(0xFFFFFFFFu, beta_l, j0 + j);
+                  const float gamma = __shfl_sync(0xFFFFFFFFu, gamma_l, j0 + j);
                   float a = __uint_as_float(sum[j]);
-                  a += bias_n[mb] * beta;
+                  a += bias * beta;
                   if (p.has_out_alpha) a *= p.out_alpha;
                   if (swiglu) {
                     const float other = __shfl_xor_sync(0xFFFFFFFFu, a, 1);
@@ -712,7 +757,7 @@ MxPlan mx_plan(const MoeGemmArgs& a) {
   pl.km = (pl.f4 && tb == 16 && pl.mb == 1 && a.tile_n == 0 && pl.KT >= 3) ? 1 : 0;
   pl.n_groups = (int)cdiv64(pl.NB, pl.mb);
   pl.chunk_bytes = (int64_t)pl.n_mma * (pl.f4 ? 64 : 128) + 1024;
-  const int ctl_bytes = MX_CTL_BYTES + mx_tok_bytes(pl.f4);
+  const int ctl_bytes = MX_CTL_BYTES;
   if (pl.km) {
     pl.mb = 3;                                       // tiles of a stage; n_groups stays the number of weight blocks
     pl.stage_bytes = 3 * MX_W_TILE_TX + 3 * (int)pl.chunk_bytes + 2048;
@@ -730,9 +775,11 @@ MxPlan mx_plan(const MoeGemmArgs& a) {
 }
 
 template <typename TY, int MB, bool F4, bool KM = false>
-int launch_mx(const GemmParams& p, const MxParams& q, const MxPlan& pl, const MxMaps& w_map, int idle_sms, cudaStream_t st) {
-  const int smem = pl.stages * pl.stage_bytes + MX_CTL_BYTES + mx_tok_bytes(pl.f4) + 1024;
-  const int64_t items = pl.grid_m * pl.n_groups;
+int launch_mx(const GemmParams& p, MxParams q, const MxPlan& pl, const MxMaps& w_map, int idle_sms, cudaStream_t st) {
+  const int room = MX_SMEM_LIMIT - 1024 - MX_CTL_BYTES - MX_TOK_BYTES<TY>;
+  if (q.stages * q.stage_bytes > room) q.stages = room / q.stage_bytes;
+  const int smem = q.stages * q.stage_bytes + MX_CTL_BYTES + MX_TOK_BYTES<TY> + 1024;
+  const int64_t items = pl.grid_m * (KM ? pl.n_groups : pl.NB);        // blocks: the last round's are dealt out one by one
   int sms = moe_sm_count() - idle_sms;
   if (sms < 1) sms = 1;
   const int grid = (int)(items < sms ? items : sms);
@@ -831,7 +878,7 @@ int moe_gemm_mx_launch(const GemmParams& p_in, const MoeGemmArgs& a, const Token
   q.xq = (const uint8_t*)a.mx_workspace; q.chunk_bytes = pl.chunk_bytes;
   q.n_mma = pl.n_mma; q.tb = pl.tb; q.split = pl.split;
   q.KT = pl.KT; q.NB = pl.NB; q.stages = pl.stages; q.stage_bytes = pl.stage_bytes; q.acc_bufs = pl.acc_bufs;
-  q.n_groups = pl.n_groups; q.grid_m = pl.grid_m;
+  q.grid_m = pl.grid_m;
   MxMaps w_map;
   for (int nb = 1; nb <= 3; ++nb)
     if (int rc = make_w_map(a, pl.KT, pl.NB, pl.f4 != 0, nb <= pl.mb ? nb : pl.mb, &w_map.m[nb - 1])) return rc;

@@ -619,12 +619,17 @@ gemm_mx_pair_kernel(const GemmParams p, const PairParams a, const __grid_constan
     auto emit = [&](const PairOut& out, const uint32_t (&sums)[16], uint32_t tab, int c, int block) {
       if constexpr (TOK_TERMS<TY> != 0) {
         if (block >= NB) return;                       // (both warps of the pair)
-        float y[1][8];
-        swiglu_chunk(p, sums, out.bias, odd, y[0]);
-        const uint32_t at = tab + (uint32_t)(c + (tok.i >> 2)) * 8u;
+        float y[8];
+        swiglu_chunk(p, sums, out.bias, odd, y);
+        stage_tokens<TY>(tok.at, y, 8 * odd, ((qd & 1) << 4) + (own >> 1));
+        tok.sync();
+        const int token = tok.i >> 2, l4 = tok.i & 3;
+        const StagedRow row = staged_row<TY>(tok.at, token, l4);
+        tok.sync();                                    // the stage may be written again
+        const uint32_t at = tab + (uint32_t)(c + token) * 8u;
         const uint2 q = lds64(at), s = lds64(at + 2048u);
-        emit_tokens<TY>(a.out, tok, y, 1, ((qd & 1) << 4) + (own >> 1), odd, 2 * block + half, (uint8_t*)(((uint64_t)q.y << 32) | q.x),
-                        (uint8_t*)(((uint64_t)s.y << 32) | s.x), block == NB - 1 && 2 * NB + half < 4 * a.out.KT);
+        emit_group<TY>(a.out, row, l4, token & 7, 2 * block + half, (uint8_t*)(((uint64_t)q.y << 32) | q.x),
+                       (uint8_t*)(((uint64_t)s.y << 32) | s.x), block == NB - 1 && 2 * NB + half < 4 * a.out.KT);
       } else {
         pair_emit<TY>(p, out, sums, tab, c);
       }

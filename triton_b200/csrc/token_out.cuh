@@ -67,21 +67,22 @@ __device__ __forceinline__ void two_terms(float (&v)[N], F all, uint32_t (&h)[N 
 }
 
 // ---- epilogue ------------------------------------------------------------------------------------------------------
-// Accumulator [weight row = lane][token = column], gate and linear in neighbouring lanes: the lane pair swaps halves of a 16-token
-// chunk, and lane `odd` gets the outputs of tokens 8 odd .. + 7 of the pair's column.
-__device__ __forceinline__ void swiglu_chunk(const GemmParams& p, const uint32_t (&raw)[16], float bias, int odd, float (&y)[8]) {
-  float v[16];
+// Accumulator [weight row = lane][token = column], gate and linear in neighbouring lanes: the lane pair swaps halves of N tokens, and lane
+// `odd` gets the outputs of tokens N / 2 odd .. of the pair's column.
+template <int N>
+__device__ __forceinline__ void swiglu_chunk(const GemmParams& p, const uint32_t (&raw)[N], float bias, int odd, float (&y)[N / 2]) {
+  float v[N];
 #pragma unroll
-  for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(raw[j]) + bias;
+  for (int j = 0; j < N; ++j) v[j] = __uint_as_float(raw[j]) + bias;
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const float recv = __shfl_xor_sync(0xFFFFFFFFu, odd ? v[j] : v[8 + j], 1);
-    y[j] = gemm_swiglu(odd ? recv : v[j], odd ? v[8 + j] : recv, p.act_alpha, p.act_limit, p.act_has_limit);
+  for (int j = 0; j < N / 2; ++j) {
+    const float recv = __shfl_xor_sync(0xFFFFFFFFu, odd ? v[j] : v[N / 2 + j], 1);
+    y[j] = gemm_swiglu(odd ? recv : v[j], odd ? v[N / 2 + j] : recv, p.act_alpha, p.act_limit, p.act_has_limit);
   }
 }
 
 // Two warps hold a group of 32 outputs (64 weight rows) of 16 tokens.  They meet in shared memory ([token][72 bytes]: rows of 18
-// words keep the lanes of a warp on distinct banks), then four lanes take a token, eight outputs each.
+// words keep the lanes of a warp on distinct banks), then four lanes take a row of a group, eight outputs each.
 constexpr int TOK_PITCH = 72, TOK_STAGE = 16 * TOK_PITCH;
 struct TokStage {
   uint32_t at;                   // shared memory of the pair of warps
@@ -102,114 +103,98 @@ __device__ __forceinline__ uint2 lds64(uint32_t a) {
   return v;
 }
 
-// y[u]: outputs of tokens 8 odd .. + 7 in column `col` (0 .. 31) of group g + 2 u, for `live` of the U neighbouring weight blocks (a
-// stage each, their chains side by side); q, s: lines of token i >> 2 of the chunk at k step 0 (q NULL: not stored).  zero_next: the
-// group two past the last block's is past K too, and zero.
-template <typename TY, int U>
-__device__ __forceinline__ void emit_tokens(const TokenOut& o, const TokStage& st, const float (&y)[U][8], int live, int col, int odd, int g,
-                                            uint8_t* q, uint8_t* s, bool zero_next) {
-  constexpr int TERMS = TOK_TERMS<TY>;
-  const uint32_t w = st.at + (uint32_t)(odd * 8 * TOK_PITCH + col * (TERMS == 1 ? 1 : 2));
+// outputs of tokens token0 .. + N - 1 in column `col` (0 .. 31) of the group staged at `at`
+template <typename TY, int N>
+__device__ __forceinline__ void stage_tokens(uint32_t at, const float (&y)[N], int token0, int col) {
+  const uint32_t w = at + (uint32_t)(token0 * TOK_PITCH + col * (TOK_TERMS<TY> == 1 ? 1 : 2));
 #pragma unroll
-  for (int u = 0; u < U; ++u)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const uint32_t at = w + (uint32_t)(u * TOK_STAGE + j * TOK_PITCH);
-      if constexpr (TERMS == 1)
-        asm volatile("st.shared.u8 [%0], %1;" ::"r"(at), "r"((uint32_t)from_f32<__nv_fp8_e4m3>(y[u][j]).__x) : "memory");
-      else
-        asm volatile("st.shared.u16 [%0], %1;" ::"r"(at), "h"(__bfloat16_as_ushort(__float2bfloat16_rn(y[u][j]))) : "memory");
-    }
-  st.sync();
-  const int token = st.i >> 2, l4 = st.i & 3;
-  const uint32_t r = st.at + (uint32_t)(token * TOK_PITCH + l4 * (TERMS == 1 ? 8 : 16));
-  uint2 lo[U], hi[U];
-#pragma unroll
-  for (int u = 0; u < U; ++u) {
-    lo[u] = lds64(r + (uint32_t)(u * TOK_STAGE));
-    if constexpr (TERMS != 1) hi[u] = lds64(r + (uint32_t)(u * TOK_STAGE) + 8u);
+  for (int j = 0; j < N; ++j) {
+    if constexpr (TOK_TERMS<TY> == 1)
+      asm volatile("st.shared.u8 [%0], %1;" ::"r"(w + (uint32_t)(j * TOK_PITCH)), "r"((uint32_t)from_f32<__nv_fp8_e4m3>(y[j]).__x) : "memory");
+    else
+      asm volatile("st.shared.u16 [%0], %1;" ::"r"(w + (uint32_t)(j * TOK_PITCH)), "h"(__bfloat16_as_ushort(__float2bfloat16_rn(y[j]))) : "memory");
   }
-  st.sync();                                           // the stage may be written again
-  const int x7 = token & 7;                            // (chunks start at multiples of 8 rows)
+}
+
+// This lane's eight values (l4: which) of a staged row
+struct StagedRow { uint2 lo, hi; };
+template <typename TY> __device__ __forceinline__ StagedRow staged_row(uint32_t at, int token, int l4) {
+  const uint32_t r = at + (uint32_t)(token * TOK_PITCH + l4 * (TOK_TERMS<TY> == 1 ? 8 : 16));
+  StagedRow v{lds64(r), make_uint2(0, 0)};
+  if constexpr (TOK_TERMS<TY> != 1) v.hi = lds64(r + 8u);
+  return v;
+}
+
+// The row, group g of its token: q, s are the token's line and scales at k step 0 (q NULL: not stored), x7 its row mod 8.  All 32 lanes
+// call, four neighbouring ones a row.  zero_next: group g + 2 is past the last weight block, and zero.
+template <typename TY>
+__device__ __forceinline__ void emit_group(const TokenOut& o, const StagedRow& row, int l4, int x7, int g, uint8_t* q, uint8_t* s, bool zero_next) {
+  constexpr int TERMS = TOK_TERMS<TY>;
   // the value bytes of these lanes in group gg, its scale
   auto value = [&](int gg) {
     uint8_t* line = q + (gg >> 2) * o.q_step;
     if constexpr (TERMS == 4) return line + (((gg & 3) ^ (x7 >> 1 & 3)) << 4) + l4 * 4;
     else return line + (((2 * (gg & 3) + (l4 >> 1)) ^ x7) << 4) + (l4 & 1) * 8;
   };
-  auto scale = [&](int gg) { return s + (gg >> 2) * o.s_step + (gg & 3); };
+  uint8_t *d = value(g), *sd = s + (g >> 2) * o.s_step + (g & 3);
   if constexpr (TERMS == 1) {
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-      if (q && u < live) {
-        *reinterpret_cast<uint2*>(value(g + 2 * u)) = lo[u];
-        if (l4 == 0) *scale(g + 2 * u) = 127;          // 1.0
-      }
+    if (q) {
+      *reinterpret_cast<uint2*>(d) = row.lo;
+      if (l4 == 0) sd[0] = 127;                        // 1.0
+    }
   } else {
-    float v[U][8];
+    const uint32_t raw[4] = {row.lo.x, row.lo.y, row.hi.x, row.hi.y};
+    float v[8];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const uint32_t raw[4] = {lo[u].x, lo[u].y, hi[u].x, hi[u].y};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        v[u][2 * j] = __uint_as_float(raw[j] << 16);
-        v[u][2 * j + 1] = __uint_as_float(raw[j] & 0xFFFF0000u);
-      }
+    for (int j = 0; j < 4; ++j) {
+      v[2 * j] = __uint_as_float(raw[j] << 16);
+      v[2 * j + 1] = __uint_as_float(raw[j] & 0xFFFF0000u);
     }
     if constexpr (TERMS == 4) {
-      bool nan[U][8];
+      bool nan[8];
 #pragma unroll
-      for (int u = 0; u < U; ++u)
+      for (int j = 0; j < 8; ++j) nan[j] = v[j] != v[j];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) nan[u][j] = v[u][j] != v[u][j];
-#pragma unroll
-      for (int t = 0; t < 4; ++t)
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          uint32_t codes;
-          const uint32_t sb = e2m1_term(t, v[u], nan[u], codes, [](uint32_t top) {
-            top = max(top, __shfl_xor_sync(0xFFFFFFFFu, top, 1));
-            return max(top, __shfl_xor_sync(0xFFFFFFFFu, top, 2));
-          });
-          if (q && u < live) {
-            *reinterpret_cast<uint32_t*>(value(g + 2 * u) + t * o.lo_q) = codes;
-            if (l4 == 0) scale(g + 2 * u)[(t & 1) * 256 + (t >> 1) * 4] = (uint8_t)sb;      // row t * 16 + r of the chunk
-          }
+      for (int t = 0; t < 4; ++t) {
+        uint32_t codes;
+        const uint32_t sb = e2m1_term(t, v, nan, codes, [](uint32_t top) {
+          top = max(top, __shfl_xor_sync(0xFFFFFFFFu, top, 1));
+          return max(top, __shfl_xor_sync(0xFFFFFFFFu, top, 2));
+        });
+        if (q) {
+          *reinterpret_cast<uint32_t*>(d + t * o.lo_q) = codes;
+          if (l4 == 0) sd[(t & 1) * 256 + (t >> 1) * 4] = (uint8_t)sb;     // row t * 16 + r of the chunk
         }
+      }
     } else {
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        uint32_t h[2], l[2], sh, sl;
-        float amax;
-        two_terms<8>(v[u], [](float m) {
-          m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, 1));
-          return fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, 2));
-        }, h, l, sh, sl, amax);
-        if (o.permuted) {                              // k inside eight: even, then odd
-          const uint32_t h0 = __byte_perm(h[0], h[1], 0x6420), l0 = __byte_perm(l[0], l[1], 0x6420);
-          h[1] = __byte_perm(h[0], h[1], 0x7531); h[0] = h0;
-          l[1] = __byte_perm(l[0], l[1], 0x7531); l[0] = l0;
-        }
-        if (q && u < live) {
-          uint8_t* d = value(g + 2 * u);
-          *reinterpret_cast<uint2*>(d) = make_uint2(h[0], h[1]);
-          *reinterpret_cast<uint2*>(d + o.lo_q) = make_uint2(l[0], l[1]);
-          if (l4 == 0) {
-            scale(g + 2 * u)[0] = (uint8_t)sh;
-            scale(g + 2 * u)[o.lo_s] = (uint8_t)sl;
-          }
+      uint32_t h[2], l[2], sh, sl;
+      float amax;
+      two_terms<8>(v, [](float m) {
+        m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, 1));
+        return fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, 2));
+      }, h, l, sh, sl, amax);
+      if (o.permuted) {                                // k inside eight: even, then odd
+        const uint32_t h0 = __byte_perm(h[0], h[1], 0x6420), l0 = __byte_perm(l[0], l[1], 0x6420);
+        h[1] = __byte_perm(h[0], h[1], 0x7531); h[0] = h0;
+        l[1] = __byte_perm(l[0], l[1], 0x7531); l[0] = l0;
+      }
+      if (q) {
+        *reinterpret_cast<uint2*>(d) = make_uint2(h[0], h[1]);
+        *reinterpret_cast<uint2*>(d + o.lo_q) = make_uint2(l[0], l[1]);
+        if (l4 == 0) {
+          sd[0] = (uint8_t)sh;
+          sd[o.lo_s] = (uint8_t)sl;
         }
       }
     }
   }
   if (zero_next && q) {
-    const int gz = g + 2 * live;
-#pragma unroll
+    uint8_t* z = value(g + 2);
+#pragma unroll 1
     for (int t = 0; t < TERMS; ++t) {
-      uint8_t* d = value(gz) + t * o.lo_q;
-      if constexpr (TERMS == 4) *reinterpret_cast<uint32_t*>(d) = 0;
-      else *reinterpret_cast<uint2*>(d) = make_uint2(0, 0);
-      if (l4 == 0) scale(gz)[TERMS == 4 ? (t & 1) * 256 + (t >> 1) * 4 : t * o.lo_s] = 127;
+      if constexpr (TERMS == 4) *reinterpret_cast<uint32_t*>(z + t * o.lo_q) = 0;
+      else *reinterpret_cast<uint2*>(z + t * o.lo_q) = make_uint2(0, 0);
+      if (l4 == 0) sd[(TERMS == 4 ? (t & 1) * 256 + (t >> 1) * 4 : t * o.lo_s) + 2] = 127;
     }
   }
 }

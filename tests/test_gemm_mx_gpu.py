@@ -537,18 +537,19 @@ def test_pair_kernel_values_beyond_two_terms(tiled, sizes, mode, device):
         assert (got.double() - ref)[keep].norm() <= (2.0 ** -8 if mode == "bf16 out" else 1e-4) * ref[keep].norm() + 1e-6
 
 
-@pytest.mark.parametrize("form", ["tb16", "tb32", "tb64", "pair", "pair default tiles", "mixed"])
+@pytest.mark.parametrize("form", ["tb16", "tb32", "tb64", "tb32 wide", "tb64 wide", "pair", "pair default tiles", "mixed"])
 @pytest.mark.parametrize("T, ff", [(3, 320), (70, 736), (200, 320)])
 @pytest.mark.parametrize("kind", ["bf16", "e4m3", "no limit", "inf"])
 def test_rows_handed_over_as_tokens(form, T, ff, kind, device):
     """fc1's rows written as fc2's tokens: the bits of the two products run apart.  Odd and even counts of weight blocks (5 and 11.5),
-    k steps that are partly past K, one to many token blocks per expert, both kernels.  Without a limit on the activation the rows go
+    k steps that are partly past K, one to many token blocks per expert, tiles of one and of three weight
+    blocks (there a chunk has the lines that its block's rows need), both kernels.  Without a limit on the activation the rows go
     through y; a token with an infinity is computed beside the pair kernel and joins the others there."""
     from triton_b200 import _lib
     from triton_b200.moe import _NoTimer, moe_layer_forward
     from triton_b200.testing import make_synthetic_layer
     E, k, d = 6, 2, 512
-    if kind == "e4m3" and form in ("tb64", "pair default tiles"):
+    if kind == "e4m3" and form in ("tb64", "tb64 wide", "pair default tiles"):
         pytest.skip("the same paths as with other blocks; e4m3 tokens have no kernel on the default tiles")
     lw = make_synthetic_layer(E, d, ff, device, seed=3, block_scaled=form != "pair default tiles")
     lw.limit = None if kind == "no limit" else 7.0
@@ -558,7 +559,8 @@ def test_rows_handed_over_as_tokens(form, T, ff, kind, device):
         x[T // 2, 5] = float("inf")
     x = x.to(torch.float8_e4m3fn) if kind == "e4m3" else x
     logits = torch.randn(T, E, device=device, generator=g) + torch.randn(E, device=device, generator=g)
-    constraint = {"tb16": {"block_m": 16}, "tb32": {"block_m": 32}, "tb64": {"block_m": 64}, "pair": {"block_m": 256},
+    constraint = {"tb16": {"block_m": 16}, "tb32": {"block_m": 32}, "tb64": {"block_m": 64}, "tb32 wide": {"block_m": 32, "block_n": 384},
+                  "tb64 wide": {"block_m": 64, "block_n": 384}, "pair": {"block_m": 256},
                   "pair default tiles": {"kernel": "mx"}, "mixed": {}}[form]
     lw.block_scaled_max_rows_per_expert = 10 ** 6
     with tb.scoped_opt_flags_constraints(constraint):

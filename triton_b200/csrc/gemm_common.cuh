@@ -25,10 +25,11 @@ struct GemmParams {
 
 // Where a SwiGLU product leaves its rows instead of y: in the operand form of the product that follows (token_out.cuh)
 struct TokenOut {
-  uint8_t* q = nullptr; uint8_t* s = nullptr;   // values and scales of the first row at k step 0; NULL: rows go to y
+  uint8_t* q = nullptr; uint8_t* s = nullptr;   // values (chunk form: chunks) and scales of the first row at k step 0; NULL: rows go to y
   int64_t q_step = 0, s_step = 0;               // bytes from a k step to the next
   int64_t block_bytes = 0;                      // chunk form: bytes from a token block to the next
-  int lo_q = 0, lo_s = 0;                       // bytes from a term's line and scale to the next term's (scale: two terms only)
+  int n_one = 0;                                // chunk form, one term: lines ahead of the scales
+  int fit = 0;                                  // chunk form: a term takes the lines its block's rows need, else tb
   int terms = 0;                                // 1, 2: e4m3; 4: e2m1
   int tb = 0;                                   // rows of a token block; 0: the pair kernel's lines
   int permuted = 0;                             // k inside eight in the order of the default weight tiles

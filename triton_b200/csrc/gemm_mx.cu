@@ -48,23 +48,25 @@ constexpr int MX_SF_COLS = 16;                 // tensor-memory columns of scale
 constexpr int MX_SF_BASE = 512 - MX_MAX_STAGES * MX_SF_COLS;    // 384: accumulators live below
 constexpr int MX_SMEM_LIMIT = 227 * 1024;
 constexpr int MX_CTL_BARS = 3 * MX_MAX_STAGES + 5;          // full, empty, scales-ready rings; 2 + 2 accumulator; drain
-constexpr int MX_CTL_BYTES = MX_CTL_BARS * 8 + 16;          // + tensor-memory base, abort flag
+constexpr int MX_CTL_BYTES = MX_CTL_BARS * 8 + 16 + MX_MAX_STAGES * 4;      // + tensor-memory base, abort flag, columns of the tile that starts with a stage
 // rows on their way to the next product's tokens: a stage per two epilogue warps and weight block of the tile
 template <typename TY> constexpr int MX_TOK_BYTES = TOK_TERMS<TY> ? 6 * TOK_STAGE : 0;
 
 struct MxParams {
-  const uint8_t* xq;            // packed token chunks: [slot][k step][n_mma rows x 128 B | 1024 B scale area]
+  const uint8_t* xq;            // packed token chunks: [slot][k step][lines of the terms | 512 B of scales], at most chunk_bytes
   int64_t chunk_bytes;
-  int n_mma;                    // MMA N: token columns (hi and lo when split)
+  int n_mma;                    // MMA N at most: token columns (hi and lo when split); accumulators are this far apart
   int tb;                       // token rows per block (16, 32, 64 or 128)
   int split;                    // terms of a token: 1, 2 (bf16 as hi + lo e4m3) or 4 (bf16 as e2m1 terms); term t of
-                                // token j is column t * tb + j
+                                // token j is column t * lines + j, lines = tb or (FIT) what the block's rows need
   int KT, NB;                   // 128-k steps, 128-row weight blocks
   int stages, stage_bytes;
   int acc_bufs;
   int64_t grid_m;               // static bound on token blocks (dense problems: exact)
   TokenOut out;                 // the rows as the next product's tokens
 };
+
+constexpr bool mx_fits(bool f4, int mb) { return !f4 && mb == 3; }
 
 struct MxMaps {
   CUtensorMap m[3];             // boxes of 1, 2 and 3 weight blocks
@@ -137,7 +139,7 @@ __device__ __forceinline__ bool mx_map_block(const GemmParams& p, int tb, int64_
 
 // ============================================================================================================
 // Pack kernel: token rows -> per (token block, k step) chunks in the operand layout of the MMA.
-//   row r of the chunk (r < n_mma) is 128 bytes = 128 e4m3 values of k = 128 kt .. +127, its 16-byte pieces XOR-
+//   line r of the chunk (term t of row j: r = t * lines + j) is 128 bytes = 128 e4m3 values of k = 128 kt .. +127, its 16-byte pieces XOR-
 //   swizzled with (r & 7) like a 128-byte-swizzled TMA tile; the scale of (row r, group g) is byte
 //   (r % 32) * 16 + (r / 32) * 4 + g of the 512 bytes that follow the rows.
 // grid = (token blocks, k steps); a warp takes a row at a time, a lane 4 consecutive k.
@@ -146,7 +148,7 @@ struct PackParams {
   const void* x; int64_t ld_x; int64_t rows_x;        // source rows; ld in elements
   const uint8_t* x_scale; int64_t ld_xs;              // e8m0 [rows_x, K / 32] for MXFP8 sources, else NULL
   const int32_t* gather;
-  int K, KT, tb, n_mma;
+  int K, KT, tb, n_mma, fit;
   int64_t chunk_bytes;
   uint8_t* out;
 };
@@ -159,7 +161,8 @@ __global__ void __launch_bounds__(256) mx_pack_x_kernel(const GemmParams p, cons
   int e; int64_t row0; int rows;
   if (!mx_map_block(p, a.tb, slot, e, row0, rows)) return;
   uint8_t* chunk = a.out + (slot * a.KT + kt) * a.chunk_bytes;
-  uint8_t* sc = chunk + (int64_t)a.n_mma * 128;
+  const int lines = !SPLIT ? a.n_mma : a.fit ? chunk_lines(rows) : a.tb;
+  uint8_t* sc = chunk + (SPLIT ? 2 : 1) * lines * 128;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int k = kt * 128 + lane * 4;
   const int g = lane >> 3;
@@ -192,7 +195,7 @@ __global__ void __launch_bounds__(256) mx_pack_x_kernel(const GemmParams p, cons
       uint32_t sb_lo; float s_lo, i_lo;
       mx8_scale(rmax, sb_lo, s_lo, i_lo);
       const uint32_t l01 = f32x2_to_e4m3x2(rs[0] * i_lo, rs[1] * i_lo), l23 = f32x2_to_e4m3x2(rs[2] * i_lo, rs[3] * i_lo);
-      const int r_lo = a.tb + r;
+      const int r_lo = lines + r;
       *reinterpret_cast<uint32_t*>(chunk + r * 128 + ((piece ^ (uint32_t)(r & 7)) << 4) + within) = h01 | (h23 << 16);
       *reinterpret_cast<uint32_t*>(chunk + r_lo * 128 + ((piece ^ (uint32_t)(r_lo & 7)) << 4) + within) = l01 | (l23 << 16);
       if ((lane & 7) == 0) {
@@ -213,7 +216,7 @@ __global__ void __launch_bounds__(256) mx_pack_x_kernel(const GemmParams p, cons
 }
 
 // ---- four e2m1 terms -----------------------------------------------------------------------------------------
-// Chunk of the four-term form: row r (r < 4 tb; term t of token j is row t * tb + j) is 64 bytes = 128 e2m1 values, low
+// Chunk of the four-term form: line r (r < 4 tb; term t of token j is line t * tb + j) is 64 bytes = 128 e2m1 values, low
 // nibble first, its 16-byte pieces XOR-swizzled with ((r >> 1) & 3) like a 64-byte-swizzled TMA tile; scales as above.
 // Two values at a time by the conversion instructions (round to nearest, ties to the even code; |q| <= 6 but for Inf, which
 // saturates): with compares and selects per value, and a warp reduction under four masks, the pack of 64 tokens for 128 experts
@@ -305,13 +308,13 @@ __device__ __forceinline__ void tmem_ld_n(uint32_t taddr, uint32_t (&r)[4]) {
 }
 __device__ __forceinline__ void tmem_ld_n(uint32_t taddr, uint32_t (&r)[16]) { tmem_ld16(taddr, r); }
 template <bool F4, int N>
-__device__ __forceinline__ void mx_sums(uint32_t taddr, int split, int tb, uint32_t (&sum)[N]) {
+__device__ __forceinline__ void mx_sums(uint32_t taddr, int split, int lines, uint32_t (&sum)[N]) {
   uint32_t t1[N], t2[N], t3[N];
   tmem_ld_n(taddr, sum);
-  if (split > 1) tmem_ld_n(taddr + (uint32_t)tb, t1);
+  if (split > 1) tmem_ld_n(taddr + (uint32_t)lines, t1);
   if constexpr (F4) {
-    tmem_ld_n(taddr + 2u * (uint32_t)tb, t2);
-    tmem_ld_n(taddr + 3u * (uint32_t)tb, t3);
+    tmem_ld_n(taddr + 2u * (uint32_t)lines, t2);
+    tmem_ld_n(taddr + 3u * (uint32_t)lines, t3);
   }
   tmem_ld_wait();
 #pragma unroll
@@ -340,6 +343,9 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
   static_assert(!KM || (F4 && MB == 3), "the k-step form is built for the four-term kernel with three tiles per stage");
   constexpr uint32_t W_TILE = F4 ? MX_W_TILE_TX : MX_W_TILE;       // bytes of a weight block in shared memory
   constexpr uint32_t X_ROW = F4 ? 64u : 128u;                      // bytes of a token row of a k step
+  // The two-term form of large problems copies and multiplies, of a token block, what its rows need (16, 32 or 64 lines a term): 300 tokens
+  // of 128 experts 324 -> 306 us per step.  Elsewhere it costs a tile's start more than it saves: 16 tokens 62.3 -> 63.9.
+  constexpr bool FIT = mx_fits(F4, MB);
   constexpr int NACC = KM ? 1 : MB;                                // accumulators (weight blocks) of a tile
   constexpr int SF_COLS = KM ? 24 : MX_SF_COLS;                    // scale columns of a stage: KM has three token chunks
   extern __shared__ uint8_t smem_raw[];
@@ -362,6 +368,7 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
   uint8_t* ctl_ptr = smem + (size_t)STAGES * (size_t)q.stage_bytes;
   volatile uint32_t* s_tmem = reinterpret_cast<volatile uint32_t*>(ctl_ptr + MX_CTL_BARS * 8);
   volatile int* s_abort = reinterpret_cast<volatile int*>(ctl_ptr + MX_CTL_BARS * 8 + 4);
+  volatile int* s_cols = reinterpret_cast<volatile int*>(ctl_ptr + MX_CTL_BARS * 8 + 16);      // per stage
   Ctl ctl{s_abort, p.status};
 
   if (threadIdx.x == 0) {
@@ -416,23 +423,30 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
     while (ok && sched.next(pid_m, nb0, mb_live)) {
       int e; int64_t row0; int rows;
       mx_map_block(p, q.tb, pid_m, e, row0, rows);
-      const uint32_t chunk = (uint32_t)q.chunk_bytes;
+      // columns of the tile and bytes of a chunk: what its rows need
+      int cols = q.n_mma;
+      if (FIT && q.split > 1) cols = 2 * chunk_lines(__shfl_sync(0xFFFFFFFFu, rows, 0));
+      const uint32_t chunk = (uint32_t)q.chunk_bytes, live = FIT ? (uint32_t)cols * X_ROW + 512u : chunk;
       const uint8_t* xsrc = q.xq + pid_m * KT * chunk;
       int tile = __shfl_sync(0xFFFFFFFFu, e, 0) * KT * NB + nb0;             // weight tile of the stage's first k step
       with_steps([&](auto steps) {
         constexpr int S = decltype(steps)::value;
         const int stages = (KT + S - 1) / S;
         const CUtensorMap* w_map = &w_maps.m[S > 1 ? 0 : mb_live - 1];
-        auto weights = [&](int kt, uint32_t st, uint32_t bar) {
+        auto weights = [&](int kt, uint32_t stage, uint32_t st, uint32_t bar) {
+          if (FIT && kt == 0) {                        // (the arrival below publishes it)
+            if (lane == 0) s_cols[stage] = cols;
+            __syncwarp();
+          }
           if constexpr (S > 1) {
             const int k_live = min(S, KT - S * kt);
-            elect_expect_tx(bar, (uint32_t)k_live * ((uint32_t)(MX_W_TILE_TX + MX_WS_TILE) + chunk));
+            elect_expect_tx(bar, (uint32_t)k_live * ((uint32_t)(MX_W_TILE_TX + MX_WS_TILE) + live));
             for (int i = 0; i < k_live; ++i, tile += NB) {
               elect_tile_3d(st + (uint32_t)i * W_TILE, w_map, 0, 0, tile, bar);
               elect_bulk_g2s(st + off_ws(S) + (uint32_t)i * MX_WS_TILE, p.w_scale + (int64_t)tile * MX_WS_TILE, (uint32_t)MX_WS_TILE, bar);
             }
           } else {
-            elect_expect_tx(bar, (uint32_t)(mb_live * (MX_W_TILE_TX + MX_WS_TILE)) + chunk);
+            elect_expect_tx(bar, (uint32_t)(mb_live * (MX_W_TILE_TX + MX_WS_TILE)) + live);
             elect_tile_3d(st, w_map, 0, 0, tile, bar);
             elect_bulk_g2s(st + off_ws(1), p.w_scale + (int64_t)tile * MX_WS_TILE, (uint32_t)(mb_live * MX_WS_TILE), bar);
             tile += NB;
@@ -441,7 +455,7 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
         int ahead = 0;                                 // stages that have their weights
         if (!waited) {
           waited = true;
-          for (; ahead < min(STAGES, stages); ++ahead) weights(ahead, sbase + (uint32_t)ahead * (uint32_t)q.stage_bytes, BAR_FULL(ahead));
+          for (; ahead < min(STAGES, stages); ++ahead) weights(ahead, (uint32_t)ahead, sbase + (uint32_t)ahead * (uint32_t)q.stage_bytes, BAR_FULL(ahead));
           pdl_wait();
         }
         for (int kt = 0; kt < stages; ++kt, ++issued) {
@@ -449,11 +463,15 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
           if (kt >= ahead) {
             ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_EMPTY(s), ph, ctl, 601));
             if (!ok) break;
-            weights(kt, st, bar);
+            weights(kt, s, st, bar);
           }
-          const uint32_t bytes = S > 1 ? (uint32_t)min(S, KT - S * kt) * chunk : chunk;
-          elect_bulk_g2s(st + off_x(S), xsrc, bytes, bar);
-          xsrc += bytes;
+          const int k_live = S > 1 ? min(S, KT - S * kt) : 1;
+          if (!FIT || S == 1) {
+            elect_bulk_g2s(st + off_x(S), xsrc, (uint32_t)k_live * live, bar);
+            xsrc += (uint32_t)k_live * chunk;
+          } else {
+            for (int i = 0; i < k_live; ++i, xsrc += chunk) elect_bulk_g2s(st + off_x(S) + (uint32_t)i * chunk, xsrc, live, bar);
+          }
           if (++s == (uint32_t)STAGES) { s = 0; ph ^= 1u; }
         }
       });
@@ -466,7 +484,7 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
     __syncwarp();
   } else if (warp == 1) {
     // ================================= MMA issuer =====================================================
-    const uint32_t idesc = F4 ? mx4_idesc(q.n_mma, 0) : mx_idesc(q.n_mma, 0);
+    uint32_t idesc = F4 ? mx4_idesc(q.n_mma, 0) : mx_idesc(q.n_mma, 0);
     pdl_begin();
     uint32_t s = 0, ph = 0, tc = 0;                    // stage and parity of the next k step
     bool ok = true, ready = false;                     // ready: the next step was complete when the last one was issued
@@ -486,6 +504,7 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
           if (!__all_sync(0xFFFFFFFFu, ready)) ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_SF(s), ph, ctl, 602));
           if (!ok) break;
           tc_fence_after();
+          if (FIT && kt == 0) idesc = mx_idesc(__shfl_sync(0xFFFFFFFFu, s_cols[s], 0), 0);
           const uint32_t st = sbase + s * (uint32_t)q.stage_bytes;
           const uint32_t sf = tmem_base + SF_BASE + s * SF_COLS;
           const uint32_t a_lo = MX_DESC_LO | (st >> 4), b_lo = MX_DESC_LO | ((st + off_x(S)) >> 4);
@@ -543,12 +562,14 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
       with_steps([&](auto steps) {
         constexpr int S = decltype(steps)::value;
         const int stages = (KT + S - 1) / S;
+        uint32_t scales_at = (uint32_t)q.n_mma * X_ROW;      // of a chunk's scales
         for (int kt = 0; kt < stages; ++kt, ++it) {
           const int s = it % STAGES;
           ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_FULL(s), (it / STAGES) & 1u, ctl, 607));
           if (!ok) break;
           const uint32_t st = sbase + (uint32_t)s * (uint32_t)q.stage_bytes;
           const uint32_t taddr = tmem_base + ((uint32_t)(qd * 32) << 16) + SF_BASE + (uint32_t)(s * SF_COLS);
+          if (FIT && kt == 0) scales_at = (uint32_t)s_cols[s] * X_ROW;
           // S > 1: the weight scales of the k steps, then the token scales of their chunks
           constexpr int NV = S > 1 ? 2 * S : MB + 1;
           const int live = S > 1 ? min(S, KT - S * kt) : mb_live;
@@ -557,7 +578,7 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
           for (int i = 0; i < NV; ++i) {
             const int j = S > 1 && i >= S ? i - S : i;
             uint32_t at = st + off_ws(S) + (uint32_t)j * MX_WS_TILE;
-            if (S > 1 ? i >= S : i == MB) at = st + off_x(S) + (S > 1 ? (uint32_t)j * (uint32_t)q.chunk_bytes : 0u) + (uint32_t)q.n_mma * X_ROW;
+            if (S > 1 ? i >= S : i == MB) at = st + off_x(S) + (S > 1 ? (uint32_t)j * (uint32_t)q.chunk_bytes : 0u) + scales_at;
             v[i] = j < live || (S == 1 && i == MB) ? lds128(at + (uint32_t)lane * 16u) : make_uint4(0, 0, 0, 0);
           }
           if constexpr (NV >= 4)
@@ -607,9 +628,11 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
         for (int i = 1; i < NACC; ++i) b = mb == i ? bias_n[i] : b;
         return b;
       };
-      int off = 0, first_block = 0;
+      const int lines = FIT ? chunk_lines(rows) : q.tb;
+      int off = 0, size = 0, first_block = 0;
       if constexpr (TOK_TERMS<TY> != 0) {
         off = p.slice_offs[e];
+        size = p.slice_sizes[e];
         if (q.out.tb) first_block = q.out.block_offs[e];
       }
       ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_ACC_FULL(ab), (tc / (uint32_t)q.acc_bufs) & 1u, ctl, 604));
@@ -630,7 +653,7 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
             for (int j0 = 0; j0 < jmax; j0 += TG) {
               uint32_t sum[TG];
               float y[TG / 2];
-              mx_sums<F4>(taddr + (uint32_t)j0, q.split, q.tb, sum);
+              mx_sums<F4>(taddr + (uint32_t)j0, q.split, lines, sum);
               swiglu_chunk(p, sum, bias, lane & 1, y);
               stage_tokens<TY>(tok.at + (uint32_t)(mb * TOK_STAGE), y, j0 + TG / 2 * (lane & 1), ((qd & 1) << 4) + (lane >> 1));
             }
@@ -644,7 +667,7 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
             for (int i = 1; i < NACC; ++i)             // (t / jmax)
               if (token >= jmax) { ++mb; token -= jmax; }
             uint8_t *tq = nullptr, *ts = nullptr;
-            if (t < jmax * mb_live) token_addr(q.out, e, off, first_block, (int)(row0 - off) + c0 + token, tq, ts);
+            if (t < jmax * mb_live) token_addr(q.out, e, off, size, first_block, (int)(row0 - off) + c0 + token, tq, ts);
             else mb = token = 0;
             emit_group<TY>(q.out, staged_row<TY>(tok.at + (uint32_t)(mb * TOK_STAGE), token, l4), l4, token & 7, 2 * (nb0 + mb) + half, tq, ts,
                            nb0 + mb == NB - 1 && 2 * NB + half < 4 * q.out.KT);
@@ -673,7 +696,7 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
 #pragma unroll 1
             for (int j0 = 0; j0 < jmax; j0 += TG) {
               uint32_t sum[TG];
-              mx_sums<F4>(taddr + (uint32_t)j0, q.split, q.tb, sum);
+              mx_sums<F4>(taddr + (uint32_t)j0, q.split, lines, sum);
 #pragma unroll
               for (int j = 0; j < TG; ++j) {
                 if (j0 + j < jmax) {                              // warp-uniform
@@ -832,13 +855,12 @@ int moe_gemm_mx_terms(const MoeGemmArgs& a) { return mx_plan(a).split; }
 bool moe_gemm_mx_token_out(const MoeGemmArgs& a, TokenOut& o) {
   const MxPlan pl = mx_plan(a);
   if (a.slice_sizes == nullptr || a.mx_workspace == nullptr || a.mx_workspace_bytes < pl.ws_bytes || (pl.split == 4 && pl.tb != 16)) return false;
-  const int row = pl.split == 4 ? 64 : 128;
   int log2_tb = 4;
   while ((1 << log2_tb) < pl.tb) ++log2_tb;
-  o.q = (uint8_t*)a.mx_workspace; o.s = o.q + (int64_t)pl.n_mma * row;
+  o.q = o.s = (uint8_t*)a.mx_workspace;
   o.q_step = o.s_step = pl.chunk_bytes;
   o.block_bytes = pl.KT * pl.chunk_bytes;
-  o.lo_q = pl.tb * row; o.lo_s = pl.tb == 16 ? 256 : pl.tb / 32 * 4;     // scale of row r: 16 (r % 32) + 4 (r / 32)
+  o.n_one = pl.n_mma; o.fit = mx_fits(pl.f4 != 0, pl.mb);
   o.terms = pl.split; o.tb = pl.tb; o.KT = pl.KT;
   o.block_offs = a.block_offs_16 + (log2_tb - 4) * a.ld_block_offs;
   return true;
@@ -862,7 +884,7 @@ int moe_gemm_mx_launch(const GemmParams& p_in, const MoeGemmArgs& a, const Token
   pk.x = a.x; pk.ld_x = a.ld_x; pk.rows_x = a.rows_x;
   pk.x_scale = a.x_scale; pk.ld_xs = a.ld_x_scale;
   pk.gather = a.gather_indx;
-  pk.K = a.K; pk.KT = pl.KT; pk.tb = pl.tb; pk.n_mma = pl.n_mma;
+  pk.K = a.K; pk.KT = pl.KT; pk.tb = pl.tb; pk.n_mma = pl.n_mma; pk.fit = mx_fits(pl.f4 != 0, pl.mb);
   pk.chunk_bytes = pl.chunk_bytes;
   pk.out = (uint8_t*)a.mx_workspace;
   const dim3 pgrid((unsigned)pl.grid_m, (unsigned)pl.KT);

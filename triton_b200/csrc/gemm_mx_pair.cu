@@ -236,13 +236,16 @@ __device__ __noinline__ uint32_t exact_rows(const GemmParams& p, const PairPackP
       const uint4* y = reinterpret_cast<const uint4*>((const __nv_bfloat16*)p.y + d * p.ld_y);
       uint8_t *q, *s;
       const int off = p.slice_offs[e], rr = (int)(m - off);
-      token_addr(a.out, e, off, a.out.tb ? a.out.block_offs[e] : 0, rr, q, s);
+      token_addr(a.out, e, off, p.slice_sizes[e], a.out.tb ? a.out.block_offs[e] : 0, rr, q, s);
+      int lo_q, lo_s;
+      token_strides(a.out, s, lo_q, lo_s);
+      s = (uint8_t*)((uintptr_t)s & ~(uintptr_t)3);
       for (int g = threadIdx.x; g < 4 * a.out.KT; g += 256) {
         uint4 raw[4] = {};
         if (g < p.N >> 6)
           for (int i = 0; i < 4; ++i) raw[i] = y[g * 4 + i];
-        if (a.out.permuted) pack_group2<true>(raw, rr & 7, g, q + (g >> 2) * a.out.q_step, a.out.lo_q, s + (g >> 2) * a.out.s_step, a.out.lo_s);
-        else pack_group2<false>(raw, rr & 7, g, q + (g >> 2) * a.out.q_step, a.out.lo_q, s + (g >> 2) * a.out.s_step, a.out.lo_s);
+        if (a.out.permuted) pack_group2<true>(raw, rr & 7, g, q + (g >> 2) * a.out.q_step, lo_q, s + (g >> 2) * a.out.s_step, lo_s);
+        else pack_group2<false>(raw, rr & 7, g, q + (g >> 2) * a.out.q_step, lo_q, s + (g >> 2) * a.out.s_step, lo_s);
       }
     }
   }
@@ -644,7 +647,7 @@ gemm_mx_pair_kernel(const GemmParams p, const PairParams a, const __grid_constan
         if (TERMS == 2 && stored && a.done) stored = !((a.done[(padded_base(t.e, t.off) + t.first + tid) >> 4] >> (tid & 15)) & 1u);
         if constexpr (TOK_TERMS<TY> != 0) {            // line and scales of the row as the next product's token, in place of row and weights
           uint8_t *q = nullptr, *s = nullptr;
-          if (stored) token_addr(a.out, t.e, t.off, a.out.tb ? a.out.block_offs[t.e] : 0, t.first + tid, q, s);
+          if (stored) token_addr(a.out, t.e, t.off, p.slice_sizes[t.e], a.out.tb ? a.out.block_offs[t.e] : 0, t.first + tid, q, s);
           asm volatile("st.shared.u64 [%0], %1;" ::"r"(tab + (uint32_t)tid * 8u), "l"(q) : "memory");
           asm volatile("st.shared.u64 [%0], %1;" ::"r"(tab + 2048u + (uint32_t)tid * 8u), "l"(s) : "memory");
         } else {
@@ -896,7 +899,6 @@ bool moe_gemm_mx_pair_token_out(const MoeGemmArgs& a, TokenOut& o) {
   if (a.mx_workspace == nullptr || a.mx_workspace_bytes < pl.ws_bytes) return false;
   o.q = (uint8_t*)a.mx_workspace; o.s = o.q + pl.xs_off;
   o.q_step = pl.terms * pl.prows * 128; o.s_step = pl.terms * pl.prows * 4;
-  o.lo_q = 1024; o.lo_s = 32;
   o.terms = pl.terms; o.permuted = a.w_kind == MOE_W_MX4_B200; o.KT = pl.KT;
   return true;
 }

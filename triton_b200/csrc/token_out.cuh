@@ -23,19 +23,31 @@ template <> constexpr int TOK_TERMS<Tok4> = 4;
 // group of 32
 __device__ __forceinline__ int64_t padded_base(int e, int off) { return (int64_t)(off & ~31) + 32 * (int64_t)e; }
 
-// Values (one line of 64 or 128 bytes) and scales of row r of expert e, whose rows start at `off`, at k step 0.  first_block:
-// chunk form, o.block_offs[e].
-__device__ __forceinline__ void token_addr(const TokenOut& o, int e, int off, int first_block, int r, uint8_t*& q, uint8_t*& s) {
+// Lines a term of a token block of `rows` rows takes in its chunk where chunks fit their rows: 16, 32 or 64.
+__device__ __forceinline__ int chunk_lines(int rows) { return rows <= 16 ? 16 : rows <= 32 ? 32 : 64; }
+// scale of line r of a chunk, from the start of its scales
+__device__ __forceinline__ int chunk_scale(int r) { return (r & 31) * 16 + (r >> 5) * 4; }
+
+// Values (one line of 64 or 128 bytes) and scales of row r of expert e, whose `size` rows start at `off`, at k step 0.  first_block:
+// chunk form, o.block_offs[e].  The low two bits of s: log2 of the lines of a term / 8 (chunk form of several terms).
+__device__ __forceinline__ void token_addr(const TokenOut& o, int e, int off, int size, int first_block, int r, uint8_t*& q, uint8_t*& s) {
   if (o.tb == 0) {
     const int64_t prow = padded_base(e, off) + r, line = o.terms * (prow & ~(int64_t)7) + (prow & 7);
     q = o.q + line * 128;
     s = o.s + line * 4;
   } else {
-    const int j = r / o.tb, rr = r - j * o.tb;
-    const int64_t at = (int64_t)(first_block + j) * o.block_bytes;
-    q = o.q + at + rr * (o.terms == 4 ? 64 : 128);
-    s = o.s + at + (rr & 31) * 16 + (rr >> 5) * 4;
+    const int j = r / o.tb, rr = r - j * o.tb, row = o.terms == 4 ? 64 : 128;
+    const int lines = o.fit ? chunk_lines(min(o.tb, size - j * o.tb)) : o.tb;
+    uint8_t* chunk = o.q + (int64_t)(first_block + j) * o.block_bytes;
+    q = chunk + rr * row;
+    s = chunk + (o.terms == 1 ? o.n_one : o.terms * lines) * row + chunk_scale(rr) + (o.terms == 1 ? 0 : 28 - __clz(lines));
   }
+}
+// from a term's line and scale to the next term's (scale: two terms)
+__device__ __forceinline__ void token_strides(const TokenOut& o, const uint8_t* s, int& lo_q, int& lo_s) {
+  const int lines = 8 << ((uintptr_t)s & 3u);
+  lo_q = o.tb == 0 ? 1024 : lines * (o.terms == 4 ? 64 : 128);
+  lo_s = o.tb == 0 ? 32 : lines < 32 ? lines * 16 : lines / 8;
 }
 
 // N values of a 32-group as two e4m3 terms, N / 8 words of eight codes each in the order of k; the group's maxima come from `all`
@@ -130,7 +142,12 @@ template <typename TY> __device__ __forceinline__ StagedRow staged_row(uint32_t 
 template <typename TY>
 __device__ __forceinline__ void emit_group(const TokenOut& o, const StagedRow& row, int l4, int x7, int g, uint8_t* q, uint8_t* s, bool zero_next) {
   constexpr int TERMS = TOK_TERMS<TY>;
-  // the value bytes of these lanes in group gg, its scale
+  int lo_q, lo_s;
+  token_strides(o, s, lo_q, lo_s);
+  s = (uint8_t*)((uintptr_t)s & ~(uintptr_t)3);
+  // scale of term t: with four terms line 16 t + r of the chunk
+  auto term_scale = [&](int t) { return TERMS == 4 ? (t & 1) * 256 + (t >> 1) * 4 : t * lo_s; };
+  // the value bytes of these lanes in group gg
   auto value = [&](int gg) {
     uint8_t* line = q + (gg >> 2) * o.q_step;
     if constexpr (TERMS == 4) return line + (((gg & 3) ^ (x7 >> 1 & 3)) << 4) + l4 * 4;
@@ -162,8 +179,8 @@ __device__ __forceinline__ void emit_group(const TokenOut& o, const StagedRow& r
           return max(top, __shfl_xor_sync(0xFFFFFFFFu, top, 2));
         });
         if (q) {
-          *reinterpret_cast<uint32_t*>(d + t * o.lo_q) = codes;
-          if (l4 == 0) sd[(t & 1) * 256 + (t >> 1) * 4] = (uint8_t)sb;     // row t * 16 + r of the chunk
+          *reinterpret_cast<uint32_t*>(d + t * lo_q) = codes;
+          if (l4 == 0) sd[term_scale(t)] = (uint8_t)sb;
         }
       }
     } else {
@@ -180,10 +197,10 @@ __device__ __forceinline__ void emit_group(const TokenOut& o, const StagedRow& r
       }
       if (q) {
         *reinterpret_cast<uint2*>(d) = make_uint2(h[0], h[1]);
-        *reinterpret_cast<uint2*>(d + o.lo_q) = make_uint2(l[0], l[1]);
+        *reinterpret_cast<uint2*>(d + lo_q) = make_uint2(l[0], l[1]);
         if (l4 == 0) {
           sd[0] = (uint8_t)sh;
-          sd[o.lo_s] = (uint8_t)sl;
+          sd[lo_s] = (uint8_t)sl;
         }
       }
     }
@@ -192,9 +209,9 @@ __device__ __forceinline__ void emit_group(const TokenOut& o, const StagedRow& r
     uint8_t* z = value(g + 2);
 #pragma unroll 1
     for (int t = 0; t < TERMS; ++t) {
-      if constexpr (TERMS == 4) *reinterpret_cast<uint32_t*>(z + t * o.lo_q) = 0;
-      else *reinterpret_cast<uint2*>(z + t * o.lo_q) = make_uint2(0, 0);
-      if (l4 == 0) sd[(TERMS == 4 ? (t & 1) * 256 + (t >> 1) * 4 : t * o.lo_s) + 2] = 127;
+      if constexpr (TERMS == 4) *reinterpret_cast<uint32_t*>(z + t * lo_q) = 0;
+      else *reinterpret_cast<uint2*>(z + t * lo_q) = make_uint2(0, 0);
+      if (l4 == 0) sd[term_scale(t) + 2] = 127;
     }
   }
 }

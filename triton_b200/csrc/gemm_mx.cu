@@ -66,7 +66,7 @@ struct MxParams {
   TokenOut out;                 // the rows as the next product's tokens
 };
 
-constexpr bool mx_fits(bool f4, int mb) { return !f4 && mb == 3; }
+inline bool mx_fits(int split, int mb) { return split == 2 && mb == 3; }
 
 struct MxMaps {
   CUtensorMap m[3];             // boxes of 1, 2 and 3 weight blocks
@@ -337,15 +337,15 @@ __device__ __forceinline__ void mx_sums(uint32_t taddr, int split, int lines, ui
 // one k step of three blocks -- for steps with so few tiles that a CTA gets single weight blocks (one to four tokens: 60
 // to 165 three-block tiles for 148 SMs).  A stage of one 8 KB tile cannot keep a per-SM copy pipeline busy (a ring of
 // 8 KB stages streams 3.3 TB/s over the GPU however many are in flight, 24 KB stages 7.1 TB/s).
-template <typename TY, int MB, bool F4, bool KM = false>
+// FIT (two-term form, MB = 3): a tile copies and multiplies, of a token block, what its rows need (16, 32 or 64 lines a term): 300 tokens of
+// 128 experts 303.6 -> 287.6 us per step.  With four terms (8 or 16 lines) or single blocks it costs a tile's start more than it saves (16
+// tokens 62.3 -> 63.9), and e4m3 tokens pay 5 % for the code alone.
+template <typename TY, int MB, bool F4, bool KM = false, bool FIT = false>
 __global__ void __launch_bounds__(MX_THREADS, 1)
 gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxMaps w_maps) {
   static_assert(!KM || (F4 && MB == 3), "the k-step form is built for the four-term kernel with three tiles per stage");
   constexpr uint32_t W_TILE = F4 ? MX_W_TILE_TX : MX_W_TILE;       // bytes of a weight block in shared memory
   constexpr uint32_t X_ROW = F4 ? 64u : 128u;                      // bytes of a token row of a k step
-  // The two-term form of large problems copies and multiplies, of a token block, what its rows need (16, 32 or 64 lines a term): 300 tokens
-  // of 128 experts 324 -> 306 us per step.  Elsewhere it costs a tile's start more than it saves: 16 tokens 62.3 -> 63.9.
-  constexpr bool FIT = mx_fits(F4, MB);
   constexpr int NACC = KM ? 1 : MB;                                // accumulators (weight blocks) of a tile
   constexpr int SF_COLS = KM ? 24 : MX_SF_COLS;                    // scale columns of a stage: KM has three token chunks
   extern __shared__ uint8_t smem_raw[];
@@ -425,7 +425,7 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
       mx_map_block(p, q.tb, pid_m, e, row0, rows);
       // columns of the tile and bytes of a chunk: what its rows need
       int cols = q.n_mma;
-      if (FIT && q.split > 1) cols = 2 * chunk_lines(__shfl_sync(0xFFFFFFFFu, rows, 0));
+      if (FIT) cols = 2 * chunk_lines(__shfl_sync(0xFFFFFFFFu, rows, 0));
       const uint32_t chunk = (uint32_t)q.chunk_bytes, live = FIT ? (uint32_t)cols * X_ROW + 512u : chunk;
       const uint8_t* xsrc = q.xq + pid_m * KT * chunk;
       int tile = __shfl_sync(0xFFFFFFFFu, e, 0) * KT * NB + nb0;             // weight tile of the stage's first k step
@@ -466,7 +466,7 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
             weights(kt, s, st, bar);
           }
           const int k_live = S > 1 ? min(S, KT - S * kt) : 1;
-          if (!FIT || S == 1) {
+          if (S == 1 || !FIT) {
             elect_bulk_g2s(st + off_x(S), xsrc, (uint32_t)k_live * live, bar);
             xsrc += (uint32_t)k_live * chunk;
           } else {
@@ -797,7 +797,7 @@ MxPlan mx_plan(const MoeGemmArgs& a) {
   return pl;
 }
 
-template <typename TY, int MB, bool F4, bool KM = false>
+template <typename TY, int MB, bool F4, bool KM = false, bool FIT = false>
 int launch_mx(const GemmParams& p, MxParams q, const MxPlan& pl, const MxMaps& w_map, int idle_sms, cudaStream_t st) {
   const int room = MX_SMEM_LIMIT - 1024 - MX_CTL_BYTES - MX_TOK_BYTES<TY>;
   if (q.stages * q.stage_bytes > room) q.stages = room / q.stage_bytes;
@@ -806,8 +806,8 @@ int launch_mx(const GemmParams& p, MxParams q, const MxPlan& pl, const MxMaps& w
   int sms = moe_sm_count() - idle_sms;
   if (sms < 1) sms = 1;
   const int grid = (int)(items < sms ? items : sms);
-  MOE_CHECK_CUDA(cudaFuncSetAttribute(gemm_mx_kernel<TY, MB, F4, KM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  MOE_CHECK_CUDA(launch_pdl(gemm_mx_kernel<TY, MB, F4, KM>, dim3(grid), dim3(MX_THREADS), (size_t)smem, st, p, q, w_map));
+  MOE_CHECK_CUDA(cudaFuncSetAttribute(gemm_mx_kernel<TY, MB, F4, KM, FIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  MOE_CHECK_CUDA(launch_pdl(gemm_mx_kernel<TY, MB, F4, KM, FIT>, dim3(grid), dim3(MX_THREADS), (size_t)smem, st, p, q, w_map));
   MOE_CHECK_LAUNCH();
   return MOE_OK;
 }
@@ -820,7 +820,13 @@ int launch_mx_ty(const GemmParams& p, const MxParams& q, const MxPlan& pl, const
     if (pl.f4) return pl.mb == 3 ? launch_mx<TY, 3, true>(p, q, pl, w_map, idle_sms, st) : launch_mx<TY, 1, true>(p, q, pl, w_map, idle_sms, st);
   }
   if constexpr (TOK_TERMS<TY> == 4) return MOE_ERR_UNSUPPORTED;
-  else return pl.mb == 3 ? launch_mx<TY, 3, false>(p, q, pl, w_map, idle_sms, st) : launch_mx<TY, 1, false>(p, q, pl, w_map, idle_sms, st);
+  else {
+    if (pl.mb != 3) return launch_mx<TY, 1, false>(p, q, pl, w_map, idle_sms, st);
+    if constexpr (TOK_TERMS<TY> != 1)
+      if (mx_fits(pl.split, pl.mb)) return launch_mx<TY, 3, false, false, true>(p, q, pl, w_map, idle_sms, st);
+    if constexpr (TOK_TERMS<TY> != 2) return launch_mx<TY, 3, false>(p, q, pl, w_map, idle_sms, st);
+    return MOE_ERR_UNSUPPORTED;
+  }
 }
 
 }  // namespace
@@ -860,7 +866,7 @@ bool moe_gemm_mx_token_out(const MoeGemmArgs& a, TokenOut& o) {
   o.q = o.s = (uint8_t*)a.mx_workspace;
   o.q_step = o.s_step = pl.chunk_bytes;
   o.block_bytes = pl.KT * pl.chunk_bytes;
-  o.n_one = pl.n_mma; o.fit = mx_fits(pl.f4 != 0, pl.mb);
+  o.n_one = pl.n_mma; o.fit = mx_fits(pl.split, pl.mb);
   o.terms = pl.split; o.tb = pl.tb; o.KT = pl.KT;
   o.block_offs = a.block_offs_16 + (log2_tb - 4) * a.ld_block_offs;
   return true;
@@ -884,7 +890,7 @@ int moe_gemm_mx_launch(const GemmParams& p_in, const MoeGemmArgs& a, const Token
   pk.x = a.x; pk.ld_x = a.ld_x; pk.rows_x = a.rows_x;
   pk.x_scale = a.x_scale; pk.ld_xs = a.ld_x_scale;
   pk.gather = a.gather_indx;
-  pk.K = a.K; pk.KT = pl.KT; pk.tb = pl.tb; pk.n_mma = pl.n_mma; pk.fit = mx_fits(pl.f4 != 0, pl.mb);
+  pk.K = a.K; pk.KT = pl.KT; pk.tb = pl.tb; pk.n_mma = pl.n_mma; pk.fit = mx_fits(pl.split, pl.mb);
   pk.chunk_bytes = pl.chunk_bytes;
   pk.out = (uint8_t*)a.mx_workspace;
   const dim3 pgrid((unsigned)pl.grid_m, (unsigned)pl.KT);

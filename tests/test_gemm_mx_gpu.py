@@ -538,13 +538,14 @@ def test_pair_kernel_values_beyond_two_terms(tiled, sizes, mode, device):
 
 
 @pytest.mark.parametrize("form", ["tb16", "tb32", "tb64", "tb32 wide", "tb64 wide", "pair", "pair default tiles", "mixed"])
-@pytest.mark.parametrize("T, ff", [(3, 320), (70, 736), (200, 320)])
+@pytest.mark.parametrize("T, ff", [(3, 320), (70, 736), (200, 320), (1300, 320)])
 @pytest.mark.parametrize("kind", ["bf16", "e4m3", "no limit", "inf"])
 def test_rows_handed_over_as_tokens(form, T, ff, kind, device):
     """fc1's rows written as fc2's tokens: the bits of the two products run apart.  Odd and even counts of weight blocks (5 and 11.5),
     k steps that are partly past K, one to many token blocks per expert, tiles of one and of three weight
     blocks (there a chunk has the lines that its block's rows need), both kernels.  Without a limit on the activation the rows go
-    through y; a token with an infinity is computed beside the pair kernel and joins the others there."""
+    through y; a token with an infinity is computed beside the pair kernel and joins the others there.  (1300 tokens: the pair kernel's
+    token pass by token, in the operators by position.)"""
     from triton_b200 import _lib
     from triton_b200.moe import _NoTimer, moe_layer_forward
     from triton_b200.testing import make_synthetic_layer

@@ -319,6 +319,7 @@ Tensor layer(const Tensor& x, const Tensor& logits, int64_t k, const py::tuple& 
   set_temp(g1, base + o_y, t1, ws1);
   set_temp(g2, base + o_tmp, t2, ws2);
   g1.gather_indx = (int32_t*)(base + o_tok);
+  g1.x_positions = (int32_t*)(base + o_row); g1.x_experts = (int16_t*)(base + o_indx); g1.x_k = (int)k;
   if (limit) { g1.act_limit = (float)*limit; g1.act_has_limit = 1; }
   g1.y = base + o_h; g1.ld_y = ff;
   g2.x = base + o_h; g2.rows_x = n;

@@ -217,6 +217,27 @@ def test_small_batch_routing_at_its_lane_splits(T, E, k, device):
     assert torch.equal(ragged.block_offs_data, ref.block_offs_data) and torch.equal(ragged.block_schedule_data, ref.block_schedule_data)
 
 
+@pytest.mark.parametrize("T", [24, 33, 64, 255, 257, 1000, 1025, 1536, 1537, 2041, 2048])
+@pytest.mark.parametrize("E, k", [(8, 8), (20, 1), (100, 2), (128, 4), (256, 16)])
+def test_routing_in_one_cluster(T, E, k, device):
+    """Either side of where a cluster of eight blocks takes the step: shares of every size (empty and partial last ones among them), lanes per
+    row, rounds of entries per warp, ties across the shares."""
+    torch.manual_seed(T + E)
+    logits = torch.randn(T, E)
+    logits[:, min(3, E - 1)] = logits[:, 0]
+    ragged, gather, scatter, sp = routing(logits.to(device), k)
+    vals, indx, bm = oracle.topk_oracle(logits, k, True)
+    col_sum, col, row = oracle.bitmatrix_metadata_oracle(indx, E)
+    md = sp.mask_metadata
+    assert torch.equal(sp.indx.cpu().int(), indx.int()) and torch.equal(sp.mask.storage.data.cpu(), bm)
+    torch.testing.assert_close(sp.vals.cpu(), vals, atol=2e-6, rtol=2e-5)
+    assert torch.equal(md.col_sum.cpu(), col_sum) and torch.equal(md.col_sorted_indx.cpu(), col) and torch.equal(md.row_sorted_indx.cpu(), row)
+    offs, block_offs, sched = oracle.ragged_metadata_oracle(col_sum, T * k)
+    assert torch.equal(ragged.slice_offs.cpu(), offs) and torch.equal(ragged.block_offs_data.cpu(), block_offs)
+    assert torch.equal(ragged.block_schedule_data.cpu(), sched)
+    assert torch.equal(gather.cpu().int(), (col // k).int())
+
+
 @pytest.mark.parametrize("call", ["row count", "reduce output", "router weight", "router bias"])
 def test_host_tensors_are_refused(call, device):
     """A tensor in host memory beside device tensors is refused, not handed to a kernel."""

@@ -640,8 +640,9 @@ extern "C" __attribute__((visibility("default"))) int moe_ragged_metadata_remap(
 }
 
 // ---------------------------------------------------------------------------------------------------------
-// moe_route: the whole routing step in three launches (the standalone entry points above take five); batches of up to
-// 256 tokens in one launch of five independent blocks (route_small_kernel, at the end of this section).
+// moe_route: the whole routing step in three launches (the standalone entry points above take five); small batches in one launch of five
+// independent blocks (route_small_kernel), those of up to some 1500 tokens in one launch of a cluster of eight (route_cluster_kernel,
+// both at the end of this section; rule: route_form).
 //   A  topk_quad_kernel<HIST>   top-k + softmax + bitmatrix row of every token, and the expert histogram of each block
 //      (route_topk_hist_kernel  of 128 tokens (partial[blk][e]) in the same pass over the logits;
 //       for other k)
@@ -854,7 +855,7 @@ __global__ void __launch_bounds__(1024) route_scan_ragged_kernel(const int32_t* 
              n_sched);
 }
 
-// The whole routing step of a small batch (at most 256 tokens, at most 256 experts, k in {1, 2, 4, 8, 16}) in ONE launch
+// The whole routing step of a small batch (at most 256 tokens, at most 256 experts, k in {1, 2, 4, 8, 16}; see route_form) in ONE launch
 // of five blocks of 1024 threads that do not wait on one another: every block selects the top-k of every row for itself
 // (`parts` lanes per row: all that 1024 threads can give a row, up to a warp; 128 KB of logits at most) and counts the picks;
 // block 0 stores the selection, the expert offsets (ragged row 0) and the positions of the entries, blocks 1..4 each build
@@ -956,12 +957,153 @@ __global__ void __launch_bounds__(1024) route_small_kernel(
 
 constexpr int kRouteSmallTokens = 256;
 
+// The whole routing step of a batch of up to 2048 tokens in one launch of one cluster: eight blocks take an eighth of the tokens each, read
+// one another's expert counts through distributed shared memory behind a cluster barrier, and rank their own entries on top of
+// them; blocks 3 to 7 build a row of the ragged metadata each.
+constexpr int kRouteClusterTokens = 2048, kRouteCluster = 8;
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ int ld_cluster(const int32_t* shared, uint32_t rank) {      // the same variable of another block
+  uint32_t at = (uint32_t)__cvta_generic_to_shared(shared), v;
+  asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %1, %2;\n\tld.shared::cluster.u32 %0, [ra];\n\t}" : "=r"(v) : "r"(at), "r"(rank) : "memory");
+  return (int)v;
+}
+
+template <typename T, int K>
+__global__ void __launch_bounds__(1024) route_cluster_kernel(
+    const T* logits, int64_t ld_logits, int T_rows, int E, int parts, int apply_softmax, T* vals, int64_t ld_vals, int16_t* indx,
+    int64_t ld_indx, uint32_t* bitmatrix, int64_t bm_stride_row, int64_t bm_stride_word, int32_t* col_sum, int32_t* col_sorted,
+    int32_t* row_sorted, int32_t* slice_offs, int32_t* block_offs, int64_t ld_block_offs, int32_t* block_sched, int64_t ld_sched,
+    int64_t n_sched, const PerPosition out) {
+  // [E + 1] own counts, [E + 1] sizes, [E + 1] scan input, [E + 1] offsets, [E] entries of the blocks before, [n] values, [n] picks (int16),
+  // [warps in use][E] counters (uint16)
+  extern __shared__ int32_t s_mem[];
+  __shared__ int32_t s_warp[33];
+  pdl_begin();
+  const int rank = (int)cluster_rank(), per_block = (T_rows + kRouteCluster - 1) / kRouteCluster, tok0 = rank * per_block;
+  const int tokens = max(0, min(per_block, T_rows - tok0)), n = tokens * K, n_max = per_block * K;
+  int32_t* s_own = s_mem;
+  int32_t* s_size = s_own + (E + 1);
+  int32_t* s_nb = s_size + (E + 1);
+  int32_t* s_offs = s_nb + (E + 1);
+  int32_t* s_before = s_offs + (E + 1);
+  float* s_val = reinterpret_cast<float*>(s_before + E);
+  int16_t* s_pick = reinterpret_cast<int16_t*>(s_val + n_max);
+  uint16_t* s_cnt = reinterpret_cast<uint16_t*>(s_pick + n_max);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rounds = (n_max + 1023) >> 10, per = rounds * 32, warps = (n_max + per - 1) / per;      // entries of a warp, warps with entries
+  for (int e = threadIdx.x; e <= E; e += blockDim.x) s_own[e] = 0;
+  for (int i = threadIdx.x; i < warps * E; i += blockDim.x) s_cnt[i] = 0;
+  __syncthreads();
+  {
+    const int part = threadIdx.x & (parts - 1), row = threadIdx.x / parts;
+    const bool live = row < tokens;
+    if (__any_sync(0xFFFFFFFFu, live)) {
+      const TopK<K> tk = quad_select<T, K>(logits + (int64_t)(tok0 + (live ? row : 0)) * ld_logits, E, part, parts);
+      if (live)
+        quad_store<T, K>(tk, part, tok0 + row, E, apply_softmax, vals, ld_vals, indx, ld_indx, bitmatrix, bm_stride_row, bm_stride_word, s_own,
+                         parts, s_pick + row * K, s_val + row * K);
+    }
+  }
+  __syncthreads();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  // meanwhile the counts of the warps' shares
+  uint16_t* my = s_cnt + warp * E;
+  if (warp < warps)
+    for (int r = 0; r < rounds; ++r) {
+      const int j = warp * per + r * 32 + lane, c = j < n ? s_pick[j] : -1;
+      const unsigned peers = __match_any_sync(0xFFFFFFFFu, c);
+      if (c >= 0 && (peers & ((1u << lane) - 1u)) == 0) my[c] += (uint16_t)__popc(peers);
+      __syncwarp();
+    }
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+    int v[kRouteCluster], before = 0, total = 0;
+#pragma unroll
+    for (int i = 0; i < kRouteCluster; ++i) v[i] = ld_cluster(s_own + e, (uint32_t)i);
+#pragma unroll
+    for (int i = 0; i < kRouteCluster; ++i) {
+      if (i < rank) before += v[i];
+      total += v[i];
+    }
+    s_size[e] = total;
+    s_before[e] = before;
+    if (rank == 0) col_sum[e] = total;
+  }
+  if (threadIdx.x == 0) s_size[E] = 0;
+  __syncthreads();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");      // the others' counts have been read
+  // stable expert-major positions: a warp ranks `per` entries in order, on top of the counts of the warps and blocks before it
+  if (rank == kRouteCluster - 5)
+    ragged_row(0, s_size, E, s_nb, s_offs, s_warp, slice_offs, nullptr, block_offs, ld_block_offs, block_sched, ld_sched, n_sched);
+  else
+    block_exclusive_scan(s_size, s_offs, E, s_warp);
+  __syncthreads();
+  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+    int run = s_offs[e] + s_before[e];
+    for (int w0 = 0; w0 < warps; w0 += 8) {
+      int v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = w0 + u < warps ? s_cnt[(w0 + u) * E + e] : 0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        if (w0 + u < warps) s_cnt[(w0 + u) * E + e] = (uint16_t)run;
+        run += v[u];
+      }
+    }
+  }
+  __syncthreads();
+  if (warp < warps)
+    for (int r = 0; r < rounds; ++r) {
+      const int j = warp * per + r * 32 + lane, c = j < n ? s_pick[j] : -1;
+      const unsigned peers = __match_any_sync(0xFFFFFFFFu, c);
+      const int before = __popc(peers & ((1u << lane) - 1u));
+      const int base = c >= 0 ? my[c] : 0;
+      __syncwarp();
+      if (c >= 0 && before == 0) my[c] = (uint16_t)(base + __popc(peers));
+      __syncwarp();
+      if (c >= 0) {
+        const int pos = base + before, flat = tok0 * K + j;
+        row_sorted[flat] = pos;
+        col_sorted[pos] = flat;
+        if (out.token) {
+          out.token[pos] = flat / K;
+          if (out.weight) out.weight[pos] = s_val[j];
+        }
+      }
+    }
+  if (rank > kRouteCluster - 5)
+    ragged_row(rank - (kRouteCluster - 5), s_size, E, s_nb, s_offs, s_warp, slice_offs, nullptr, block_offs, ld_block_offs, block_sched, ld_sched,
+               n_sched);
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");        // no block leaves while its counts are read
+}
+
 }  // namespace
 
 extern "C" __attribute__((visibility("default"))) size_t moe_route_workspace(int64_t T, int E, int k) {
   (void)k;
   const int64_t nb = cdiv64(T > 0 ? T : 1, kRouteTokPerBlock);
   return (size_t)((2 * nb * E + E) * (int64_t)sizeof(int32_t));
+}
+
+// us per call in a graph (small, cluster, three launches):
+//   128 experts, k = 4:  16 tokens 6.3, 7.0;  32  8.3, 7.2;  64  8.7, 7.7;  256  14.2, 10.8;  300  -, 9.2, 14.7;  1024  -, 12.8, 15.0;
+//                        1536  -, 14.5, 15.1;  2048  -, 17.3, 15.0
+//   64 experts, k = 8:   16 tokens 8.0, 7.5;  256  16.1, 14.5;  1536  -, 16.1, 18.5;  2048  -, 19.4, 18.9
+//   64 experts, k = 4:   32 tokens 8.3, 7.1;  96  7.5, 7.9;  192  9.2, 9.5;  256  11.2, 10.4;  2048  -, 14.1, 13.7
+//   32 experts, k = 4:   64 tokens 7.9, 7.4;  96  6.8, 7.8;  256  9.4, 10.5;  300  -, 8.4, 12.9;  2048  -, 12.0, 13.3
+//   8 experts, k = 2:    64 tokens 5.9, 7.0;  256  5.9, 8.1;  300  -, 7.1, 13.3;  2048  -, 8.0, 13.6
+// The small form repeats the whole selection in five blocks, the cluster has an eighth of it in each of eight and two barriers; past some
+// 1500 tokens eight SMs are fewer than the selection wants.
+enum { ROUTE_SMALL, ROUTE_CLUSTER, ROUTE_LAUNCHES };
+static int route_form(int64_t T, int E, int k) {
+  if (!(k == 1 || k == 2 || k == 4 || k == 8 || k == 16)) return ROUTE_LAUNCHES;
+  if (T <= kRouteSmallTokens) return T >= 24 && k >= 4 && (E * k >= 512 || T <= 64) ? ROUTE_CLUSTER : ROUTE_SMALL;
+  return T <= (E * k <= 128 ? kRouteClusterTokens : 1536) ? ROUTE_CLUSTER : ROUTE_LAUNCHES;
 }
 
 static int route_launch(
@@ -982,7 +1124,8 @@ static int route_launch(
   MOE_CHECK_ARG(workspace_bytes >= moe_route_workspace(T, E, k), "moe_route: workspace too small (%zu < %zu)", workspace_bytes,
                 moe_route_workspace(T, E, k));
   cudaStream_t st = (cudaStream_t)stream;
-  if (T <= kRouteSmallTokens && (k == 1 || k == 2 || k == 4 || k == 8 || k == 16)) {
+  const int form = route_form(T, E, k);
+  if (form == ROUTE_SMALL) {
     const int n = (int)T * k, warps = (n + 31) / 32 < 32 ? (n + 31) / 32 : 32;
     const size_t smem_s = (size_t)(3 * (E + 1) + n) * sizeof(int32_t) + (size_t)(n + warps * E) * sizeof(int16_t);   // < 48 KB
     const int parts = T <= 32 ? 32 : T <= 64 ? 16 : T <= 128 ? 8 : 4;
@@ -1001,6 +1144,40 @@ static int route_launch(
       default: MOE_ROUTE_SMALL(16); break;
     }
 #undef MOE_ROUTE_SMALL
+    MOE_CHECK_LAUNCH();
+    return MOE_OK;
+  }
+  if (form == ROUTE_CLUSTER) {
+    const int per_block = ((int)T + kRouteCluster - 1) / kRouteCluster, n = per_block * k, warps = (n + 31) / 32 < 32 ? (n + 31) / 32 : 32;
+    const size_t smem_c = (size_t)(5 * E + 4 + n) * sizeof(int32_t) + (size_t)(n + warps * E) * sizeof(int16_t);      // < 48 KB
+    const int parts = per_block <= 32 ? 32 : per_block <= 64 ? 16 : per_block <= 128 ? 8 : 4;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kRouteCluster);
+    cfg.blockDim = dim3(1024);
+    cfg.dynamicSmemBytes = smem_c;
+    cfg.stream = st;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = kRouteCluster; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
+#define MOE_ROUTE_CLUSTER(KK)                                                                                            \
+  MOE_DISPATCH_FLOAT(dtype, Tv, {                                                                                         \
+    MOE_CHECK_CUDA(cudaLaunchKernelEx(&cfg, route_cluster_kernel<Tv, KK>, (const Tv*)logits, ld_logits, (int)T, E, parts,    \
+                                      apply_softmax, (Tv*)vals, ld_vals, indx, ld_indx, bitmatrix, bm_stride_row,            \
+                                      bm_stride_word, col_sum, col_sorted, row_sorted, slice_offs, block_offs,               \
+                                      ld_block_offs, block_sched, ld_sched, n_sched, out));                                  \
+  })
+    switch (k) {
+      case 1: MOE_ROUTE_CLUSTER(1); break;
+      case 2: MOE_ROUTE_CLUSTER(2); break;
+      case 4: MOE_ROUTE_CLUSTER(4); break;
+      case 8: MOE_ROUTE_CLUSTER(8); break;
+      default: MOE_ROUTE_CLUSTER(16); break;
+    }
+#undef MOE_ROUTE_CLUSTER
     MOE_CHECK_LAUNCH();
     return MOE_OK;
   }

@@ -109,3 +109,9 @@ def test_router_topk_against_reference_fixture(golden, name, device):
     assert torch.equal(sp.indx.cpu().int()[same], g["indx"].int()[same])
     assert torch.equal(sp.mask.storage.data.cpu()[: ref.shape[0]][same], g["bitmatrix"][same])
     assert (sp.vals.cpu().float()[same] - g["vals"].float()[same]).abs().max().item() <= 2.0 ** -8
+
+
+@pytest.mark.parametrize("case", [(129, 2880, 128, 4), (131, 512, 20, 2), (137, 1024, 256, 8), (1800, 512, 64, 4), (4100, 320, 100, 4), (8000, 576, 16, 2)])
+def test_router_topk_slices_of_a_cluster(case, device):
+    """2, 4 and 8 slices of K per token block, last blocks of 1, 3, 9, 4 and 64 rows: shares of the rows that are empty or partial."""
+    test_router_topk_against_oracle(case, torch.float32, True, device)

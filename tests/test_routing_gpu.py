@@ -104,6 +104,20 @@ def test_expert_sort_at_the_segments_of_its_scan(T, E, k, device):
     assert torch.equal(col_sum.cpu(), o_sum.int()) and torch.equal(col.cpu(), o_col.int()) and torch.equal(row.cpu(), o_row.int())
 
 
+@pytest.mark.parametrize("T, E, k, n_rows", [(1, 1, 1, None), (7, 3, 2, 5), (9, 256, 1, None), (8192, 256, 4, None), (8193, 256, 4, None),
+                                             (10922, 20, 3, 10000), (3000, 33, 5, 0)])
+def test_expert_sort_in_one_cluster(T, E, k, n_rows, device):
+    # up to 32768 entries: eight shares (empty and partial ones), dropped entries and rows past a device-side bound
+    torch.manual_seed(T + E)
+    indx = torch.randint(-1 if E > 3 else 0, E, (T, k)).short()
+    bound = None if n_rows is None else torch.tensor([n_rows], dtype=torch.int32, device=device)
+    col_sum, col, row = _lib.host().bitmatrix_metadata(indx.to(device), E, bound)
+    kept = indx.clone()
+    kept[T if n_rows is None else n_rows:] = -1
+    o_sum, o_col, o_row = oracle.bitmatrix_metadata_oracle(kept, E)
+    assert torch.equal(col_sum.cpu(), o_sum.int()) and torch.equal(col.cpu(), o_col.int()) and torch.equal(row.cpu(), o_row.int())
+
+
 @pytest.mark.parametrize("n_slices", [1, 7, 33, 911, 1025])
 def test_ragged_metadata_and_remap(n_slices, device):
     # reference tests/test_tensor.py:243-277

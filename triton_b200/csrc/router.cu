@@ -9,9 +9,10 @@
 // 128-byte swizzle) through a ring of stages, warp 1 issues tcgen05.mma.kind::f16 (M = 128 tokens, N = E experts) into
 // one fp32 accumulator in tensor memory, warps 2-17 select: they spill the accumulator to shared memory and several
 // threads per token row add the bias and keep the k best in registers.  With few tokens K is cut into slices so that many SMs pull the
-// operands: every slice adds its partial logits into an fp32 scratch with red.global.add, and the CTA that finishes
-// last for a token block (a counter per block) reads the sums back, does the selection and leaves scratch and counter
-// zero, as it found them.
+// operands: the slices of a token block are a cluster, every CTA leaves its partial logits in its own shared memory, and behind a
+// cluster barrier each sums a share of the rows over all of them (distributed shared memory, in the order of the slices) and selects
+// for it.  (As partial sums in an fp32 scratch by red.global.add, with the selection in the CTA that came last: 4100 tokens of 2880 x 128
+// with the sort behind it 31.7 us, so 26.3; 128 tokens 25.0 and 21.4.)
 // Every mbarrier wait is bounded.
 #include "gemm_tc_common.cuh"
 #include "topk_select.cuh"
@@ -34,8 +35,6 @@ struct RouterParams {
   void* vals; int vals_dtype; int64_t ld_vals;
   int16_t* indx; int64_t ld_indx;
   uint32_t* bitmatrix; int64_t bm_stride_row, bm_stride_word;
-  float* acc;                     // [blocks * 128, n_mma] partial sums (splits > 1)
-  int32_t* counters;              // [blocks]
   int32_t* status;
 };
 
@@ -72,16 +71,27 @@ __device__ __forceinline__ void rt_store_row(const RouterParams& p, int64_t row,
   }
 }
 
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// a word at the same place of shared memory in slice `rank` of the cluster
+__device__ __forceinline__ uint32_t ld_slice_u32(uint32_t at, int splits, int rank) {
+  uint32_t v;
+  if (splits == 1) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(at) : "memory");
+  else asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %1, %2;\n\tld.shared::cluster.u32 %0, [ra];\n\t}" : "=r"(v) : "r"(at), "r"(rank) : "memory");
+  return v;
+}
+
 template <int K>
 __global__ void __launch_bounds__(RT_THREADS, 1)
 router_topk_kernel(const RouterParams p, const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const uint32_t sbase = smem_u32(smem);
+  float* mat = reinterpret_cast<float*>(smem);
   __shared__ __align__(8) uint64_t bars[2 * RT_STAGES_MAX + 1];
   __shared__ uint32_t s_tmem;
   __shared__ int s_abort;
-  __shared__ int s_last;
   __shared__ float s_bias[256];
   const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;     // warp-uniform for the compiler
   const int STAGES = p.stages;
@@ -100,7 +110,6 @@ router_topk_kernel(const RouterParams p, const __grid_constant__ CUtensorMap x_m
     }
     mbar_init(BAR_ACC, 1);
     s_abort = 0;
-    s_last = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (threadIdx.x == 32) {
@@ -118,7 +127,7 @@ router_topk_kernel(const RouterParams p, const __grid_constant__ CUtensorMap x_m
   pdl_begin();
 
   const int64_t blk = blockIdx.x;
-  const int split = blockIdx.y;
+  const int split = blockIdx.y;                 // rank in the cluster of a token block's slices
   const int kt0 = (int)((int64_t)p.KT * split / p.splits), kt1 = (int)((int64_t)p.KT * (split + 1) / p.splits);
   const int n_steps = kt1 - kt0;
 
@@ -160,116 +169,105 @@ router_topk_kernel(const RouterParams p, const __grid_constant__ CUtensorMap x_m
     if (!ok) mbar_wait(BAR_ACC, 0, ctl, 803);
     __syncwarp();
   } else {
-    // ---- selection: 16 warps ------------------------------------------------------------------------------
-    // Stage A brings the block's logits into shared memory as [expert][token row] (the operand stages are free by now):
-    // from tensor memory when this CTA holds the whole sum, else each warp adds its share of the partial sums into the
-    // global scratch and the CTA that arrives last copies the totals back.  Stage B: P threads per token row (adjacent
-    // lanes), each walks every P-th expert with its own best-k list, the lists of a row meet by shuffles.  A single
-    // thread per row spent 12 us of dependent compare-and-select chains on 128 experts.
+    // ---- 16 warps: this slice's logits into shared memory as [expert][token row] (the operand stages are free by then) ----
     const int qd = warp & 3, grp = (warp - 2) >> 2;            // lane quarter of tensor memory, share of its columns
     const int sid = threadIdx.x - 64;
-    const int r = qd * 32 + lane;
     // the bias once per CTA, while the main loop runs (read per logit from global memory it made the selection wait on
     // one load after the other)
     if (sid < 256) s_bias[sid] = (p.bias && sid < p.E) ? load_bias(p.bias, p.bias_dtype, sid) : 0.0f;
-    mbar_wait(BAR_ACC, 0, ctl, 804);
-    asm volatile("bar.sync 1, 512;" ::: "memory");
-    const bool ok = *(volatile int*)&s_abort == 0;              // the same answer in all sixteen warps
-    tc_fence_after();
-    const uint32_t taddr = tmem + ((uint32_t)(qd * 32) << 16);
-    const int rows_blk = (int)min((int64_t)RT_BLOCK_T, p.T - blk * RT_BLOCK_T);
-    float* mat = reinterpret_cast<float*>(smem);
-    bool finish = p.splits == 1;
-    if (ok) {
-      float* dst = p.acc + blk * RT_BLOCK_T * p.n_mma + r;      // scratch of a block: [expert][token row]
+    if (__all_sync(0xFFFFFFFFu, mbar_wait(BAR_ACC, 0, ctl, 804))) {
+      tc_fence_after();
+      const uint32_t taddr = tmem + ((uint32_t)(qd * 32) << 16);
       for (int c0 = grp * 16; c0 < p.n_mma; c0 += 64) {
         uint32_t v[16];
         tmem_ld16(taddr + (uint32_t)c0, v);
         tmem_ld_wait();
-        if (p.splits == 1) {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) mat[(c0 + j) * RT_MAT_LD + r] = __uint_as_float(v[j]);
-        } else if (r < rows_blk) {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) atomicAdd(dst + (c0 + j) * RT_BLOCK_T, __uint_as_float(v[j]));
-        }
+        for (int j = 0; j < 16; ++j) mat[(c0 + j) * RT_MAT_LD + qd * 32 + lane] = __uint_as_float(v[j]);
       }
-      if (p.splits > 1) {
-        __threadfence();
-        asm volatile("bar.sync 1, 512;" ::: "memory");
-        if (sid == 0) {
-          const int prev = atomicAdd(p.counters + blk, 1);
-          s_last = (prev == p.splits - 1) ? 1 : 0;
-          __threadfence();
-        }
-        asm volatile("bar.sync 1, 512;" ::: "memory");
-        finish = s_last != 0;
-        if (finish) {
-          // the live rows only, eight independent loads per thread at a time (one after the other this copy took 8 us)
-          const float* src = p.acc + blk * RT_BLOCK_T * p.n_mma;
-          int lr = 0;
-          while ((1 << lr) < rows_blk) ++lr;
-          const int total = p.n_mma << lr;
-          for (int i0 = sid; i0 < total; i0 += 512 * 8) {
-            float v[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-              const int i = i0 + u * 512;
-              v[u] = i < total ? __ldcg(src + (i >> lr) * RT_BLOCK_T + (i & ((1 << lr) - 1))) : 0.0f;
-            }
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-              const int i = i0 + u * 512;
-              if (i < total) {
-                mat[(i >> lr) * RT_MAT_LD + (i & ((1 << lr) - 1))] = v[u];
-                // leave the scratch as it was found: all zero
-                const_cast<float*>(src)[(i >> lr) * RT_BLOCK_T + (i & ((1 << lr) - 1))] = 0.0f;
-              }
-            }
-          }
-          if (sid == 0) p.counters[blk] = 0;
-        }
-      }
-      asm volatile("bar.sync 1, 512;" ::: "memory");
-    }
-    if (ok && finish) {
-      // P threads per row: 4 for a full block, 8 when the block holds at most 64 rows (more threads per row would
-      // spend in merge rounds what they save on the walk)
-      const int lp = rows_blk <= 64 ? 3 : 2;
-      const int P = 1 << lp;
-      const int part = lane & (P - 1);
-      const int rr = (sid >> 5) * (32 >> lp) + (lane >> lp);
-      const int64_t row = blk * RT_BLOCK_T + rr;
-      const bool live = rr < rows_blk;
-      constexpr int NSUB = K <= 4 ? 2 : 1;
-      TopK<K> sub[NSUB];
-      const int rq = rr & (RT_BLOCK_T - 1);
-#pragma unroll 1
-      for (int e0 = part; e0 < p.E; e0 += P * NSUB * 4) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-#pragma unroll
-          for (int u = 0; u < NSUB; ++u) {          // the lists alternate: independent chains side by side
-            const int e = e0 + (j * NSUB + u) * P;
-            if (e < p.E) {
-              float x = mat[e * RT_MAT_LD + rq] + s_bias[e];
-              if (p.round_bf16) x = __bfloat162float(__float2bfloat16(x));
-              if (p.logits_out && live) p.logits_out[row * p.ld_logits + e] = x;
-              sub[u].push(x, e);
-            }
-          }
-        }
-      }
-      TopK<K> tk = sub[0];
-#pragma unroll
-      for (int u = 1; u < NSUB; ++u) tk.merge(sub[u].key, sub[u].idx);
-      tk.merge_lanes(P);
-      if (live && part == 0) rt_store_row<K>(p, row, tk);
     }
   }
 
   tc_fence_before();
   __syncthreads();
+  if (p.splits > 1) cluster_barrier();
+  if (warp >= 2) {
+    // ---- selection: P threads per token row (adjacent lanes), each walks every P-th expert with its own best-k list, the lists of a row
+    // meet by shuffles.  A single thread per row spent 12 us of dependent compare-and-select chains on 128 experts. ----
+    const int sid = threadIdx.x - 64;
+    const int rows_blk = (int)min((int64_t)RT_BLOCK_T, p.T - blk * RT_BLOCK_T);
+    int lr = 0;
+    while ((1 << lr) < rows_blk) ++lr;
+    lr = max(0, lr - (31 - __clz(p.splits)));                  // this CTA's share of the rows: 2^lr from r0 on
+    const int r0 = split << lr, rows = min(1 << lr, rows_blk - r0);
+    bool ok = true;
+    for (int i = 0; i < p.splits; ++i) ok = ok && ld_slice_u32(smem_u32((const void*)&s_abort), p.splits, i) == 0;
+    if (ok && rows > 0) {
+      if (p.splits > 1) {
+        const int total = p.n_mma << lr;
+        for (int i0 = sid; i0 < total; i0 += 512 * 4) {
+          float sum[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int i = i0 + u * 512;
+            sum[u] = 0.0f;
+            if (i < total) {
+              const uint32_t at = smem_u32(mat + (i >> lr) * RT_MAT_LD + r0 + (i & ((1 << lr) - 1)));
+#pragma unroll 1
+              for (int j = 0; j < p.splits; j += 2) {
+                const float x = __uint_as_float(ld_slice_u32(at, p.splits, j)), y = __uint_as_float(ld_slice_u32(at, p.splits, j + 1));
+                sum[u] += x;
+                sum[u] += y;
+              }
+            }
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {                        // (only this CTA reads these rows of its own matrix)
+            const int i = i0 + u * 512;
+            if (i < total) mat[(i >> lr) * RT_MAT_LD + r0 + (i & ((1 << lr) - 1))] = sum[u];
+          }
+        }
+        asm volatile("bar.sync 1, 512;" ::: "memory");
+      }
+      // P threads per row: 4 for a full block, 8 for at most 64 rows (more threads per row would spend in merge rounds what they save on
+      // the walk)
+      const int lp = rows <= 64 ? 3 : 2;
+      const int P = 1 << lp;
+      const int part = sid & (P - 1);
+      const int rr = sid >> lp;
+      if (__any_sync(0xFFFFFFFFu, rr < rows)) {
+        const int64_t row = blk * RT_BLOCK_T + r0 + rr;
+        const bool live = rr < rows;
+        constexpr int NSUB = K <= 4 ? 2 : 1;
+        TopK<K> sub[NSUB];
+        const int rq = (r0 + rr) & (RT_BLOCK_T - 1);
+#pragma unroll 1
+        for (int e0 = part; e0 < p.E; e0 += P * NSUB * 4) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+#pragma unroll
+            for (int u = 0; u < NSUB; ++u) {        // the lists alternate: independent chains side by side
+              const int e = e0 + (j * NSUB + u) * P;
+              if (e < p.E) {
+                float x = mat[e * RT_MAT_LD + rq] + s_bias[e];
+                if (p.round_bf16) x = __bfloat162float(__float2bfloat16(x));
+                if (p.logits_out && live) p.logits_out[row * p.ld_logits + e] = x;
+                sub[u].push(x, e);
+              }
+            }
+          }
+        }
+        TopK<K> tk = sub[0];
+#pragma unroll
+        for (int u = 1; u < NSUB; ++u) tk.merge(sub[u].key, sub[u].idx);
+        tk.merge_lanes(P);
+        if (live && part == 0) rt_store_row<K>(p, row, tk);
+      }
+    }
+    __syncwarp();
+  }
+  if (p.splits > 1) cluster_barrier();                  // no CTA leaves while its logits are read
+
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols) : "memory");
@@ -310,7 +308,6 @@ int rt_make_map(const void* base, int64_t rows, int64_t K, int64_t ld, int box_r
 struct RouterPlan {
   int64_t blocks;
   int n_mma, KT, splits, stages;
-  size_t acc_off, ws_bytes;
 };
 
 RouterPlan rt_plan(int64_t T, int64_t K, int E) {
@@ -318,26 +315,23 @@ RouterPlan rt_plan(int64_t T, int64_t K, int E) {
   pl.blocks = cdiv64(T, RT_BLOCK_T);
   pl.n_mma = (E + 15) / 16 * 16;
   pl.KT = (int)cdiv64(K, 64);
-  // few token blocks: cut K so that many SMs pull a share of the operands.  Every slice adds a full block of partial
-  // logits to the scratch, so slices get longer as blocks get more: at least 2 k steps with one block, 12 from six on
-  int64_t s = moe_sm_count() / (pl.blocks > 0 ? pl.blocks : 1);
-  const int64_t min_steps = pl.blocks >= 6 ? 12 : 2 * pl.blocks;
-  if (s > pl.KT / min_steps) s = pl.KT / min_steps;
-  if (s < 1) s = 1;
-  pl.splits = (int)s;
+  // Few token blocks: cut K so that many SMs pull a share of the operands, into the 2, 4 or 8 CTAs of a cluster, two k steps each at
+  // least.  (Clusters of eight have an SM to a CTA only up to some 14 at a time: with 16, 2048 tokens took 37.9 us with the sort behind
+  // it, 26 with slices of four.)
+  int s = 1;
+  while (s < 8 && 2 * s * pl.blocks <= (s == 4 ? moe_sm_count() * 3 / 4 : moe_sm_count()) && pl.KT >= 4 * s) s *= 2;
+  pl.splits = s;
   const int stage_bytes = RT_BLOCK_T * 128 + ((pl.n_mma * 128 + 1023) & ~1023);
   int st = (200 * 1024) / stage_bytes;
   pl.stages = st > RT_STAGES_MAX ? RT_STAGES_MAX : st;
-  pl.acc_off = (size_t)((pl.blocks * 4 + 255) / 256 * 256);
-  pl.ws_bytes = pl.splits > 1 ? pl.acc_off + (size_t)pl.blocks * RT_BLOCK_T * pl.n_mma * 4 : 0;
   return pl;
 }
 
 }  // namespace
 
 extern "C" __attribute__((visibility("default"))) size_t moe_router_topk_workspace_bytes(int64_t T, int64_t K, int E) {
-  if (T <= 0 || K <= 0 || E <= 0) return 0;
-  return rt_plan(T, K, E).ws_bytes;
+  (void)T; (void)K; (void)E;
+  return 0;                                             // the partial sums stay on chip
 }
 
 extern "C" __attribute__((visibility("default"))) int moe_router_topk(
@@ -369,24 +363,29 @@ extern "C" __attribute__((visibility("default"))) int moe_router_topk(
   p.vals = vals; p.vals_dtype = vals_dtype; p.ld_vals = ld_vals;
   p.indx = indx; p.ld_indx = ld_indx;
   p.bitmatrix = bitmatrix; p.bm_stride_row = bm_stride_row; p.bm_stride_word = bm_stride_word;
-  p.acc = nullptr; p.counters = nullptr; p.status = status;
-  if (pl.splits > 1) {
-    MOE_CHECK_ARG(workspace && workspace_bytes >= pl.ws_bytes && (uintptr_t)workspace % 16 == 0,
-                  "moe_router_topk: needs a 16-byte aligned workspace of moe_router_topk_workspace_bytes() = %lld bytes (got %lld)",
-                  (long long)pl.ws_bytes, (long long)workspace_bytes);
-    p.counters = (int32_t*)workspace;
-    p.acc = (float*)((uint8_t*)workspace + pl.acc_off);
-  }
+  p.status = status;
+  (void)workspace; (void)workspace_bytes;
   CUtensorMap x_map, w_map;
   if (int rc = rt_make_map(x, T, K, ld_x, RT_BLOCK_T, &x_map)) return rc;
   if (int rc = rt_make_map(wg_t, E, K, ld_wg, pl.n_mma, &w_map)) return rc;
   const int stage_bytes = RT_BLOCK_T * 128 + ((pl.n_mma * 128 + 1023) & ~1023);
   const int smem = pl.stages * stage_bytes + 1024;
-  const dim3 grid((unsigned)pl.blocks, (unsigned)pl.splits);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)pl.blocks, (unsigned)pl.splits);
+  cfg.blockDim = dim3(RT_THREADS);
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = 1; at[1].val.clusterDim.y = (unsigned)pl.splits; at[1].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = pl.splits > 1 ? 2 : 1;
 #define RT_LAUNCH(KK)                                                                                                    \
   do {                                                                                                                   \
     MOE_CHECK_CUDA(cudaFuncSetAttribute(router_topk_kernel<KK>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));     \
-    MOE_CHECK_CUDA(launch_pdl(router_topk_kernel<KK>, grid, dim3(RT_THREADS), smem, st, p, x_map, w_map));               \
+    MOE_CHECK_CUDA(cudaLaunchKernelEx(&cfg, router_topk_kernel<KK>, p, x_map, w_map));                                   \
   } while (0)
   switch (k) {
     case 1: RT_LAUNCH(1); break;

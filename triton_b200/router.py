@@ -47,20 +47,12 @@ def router_topk(x: torch.Tensor, wg: torch.Tensor, bg, k: int, apply_softmax: bo
     if not router_topk_supported(x, wg, k):
         logits = (x.float() @ wg.float() + (0 if bg is None else bg.float())).to(logits_dtype)
         return _two_steps(logits, k, apply_softmax, return_logits)
-    lib = _lib.load()
-    T, K = x.shape
-    E = wg.shape[1]
+    T, E = x.shape[0], wg.shape[1]
     dev = x.device
     logits = torch.empty((T, E), dtype=torch.float32, device=dev) if return_logits else None
-    ws_bytes = lib.moe_router_topk_workspace_bytes(T, K, E)
-    ws = _lib.zero_scratch(dev, ws_bytes) if ws_bytes > 0 else None
-    if ws_bytes > 0 and ws is None:
-        # no zeroed scratch to be had now (first use inside a graph capture): the two steps apart
-        logits = torch.addmm(bg.to(x.dtype), x, wg) if bg is not None else x @ wg
-        return _two_steps(logits.to(logits_dtype), k, apply_softmax, return_logits)
     if bg is not None and bg.dtype not in (torch.float32, torch.bfloat16):
         bg = bg.float()
-    vals, indx, bm = _lib.host().router(x, wg, bg, k, bool(apply_softmax), logits_dtype == torch.bfloat16, logits, ws, ws_bytes,
+    vals, indx, bm = _lib.host().router(x, wg, bg, k, bool(apply_softmax), logits_dtype == torch.bfloat16, logits, None, 0,
                                         _status_word(dev))
     sp = SparseMatrix(indx=indx, vals=vals, mask=bit_tensor(bm, T, E))
     return (sp, logits) if return_logits else sp

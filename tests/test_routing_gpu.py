@@ -252,6 +252,22 @@ def test_routing_in_one_cluster(T, E, k, device):
     assert torch.equal(gather.cpu().int(), (col // k).int())
 
 
+@pytest.mark.parametrize("T, E, k", [(257, 20, 3), (2049, 128, 4), (8193, 200, 6), (8300, 256, 8), (8321, 256, 8), (18176, 32, 1), (18305, 32, 1), (300, 256, 40)])
+def test_routing_in_two_launches(T, E, k, device):
+    """Either side of where the blocks that rank also add up the counts (their number and the length of a block's list decide), k that the quad
+    top-k does not take, entries of several rounds per warp, a last block of one token."""
+    torch.manual_seed(T + E)
+    logits = torch.randn(T, E)
+    ragged, gather, scatter, sp = routing(logits.to(device), k)
+    _, indx, _ = oracle.topk_oracle(logits, k, True)
+    col_sum, col, row = oracle.bitmatrix_metadata_oracle(indx, E)
+    md = sp.mask_metadata
+    assert torch.equal(md.col_sum.cpu(), col_sum) and torch.equal(md.col_sorted_indx.cpu(), col) and torch.equal(md.row_sorted_indx.cpu(), row)
+    offs, block_offs, sched = oracle.ragged_metadata_oracle(col_sum, T * k)
+    assert torch.equal(ragged.slice_offs.cpu(), offs) and torch.equal(ragged.block_offs_data.cpu(), block_offs)
+    assert torch.equal(ragged.block_schedule_data.cpu(), sched)
+
+
 @pytest.mark.parametrize("call", ["row count", "reduce output", "router weight", "router bias"])
 def test_host_tensors_are_refused(call, device):
     """A tensor in host memory beside device tensors is refused, not handed to a kernel."""

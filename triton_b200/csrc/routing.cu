@@ -760,7 +760,7 @@ extern "C" __attribute__((visibility("default"))) int moe_ragged_metadata_remap(
 }
 
 // ---------------------------------------------------------------------------------------------------------
-// moe_route: the whole routing step in three launches (the standalone entry points above take five); small batches in one launch of five
+// moe_route: the whole routing step in two or three launches (the standalone entry points above take more); small batches in one launch of five
 // independent blocks (route_small_kernel), those of up to some 1500 tokens in one launch of a cluster of eight (route_cluster_kernel,
 // both at the end of this section; rule: route_form).
 //   A  topk_quad_kernel<HIST>   top-k + softmax + bitmatrix row of every token, and the expert histogram of each block
@@ -973,6 +973,121 @@ __global__ void __launch_bounds__(1024) route_scan_ragged_kernel(const int32_t* 
   // ---- 2. expert offsets, then the ragged metadata: row 0 = slice_offs (= col_offs), rows 1..4 = block sizes 16..128 --
   ragged_row(role - 1, s_size, E, s_nb, s_offs, s_warp, slice_offs, col_offs, block_offs, ld_block_offs, block_sched, ld_sched,
              n_sched);
+}
+
+// Second and last launch of batches whose blocks are a wave: blocks 0 .. n_blocks - 1 add up the counts of the blocks before theirs and
+// of all (64 KB for 16384 tokens and 128 experts, from L2) and rank their entries, five more build the ragged metadata.  With the sums in a
+// launch between (route_scan_ragged_kernel) 2049 tokens of 128 experts, k = 4, took 15.2 us and 16384 18.2, so 11.6 and 16.6; past a wave of
+// blocks (24576: 23.9 and 27.5) and for long lists per block (200 experts, k = 6: 8192 tokens 39.0 and 33.2, 16384 43.4 and 51.4) it stays.
+__global__ void __launch_bounds__(1024) route_finish_kernel(const int16_t* indx, int64_t ld_indx, int64_t T_rows, int E, int k, const int32_t* partial,
+                                                            int n_blocks, int32_t* col_sum, int32_t* col_sorted, int32_t* row_sorted,
+                                                            int32_t* slice_offs, int32_t* block_offs, int64_t ld_block_offs,
+                                                            int32_t* block_sched, int64_t ld_sched, int64_t n_sched, const PerPosition out) {
+  // [1024] segment sums, [1024] of them before this block, [E + 1] sizes, [E + 1] scan input, [E + 1] offsets, [E] entries before,
+  // [warps in use][E] counters, [entries] experts (int16)
+  extern __shared__ int32_t s_mem[];
+  __shared__ int32_t s_warp[33];
+  pdl_begin();
+  int32_t* s_tot = s_mem;
+  int32_t* s_bef = s_tot + 1024;
+  int32_t* s_size = s_bef + 1024;
+  int32_t* s_nb = s_size + (E + 1);
+  int32_t* s_offs = s_nb + (E + 1);
+  int32_t* s_before = s_offs + (E + 1);
+  int32_t* s_cnt = s_before + E;
+  const int own = (int)blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool ranks = own < n_blocks;
+  const int64_t tok0 = (int64_t)own * kRouteTokPerBlock;
+  const int n = ranks ? (int)min((int64_t)kRouteTokPerBlock, T_rows - tok0) * k : 0;
+  const int rounds = (kRouteTokPerBlock * k + 1023) >> 10, per = rounds * 32, warps = (kRouteTokPerBlock * k + per - 1) / per;
+  int16_t* s_pick = reinterpret_cast<int16_t*>(s_cnt + warps * E);
+  // ---- counts of an expert, by S segments of blocks ----
+  int Ep = 1;
+  while (Ep < E) Ep <<= 1;
+  const int S = 1024 / Ep, e = threadIdx.x % Ep, seg = threadIdx.x / Ep;
+  const int seg_blocks = (n_blocks + S - 1) / S, lo = min(seg * seg_blocks, n_blocks), hi = min(lo + seg_blocks, n_blocks);
+  int tot = 0, bef = 0;
+  if (e < E)
+    for (int b0 = lo; b0 < hi; b0 += 16) {
+      int v[16];
+#pragma unroll
+      for (int u = 0; u < 16; ++u) v[u] = b0 + u < hi ? partial[(int64_t)(b0 + u) * E + e] : 0;
+#pragma unroll
+      for (int u = 0; u < 16; ++u) {
+        tot += v[u];
+        if (b0 + u < own) bef += v[u];
+      }
+    }
+  s_tot[threadIdx.x] = tot;
+  s_bef[threadIdx.x] = bef;
+  for (int j = threadIdx.x; j < n; j += blockDim.x) {
+    const int token = j / k;
+    s_pick[j] = indx[(tok0 + token) * ld_indx + (j - token * k)];
+  }
+  for (int i = threadIdx.x; i < warps * E; i += blockDim.x) s_cnt[i] = 0;
+  __syncthreads();
+  if (seg == 0 && e < E) {
+    int total = 0, before = 0;
+    for (int i = 0; i < S; ++i) {
+      total += s_tot[i * Ep + e];
+      before += s_bef[i * Ep + e];
+    }
+    s_size[e] = total;
+    s_before[e] = before;
+  }
+  if (threadIdx.x == 0) s_size[E] = 0;
+  int32_t* my = s_cnt + warp * E;
+  if (ranks && warp < warps)
+    for (int r = 0; r < rounds; ++r) {
+      const int j = warp * per + r * 32 + lane, c = j < n ? s_pick[j] : -1;
+      const unsigned peers = __match_any_sync(0xFFFFFFFFu, c);
+      if (c >= 0 && (peers & ((1u << lane) - 1u)) == 0) my[c] += __popc(peers);
+      __syncwarp();
+    }
+  __syncthreads();
+  if (!ranks) {
+    if (own == n_blocks)
+      for (int i = threadIdx.x; i < E; i += blockDim.x) col_sum[i] = s_size[i];
+    ragged_row(own - n_blocks, s_size, E, s_nb, s_offs, s_warp, slice_offs, nullptr, block_offs, ld_block_offs, block_sched, ld_sched, n_sched);
+    return;
+  }
+  // ---- stable expert-major positions: a warp ranks `per` entries in order, on top of the counts of the warps and blocks before it ----
+  block_exclusive_scan(s_size, s_offs, E, s_warp);
+  for (int i = threadIdx.x; i < E; i += blockDim.x) {
+    int run = s_offs[i] + s_before[i];
+    for (int w0 = 0; w0 < warps; w0 += 8) {
+      int v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = w0 + u < warps ? s_cnt[(w0 + u) * E + i] : 0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        if (w0 + u < warps) s_cnt[(w0 + u) * E + i] = run;
+        run += v[u];
+      }
+    }
+  }
+  __syncthreads();
+  if (warp < warps)
+    for (int r = 0; r < rounds; ++r) {
+      const int j = warp * per + r * 32 + lane, c = j < n ? s_pick[j] : -1;
+      const unsigned peers = __match_any_sync(0xFFFFFFFFu, c);
+      const int before = __popc(peers & ((1u << lane) - 1u));
+      const int base = c >= 0 ? my[c] : 0;
+      __syncwarp();
+      if (c >= 0 && before == 0) my[c] = base + __popc(peers);
+      __syncwarp();
+      if (c >= 0) {
+        const int pos = base + before;
+        const int64_t flat = tok0 * k + j;
+        row_sorted[flat] = pos;
+        col_sorted[pos] = (int32_t)flat;
+        if (out.token) {
+          const int64_t token = tok0 + j / k;
+          out.token[pos] = (int32_t)token;
+          if (out.weight) out.weight[pos] = out.vals[token * out.ld_vals + j % k];
+        }
+      }
+    }
 }
 
 // The whole routing step of a small batch (at most 256 tokens, at most 256 experts, k in {1, 2, 4, 8, 16}; see route_form) in ONE launch
@@ -1315,6 +1430,14 @@ static int route_launch(
   }
 #undef MOE_ROUTE_QUAD
   MOE_CHECK_LAUNCH();
+  const int entries = kRouteTokPerBlock * k, warps = entries / 32 < 32 ? entries / 32 : 32;
+  const size_t smem_f = (size_t)(2048 + 3 * (E + 1) + E + warps * E) * sizeof(int32_t) + (size_t)entries * sizeof(int16_t);
+  if (nb + 5 <= (E * k <= 1024 ? moe_sm_count() : 69) && smem_f <= 48 * 1024) {
+    MOE_CHECK_CUDA(launch_pdl(route_finish_kernel, dim3((unsigned)nb + 5), dim3(1024), smem_f, st, indx, ld_indx, T, E, k, partial, (int)nb, col_sum,
+                              col_sorted, row_sorted, slice_offs, block_offs, ld_block_offs, block_sched, ld_sched, n_sched, out));
+    MOE_CHECK_LAUNCH();
+    return MOE_OK;
+  }
   const size_t smem_b = (size_t)(1024 + 3 * (E + 1)) * sizeof(int32_t);
   MOE_CHECK_CUDA(launch_pdl(route_scan_ragged_kernel, dim3(6), dim3(1024), smem_b, st, partial, scanned, nb, E, col_sum, col_offs,
                             slice_offs, block_offs, ld_block_offs, block_sched, ld_sched, n_sched));

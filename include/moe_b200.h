@@ -80,16 +80,16 @@ int moe_topk_fwd(const void* logits, int dtype, int64_t T, int E, int k, int app
 /* Replaces tensor_details/bitmatrix.py:110-150 (make_bitmatrix_metadata: sum_bitmatrix_rows +
  * stage1 + stage2): histogram col_sum[E], col_sorted_indx[T*k], row_sorted_indx[T*k] (stable
  * counting sort of the flat (token,slot) entries by expert; -1 padded).
- * workspace: moe_bitmatrix_metadata_workspace(T, E, k) bytes of device scratch.                    */
+ * workspace: moe_bitmatrix_metadata_workspace(T, E, k) bytes of device scratch (not used up to 32768 entries of 256 experts). */
 size_t moe_bitmatrix_metadata_workspace(int64_t T, int E, int k);
 int moe_bitmatrix_metadata(const int16_t* indx, int64_t ld_indx, int64_t T, int E, int k,
                            const int32_t* n_rows_dev, int32_t* col_sum, int32_t* col_sorted,
                            int32_t* row_sorted, void* workspace, size_t workspace_bytes, void* stream);
 
-/* The whole routing step of a layer in three launches (one for up to 256 tokens): moe_topk_fwd +
+/* The whole routing step of a layer in one launch (up to some 1500 tokens) to three: moe_topk_fwd +
  * moe_bitmatrix_metadata + moe_ragged_metadata (topk.py:106-141 -> tensor.py:202-209 -> ragged_tensor.py:183-210 of the
  * reference, what its test helper `routing` composes, tests/test_distributed.py:203-210) with the expert histogram taken
- * in the top-k pass and the ragged metadata built beside the scan of the histograms.  Every one of the T rows is valid (no device-side row
+ * in the top-k pass and the ragged metadata built beside the sort.  Every one of the T rows is valid (no device-side row
  * bound, no provided indices); n_expts <= 256, otherwise MOE_ERR_UNSUPPORTED and the caller uses the separate entry
  * points.  Outputs as for those entry points; workspace of moe_route_workspace(T, n_expts, k) bytes.               */
 size_t moe_route_workspace(int64_t T, int E, int k);
@@ -121,11 +121,9 @@ int moe_route_positions(const float* logits, int64_t T, int E, int k, int apply_
  *   round_bf16: round every logit to bf16 before the selection (what a bf16 router output does in the two-step form).
  *   logits_out: NULL, or [T, E] fp32 that receives the logits the selection saw.
  *   vals [T, k] fp32 or bf16, indx, bitmatrix: as for moe_topk_fwd.
- * With few tokens K is cut into slices over the SMs and the partial logits meet in `workspace`
- * (moe_router_topk_workspace_bytes, 16-byte aligned): it must be ALL ZERO when the call starts and the call leaves it
- * all zero again, so one cudaMemset after allocating it serves every later call on the same stream (calls that share a
- * workspace must not overlap; clear it again after a call that reported a device status).  The fp32 sums of the slices
- * are formed in no fixed order.  A bounded wait that expires writes 801..804 to *status.                            */
+ * With few tokens K is cut into slices over the SMs of a cluster, whose partial logits meet in shared memory, in a fixed order: no
+ * workspace is needed (moe_router_topk_workspace_bytes is 0; what is passed is not touched).  A bounded wait that expires writes 801..804
+ * to *status.                                                                                                       */
 size_t moe_router_topk_workspace_bytes(int64_t T, int64_t K, int E);
 int moe_router_topk(const void* x, int64_t T, int64_t K, int64_t ld_x, const void* wg_t, int64_t ld_wg,
                     const void* bias, int bias_dtype, int E, int k, int apply_softmax, int round_bf16,

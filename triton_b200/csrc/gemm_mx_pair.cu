@@ -8,7 +8,7 @@
 //
 // (Elements far below their group of 32's largest lose what lies below 2^-23 of it, as much as an fp32 sum rounds away.)
 // A row with a value beyond e4m3's scales (infinite, or near the end of bf16's range) is computed by the pack kernel in fp32, and
-// the GEMM kernel does not store it.  (The pack kernel's word per 16 rows and its look-up cost about 1 us of 183 for fc1 + fc2 of 32
+// the GEMM kernel does not store it.  (The pack kernel's mark per row and its look-up cost about 1 us of 183 for fc1 + fc2 of 32
 // experts, 300 tokens; the same recomputation called from this kernel's epilogue took 7, by the code the call made of the rest.)
 //
 // What bounds it.  Shared memory, 128 B per cycle and SM: every operand byte is written once and read once per MMA, and an

@@ -17,7 +17,7 @@ struct Lib {
 #define MOE_HOST_FUNCTIONS(X)                                                                                            \
   X(moe_last_error) X(moe_route) X(moe_route_positions) X(moe_route_workspace) X(moe_grouped_gemm) X(moe_gemm_mx_workspace_bytes) \
   X(moe_reduce) X(moe_downcast_mxfp4) X(moe_upcast_mxfp4) X(moe_bitmatrix_metadata) X(moe_bitmatrix_metadata_workspace) \
-  X(moe_router_topk) X(moe_router_topk_workspace_bytes) X(moe_copy2) \
+  X(moe_router_topk) X(moe_copy2) \
   X(moe_gemm_kernel_name) X(moe_grouped_gemm_chain)
 #define X(name) decltype(&::name) name = nullptr;
   MOE_HOST_FUNCTIONS(X)
@@ -410,9 +410,9 @@ Tensor reduce(const Tensor& x, int64_t dim, const OptTensor& y_, py::object y_dt
 }
 
 // ---- router --------------------------------------------------------------------------------------------------------
-// -> vals, indx, bitmatrix view; wg in the kernel's memory order, `scratch` zero and large enough (or None)
+// -> vals, indx, bitmatrix view; wg in the kernel's memory order
 py::tuple router(const Tensor& x, const Tensor& wg, const OptTensor& bg, int64_t k, bool softmax, bool round_bf16, const OptTensor& logits,
-                 const OptTensor& scratch, int64_t scratch_bytes, const Tensor& status) {
+                 const Tensor& status) {
   need_cuda(x); need_cuda(wg);
   if (bg) need_cuda(*bg);
   const int64_t T = x.size(0), K = x.size(1), E = wg.size(1);
@@ -423,8 +423,7 @@ py::tuple router(const Tensor& x, const Tensor& wg, const OptTensor& bg, int64_t
     check(lib.moe_router_topk(x.data_ptr(), T, K, x.stride(0), wg.data_ptr(), wg.stride(1), bg ? bg->data_ptr() : nullptr,
                               bg ? dtype_code(*bg) : 0, (int)E, (int)k, softmax, round_bf16, logits ? logits->data_ptr<float>() : nullptr, E,
                               vals.data_ptr(), dtype_code(vals), k, indx.data_ptr<int16_t>(), k, (uint32_t*)bm.data_ptr(), bm.stride(0),
-                              bm.stride(1), scratch ? scratch->data_ptr() : nullptr, scratch ? (size_t)scratch_bytes : 0,
-                              status.data_ptr<int32_t>(), stream()),
+                              bm.stride(1), nullptr, 0, status.data_ptr<int32_t>(), stream()),
           "moe_router_topk");
   return py::make_tuple(vals, indx, bm);
 }

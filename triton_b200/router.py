@@ -52,7 +52,6 @@ def router_topk(x: torch.Tensor, wg: torch.Tensor, bg, k: int, apply_softmax: bo
     logits = torch.empty((T, E), dtype=torch.float32, device=dev) if return_logits else None
     if bg is not None and bg.dtype not in (torch.float32, torch.bfloat16):
         bg = bg.float()
-    vals, indx, bm = _lib.host().router(x, wg, bg, k, bool(apply_softmax), logits_dtype == torch.bfloat16, logits, None, 0,
-                                        _status_word(dev))
+    vals, indx, bm = _lib.host().router(x, wg, bg, k, bool(apply_softmax), logits_dtype == torch.bfloat16, logits, _status_word(dev))
     sp = SparseMatrix(indx=indx, vals=vals, mask=bit_tensor(bm, T, E))
     return (sp, logits) if return_logits else sp

@@ -49,9 +49,8 @@ template <bool VEC> __device__ __forceinline__ uint4 load_group(const uint8_t* s
 // group), four neighbouring lanes the 64 bytes of a row.  SCALED: the block-scaled layout (tiles [E][k_tile][n_block],
 // rows of 64 bytes as they are), else [E][n_tile][k_tile] with the [group][row] order and interleaved nibbles described above.
 template <bool SCALED, bool VEC>
-__global__ void __launch_bounds__(256) to_tiles_values(const uint8_t* q, int64_t q_stride_e, int64_t q_stride_n,
-                                                       int E, int K, int N, int NT, int KT, uint4* out) {
-  pdl_begin();
+__global__ void __launch_bounds__(256) to_tiles_values(const uint8_t* __restrict__ q, int64_t q_stride_e, int64_t q_stride_n,
+                                                       int E, int K, int N, int NT, int KT, uint4* __restrict__ out) {
   const int64_t tiles = (int64_t)E * NT * KT;
   for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
     const int kt = SCALED ? (int)(tile / NT % KT) : (int)(tile % KT);
@@ -77,9 +76,8 @@ __global__ void __launch_bounds__(256) to_tiles_values(const uint8_t* q, int64_t
 // lone bytes at the pitch of a row (16 x 2880 x 5760: 15.5 us, so 8.5).  MX: the block-scaled order [E][k step][block].
 constexpr int SCALE_ROWS_SMEM = 48 * 1024;
 template <bool MX>
-__global__ void __launch_bounds__(256) scales_from_rows(const uint8_t* s, int64_t s_stride_e, int groups, int N, int NB, int KT,
-                                                        uint32_t* out) {
-  pdl_begin();
+__global__ void __launch_bounds__(256) scales_from_rows(const uint8_t* __restrict__ s, int64_t s_stride_e, int groups, int N, int NB, int KT,
+                                                        uint32_t* __restrict__ out) {
   extern __shared__ uint32_t s_words[];              // [rows][groups] bytes
   const int nb = blockIdx.x % NB, e = blockIdx.x / NB, rows = min(TN, N - nb * TN);
   const uint8_t* src = s + (int64_t)e * s_stride_e + (int64_t)nb * TN * groups;       // 4-byte aligned: TN is a multiple of 4
@@ -104,12 +102,12 @@ __global__ void __launch_bounds__(256) scales_from_rows(const uint8_t* s, int64_
 // false: the scales are laid out in some other way
 template <bool MX>
 bool launch_scales_from_rows(const uint8_t* s, int64_t s_stride_e, int64_t s_stride_k, int64_t s_stride_n, int E, int K, int N, int NB, int KT,
-                             uint32_t* out, cudaStream_t st, cudaError_t& err) {
+                             uint32_t* out, cudaStream_t st) {
   const int groups = K / 32, smem = TN * groups;
   if (K % 32 || s_stride_k != 1 || s_stride_n != groups || s_stride_e % 4 || (uintptr_t)s % 4 || smem > SCALE_ROWS_SMEM ||
       (int64_t)E * NB >= 2147483647LL)
     return false;
-  err = launch_pdl(scales_from_rows<MX>, dim3((unsigned)(E * NB)), dim3(256), smem, st, s, s_stride_e, groups, N, NB, KT, out);
+  scales_from_rows<MX><<<(unsigned)(E * NB), 256, smem, st>>>(s, s_stride_e, groups, N, NB, KT, out);
   return true;
 }
 
@@ -161,13 +159,14 @@ __global__ void __launch_bounds__(256) from_b200_kernel(const uint32_t* __restri
 }
 
 template <bool SCALED>
-cudaError_t launch_to_tiles(const uint8_t* q, int64_t q_stride_e, int64_t q_stride_n, int E, int K, int N, int NT, int KT, uint8_t* out,
+void launch_to_tiles(const uint8_t* q, int64_t q_stride_e, int64_t q_stride_n, int E, int K, int N, int NT, int KT, uint8_t* out,
                      cudaStream_t st) {
   const int64_t tiles = (int64_t)E * NT * KT, cap = (int64_t)moe_sm_count() * 32;
   const int grid = (int)(tiles < cap ? tiles : cap);
   if ((uintptr_t)q % 16 == 0 && q_stride_e % 16 == 0 && q_stride_n % 16 == 0)
-    return launch_pdl(to_tiles_values<SCALED, true>, dim3(grid), dim3(256), 0, st, q, q_stride_e, q_stride_n, E, K, N, NT, KT, (uint4*)out);
-  return launch_pdl(to_tiles_values<SCALED, false>, dim3(grid), dim3(256), 0, st, q, q_stride_e, q_stride_n, E, K, N, NT, KT, (uint4*)out);
+    to_tiles_values<SCALED, true><<<grid, 256, 0, st>>>(q, q_stride_e, q_stride_n, E, K, N, NT, KT, (uint4*)out);
+  else
+    to_tiles_values<SCALED, false><<<grid, 256, 0, st>>>(q, q_stride_e, q_stride_n, E, K, N, NT, KT, (uint4*)out);
 }
 
 int grid_for(int64_t total) {
@@ -198,15 +197,13 @@ extern "C" __attribute__((visibility("default"))) int moe_weight_layout_to_b200(
   const int NT = (int)cdiv64(N, TN), KT = (int)cdiv64(K, TK);
   cudaStream_t st = (cudaStream_t)stream;
   if (q) {
-    MOE_CHECK_CUDA(launch_to_tiles<false>(q, q_stride_e, q_stride_n, E, K, N, NT, KT, out_values, st));
+    launch_to_tiles<false>(q, q_stride_e, q_stride_n, E, K, N, NT, KT, out_values, st);
     MOE_CHECK_LAUNCH();
   }
   if (scale) {
-    cudaError_t err = cudaSuccess;
-    if (!launch_scales_from_rows<false>(scale, s_stride_e, s_stride_k, s_stride_n, E, K, N, NT, KT, (uint32_t*)out_scales, st, err))
+    if (!launch_scales_from_rows<false>(scale, s_stride_e, s_stride_k, s_stride_n, E, K, N, NT, KT, (uint32_t*)out_scales, st))
       to_b200_scales<<<grid_for((int64_t)E * NT * KT * TN), 256, 0, st>>>(scale, s_stride_e, s_stride_k, s_stride_n, E, K,
                                                                          N, NT, KT, (uint32_t*)out_scales);
-    MOE_CHECK_CUDA(err);
     MOE_CHECK_LAUNCH();
   }
   return MOE_OK;
@@ -296,15 +293,13 @@ extern "C" __attribute__((visibility("default"))) int moe_weight_layout_to_b200m
   const int NB = (int)cdiv64(N, TN), KT = (int)cdiv64(K, TK);
   cudaStream_t st = (cudaStream_t)stream;
   if (q) {
-    MOE_CHECK_CUDA(launch_to_tiles<true>(q, q_stride_e, q_stride_n, E, K, N, NB, KT, out_values, st));
+    launch_to_tiles<true>(q, q_stride_e, q_stride_n, E, K, N, NB, KT, out_values, st);
     MOE_CHECK_LAUNCH();
   }
   if (scale) {
-    cudaError_t err = cudaSuccess;
-    if (!launch_scales_from_rows<true>(scale, s_stride_e, s_stride_k, s_stride_n, E, K, N, NB, KT, (uint32_t*)out_scales, st, err))
+    if (!launch_scales_from_rows<true>(scale, s_stride_e, s_stride_k, s_stride_n, E, K, N, NB, KT, (uint32_t*)out_scales, st))
       to_b200mx_scales<<<grid_for((int64_t)E * NB * KT * TN), 256, 0, st>>>(scale, s_stride_e, s_stride_k, s_stride_n, E, K,
                                                                            N, NB, KT, (uint32_t*)out_scales);
-    MOE_CHECK_CUDA(err);
     MOE_CHECK_LAUNCH();
   }
   return MOE_OK;

@@ -206,9 +206,8 @@ template <> __device__ __forceinline__ float2 pair_absmax<float>(const float2 (&
 
 template <typename T>
 __global__ void __launch_bounds__(256, sizeof(T) == 2 ? 4 : 2) downcast_cols_kernel(
-    const T* x, int64_t outer, int groups, int col_blocks, int group_blocks, int64_t sx_batch, int64_t sx_quant,
-    uint8_t* q, uint8_t* scale, int mode) {
-  pdl_begin();
+    const T* __restrict__ x, int64_t outer, int groups, int col_blocks, int group_blocks, int64_t sx_batch, int64_t sx_quant,
+    uint8_t* __restrict__ q, uint8_t* __restrict__ scale, int mode) {
   using Raw = typename Pair<T>::Raw;
   __shared__ __align__(16) uint8_t s_q[CT_GROUPS * CT_PITCH];
   __shared__ uint8_t s_s[CT_COLS * CT_GROUPS];
@@ -549,9 +548,9 @@ extern "C" __attribute__((visibility("default"))) int moe_downcast_mxfp4(const v
                                   (const T*)x, batch * outer, quant, outer, sx_batch, sx_outer, q, scale, rounding_mode));
     } else if (cols_ok) {
       const int groups = (int)(quant >> 5);
-      MOE_CHECK_CUDA(launch_pdl(downcast_cols_kernel<T>, dim3((unsigned)col_tiles(batch, outer, quant)), dim3(256), 0, st, (const T*)x,
-                                outer, groups, (int)cdiv64(outer, CT_COLS), (int)cdiv64(groups, CT_GROUPS), sx_batch, sx_quant, q,
-                                scale, rounding_mode));
+      downcast_cols_kernel<T><<<(unsigned)col_tiles(batch, outer, quant), 256, 0, st>>>(
+          (const T*)x, outer, groups, (int)cdiv64(outer, CT_COLS), (int)cdiv64(groups, CT_GROUPS), sx_batch, sx_quant, q, scale,
+          rounding_mode);
     } else {
       MOE_CHECK_ARG((uintptr_t)q % 16 == 0, "moe_downcast_mxfp4: q must be 16-byte aligned");
       const int64_t total = batch * outer * (quant >> 5);

@@ -111,7 +111,35 @@ def test_router_topk_against_reference_fixture(golden, name, device):
     assert (sp.vals.cpu().float()[same] - g["vals"].float()[same]).abs().max().item() <= 2.0 ** -8
 
 
-@pytest.mark.parametrize("case", [(129, 2880, 128, 4), (131, 512, 20, 2), (137, 1024, 256, 8), (1800, 512, 64, 4), (4100, 320, 100, 4), (8000, 576, 16, 2)])
+@pytest.mark.parametrize("case", [(129, 2880, 128, 4), (131, 512, 20, 2), (137, 1024, 256, 8), (386, 1024, 64, 4), (4100, 1536, 100, 4), (8000, 1536, 16, 2)])
 def test_router_topk_slices_of_a_cluster(case, device):
-    """2, 4 and 8 slices of K per token block, last blocks of 1, 3, 9, 4 and 64 rows: shares of the rows that are empty or partial."""
+    """2 to 11 slices of K per token block, last blocks of 1, 3, 9, 2, 4 and 64 rows: shares of the rows that are empty or partial."""
     test_router_topk_against_oracle(case, torch.float32, True, device)
+
+
+@pytest.mark.parametrize("T, K, E, slices", [(1, 4096, 256, 32), (64, 2880, 128, 22), (200, 2880, 48, 11), (300, 2880, 100, 7), (1000, 2880, 128, 3),
+                                             (6000, 2880, 32, 3), (8000, 1600, 16, 2), (700, 512, 64, 1)])
+def test_router_logits_are_the_sums_of_their_slices(T, K, E, slices, device):
+    """Bit for bit: K is cut into this many slices and no other, each is summed as the product of its own columns, and the slices are added
+    in their order, first those of a CTA (eight at most).  The cut decides how far the logits are from the exact ones."""
+    if torch.cuda.get_device_properties(device).multi_processor_count != 148:
+        pytest.skip("the number of slices goes by the SMs")
+    x, wg, _ = make(T, K, E, T + K + E, False)
+    x, wg = x.to(device), tb.prepare_router_weight(wg.to(device))
+
+    def logits(x, wg):
+        return tb.router_topk(x, wg, None, 1, logits_dtype=torch.float32, return_logits=True)[1]
+
+    got = logits(x, wg)
+    if slices == 1:
+        ref = logits(torch.cat([x, x[:1].expand(9600 - T, K)]), wg)[:T]           # 75 token blocks: K is not cut
+    else:
+        ctas, steps, ref = min(slices, 8), (K + 63) // 64, 0
+        k = [64 * (steps * i // slices) for i in range(slices)] + [K]
+        for c in range(ctas):
+            own = 0
+            for i in range(slices * c // ctas, slices * (c + 1) // ctas):
+                own = own + logits(x[:, k[i]:k[i + 1]], wg[k[i]:k[i + 1]])
+            ref = ref + own
+    tb.matmul_check_status()
+    assert torch.equal(got, ref)

@@ -5,14 +5,15 @@
 // (triton_kernels bench/bench_mlp.py:70, topk.py:25-141); the selection rule, the softmax and the bitmatrix layout
 // are those of topk_details/_topk_forward.py:91-150 (largest value first, equal values to the smaller expert index).
 //
-// One CTA per (block of 128 tokens, slice of K).  Warp 0 streams x and Wg^T tiles (128 x 64 bf16 and E x 64 bf16, TMA,
+// One CTA per (block of 128 tokens, share of K).  Warp 0 streams x and Wg^T tiles (128 x 64 bf16 and E x 64 bf16, TMA,
 // 128-byte swizzle) through a ring of stages, warp 1 issues tcgen05.mma.kind::f16 (M = 128 tokens, N = E experts) into
 // one fp32 accumulator in tensor memory, warps 2-17 select: they spill the accumulator to shared memory and several
 // threads per token row add the bias and keep the k best in registers.  With few tokens K is cut into slices so that many SMs pull the
-// operands: the slices of a token block are a cluster, every CTA leaves its partial logits in its own shared memory, and behind a
-// cluster barrier each sums a share of the rows over all of them (distributed shared memory, in the order of the slices) and selects
-// for it.  (As partial sums in an fp32 scratch by red.global.add, with the selection in the CTA that came last: 4100 tokens of 2880 x 128
-// with the sort behind it 31.7 us, so 26.3; 128 tokens 25.0 and 21.4.)
+// operands: the slices of a token block are spread over a cluster, every CTA leaves the sum of its slices in its own shared memory, and
+// behind a cluster barrier each sums a share of the rows over all of them (distributed shared memory; everything in the order of the
+// slices) and selects for it.  With the sort behind it, K = 2880, 128 experts, in a graph: 1 token 15.1 us, 64 17.0, 1024 25.0, 4100 30.1,
+// 16384 39.5; as partial sums in an fp32 scratch by red.global.add, with the selection in the CTA that came last: 19.9, 23.9, 33.7, 35.7, 42.5.
+// What bounds it: an SM takes in 32 B a cycle, 32 KB a k step.
 // Every mbarrier wait is bounded.
 #include "gemm_tc_common.cuh"
 #include "topk_select.cuh"
@@ -27,7 +28,7 @@ constexpr int RT_BLOCK_T = 128;
 struct RouterParams {
   int64_t T;
   int E, n_mma, k, KT;            // experts, E rounded up to 16, picks per token, 64-k steps
-  int splits, stages;
+  int slices, splits, stages;     // of K, CTAs they are spread over
   int apply_softmax;
   int round_bf16;                 // logits rounded to bf16 before the selection (a bf16 router output, as the two-launch form has it)
   const void* bias; int bias_dtype;
@@ -89,7 +90,7 @@ router_topk_kernel(const RouterParams p, const __grid_constant__ CUtensorMap x_m
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const uint32_t sbase = smem_u32(smem);
   float* mat = reinterpret_cast<float*>(smem);
-  __shared__ __align__(8) uint64_t bars[2 * RT_STAGES_MAX + 1];
+  __shared__ __align__(8) uint64_t bars[2 * RT_STAGES_MAX + 4];
   __shared__ uint32_t s_tmem;
   __shared__ int s_abort;
   __shared__ float s_bias[256];
@@ -99,16 +100,21 @@ router_topk_kernel(const RouterParams p, const __grid_constant__ CUtensorMap x_m
   const uint32_t stage_bytes = X_BYTES + ((W_BYTES + 1023u) & ~1023u);
   auto BAR_FULL = [&](int s) { return smem_u32(&bars[s]); };
   auto BAR_EMPTY = [&](int s) { return smem_u32(&bars[RT_STAGES_MAX + s]); };
-  const uint32_t BAR_ACC = smem_u32(&bars[2 * RT_STAGES_MAX]);
+  auto BAR_ACC = [&](int a) { return smem_u32(&bars[2 * RT_STAGES_MAX + a]); };              // a slice's sums are complete
+  auto BAR_ACC_FREE = [&](int a) { return smem_u32(&bars[2 * RT_STAGES_MAX + 2 + a]); };     // and have been read
   Ctl ctl{&s_abort, p.status};
-  const uint32_t tmem_cols = p.n_mma <= 32 ? 32u : p.n_mma <= 64 ? 64u : p.n_mma <= 128 ? 128u : 256u;
+  const uint32_t acc_cols = p.n_mma <= 32 ? 32u : p.n_mma <= 64 ? 64u : p.n_mma <= 128 ? 128u : 256u;
+  const uint32_t tmem_cols = p.slices > p.splits ? 2u * acc_cols : acc_cols;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < RT_STAGES_MAX; ++s) {
       mbar_init(BAR_FULL(s), 1);
       mbar_init(BAR_EMPTY(s), 1);
     }
-    mbar_init(BAR_ACC, 1);
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(BAR_ACC(a), 1);
+      mbar_init(BAR_ACC_FREE(a), 16);
+    }
     s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -128,22 +134,25 @@ router_topk_kernel(const RouterParams p, const __grid_constant__ CUtensorMap x_m
 
   const int64_t blk = blockIdx.x;
   const int split = blockIdx.y;                 // rank in the cluster of a token block's slices
-  const int kt0 = (int)((int64_t)p.KT * split / p.splits), kt1 = (int)((int64_t)p.KT * (split + 1) / p.splits);
-  const int n_steps = kt1 - kt0;
+  const int sl0 = p.slices * split / p.splits, n_slices = p.slices * (split + 1) / p.splits - sl0;
+  auto slice_k = [&](int i) { return (int)((int64_t)p.KT * (sl0 + i) / p.slices); };      // first k step of this CTA's slice i
 
   if (warp == 0) {
     bool ok = true;
     int it = 0;
-    for (; it < n_steps && ok; ++it) {
-      const int s = it % STAGES;
-      ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_EMPTY(s), ((it / STAGES) & 1u) ^ 1u, ctl, 801));
-      if (!ok) break;
-      const uint32_t st = sbase + (uint32_t)s * stage_bytes;
-      elect_expect_tx(BAR_FULL(s), X_BYTES + W_BYTES);
-      // token blocks start at different k steps: CTAs that run side by side do not all ask for the same Wg tile
-      const int kt = kt0 + (int)((it + blk * 5) % n_steps);
-      elect_tile_2d(st, &x_map, kt * 64, (int)(blk * RT_BLOCK_T), BAR_FULL(s));
-      elect_tile_2d(st + X_BYTES, &w_map, kt * 64, 0, BAR_FULL(s));
+    for (int i = 0; i < n_slices && ok; ++i) {
+      const int kt0 = slice_k(i), n_steps = slice_k(i + 1) - kt0;
+      for (int j = 0; j < n_steps; ++j, ++it) {
+        const int s = it % STAGES;
+        ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_EMPTY(s), ((it / STAGES) & 1u) ^ 1u, ctl, 801));
+        if (!ok) break;
+        const uint32_t st = sbase + (uint32_t)s * stage_bytes;
+        elect_expect_tx(BAR_FULL(s), X_BYTES + W_BYTES);
+        // token blocks start at different k steps: CTAs that run side by side do not all ask for the same Wg tile
+        const int kt = kt0 + (int)((j + blk * 5) % n_steps);
+        elect_tile_2d(st, &x_map, kt * 64, (int)(blk * RT_BLOCK_T), BAR_FULL(s));
+        elect_tile_2d(st + X_BYTES, &w_map, kt * 64, 0, BAR_FULL(s));
+      }
     }
     if (!ok && lane == 0) {
       const int lo = it > STAGES ? it - STAGES : 0;
@@ -154,36 +163,68 @@ router_topk_kernel(const RouterParams p, const __grid_constant__ CUtensorMap x_m
   } else if (warp == 1) {
     bool ok = true;
     const uint32_t idesc = make_idesc(p.n_mma);
-    for (int it = 0; it < n_steps && ok; ++it) {
-      const int s = it % STAGES;
-      ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_FULL(s), (it / STAGES) & 1u, ctl, 802));
-      if (!ok) break;
-      tc_fence_after();
-      const uint32_t st = sbase + (uint32_t)s * stage_bytes;
-      const uint32_t a_lo = DESC_LO | (st >> 4), b_lo = DESC_LO | ((st + X_BYTES) >> 4);
+    int it = 0;
+    for (int i = 0; i < n_slices && ok; ++i) {
+      const int n_steps = slice_k(i + 1) - slice_k(i);
+      const uint32_t acc = tmem + (uint32_t)(i & 1) * acc_cols;
+      if (i >= 2) {
+        ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_ACC_FREE(i & 1), ((i >> 1) & 1u) ^ 1u, ctl, 803));
+        tc_fence_after();
+      }
+      for (int j = 0; j < n_steps && ok; ++j, ++it) {
+        const int s = it % STAGES;
+        ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_FULL(s), (it / STAGES) & 1u, ctl, 802));
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t st = sbase + (uint32_t)s * stage_bytes;
+        const uint32_t a_lo = DESC_LO | (st >> 4), b_lo = DESC_LO | ((st + X_BYTES) >> 4);
 #pragma unroll
-      for (int kk = 0; kk < 4; ++kk) elect_mma_bf16(tmem, a_lo + kk * 2, b_lo + kk * 2, idesc, (it | kk) ? 1u : 0u);
-      elect_commit(BAR_EMPTY(s));
+        for (int kk = 0; kk < 4; ++kk) elect_mma_bf16(acc, a_lo + kk * 2, b_lo + kk * 2, idesc, (j | kk) ? 1u : 0u);
+        elect_commit(BAR_EMPTY(s));
+      }
+      elect_commit(BAR_ACC(i & 1));     // arrives when every MMA above has retired
+      if (!ok)                          // aborting: let the MMAs that were already issued retire before tensor memory is freed
+        for (uint32_t w = 0; w < (1u << 16) && !mbar_test(BAR_ACC(i & 1), (i >> 1) & 1u); ++w) __nanosleep(64);
     }
-    elect_commit(BAR_ACC);              // arrives when every MMA above has retired
-    if (!ok) mbar_wait(BAR_ACC, 0, ctl, 803);
     __syncwarp();
   } else {
-    // ---- 16 warps: this slice's logits into shared memory as [expert][token row] (the operand stages are free by then) ----
+    // ---- 16 warps: the sums of this CTA's slices, in their order, into shared memory as [expert][token row] (the operand stages are free
+    // by then) ----
     const int qd = warp & 3, grp = (warp - 2) >> 2;            // lane quarter of tensor memory, share of its columns
     const int sid = threadIdx.x - 64;
     // the bias once per CTA, while the main loop runs (read per logit from global memory it made the selection wait on
     // one load after the other)
     if (sid < 256) s_bias[sid] = (p.bias && sid < p.E) ? load_bias(p.bias, p.bias_dtype, sid) : 0.0f;
-    if (__all_sync(0xFFFFFFFFu, mbar_wait(BAR_ACC, 0, ctl, 804))) {
+    float sum[4][16];
+    bool ok = true;
+    for (int i = 0; i < n_slices && ok; ++i) {
+      ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_ACC(i & 1), (i >> 1) & 1u, ctl, 804));
+      if (!ok) break;
       tc_fence_after();
-      const uint32_t taddr = tmem + ((uint32_t)(qd * 32) << 16);
-      for (int c0 = grp * 16; c0 < p.n_mma; c0 += 64) {
-        uint32_t v[16];
-        tmem_ld16(taddr + (uint32_t)c0, v);
-        tmem_ld_wait();
+      const uint32_t taddr = tmem + (uint32_t)(i & 1) * acc_cols + ((uint32_t)(qd * 32) << 16);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) mat[(c0 + j) * RT_MAT_LD + qd * 32 + lane] = __uint_as_float(v[j]);
+      for (int c = 0; c < 4; ++c) {
+        const int c0 = grp * 16 + c * 64;
+        if (c0 < p.n_mma) {
+          uint32_t v[16];
+          tmem_ld16(taddr + (uint32_t)c0, v);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 16; ++j) sum[c][j] = i ? sum[c][j] + __uint_as_float(v[j]) : __uint_as_float(v[j]);
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(BAR_ACC_FREE(i & 1));
+    }
+    if (ok) {
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const int c0 = grp * 16 + c * 64;
+        if (c0 < p.n_mma) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) mat[(c0 + j) * RT_MAT_LD + qd * 32 + lane] = sum[c][j];
+        }
       }
     }
   }
@@ -198,7 +239,7 @@ router_topk_kernel(const RouterParams p, const __grid_constant__ CUtensorMap x_m
     const int rows_blk = (int)min((int64_t)RT_BLOCK_T, p.T - blk * RT_BLOCK_T);
     int lr = 0;
     while ((1 << lr) < rows_blk) ++lr;
-    lr = max(0, lr - (31 - __clz(p.splits)));                  // this CTA's share of the rows: 2^lr from r0 on
+    lr = max(0, lr - (31 - __clz(p.splits)));                  // this CTA's share of the rows: 2^lr from r0 on (none for some CTAs)
     const int r0 = split << lr, rows = min(1 << lr, rows_blk - r0);
     bool ok = true;
     for (int i = 0; i < p.splits; ++i) ok = ok && ld_slice_u32(smem_u32((const void*)&s_abort), p.splits, i) == 0;
@@ -215,9 +256,10 @@ router_topk_kernel(const RouterParams p, const __grid_constant__ CUtensorMap x_m
               const uint32_t at = smem_u32(mat + (i >> lr) * RT_MAT_LD + r0 + (i & ((1 << lr) - 1)));
 #pragma unroll 1
               for (int j = 0; j < p.splits; j += 2) {
-                const float x = __uint_as_float(ld_slice_u32(at, p.splits, j)), y = __uint_as_float(ld_slice_u32(at, p.splits, j + 1));
+                const float x = __uint_as_float(ld_slice_u32(at, p.splits, j));
+                const float y = j + 1 < p.splits ? __uint_as_float(ld_slice_u32(at, p.splits, j + 1)) : 0.0f;
                 sum[u] += x;
-                sum[u] += y;
+                if (j + 1 < p.splits) sum[u] += y;
               }
             }
           }
@@ -307,7 +349,7 @@ int rt_make_map(const void* base, int64_t rows, int64_t K, int64_t ld, int box_r
 
 struct RouterPlan {
   int64_t blocks;
-  int n_mma, KT, splits, stages;
+  int n_mma, KT, slices, splits, stages;
 };
 
 RouterPlan rt_plan(int64_t T, int64_t K, int E) {
@@ -315,12 +357,15 @@ RouterPlan rt_plan(int64_t T, int64_t K, int E) {
   pl.blocks = cdiv64(T, RT_BLOCK_T);
   pl.n_mma = (E + 15) / 16 * 16;
   pl.KT = (int)cdiv64(K, 64);
-  // Few token blocks: cut K so that many SMs pull a share of the operands, into the 2, 4 or 8 CTAs of a cluster, two k steps each at
-  // least.  (Clusters of eight have an SM to a CTA only up to some 14 at a time: with 16, 2048 tokens took 37.9 us with the sort behind
-  // it, 26 with slices of four.)
-  int s = 1;
-  while (s < 8 && 2 * s * pl.blocks <= (s == 4 ? moe_sm_count() * 3 / 4 : moe_sm_count()) && pl.KT >= 4 * s) s *= 2;
-  pl.splits = s;
+  // Few token blocks: cut K so that many SMs pull a share of the operands.  Slices get longer as blocks get more: at least 2 k steps
+  // with one block, 12 from six on.  They go to the CTAs of a cluster, eight at most (the portable size), several to each where there are
+  // more.  Not a matter of speed alone: the error of a slice's sum grows with its steps (64 tokens, K = 2880: 22 slices 1.1e-7 from the
+  // exact logits, eight 2.3e-7; 6000 tokens: three 6.4e-7, two 9.9e-7), and its last bit can become a step of the logit rounded to bf16.
+  int64_t s = moe_sm_count() / (pl.blocks > 0 ? pl.blocks : 1);
+  const int64_t min_steps = pl.blocks >= 6 ? 12 : 2 * pl.blocks;
+  if (s > pl.KT / min_steps) s = pl.KT / min_steps;
+  pl.slices = s < 1 ? 1 : (int)s;
+  pl.splits = pl.slices > 8 ? 8 : pl.slices;
   const int stage_bytes = RT_BLOCK_T * 128 + ((pl.n_mma * 128 + 1023) & ~1023);
   int st = (200 * 1024) / stage_bytes;
   pl.stages = st > RT_STAGES_MAX ? RT_STAGES_MAX : st;
@@ -356,7 +401,7 @@ extern "C" __attribute__((visibility("default"))) int moe_router_topk(
   const RouterPlan pl = rt_plan(T, K, E);
   cudaStream_t st = (cudaStream_t)stream;
   RouterParams p;
-  p.T = T; p.E = E; p.n_mma = pl.n_mma; p.k = k; p.KT = pl.KT; p.splits = pl.splits; p.stages = pl.stages;
+  p.T = T; p.E = E; p.n_mma = pl.n_mma; p.k = k; p.KT = pl.KT; p.slices = pl.slices; p.splits = pl.splits; p.stages = pl.stages;
   p.apply_softmax = apply_softmax; p.round_bf16 = round_bf16;
   p.bias = bias; p.bias_dtype = bias_dtype;
   p.logits_out = logits_out; p.ld_logits = ld_logits;

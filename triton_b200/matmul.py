@@ -125,7 +125,7 @@ _STATUS_TEXT = {
     613: "block-scaled pair kernel: the MMA warp waited for a free accumulator", 614: "block-scaled pair kernel: the final MMA drain",
     615: "block-scaled pair kernel: a scale loader waited for a stage", 616: "block-scaled pair kernel: the epilogue waited for an accumulator",
     801: "router kernel: the producer waited for a free stage", 802: "router kernel: the MMA thread waited for a stage",
-    803: "router kernel: the final MMA drain", 804: "router kernel: the selection waited for the accumulator",
+    803: "router kernel: the MMA warp waited for a free accumulator", 804: "router kernel: the selection waited for the accumulator",
     901: "expert-parallel peer barrier: a rank did not arrive within the limit; the step after it read stale peer buffers",
 }
 

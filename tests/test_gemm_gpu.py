@@ -485,35 +485,60 @@ def test_layer_in_one_call_sizes_its_workspace_for_the_activation(block_scaled, 
     assert torch.equal(one, many)
 
 
-@pytest.mark.parametrize("tokens", [3, 40, 300, 1300])
-def test_layer_step_captured_behind_a_join(tokens, device):
+@pytest.mark.parametrize("tokens, experts, dtype", [(3, 8, "bf16"), (40, 8, "bf16"), (300, 8, "bf16"), (1300, 8, "bf16"), (2100, 16, "bf16"),
+                                                    (40, 8, "e4m3"), (300, 8, "e4m3"), (1300, 8, "e4m3")])
+def test_layer_step_captured_behind_a_join(tokens, experts, dtype, device):
     """A step captured where its stream has just joined another one (two predecessors, neither of them a kernel of this package), and a second
-    step right behind it on the first one's result: the bits of the eager steps."""
+    step with other routing right behind it on the first one's result.  Before every replay tokens, logits (with very different expert
+    loads) and weights are overwritten in place: a kernel that reads what the replay before has left gives other bits than the eager steps.
+    One to three launches of routing, tokens packed by position and by row, both block-scaled kernels."""
     from triton_b200.moe import moe_layer_forward
     from triton_b200.testing import make_synthetic_layer
-    E, d, k = 8, 512, 2
-    lw = make_synthetic_layer(E, d, 736, device, seed=3, block_scaled=True)
+    d, k, sets = 512, 2, 3
+    type_ = torch.float8_e4m3fn if dtype == "e4m3" else torch.bfloat16
+    weights = [make_synthetic_layer(experts, d, 736, device, seed=3 + i, block_scaled=True) for i in range(sets + 1)]
+    lw = weights.pop()
+    names = ["w1", "w1_scale", "b1", "w2", "w2_scale", "b2", "w1_bs", "w1_bs_scale", "w2_bs", "w2_bs_scale"]
+
+    def parts(layer):
+        return [t if isinstance(t, torch.Tensor) else t.storage.data for t in (getattr(layer, n) for n in names)]
+
     g = torch.Generator(device=device).manual_seed(tokens)
-    x, logits = torch.randn(tokens, d, device=device, generator=g).bfloat16(), torch.randn(tokens, E, device=device, generator=g)
+    inputs = [[torch.randn(tokens, d, device=device, generator=g)] + [torch.randn(tokens, experts, device=device, generator=g)
+               + 3 * torch.randn(experts, device=device, generator=g) for _ in range(2)] for _ in range(sets)]
+    x, logits, logits2 = (torch.zeros_like(t) for t in inputs[0])
     side = torch.cuda.Stream(device=device)
+
+    def fill(i):
+        for to, frm in zip([x, logits, logits2, *parts(lw)], [*inputs[i], *parts(weights[i])]):
+            to.view(torch.uint8).copy_(frm.view(torch.uint8))
 
     def step():
         side.wait_stream(torch.cuda.current_stream(device))
         with torch.cuda.stream(side):
-            xs = x * 2
+            xs = (x * 2).to(type_)
         ls = logits + 1
         torch.cuda.current_stream(device).wait_stream(side)
         xs.record_stream(torch.cuda.current_stream(device))
         z = moe_layer_forward(xs, ls, lw, k)
-        return z, moe_layer_forward(z, ls, lw, k)
+        return z, moe_layer_forward(z.to(type_), logits2, lw, k)
 
-    eager = [t.clone() for t in step()]
-    torch.cuda.synchronize()
+    eager = []
+    for i in range(sets):
+        fill(i)
+        eager.append([t.clone() for t in step()])
+        torch.cuda.synchronize()
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph):
         captured = step()
-    for _ in range(3):
+    got = []
+    order = [1, 0, 2, 2, 1, 0]
+    for i in order:
+        fill(i)
         graph.replay()
+        got.append([t.clone() for t in captured])
     torch.cuda.synchronize()
     tb.matmul_check_status()
-    assert all(torch.equal(a, b) for a, b in zip(eager, captured))
+    for i, replayed in zip(order, got):
+        assert all(torch.equal(a, b) for a, b in zip(eager[i], replayed))
+    assert not torch.equal(eager[0][1], eager[1][1])

@@ -441,3 +441,26 @@ def test_wide_swiglu_product_over_few_k_stays_with_the_bf16_kernel():
     from triton_b200 import _lib
     plain = _lib.host().gemm_kernel(_lib.MOE_W_MX4_B200, 16, 512, 4096, 16 * 1024, torch.bfloat16, torch.bfloat16, (0, 0, 0, 0))
     assert plain == "gemm_mx_pair_kernel"
+
+
+def test_kernels_read_nothing_of_the_chain_ahead_of_their_wait():
+    """Memory that earlier kernels of the stream wrote is visible behind griddepcontrol.wait and not before.  Every kernel that waits does so
+    with all its threads, in one place, and ahead of it touches neither metadata, operands nor weights, but for hints to L2."""
+    import pathlib
+    import re
+    csrc = pathlib.Path(triton_b200.__file__).parent / "csrc"
+    waiting, launched = set(), set()
+    for path in sorted(csrc.glob("*.cu")):
+        text = re.sub(r"//[^\n]*", "", path.read_text())
+        launched |= set(re.findall(r"launch_pdl\(\s*(?:pack|(\w+))", text)) - {""}
+        for m in re.finditer(r"__global__ void\s+(?:__launch_bounds__\((?:[^()]|\([^()]*\))*\)\s*)?(\w+)\(", text):
+            body = text[m.end():]
+            body = body[:body.index("\n}\n")]
+            if "pdl_" not in body:
+                continue
+            waiting.add(m.group(1))
+            assert re.findall(r"\n( *)pdl_begin\(\);", body) == ["  "] and "pdl_wait" not in body, f"{path.name}: {m.group(1)}"
+            ahead = body[body.index("{"):body.index("pdl_begin();")]
+            reads = r"slice_sizes|slice_offs|block_offs|block_sched|p\.bias|gather|pair_prefix|map_block|map_ptile|elect_(tile|bulk|expect)|ld_?global|__ldg|cp_async"
+            assert not re.search(reads, ahead), f"{path.name}: {m.group(1)}: {re.search(reads, ahead).group(0)}"
+    assert launched <= waiting and {"gemm_mx_kernel", "gemm_mx_pair_kernel", "router_topk_kernel", "route_cluster_kernel"} <= waiting

@@ -40,11 +40,24 @@ void moe_count_launch();   // one kernel launch (api.cu keeps the process-wide c
 // next kernel of the stream may start once every block of this one has passed pdl_launch_dependents() or left, and whatever it
 // reads or writes comes after its own pdl_wait(), which returns when its predecessors have completed and their writes are
 // visible (so those kernels take their pointers without __restrict__: a load through such a pointer may move ahead of the
-// wait).  Launch and prologue of a kernel then overlap the tail of the one before.  A kernel waits before it lets its
-// dependents go, so at most one kernel is ahead of a running one, and every grid before that one has completed.
+// wait).  Launch and prologue of a kernel then overlap the tail of the one before.  A kernel waits, with all its threads, before
+// it lets its dependents go, so at most one kernel is ahead of a running one.  It reads nothing of device memory ahead of the wait,
+// not even what kernels further back wrote: that they have completed orders nothing for a kernel that has not waited.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_begin() { pdl_wait(); pdl_launch_dependents(); }
+
+// What a kernel may do ahead of its wait is to ask L2 for memory it expects to need: a hint that is wrong, or older than the memory, is
+// without effect on what is loaded later.  Words that steer it are read past L1, where an early copy would stay, and are read again
+// behind the wait for all else.
+__device__ __forceinline__ int ld_hint(const int32_t* a) {
+  int v;
+  asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void l2_hint(const void* a, uint32_t bytes) {       // 16-byte aligned, a multiple of 16
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"(bytes) : "memory");
+}
 
 template <typename... KArgs, typename... Args>
 cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {

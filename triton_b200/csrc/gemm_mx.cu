@@ -63,6 +63,7 @@ struct MxParams {
   int stages, stage_bytes;
   int acc_bufs;
   int64_t grid_m;               // static bound on token blocks (dense problems: exact)
+  uint32_t hint_m;              // and on the entries of the schedule that may be read before they are known to be written
   TokenOut out;                 // the rows as the next product's tokens
 };
 
@@ -302,6 +303,29 @@ __device__ __forceinline__ void mma_mx(uint32_t d_tmem, uint32_t a_lo, uint32_t 
         : "memory");
 }
 
+// Asks L2 for the weights of this CTA's first stages (a warp, ahead of its wait for the kernel before, whose CTA on this SM may have left
+// long before its last one does).  Decode of one token 38.2 -> 36.9 us per step, 16 tokens of 32 experts 70.8 -> 68.1.  (With the
+// metadata read ahead of the wait for good, and the first weights loaded into shared memory there: 34.8 and 64.3, but
+// only the wait makes visible what the stream's kernels wrote, those further back included.)
+template <int NACC>
+__device__ __forceinline__ void mx_hint_weights(const GemmParams& p, const MxParams& q, int narrow_steps, int lane) {
+  const int KT = q.KT, NB = q.NB;
+  uint32_t useful_m = (uint32_t)q.grid_m;
+  if (p.slice_sizes) useful_m = min((uint32_t)ld_hint(p.block_offs + p.E), q.hint_m);
+  MxSched sched(useful_m, NB, NACC);
+  int64_t pid_m;
+  int nb0, mb_live;
+  if (!sched.next(pid_m, nb0, mb_live)) return;
+  const int e = p.slice_sizes ? ld_hint(p.block_sched + pid_m) & 0xFFFF : 0;
+  if (e >= p.E) return;
+  const int steps = min(KT, q.stages * (NACC == 1 || sched.narrow ? narrow_steps : 1));
+  for (int kt = lane; kt < steps; kt += 32) {
+    const int64_t tile = ((int64_t)e * KT + kt) * NB + nb0;
+    l2_hint((const uint8_t*)p.w + tile * MX_W_TILE_TX, (uint32_t)(mb_live * MX_W_TILE_TX));
+    l2_hint(p.w_scale + tile * MX_WS_TILE, (uint32_t)(mb_live * MX_WS_TILE));
+  }
+}
+
 // sums of N tokens over their terms, smallest first
 __device__ __forceinline__ void tmem_ld_n(uint32_t taddr, uint32_t (&r)[4]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
@@ -396,8 +420,9 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xFFFFFFFFu, *s_tmem, 0);
 
-  // (Whatever is read ahead of pdl_wait -- ragged metadata, weights -- is older than the kernel before this one, which let this one start
-  // when its own predecessors had completed.)
+  // (a scale loader: it waits longest for its first work)
+  if (warp == MX_THREADS / 32 - 1) mx_hint_weights<NACC>(p, q, KM ? 3 : NACC == 3 ? 2 : 1, lane);
+  pdl_begin();
   const int KT = q.KT, NB = q.NB;
   uint32_t useful_m = (uint32_t)q.grid_m;
   if (p.slice_sizes) useful_m = (uint32_t)__shfl_sync(0xFFFFFFFFu, p.block_offs[p.E], 0);
@@ -415,11 +440,8 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
 
   if (warp == 0) {
     // ================================= producer =======================================================
-    // The weights of the first tile's first stages are requested ahead of the wait for the kernel before (whose CTA on this SM may have
-    // left long before its last one does), their tokens behind it: with the chains of a tile's blocks side by side in the epilogue,
-    // decode of one token 38.3 -> 35.3 us per step, 16 tokens of 32 experts 74.4 -> 68.6.
     uint32_t s = 0, ph = 1, issued = 0;
-    bool ok = true, waited = false;
+    bool ok = true;
     while (ok && sched.next(pid_m, nb0, mb_live)) {
       int e; int64_t row0; int rows;
       mx_map_block(p, q.tb, pid_m, e, row0, rows);
@@ -433,13 +455,16 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
         constexpr int S = decltype(steps)::value;
         const int stages = (KT + S - 1) / S;
         const CUtensorMap* w_map = &w_maps.m[S > 1 ? 0 : mb_live - 1];
-        auto weights = [&](int kt, uint32_t stage, uint32_t st, uint32_t bar) {
+        for (int kt = 0; kt < stages; ++kt, ++issued) {
+          const uint32_t st = sbase + s * (uint32_t)q.stage_bytes, bar = BAR_FULL(s);
+          ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_EMPTY(s), ph, ctl, 601));
+          if (!ok) break;
           if (FIT && kt == 0) {                        // (the arrival below publishes it)
-            if (lane == 0) s_cols[stage] = cols;
+            if (lane == 0) s_cols[s] = cols;
             __syncwarp();
           }
+          const int k_live = S > 1 ? min(S, KT - S * kt) : 1;
           if constexpr (S > 1) {
-            const int k_live = min(S, KT - S * kt);
             elect_expect_tx(bar, (uint32_t)k_live * ((uint32_t)(MX_W_TILE_TX + MX_WS_TILE) + live));
             for (int i = 0; i < k_live; ++i, tile += NB) {
               elect_tile_3d(st + (uint32_t)i * W_TILE, w_map, 0, 0, tile, bar);
@@ -451,21 +476,6 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
             elect_bulk_g2s(st + off_ws(1), p.w_scale + (int64_t)tile * MX_WS_TILE, (uint32_t)(mb_live * MX_WS_TILE), bar);
             tile += NB;
           }
-        };
-        int ahead = 0;                                 // stages that have their weights
-        if (!waited) {
-          waited = true;
-          for (; ahead < min(STAGES, stages); ++ahead) weights(ahead, (uint32_t)ahead, sbase + (uint32_t)ahead * (uint32_t)q.stage_bytes, BAR_FULL(ahead));
-          pdl_wait();
-        }
-        for (int kt = 0; kt < stages; ++kt, ++issued) {
-          const uint32_t st = sbase + s * (uint32_t)q.stage_bytes, bar = BAR_FULL(s);
-          if (kt >= ahead) {
-            ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_EMPTY(s), ph, ctl, 601));
-            if (!ok) break;
-            weights(kt, s, st, bar);
-          }
-          const int k_live = S > 1 ? min(S, KT - S * kt) : 1;
           if (S == 1 || !FIT) {
             elect_bulk_g2s(st + off_x(S), xsrc, (uint32_t)k_live * live, bar);
             xsrc += (uint32_t)k_live * chunk;
@@ -485,7 +495,6 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
   } else if (warp == 1) {
     // ================================= MMA issuer =====================================================
     uint32_t idesc = F4 ? mx4_idesc(q.n_mma, 0) : mx_idesc(q.n_mma, 0);
-    pdl_begin();
     uint32_t s = 0, ph = 0, tc = 0;                    // stage and parity of the next k step
     bool ok = true, ready = false;                     // ready: the next step was complete when the last one was issued
     for (; ok && sched.next(pid_m, nb0, mb_live); ++tc) {
@@ -639,7 +648,6 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
       if constexpr (TOK_TERMS<TY> != 0) ok = tok.all(ok);
       if (!ok) break;
       tc_fence_after();
-      if (tc == 0) pdl_wait();                         // ahead of the first store
       for (int c0 = 0; c0 < rows; c0 += 16) {
         if constexpr (TOK_TERMS<TY> != 0) {
           // the rows of the tile's groups into their stages, then the groups of all of them to the threads, four lanes each: with the few
@@ -907,6 +915,7 @@ int moe_gemm_mx_launch(const GemmParams& p_in, const MoeGemmArgs& a, const Token
   q.n_mma = pl.n_mma; q.tb = pl.tb; q.split = pl.split;
   q.KT = pl.KT; q.NB = pl.NB; q.stages = pl.stages; q.stage_bytes = pl.stage_bytes; q.acc_bufs = pl.acc_bufs;
   q.grid_m = pl.grid_m;
+  q.hint_m = (uint32_t)(a.slice_sizes && a.ld_block_sched < pl.grid_m ? a.ld_block_sched : pl.grid_m);
   MxMaps w_map;
   for (int nb = 1; nb <= 3; ++nb)
     if (int rc = make_w_map(a, pl.KT, pl.NB, pl.f4 != 0, nb <= pl.mb ? nb : pl.mb, &w_map.m[nb - 1])) return rc;

@@ -506,17 +506,6 @@ gemm_mx_pair_kernel(const GemmParams p, const PairParams a, const __grid_constan
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(ctl0 + PP_OFF_MISC), "r"((uint32_t)TMEM_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
-  // (Whatever is read ahead of pdl_wait -- ragged metadata, weights -- is older than the kernel before this one, which let this one start
-  // when its own predecessors had completed.)
-  if (warp == PP_SF_WARP0) {                           // tile prefix over experts
-    pair_prefix(p, s_prefix, a.nmax, lane);
-  }
-  tc_fence_before();
-  __syncthreads();
-  cluster_sync_all();                                  // the other CTA's barriers exist before anyone signals them
-  tc_fence_after();
-  const uint32_t tmem_base = __shfl_sync(0xFFFFFFFFu, *s_tmem, 0);
-
   const int KT = a.KT, NB = a.NB;
   const int MB = (NB + 1) >> 1, MT = (MB + UPT - 1) / UPT;      // 256-row weight blocks, tiles of UPT of them
   // The blocks of a tile: CTA r takes the neighbouring blocks 4 t + 2 r and + 1 (one copy each stage), a block of the MMA is one
@@ -531,15 +520,36 @@ gemm_mx_pair_kernel(const GemmParams p, const PairParams a, const __grid_constan
     b.units = wide ? 2 : 1;
     return b;
   };
+  if (warp == 3) {
+    // Ahead of the wait for the kernel before (whose CTA on this SM may have left long before its last one does): L2 is asked for the weights
+    // of the first tile's first stages (8 experts of 512 x 2048, 256 tokens: 30.5 -> 29.0 us per step).
+    const int e = pair_hint_expert(p, a.nmax, pair / MT, lane);
+    const Blocks b = blocks_of(pair);
+    if (e >= 0) {
+      for (int i = lane; i < (TILED ? b.own : STAGES); i += 32) {
+        const int64_t tile = TILED ? (int64_t)(e * NB + b.first + i) * KT : (int64_t)(e * KT + i) * NB + b.first;
+        const uint32_t n = (uint32_t)(TILED ? STAGES : b.own);
+        if (n == 0) break;
+        l2_hint((const uint8_t*)p.w + tile * 8192, n * 8192u);
+        l2_hint(p.w_scale + tile * 512, n * 512u);
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();                                  // the other CTA's barriers exist before anyone signals them
+  tc_fence_after();
+  const uint32_t tmem_base = __shfl_sync(0xFFFFFFFFu, *s_tmem, 0);
+  pdl_begin();
+  if (warp == PP_SF_WARP0) pair_prefix(p, s_prefix, a.nmax, lane);      // tile prefix over experts
+  __syncthreads();
   const int n_tiles = __shfl_sync(0xFFFFFFFFu, s_prefix[p.slice_sizes ? p.E : 1], 0) * MT;
 
   if (warp < PP_SF_WARP0) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_ISSUE));
   if (warp == 0) {
     // ================================= producer =======================================================
-    // The weights of the first tile's first stages are requested ahead of the wait for the kernel before (whose CTA on this SM may have
-    // left long before its last one does), their tokens behind it (8 experts of 512 x 2048, 256 tokens: 29.8 -> 27.9 us per step).
     uint32_t s = 0, ph = 1, issued = 0;
-    bool ok = true, waited = false;
+    bool ok = true;
     PTile nxt;                                         // the next tile is looked up while this one streams
     if (pair < n_tiles) nxt = map_ptile(p, s_prefix, pair / MT);
     for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
@@ -554,31 +564,19 @@ gemm_mx_pair_kernel(const GemmParams p, const PairParams a, const __grid_constan
       const uint8_t* xs = a.xs + TERMS * ((int64_t)prow0 * 4);
       const int64_t q_step = TERMS * a.prows * 128, s_step = TERMS * a.prows * 4;
       int c2 = TILED ? 0 : b.first, c3 = TILED ? e * NB + b.first : e * KT;
-      auto weights = [&](uint32_t st, uint32_t bar) {
+      for (int kt = 0; kt < KT; ++kt, ++issued) {
+        ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_EMPTY(s), ph, ctl, 611));
+        if (!ok) break;
+        const uint32_t st = sbase + s * (uint32_t)a.stage_bytes, bar = BAR_FULL(s);
         elect_expect_tx(bar, tx);
         if (b.own > 0) {
           elect_tile_4d(st, wm, 0, 0, c2, c3, bar);
           elect_tile_3d(st + OFF_WS, sm, 0, c2, c3, bar);
         }
-        if (TILED) ++c2; else ++c3;
-      };
-      int ahead = 0;                                   // stages that have their weights
-      if (!waited) {
-        waited = true;
-        for (; ahead < STAGES; ++ahead)                // (at most as many stages as k steps)
-          weights(sbase + (uint32_t)ahead * (uint32_t)a.stage_bytes, BAR_FULL(ahead));
-        pdl_wait();
-      }
-      for (int kt = 0; kt < KT; ++kt, ++issued) {
-        const uint32_t st = sbase + s * (uint32_t)a.stage_bytes, bar = BAR_FULL(s);
-        if (kt >= ahead) {
-          ok = __all_sync(0xFFFFFFFFu, mbar_wait(BAR_EMPTY(s), ph, ctl, 611));
-          if (!ok) break;
-          weights(st, bar);
-        }
         elect_bulk_g2s(st + OFF_X, xq, bx, bar);
         elect_bulk_g2s(st + OFF_XS, xs, bs, bar);
         xq += q_step; xs += s_step;
+        if (TILED) ++c2; else ++c3;
         if (++s == (uint32_t)STAGES) { s = 0; ph ^= 1u; }
         if (kt == 0 && tile + n_pairs < n_tiles) nxt = map_ptile(p, s_prefix, (tile + n_pairs) / MT);
       }
@@ -653,7 +651,7 @@ gemm_mx_pair_kernel(const GemmParams p, const PairParams a, const __grid_constan
     }
     __syncwarp();
   } else if (warp < PP_SF_WARP0) {
-    pdl_begin();                                       // (else only fills the warpgroup)
+    // (fills the warpgroup)
   } else if (warp < PP_EPI_WARP0) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_SF));
     // ================================= scale loaders ==================================================
@@ -710,7 +708,6 @@ gemm_mx_pair_kernel(const GemmParams p, const PairParams a, const __grid_constan
     }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS_EPI));
-    pdl_wait();
     // ================================= epilogue =======================================================
     // The warps of a lane quarter take the 16-token chunks of a unit in turn.
     const int ew = warp - PP_EPI_WARP0, qd = warp & 3, grp = ew >> 2;

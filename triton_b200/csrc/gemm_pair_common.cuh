@@ -57,23 +57,51 @@ constexpr int PAIR_PREFIX_INTS = 3 * MAX_PREFIX_EXPERTS + 1;
 __device__ __forceinline__ void pair_prefix(const GemmParams& p, int32_t* s_prefix, int nmax, int lane) {       // one warp
   const int n = p.slice_sizes ? p.E : 1;
   int run = 0;
+  for (int e0 = 0; e0 < n; e0 += 128) {
+    int sizes[4], offs[4];                             // loads of 128 experts side by side
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int e = e0 + 32 * i + lane;
+      sizes[i] = e < n ? max(p.slice_sizes ? p.slice_sizes[e] : (int)p.M, 0) : 0;
+      offs[i] = e < n && p.slice_sizes ? p.slice_offs[e] : 0;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int e = e0 + 32 * i + lane;
+      int v = (sizes[i] + nmax - 1) / nmax;
+      if (e < n) {
+        s_prefix[MAX_PREFIX_EXPERTS + 1 + e] = sizes[i];
+        s_prefix[2 * MAX_PREFIX_EXPERTS + 1 + e] = offs[i];
+      }
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xFFFFFFFFu, v, o);
+        if (lane >= o) v += t;
+      }
+      if (e < n) s_prefix[e + 1] = run + v;
+      run += __shfl_sync(0xFFFFFFFFu, v, 31);
+    }
+  }
+  if (lane == 0) s_prefix[0] = 0;
+}
+// The expert that token tile tt belongs to by what ld_hint reads, -1: none (one warp).
+__device__ __forceinline__ int pair_hint_expert(const GemmParams& p, int nmax, int tt, int lane) {
+  const int n = p.slice_sizes ? p.E : 1;
+  int run = 0;
   for (int e0 = 0; e0 < n; e0 += 32) {
     const int e = e0 + lane;
-    const int size = e < n ? max(p.slice_sizes ? p.slice_sizes[e] : (int)p.M, 0) : 0;
-    int v = (size + nmax - 1) / nmax;
-    if (e < n) {
-      s_prefix[MAX_PREFIX_EXPERTS + 1 + e] = size;
-      s_prefix[2 * MAX_PREFIX_EXPERTS + 1 + e] = p.slice_sizes ? p.slice_offs[e] : 0;
-    }
+    const int size = e < n ? max(p.slice_sizes ? ld_hint(p.slice_sizes + e) : (int)p.M, 0) : 0;
+    int v = size / nmax + (size % nmax != 0);
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int t = __shfl_up_sync(0xFFFFFFFFu, v, o);
       if (lane >= o) v += t;
     }
-    if (e < n) s_prefix[e + 1] = run + v;
+    const unsigned past = __ballot_sync(0xFFFFFFFFu, e < n && run + v > tt);
+    if (past) return e0 + __ffs(past) - 1;
     run += __shfl_sync(0xFFFFFFFFu, v, 31);
   }
-  if (lane == 0) s_prefix[0] = 0;
+  return -1;
 }
 
 // Token tile tt: rows of one expert, in groups of 32 dealt evenly over the expert's tiles (a tail of a few rows does not

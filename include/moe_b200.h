@@ -270,8 +270,10 @@ typedef struct {
 } MoeGemmArgs;
 int moe_grouped_gemm(const MoeGemmArgs* args_host, void* stream);
 /* Two products in a row: the same as moe_grouped_gemm of `first` and then of `second`, whose x is the first's y.  Where both run on
- * block-scaled kernels and their workspaces do not overlap, the first product leaves its rows as the second's tokens in that
- * workspace and y is scratch (its contents are then undefined).  The results of the second product are the same. */
+ * block-scaled kernels and the second reads the first's rows as they are (same rows, pitch and ragged structure), from a workspace that
+ * holds neither the first's nor its tokens, their scales and their indices, the first product leaves its rows as the second's tokens in
+ * that workspace and y is scratch (its contents are then undefined).  The results of the second product are the same.  The first's
+ * weights, bias and ragged metadata must not lie in the second's workspace. */
 int moe_grouped_gemm_chain(const MoeGemmArgs* first_host, const MoeGemmArgs* second_host, void* stream);
 size_t moe_gemm_mx_workspace_bytes(const MoeGemmArgs* args_host);
 /* Name of the kernel that moe_grouped_gemm launches for these arguments (with the workspace of the size above given), "" for an

@@ -1,0 +1,144 @@
+"""Two products in a row through the C entry point: the same as the two products called one after the other, whatever the caller's buffers
+look like.  The argument block is read from the header, so these tests call the library as a C program does."""
+import ctypes as C
+import re
+from pathlib import Path
+
+import pytest
+import torch
+
+from triton_b200 import _lib, routing
+from triton_b200.testing import make_synthetic_layer
+
+pytestmark = pytest.mark.gpu
+
+HEADER = re.sub(r"/\*.*?\*/", "", (Path(__file__).resolve().parent.parent / "include" / "moe_b200.h").read_text(), flags=re.S)
+CONST = {m[0]: int(m[1]) for m in re.findall(r"\b(MOE_[A-Z0-9_]+)\s*=?\s+(\d+)", HEADER)}
+
+
+def _struct(name):
+    body = re.search(r"typedef struct \{([^}]*)\} %s;" % name, HEADER).group(1)
+    types = {"int": C.c_int, "int64_t": C.c_int64, "float": C.c_float}
+    fields = []
+    for decl in filter(None, (d.strip() for d in body.split(";"))):
+        base, names = re.fullmatch(r"(?:const )?(\w+\s*\*?)\s*(.*)", decl, flags=re.S).groups()
+        for n in names.split(","):
+            array = re.fullmatch(r"\s*(\w+)\[(\w+)\]", n)
+            t = C.c_void_p if "*" in base else types[base.strip()]
+            fields.append((array.group(1), t * CONST[array.group(2)]) if array else (n.strip(), t))
+    return type(name, (C.Structure,), {"_fields_": fields})
+
+
+Args = _struct("MoeGemmArgs")
+E, K, D, FF = 6, 2, 512, 320
+
+
+class Problem:
+    """fc1 + SwiGLU and fc2 of a layer as two argument blocks; `pitch1`, `pitch2`: row pitch of the rows between as the first writes and the
+    second reads them."""
+
+    def __init__(self, T, device, block=0, pitch1=FF, pitch2=FF, e4m3=False, by_row=False):
+        g = torch.Generator(device=device).manual_seed(T)
+        dt = torch.float8_e4m3fn if e4m3 else torch.bfloat16
+        self.x = torch.randn(T, D, device=device, generator=g).bfloat16().to(dt)
+        logits = torch.randn(T, E, device=device, generator=g) + torch.randn(E, device=device, generator=g)
+        lw = make_synthetic_layer(E, D, FF, device, seed=3, block_scaled=True)
+        ragged, self.gather, scatter, sp = routing(logits, K)
+        self.M = M = T * K
+        self.gather = self.gather.int().contiguous()
+        self.h = torch.zeros(M + 1, max(pitch1, pitch2), device=device, dtype=torch.bfloat16).to(dt)
+        self.y = torch.zeros(M, D, device=device, dtype=torch.bfloat16)
+        self.status = torch.zeros(1, dtype=torch.int32, device=device)
+        self.keep = [lw, ragged, scatter, sp, sp.mask_metadata]
+        a, b = Args(), Args()
+        code, size = (CONST["MOE_F8E4M3"], 1) if e4m3 else (CONST["MOE_BF16"], 2)
+        for p, (w, ws, bias, k, n) in ((a, (lw.w1_bs, lw.w1_bs_scale, lw.b1, D, 2 * FF)), (b, (lw.w2_bs, lw.w2_bs_scale, lw.b2, FF, D))):
+            p.w_kind, p.w, p.w_scale, p.E, p.K, p.N, p.M = _lib.MOE_W_MX4_B200MX, w.storage.data.data_ptr(), ws.storage.data.data_ptr(), E, k, n, M
+            p.slice_sizes, p.slice_offs = ragged.slice_sizes.data_ptr(), ragged.slice_offs.data_ptr()
+            p.block_offs_16, p.block_sched_16 = ragged.block_offs_data.data_ptr(), ragged.block_schedule_data.data_ptr()
+            p.ld_block_offs, p.ld_block_sched = ragged.block_offs_data.stride(0), ragged.block_schedule_data.stride(0)
+            p.bias, p.bias_dtype, p.ld_bias = bias.data_ptr(), CONST["MOE_F32"] if bias.dtype == torch.float32 else CONST["MOE_BF16"], bias.stride(0)
+            p.tile_m, p.status = block, self.status.data_ptr()
+            p.x_dtype = code
+        a.x, a.ld_x, a.rows_x, a.gather_indx = self.x.data_ptr(), D, T, self.gather.data_ptr()
+        if by_row:
+            self.keep.append(sp.indx.contiguous())
+            a.x_positions, a.x_experts, a.x_k = sp.mask_metadata.row_sorted_indx.data_ptr(), self.keep[-1].data_ptr(), K
+        a.activation, a.act_alpha, a.act_limit, a.act_has_limit = CONST["MOE_ACT_SWIGLU"], 1.702, 7.0, 1
+        a.y, a.y_dtype, a.ld_y = self.h.data_ptr(), code, pitch1
+        b.x, b.ld_x, b.rows_x = self.h.data_ptr(), pitch2, M
+        b.y, b.y_dtype, b.ld_y = self.y.data_ptr(), CONST["MOE_BF16"], D
+        lib = _lib.load()
+        self.room = [int(lib.moe_gemm_mx_workspace_bytes(C.byref(p))) for p in (a, b)]
+        self.ws = [torch.zeros(n + 4096, dtype=torch.uint8, device=device) for n in self.room]
+        for p, n, ws in zip((a, b), self.room, self.ws):
+            p.mx_workspace, p.mx_workspace_bytes = (ws.data_ptr() + 1023) // 1024 * 1024, n
+        self.a, self.b = a, b
+
+    def move(self, t, offset):
+        """`t` into the second product's workspace, at `offset`; -> its address there."""
+        raw = t.reshape(-1).view(torch.uint8)
+        at = self.b.mx_workspace + offset
+        lo = at - self.ws[1].data_ptr()
+        assert lo + raw.numel() <= self.ws[1].numel()
+        self.ws[1][lo:lo + raw.numel()].copy_(raw)
+        return at
+
+    def run(self, chain):
+        """-> the second product's rows and the launches that took."""
+        lib = _lib.load()
+        self.h.view(torch.uint8).zero_()
+        self.y.zero_()
+        n0, st = lib.moe_launch_count(), torch.cuda.current_stream().cuda_stream
+        if chain:
+            _lib.check(lib.moe_grouped_gemm_chain(C.byref(self.a), C.byref(self.b), st), "chain")
+        else:
+            _lib.check(lib.moe_grouped_gemm(C.byref(self.a), st), "first")
+            _lib.check(lib.moe_grouped_gemm(C.byref(self.b), st), "second")
+        torch.cuda.synchronize()
+        assert int(self.status) == 0
+        return self.y.clone(), lib.moe_launch_count() - n0
+
+
+# tokens and tile_m: four e2m1 terms, two e4m3 terms of 32 rows, the pair kernel
+FORMS = [(20, 16), (70, 32), (300, 256)]
+
+
+@pytest.mark.parametrize("T, block", FORMS)
+@pytest.mark.parametrize("e4m3", [False, True])
+def test_rows_are_handed_over(T, block, e4m3, device):
+    p = Problem(T, device, block, e4m3=e4m3)
+    (apart, n), (chain, m) = p.run(False), p.run(True)
+    assert m == n - 1 and torch.equal(apart, chain) and bool(apart.abs().sum() > 0)
+
+
+@pytest.mark.parametrize("T, block", FORMS)
+@pytest.mark.parametrize("pitch1, pitch2", [(FF + 64, FF + 64), (FF, FF + 64), (FF + 64, FF)])
+def test_pitches_of_the_rows_between(T, block, pitch1, pitch2, device):
+    """The second product reads other rows than the first wrote where the pitches differ."""
+    p = Problem(T, device, block, pitch1, pitch2)
+    (apart, n), (chain, m) = p.run(False), p.run(True)
+    assert torch.equal(apart, chain) and m == (n - 1 if pitch1 == pitch2 else n)
+
+
+@pytest.mark.parametrize("T, block", FORMS)
+def test_second_product_with_fewer_rows(T, block, device):
+    """Rows past rows_x count as zero."""
+    p = Problem(T, device, block)
+    p.b.rows_x = p.M - 5
+    (apart, n), (chain, m) = p.run(False), p.run(True)
+    assert torch.equal(apart, chain) and m == n
+
+
+@pytest.mark.parametrize("T, block", FORMS)
+@pytest.mark.parametrize("operand", ["x", "gather"])
+def test_operands_in_the_second_workspace(T, block, operand, device):
+    """What the first product reads may lie in the workspace that the second one fills later."""
+    p = Problem(T, device, block)
+    want, n = p.run(False)
+    if operand == "x":
+        p.a.x = p.move(p.x, 0)
+    else:
+        p.a.gather_indx = p.move(p.gather, p.room[1] // 2 // 1024 * 1024)
+    got, m = p.run(True)
+    assert torch.equal(want, got) and m == n

@@ -174,19 +174,25 @@ extern "C" __attribute__((visibility("default"))) int moe_grouped_gemm(const Moe
 }
 
 // Whether product a may leave its rows as the tokens of product b, and where.  Both run on block-scaled kernels; b takes exactly a's
-// rows, in the same ragged structure, from workspace of its own; nothing but bias and activation is between.  bf16 rows: a limit on the
-// activation, which bounds them far below where two terms stop holding a value (the pack kernels have a way for such rows):
+// rows (all of them, at the pitch they would be written with), in the same ragged structure, from workspace of its own that holds
+// nothing a reads; nothing but bias and activation is between.  bf16 rows: a limit on the activation, which bounds them far below where two terms stop holding a value (the pack kernels have a way for such rows):
 // |silu(g)| <= max(limit, 0.28 / alpha) and the factor <= limit + 1.
 static bool hands_over(const MoeGemmArgs& a, Kernel ka, const MoeGemmArgs& b, Kernel kb, TokenOut& out) {
   if ((ka != K_MX_PAIR && ka != K_MX) || (kb != K_MX_PAIR && kb != K_MX)) return false;
   if (a.activation != MOE_ACT_SWIGLU || a.N % 64 != 0 || a.N != 2 * b.K || a.M != b.M || a.E != b.E || b.x != a.y || b.x_dtype != a.y_dtype ||
-      b.gather_indx || b.x_scale || a.scatter_indx || a.betas || a.gammas || a.has_out_alpha || a.n_y_peers > 0)
+      b.ld_x != a.ld_y || b.rows_x < b.M || b.gather_indx || b.x_scale || a.scatter_indx || a.betas || a.gammas || a.has_out_alpha || a.n_y_peers > 0)
     return false;
   if (!a.slice_sizes || a.slice_sizes != b.slice_sizes || a.slice_offs != b.slice_offs || a.block_offs_16 != b.block_offs_16 ||
       a.block_sched_16 != b.block_sched_16)
     return false;
-  const uint8_t *wa = (const uint8_t*)a.mx_workspace, *wb = (const uint8_t*)b.mx_workspace;
-  if (wa < wb + b.mx_workspace_bytes && wb < wa + a.mx_workspace_bytes) return false;
+  const uint8_t* wb = (const uint8_t*)b.mx_workspace;
+  auto within = [&](const void* at, int64_t bytes) {
+    return at && (const uint8_t*)at < wb + b.mx_workspace_bytes && wb < (const uint8_t*)at + bytes;
+  };
+  if (within(a.mx_workspace, a.mx_workspace_bytes) || within(a.x, a.rows_x * a.ld_x * (a.x_dtype == MOE_BF16 ? 2 : 1)) ||
+      within(a.x_scale, a.rows_x * a.ld_x_scale) || within(a.gather_indx, a.M * 4) || within(a.x_positions, a.rows_x * a.x_k * 4) ||
+      within(a.x_experts, a.rows_x * a.x_k * 2))
+    return false;
   const bool bf16 = a.y_dtype == MOE_BF16;
   if (bf16 && !(a.act_has_limit && a.act_limit > 0.0f && a.act_limit < 1e9f && a.act_alpha > 1e-9f)) return false;
   if (!bf16 && a.y_dtype != MOE_F8E4M3) return false;

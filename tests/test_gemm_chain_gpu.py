@@ -7,7 +7,7 @@ from pathlib import Path
 import pytest
 import torch
 
-from triton_b200 import _lib, routing
+from triton_b200 import _lib, make_ragged_tensor_metadata, routing
 from triton_b200.testing import make_synthetic_layer
 
 pytestmark = pytest.mark.gpu
@@ -37,7 +37,7 @@ class Problem:
     """fc1 + SwiGLU and fc2 of a layer as two argument blocks; `pitch1`, `pitch2`: row pitch of the rows between as the first writes and the
     second reads them."""
 
-    def __init__(self, T, device, block=0, pitch1=FF, pitch2=FF, e4m3=False, by_row=False):
+    def __init__(self, T, device, block=0, pitch1=FF, pitch2=FF, e4m3=False):
         g = torch.Generator(device=device).manual_seed(T)
         dt = torch.float8_e4m3fn if e4m3 else torch.bfloat16
         self.x = torch.randn(T, D, device=device, generator=g).bfloat16().to(dt)
@@ -61,9 +61,6 @@ class Problem:
             p.tile_m, p.status = block, self.status.data_ptr()
             p.x_dtype = code
         a.x, a.ld_x, a.rows_x, a.gather_indx = self.x.data_ptr(), D, T, self.gather.data_ptr()
-        if by_row:
-            self.keep.append(sp.indx.contiguous())
-            a.x_positions, a.x_experts, a.x_k = sp.mask_metadata.row_sorted_indx.data_ptr(), self.keep[-1].data_ptr(), K
         a.activation, a.act_alpha, a.act_limit, a.act_has_limit = CONST["MOE_ACT_SWIGLU"], 1.702, 7.0, 1
         a.y, a.y_dtype, a.ld_y = self.h.data_ptr(), code, pitch1
         b.x, b.ld_x, b.rows_x = self.h.data_ptr(), pitch2, M
@@ -142,3 +139,37 @@ def test_operands_in_the_second_workspace(T, block, operand, device):
         p.a.gather_indx = p.move(p.gather, p.room[1] // 2 // 1024 * 1024)
     got, m = p.run(True)
     assert torch.equal(want, got) and m == n
+
+
+@pytest.mark.parametrize("k", [2, 512, 513, 800])
+def test_positions_of_a_row_beyond_a_block_of_shared_memory(k, device):
+    """A row of x may go to any number of positions: the token pass by row holds those of eight rows, beyond that the pass goes by position."""
+    p = Problem(20, device, 256)
+    a, rows = p.a, 1184                                        # eight rows for each of 148 SMs: from there on by row
+    g = torch.Generator(device=device).manual_seed(k)
+    x = torch.randn(rows, D, device=device, generator=g).bfloat16()
+    experts = torch.randint(0, E, (rows * k,), device=device, generator=g).short()
+    order = torch.argsort(experts, stable=True)
+    positions = torch.empty(rows * k, dtype=torch.int32, device=device)
+    positions[order] = torch.arange(rows * k, dtype=torch.int32, device=device)
+    gather = (order // k).int()
+    ragged = make_ragged_tensor_metadata(torch.bincount(experts.long(), minlength=E).int(), rows * k)
+    a.x, a.rows_x, a.M, a.gather_indx, a.N = x.data_ptr(), rows, rows * k, gather.data_ptr(), 128
+    a.slice_sizes, a.slice_offs = ragged.slice_sizes.data_ptr(), ragged.slice_offs.data_ptr()
+    a.block_offs_16, a.block_sched_16 = ragged.block_offs_data.data_ptr(), ragged.block_schedule_data.data_ptr()
+    a.ld_block_offs, a.ld_block_sched = ragged.block_offs_data.stride(0), ragged.block_schedule_data.stride(0)
+    lib, st = _lib.load(), torch.cuda.current_stream().cuda_stream
+    ws = torch.empty(int(lib.moe_gemm_mx_workspace_bytes(C.byref(a))) + 1024, dtype=torch.uint8, device=device)
+    a.mx_workspace, a.mx_workspace_bytes = (ws.data_ptr() + 1023) // 1024 * 1024, ws.numel() - 1024
+    out = []
+    for by_row in (False, True):
+        y = torch.zeros(rows * k, 64, device=device, dtype=torch.bfloat16)
+        a.y, a.ld_y = y.data_ptr(), 64
+        if by_row:
+            a.x_positions, a.x_experts, a.x_k = positions.data_ptr(), experts.data_ptr(), k
+        assert lib.moe_gemm_kernel_name(C.byref(a)) == b"gemm_mx_pair_kernel"
+        _lib.check(lib.moe_grouped_gemm(C.byref(a), st), "product")
+        torch.cuda.synchronize()
+        assert int(p.status) == 0
+        out.append(y)
+    assert torch.equal(*out) and bool(out[0].abs().sum() > 0)

@@ -302,6 +302,7 @@ __global__ void __launch_bounds__(256) mx_pair_pack2_kernel(const __grid_constan
 // and quantised once and its lines are written k times.  16384 rows of 2880, four positions each: 137 us by position, 105 by row (390 MB out);
 // the prefill step 3144 -> 3081 us, with 8192 e4m3 rows 910 -> 903.
 constexpr int PACK_TOKENS = 8;
+constexpr int PACK_MAX_K = 512;                        // positions of a row: PACK_TOKENS x k words of 8 bytes in the 48 KB that need no opt-in
 // padded row of pick j of row t
 __device__ __forceinline__ int64_t pick_prow(const GemmParams& p, const PairPackParams& a, int64_t t, int j, int& e, int64_t& m) {
   e = a.experts[t * a.k + j];
@@ -1031,9 +1032,9 @@ int moe_gemm_mx_pair_launch(const GemmParams& p_in, const MoeGemmArgs& a, const 
   pk.out = out;
   pk.positions = nullptr; pk.experts = nullptr; pk.k = 0;
   if (!packed) {
-    // by rows of x where every one of them has its k positions, several, and their blocks fill the SMs (256 rows, two positions each: 27.6 us
-    // per layer step by position, 28.1 by row)
-    if (a.x_positions && a.x_experts && a.x_k > 1 && a.slice_sizes && a.rows_x * a.x_k == a.M &&
+    // by rows of x where every one of them has its k positions, several (and no more than a block has shared memory for), and their blocks
+    // fill the SMs (256 rows, two positions each: 27.6 us per layer step by position, 28.1 by row)
+    if (a.x_positions && a.x_experts && a.x_k > 1 && a.x_k <= PACK_MAX_K && a.slice_sizes && a.rows_x * a.x_k == a.M &&
         a.rows_x >= (int64_t)PACK_TOKENS * moe_sm_count()) {
       pk.positions = a.x_positions; pk.experts = a.x_experts; pk.k = a.x_k;
       auto pack = pl.terms == 1 ? mx_pair_pack1_rows_kernel : tiled ? mx_pair_pack2_rows_kernel<true> : mx_pair_pack2_rows_kernel<false>;

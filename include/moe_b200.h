@@ -122,7 +122,7 @@ int moe_route_positions(const float* logits, int64_t T, int E, int k, int apply_
  *   logits_out: NULL, or [T, E] fp32 that receives the logits the selection saw.
  *   vals [T, k] fp32 or bf16, indx, bitmatrix: as for moe_topk_fwd.
  * With few tokens K is cut into slices over the SMs of a cluster, whose partial logits meet in shared memory, in a fixed order: no
- * workspace is needed (moe_router_topk_workspace_bytes is 0; what is passed is not touched).  A bounded wait that expires writes 801..804
+ * workspace is needed (moe_router_topk_workspace_bytes is 0 and what is passed is not touched; both are kept for callers that pass one).  A bounded wait that expires writes 801..804
  * to *status.                                                                                                       */
 size_t moe_router_topk_workspace_bytes(int64_t T, int64_t K, int E);
 int moe_router_topk(const void* x, int64_t T, int64_t K, int64_t ld_x, const void* wg_t, int64_t ld_wg,
@@ -136,7 +136,7 @@ int moe_router_topk(const void* x, int64_t T, int64_t K, int64_t ld_x, const voi
  * all device memory to its own pools at start-up, or a latency-critical section where cudaMalloc, which
  * synchronises the device, is not acceptable.  The scratch is a fixed 1 MiB array inside the library
  * (moe_bitmatrix_metadata_noalloc_capacity() bytes, held by every GPU that loads the library until the
- * process exits); inputs and outputs are still the caller's.  It serves problems with
+ * process exits; not used up to 32768 entries of 256 experts); inputs and outputs are still the caller's.  It serves problems with
  * (ceil(T / 256) * E + E) * 4 <= capacity, e.g. T = 65536 tokens with E = 128 experts, or 8192 tokens with
  * E = 4096, and returns MOE_ERR_ARG with a message for anything larger.  It calls no cudaMalloc / cudaFree or
  * other allocating routine.  The first call on a device looks up the array's device address

@@ -965,15 +965,19 @@ int launch_mx_pair_ty(const GemmParams& p, const PairParams& q, const MoeGemmArg
 // experts of 1024 rows: 72 here, 57 there; 16 experts 132 and 109; without the activation 64 and 61, 114 and 116).
 // (Both kernels lose up to a third of a wave, so no line in these sizes is right everywhere: over 500 products of 48 to 1024 rows
 // this one is 2 % from the better kernel on average, most of it at 100-400 balanced rows of K <= 1024.)
-// Block-scaled tiles (against the decode forms of gemm_mx.cu), tile_m = 256 asks for it.  bf16 tokens from 20 rows on: 32 experts of
-// 2880 x 5760, 16 rows 126 there, 144 here, 24 rows 135 and 145, 32 rows 165 and 150; 128 experts, 16 rows 416 and 427, 24 rows 467
-// and 437, but with logits biased by N(0, 1) per expert 12 rows on average 326 and 309, 16 rows 360 and 306 (what an expert has
-// decides, not the mean); 64 experts of 1024 x 1536, 12 rows 52 and 53, 16 rows 61 and 53.
-// Small ones once the decode kernel's tiles of 32 rows x 128 weight rows (half a block lost per expert) are more than a wave, up to
+// Block-scaled tiles (against the decode forms of gemm_mx.cu), tile_m = 256 asks for it.  bf16 tokens from 20 rows on, e4m3 tokens, one
+// term, from 16: what an expert has decides, not the mean, and the lines lie between even routing, where the decode form stays ahead up to
+// some 24 rows, and logits biased by N(0, 1) per expert, where this one is ahead from 8 to 16 rows on.  Whole layer steps, four picks
+// (decode form, this one; even, then biased):
+//   bf16   32 experts of 2880 x 5760:  16 rows 117, 133; 113, 115.  24 rows 129, 136; 128, 131.  32 rows 150, 140; 150, 134
+//          128 experts of the same:    8 rows 358, 392; 323, 274.  16 rows 385, 404; 339, 303.  24 rows 419, 414; 412, 331
+//          64 experts of 1024 x 1536:  12 rows 50, 52; 53, 51.  16 rows 55, 55; 56, 53.  24 rows 57, 54; 63, 56
+//   e4m3   32 experts of 2880 x 5760:  16 rows 108, 127; 103, 108.  24 rows 117, 129; 117, 121.  32 rows 135, 132; 135, 127
+//          128 experts of the same:    8 rows 357, 402; 273, 257.  16 rows 356, 390; 301, 279.  24 rows 373, 402; 350, 289.  32 rows 450, 407; 431, 341
+//          64 experts of 1024 x 1536:  16 rows 50, 53; 51, 54.  24 rows 51, 52; 57, 55
+// Small ones (products with their token packs) once the decode kernel's tiles of 32 rows x 128 weight rows (half a block lost per expert) are more than a wave, up to
 // which it takes one tile's time: a product of 32 experts of 512 x 512, 16 rows 10 there, 11 here, 64 rows 21 and 13; 8 experts of
 // 512 x 2048, 16 rows 9 and 11, 80 rows 20 and 13; of 2048 x 512, 96 rows 17 and 21.
-// e4m3 tokens, one term, from 16 on: 32 experts of 2880 x 5760, 16 rows 113 and 136, 32 rows 149 and 140; 128 experts, 16 rows 366 and
-// 403, biased 301 and 256, 32 rows 514 and 435; 64 experts of 1024 x 1536, 16 rows 57 and 52.
 bool moe_gemm_mx_pair_wanted(const MoeGemmArgs& a) {
   if (a.slice_sizes && a.E > MAX_PREFIX_EXPERTS) return false;
   if (a.M >= (1ll << 31) - (1 << 20) || a.kernel == MOE_GEMM_MX_F4 || a.tile_n != 0) return false;

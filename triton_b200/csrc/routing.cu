@@ -3,8 +3,9 @@
 //
 // Semantics follow triton_kernels topk_details/_topk_forward.py:15-150, tensor_details/bitmatrix.py:43-150
 // and tensor_details/ragged_tensor.py:128-210, 310-381; the kernels themselves are organised
-// differently (one warp per token row for the top-k; a three-pass counting sort instead of
-// per-block bitonic sorts; one launch each for the ragged metadata and its remap).
+// differently (four lanes per token row for the top-k, a warp for other k; a counting sort, in one cluster for up to 32768 entries, else
+// in three passes, instead of per-block bitonic sorts; one launch each for the ragged metadata and its remap; the
+// whole step in one to three launches).
 #include "common.cuh"
 #include "topk_select.cuh"
 
@@ -225,7 +226,7 @@ __global__ void __launch_bounds__(HIST ? 1024 : 256) topk_quad_kernel(
 // ---------------------------------------------------------------------------------------------------
 // Expert histogram + stable expert-major sort.  Flat entry i = token * k + slot, expert c = indx[i]
 // (negative, or token >= n_rows: dropped).  row_sorted[i] = col_offs[c] + #{j < i : indx[j] == c},
-// col_sorted = inverse permutation; both -1 padded.
+// col_sorted = inverse permutation; both -1 padded.  Three passes (up to 32768 entries of 256 experts: bm_cluster_kernel below):
 //   pass 1: per block of kTokPerBlock tokens, a shared-memory histogram -> partial[blk][e]; both index arrays
 //           pre-filled with -1.
 //   pass 2: exclusive scan of partial[.][e] over blocks, totals -> col_sum, their exclusive scan -> col_offs.
@@ -760,16 +761,17 @@ extern "C" __attribute__((visibility("default"))) int moe_ragged_metadata_remap(
 }
 
 // ---------------------------------------------------------------------------------------------------------
-// moe_route: the whole routing step in two or three launches (the standalone entry points above take more); small batches in one launch of five
-// independent blocks (route_small_kernel), those of up to some 1500 tokens in one launch of a cluster of eight (route_cluster_kernel,
-// both at the end of this section; rule: route_form).
+// moe_route: the whole routing step in one to three launches (the standalone entry points above take more).  Small batches: one launch of five
+// independent blocks (route_small_kernel); up to some 1500 tokens: one launch of a cluster of eight (route_cluster_kernel, both at the end of
+// this section; rule: route_form).  Others: A, then route_finish_kernel where its blocks are a wave, else B and C.
 //   A  topk_quad_kernel<HIST>   top-k + softmax + bitmatrix row of every token, and the expert histogram of each block
 //      (route_topk_hist_kernel  of 128 tokens (partial[blk][e]) in the same pass over the logits;
 //       for other k)
 //   B  route_scan_ragged_kernel six blocks: exclusive scan of partial over the blocks and the expert totals (col_sum);
 //                               their exclusive scan (col_offs = slice_offs); block_offs and block schedules of the four
 //                               block sizes of the ragged metadata, which depend on the totals only;
-//   C  bm_rank_kernel           positions of the entries (unchanged).
+//   C  bm_rank_kernel           positions of the entries (unchanged);
+//   or  route_finish_kernel     B and C at once: every ranking block adds up the counts it needs itself.
 // Every token row is valid in this form (no device-side row bound, no provided indices), so each (token, slot) entry
 // receives a position and the index arrays need no -1 pre-fill.
 namespace {
@@ -977,8 +979,7 @@ __global__ void __launch_bounds__(1024) route_scan_ragged_kernel(const int32_t* 
 
 // Second and last launch of batches whose blocks are a wave: blocks 0 .. n_blocks - 1 add up the counts of the blocks before theirs and
 // of all (64 KB for 16384 tokens and 128 experts, from L2) and rank their entries, five more build the ragged metadata.  With the sums in a
-// launch between (route_scan_ragged_kernel) 2049 tokens of 128 experts, k = 4, took 15.2 us and 16384 18.2, so 11.6 and 16.6; past a wave of
-// blocks (24576: 23.9 and 27.5) and for long lists per block (200 experts, k = 6: 8192 tokens 39.0 and 33.2, 16384 43.4 and 51.4) it stays.
+// launch between (route_scan_ragged_kernel) 2049 tokens of 128 experts, k = 4, take 14.5 us, so 11.3 (rule and figures where it is launched).
 __global__ void __launch_bounds__(1024) route_finish_kernel(const int16_t* indx, int64_t ld_indx, int64_t T_rows, int E, int k, const int32_t* partial,
                                                             int n_blocks, int32_t* col_sum, int32_t* col_sorted, int32_t* row_sorted,
                                                             int32_t* slice_offs, int32_t* block_offs, int64_t ld_block_offs,
@@ -1192,7 +1193,7 @@ __global__ void __launch_bounds__(1024) route_small_kernel(
 
 constexpr int kRouteSmallTokens = 256;
 
-// The whole routing step of a batch of up to 2048 tokens in one launch of one cluster: eight blocks take an eighth of the tokens each, read
+// The whole routing step of a batch of up to 1536 tokens (2048 with short lists, see route_form) in one launch of one cluster: eight blocks take an eighth of the tokens each, read
 // one another's expert counts through distributed shared memory behind a cluster barrier, and rank their own entries on top of
 // them; blocks 3 to 7 build a row of the ragged metadata each.
 constexpr int kRouteClusterTokens = 2048;
@@ -1314,15 +1315,18 @@ extern "C" __attribute__((visibility("default"))) size_t moe_route_workspace(int
   return (size_t)((2 * nb * E + E) * (int64_t)sizeof(int32_t));
 }
 
-// us per call in a graph (small, cluster, three launches):
-//   128 experts, k = 4:  16 tokens 6.3, 7.0;  32  8.3, 7.2;  64  8.7, 7.7;  256  14.2, 10.8;  300  -, 9.2, 14.7;  1024  -, 12.8, 15.0;
-//                        1536  -, 14.5, 15.1;  2048  -, 17.3, 15.0
-//   64 experts, k = 8:   16 tokens 8.0, 7.5;  256  16.1, 14.5;  1536  -, 16.1, 18.5;  2048  -, 19.4, 18.9
-//   64 experts, k = 4:   32 tokens 8.3, 7.1;  96  7.5, 7.9;  192  9.2, 9.5;  256  11.2, 10.4;  2048  -, 14.1, 13.7
-//   32 experts, k = 4:   64 tokens 7.9, 7.4;  96  6.8, 7.8;  256  9.4, 10.5;  300  -, 8.4, 12.9;  2048  -, 12.0, 13.3
-//   8 experts, k = 2:    64 tokens 5.9, 7.0;  256  5.9, 8.1;  300  -, 7.1, 13.3;  2048  -, 8.0, 13.6
+// us per call in a graph (small, cluster, two launches, three launches):
+//   128 experts, k = 4:  16 tokens 5.6, 6.4;  32  7.7, 6.5;  64  8.1, 7.0;  256  13.6, 10.0, 10.4;  300  -, 8.5, 10.5, 13.6;  512  -, 10.5, 10.7, 13.6;
+//                        768  -, 10.4, 11.2, 14.1;  1024  -, 12.2, 11.5, 14.2;  1536  -, 13.8, 11.3, 14.4;  2048  -, 16.7, 11.6, 14.4
+//   64 experts, k = 8:   16 tokens 7.4, 7.0;  256  15.5, 13.9, 12.4;  300  -, 10.3, 12.4, 17.1;  768  -, 12.6, 12.9, 17.5;
+//                        1024  -, 15.2, 12.9, 17.6;  1536  -, 15.4, 13.2, 17.9;  2048  -, 18.9, 13.5, 18.0
+//   64 experts, k = 4:   32 tokens 7.7, 6.4;  96  6.8, 7.2;  256  10.6, 9.9, 8.8;  768  -, 9.1, 9.3;  1536  -, 11.4, 9.8, 13.1
+//   32 experts, k = 4:   64 tokens 7.4, 6.8;  96  6.3, 7.2;  256  8.8, 9.8, 7.9;  300  -, 7.9, 8.0, 11.9;  1024  -, 9.7, 8.4;  2048  -, 11.3, 8.6, 12.8
+//   8 experts, k = 2:    64 tokens 5.3, 6.0;  256  5.2, 7.6, 6.6;  300  -, 6.5, 6.7, 12.5;  2048  -, 7.4, 7.2, 12.9
+//   256 experts, k = 16: 64 tokens 26.8, 11.7, 36.7;  768  -, 29.7, 39.9;  1536  -, 44.2, 40.5;  2048  -, 56.1, 41.5
 // The small form repeats the whole selection in five blocks, the cluster has an eighth of it in each of eight and two barriers; past some
-// 1500 tokens eight SMs are fewer than the selection wants.
+// 1500 tokens eight SMs are fewer than the selection wants.  The lines above 256 tokens lie where the cluster meets three
+// launches; two launches (which only the sizes beyond take) would be ahead of it from 512 to 1024 tokens on, with 256 experts and k = 16 from 1500.
 enum { ROUTE_SMALL, ROUTE_CLUSTER, ROUTE_LAUNCHES };
 static int route_form(int64_t T, int E, int k) {
   if (!(k == 1 || k == 2 || k == 4 || k == 8 || k == 16)) return ROUTE_LAUNCHES;
@@ -1432,7 +1436,13 @@ static int route_launch(
   MOE_CHECK_LAUNCH();
   const int entries = kRouteTokPerBlock * k, warps = entries / 32 < 32 ? entries / 32 : 32;
   const size_t smem_f = (size_t)(2048 + 3 * (E + 1) + E + warps * E) * sizeof(int32_t) + (size_t)entries * sizeof(int16_t);
-  if (nb + 5 <= (E * k <= 1024 ? moe_sm_count() : 69) && smem_f <= 48 * 1024) {
+  // Two launches while the blocks are a wave, and with long lists while there are at most 64 of 128 tokens (and the five of the ragged
+  // metadata): every one of them reads the counts of all.  us with two and three launches: 128 experts, k = 4: 8192 tokens 11.9, 16.1;
+  // 16384 16.7, 17.7; 18304 18.1, 18.6; 24576 26.9, 23.5.  k = 8: 16384 25.0, 26.1; 24576 38.2, 36.5.  200 experts, k = 6: 8192 32.6, 38.4;
+  // 12288 51.4, 40.4.  256 experts, k = 8: 8192 22.1, 29.3; 12288 35.6, 31.6.  The line goes by E k: 256 experts, k = 4 are on the
+  // long side of it by their counts (8192 15.2, 19.7; 12288 23.4, 21.4; 16384 24.3, 23.1), 128 experts, k = 16 on the short one
+  // (16384 41.2, 44.1).
+  if (nb + 5 <= (E * k <= 1024 ? moe_sm_count() : 64 + 5) && smem_f <= 48 * 1024) {
     MOE_CHECK_CUDA(launch_pdl(route_finish_kernel, dim3((unsigned)nb + 5), dim3(1024), smem_f, st, indx, ld_indx, T, E, k, partial, (int)nb, col_sum,
                               col_sorted, row_sorted, slice_offs, block_offs, ld_block_offs, block_sched, ld_sched, n_sched, out));
     MOE_CHECK_LAUNCH();
@@ -1478,7 +1488,8 @@ extern "C" __attribute__((visibility("default"))) int moe_route_positions(
 // library a scratch buffer because they cannot allocate one at that point -- a serving process that handed
 // all device memory to its own pools at start-up, or a latency-critical section in which cudaMalloc (which
 // synchronises the device) is not acceptable.  The three sort passes need nb * E + E ints of scratch
-// (nb = ceil(T / 256)); here that scratch is a fixed array inside the library image.
+// (nb = ceil(T / 256)); here that scratch is a fixed array inside the library image (up to 32768 entries of 256 experts the sort is
+// one cluster and does not touch it).
 //
 // Cost: every GPU that loads libmoe_b200.so carries kNoAllocScratchBytes (1 MiB) of device memory until the
 // process exits, whether or not this entry point is ever called.

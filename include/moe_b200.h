@@ -266,7 +266,8 @@ typedef struct {
   const int32_t* x_positions;                      /* optional, what gather_indx says the other way round: row t of x goes to */
   const int16_t* x_experts; int x_k;               /* positions x_positions[t * x_k + j] (all of the M = rows_x * x_k positions
                                                       occur once), rows of expert x_experts[t * x_k + j].  With it the pair
-                                                      kernel's token pass reads a row once instead of x_k times. */
+                                                      kernel's token pass reads a row once instead of x_k times
+                                                      (x_k up to 512). */
 } MoeGemmArgs;
 int moe_grouped_gemm(const MoeGemmArgs* args_host, void* stream);
 /* Two products in a row: the same as moe_grouped_gemm of `first` and then of `second`, whose x is the first's y.  Where both run on

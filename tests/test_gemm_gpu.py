@@ -485,13 +485,46 @@ def test_layer_in_one_call_sizes_its_workspace_for_the_activation(block_scaled, 
     assert torch.equal(one, many)
 
 
+@pytest.mark.parametrize("tokens", [3, 40, 300, 1300])
+def test_layer_step_captured_behind_a_join(tokens, device):
+    """A step captured where its stream has just joined another one (two predecessors, neither of them a kernel of this package), and a second
+    step right behind it on the first one's result: the bits of the eager steps."""
+    from triton_b200.moe import moe_layer_forward
+    from triton_b200.testing import make_synthetic_layer
+    E, d, k = 8, 512, 2
+    lw = make_synthetic_layer(E, d, 736, device, seed=3, block_scaled=True)
+    g = torch.Generator(device=device).manual_seed(tokens)
+    x, logits = torch.randn(tokens, d, device=device, generator=g).bfloat16(), torch.randn(tokens, E, device=device, generator=g)
+    side = torch.cuda.Stream(device=device)
+
+    def step():
+        side.wait_stream(torch.cuda.current_stream(device))
+        with torch.cuda.stream(side):
+            xs = x * 2
+        ls = logits + 1
+        torch.cuda.current_stream(device).wait_stream(side)
+        xs.record_stream(torch.cuda.current_stream(device))
+        z = moe_layer_forward(xs, ls, lw, k)
+        return z, moe_layer_forward(z, ls, lw, k)
+
+    eager = [t.clone() for t in step()]
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = step()
+    for _ in range(3):
+        graph.replay()
+    torch.cuda.synchronize()
+    tb.matmul_check_status()
+    assert all(torch.equal(a, b) for a, b in zip(eager, captured))
+
+
 @pytest.mark.parametrize("tokens, experts, dtype", [(3, 8, "bf16"), (40, 8, "bf16"), (300, 8, "bf16"), (1300, 8, "bf16"), (2100, 16, "bf16"),
                                                     (40, 8, "e4m3"), (300, 8, "e4m3"), (1300, 8, "e4m3")])
-def test_layer_step_captured_behind_a_join(tokens, experts, dtype, device):
-    """A step captured where its stream has just joined another one (two predecessors, neither of them a kernel of this package), and a second
-    step with other routing right behind it on the first one's result.  Before every replay tokens, logits (with very different expert
+def test_captured_layer_steps_with_changed_inputs(tokens, experts, dtype, device):
+    """As above, the second step with routing of its own.  Before every replay tokens, logits (with very different expert
     loads) and weights are overwritten in place: a kernel that reads what the replay before has left gives other bits than the eager steps.
-    One to three launches of routing, tokens packed by position and by row, both block-scaled kernels."""
+    Routing in one and in two launches, tokens packed by position and by row, both block-scaled kernels."""
     from triton_b200.moe import moe_layer_forward
     from triton_b200.testing import make_synthetic_layer
     d, k, sets = 512, 2, 3

@@ -111,9 +111,10 @@ def test_router_topk_against_reference_fixture(golden, name, device):
     assert (sp.vals.cpu().float()[same] - g["vals"].float()[same]).abs().max().item() <= 2.0 ** -8
 
 
-@pytest.mark.parametrize("case", [(129, 2880, 128, 4), (131, 512, 20, 2), (137, 1024, 256, 8), (386, 1024, 64, 4), (4100, 1536, 100, 4), (8000, 1536, 16, 2)])
+@pytest.mark.parametrize("case", [(129, 2880, 128, 4), (131, 512, 20, 2), (137, 1024, 256, 8), (1800, 512, 64, 4), (4100, 320, 100, 4), (8000, 576, 16, 2),
+                                  (386, 1024, 64, 4), (4100, 1536, 100, 4), (8000, 1536, 16, 2)])
 def test_router_topk_slices_of_a_cluster(case, device):
-    """2 to 11 slices of K per token block, last blocks of 1, 3, 9, 2, 4 and 64 rows: shares of the rows that are empty or partial."""
+    """1 to 11 slices of K per token block, last blocks of 1, 2, 3, 4, 8, 9 and 64 rows: shares of the rows that are empty or partial."""
     test_router_topk_against_oracle(case, torch.float32, True, device)
 
 

@@ -134,6 +134,21 @@ __device__ __forceinline__ void elect_tile_3d(uint32_t dst, const CUtensorMap* t
       "l"(tmap), "r"(x), "r"(y), "r"(z), "r"(bar)
       : "memory");
 }
+__device__ __forceinline__ void elect_tile_3d_hint(uint32_t dst, const CUtensorMap* tmap, int x, int y, int z, uint32_t bar, uint64_t policy) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\telect.sync _|q, 0xFFFFFFFF;\n\t"
+      "@q cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3, %4}], [%5], %6;\n\t}" ::"r"(dst),
+      "l"(tmap), "r"(x), "r"(y), "r"(z), "r"(bar), "l"(policy)
+      : "memory");
+}
+// the same with a cache policy
+__device__ __forceinline__ void elect_bulk_g2s_hint(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar, uint64_t policy) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\telect.sync _|q, 0xFFFFFFFF;\n\t"
+      "@q cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;\n\t}" ::"r"(dst),
+      "l"(src), "r"(bytes), "r"(bar), "l"(policy)
+      : "memory");
+}
 __device__ __forceinline__ void elect_tile_4d(uint32_t dst, const CUtensorMap* tmap, int x, int y, int z, int w, uint32_t bar) {
   asm volatile(
       "{\n\t.reg .pred q;\n\telect.sync _|q, 0xFFFFFFFF;\n\t"

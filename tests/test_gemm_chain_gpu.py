@@ -173,3 +173,54 @@ def test_positions_of_a_row_beyond_a_block_of_shared_memory(k, device):
         assert int(p.status) == 0
         out.append(y)
     assert torch.equal(*out) and bool(out[0].abs().sum() > 0)
+
+
+class Passes:
+    """One product over `rows` rows of x, each at k positions, to be called without and with the positions of every row."""
+
+    def __init__(self, rows, k, depth, block, device, e4m3=False):
+        g = torch.Generator(device=device).manual_seed(rows * k)
+        x = torch.randn(rows, depth, device=device, generator=g).bfloat16()
+        self.x = x.to(torch.float8_e4m3fn) if e4m3 else x
+        lw = make_synthetic_layer(E, depth, 64, device, seed=3, block_scaled=True)
+        experts = torch.randint(0, E, (rows * k,), device=device, generator=g).short()
+        experts[: rows * k // 2] = 1                               # one expert of several blocks
+        order = torch.argsort(experts, stable=True)
+        positions = torch.empty(rows * k, dtype=torch.int32, device=device)
+        positions[order] = torch.arange(rows * k, dtype=torch.int32, device=device)
+        gather = (order // k).int()
+        ragged = make_ragged_tensor_metadata(torch.bincount(experts.long(), minlength=E).int(), rows * k)
+        self.status = torch.zeros(1, dtype=torch.int32, device=device)
+        self.n, self.k, self.experts, self.positions = rows * k, k, experts, positions
+        self.keep = [lw, gather, ragged]
+        a = self.a = Args()
+        a.w_kind, a.w, a.w_scale = _lib.MOE_W_MX4_B200MX, lw.w1_bs.storage.data.data_ptr(), lw.w1_bs_scale.storage.data.data_ptr()
+        a.E, a.K, a.N, a.M = E, depth, 128, rows * k
+        a.slice_sizes, a.slice_offs = ragged.slice_sizes.data_ptr(), ragged.slice_offs.data_ptr()
+        a.block_offs_16, a.block_sched_16 = ragged.block_offs_data.data_ptr(), ragged.block_schedule_data.data_ptr()
+        a.ld_block_offs, a.ld_block_sched = ragged.block_offs_data.stride(0), ragged.block_schedule_data.stride(0)
+        a.x, a.ld_x, a.rows_x, a.gather_indx = self.x.data_ptr(), depth, rows, gather.data_ptr()
+        a.x_dtype, a.y_dtype, a.ld_y = CONST["MOE_F8E4M3" if e4m3 else "MOE_BF16"], CONST["MOE_BF16"], 128
+        a.tile_m, a.status = block, self.status.data_ptr()
+
+    def run(self, by_row, kernel):
+        lib, a = _lib.load(), self.a
+        ws = torch.empty(int(lib.moe_gemm_mx_workspace_bytes(C.byref(a))) + 1024, dtype=torch.uint8, device=self.x.device)
+        a.mx_workspace, a.mx_workspace_bytes = (ws.data_ptr() + 1023) // 1024 * 1024, ws.numel() - 1024
+        y = torch.zeros(self.n, 128, device=self.x.device, dtype=torch.bfloat16)
+        a.y = y.data_ptr()
+        a.x_positions, a.x_experts, a.x_k = (self.positions.data_ptr(), self.experts.data_ptr(), self.k) if by_row else (None, None, 0)
+        assert lib.moe_gemm_kernel_name(C.byref(a)) == kernel
+        _lib.check(lib.moe_grouped_gemm(C.byref(a), torch.cuda.current_stream().cuda_stream), "product")
+        torch.cuda.synchronize()
+        assert int(self.status) == 0
+        return y
+
+
+# blocks of four e2m1 terms, of two e4m3 terms that fit their rows and that do not, e4m3 tokens; depths of whole and of cut k steps
+@pytest.mark.parametrize("block, e4m3", [(16, False), (32, False), (64, False), (32, True)])
+@pytest.mark.parametrize("rows, k, depth", [(1, 1, 96), (5, 3, 512), (17, 4, 736), (33, 2, 160), (3, 40, 128)])
+def test_decode_tokens_by_row_are_those_by_position(block, e4m3, rows, k, depth, device):
+    p = Passes(rows, k, depth, block, device, e4m3)
+    by_position, by_row = p.run(False, b"gemm_mx_kernel"), p.run(True, b"gemm_mx_kernel")
+    assert torch.equal(by_position, by_row) and bool(by_row.abs().sum() > 0)

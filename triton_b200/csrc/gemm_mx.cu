@@ -155,6 +155,49 @@ struct PackParams {
   uint8_t* out;
 };
 
+// four consecutive values of row `src` (lane l of a warp: k = 128 kt + 4 l), 0 where there are none
+__device__ __forceinline__ void pack_load4(const PackParams& a, int64_t src, int k, bool live, float (&v)[4]) {
+  uint2 raw = make_uint2(0, 0);
+  if (live) raw = *reinterpret_cast<const uint2*>((const __nv_bfloat16*)a.x + src * a.ld_x + k);
+  v[0] = __uint_as_float(raw.x << 16); v[1] = __uint_as_float(raw.x & 0xFFFF0000u);
+  v[2] = __uint_as_float(raw.y << 16); v[3] = __uint_as_float(raw.y & 0xFFFF0000u);
+}
+__device__ __forceinline__ void pack_load1(const PackParams& a, int64_t src, int k, bool live, uint32_t& word, uint32_t& s) {
+  word = 0;
+  s = 127;
+  if (live) {
+    word = *reinterpret_cast<const uint32_t*>((const uint8_t*)a.x + src * a.ld_x + k);
+    if (a.x_scale) s = a.x_scale[src * a.ld_xs + (k >> 5)];
+  }
+}
+struct TwoTerms { uint32_t hi, lo, s_hi, s_lo; };
+__device__ __forceinline__ void pack_two_terms(const float (&v)[4], TwoTerms& q) {
+  float amax = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
+#pragma unroll
+  for (int o = 1; o <= 4; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
+  if (!(amax < 3.0e38f)) amax = 3.0e38f;          // Inf / NaN in the group: keep the scale finite
+  float s_hi, i_hi;
+  mx8_scale(amax, q.s_hi, s_hi, i_hi);
+  const uint32_t h01 = f32x2_to_e4m3x2(v[0] * i_hi, v[1] * i_hi), h23 = f32x2_to_e4m3x2(v[2] * i_hi, v[3] * i_hi);
+  const float2 f01 = e4m3x2_to_f32x2(h01), f23 = e4m3x2_to_f32x2(h23);
+  float rs[4] = {v[0] - f01.x * s_hi, v[1] - f01.y * s_hi, v[2] - f23.x * s_hi, v[3] - f23.y * s_hi};
+  float rmax = fmaxf(fmaxf(fabsf(rs[0]), fabsf(rs[1])), fmaxf(fabsf(rs[2]), fabsf(rs[3])));
+#pragma unroll
+  for (int o = 1; o <= 4; o <<= 1) rmax = fmaxf(rmax, __shfl_xor_sync(0xFFFFFFFFu, rmax, o));
+  if (!(rmax < 3.0e38f)) rmax = 0.0f;
+  float s_lo, i_lo;
+  mx8_scale(rmax, q.s_lo, s_lo, i_lo);
+  const uint32_t l01 = f32x2_to_e4m3x2(rs[0] * i_lo, rs[1] * i_lo), l23 = f32x2_to_e4m3x2(rs[2] * i_lo, rs[3] * i_lo);
+  q.hi = h01 | (h23 << 16);
+  q.lo = l01 | (l23 << 16);
+}
+// a lane's four e4m3 codes in line `line` of a chunk of `lines` lines, and its group's scale
+__device__ __forceinline__ void pack_store8(uint8_t* chunk, int lines, int line, uint32_t g, int lane, uint32_t codes, uint32_t s) {
+  const uint32_t piece = (uint32_t)(lane >> 2), within = (uint32_t)(lane & 3) * 4u;
+  *reinterpret_cast<uint32_t*>(chunk + line * 128 + ((piece ^ (uint32_t)(line & 7)) << 4) + within) = codes;
+  if ((lane & 7) == 0) chunk[lines * 128 + (line & 31) * 16 + (line >> 5) * 4 + g] = (uint8_t)s;
+}
+
 template <bool SPLIT>
 __global__ void __launch_bounds__(256) mx_pack_x_kernel(const GemmParams p, const PackParams a) {
   pdl_begin();
@@ -164,55 +207,25 @@ __global__ void __launch_bounds__(256) mx_pack_x_kernel(const GemmParams p, cons
   if (!mx_map_block(p, a.tb, slot, e, row0, rows)) return;
   uint8_t* chunk = a.out + (slot * a.KT + kt) * a.chunk_bytes;
   const int lines = !SPLIT ? a.n_mma : a.fit ? chunk_lines(rows) : a.tb;
-  uint8_t* sc = chunk + (SPLIT ? 2 : 1) * lines * 128;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int k = kt * 128 + lane * 4;
-  const int g = lane >> 3;
-  const uint32_t piece = (uint32_t)(lane >> 2), within = (uint32_t)(lane & 3) * 4u;
+  const uint32_t g = (uint32_t)(lane >> 3);
   for (int r = warp; r < rows; r += 8) {
     const int64_t m = row0 + r;
     int64_t src = a.gather ? (int64_t)a.gather[m] : m;
     if (src >= a.rows_x) src = -1;
     const bool live = src >= 0 && k < a.K;        // K % 32 == 0: a lane's four values are in or out together
     if constexpr (SPLIT) {
-      float v[4] = {0.f, 0.f, 0.f, 0.f};
-      if (live) {
-        const uint2 raw = *reinterpret_cast<const uint2*>((const __nv_bfloat16*)a.x + src * a.ld_x + k);
-        v[0] = __uint_as_float(raw.x << 16); v[1] = __uint_as_float(raw.x & 0xFFFF0000u);
-        v[2] = __uint_as_float(raw.y << 16); v[3] = __uint_as_float(raw.y & 0xFFFF0000u);
-      }
-      float amax = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
-#pragma unroll
-      for (int o = 1; o <= 4; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
-      if (!(amax < 3.0e38f)) amax = 3.0e38f;      // Inf / NaN in the group: keep the scale finite
-      uint32_t sb_hi; float s_hi, i_hi;
-      mx8_scale(amax, sb_hi, s_hi, i_hi);
-      const uint32_t h01 = f32x2_to_e4m3x2(v[0] * i_hi, v[1] * i_hi), h23 = f32x2_to_e4m3x2(v[2] * i_hi, v[3] * i_hi);
-      const float2 f01 = e4m3x2_to_f32x2(h01), f23 = e4m3x2_to_f32x2(h23);
-      float rs[4] = {v[0] - f01.x * s_hi, v[1] - f01.y * s_hi, v[2] - f23.x * s_hi, v[3] - f23.y * s_hi};
-      float rmax = fmaxf(fmaxf(fabsf(rs[0]), fabsf(rs[1])), fmaxf(fabsf(rs[2]), fabsf(rs[3])));
-#pragma unroll
-      for (int o = 1; o <= 4; o <<= 1) rmax = fmaxf(rmax, __shfl_xor_sync(0xFFFFFFFFu, rmax, o));
-      if (!(rmax < 3.0e38f)) rmax = 0.0f;
-      uint32_t sb_lo; float s_lo, i_lo;
-      mx8_scale(rmax, sb_lo, s_lo, i_lo);
-      const uint32_t l01 = f32x2_to_e4m3x2(rs[0] * i_lo, rs[1] * i_lo), l23 = f32x2_to_e4m3x2(rs[2] * i_lo, rs[3] * i_lo);
-      const int r_lo = lines + r;
-      *reinterpret_cast<uint32_t*>(chunk + r * 128 + ((piece ^ (uint32_t)(r & 7)) << 4) + within) = h01 | (h23 << 16);
-      *reinterpret_cast<uint32_t*>(chunk + r_lo * 128 + ((piece ^ (uint32_t)(r_lo & 7)) << 4) + within) = l01 | (l23 << 16);
-      if ((lane & 7) == 0) {
-        sc[(r & 31) * 16 + (r >> 5) * 4 + g] = (uint8_t)sb_hi;
-        sc[(r_lo & 31) * 16 + (r_lo >> 5) * 4 + g] = (uint8_t)sb_lo;
-      }
+      float v[4];
+      pack_load4(a, src, k, live, v);
+      TwoTerms q;
+      pack_two_terms(v, q);
+      pack_store8(chunk, 2 * lines, r, g, lane, q.hi, q.s_hi);
+      pack_store8(chunk, 2 * lines, lines + r, g, lane, q.lo, q.s_lo);
     } else {
-      uint32_t w = 0;
-      if (live) w = *reinterpret_cast<const uint32_t*>((const uint8_t*)a.x + src * a.ld_x + k);
-      *reinterpret_cast<uint32_t*>(chunk + r * 128 + ((piece ^ (uint32_t)(r & 7)) << 4) + within) = w;
-      if ((lane & 7) == 0) {
-        uint8_t s = 127;
-        if (live && a.x_scale) s = a.x_scale[src * a.ld_xs + (k >> 5)];
-        sc[(r & 31) * 16 + (r >> 5) * 4 + g] = s;
-      }
+      uint32_t word, s;
+      pack_load1(a, src, k, live, word, s);
+      pack_store8(chunk, lines, r, g, lane, word, s);
     }
   }
 }
@@ -227,6 +240,16 @@ __global__ void __launch_bounds__(256) mx_pack_x_kernel(const GemmParams p, cons
 // four warps instead of eight: 8 % slower.)  (A warp per (token block, k step, four rows) with the rows' chains side by side, and dead warps grouped into whole
 // CTAs, was tried in place of the loop over rows below: 2.3 x slower.  A row's four-term chain is latency, and four of
 // them in one warp add up where eight warps of a CTA overlap them.)
+__device__ __forceinline__ uint32_t group_max_bits(uint32_t top) {        // over the 8 lanes that hold a group
+#pragma unroll
+  for (int o = 1; o <= 4; o <<= 1) top = max(top, __shfl_xor_sync(0xFFFFFFFFu, top, o));
+  return top;
+}
+// a lane's four e2m1 codes in line `line` of a chunk of `lines` lines, and its group's scale
+__device__ __forceinline__ void pack_store4(uint8_t* chunk, int lines, int line, uint32_t g, int lane, uint32_t codes, uint32_t sb) {
+  *reinterpret_cast<uint16_t*>(chunk + line * 64 + ((g ^ (uint32_t)((line >> 1) & 3)) << 4) + (uint32_t)(lane & 7) * 2u) = (uint16_t)codes;      // a 32-group is one 16-byte piece
+  if ((lane & 7) == 0) chunk[lines * 64 + (line & 31) * 16 + (line >> 5) * 4 + (int)g] = (uint8_t)sb;
+}
 __global__ void __launch_bounds__(256) mx_pack_x4_kernel(const GemmParams p, const PackParams a) {
   pdl_begin();
   const int64_t slot = blockIdx.x;
@@ -234,33 +257,89 @@ __global__ void __launch_bounds__(256) mx_pack_x4_kernel(const GemmParams p, con
   int e; int64_t row0; int rows;
   if (!mx_map_block(p, a.tb, slot, e, row0, rows)) return;
   uint8_t* chunk = a.out + (slot * a.KT + kt) * a.chunk_bytes;
-  uint8_t* sc = chunk + (int64_t)a.n_mma * 64;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int k = kt * 128 + lane * 4;
-  const uint32_t g = (uint32_t)(lane >> 3), within = (uint32_t)(lane & 7) * 2u;     // a 32-group is one 16-byte piece
+  const uint32_t g = (uint32_t)(lane >> 3);
   for (int r = warp; r < rows; r += 8) {
     const int64_t m = row0 + r;
     int64_t src = a.gather ? (int64_t)a.gather[m] : m;
     if (src >= a.rows_x) src = -1;
-    float v[4] = {0.f, 0.f, 0.f, 0.f};
-    if (src >= 0 && k < a.K) {
-      const uint2 raw = *reinterpret_cast<const uint2*>((const __nv_bfloat16*)a.x + src * a.ld_x + k);
-      v[0] = __uint_as_float(raw.x << 16); v[1] = __uint_as_float(raw.x & 0xFFFF0000u);
-      v[2] = __uint_as_float(raw.y << 16); v[3] = __uint_as_float(raw.y & 0xFFFF0000u);
-    }
+    float v[4];
+    pack_load4(a, src, k, src >= 0 && k < a.K, v);
     const bool nan[4] = {v[0] != v[0], v[1] != v[1], v[2] != v[2], v[3] != v[3]};      // e2m1 has no NaN: such a value counts as 0
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
       uint32_t codes;
-      const uint32_t sb = e2m1_term(t, v, nan, codes, [](uint32_t top) {       // over the 8 lanes that hold the group
-#pragma unroll
-        for (int o = 1; o <= 4; o <<= 1) top = max(top, __shfl_xor_sync(0xFFFFFFFFu, top, o));
-        return top;
-      });
-      const int rt = t * a.tb + r;
-      *reinterpret_cast<uint16_t*>(chunk + rt * 64 + ((g ^ (uint32_t)((rt >> 1) & 3)) << 4) + within) = (uint16_t)codes;
-      if ((lane & 7) == 0) sc[(rt & 31) * 16 + (rt >> 5) * 4 + (int)g] = (uint8_t)sb;
+      const uint32_t sb = e2m1_term(t, v, nan, codes, group_max_bits);
+      pack_store4(chunk, a.n_mma, t * a.tb + r, g, lane, codes, sb);
     }
+  }
+}
+
+// The same with the tokens of x in turn, given the positions of every one (positions, experts: k per token): a warp takes a token's k step,
+// quantises it once and writes its lines for each of the k positions.  The pass is a chain of latencies: by position it runs a block
+// for every (token block, k step) the schedule may hold, most of them without rows, and a warp's rows follow one another.  64 tokens of 128
+// experts 7.2 -> 4.0 us of a step, 300 tokens 10.3 -> 5.1; steps of 64 tokens of 128 and 32 experts 159.2 -> 155.3 and 100.5 -> 97.9.
+struct PackRows {
+  const int32_t* positions; const int16_t* experts;      // [rows_x, k]
+  int k;
+};
+// chunk (at its k step) and lines of a term of pick `at` of [rows_x, k], and the row in its block
+struct PickChunk { uint8_t* chunk; int r, lines; };
+__device__ __forceinline__ PickChunk pick_chunk(const GemmParams& p, const PackParams& a, const PackRows& w, int64_t at, int kt, bool split) {
+  const int e = w.experts[at], rr = w.positions[at] - p.slice_offs[e], j = rr / a.tb;
+  PickChunk c;
+  c.r = rr - j * a.tb;
+  c.lines = !split ? a.n_mma : a.fit ? chunk_lines(min(a.tb, p.slice_sizes[e] - j * a.tb)) : a.tb;
+  c.chunk = a.out + ((int64_t)(p.block_offs[e] + j) * a.KT + kt) * a.chunk_bytes;
+  return c;
+}
+// `store`(chunk, r, lines) for each pick of token t, by the whole warp
+template <typename F>
+__device__ __forceinline__ void each_pick(const GemmParams& p, const PackParams& a, const PackRows& w, int64_t t, int kt, bool split, F store) {
+  const int lane = threadIdx.x & 31;
+  for (int j0 = 0; j0 < w.k; j0 += 32) {
+    PickChunk own{nullptr, 0, 0};
+    if (j0 + lane < w.k) own = pick_chunk(p, a, w, t * w.k + j0 + lane, kt, split);
+    for (int j = 0; j < min(32, w.k - j0); ++j)
+      store((uint8_t*)__shfl_sync(0xFFFFFFFFu, (unsigned long long)own.chunk, j), __shfl_sync(0xFFFFFFFFu, own.r, j),
+            __shfl_sync(0xFFFFFFFFu, own.lines, j));
+  }
+}
+// FORM: terms of a token
+template <int FORM>
+__global__ void __launch_bounds__(256) mx_pack_rows_kernel(const GemmParams p, const PackParams a, const PackRows w) {
+  pdl_begin();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t unit = (int64_t)blockIdx.x * 8 + warp, t = unit / a.KT;
+  if (t >= a.rows_x) return;
+  const int kt = (int)(unit - t * a.KT), k = kt * 128 + lane * 4;
+  const bool live = k < a.K;
+  const uint32_t g = (uint32_t)(lane >> 3);
+  if constexpr (FORM == 4) {
+    float v[4];
+    pack_load4(a, t, k, live, v);
+    const bool nan[4] = {v[0] != v[0], v[1] != v[1], v[2] != v[2], v[3] != v[3]};
+    uint32_t codes[4], sb[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) sb[i] = e2m1_term(i, v, nan, codes[i], group_max_bits);
+    each_pick(p, a, w, t, kt, true, [&](uint8_t* chunk, int r, int lines) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) pack_store4(chunk, a.n_mma, i * lines + r, g, lane, codes[i], sb[i]);
+    });
+  } else if constexpr (FORM == 2) {
+    float v[4];
+    pack_load4(a, t, k, live, v);
+    TwoTerms q;
+    pack_two_terms(v, q);
+    each_pick(p, a, w, t, kt, true, [&](uint8_t* chunk, int r, int lines) {
+      pack_store8(chunk, 2 * lines, r, g, lane, q.hi, q.s_hi);
+      pack_store8(chunk, 2 * lines, lines + r, g, lane, q.lo, q.s_lo);
+    });
+  } else {
+    uint32_t word, s;
+    pack_load1(a, t, k, live, word, s);
+    each_pick(p, a, w, t, kt, false, [&](uint8_t* chunk, int r, int lines) { pack_store8(chunk, lines, r, g, lane, word, s); });
   }
 }
 
@@ -915,8 +994,14 @@ int moe_gemm_mx_launch(const GemmParams& p_in, const MoeGemmArgs& a, const Token
   const dim3 pgrid((unsigned)pl.grid_m, (unsigned)pl.KT);
   MOE_CHECK_ARG(pl.grid_m * pl.n_groups < 2147483647LL - 65536, "moe_grouped_gemm: too many token blocks");
   if (!packed) {
-    auto pack = pl.f4 ? mx_pack_x4_kernel : pl.split > 1 ? mx_pack_x_kernel<true> : mx_pack_x_kernel<false>;
-    MOE_CHECK_CUDA(launch_pdl(pack, pgrid, dim3(256), 0, st, p, pk));
+    if (a.x_positions && a.x_experts && a.x_k > 0 && a.slice_sizes && a.rows_x * a.x_k == a.M && cdiv64(a.rows_x * pl.KT, 8) < 2147483647LL) {
+      const PackRows rows{a.x_positions, a.x_experts, a.x_k};
+      auto pack = pl.f4 ? mx_pack_rows_kernel<4> : pl.split > 1 ? mx_pack_rows_kernel<2> : mx_pack_rows_kernel<1>;
+      MOE_CHECK_CUDA(launch_pdl(pack, dim3((unsigned)cdiv64(a.rows_x * pl.KT, 8)), dim3(256), 0, st, p, pk, rows));
+    } else {
+      auto pack = pl.f4 ? mx_pack_x4_kernel : pl.split > 1 ? mx_pack_x_kernel<true> : mx_pack_x_kernel<false>;
+      MOE_CHECK_CUDA(launch_pdl(pack, pgrid, dim3(256), 0, st, p, pk));
+    }
     MOE_CHECK_LAUNCH();
   }
 

@@ -64,7 +64,7 @@ template <int FORM> constexpr int SF_COLS = FORM == PP_TWO ? 24 : 16;      // te
 struct PairParams {
   const uint8_t* xq;            // [k step][padded row / 8][term][8 rows][128 B], 16-byte pieces swizzled with (row & 7)
   const uint8_t* xs;            // [k step][padded row / 8][term][8 rows][4 B]: e8m0 of the four 32-groups
-  const uint8_t* done;          // [padded row]: the pack kernel has written its outputs itself (two-term tokens)
+  const uint32_t* done;         // [padded row], not zero: the pack kernel has written its outputs itself (two-term tokens)
   int64_t prows;                // padded rows: expert e's rows start at (slice_offs[e] & ~31) + 32 e
   int KT, NB;                   // 128-k steps, 128-row weight blocks
   int nmax;                     // token columns of a tile at most, a multiple of 32
@@ -92,7 +92,8 @@ struct PairPackParams {
   int K, KT, NB, y_dtype;
   int64_t prows;
   uint8_t* xq; uint8_t* xs;
-  uint8_t* done;
+  uint32_t* done;
+  int parts;                     // blocks (1, 2 or 4) that share the groups of 16 rows; each has its bytes of the rows' words
   const int32_t* positions; const int16_t* experts;      // [rows_x, k]: where the rows of x go (NULL: gather says)
   int k;
   TokenOut out;                  // the product's rows are the next one's tokens: those computed here go there too
@@ -273,14 +274,15 @@ __device__ __noinline__ uint32_t exact_rows(const GemmParams& p, const PairPackP
 // no exchange between lanes, 64 bytes in, a 32-byte sector out per term.  With eight k per lane and four lanes to a group, 65536
 // rows of 2880 took 153 us and 4800 rows 20.3, so 141 and 16.8.
 template <bool TILED>
-__global__ void __launch_bounds__(256) mx_pair_pack2_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ PairPackParams a) {
+__global__ void __launch_bounds__(256, 3) mx_pair_pack2_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ PairPackParams a) {
   pdl_begin();
   int e; int64_t row0, prow0; int rows;
-  if (!pack_block(p, blockIdx.x, e, row0, rows, prow0)) return;
-  const int G = a.KT * 4;
+  const int part = (int)(blockIdx.x & (unsigned)(a.parts - 1));
+  if (!pack_block(p, blockIdx.x / (unsigned)a.parts, e, row0, rows, prow0)) return;
+  const int kt0 = part * a.KT / a.parts, G = ((part + 1) * a.KT / a.parts - kt0) * 4;      // groups of this part's k steps
   bool beyond = false;
   for (int t = threadIdx.x; t < rows * G; t += 256) {
-    const int r = t / G, g = t - r * G;
+    const int r = t / G, g = kt0 * 4 + t - r * G;
     int64_t src = a.gather ? (int64_t)a.gather[row0 + r] : row0 + r;
     if (src >= a.rows_x) src = -1;
     uint4 raw[4] = {};
@@ -295,7 +297,13 @@ __global__ void __launch_bounds__(256) mx_pair_pack2_kernel(const __grid_constan
   }
   uint32_t done = 0;
   if (__syncthreads_or(beyond)) done = exact_rows<TILED>(p, a, e, row0, rows);
-  if ((int)threadIdx.x < rows) a.done[prow0 + threadIdx.x] = (uint8_t)((done >> threadIdx.x) & 1u);
+  if ((int)threadIdx.x < rows) {
+    uint32_t* word = a.done + prow0 + threadIdx.x;
+    const uint32_t bit = (done >> threadIdx.x) & 1u;
+    if (a.parts == 1) *word = bit;
+    else if (a.parts == 2) ((uint16_t*)word)[part] = (uint16_t)bit;
+    else ((uint8_t*)word)[part] = (uint8_t)bit;
+  }
 }
 
 // The same with the rows of x in turn, given the positions of every one (positions, experts: k per row): a row that k experts take is read
@@ -341,7 +349,7 @@ __global__ void __launch_bounds__(256) mx_pair_pack2_rows_kernel(const __grid_co
   }
   __syncthreads();
   const uint32_t beyond = s_beyond;
-  for (int i = threadIdx.x; i < n * a.k; i += 256) a.done[s_prow[i]] = (uint8_t)((beyond >> (i / a.k)) & 1u);
+  for (int i = threadIdx.x; i < n * a.k; i += 256) a.done[s_prow[i]] = (beyond >> (i / a.k)) & 1u;
   if (beyond)
     for (int i = 0; i < n * a.k; ++i)
       if ((beyond >> (i / a.k)) & 1u) {
@@ -846,7 +854,7 @@ PairPlan pair_plan(const MoeGemmArgs& a) {
   pl.prows = cdiv64(a.M, 32) * 32 + 32 * (E + 1);
   pl.xs_off = pl.terms * pl.KT * pl.prows * 128;
   pl.done_off = pl.xs_off + pl.terms * pl.KT * pl.prows * 4;
-  pl.ws_bytes = pl.done_off + pl.prows;
+  pl.ws_bytes = pl.done_off + pl.prows * 4;
   return pl;
 }
 
@@ -1031,10 +1039,11 @@ int moe_gemm_mx_pair_launch(const GemmParams& p_in, const MoeGemmArgs& a, const 
   pk.x_scale = a.x_scale; pk.ld_xs = a.ld_x_scale;
   pk.gather = a.gather_indx;
   pk.K = a.K; pk.KT = pl.KT; pk.NB = pl.NB; pk.y_dtype = a.y_dtype; pk.prows = pl.prows;
-  pk.xq = (uint8_t*)a.mx_workspace; pk.xs = pk.xq + pl.xs_off; pk.done = pk.xq + pl.done_off;
+  pk.xq = (uint8_t*)a.mx_workspace; pk.xs = pk.xq + pl.xs_off; pk.done = (uint32_t*)(pk.xq + pl.done_off);
   const bool tiled = a.w_kind == MOE_W_MX4_B200;
   pk.out = out;
   pk.positions = nullptr; pk.experts = nullptr; pk.k = 0;
+  pk.parts = 1;
   if (!packed) {
     // by rows of x where every one of them has its k positions, several (and no more than a block has shared memory for), and their blocks
     // fill the SMs (256 rows, two positions each: 27.6 us per layer step by position, 28.1 by row)
@@ -1046,7 +1055,10 @@ int moe_gemm_mx_pair_launch(const GemmParams& p_in, const MoeGemmArgs& a, const 
                                 pl.terms == 1 ? 0 : (size_t)PACK_TOKENS * a.x_k * sizeof(int64_t), st, p, pk));
     } else {
       auto pack = pl.terms == 1 ? mx_pair_pack1_kernel : tiled ? mx_pair_pack2_kernel<true> : mx_pair_pack2_kernel<false>;
-      MOE_CHECK_CUDA(launch_pdl(pack, dim3((unsigned)blocks16), dim3(256), 0, st, p, pk));
+      // Blocks of 16 rows in parts of a turn or two of their threads (32 experts of 2880 x 5760, 256 tokens: 146.3 us per step whole, 144.9 in two
+      // parts, 144.1 in four; 512 deep, four k steps: 29.4 whole, 30.1 in four).
+      if (pl.terms == 2) pk.parts = pl.KT >= 16 ? 4 : pl.KT >= 8 ? 2 : 1;
+      MOE_CHECK_CUDA(launch_pdl(pack, dim3((unsigned)(blocks16 * pk.parts)), dim3(256), 0, st, p, pk));
     }
     MOE_CHECK_LAUNCH();
   }

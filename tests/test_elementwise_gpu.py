@@ -50,6 +50,20 @@ def test_reduce(shape, dim, mask_mode, device):
     torch.testing.assert_close(y.cpu().float(), ref.float(), atol=1e-2, rtol=1e-2)
 
 
+# slots around the four that are loaded together; rows apart from one another and slots outermost
+@pytest.mark.parametrize("R", [1, 3, 4, 5, 8, 9])
+@pytest.mark.parametrize("slots_first", [False, True])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_plain_sum_adds_the_slots_in_order(R, slots_first, dtype, device):
+    g = torch.Generator(device=device).manual_seed(R)
+    x = torch.randn((R, 37, 48) if slots_first else (37, R, 48), device=device, generator=g).to(dtype)[..., :40]
+    y, _ = tb.reduce(x, 0 if slots_first else 1)
+    want = torch.zeros(37, 40, device=device)
+    for r in range(R):
+        want += (x[r] if slots_first else x[:, r]).float()
+    assert torch.equal(y, want.to(dtype))
+
+
 @pytest.mark.parametrize("n_out, d", [(500, 96), (5000, 2880), (40000, 64), (700001, 32)])
 def test_gather_rows_over_peer_buffers(n_out, d, device):
     """moe_gather_rows_peers with three buffers on one device standing in for three ranks: -1 writes zeros, -2 leaves

@@ -267,6 +267,38 @@ extern "C" __attribute__((visibility("default"))) int moe_swiglu(const void* a, 
   return MOE_OK;
 }
 
+// The plain sum over R slots of rows of 16-byte vectors: HBM-bound, so the loads of four slots are under way before the first is added (with one
+// at a time a thread had 16 bytes in flight: the combine of 16384 tokens 104 -> 93 us, of 8192 50 -> 44).  Same order of additions as reduce_kernel.
+template <typename TX, typename TY>
+__global__ void __launch_bounds__(256) sum_slots_kernel(const TX* x, int R, uint32_t per_row, uint32_t total, int64_t sx_r, int64_t sx_0, TY* y,
+                                                        int64_t sy_0) {
+  pdl_begin();
+  for (uint32_t i = blockIdx.x * 256u + threadIdx.x; i < total; i += gridDim.x * 256u) {
+    const uint32_t s0 = i / per_row, c = (i - s0 * per_row) * 8u;
+    const TX* src = x + s0 * sx_0 + c;
+    float acc[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[j] = 0.0f;
+    for (int r0 = 0; r0 < R; r0 += 4) {
+      uint4 raw[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (r0 + u < R) raw[u] = __ldcs(reinterpret_cast<const uint4*>(src + (r0 + u) * sx_r));
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (r0 + u < R) {
+          const TX* e = reinterpret_cast<const TX*>(&raw[u]);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) acc[j] += to_f32<TX>(e[j]);
+        }
+    }
+    TY o[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) o[j] = from_f32<TY>(acc[j]);
+    *reinterpret_cast<uint4*>(y + s0 * sy_0 + c) = *reinterpret_cast<const uint4*>(o);
+  }
+}
+
 template <typename TX, typename TY>
 static int launch_reduce(const void* x, int64_t R, int64_t S0, int64_t S1, int64_t sx_r, int64_t sx_0, int64_t sx_1,
                          const void* mask, int mb, int64_t sm_r, int64_t sm_0, int64_t sm_1, const float* scale,
@@ -275,6 +307,13 @@ static int launch_reduce(const void* x, int64_t R, int64_t S0, int64_t S1, int64
   if constexpr (sizeof(TX) == 2 && sizeof(TY) == 2) {
     const bool vec = sx_1 == 1 && sy_1 == 1 && S1 % 8 == 0 && sx_r % 8 == 0 && sx_0 % 8 == 0 && sy_0 % 8 == 0 &&
                      (uintptr_t)x % 16 == 0 && (uintptr_t)y % 16 == 0 && (!mask || sm_1 == 0) && (!scale || ss_1 == 0);
+    const int64_t total = S0 * (S1 / 8);
+    if (vec && !mask && !scale && total < (1ll << 31) && R < (1 << 20)) {
+      MOE_CHECK_CUDA(launch_pdl(sum_slots_kernel<TX, TY>, dim3(grid_for(total, 256)), dim3(256), 0, st, (const TX*)x, (int)R, (uint32_t)(S1 / 8),
+                                (uint32_t)total, sx_r, sx_0, (TY*)y, sy_0));
+      MOE_CHECK_LAUNCH();
+      return MOE_OK;
+    }
     if (vec) {
       MOE_CHECK_CUDA(launch_pdl(reduce_kernel<TX, TY, true>, dim3(grid_for(S0 * (S1 / 8), 256)), dim3(256), 0, st, (const TX*)x, R, S0, S1,
                                 sx_r, sx_0, sx_1, mask, mb, sm_r, sm_0, sm_1, scale, ss_r, ss_0, ss_1, (TY*)y, sy_0, sy_1));

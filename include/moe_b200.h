@@ -313,6 +313,15 @@ int moe_ep_combine_index(const int32_t* row_sorted, const int16_t* expt_indx, co
                          int64_t n_local, int64_t rows_per_peer, int32_t* out, void* stream);
 /* Two copies of device memory in one launch (16-byte aligned pointers, any sizes; the second may be empty). */
 int moe_copy2(void* dst0, const void* src0, int64_t bytes0, void* dst1, const void* src1, int64_t bytes1, void* stream);
+/* A captured step between the copies of its inputs and of its result: a clone of `graph` (a cudaGraph_t over static buffers) with a copy
+ * into in0 and in1 ahead of it and a copy out of `out` behind it, instantiated.  roots_wait: the graph's first kernels wait for the one
+ * before by themselves (griddepcontrol.wait, as those of moe_route do) and may be launched ahead of its end.  Every launch names the caller's buffers of the same sizes
+ * (16-byte aligned); they are read and written in the order of `stream`.  The graph's buffers must outlive the step.  One launch at
+ * a time per step: the call is not safe in several threads at once. */
+int moe_step_graph_create(void* graph, int roots_wait, void* in0, int64_t bytes0, void* in1, int64_t bytes1, const void* out,
+                          int64_t bytes_out, void** step);
+int moe_step_graph_launch(void* step, const void* src0, const void* src1, void* dst, void* stream);
+void moe_step_graph_destroy(void* step);
 int moe_gather_rows(const void* src, int64_t ld_src, const int32_t* row_indx, int64_t n_rows_out, int64_t row_bytes,
                     void* dst, int64_t ld_dst, void* stream);
 /* moe_gather_rows over rows that live on several devices: global row g = row_indx[r] is row g % rows_per_peer of

@@ -297,6 +297,35 @@ def test_graphed_layer_equals_eager_layer(tokens, layer_20b, device):
         assert torch.equal(want, got)
 
 
+@pytest.mark.parametrize("form", ["plain", "strided x", "offset x", "other types"])
+def test_graphed_layer_takes_inputs_of_any_layout(form, layer_20b, device):
+    """Inputs that the step's own copies do not take (strides, alignment, types) are copied ahead of the replay; either way the
+    step's buffers hold the call's inputs and result afterwards, and an earlier result stays as it is."""
+    from triton_b200.moe import GraphedMoeLayer, moe_layer_forward
+    lw, _, _ = layer_20b
+    T = 5
+    graphed = GraphedMoeLayer(lw, 4, T, 2880, 32, device)
+    g = torch.Generator(device=device).manual_seed(3)
+    first = graphed(torch.randn(T, 2880, device=device, generator=g).bfloat16(), torch.randn(T, 32, device=device, generator=g))
+    kept = first.clone()
+    x, logits = torch.randn(T, 2880, device=device, generator=g).bfloat16(), torch.randn(T, 32, device=device, generator=g)
+    xi, li = x, logits
+    if form == "strided x":
+        xi = torch.zeros(T, 2 * 2880, device=device, dtype=torch.bfloat16)[:, :2880].copy_(x)
+    elif form == "offset x":
+        xi = torch.zeros(T * 2880 + 1, device=device, dtype=torch.bfloat16)[1:].view(T, 2880).copy_(x)
+    elif form == "other types":
+        xi, li = x.float(), logits.double()
+    got = graphed(xi, li)
+    assert torch.equal(got, moe_layer_forward(x, logits, lw, 4)) and torch.equal(first, kept)
+    assert torch.equal(graphed.x, x) and torch.equal(graphed.logits, logits) and torch.equal(graphed.z, got)
+    graphed.z.zero_()
+    assert torch.equal(graphed.replay(), got) and got.data_ptr() != graphed.z.data_ptr()
+    with pytest.raises(RuntimeError):
+        graphed(x[:4], logits[:4])
+    tb.matmul_check_status()
+
+
 def test_host_streaming_layer(layer_20b, device):
     """Steps fed from and returned to pinned host memory through the three-stream pipeline equal the eager layer."""
     from triton_b200.moe import HostStreamingLayer, moe_layer_forward

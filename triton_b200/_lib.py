@@ -75,6 +75,9 @@ PROTOTYPES = {
     "moe_ep_pull_index": (i32, [vp, vp, vp, vp, i64, i32, vp, vp, vp]),
     "moe_ep_combine_index": (i32, [vp, vp, vp, i64, i64, i64, vp, vp]),
     "moe_copy2": (i32, [vp, vp, i64, vp, vp, i64, vp]),
+    "moe_step_graph_create": (i32, [vp, i32, vp, i64, vp, i64, vp, i64, vp]),
+    "moe_step_graph_launch": (i32, [vp, vp, vp, vp, vp]),
+    "moe_step_graph_destroy": (None, [vp]),
     "moe_gather_rows": (i32, [vp, i64, vp, i64, i64, vp, i64, vp]),
     "moe_gather_rows_peers": (i32, [vp, i32, i64, i64, vp, i64, i64, vp, i64, vp]),
     "moe_peer_barrier": (i32, [vp, i32, i32, vp, vp, vp]),

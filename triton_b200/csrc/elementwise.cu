@@ -6,6 +6,8 @@
 // Combine semantics: triton_kernels reduce.py:1181-1214 (fp32 sum over the reduced axis of
 // mask * scale * x, cast to the output type).
 #include "common.cuh"
+#include <memory>
+#include <vector>
 
 namespace {
 
@@ -383,6 +385,96 @@ extern "C" __attribute__((visibility("default"))) int moe_copy2(void* dst0, cons
   MOE_CHECK_LAUNCH();
   return MOE_OK;
 }
+
+// A replayed step's copies as nodes of its graph.  Launched around the replay they cost it two boundaries between a launch and a graph, of 3 and 1 us, which no
+// launch attribute bridges; as nodes they follow one another like the kernels of the step.
+namespace {
+struct StepGraph {
+  cudaGraph_t graph = nullptr;
+  cudaGraphExec_t exec = nullptr;
+  cudaGraphNode_t in = nullptr, out = nullptr;
+  uint8_t *d0 = nullptr, *d1 = nullptr;
+  const uint8_t* z = nullptr;
+  int64_t n0 = 0, n1 = 0, nz = 0;
+  ~StepGraph() {
+    if (exec) cudaGraphExecDestroy(exec);
+    if (graph) cudaGraphDestroy(graph);
+  }
+};
+// copy2_kernel as a node: `apply` gets the parameters
+template <typename F>
+cudaError_t with_copy_params(uint8_t* d0, const uint8_t* s0, int64_t n0, uint8_t* d1, const uint8_t* s1, int64_t n1, F apply) {
+  void* args[6] = {&d0, &s0, &n0, &d1, &s1, &n1};
+  cudaKernelNodeParams k = {};
+  k.func = (void*)copy2_kernel;
+  k.gridDim = dim3((unsigned)grid_for(n0 / 16 + n1 / 16 + 1, 256));
+  k.blockDim = dim3(256);
+  k.kernelParams = args;
+  return apply(&k);
+}
+int step_graph_build(StepGraph& s, cudaGraph_t graph, bool roots_wait) {
+  MOE_CHECK_CUDA(cudaGraphClone(&s.graph, graph));
+  size_t n = 0;
+  MOE_CHECK_CUDA(cudaGraphGetNodes(s.graph, nullptr, &n));
+  MOE_CHECK_ARG(n > 0, "moe_step_graph_create: the graph is empty");
+  std::vector<cudaGraphNode_t> nodes(n), roots, leaves;
+  MOE_CHECK_CUDA(cudaGraphGetNodes(s.graph, nodes.data(), &n));
+  for (cudaGraphNode_t node : nodes) {
+    size_t before = 0, behind = 0;
+    MOE_CHECK_CUDA(cudaGraphNodeGetDependencies_v2(node, nullptr, nullptr, &before));
+    MOE_CHECK_CUDA(cudaGraphNodeGetDependentNodes_v2(node, nullptr, nullptr, &behind));
+    if (!before) roots.push_back(node);
+    if (!behind) leaves.push_back(node);
+  }
+  MOE_CHECK_CUDA(with_copy_params(s.d0, s.d0, s.n0, s.d1, s.d1, s.n1,
+                                  [&](const cudaKernelNodeParams* k) { return cudaGraphAddKernelNode(&s.in, s.graph, nullptr, 0, k); }));
+  MOE_CHECK_CUDA(with_copy_params(const_cast<uint8_t*>(s.z), s.z, s.nz, nullptr, nullptr, 0,
+                                  [&](const cudaKernelNodeParams* k) { return cudaGraphAddKernelNode(&s.out, s.graph, nullptr, 0, k); }));
+  // programmatic where the kernel behind waits for the one ahead by itself, as the copy does
+  auto is_kernel = [](cudaGraphNode_t node) {
+    cudaGraphNodeType t;
+    return cudaGraphNodeGetType(node, &t) == cudaSuccess && t == cudaGraphNodeTypeKernel;
+  };
+  cudaGraphEdgeData programmatic = {}, plain = {};
+  programmatic.from_port = cudaGraphKernelNodePortProgrammatic;
+  programmatic.type = cudaGraphDependencyTypeProgrammatic;
+  for (cudaGraphNode_t node : roots)
+    MOE_CHECK_CUDA(cudaGraphAddDependencies_v2(s.graph, &s.in, &node, roots_wait && is_kernel(node) ? &programmatic : &plain, 1));
+  for (cudaGraphNode_t node : leaves)
+    MOE_CHECK_CUDA(cudaGraphAddDependencies_v2(s.graph, &node, &s.out, is_kernel(node) ? &programmatic : &plain, 1));
+  MOE_CHECK_CUDA(cudaGraphInstantiate(&s.exec, s.graph, 0));
+  return MOE_OK;
+}
+}  // namespace
+
+extern "C" __attribute__((visibility("default"))) int moe_step_graph_create(void* graph, int roots_wait, void* in0, int64_t bytes0, void* in1,
+                                                                            int64_t bytes1, const void* out, int64_t bytes_out, void** step) {
+  MOE_CHECK_ARG(graph && step && in0 && in1 && out && bytes0 > 0 && bytes1 > 0 && bytes_out > 0, "moe_step_graph_create: NULL or empty argument");
+  MOE_CHECK_ARG((((uintptr_t)in0 | (uintptr_t)in1 | (uintptr_t)out) & 15) == 0, "moe_step_graph_create: buffers must be 16-byte aligned");
+  auto s = std::make_unique<StepGraph>();
+  s->d0 = (uint8_t*)in0; s->n0 = bytes0;
+  s->d1 = (uint8_t*)in1; s->n1 = bytes1;
+  s->z = (const uint8_t*)out; s->nz = bytes_out;
+  if (int rc = step_graph_build(*s, (cudaGraph_t)graph, roots_wait != 0)) return rc;
+  *step = s.release();
+  return MOE_OK;
+}
+
+extern "C" __attribute__((visibility("default"))) int moe_step_graph_launch(void* step, const void* src0, const void* src1, void* dst, void* stream) {
+  MOE_CHECK_ARG(step && src0 && src1 && dst, "moe_step_graph_launch: NULL argument");
+  MOE_CHECK_ARG((((uintptr_t)src0 | (uintptr_t)src1 | (uintptr_t)dst) & 15) == 0, "moe_step_graph_launch: buffers must be 16-byte aligned");
+  const StepGraph& s = *(const StepGraph*)step;
+  MOE_CHECK_CUDA(with_copy_params(s.d0, (const uint8_t*)src0, s.n0, s.d1, (const uint8_t*)src1, s.n1,
+                                  [&](const cudaKernelNodeParams* k) { return cudaGraphExecKernelNodeSetParams(s.exec, s.in, k); }));
+  MOE_CHECK_CUDA(with_copy_params((uint8_t*)dst, s.z, s.nz, nullptr, nullptr, 0,
+                                  [&](const cudaKernelNodeParams* k) { return cudaGraphExecKernelNodeSetParams(s.exec, s.out, k); }));
+  moe_count_launch();
+  moe_count_launch();
+  MOE_CHECK_CUDA(cudaGraphLaunch(s.exec, (cudaStream_t)stream));
+  return MOE_OK;
+}
+
+extern "C" __attribute__((visibility("default"))) void moe_step_graph_destroy(void* step) { delete (StepGraph*)step; }
 
 extern "C" __attribute__((visibility("default"))) int moe_gather_rows(const void* src, int64_t ld_src, const int32_t* row_indx, int64_t n_rows_out,
                                int64_t row_bytes, void* dst, int64_t ld_dst, void* stream) {

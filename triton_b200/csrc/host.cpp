@@ -17,7 +17,7 @@ struct Lib {
 #define MOE_HOST_FUNCTIONS(X)                                                                                            \
   X(moe_last_error) X(moe_route) X(moe_route_positions) X(moe_route_workspace) X(moe_grouped_gemm) X(moe_gemm_mx_workspace_bytes) \
   X(moe_reduce) X(moe_downcast_mxfp4) X(moe_upcast_mxfp4) X(moe_bitmatrix_metadata) X(moe_bitmatrix_metadata_workspace) \
-  X(moe_router_topk) X(moe_copy2) \
+  X(moe_router_topk) X(moe_copy2) X(moe_step_graph_create) X(moe_step_graph_launch) X(moe_step_graph_destroy) \
   X(moe_gemm_kernel_name) X(moe_grouped_gemm_chain)
 #define X(name) decltype(&::name) name = nullptr;
   MOE_HOST_FUNCTIONS(X)
@@ -456,9 +456,34 @@ Tensor copy_of(const Tensor& src) {
   return out;
 }
 
+// A captured layer step, routing first, with its copies (moe_step_graph_create): x and logits in, a new tensor out.
+class StepGraph {
+ public:
+  StepGraph(int64_t graph, const Tensor& x, const Tensor& logits, const Tensor& z) : x_(x), logits_(logits), z_(z) {
+    check(lib.moe_step_graph_create(reinterpret_cast<void*>(graph), 1, x.data_ptr(), (int64_t)x.nbytes(), logits.data_ptr(), (int64_t)logits.nbytes(),
+                                    z.data_ptr(), (int64_t)z.nbytes(), &step_),
+          "moe_step_graph_create");
+  }
+  ~StepGraph() { lib.moe_step_graph_destroy(step_); }
+  StepGraph(const StepGraph&) = delete;
+  StepGraph& operator=(const StepGraph&) = delete;
+  // None where the inputs are not plain copies of the step's on the current device
+  std::optional<Tensor> run(const Tensor& x, const Tensor& logits) {
+    if (!plain_copy(x_, x) || !plain_copy(logits_, logits) || x_.device().index() != c10::cuda::current_device()) return std::nullopt;
+    Tensor out = at::empty(z_.sizes(), z_.options());
+    check(lib.moe_step_graph_launch(step_, x.data_ptr(), logits.data_ptr(), out.data_ptr(), stream()), "moe_step_graph_launch");
+    return out;
+  }
+
+ private:
+  Tensor x_, logits_, z_;
+  void* step_ = nullptr;
+};
+
 }  // namespace
 
 PYBIND11_MODULE(_host, m) {
+  py::class_<StepGraph>(m, "StepGraph").def(py::init<int64_t, const Tensor&, const Tensor&, const Tensor&>()).def("run", &StepGraph::run);
   m.def("copy2", &copy2);
   m.def("copy_of", &copy_of);
   m.def("bind", &bind);

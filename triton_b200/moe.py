@@ -236,9 +236,14 @@ class GraphedMoeLayer:
                 self.forward(self.x, self.logits)
         torch.cuda.current_stream(device).wait_stream(side)
         torch.cuda.synchronize(device)
-        self.graph = torch.cuda.CUDAGraph()
+        self.graph = torch.cuda.CUDAGraph(keep_graph=True)
         with torch.cuda.graph(self.graph):
             self.z = self.forward(self.x, self.logits)
+        self.graph.instantiate()
+        # the layer's own step also as a graph with the copies of a call in it (1 token 33.0 -> 28.7 us)
+        self.step = None
+        if forward is None and self.z.numel() > 0:
+            self.step = _lib.host().StepGraph(self.graph.raw_cuda_graph(), self.x, self.logits, self.z)
 
     def replay(self):
         """Replay on the graph's own input buffers (`self.x`, `self.logits`); the result is `self.z`."""
@@ -248,6 +253,10 @@ class GraphedMoeLayer:
     def __call__(self, x, logits):
         # both inputs in one native call and launch: as two copy_ and a clone around the replay they took 19 us of a step
         host = _lib.host()
+        if self.step is not None:
+            z = self.step.run(x, logits)
+            if z is not None:
+                return z
         host.copy2(self.x, x, self.logits, logits)
         self.graph.replay()
         # a copy, so that the caller may still be reading one result (a download, say) while the next step replays

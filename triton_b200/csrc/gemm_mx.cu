@@ -8,7 +8,7 @@
 //
 // Operand roles are swapped with respect to the bf16 kernel: the WEIGHTS are the M = 128 operand (a tile is 128
 // weight rows x 128 k) and the TOKENS are the N operand (16 .. 128 columns), so that a handful of tokens costs a
-// handful of accumulator columns.  A CTA tile is MB (1 or 3) weight blocks x one block of tokens; the token block
+// handful of accumulator columns.  A CTA tile is MB (1 to 3) weight blocks x one block of tokens; the token block
 // stays in shared memory per k step and is shared by the MB weight blocks.
 //
 // bf16 activations are split into two e4m3 terms, hi = mxfp8(x) and lo = mxfp8(x - hi), each with its own e8m0
@@ -68,7 +68,7 @@ struct MxParams {
   TokenOut out;                 // the rows as the next product's tokens
 };
 
-inline bool mx_fits(int split, int mb) { return split == 2 && mb == 3; }
+inline bool mx_fits(int split, int mb) { return split == 2 && mb > 1; }
 
 struct MxMaps {
   CUtensorMap m[3];             // boxes of 1, 2 and 3 weight blocks
@@ -441,7 +441,7 @@ __device__ __forceinline__ void mx_sums(uint32_t taddr, int split, int lines, ui
 // one k step of three blocks -- for steps with so few tiles that a CTA gets single weight blocks (one to four tokens: 60
 // to 165 three-block tiles for 148 SMs).  A stage of one 8 KB tile cannot keep a per-SM copy pipeline busy (a ring of
 // 8 KB stages streams 3.3 TB/s over the GPU however many are in flight, 24 KB stages 7.1 TB/s).
-// FIT (two-term form, MB = 3): a tile copies and multiplies, of a token block, what its rows need (16, 32 or 64 lines a term): 300 tokens of
+// FIT (two-term form, MB = 2 or 3): a tile copies and multiplies, of a token block, what its rows need (16, 32 or 64 lines a term): 300 tokens of
 // 128 experts 303.6 -> 287.6 us per step.  With four terms (8 or 16 lines) or single blocks it costs a tile's start more than it saves (16
 // tokens 62.3 -> 63.9), and e4m3 tokens pay 5 % for the code alone.
 template <typename TY, int MB, bool F4, bool KM = false, bool FIT = false>
@@ -670,7 +670,7 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
           const uint32_t taddr = tmem_base + ((uint32_t)(qd * 32) << 16) + SF_BASE + (uint32_t)(s * SF_COLS);
           if (FIT && kt == 0) scales_at = (uint32_t)s_cols[s] * X_ROW;
           // S > 1: the weight scales of the k steps, then the token scales of their chunks
-          constexpr int NV = S > 1 ? 2 * S : MB + 1;
+          constexpr int LOADS = S > 1 ? 2 * S : MB + 1, NV = LOADS == 3 ? 4 : LOADS;
           const int live = S > 1 ? min(S, KT - S * kt) : mb_live;
           uint4 v[NV];
 #pragma unroll
@@ -678,7 +678,7 @@ gemm_mx_kernel(const GemmParams p, const MxParams q, const __grid_constant__ MxM
             const int j = S > 1 && i >= S ? i - S : i;
             uint32_t at = st + off_ws(S) + (uint32_t)j * MX_WS_TILE;
             if (S > 1 ? i >= S : i == MB) at = st + off_x(S) + (S > 1 ? (uint32_t)j * (uint32_t)q.chunk_bytes : 0u) + scales_at;
-            v[i] = j < live || (S == 1 && i == MB) ? lds128(at + (uint32_t)lane * 16u) : make_uint4(0, 0, 0, 0);
+            v[i] = (i < LOADS && j < live) || (S == 1 && i == MB) ? lds128(at + (uint32_t)lane * 16u) : make_uint4(0, 0, 0, 0);
           }
           if constexpr (NV >= 4)
             asm volatile(
@@ -869,10 +869,13 @@ MxPlan mx_plan(const MoeGemmArgs& a) {
   pl.KT = (int)cdiv64(a.K, 128);
   pl.NB = (int)cdiv64(a.N, 128);
   pl.grid_m = a.slice_sizes ? blocks_bound(a.E, a.M, tb) : cdiv64(a.M, tb);
-  // three weight blocks per CTA tile share one token tile (fewer token bytes per weight byte); one block when there
-  // would be too few tiles to fill the SMs
-  const int64_t items3 = pl.grid_m * cdiv64(pl.NB, 3);
-  pl.mb = (a.tile_n == 128) ? 1 : ((a.tile_n == 384 || items3 >= (int64_t)moe_sm_count()) ? 3 : 1);
+  // several weight blocks per CTA tile share one token tile (fewer token bytes per weight byte); one block when there
+  // would be too few tiles to fill the SMs.  Three of packed weights; two where a value takes a byte of shared memory, of which the ring holds five stages
+  // where it takes three of three: what bounds those forms is the weights in flight per SM, 82 KB against 74, less the stage at work (bf16, 300 and 500
+  // tokens of 128 experts 248 -> 238 and 349 -> 326 us per step, 150 tokens of 32 experts of 4096 x 4096 212 -> 193; e4m3, 64 and 100 tokens
+  // of 32 experts 99.9 -> 92.5 and 103.2 -> 95.6).
+  const int wide = pl.f4 ? 3 : 2;
+  pl.mb = a.tile_n == 128 ? 1 : a.tile_n == 384 ? 3 : pl.grid_m * cdiv64(pl.NB, wide) >= (int64_t)moe_sm_count() ? wide : 1;
   // too few tiles for three blocks each, four-term form: single weight blocks, three k steps of one block per stage
   // (a stage of one 8 KB tile does not keep a copy pipeline busy)
   pl.km = (pl.f4 && tb == 16 && pl.mb == 1 && a.tile_n == 0 && pl.KT >= 3) ? 1 : 0;
@@ -919,6 +922,10 @@ int launch_mx_ty(const GemmParams& p, const MxParams& q, const MxPlan& pl, const
   }
   if constexpr (TOK_TERMS<TY> == 4) return MOE_ERR_UNSUPPORTED;
   else {
+    if constexpr (TOK_TERMS<TY> != 2)
+      if (pl.mb == 2 && pl.split == 1) return launch_mx<TY, 2, false>(p, q, pl, w_map, idle_sms, st);
+    if constexpr (TOK_TERMS<TY> != 1)
+      if (pl.mb == 2 && pl.split == 2) return launch_mx<TY, 2, false, false, true>(p, q, pl, w_map, idle_sms, st);
     if (pl.mb != 3) return launch_mx<TY, 1, false>(p, q, pl, w_map, idle_sms, st);
     if constexpr (TOK_TERMS<TY> != 1)
       if (mx_fits(pl.split, pl.mb)) return launch_mx<TY, 3, false, false, true>(p, q, pl, w_map, idle_sms, st);

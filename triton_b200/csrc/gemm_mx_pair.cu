@@ -973,16 +973,17 @@ int launch_mx_pair_ty(const GemmParams& p, const PairParams& q, const MoeGemmArg
 // experts of 1024 rows: 72 here, 57 there; 16 experts 132 and 109; without the activation 64 and 61, 114 and 116).
 // (Both kernels lose up to a third of a wave, so no line in these sizes is right everywhere: over 500 products of 48 to 1024 rows
 // this one is 2 % from the better kernel on average, most of it at 100-400 balanced rows of K <= 1024.)
-// Block-scaled tiles (against the decode forms of gemm_mx.cu), tile_m = 256 asks for it.  bf16 tokens from 20 rows on, e4m3 tokens, one
-// term, from 16: what an expert has decides, not the mean, and the lines lie between even routing, where the decode form stays ahead up to
-// some 24 rows, and logits biased by N(0, 1) per expert, where this one is ahead from 8 to 16 rows on.  Whole layer steps, four picks
-// (decode form, this one; even, then biased):
-//   bf16   32 experts of 2880 x 5760:  16 rows 117, 133; 113, 115.  24 rows 129, 136; 128, 131.  32 rows 150, 140; 150, 134
-//          128 experts of the same:    8 rows 358, 392; 323, 274.  16 rows 385, 404; 339, 303.  24 rows 419, 414; 412, 331
-//          64 experts of 1024 x 1536:  12 rows 50, 52; 53, 51.  16 rows 55, 55; 56, 53.  24 rows 57, 54; 63, 56
-//   e4m3   32 experts of 2880 x 5760:  16 rows 108, 127; 103, 108.  24 rows 117, 129; 117, 121.  32 rows 135, 132; 135, 127
-//          128 experts of the same:    8 rows 357, 402; 273, 257.  16 rows 356, 390; 301, 279.  24 rows 373, 402; 350, 289.  32 rows 450, 407; 431, 341
-//          64 experts of 1024 x 1536:  16 rows 50, 53; 51, 54.  24 rows 51, 52; 57, 55
+// Block-scaled tiles (against the decode forms of gemm_mx.cu), tile_m = 256 asks for it.  What an expert has decides, not the mean, so the lines lie
+// between even routing and logits biased by N(0, 1) per expert, under which some experts have several blocks of the decode form.  bf16 tokens from 20
+// rows on, but from 25 where the product's tiles here are more than one and up to eight rounds of the pairs: a last round partly filled costs a good
+// part of the whole then.  e4m3 tokens, one term, from 16 (up to eight rounds even routing would stay ahead on the decode form to 28 and more).  Whole
+// layer steps, four picks (decode form, this one; even, then biased):
+//   bf16   128 experts of 2880 x 5760:  20 rows 429, 452; 377, 357.  24 rows 449, 437; 436, 391
+//          32 experts of the same:  20 rows 109, 131; 123, 129.  25 rows 118, 134; 133, 131.  30 rows 135, 138; 141, 136.  40 rows 172, 143; 164, 149
+//          64 experts of 1440 x 2880:  20 rows 86, 96; 81, 88.  25 rows 84, 95; 94, 94.  32 rows 101, 98; 102, 97
+//   e4m3   128 experts of 2880 x 5760:  16 rows 359, 397; 307, 287.  20 rows 361, 396; 338, 295.  24 rows 376, 406; 377, 314
+//          32 experts of the same:  16 rows 102, 129; 100, 121.  25 rows 110, 131; 122, 127.  32 rows 130, 133; 135, 132
+//          64 experts of 1440 x 2880:  16 rows 77, 91; 75, 80.  25 rows 79, 91; 87, 89
 // Small ones (products with their token packs) once the decode kernel's tiles of 32 rows x 128 weight rows (half a block lost per expert) are more than a wave, up to
 // which it takes one tile's time: a product of 32 experts of 512 x 512, 16 rows 10 there, 11 here, 64 rows 21 and 13; 8 experts of
 // 512 x 2048, 16 rows 9 and 11, 80 rows 20 and 13; of 2048 x 512, 96 rows 17 and 21.
@@ -1005,7 +1006,10 @@ bool moe_gemm_mx_pair_wanted(const MoeGemmArgs& a) {
   if (a.tile_m == 256) return true;
   if (a.tile_m != 0 || a.kernel == MOE_GEMM_MX_F8) return false;
   if (a.x_dtype != MOE_BF16) return per >= 16;
-  if (load >= (1 << 24)) return per >= 20;
+  if (load >= (1 << 24)) {
+    const int64_t tiles = experts * cdiv64(a.N, 512), pairs = moe_sm_count() / 2;
+    return per >= (tiles > pairs && tiles <= 8 * pairs ? 25 : 20);
+  }
   return experts * (per + 16) / 32 * cdiv64(a.N, 128) > moe_sm_count();
 }
 

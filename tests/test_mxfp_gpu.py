@@ -188,3 +188,41 @@ def test_tiles_of_storage_that_stands_for_several_experts(block_scaled, device):
         three = t.transpose(1, 2).repeat(E, 1, 1).transpose(1, 2)
         got, want = (convert_layout(Tensor(Storage(d, StridedLayout(major_dim=-2)), dtype=dtype, shape=shape), layout) for d in (t, three))
         assert torch.equal(got.storage.data, want.storage.data)
+
+
+# groups around a block's 256 and 512, a ragged last turn of a whole grid; rows without a gap against the same rows 32 elements apart
+@pytest.mark.parametrize("rows, quant", [(1, 32), (5, 1632), (8, 1024), (257, 32), (3, 5472), (33, 8192), (2500, 15552)])
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16, torch.float32])
+def test_rows_without_a_gap_are_the_rows_with_one(rows, quant, dt, device):
+    if dt is torch.float32 and rows > 1000:
+        pytest.skip("one turn of the grid is in the two-byte types")
+    g = torch.Generator(device=device).manual_seed(rows)
+    wide = torch.randn(rows, quant + 32, device=device, generator=g)
+    wide = (wide * torch.exp2(torch.randint(-20, 12, (rows, 1), device=device, generator=g))).to(dt)
+    wide[0, :2] = torch.tensor([float("nan"), -0.0], dtype=dt)
+    x = wide[:, :quant]
+    q, s = downcast_to_mxfp(x.contiguous(), torch.uint8, axis=1)
+    q_gap, s_gap = downcast_to_mxfp(x, torch.uint8, axis=1)
+    assert torch.equal(q, q_gap) and torch.equal(s, s_gap)
+    back = upcast_from_mxfp(q, s, dt, axis=1)
+    if rows < 100:
+        assert torch.equal(bits(back.cpu()), bits(oracle.upcast_from_mxfp_oracle(q.cpu(), s.cpu(), dt, 1).contiguous()))
+    else:                                                          # the codes' own values in fp32, scaled and rounded once
+        table = torch.tensor([0, 0.5, 1, 1.5, 2, 3, 4, 6, -0.0, -0.5, -1, -1.5, -2, -3, -4, -6], device=device)
+        for r in (0, rows // 2, rows - 1):
+            codes = torch.stack([q[r] & 15, q[r] >> 4], 1).reshape(-1).long()
+            want = table[codes] * torch.exp2(s[r].float() - 127).repeat_interleave(32)
+            assert torch.equal(back[r].float()[8:], want.to(dt).float()[8:])
+
+
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16, torch.float32])
+def test_upcast_down_columns_is_that_along_rows(dt, device):
+    """Every scale byte with every code, neighbouring columns with scales on either side of what the look-up takes."""
+    codes = torch.arange(16, dtype=torch.uint8)
+    q = (codes | (codes.flip(0) << 4)).repeat(512, 1).to(device)
+    s = torch.cat([torch.arange(256), torch.arange(256)[torch.randperm(256, generator=torch.Generator().manual_seed(0))]]).to(torch.uint8).view(512, 1).to(device)
+    rows = upcast_from_mxfp(q, s, dt, axis=1)
+    cols = upcast_from_mxfp(q.t(), s.t(), dt, axis=0)
+    nan = torch.isnan(rows)
+    assert torch.equal(torch.isnan(cols.t()), nan) and bool(nan.any())
+    assert torch.equal(bits(rows)[~nan], bits(cols.t().contiguous())[~nan])

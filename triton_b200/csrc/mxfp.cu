@@ -56,7 +56,7 @@ __device__ __forceinline__ uint32_t e2m1x2(float lo, float hi) {
 // One thread owns whole 32-groups: 64 (or 128) contiguous input bytes as 16-byte loads, one division and one scale
 // per group, one 16-byte store of the 32 codes and one byte of scale.  GROUPS_UNROLL groups are loaded before the first
 // is converted, so that enough bytes are in flight per SM to cover the HBM latency.
-constexpr int GROUPS_UNROLL = 2;
+constexpr int GROUPS_UNROLL = 2, DENSE_BLOCKS = 4;
 
 template <typename T> __device__ __forceinline__ void unpack16(const uint4& r, float* v);
 template <> __device__ __forceinline__ void unpack16<__nv_bfloat16>(const uint4& r, float* v) {
@@ -80,19 +80,44 @@ template <> __device__ __forceinline__ void unpack16<float>(const uint4& r, floa
   v[0] = __uint_as_float(r.x); v[1] = __uint_as_float(r.y); v[2] = __uint_as_float(r.z); v[3] = __uint_as_float(r.w);
 }
 
+// max |x| of a group; NaN operands lose, as with fmaxf.  Two-byte types by packed maxima of the pairs.
+template <typename T> struct Two;
+template <> struct Two<__nv_bfloat16> { using type = __nv_bfloat162; };
+template <> struct Two<__half> { using type = __half2; };
+template <typename T, int VPG> __device__ __forceinline__ float group_absmax(const uint4 (&raw)[VPG]) {
+  if constexpr (sizeof(T) == 2) {
+    using T2 = typename Two<T>::type;
+    T2 m[4];
+#pragma unroll
+    for (int k = 0; k < VPG; ++k) {
+      const uint32_t w[4] = {raw[k].x, raw[k].y, raw[k].z, raw[k].w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const T2 v = __habs2(*reinterpret_cast<const T2*>(&w[j]));
+        m[j] = k == 0 ? v : __hmax2(m[j], v);
+      }
+    }
+    const T2 t = __hmax2(__hmax2(m[0], m[1]), __hmax2(m[2], m[3]));
+    return fmaxf(fmaxf(0.0f, to_f32<T>(t.x)), to_f32<T>(t.y));
+  } else {
+    float m = 0.0f;
+#pragma unroll
+    for (int k = 0; k < VPG; ++k) {
+      float v[32 / VPG];
+      unpack16<T>(raw[k], v);
+#pragma unroll
+      for (int j = 0; j < 32 / VPG; ++j) m = fmaxf(m, fabsf(v[j]));
+    }
+    return m;
+  }
+}
+
 // the 32 values of a group as VPG raw 16-byte vectors -> scale bits and 16 bytes of codes.  The vectors are unpacked
 // twice (once for the maximum, once for the codes) instead of holding 32 floats across the division.
 template <typename T, int VPG>
 __device__ __forceinline__ uint4 quantise_raw(const uint4 (&raw)[VPG], int mode, uint32_t& sc) {
   constexpr int EPV = 32 / VPG;
-  float m = 0.0f;
-#pragma unroll
-  for (int k = 0; k < VPG; ++k) {
-    float v[EPV];
-    unpack16<T>(raw[k], v);
-#pragma unroll
-    for (int j = 0; j < EPV; ++j) m = fmaxf(m, fabsf(v[j]));
-  }
+  const float m = group_absmax<T, VPG>(raw);
   sc = scale_bits(m, mode);
   const float inv = inv_scale(sc);
   uint32_t w[4];
@@ -160,6 +185,33 @@ __global__ void __launch_bounds__(256, sizeof(T) == 2 ? 3 : 2) downcast_rows_ker
       }
       cur[u].next();
     }
+  }
+}
+
+// Rows that follow one another without a gap: groups are numbered through, so a thread has one index where the kernel above keeps a row and a chunk
+// for each of its groups and multiplies three pitches: 64 registers, so a fourth block per SM.  8192 x 8192 bf16 to codes and back 62.1 -> 51.0 us with
+// this kernel and upcast_dense_kernel (with three blocks per SM 51.1, with five and spills 53.5).
+template <typename T>
+__global__ void __launch_bounds__(256, sizeof(T) == 2 ? DENSE_BLOCKS : 2) downcast_dense_kernel(const T* x, int64_t total, uint8_t* q, uint8_t* scale, int mode) {
+  pdl_begin();
+  constexpr int VPG = 2 * (int)sizeof(T);                // vectors per group
+  const int64_t stride = (int64_t)gridDim.x * (GROUPS_UNROLL * 256);
+  for (int64_t g0 = (int64_t)blockIdx.x * (GROUPS_UNROLL * 256) + threadIdx.x; g0 < total; g0 += stride) {
+    uint4 raw[GROUPS_UNROLL][VPG];
+#pragma unroll
+    for (int u = 0; u < GROUPS_UNROLL; ++u)
+      if (g0 + u * 256 < total) {
+        const uint4* src = reinterpret_cast<const uint4*>(x + (g0 + u * 256) * 32);
+#pragma unroll
+        for (int k = 0; k < VPG; ++k) raw[u][k] = __ldcs(src + k);
+      }
+#pragma unroll
+    for (int u = 0; u < GROUPS_UNROLL; ++u)
+      if (g0 + u * 256 < total) {
+        uint32_t sc;
+        reinterpret_cast<uint4*>(q)[g0 + u * 256] = quantise_raw<T, VPG>(raw[u], mode, sc);
+        scale[g0 + u * 256] = (uint8_t)(sc >> 23);
+      }
   }
 }
 
@@ -349,6 +401,97 @@ __device__ __forceinline__ uint4 upcast8_bf16(uint32_t w, uint32_t sb) {
                     __byte_perm(r[2], r[3], 0x7632));
 }
 
+// Eight codes by table look-up: a byte permute takes four codes as its selectors, bits 0-2 the magnitude, and picks the low or high bytes of
+// their values; bit 3 asks for the sign of a byte of ones instead.  Then a multiplication by the scale, exact where `looks_up` says so: products and
+// scale are normal or subnormal numbers of the type and none has to be clamped.  (fp32 values are bf16 values and sixteen zero bits.)
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
+  uint32_t d;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
+  return d;
+}
+template <typename T> __device__ __forceinline__ bool looks_up(uint32_t sb);
+template <> __device__ __forceinline__ bool looks_up<__nv_bfloat16>(uint32_t sb) { return sb < 253u; }
+template <> __device__ __forceinline__ bool looks_up<float>(uint32_t sb) { return sb < 253u; }
+template <> __device__ __forceinline__ bool looks_up<__half>(uint32_t sb) { return sb - 113u <= 140u - 113u; }      // 2^-14 .. 2^13
+// values of the codes in bits 0-15 of w, two to a word (fp32: as bf16)
+template <typename T> __device__ __forceinline__ void lookup4(uint32_t w, uint32_t& r0, uint32_t& r1) {
+  const uint32_t mag = w & 0x7777u;
+  const uint32_t sign = (prmt(0x80808080u, 0x80808080u, w) << 1) & 0x80808080u;      // 0xFF for a negative code, else 0x80
+  if constexpr (std::is_same<T, __half>::value) {
+    const uint32_t hi = prmt(0x3E3C3800u, 0x46444240u, mag) | sign;         // of 0, .5, 1, 1.5 and 2, 3, 4, 6; low bytes are zero
+    r0 = prmt(hi, 0u, 0x1404u);
+    r1 = prmt(hi, 0u, 0x3424u);
+  } else {
+    const uint32_t lo = prmt(0xC0800000u, 0xC0804000u, mag), hi = prmt(0x3F3F3F00u, 0x40404040u, mag) | sign;
+    r0 = prmt(lo, hi, 0x5140u);
+    r1 = prmt(lo, hi, 0x7362u);
+  }
+}
+// eight elements, scaled
+template <typename T> __device__ __forceinline__ void lookup8(uint32_t w, uint32_t sb, uint32_t (&r)[2 * sizeof(T)]) {
+  uint32_t v[4];
+  lookup4<T>(w, v[0], v[1]);
+  lookup4<T>(w >> 16, v[2], v[3]);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+      r[i] = bf16x2_mul_rn(v[i], (sb << 7) * 0x10001u);
+    } else if constexpr (std::is_same<T, __half>::value) {
+      const uint32_t s2 = ((sb - 112u) << 10) * 0x10001u;
+      const __half2 p = __hmul2(*reinterpret_cast<const __half2*>(&v[i]), *reinterpret_cast<const __half2*>(&s2));
+      r[i] = *reinterpret_cast<const uint32_t*>(&p);
+    } else {
+      const float s = __uint_as_float(sb << 23);
+      r[2 * i] = __float_as_uint(__uint_as_float(v[i] << 16) * s);
+      r[2 * i + 1] = __float_as_uint(__uint_as_float(v[i] & 0xFFFF0000u) * s);
+    }
+  }
+}
+
+// Rows that follow one another without a gap: a thread 64 bytes, numbered through.  The kernel below issues 0.78 instructions a cycle and waits for the
+// integer pipe (35 us for 8192 x 8192 bf16): two thirds of them are positions, shifts and masks.  us for 8192 x 8192 to codes and back, before and now:
+// bf16 62.1 -> 51.0, fp16 92 -> 51.0, fp32 138 -> 110; 2048 x 2048 bf16 10.2 -> 5.8.  (With 32 bytes a thread bf16 52.4 and 7.3, with 128 fp32 122.)
+constexpr int UP_DENSE_UNROLL = 2;
+template <typename T>
+__global__ void __launch_bounds__(256) upcast_dense_kernel(const uint8_t* q, const uint8_t* scale, T* out, int64_t total) {
+  pdl_begin();
+  constexpr int N = 64 / (int)sizeof(T), W = N / 8;      // elements of a thread, words of their codes
+  using Codes = std::conditional_t<W == 4, uint4, uint2>;
+  const int64_t stride = (int64_t)gridDim.x * (UP_DENSE_UNROLL * 256);
+  for (int64_t i0 = (int64_t)blockIdx.x * (UP_DENSE_UNROLL * 256) + threadIdx.x; i0 < total; i0 += stride) {
+    Codes w[UP_DENSE_UNROLL];
+    uint32_t sb[UP_DENSE_UNROLL];
+#pragma unroll
+    for (int u = 0; u < UP_DENSE_UNROLL; ++u)
+      if (i0 + u * 256 < total) {
+        w[u] = reinterpret_cast<const Codes*>(q)[i0 + u * 256];
+        sb[u] = scale[(i0 + u * 256) * N / 32];
+      }
+#pragma unroll
+    for (int u = 0; u < UP_DENSE_UNROLL; ++u)
+      if (i0 + u * 256 < total) {
+        const uint32_t* word = reinterpret_cast<const uint32_t*>(&w[u]);
+        T* dst = out + (i0 + u * 256) * N;
+        auto store = [&](const uint4* v) {
+          st_v8(dst, v[0], v[1]);
+          st_v8(dst + N / 2, v[2], v[3]);
+        };
+        if (looks_up<T>(sb[u])) {
+          uint32_t r[W][2 * sizeof(T)];
+#pragma unroll
+          for (int k = 0; k < W; ++k) lookup8<T>(word[k], sb[u], r[k]);
+          store(reinterpret_cast<const uint4*>(r));
+        } else {
+          const float s = __uint_as_float(sb[u] << 23);
+          alignas(16) T e[N];
+#pragma unroll
+          for (int k = 0; k < N; ++k) e[k] = dequant_one<T>((word[k / 8] >> (4 * (k % 8))) & 0xFu, s, sb[u] == 0xFFu);
+          store(reinterpret_cast<const uint4*>(e));
+        }
+      }
+  }
+}
+
 // HBM-bound, four fifths of it writes: with 16-byte stores (a sector in two) 8192 x 8192 to bf16 took 45.3 us on cold inputs, with
 // a sector per lane 35.6 (4.8 TB/s over 169.9 MB).
 constexpr int ROWS_UNROLL = 4;
@@ -457,20 +600,20 @@ __global__ void __launch_bounds__(256) upcast_cols_kernel(const uint8_t* q, cons
   const uint32_t sb0 = s_s[lane * 16 + warp], sb1 = s_s[lane * 16 + 8 + warp];
   const uint32_t w0[4] = {a0.x, a0.y, a0.z, a0.w}, w1[4] = {a1.x, a1.y, a1.z, a1.w};
   T* dst = out + b * so_batch + (int64_t)g * 32 * so_quant + col;
-  if constexpr (std::is_same<T, __nv_bfloat16>::value) {
-    if (sb0 < 253u && sb1 < 253u) {
+  if (looks_up<T>(sb0) && looks_up<T>(sb1)) {
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const uint4 v0 = upcast8_bf16(w0[k], sb0), v1 = upcast8_bf16(w1[k], sb1);       // pairs of elements of one column
-        const uint32_t p0[4] = {v0.x, v0.y, v0.z, v0.w}, p1[4] = {v1.x, v1.y, v1.z, v1.w};
+    for (int k = 0; k < 4; ++k) {
+      uint32_t p0[2 * sizeof(T)], p1[2 * sizeof(T)];               // eight elements of either column
+      lookup8<T>(w0[k], sb0, p0);
+      lookup8<T>(w1[k], sb1, p1);
 #pragma unroll
-        for (int h = 0; h < 4; ++h) {
-          *reinterpret_cast<uint32_t*>(dst + (8 * k + 2 * h) * so_quant) = __byte_perm(p0[h], p1[h], 0x5410);
-          *reinterpret_cast<uint32_t*>(dst + (8 * k + 2 * h + 1) * so_quant) = __byte_perm(p0[h], p1[h], 0x7632);
-        }
+      for (int h = 0; h < 8; ++h) {
+        T* at = dst + (8 * k + h) * so_quant;
+        if constexpr (sizeof(T) == 2) *reinterpret_cast<uint32_t*>(at) = __byte_perm(p0[h >> 1], p1[h >> 1], h & 1 ? 0x7632 : 0x5410);
+        else *reinterpret_cast<uint2*>(at) = make_uint2(p0[h], p1[h]);
       }
-      return;
     }
+    return;
   }
   const float f0 = __uint_as_float(sb0 << 23), f1 = __uint_as_float(sb1 << 23);
   const bool n0 = sb0 == 0xFFu, n1 = sb1 == 0xFFu;
@@ -538,7 +681,11 @@ extern "C" __attribute__((visibility("default"))) int moe_downcast_mxfp4(const v
     const bool cols_ok = sx_outer == 1 && sx_quant != 1 && outer % 2 == 0 && ((uintptr_t)x % (2 * sizeof(T)) == 0) &&
                          (sx_quant % 2 == 0) && (sx_batch % 2 == 0) && ((uintptr_t)q % 16 == 0) &&
                          col_tiles(batch, outer, quant) < 2147483647LL;
-    if (rows_ok && (uintptr_t)q % 16 == 0) {
+    if (rows_ok && (uintptr_t)q % 16 == 0 && sx_outer == quant && (batch == 1 || sx_batch == outer * quant)) {
+      const int64_t total = batch * outer * (quant >> 5);
+      MOE_CHECK_CUDA(launch_pdl(downcast_dense_kernel<T>, dim3(grid_for(total, GROUPS_UNROLL * 256)), dim3(256), 0, st, (const T*)x, total, q, scale,
+                                rounding_mode));
+    } else if (rows_ok && (uintptr_t)q % 16 == 0) {
       const int64_t total = batch * outer * (quant >> 5);
       if (total + (int64_t)GROUPS_UNROLL * 256 * moe_sm_count() * 16 < 2147483647LL)       // 32-bit row / group counters
         MOE_CHECK_CUDA(launch_pdl(downcast_rows_kernel<T, int32_t>, dim3(grid_for(total, GROUPS_UNROLL * 256)), dim3(256), 0, st,
@@ -576,7 +723,10 @@ extern "C" __attribute__((visibility("default"))) int moe_upcast_mxfp4(const uin
                          (so_batch % align == 0) && ((uintptr_t)q % 4 == 0);
     const bool wide = rows_ok && (uintptr_t)out % 32 == 0 && so_outer % (2 * align) == 0 && so_batch % (2 * align) == 0 &&
                       (uintptr_t)q % 8 == 0;
-    if (wide) {
+    if (wide && (uintptr_t)q % 16 == 0 && so_outer == quant && (batch == 1 || so_batch == outer * quant)) {
+      const int64_t total = batch * outer * (quant * (int64_t)sizeof(T) >> 6);
+      MOE_CHECK_CUDA(launch_pdl(upcast_dense_kernel<T>, dim3(grid_for(total, UP_DENSE_UNROLL * 256)), dim3(256), 0, st, q, scale, (T*)out, total));
+    } else if (wide) {
       const int64_t total = batch * outer * (quant * (int64_t)sizeof(T) >> 5);
       MOE_CHECK_CUDA(launch_pdl(upcast_rows_kernel<T, true>, dim3(grid_for(total, ROWS_UNROLL * 256)), dim3(256), 0, st, q, scale,
                                 (T*)out, batch * outer, quant, outer, so_batch, so_outer));

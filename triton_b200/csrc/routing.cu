@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(HIST ? 1024 : 256) topk_quad_kernel(
 // ---------------------------------------------------------------------------------------------------
 // Expert histogram + stable expert-major sort.  Flat entry i = token * k + slot, expert c = indx[i]
 // (negative, or token >= n_rows: dropped).  row_sorted[i] = col_offs[c] + #{j < i : indx[j] == c},
-// col_sorted = inverse permutation; both -1 padded.  Three passes (up to 32768 entries of 256 experts: bm_cluster_kernel below):
+// col_sorted = inverse permutation; both -1 padded.  Three passes (up to 32768 entries of 256 experts: bm_wide_kernel below):
 //   pass 1: per block of kTokPerBlock tokens, a shared-memory histogram -> partial[blk][e]; both index arrays
 //           pre-filled with -1.
 //   pass 2: exclusive scan of partial[.][e] over blocks, totals -> col_sum, their exclusive scan -> col_offs.
@@ -439,93 +439,86 @@ __device__ __forceinline__ int ld_cluster(const int32_t* shared, uint32_t rank) 
 }
 
 
-// The sort of up to 32768 entries in one launch of one cluster: eight blocks take an eighth of the entries each, read one another's expert
-// counts through distributed shared memory and rank their own on top of them.  Behind the router as three launches: 4100 tokens, k = 4,
-// of 128 experts 26.3 us, so 23.5; 16 tokens 19.2 and 16.0.
-constexpr int kSortClusterEntries = 32768;
-__global__ void __launch_bounds__(1024) bm_cluster_kernel(const int16_t* indx, int64_t ld_indx, int T_rows, int E, int k, const int32_t* n_rows_dev,
-                                                         int32_t* col_sum, int32_t* col_sorted, int32_t* row_sorted) {
-  // [E] own counts, [E] sizes, [E] offsets, [E] entries of the blocks before, [warps in use][E] counters (uint16), [n] experts (int16)
+// The sort of up to 32768 entries in one launch of blocks that do not wait on one another: a block ranks 1024 entries, one to a thread, and
+// counts all of them for itself, those ahead of its own apart (two counters per expert, in four copies against threads that
+// meet on one).  Every chain is short: a read of at most 64 KB from L2, its counts, a scan of the experts, a prefix over the warps.  As one cluster of eight
+// blocks with an eighth of the entries each the counts took two cluster barriers and three rounds of a warp's matches.  Behind the router, before and now: 1 token
+// 16.6 -> 16.0 us, 4100 tokens of 128 experts, k = 4, 29.2 -> 26.7, k = 8 35.1 -> 29.7, 8192 tokens 32.9 -> 31.9.
+constexpr int kSortWideEntries = 32768, kSortWideBlock = 1024, kSortWideCopies = 4;
+__global__ void __launch_bounds__(kSortWideBlock) bm_wide_kernel(const int16_t* indx, int64_t ld_indx, int T_rows, int E, int k, const int32_t* n_rows_dev,
+                                                                 int32_t* col_sum, int32_t* col_sorted, int32_t* row_sorted) {
+  // [copies][2][E] counts, [E] sizes, [E] offsets, [E] entries of the blocks before, [32][E] first positions of a warp's entries
   extern __shared__ int32_t s_mem[];
   __shared__ int32_t s_warp[33];
   pdl_begin();
-  const int rank = (int)cluster_rank(), n_all = T_rows * k, n_max = (n_all + kRouteCluster - 1) / kRouteCluster, first = rank * n_max;
-  const int n = max(0, min(n_max, n_all - first)), n_rows = n_rows_dev ? min(*n_rows_dev, T_rows) : T_rows;
-  const int rounds = (n_max + 1023) >> 10, per = rounds * 32, warps = (n_max + per - 1) / per;      // entries of a warp, warps with entries
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int32_t* s_own = s_mem;
-  int32_t* s_size = s_own + E;
+  const int n = T_rows * k, first = (int)blockIdx.x * kSortWideBlock, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n_rows = n_rows_dev ? min(max(*n_rows_dev, 0), T_rows) : T_rows, live = n_rows * k;      // entries that count
+  int32_t* s_size = s_mem + 2 * kSortWideCopies * E;
   int32_t* s_offs = s_size + E;
   int32_t* s_before = s_offs + E;
-  uint16_t* s_cnt = reinterpret_cast<uint16_t*>(s_before + E);
-  int16_t* s_pick = reinterpret_cast<int16_t*>(s_cnt + warps * E);
-  for (int e = threadIdx.x; e < E; e += blockDim.x) s_own[e] = 0;
-  for (int i = threadIdx.x; i < warps * E; i += blockDim.x) s_cnt[i] = 0;
-  for (int j = threadIdx.x; j < n; j += blockDim.x) {
-    const int token = (first + j) / k;
-    s_pick[j] = (int16_t)entry_expert(indx, ld_indx, k, token, first + j - token * k, n_rows, E);
-  }
+  int32_t* s_cnt = s_before + E;
+  for (int i = threadIdx.x; i < 2 * kSortWideCopies * E; i += kSortWideBlock) s_mem[i] = 0;
+  for (int i = threadIdx.x; i < 32 * E; i += kSortWideBlock) s_cnt[i] = 0;
+  const int j = first + (int)threadIdx.x;
+  const int c = j < live ? entry_expert(indx, ld_indx, k, j / k, j % k, n_rows, E) : -1;
   __syncthreads();
-  uint16_t* my = s_cnt + warp * E;
-  if (warp < warps)
-    for (int r = 0; r < rounds; ++r) {
-      const int j = warp * per + r * 32 + lane, c = j < n ? s_pick[j] : -1;
-      const unsigned peers = __match_any_sync(0xFFFFFFFFu, c);
-      if (c >= 0 && (peers & ((1u << lane) - 1u)) == 0) {
-        my[c] += (uint16_t)__popc(peers);
-        atomicAdd(&s_own[c], __popc(peers));
-      }
-      __syncwarp();
-    }
-  __syncthreads();
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-  for (int e = threadIdx.x; e < E; e += blockDim.x) {
-    int v[kRouteCluster], before = 0, total = 0;
-#pragma unroll
-    for (int i = 0; i < kRouteCluster; ++i) v[i] = ld_cluster(s_own + e, (uint32_t)i);
-#pragma unroll
-    for (int i = 0; i < kRouteCluster; ++i) {
-      if (i < rank) before += v[i];
-      total += v[i];
-    }
-    s_size[e] = total;
-    s_before[e] = before;
-    if (rank == 0) col_sum[e] = total;
-  }
-  __syncthreads();
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");      // the others' counts have been read
-  block_exclusive_scan(s_size, s_offs, E, s_warp);
-  const int kept = s_offs[E - 1] + s_size[E - 1];
-  for (int e = threadIdx.x; e < E; e += blockDim.x) {
-    int run = s_offs[e] + s_before[e];
-    for (int w0 = 0; w0 < warps; w0 += 8) {
-      int v[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) v[u] = w0 + u < warps ? s_cnt[(w0 + u) * E + e] : 0;
+  int32_t* copy = s_mem + (warp & (kSortWideCopies - 1)) * 2 * E;
+  int done = 0;                                      // entries counted eight at a time: rows without a gap, on a 16-byte boundary
+  if (ld_indx == k && (uintptr_t)indx % 16 == 0) {
+    done = live & ~7;
+    for (int i = (int)threadIdx.x * 8; i < done; i += kSortWideBlock * 8) {
+      const uint4 v = *reinterpret_cast<const uint4*>(indx + i);
+      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+      int32_t* at = copy + (i >= first ? E : 0);     // (`first` is a multiple of eight)
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
-        if (w0 + u < warps) s_cnt[(w0 + u) * E + e] = (uint16_t)run;
+        const int e = (int16_t)(w[u >> 1] >> (16 * (u & 1)));
+        if (e >= 0 && e < E) atomicAdd(at + e, 1);
+      }
+    }
+  }
+  for (int i = done + (int)threadIdx.x; i < live; i += kSortWideBlock) {
+    const int e = entry_expert(indx, ld_indx, k, i / k, i % k, n_rows, E);
+    if (e >= 0) atomicAdd(copy + (i >= first ? E : 0) + e, 1);
+  }
+  const unsigned peers = __match_any_sync(0xFFFFFFFFu, c);
+  const int rank = __popc(peers & ((1u << lane) - 1u));
+  if (c >= 0 && rank == 0) s_cnt[warp * E + c] = __popc(peers);
+  __syncthreads();
+  for (int e = threadIdx.x; e < E; e += kSortWideBlock) {
+    int before = 0, total = 0;
+#pragma unroll
+    for (int i = 0; i < kSortWideCopies; ++i) {
+      before += s_mem[2 * i * E + e];
+      total += s_mem[(2 * i + 1) * E + e];
+    }
+    total += before;
+    s_size[e] = total;
+    s_before[e] = before;
+    if (blockIdx.x == 0) col_sum[e] = total;
+  }
+  __syncthreads();
+  block_exclusive_scan(s_size, s_offs, E, s_warp);
+  const int kept = s_offs[E - 1] + s_size[E - 1];
+  for (int e = threadIdx.x; e < E; e += kSortWideBlock) {
+    int run = s_offs[e] + s_before[e];
+#pragma unroll
+    for (int w0 = 0; w0 < 32; w0 += 8) {
+      int v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = s_cnt[(w0 + u) * E + e];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        s_cnt[(w0 + u) * E + e] = run;
         run += v[u];
       }
     }
   }
-  // (positions past the last entry that counts)
-  for (int i = first + threadIdx.x; i < first + n; i += blockDim.x)
-    if (i >= kept) col_sorted[i] = -1;
+  if (j < n && j >= kept) col_sorted[j] = -1;        // positions past the last entry that counts
   __syncthreads();
-  if (warp < warps)
-    for (int r = 0; r < rounds; ++r) {
-      const int j = warp * per + r * 32 + lane, c = j < n ? s_pick[j] : -1;
-      const unsigned peers = __match_any_sync(0xFFFFFFFFu, c);
-      const int before = __popc(peers & ((1u << lane) - 1u));
-      const int base = c >= 0 ? my[c] : 0;
-      __syncwarp();
-      if (c >= 0 && before == 0) my[c] = (uint16_t)(base + __popc(peers));
-      __syncwarp();
-      if (j < n) row_sorted[first + j] = c >= 0 ? base + before : -1;
-      if (c >= 0) col_sorted[base + before] = first + j;
-    }
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");        // no block leaves while its counts are read
+  const int at = c >= 0 ? s_cnt[warp * E + c] + rank : -1;
+  if (j < n) row_sorted[j] = at;
+  if (c >= 0) col_sorted[at] = j;
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -690,21 +683,10 @@ extern "C" __attribute__((visibility("default"))) int moe_bitmatrix_metadata(con
   MOE_CHECK_ARG(workspace_bytes >= moe_bitmatrix_metadata_workspace(T, E, k),
                 "moe_bitmatrix_metadata: workspace too small (%zu < %zu)", workspace_bytes,
                 moe_bitmatrix_metadata_workspace(T, E, k));
-  if (T * k <= kSortClusterEntries && E <= 256) {
-    const int n_max = ((int)(T * k) + kRouteCluster - 1) / kRouteCluster, warps = (n_max + 31) / 32 < 32 ? (n_max + 31) / 32 : 32;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(kRouteCluster);
-    cfg.blockDim = dim3(1024);
-    cfg.dynamicSmemBytes = (size_t)4 * E * sizeof(int32_t) + (size_t)(warps * E + n_max) * sizeof(int16_t);      // <= 28 KB
-    cfg.stream = st;
-    cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    at[1].id = cudaLaunchAttributeClusterDimension;
-    at[1].val.clusterDim.x = kRouteCluster; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 2;
-    MOE_CHECK_CUDA(cudaLaunchKernelEx(&cfg, bm_cluster_kernel, indx, ld_indx, (int)T, E, k, n_rows_dev, col_sum, col_sorted, row_sorted));
+  if (T * k <= kSortWideEntries && E <= 256) {
+    const size_t smem = (size_t)(2 * kSortWideCopies + 3 + 32) * E * sizeof(int32_t);      // <= 43 KB
+    MOE_CHECK_CUDA(launch_pdl(bm_wide_kernel, dim3((unsigned)cdiv64(T * k, kSortWideBlock)), dim3(kSortWideBlock), smem, st, indx, ld_indx, (int)T, E, k,
+                              n_rows_dev, col_sum, col_sorted, row_sorted));
     MOE_CHECK_LAUNCH();
     return MOE_OK;
   }

@@ -744,7 +744,7 @@ extern "C" __attribute__((visibility("default"))) int moe_ragged_metadata_remap(
 
 // ---------------------------------------------------------------------------------------------------------
 // moe_route: the whole routing step in one to three launches (the standalone entry points above take more).  Small batches: one launch of five
-// independent blocks (route_small_kernel); up to some 1500 tokens: one launch of a cluster of eight (route_cluster_kernel, both at the end of
+// independent blocks (route_small_kernel); up to 896 tokens (1536 with long lists): one launch of a cluster of eight (route_cluster_kernel, both at the end of
 // this section; rule: route_form).  Others: A, then route_finish_kernel where its blocks are a wave, else B and C.
 //   A  topk_quad_kernel<HIST>   top-k + softmax + bitmatrix row of every token, and the expert histogram of each block
 //      (route_topk_hist_kernel  of 128 tokens (partial[blk][e]) in the same pass over the logits;
@@ -1175,10 +1175,9 @@ __global__ void __launch_bounds__(1024) route_small_kernel(
 
 constexpr int kRouteSmallTokens = 256;
 
-// The whole routing step of a batch of up to 1536 tokens (2048 with short lists, see route_form) in one launch of one cluster: eight blocks take an eighth of the tokens each, read
+// The whole routing step of a batch of up to 896 tokens (1536 with long lists, see route_form) in one launch of one cluster: eight blocks take an eighth of the tokens each, read
 // one another's expert counts through distributed shared memory behind a cluster barrier, and rank their own entries on top of
 // them; blocks 3 to 7 build a row of the ragged metadata each.
-constexpr int kRouteClusterTokens = 2048;
 
 template <typename T, int K>
 __global__ void __launch_bounds__(1024) route_cluster_kernel(
@@ -1306,14 +1305,14 @@ extern "C" __attribute__((visibility("default"))) size_t moe_route_workspace(int
 //   32 experts, k = 4:   64 tokens 7.4, 6.8;  96  6.3, 7.2;  256  8.8, 9.8, 7.9;  300  -, 7.9, 8.0, 11.9;  1024  -, 9.7, 8.4;  2048  -, 11.3, 8.6, 12.8
 //   8 experts, k = 2:    64 tokens 5.3, 6.0;  256  5.2, 7.6, 6.6;  300  -, 6.5, 6.7, 12.5;  2048  -, 7.4, 7.2, 12.9
 //   256 experts, k = 16: 64 tokens 26.8, 11.7, 36.7;  768  -, 29.7, 39.9;  1536  -, 44.2, 40.5;  2048  -, 56.1, 41.5
-// The small form repeats the whole selection in five blocks, the cluster has an eighth of it in each of eight and two barriers; past some
-// 1500 tokens eight SMs are fewer than the selection wants.  The lines above 256 tokens lie where the cluster meets three
-// launches; two launches (which only the sizes beyond take) would be ahead of it from 512 to 1024 tokens on, with 256 experts and k = 16 from 1500.
+// The small form repeats the whole selection in five blocks, the cluster has an eighth of it in each of eight and two barriers; past 768 to 1024
+// tokens eight SMs are fewer than the selection wants, and two launches are ahead.  With long lists (E k > 1024) the finish of those takes
+// longest and the line lies at 1536.
 enum { ROUTE_SMALL, ROUTE_CLUSTER, ROUTE_LAUNCHES };
 static int route_form(int64_t T, int E, int k) {
   if (!(k == 1 || k == 2 || k == 4 || k == 8 || k == 16)) return ROUTE_LAUNCHES;
   if (T <= kRouteSmallTokens) return T >= 24 && k >= 4 && (E * k >= 512 || T <= 64) ? ROUTE_CLUSTER : ROUTE_SMALL;
-  return T <= (E * k <= 128 ? kRouteClusterTokens : 1536) ? ROUTE_CLUSTER : ROUTE_LAUNCHES;
+  return T <= (E * k <= 1024 ? 896 : 1536) ? ROUTE_CLUSTER : ROUTE_LAUNCHES;
 }
 
 static int route_launch(

@@ -149,6 +149,14 @@ __device__ __forceinline__ void elect_bulk_g2s_hint(uint32_t dst, const void* sr
       "l"(src), "r"(bytes), "r"(bar), "l"(policy)
       : "memory");
 }
+__device__ __forceinline__ void elect_tile_4d_hint(uint32_t dst, const CUtensorMap* tmap, int x, int y, int z, int w, uint32_t bar, uint64_t policy) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\telect.sync _|q, 0xFFFFFFFF;\n\t"
+      "@q cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3, %4, %5}], [%6], %7;\n\t}" ::"r"(dst),
+      "l"(tmap), "r"(x), "r"(y), "r"(z), "r"(w), "r"(bar), "l"(policy)
+      : "memory");
+}
+
 __device__ __forceinline__ void elect_tile_4d(uint32_t dst, const CUtensorMap* tmap, int x, int y, int z, int w, uint32_t bar) {
   asm volatile(
       "{\n\t.reg .pred q;\n\telect.sync _|q, 0xFFFFFFFF;\n\t"

@@ -40,6 +40,15 @@ struct StreamSmem {
   static_assert(ALLOC <= 232448, "shared memory budget");
 };
 
+// a copy of weights; `once`: they are the first to leave L2
+__device__ __forceinline__ void copy_weights(bool once, uint64_t policy, uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  if (once)
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(bar), "l"(policy)
+                 : "memory");
+  else
+    bulk_g2s(dst, src, bytes, bar);
+}
 __device__ __forceinline__ void mma_f16_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                               uint32_t b1) {
   asm volatile(
@@ -141,6 +150,11 @@ __global__ void __launch_bounds__(S_THREADS, 1) gemm_stream_kernel(const GemmPar
       uint32_t it = 0;
       bool ok = true;
       const uint8_t* wv = (const uint8_t*)p.w;
+      // Up to a third of a block of rows per expert, where few experts have several blocks (us per step of the operators: 24 tokens of 128 experts of
+      // 512 x 2880 81.7 -> 77.4, 25 of 1024 x 4096 105.2 -> 98.0).
+      const bool once = 3 * p.M <= S_ROWS * (int64_t)(p.slice_sizes ? p.E : 1);
+      uint64_t policy;
+      asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
       const uint8_t* ws = p.w_scale;
       for (int64_t i = i_begin; i < i_end && ok; ++i) {
         Item m;
@@ -152,8 +166,8 @@ __global__ void __launch_bounds__(S_THREADS, 1) gemm_stream_kernel(const GemmPar
           if (!ok) break;
           const uint32_t dst = sbase + C::OFF_RING + s * S_STAGE_BYTES;
           mbar_expect_tx(BAR_FULL(s), (uint32_t)S_STAGE_BYTES);
-          bulk_g2s(dst, wv + (tile0 + kt) * (2 * RAWV_BYTES), 2 * RAWV_BYTES, BAR_FULL(s));
-          bulk_g2s(dst + 2 * RAWV_BYTES, ws + (tile0 + kt) * RAWS_BYTES, RAWS_BYTES, BAR_FULL(s));
+          copy_weights(once, policy, dst, wv + (tile0 + kt) * (2 * RAWV_BYTES), 2 * RAWV_BYTES, BAR_FULL(s));
+          copy_weights(once, policy, dst + 2 * RAWV_BYTES, ws + (tile0 + kt) * RAWS_BYTES, RAWS_BYTES, BAR_FULL(s));
         }
       }
       if (!ok) {

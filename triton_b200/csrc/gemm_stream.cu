@@ -95,11 +95,6 @@ __global__ void __launch_bounds__(S_THREADS, 1) gemm_stream_kernel(const GemmPar
   float* s_xexp = reinterpret_cast<float*>(smem + C::OFF_XEXP);
   Ctl ctl{s_abort, p.status};
 
-  const int NT = (p.N + HALF_N - 1) / HALF_N;
-  const int KT_TILES = (p.K + TILE_K - 1) / TILE_K;
-  const int KG = p.K >> 5;                                  // 32-k groups (K % 32 == 0)
-  const int n_experts = p.slice_sizes ? p.E : 1;
-
   if (threadIdx.x == 0) {
     for (int s = 0; s < S_STAGES; ++s) {
       mbar_init(BAR_FULL(s), 1);
@@ -111,20 +106,19 @@ __global__ void __launch_bounds__(S_THREADS, 1) gemm_stream_kernel(const GemmPar
     *s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  pdl_begin();
+  const int NT = (p.N + HALF_N - 1) / HALF_N;
+  const int KT_TILES = (p.K + TILE_K - 1) / TILE_K;
+  const int KG = p.K >> 5;                                  // 32-k groups (K % 32 == 0)
+  const int n_experts = p.slice_sizes ? p.E : 1;
+
   // items per expert: ceil(rows / 16) row blocks x NT weight tiles; exclusive prefix in shared memory
   for (int e = threadIdx.x; e < n_experts; e += S_THREADS) {
     const int rows = p.slice_sizes ? max(p.slice_sizes[e], 0) : (int)p.M;
     s_prefix[e + 1] = ((rows + S_ROWS - 1) / S_ROWS) * NT;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int run = 0;
-    s_prefix[0] = 0;
-    for (int e = 1; e <= n_experts; ++e) {
-      run += s_prefix[e];
-      s_prefix[e] = run;
-    }
-  }
+  if (warp == 0) warp_prefix(s_prefix, n_experts, lane);
   __syncthreads();
   const int64_t total = s_prefix[n_experts];
   const int64_t i_begin = total * blockIdx.x / gridDim.x, i_end = total * (blockIdx.x + 1) / gridDim.x;
@@ -381,11 +375,11 @@ int moe_gemm_stream_launch(const GemmParams& p, const MoeGemmArgs& a, cudaStream
   if (a.y_dtype == MOE_BF16) {
     MOE_CHECK_CUDA(cudaFuncSetAttribute(gemm_stream_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         StreamSmem::ALLOC));
-    gemm_stream_kernel<__nv_bfloat16><<<grid, S_THREADS, StreamSmem::ALLOC, st>>>(p);
+    MOE_CHECK_CUDA(launch_pdl(gemm_stream_kernel<__nv_bfloat16>, dim3((unsigned)grid), dim3(S_THREADS), (size_t)StreamSmem::ALLOC, st, p));
   } else {
     MOE_CHECK_CUDA(cudaFuncSetAttribute(gemm_stream_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         StreamSmem::ALLOC));
-    gemm_stream_kernel<float><<<grid, S_THREADS, StreamSmem::ALLOC, st>>>(p);
+    MOE_CHECK_CUDA(launch_pdl(gemm_stream_kernel<float>, dim3((unsigned)grid), dim3(S_THREADS), (size_t)StreamSmem::ALLOC, st, p));
   }
   MOE_CHECK_LAUNCH();
   return MOE_OK;

@@ -78,6 +78,24 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, const C
   }
 }
 
+// prefix[1 .. n]: counts of n experts -> counts of the experts up to each, prefix[0] = 0 (one warp).  (By a single thread 128 experts took some 2 us
+// of every launch.)
+__device__ __forceinline__ void warp_prefix(int32_t* prefix, int n, int lane) {
+  int run = 0;
+  for (int e0 = 1; e0 <= n; e0 += 32) {
+    const int e = e0 + lane;
+    int v = e <= n ? prefix[e] : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xFFFFFFFFu, v, o);
+      if (lane >= o) v += t;
+    }
+    if (e <= n) prefix[e] = run + v;
+    run += __shfl_sync(0xFFFFFFFFu, v, 31);
+  }
+  if (lane == 0) prefix[0] = 0;
+}
+
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }

@@ -86,6 +86,7 @@ gemm_tc_kernel(const GemmParams p, const int64_t grid_m_static, const __grid_con
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const uint32_t sbase = smem_u32(smem);
   const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;     // warp-uniform for the compiler
+  pdl_begin();
   // 256-row tiles of consecutive token rows are fetched by TMA tile copies (x_map), everything else by cp.async
   const bool use_tma = MH == 2 && p.gather_indx == nullptr;
   // second epilogue group (see the epilogue role): only where the loader warps are free and the epilogue is heavy
@@ -138,14 +139,7 @@ gemm_tc_kernel(const GemmParams p, const int64_t grid_m_static, const __grid_con
       for (int e = threadIdx.x; e < p.E; e += NUM_THREADS)
         s_prefix[e + 1] = (max(p.slice_sizes[e], 0) + 2 * HALF_M - 1) / (2 * HALF_M);
       __syncthreads();
-      if (threadIdx.x == 0) {
-        int run = 0;
-        s_prefix[0] = 0;
-        for (int e = 1; e <= p.E; ++e) {
-          run += s_prefix[e];
-          s_prefix[e] = run;
-        }
-      }
+      if (warp == 0) warp_prefix(s_prefix, p.E, lane);
     }
   }
   tc_fence_before();
@@ -683,7 +677,7 @@ static int launch_tc(const GemmParams& p, int64_t grid_m, int64_t N, int idle_sm
   memset(&x_map, 0, sizeof(x_map));
   if (MH == 2 && p.gather_indx == nullptr)
     if (int rc = make_x_map(p, &x_map)) return rc;
-  gemm_tc_kernel<TY, MH, NH><<<grid, NUM_THREADS, Cfg<MH, NH>::SMEM_ALLOC, st>>>(p, grid_m, x_map);
+  MOE_CHECK_CUDA(launch_pdl(gemm_tc_kernel<TY, MH, NH>, dim3((unsigned)grid), dim3(NUM_THREADS), (size_t)Cfg<MH, NH>::SMEM_ALLOC, st, p, grid_m, x_map));
   MOE_CHECK_LAUNCH();
   return MOE_OK;
 }

@@ -119,14 +119,7 @@ gemm_tc_pair_kernel(const GemmParams p, const int64_t grid_m_static, const __gri
     for (int e = threadIdx.x; e < p.E; e += PAIR_THREADS)
       s_prefix[e + 1] = (max(p.slice_sizes[e], 0) + 2 * HALF_M - 1) / (2 * HALF_M);
     __syncthreads();
-    if (threadIdx.x == 0) {
-      int run = 0;
-      s_prefix[0] = 0;
-      for (int e = 1; e <= p.E; ++e) {
-        run += s_prefix[e];
-        s_prefix[e] = run;
-      }
-    }
+    if (warp == 0) warp_prefix(s_prefix, p.E, threadIdx.x & 31);
   }
   tc_fence_before();
   __syncthreads();

@@ -3,7 +3,7 @@
 //
 // Semantics follow triton_kernels topk_details/_topk_forward.py:15-150, tensor_details/bitmatrix.py:43-150
 // and tensor_details/ragged_tensor.py:128-210, 310-381; the kernels themselves are organised
-// differently (four lanes per token row for the top-k, a warp for other k; a counting sort, in one cluster for up to 32768 entries, else
+// differently (four lanes per token row for the top-k, a warp for other k; a counting sort, in one launch for up to 32768 entries, else
 // in three passes, instead of per-block bitonic sorts; one launch each for the ragged metadata and its remap; the
 // whole step in one to three launches).
 #include "common.cuh"
@@ -1470,7 +1470,7 @@ extern "C" __attribute__((visibility("default"))) int moe_route_positions(
 // all device memory to its own pools at start-up, or a latency-critical section in which cudaMalloc (which
 // synchronises the device) is not acceptable.  The three sort passes need nb * E + E ints of scratch
 // (nb = ceil(T / 256)); here that scratch is a fixed array inside the library image (up to 32768 entries of 256 experts the sort is
-// one cluster and does not touch it).
+// one launch and does not touch it).
 //
 // Cost: every GPU that loads libmoe_b200.so carries kNoAllocScratchBytes (1 MiB) of device memory until the
 // process exits, whether or not this entry point is ever called.

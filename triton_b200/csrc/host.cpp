@@ -3,6 +3,7 @@
 // 16 tokens: 180 us of host work for 100 us of kernels).  No computation happens here; the library is the one the Python
 // binding loaded (its handle is passed in), and every entry point keeps its checks and messages.
 #include <torch/extension.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAStream.h>
 #include <dlfcn.h>
 #include "../../include/moe_b200.h"
@@ -467,9 +468,11 @@ class StepGraph {
   ~StepGraph() { lib.moe_step_graph_destroy(step_); }
   StepGraph(const StepGraph&) = delete;
   StepGraph& operator=(const StepGraph&) = delete;
-  // None where the inputs are not plain copies of the step's on the current device
+  // None where the inputs are not plain copies of the step's on the current device, or the stream is being captured
   std::optional<Tensor> run(const Tensor& x, const Tensor& logits) {
-    if (!plain_copy(x_, x) || !plain_copy(logits_, logits) || x_.device().index() != c10::cuda::current_device()) return std::nullopt;
+    if (!plain_copy(x_, x) || !plain_copy(logits_, logits) || x_.device().index() != c10::cuda::current_device() ||
+        c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None)
+      return std::nullopt;
     Tensor out = at::empty(z_.sizes(), z_.options());
     check(lib.moe_step_graph_launch(step_, x.data_ptr(), logits.data_ptr(), out.data_ptr(), stream()), "moe_step_graph_launch");
     return out;

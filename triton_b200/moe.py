@@ -239,7 +239,8 @@ class GraphedMoeLayer:
         self.graph = torch.cuda.CUDAGraph(keep_graph=True)
         with torch.cuda.graph(self.graph):
             self.z = self.forward(self.x, self.logits)
-        # the layer's own step also as a graph with the copies of a call in it (1 token 32.9 -> 31.1 us); replay() instantiates the plain one when it is first called
+        self.graph.instantiate()
+        # the layer's own step also as a graph with the copies of a call in it (1 token 32.9 -> 31.1 us)
         self.step = None
         if forward is None and self.z.numel() > 0:
             self.step = _lib.host().StepGraph(self.graph.raw_cuda_graph(), self.x, self.logits, self.z)

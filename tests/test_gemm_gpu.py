@@ -326,6 +326,25 @@ def test_graphed_layer_takes_inputs_of_any_layout(form, layer_20b, device):
     tb.matmul_check_status()
 
 
+# routing of more than 256 experts and of lists that one launch does not take: the first kernel of the captured step is another one
+@pytest.mark.parametrize("E, k", [(320, 10), (320, 8), (256, 6), (64, 4)])
+def test_graphed_layer_routes_the_logits_of_its_own_call(E, k, device):
+    """The step's kernels start behind the copy of the inputs, whichever of them is first: calls with new inputs in turn equal the eager layer's
+    (large inputs, so that a kernel that did not wait would meet those of the call before)."""
+    from triton_b200.moe import GraphedMoeLayer, moe_layer_forward
+    from triton_b200.testing import make_synthetic_layer
+    T, d = 1024, 512
+    lw = make_synthetic_layer(E, d, 256, device, seed=7, block_scaled=True)
+    graphed = GraphedMoeLayer(lw, k, T, d, E, device)
+    g = torch.Generator(device=device).manual_seed(E + k)
+    inputs = [(torch.randn(T, d, device=device, generator=g).bfloat16(), torch.randn(T, E, device=device, generator=g)) for _ in range(6)]
+    want = [moe_layer_forward(x, logits, lw, k) for x, logits in inputs]
+    torch.cuda.synchronize()
+    got = [graphed(x, logits) for x, logits in inputs]
+    tb.matmul_check_status()
+    assert all(torch.equal(a, b) for a, b in zip(want, got)) and not torch.equal(want[0], want[1])
+
+
 def test_host_streaming_layer(layer_20b, device):
     """Steps fed from and returned to pinned host memory through the three-stream pipeline equal the eager layer."""
     from triton_b200.moe import HostStreamingLayer, moe_layer_forward

@@ -457,11 +457,12 @@ Tensor copy_of(const Tensor& src) {
   return out;
 }
 
-// A captured layer step, routing first, with its copies (moe_step_graph_create): x and logits in, a new tensor out.
+// A captured layer step with its copies (moe_step_graph_create): x and logits in, a new tensor out.  roots_wait: the first kernel of the
+// captured step waits for the one before by itself.
 class StepGraph {
  public:
-  StepGraph(int64_t graph, const Tensor& x, const Tensor& logits, const Tensor& z) : x_(x), logits_(logits), z_(z) {
-    check(lib.moe_step_graph_create(reinterpret_cast<void*>(graph), 1, x.data_ptr(), (int64_t)x.nbytes(), logits.data_ptr(), (int64_t)logits.nbytes(),
+  StepGraph(int64_t graph, bool roots_wait, const Tensor& x, const Tensor& logits, const Tensor& z) : x_(x), logits_(logits), z_(z) {
+    check(lib.moe_step_graph_create(reinterpret_cast<void*>(graph), roots_wait, x.data_ptr(), (int64_t)x.nbytes(), logits.data_ptr(), (int64_t)logits.nbytes(),
                                     z.data_ptr(), (int64_t)z.nbytes(), &step_),
           "moe_step_graph_create");
   }
@@ -486,7 +487,7 @@ class StepGraph {
 }  // namespace
 
 PYBIND11_MODULE(_host, m) {
-  py::class_<StepGraph>(m, "StepGraph").def(py::init<int64_t, const Tensor&, const Tensor&, const Tensor&>()).def("run", &StepGraph::run);
+  py::class_<StepGraph>(m, "StepGraph").def(py::init<int64_t, bool, const Tensor&, const Tensor&, const Tensor&>()).def("run", &StepGraph::run);
   m.def("copy2", &copy2);
   m.def("copy_of", &copy_of);
   m.def("bind", &bind);

@@ -243,7 +243,10 @@ class GraphedMoeLayer:
         # the layer's own step also as a graph with the copies of a call in it (1 token 32.9 -> 31.1 us)
         self.step = None
         if forward is None and self.z.numel() > 0:
-            self.step = _lib.host().StepGraph(self.graph.raw_cuda_graph(), self.x, self.logits, self.z)
+            # The step's first kernel may start ahead of the end of the copy where it is known to wait for it: the one-call path's is the
+            # routing, which does.  The composition of operators (more than 256 experts, say) starts with kernels that do not all wait.
+            waits = _one_call(self.x, self.logits, lw, k)
+            self.step = _lib.host().StepGraph(self.graph.raw_cuda_graph(), waits, self.x, self.logits, self.z)
 
     def replay(self):
         """Replay on the graph's own input buffers (`self.x`, `self.logits`); the result is `self.z`."""

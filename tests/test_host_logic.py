@@ -464,3 +464,24 @@ def test_kernels_read_nothing_of_the_chain_ahead_of_their_wait():
             reads = r"slice_sizes|slice_offs|block_offs|block_sched|p\.bias|gather|pair_prefix|map_block|map_ptile|elect_(tile|bulk|expect)|ld_?global|__ldg|cp_async"
             assert not re.search(reads, ahead), f"{path.name}: {m.group(1)}: {re.search(reads, ahead).group(0)}"
     assert launched <= waiting and {"gemm_mx_kernel", "gemm_mx_pair_kernel", "router_topk_kernel", "route_cluster_kernel"} <= waiting
+
+
+def test_kernels_take_tensor_memory_before_they_let_the_next_one_go():
+    """A kernel that lets its dependents go and then asks for tensor memory can find it taken by one of them, which waits for this kernel's end: all
+    warps meet between the allocation and the release."""
+    import pathlib
+    import re
+    csrc = pathlib.Path(triton_b200.__file__).parent / "csrc"
+    found = set()
+    for path in sorted(csrc.glob("*.cu")):
+        text = re.sub(r"//[^\n]*", "", path.read_text())
+        for m in re.finditer(r"__global__ void\s+(?:__launch_bounds__\((?:[^()]|\([^()]*\))*\)\s*)?(\w+)\(", text):
+            body = text[m.end():]
+            body = body[:body.index("\n}\n")]
+            if "tcgen05.alloc" not in body or "pdl_begin" not in body:
+                continue
+            found.add(m.group(1))
+            assert body.count("tcgen05.alloc") == 1
+            assert "__syncthreads();" in body[body.index("tcgen05.alloc"):].split("pdl_begin();")[0], m.group(1)
+            assert body.index("tcgen05.alloc") < body.index("pdl_begin();"), m.group(1)
+    assert {"gemm_tc_kernel", "gemm_mx_kernel", "gemm_mx_pair_kernel", "router_topk_kernel"} <= found

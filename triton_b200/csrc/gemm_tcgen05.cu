@@ -86,6 +86,14 @@ gemm_tc_kernel(const GemmParams p, const int64_t grid_m_static, const __grid_con
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const uint32_t sbase = smem_u32(smem);
   const int warp = __shfl_sync(0xFFFFFFFFu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;     // warp-uniform for the compiler
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sbase + C::OFF_MISC),
+                 "r"((uint32_t)TMEM_COLS)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  // (the memory is there before a dependent may start: one that took it on this SM would wait for this kernel's end)
+  __syncthreads();
   pdl_begin();
   // 256-row tiles of consecutive token rows are fetched by TMA tile copies (x_map), everything else by cp.async
   const bool use_tma = MH == 2 && p.gather_indx == nullptr;
@@ -125,12 +133,6 @@ gemm_tc_kernel(const GemmParams p, const int64_t grid_m_static, const __grid_con
     mbar_init(BAR_DRAIN, 1);
     *s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sbase + C::OFF_MISC),
-                 "r"((uint32_t)TMEM_COLS)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   if constexpr (MH == 2) {
     // tile prefix over experts: expert e has ceil(slice_sizes[e] / 256) tiles.  (Taken from the sizes, not from

@@ -264,10 +264,12 @@ typedef struct {
                                                       holds the rows of its own experts only); 0: M / E.  Steers the choice
                                                       of the block-scaled kernel, never a bound. */
   const int32_t* x_positions;                      /* optional, what gather_indx says the other way round: row t of x goes to */
-  const int16_t* x_experts; int x_k;               /* positions x_positions[t * x_k + j] (all of the M = rows_x * x_k positions
-                                                      occur once), rows of expert x_experts[t * x_k + j].  With it the pair
-                                                      kernel's token pass reads a row once instead of x_k times
-                                                      (x_k up to 512). */
+  const int16_t* x_experts; int x_k;               /* positions x_positions[t * x_k + j], rows of expert x_experts[t * x_k + j]
+                                                      (M = rows_x * x_k; every row of every expert occurs once, and an entry
+                                                      that is none, -1 say, is left out).  With it the token pass of the
+                                                      block-scaled kernels reads a row once instead of x_k times, and does not
+                                                      read gather_indx: the decode kernel's with any x_k, the pair kernel's
+                                                      with 2 to 512 and eight rows of x for each SM. */
 } MoeGemmArgs;
 int moe_grouped_gemm(const MoeGemmArgs* args_host, void* stream);
 /* Two products in a row: the same as moe_grouped_gemm of `first` and then of `second`, whose x is the first's y.  Where both run on

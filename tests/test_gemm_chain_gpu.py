@@ -178,18 +178,27 @@ def test_positions_of_a_row_beyond_a_block_of_shared_memory(k, device):
 class Passes:
     """One product over `rows` rows of x, each at k positions, to be called without and with the positions of every row."""
 
-    def __init__(self, rows, k, depth, block, device, e4m3=False):
+    def __init__(self, rows, k, depth, block, device, e4m3=False, dropped=False):
         g = torch.Generator(device=device).manual_seed(rows * k)
         x = torch.randn(rows, depth, device=device, generator=g).bfloat16()
         self.x = x.to(torch.float8_e4m3fn) if e4m3 else x
         lw = make_synthetic_layer(E, depth, 64, device, seed=3, block_scaled=True)
         experts = torch.randint(0, E, (rows * k,), device=device, generator=g).short()
         experts[: rows * k // 2] = 1                               # one expert of several blocks
+        lost = torch.rand(rows * k, device=device, generator=g) < 0.3 if dropped else torch.zeros(rows * k, dtype=torch.bool, device=device)
+        experts[lost] = E                                          # behind all others
         order = torch.argsort(experts, stable=True)
         positions = torch.empty(rows * k, dtype=torch.int32, device=device)
         positions[order] = torch.arange(rows * k, dtype=torch.int32, device=device)
         gather = (order // k).int()
-        ragged = make_ragged_tensor_metadata(torch.bincount(experts.long(), minlength=E).int(), rows * k)
+        ragged = make_ragged_tensor_metadata(torch.bincount(experts.long(), minlength=E)[:E].int(), rows * k)
+        self.live = int((~lost).sum())
+        if dropped:                                                # no expert, none of the experts there are, no position, one past the expert's rows
+            where = lost.nonzero().flatten()
+            experts[where[0::4]], positions[where[0::4]] = -1, -1
+            positions[where[1::4]] = 0
+            experts[where[2::4]], positions[where[2::4]] = 0, -1
+            experts[where[3::4]], positions[where[3::4]] = 0, ragged.slice_offs[1]
         self.status = torch.zeros(1, dtype=torch.int32, device=device)
         self.n, self.k, self.experts, self.positions = rows * k, k, experts, positions
         self.keep = [lw, gather, ragged]
@@ -235,3 +244,14 @@ def test_pair_tokens_in_parts_are_those_by_row(depth, device):
     by_position, by_row = p.run(False, b"gemm_mx_pair_kernel"), p.run(True, b"gemm_mx_pair_kernel")
     assert torch.equal(by_position.nan_to_num(7.0, 9.0, -9.0), by_row.nan_to_num(7.0, 9.0, -9.0))
     assert bool(torch.isfinite(by_row).all(1).sum() > 2000) and not bool(torch.isfinite(by_row).all())
+
+
+@pytest.mark.parametrize("rows, block, e4m3, kernel", [(40, 16, False, b"gemm_mx_kernel"), (40, 32, False, b"gemm_mx_kernel"), (40, 32, True, b"gemm_mx_kernel"),
+                                                       (1184, 256, False, b"gemm_mx_pair_kernel"), (1184, 256, True, b"gemm_mx_pair_kernel")])
+def test_entries_that_are_no_row_are_left_out(rows, block, e4m3, kernel, device):
+    """Dropped picks and picks of experts or positions that there are not, among those of every token: the rows that there are come out as by position."""
+    p = Passes(rows, 4, 512, block, device, e4m3, dropped=True)
+    if block == 256 and not e4m3:
+        p.x[7, 3] = float("inf")                                   # (a row that the token pass computes itself)
+    by_position, by_row = (p.run(by, kernel)[:p.live].nan_to_num(7.0, 9.0, -9.0) for by in (False, True))
+    assert torch.equal(by_position, by_row) and bool(by_row.abs().sum() > 0) and p.live < p.n

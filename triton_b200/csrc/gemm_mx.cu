@@ -284,26 +284,30 @@ struct PackRows {
   const int32_t* positions; const int16_t* experts;      // [rows_x, k]
   int k;
 };
-// chunk (at its k step) and lines of a term of pick `at` of [rows_x, k], and the row in its block
+// chunk (at its k step) and lines of a term of pick `at` of [rows_x, k], and the row in its block; no chunk where the pick is not a row of
+// one of the experts (dropped ones are -1)
 struct PickChunk { uint8_t* chunk; int r, lines; };
 __device__ __forceinline__ PickChunk pick_chunk(const GemmParams& p, const PackParams& a, const PackRows& w, int64_t at, int kt, bool split) {
-  const int e = w.experts[at], rr = w.positions[at] - p.slice_offs[e], j = rr / a.tb;
+  const int pick = w.experts[at], e = (unsigned)pick < (unsigned)p.E ? pick : 0, rows = p.slice_sizes[e];
+  const int rr = w.positions[at] - p.slice_offs[e], j = rr / a.tb;
   PickChunk c;
   c.r = rr - j * a.tb;
-  c.lines = !split ? a.n_mma : a.fit ? chunk_lines(min(a.tb, p.slice_sizes[e] - j * a.tb)) : a.tb;
-  c.chunk = a.out + ((int64_t)(p.block_offs[e] + j) * a.KT + kt) * a.chunk_bytes;
+  c.lines = !split ? a.n_mma : a.fit ? chunk_lines(min(a.tb, rows - j * a.tb)) : a.tb;
+  c.chunk = e == pick && rr >= 0 && rr < rows ? a.out + ((int64_t)(p.block_offs[e] + j) * a.KT + kt) * a.chunk_bytes : nullptr;
   return c;
 }
-// `store`(chunk, r, lines) for each pick of token t, by the whole warp
+// `store`(chunk, r, lines) for each pick of token t that has a chunk, by the whole warp
 template <typename F>
 __device__ __forceinline__ void each_pick(const GemmParams& p, const PackParams& a, const PackRows& w, int64_t t, int kt, bool split, F store) {
   const int lane = threadIdx.x & 31;
   for (int j0 = 0; j0 < w.k; j0 += 32) {
     PickChunk own{nullptr, 0, 0};
     if (j0 + lane < w.k) own = pick_chunk(p, a, w, t * w.k + j0 + lane, kt, split);
-    for (int j = 0; j < min(32, w.k - j0); ++j)
-      store((uint8_t*)__shfl_sync(0xFFFFFFFFu, (unsigned long long)own.chunk, j), __shfl_sync(0xFFFFFFFFu, own.r, j),
-            __shfl_sync(0xFFFFFFFFu, own.lines, j));
+    for (int j = 0; j < min(32, w.k - j0); ++j) {
+      uint8_t* chunk = (uint8_t*)__shfl_sync(0xFFFFFFFFu, (unsigned long long)own.chunk, j);
+      const int r = __shfl_sync(0xFFFFFFFFu, own.r, j), lines = __shfl_sync(0xFFFFFFFFu, own.lines, j);
+      if (chunk) store(chunk, r, lines);
+    }
   }
 }
 // FORM: terms of a token

@@ -311,12 +311,13 @@ __global__ void __launch_bounds__(256, 3) mx_pair_pack2_kernel(const __grid_cons
 // the prefill step 3144 -> 3081 us, with 8192 e4m3 rows 910 -> 903.
 constexpr int PACK_TOKENS = 8;
 constexpr int PACK_MAX_K = 512;                        // positions of a row: PACK_TOKENS x k words of 8 bytes in the 48 KB that need no opt-in
-// padded row of pick j of row t
+// padded row of pick j of row t; -1 where the pick is not a row of one of the experts (dropped ones are -1)
 __device__ __forceinline__ int64_t pick_prow(const GemmParams& p, const PairPackParams& a, int64_t t, int j, int& e, int64_t& m) {
-  e = a.experts[t * a.k + j];
+  const int pick = a.experts[t * a.k + j];
+  e = (unsigned)pick < (unsigned)p.E ? pick : 0;
   m = a.positions[t * a.k + j];
   const int off = p.slice_offs[e];
-  return padded_base(e, off) + (m - off);
+  return e == pick && m >= off && m < off + p.slice_sizes[e] ? padded_base(e, off) + (m - off) : -1;
 }
 template <bool TILED>
 __global__ void __launch_bounds__(256) mx_pair_pack2_rows_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ PairPackParams a) {
@@ -344,15 +345,17 @@ __global__ void __launch_bounds__(256) mx_pair_pack2_rows_kernel(const __grid_co
     if (!(quantise_group2<TILED>(raw, q) < BEYOND)) atomicOr(&s_beyond, 1u << r);
     for (int j = 0; j < a.k; ++j) {
       const int64_t prow = s_prow[r * a.k + j], line = token_line<2>(g >> 2, a.prows, prow, 0);
+      if (prow < 0) continue;
       store_group2(q, (int)prow & 7, g, a.xq + line * 128, 1024, a.xs + line * 4, 32);
     }
   }
   __syncthreads();
   const uint32_t beyond = s_beyond;
-  for (int i = threadIdx.x; i < n * a.k; i += 256) a.done[s_prow[i]] = (beyond >> (i / a.k)) & 1u;
+  for (int i = threadIdx.x; i < n * a.k; i += 256)
+    if (s_prow[i] >= 0) a.done[s_prow[i]] = (beyond >> (i / a.k)) & 1u;
   if (beyond)
     for (int i = 0; i < n * a.k; ++i)
-      if ((beyond >> (i / a.k)) & 1u) {
+      if (((beyond >> (i / a.k)) & 1u) && s_prow[i] >= 0) {
         int e; int64_t m;
         pick_prow(p, a, t0 + i / a.k, i % a.k, e, m);
         exact_position<TILED>(p, a, e, m, (const __nv_bfloat16*)a.x + (t0 + i / a.k) * a.ld_x);
@@ -374,6 +377,7 @@ __global__ void __launch_bounds__(256) mx_pair_pack1_rows_kernel(const __grid_co
     for (int j = 0; j < a.k; ++j) {
       int e; int64_t m;
       const int64_t prow = pick_prow(p, a, t, j, e, m);
+      if (prow < 0) continue;
       const uint32_t x7 = (uint32_t)prow & 7u;
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
@@ -387,6 +391,7 @@ __global__ void __launch_bounds__(256) mx_pair_pack1_rows_kernel(const __grid_co
     const int kt = i / a.k;
     int e; int64_t m;
     const int64_t prow = pick_prow(p, a, t, i - kt * a.k, e, m);
+    if (prow < 0) continue;
     uint32_t s = 0x7F7F7F7Fu;                                      // 1.0
     if (a.x_scale) {
       s = 0;

@@ -255,3 +255,15 @@ def test_entries_that_are_no_row_are_left_out(rows, block, e4m3, kernel, device)
         p.x[7, 3] = float("inf")                                   # (a row that the token pass computes itself)
     by_position, by_row = (p.run(by, kernel)[:p.live].nan_to_num(7.0, 9.0, -9.0) for by in (False, True))
     assert torch.equal(by_position, by_row) and bool(by_row.abs().sum() > 0) and p.live < p.n
+
+
+# blocks of four terms and of two
+@pytest.mark.parametrize("block", [16, 32, 64])
+@pytest.mark.parametrize("value", [float("inf"), float("nan"), 2.99e38, -3.38e38])
+def test_decode_tokens_by_row_with_the_largest_values(block, value, device):
+    p = Passes(40, 4, 512, block, device)
+    for j in range(8):
+        p.x[4 + j, 33 * j] = value                                 # at each of a lane's four places
+    p.x[20, 64:72] = value                                         # a lane that has no other
+    by_position, by_row = (p.run(by, b"gemm_mx_kernel").nan_to_num(7.0, 9.0, -9.0) for by in (False, True))
+    assert torch.equal(by_position, by_row)

@@ -225,6 +225,41 @@ def test_block_scaled_wide_dynamic_range_rows(kernel, device):
     assert oracle.rel_l2(ref, y) < 1e-3
 
 
+# each place of the four that a lane has, and of the eight; from 2.98e38 on a code times its scale is beyond the largest number
+@pytest.mark.parametrize("k", [0, 1, 2, 3, 5, 255])
+@pytest.mark.parametrize("value", [2.99e38, -3.38e38])
+@pytest.mark.parametrize("kernel, block_m, bound", [("mx-f4", 16, 5e-4), ("mx-f8", 32, 2e-5)])
+def test_block_scaled_values_near_the_largest(kernel, block_m, bound, value, k, device):
+    """A bf16 value that is nearly the largest there is keeps its terms wherever it stands (the bounds are those of the forms)."""
+    g = torch.Generator().manual_seed(k)
+    wq, ws, wdeq = quantised_weights(1, 256, 128, g)
+    x = torch.randn(12, 256, generator=g).bfloat16()
+    x[3, k] = value
+    sizes = torch.tensor([12], dtype=torch.int32)
+    y = run_mx(x, wq, ws, sizes, device, out_dtype=torch.float32, kernel=kernel, block_m=block_m).double()
+    ref = x.double() @ wdeq[0].double()
+    assert oracle.rel_l2(ref[3] * 1e-38, y[3] * 1e-38) < bound
+    rest = torch.arange(12) != 3
+    assert oracle.rel_l2(ref[rest], y[rest]) < 5e-4
+
+
+@pytest.mark.parametrize("k", [0, 1, 2, 3, 5, 255])
+@pytest.mark.parametrize("value", [float("inf"), -float("inf"), float("nan")])
+def test_four_terms_beside_a_value_that_is_not_finite(value, k, device):
+    """The other values of its group of 32 keep three terms and more, wherever it stands: seen where its own weights are zero."""
+    g = torch.Generator().manual_seed(k)
+    wq, ws, _ = quantised_weights(1, 256, 128, g)
+    low = wq[:, k // 2] & (0xF0 if k % 2 == 0 else 0x0F)             # the code of weight row k is zero for every output
+    wq[:, k // 2] = low
+    wdeq = oracle.dequant_weight_oracle(wq, ws)
+    x = torch.randn(12, 256, generator=g).bfloat16()
+    ref = x.double() @ wdeq[0].double()
+    x[3, k] = value
+    y = run_mx(x, wq, ws, torch.tensor([12], dtype=torch.int32), device, out_dtype=torch.float32, kernel="mx-f4", block_m=16).double()
+    # three terms leave 1e-3 of the group's eighth of the row
+    assert oracle.rel_l2(ref, y) < 5e-4 and oracle.rel_l2(ref[3], y[3]) < 1e-3
+
+
 def test_block_scaled_e4m3_output(device):
     """fc1 of the fp8 mode: e4m3 rows in, SwiGLU, e4m3 rows out (saturating round to nearest)."""
     g = torch.Generator().manual_seed(21)

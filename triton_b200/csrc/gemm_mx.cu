@@ -180,7 +180,7 @@ __device__ __forceinline__ void pack_two_terms(const float (&v)[4], TwoTerms& q)
   mx8_scale(amax, q.s_hi, s_hi, i_hi);
   const uint32_t h01 = f32x2_to_e4m3x2(v[0] * i_hi, v[1] * i_hi), h23 = f32x2_to_e4m3x2(v[2] * i_hi, v[3] * i_hi);
   const float2 f01 = e4m3x2_to_f32x2(h01), f23 = e4m3x2_to_f32x2(h23);
-  float rs[4] = {v[0] - f01.x * s_hi, v[1] - f01.y * s_hi, v[2] - f23.x * s_hi, v[3] - f23.y * s_hi};
+  float rs[4] = {left_over(v[0], f01.x, s_hi), left_over(v[1], f01.y, s_hi), left_over(v[2], f23.x, s_hi), left_over(v[3], f23.y, s_hi)};
   float rmax = fmaxf(fmaxf(fabsf(rs[0]), fabsf(rs[1])), fmaxf(fabsf(rs[2]), fabsf(rs[3])));
 #pragma unroll
   for (int o = 1; o <= 4; o <<= 1) rmax = fmaxf(rmax, __shfl_xor_sync(0xFFFFFFFFu, rmax, o));

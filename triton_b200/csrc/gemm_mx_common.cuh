@@ -54,16 +54,20 @@ __device__ __forceinline__ void mx4_scale(float amax, uint32_t& sb, float& scale
   scale = __uint_as_float(sb << 23);
   inv = __uint_as_float((254u - sb) << 23);
 }
+// What a term leaves of a value, in one rounding.  A product by itself is past the largest number where the group's maximum is near it (2.98e38), and
+// left to the compiler some of a lane's values got one and others not.
+__device__ __forceinline__ float left_over(float v, float code, float scale) { return fmaf(-code, scale, v); }
 // Term t of N values of a 32-group (v: what the terms before left over, and leaves); its maximum comes from `all`.  -> scale byte
+// A value that is not finite has its code in the first term and leaves nothing, so that the others keep the rest of their terms.
 template <int N, typename F>
 __device__ __forceinline__ uint32_t e2m1_term(int t, float (&v)[N], const bool (&nan)[N], uint32_t& codes, F all) {
-  // (NaN ranks above Inf where four neighbouring values are NaN, and is caught below)
+  // (first term: NaN ranks above Inf where four neighbouring values are NaN, and is caught below)
   uint32_t top = 0;
 #pragma unroll
   for (int i = 0; i < N; i += 4)
     top = max(top, __float_as_uint(fmaxf(fmaxf(fabsf(v[i]), fabsf(v[i + 1])), fmaxf(fabsf(v[i + 2]), fabsf(v[i + 3])))));
   float amax = __uint_as_float(all(top));
-  if (!(amax < 3.0e38f)) amax = t == 0 ? 3.0e38f : 0.0f;           // Inf / NaN in the group: keep the scales finite
+  if (t == 0 && !(amax < 3.0e38f)) amax = 3.0e38f;                 // Inf / NaN in the group: keep the scale finite
   uint32_t sb; float s, inv;
   mx4_scale(amax, sb, s, inv);
   codes = 0;
@@ -72,8 +76,12 @@ __device__ __forceinline__ uint32_t e2m1_term(int t, float (&v)[N], const bool (
     const uint32_t c = f32x2_to_e2m1x2(nan[i] ? 0.0f : v[i] * inv, nan[i + 1] ? 0.0f : v[i + 1] * inv);
     codes |= c << (4 * i);
     const float2 f = e2m1x2_to_f32x2(c);
-    v[i] -= f.x * s;
-    v[i + 1] -= f.y * s;
+    v[i] = left_over(v[i], f.x, s);
+    v[i + 1] = left_over(v[i + 1], f.y, s);
+    if (t == 0) {
+      if (!(fabsf(v[i]) < INFINITY)) v[i] = 0.0f;
+      if (!(fabsf(v[i + 1]) < INFINITY)) v[i + 1] = 0.0f;
+    }
   }
   return sb;
 }

@@ -64,8 +64,8 @@ __device__ __forceinline__ void two_terms(float (&v)[N], F all, uint32_t (&h)[N 
   for (int i = 0; i < N / 2; ++i) {
     const uint32_t c = f32x2_to_e4m3x2(v[2 * i] * i_hi, v[2 * i + 1] * i_hi);
     const float2 f = e4m3x2_to_f32x2(c);
-    v[2 * i] -= f.x * s_hi;
-    v[2 * i + 1] -= f.y * s_hi;
+    v[2 * i] = left_over(v[2 * i], f.x, s_hi);
+    v[2 * i + 1] = left_over(v[2 * i + 1], f.y, s_hi);
     rm = fmaxf(rm, fmaxf(fabsf(v[2 * i]), fabsf(v[2 * i + 1])));
     h[i >> 1] = (i & 1) ? (h[i >> 1] | (c << 16)) : c;
   }

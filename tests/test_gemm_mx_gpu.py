@@ -572,6 +572,22 @@ def test_pair_kernel_values_beyond_two_terms(tiled, sizes, mode, device):
         assert (got.double() - ref)[keep].norm() <= (2.0 ** -8 if mode == "bf16 out" else 1e-4) * ref[keep].norm() + 1e-6
 
 
+@pytest.mark.parametrize("per", [20, 24])
+def test_infinities_in_products_of_twenty_rows_per_expert(per, device):
+    """By the library's own choice of kernel: a token with an infinity gives infinities with the weight's sign, NaN where the weight is zero."""
+    g = torch.Generator().manual_seed(per)
+    E, K, N = 40, 448, 1024                                          # two tiles per expert: more than one round of the pairs
+    wq, ws, wdeq = quantised_weights(E, K, N, g)
+    x = torch.randn(E * per, K, generator=g).bfloat16()
+    x[3, 5], x[7 * per, 440] = float("inf"), -float("inf")
+    y = run_mx(x, wq, ws, torch.full((E,), per, dtype=torch.int32), device)
+    for m, k in ((3, 5), (7 * per, 440)):
+        w = wdeq[m // per][k].float() * x[m, k].float().sign()
+        want = torch.where(w == 0, torch.nan, w * float("inf"))
+        assert torch.equal(y[m].float().nan_to_num(7.0), want.nan_to_num(7.0))
+    assert int(torch.isfinite(y).all(1).sum()) == E * per - 2
+
+
 @pytest.mark.parametrize("form", ["tb16", "tb32", "tb64", "tb32 wide", "tb64 wide", "pair", "pair default tiles", "mixed"])
 @pytest.mark.parametrize("T, ff", [(3, 320), (70, 736), (200, 320), (1300, 320)])
 @pytest.mark.parametrize("kind", ["bf16", "e4m3", "no limit", "inf"])

@@ -418,6 +418,14 @@ def test_kernel_of_a_shard_goes_by_its_own_rows(monkeypatch):
     assert moe._local_metadata(None, None, 1, 16).expected_slice_size == 1
 
 
+@pytest.mark.parametrize("E, K, N", [(32, 2880, 5760), (32, 2880, 2880), (64, 512, 1024), (64, 1440, 2880), (128, 2880, 5760)])
+def test_infinities_are_kept_from_twenty_rows_per_expert_on(E, K, N):
+    """Large bf16 products run from there on the kernel whose token pass holds rows with an infinity, however many rounds its tiles take."""
+    from triton_b200 import _lib
+    kernel = lambda per: _lib.host().gemm_kernel(_lib.MOE_W_MX4_B200MX, E, K, N, E * per, torch.bfloat16, torch.bfloat16, (0, 0, 0, 0))
+    assert kernel(19) == "gemm_mx_kernel" and {kernel(per) for per in range(20, 48)} == {"gemm_mx_pair_kernel"}
+
+
 def test_small_block_scaled_products_leave_the_decode_kernel_after_one_wave():
     """Below 2^24 elements the decode kernel keeps a product while its 32 x 128 tiles fit the SMs (148 of them where no GPU says
     otherwise): 32 experts of 512 x 512 up to some 16 rows per expert, 8 experts of 2048 x 512 to well beyond 96."""

@@ -993,11 +993,12 @@ int launch_mx_pair_ty(const GemmParams& p, const PairParams& q, const MoeGemmArg
 // experts of 1024 rows: 72 here, 57 there; 16 experts 132 and 109; without the activation 64 and 61, 114 and 116).
 // (Both kernels lose up to a third of a wave, so no line in these sizes is right everywhere: over 500 products of 48 to 1024 rows
 // this one is 2 % from the better kernel on average, most of it at 100-400 balanced rows of K <= 1024.)
-// Block-scaled tiles (against the decode forms of gemm_mx.cu), tile_m = 256 asks for it.  What an expert has decides, not the mean, so the lines lie
-// between even routing and logits biased by N(0, 1) per expert, under which some experts have several blocks of the decode form.  bf16 tokens from 20
-// rows on, but from 25 where the product's tiles here are more than one and up to eight rounds of the pairs: a last round partly filled costs a good
-// part of the whole then.  e4m3 tokens, one term, from 16 (up to eight rounds even routing would stay ahead on the decode form to 28 and more).  Whole
-// layer steps, four picks (decode form, this one; even, then biased):
+// Block-scaled tiles (against the decode forms of gemm_mx.cu), tile_m = 256 asks for it.  bf16 tokens from 20 rows per expert on, e4m3 tokens from 16.
+// What an expert has decides the time, not the mean: under logits biased by N(0, 1) per expert some experts have several blocks of the decode form.  The
+// lines were drawn before the decode form's tiles of two blocks, with which it is ahead of this one to some 25 rows where the product's tiles here
+// are between one and eight rounds of the pairs (a last round partly filled costs a good part of the whole then).  bf16 products stay here all the same: a token
+// with an infinity gives infinities here, and large finite values there.  For e4m3 tokens the line has not been moved.  Whole layer steps,
+// four picks (decode form, this one; even, then biased):
 //   bf16   128 experts of 2880 x 5760:  20 rows 429, 452; 377, 357.  24 rows 449, 437; 436, 391
 //          32 experts of the same:  20 rows 109, 131; 123, 129.  25 rows 118, 134; 133, 131.  30 rows 135, 138; 141, 136.  40 rows 172, 143; 164, 149
 //          64 experts of 1440 x 2880:  20 rows 86, 96; 81, 88.  25 rows 84, 95; 94, 94.  32 rows 101, 98; 102, 97
@@ -1026,10 +1027,7 @@ bool moe_gemm_mx_pair_wanted(const MoeGemmArgs& a) {
   if (a.tile_m == 256) return true;
   if (a.tile_m != 0 || a.kernel == MOE_GEMM_MX_F8) return false;
   if (a.x_dtype != MOE_BF16) return per >= 16;
-  if (load >= (1 << 24)) {
-    const int64_t tiles = experts * cdiv64(a.N, 512), pairs = moe_sm_count() / 2;
-    return per >= (tiles > pairs && tiles <= 8 * pairs ? 25 : 20);
-  }
+  if (load >= (1 << 24)) return per >= 20;
   return experts * (per + 16) / 32 * cdiv64(a.N, 128) > moe_sm_count();
 }
 

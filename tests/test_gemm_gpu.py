@@ -345,6 +345,42 @@ def test_graphed_layer_routes_the_logits_of_its_own_call(E, k, device):
     assert all(torch.equal(a, b) for a, b in zip(want, got)) and not torch.equal(want[0], want[1])
 
 
+def test_graphed_layer_on_several_streams(layer_20b, device):
+    """Calls from streams that wait for nothing of one another follow one another on the step's buffers: each result is that of its own inputs."""
+    from triton_b200.moe import GraphedMoeLayer, moe_layer_forward
+    lw, _, _ = layer_20b
+    T = 64
+    graphed = GraphedMoeLayer(lw, 4, T, 2880, 32, device)
+    g = torch.Generator(device=device).manual_seed(1)
+    inputs = [(torch.randn(T, 2880, device=device, generator=g).bfloat16(), torch.randn(T, 32, device=device, generator=g)) for _ in range(12)]
+    want = [moe_layer_forward(x, logits, lw, 4) for x, logits in inputs]
+    streams = [torch.cuda.Stream(device=device) for _ in range(3)]
+    torch.cuda.synchronize()
+    got = []
+    for i, (x, logits) in enumerate(inputs):
+        with torch.cuda.stream(streams[i % 3]):
+            got.append(graphed(x, logits))
+    torch.cuda.synchronize()
+    tb.matmul_check_status()
+    assert all(torch.equal(a, b) for a, b in zip(want, got))
+
+
+def test_graphed_layer_is_refused_inside_a_capture(layer_20b, device):
+    """A replay cannot be part of another capture: the call says so, and the layer goes on working."""
+    from triton_b200.moe import GraphedMoeLayer, moe_layer_forward
+    lw, _, _ = layer_20b
+    graphed = GraphedMoeLayer(lw, 4, 5, 2880, 32, device)
+    g = torch.Generator(device=device).manual_seed(2)
+    x, logits = torch.randn(5, 2880, device=device, generator=g).bfloat16(), torch.randn(5, 32, device=device, generator=g)
+    before = graphed(x, logits)
+    with pytest.raises(RuntimeError):
+        with torch.cuda.graph(torch.cuda.CUDAGraph()):
+            graphed(x, logits)
+    torch.cuda.synchronize()
+    assert torch.equal(graphed(x, logits), before) and torch.equal(before, moe_layer_forward(x, logits, lw, 4))
+    tb.matmul_check_status()
+
+
 def test_host_streaming_layer(layer_20b, device):
     """Steps fed from and returned to pinned host memory through the three-stream pipeline equal the eager layer."""
     from triton_b200.moe import HostStreamingLayer, moe_layer_forward

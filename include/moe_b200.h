@@ -253,8 +253,8 @@ typedef struct {
      the library into two e4m3 terms (kind::mxf8f6f4) or, for token blocks of 16 rows, four e2m1 terms (kind::mxf4);
      MOE_GEMM_MX_F8 / MOE_GEMM_MX_F4 pin the form.  mx_workspace holds the re-laid-out token blocks:
      moe_gemm_mx_workspace_bytes(args) bytes, 1024-byte aligned.  For this kernel tile_m is the token block
-     (0 auto, 16, 32, 64, 128; 256 = the kernel on pairs of SMs) and tile_n 128 / 384 pins one / three weight blocks
-     per CTA tile.  bf16 tokens against the default tiles (MOE_W_MX4_B200) run on the pair kernel too where that is
+     (0 auto, 16, 32, 64, 128; 256 = the kernel on pairs of SMs) and tile_n 128 / 256 / 384 pins one / two / three weight
+     blocks per CTA tile (256: not with four terms).  bf16 tokens against the default tiles (MOE_W_MX4_B200) run on the pair kernel too where that is
      faster and mx_workspace is given (the size is 0 where it is not); MOE_GEMM_MX pins it.                      */
   const uint8_t* x_scale; int64_t ld_x_scale;
   void* mx_workspace; int64_t mx_workspace_bytes;

@@ -84,7 +84,7 @@ def dequant_act(x8, a_scale):
 
 
 @pytest.mark.parametrize("stage", ["unit-scales", "weight-scales", "act-scales"])
-@pytest.mark.parametrize("block_n", [128, 384])
+@pytest.mark.parametrize("block_n", [128, 256, 384])
 def test_block_scaled_dense_fp8_exact_products(stage, block_n, device):
     """One expert, e4m3 activations: every product is exact in the tensor core and the sum is fp32, so the result
     must match the fp32 oracle closely.  The three stages separate the value path (unit scales), the weight scales
@@ -208,6 +208,40 @@ def test_block_scaled_token_block_sizes(block_m, kernel, device):
     ref = oracle.matmul_oracle(x.float(), wdeq, None, sizes, out_dtype=torch.float32).bfloat16()
     oracle.assert_close_oracle(ref, y, maxtol=MAXTOL_MX4, rmstol=None, what="block-scaled gemm")
     assert oracle.rel_l2(ref, y) < 1e-2
+
+
+@pytest.mark.parametrize("acts, block_m", [("bf16", 16), ("bf16", 32), ("bf16", 64), ("fp8", 32), ("mxfp8", 16), ("mxfp8", 64), ("fp8", 128)])
+@pytest.mark.parametrize("K, N, mode", [(96, 640, "plain"), (320, 129, "plain"), (640, 514, "scatter"), (416, 640, "swiglu"), (160, 768, "swiglu"), (128, 256, "e4m3")])
+def test_block_scaled_tiles_of_two_weight_blocks(K, N, mode, acts, block_m, device):
+    """The tiles that products of byte-expanded operands choose: odd and even counts of weight blocks, a last block of one row, widths without
+    vector stores, experts of several token blocks, every output type.  fp32 outputs: products are exact and only the order of the sums differs."""
+    g = torch.Generator().manual_seed(K + N + block_m)
+    sizes = torch.tensor([70, 1, 0, 33, 16, 150], dtype=torch.int32)
+    E, M = 6, int(sizes.sum())
+    wq, ws, wdeq = quantised_weights(E, K, N, g)
+    x = torch.randn(M, K, generator=g).bfloat16()
+    a_scale = None
+    if acts != "bf16":
+        x = x.to(torch.float8_e4m3fn)
+        if acts == "mxfp8":
+            a_scale = torch.randint(122, 131, (M, K // 32), generator=g, dtype=torch.uint8)
+    bias = torch.randn(E, N, generator=g) * 0.1
+    scatter, gammas = (torch.randperm(M, generator=g).int(), torch.rand(M, generator=g)) if mode == "scatter" else (None, None)
+    act = (1.702, 7.0) if mode == "swiglu" else None
+    out_dtype = torch.float8_e4m3fn if mode == "e4m3" else torch.float32
+    y = run_mx(x, wq, ws, sizes, device, a_scale=a_scale, bias=bias, scatter=scatter, gammas=gammas, act=act, out_dtype=out_dtype,
+               kernel="mx-f8", block_m=block_m, block_n=256)
+    ref = oracle.matmul_oracle(x.float() if acts == "bf16" else dequant_act(x, a_scale), wdeq, bias, sizes, gammas=gammas, out_dtype=torch.float32)
+    if act:
+        ref = oracle.swiglu_oracle(ref, *act)
+    if scatter is not None:
+        ref = torch.zeros_like(ref).index_copy_(0, scatter.long(), ref)
+    if mode == "e4m3":                                               # one step of e4m3 where the sums differ at a rounding boundary
+        ref8 = ref.to(torch.float8_e4m3fn).float()
+        diff = (y.float() - ref8).abs()
+        assert (diff <= ref8.abs().clamp_min(2.0 ** -6) * 0.125).all() and (diff > 0).float().mean() < 0.02
+    else:
+        assert oracle.rel_l2(ref, y) < 2e-5
 
 
 @pytest.mark.parametrize("kernel", ["mx-f8", "mx-f4"])
@@ -588,12 +622,12 @@ def test_infinities_in_products_of_twenty_rows_per_expert(per, device):
     assert int(torch.isfinite(y).all(1).sum()) == E * per - 2
 
 
-@pytest.mark.parametrize("form", ["tb16", "tb32", "tb64", "tb32 wide", "tb64 wide", "pair", "pair default tiles", "mixed"])
+@pytest.mark.parametrize("form", ["tb16", "tb32", "tb64", "tb32 wide", "tb64 wide", "tb32 two", "tb64 two", "pair", "pair default tiles", "mixed"])
 @pytest.mark.parametrize("T, ff", [(3, 320), (70, 736), (200, 320), (1300, 320)])
 @pytest.mark.parametrize("kind", ["bf16", "e4m3", "no limit", "inf"])
 def test_rows_handed_over_as_tokens(form, T, ff, kind, device):
     """fc1's rows written as fc2's tokens: the bits of the two products run apart.  Odd and even counts of weight blocks (5 and 11.5),
-    k steps that are partly past K, one to many token blocks per expert, tiles of one and of three weight
+    k steps that are partly past K, one to many token blocks per expert, tiles of one, two and three weight
     blocks (there a chunk has the lines that its block's rows need), both kernels.  Without a limit on the activation the rows go
     through y; a token with an infinity is computed beside the pair kernel and joins the others there.  (1300 tokens: the pair kernel's
     token pass by token, in the operators by position.)"""
@@ -601,7 +635,7 @@ def test_rows_handed_over_as_tokens(form, T, ff, kind, device):
     from triton_b200.moe import _NoTimer, moe_layer_forward
     from triton_b200.testing import make_synthetic_layer
     E, k, d = 6, 2, 512
-    if kind == "e4m3" and form in ("tb64", "tb64 wide", "pair default tiles"):
+    if kind == "e4m3" and form in ("tb64", "tb64 wide", "tb64 two", "pair default tiles"):
         pytest.skip("the same paths as with other blocks; e4m3 tokens have no kernel on the default tiles")
     lw = make_synthetic_layer(E, d, ff, device, seed=3, block_scaled=form != "pair default tiles")
     lw.limit = None if kind == "no limit" else 7.0
@@ -612,7 +646,8 @@ def test_rows_handed_over_as_tokens(form, T, ff, kind, device):
     x = x.to(torch.float8_e4m3fn) if kind == "e4m3" else x
     logits = torch.randn(T, E, device=device, generator=g) + torch.randn(E, device=device, generator=g)
     constraint = {"tb16": {"block_m": 16}, "tb32": {"block_m": 32}, "tb64": {"block_m": 64}, "tb32 wide": {"block_m": 32, "block_n": 384},
-                  "tb64 wide": {"block_m": 64, "block_n": 384}, "pair": {"block_m": 256},
+                  "tb64 wide": {"block_m": 64, "block_n": 384}, "tb32 two": {"block_m": 32, "block_n": 256},
+                  "tb64 two": {"block_m": 64, "block_n": 256}, "pair": {"block_m": 256},
                   "pair default tiles": {"kernel": "mx"}, "mixed": {}}[form]
     lw.block_scaled_max_rows_per_expert = 10 ** 6
     with tb.scoped_opt_flags_constraints(constraint):

@@ -879,7 +879,8 @@ MxPlan mx_plan(const MoeGemmArgs& a) {
   // tokens of 128 experts 248 -> 238 and 349 -> 326 us per step, 150 tokens of 32 experts of 4096 x 4096 212 -> 193; e4m3, 64 and 100 tokens
   // of 32 experts 99.9 -> 92.5 and 103.2 -> 95.6).
   const int wide = pl.f4 ? 3 : 2;
-  pl.mb = a.tile_n == 128 ? 1 : a.tile_n == 384 ? 3 : pl.grid_m * cdiv64(pl.NB, wide) >= (int64_t)moe_sm_count() ? wide : 1;
+  // (Three of a byte per value are built for the constraint that asks for them alone.)
+  pl.mb = a.tile_n == 128 ? 1 : a.tile_n == 384 ? 3 : a.tile_n == 256 && !pl.f4 ? 2 : pl.grid_m * cdiv64(pl.NB, wide) >= (int64_t)moe_sm_count() ? wide : 1;
   // too few tiles for three blocks each, four-term form: single weight blocks, three k steps of one block per stage
   // (a stage of one 8 KB tile does not keep a copy pipeline busy)
   pl.km = (pl.f4 && tb == 16 && pl.mb == 1 && a.tile_n == 0 && pl.KT >= 3) ? 1 : 0;

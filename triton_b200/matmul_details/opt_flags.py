@@ -73,7 +73,7 @@ def resolve_tile_m() -> int:
 
 def resolve_tile_n() -> int:
     """`block_n` constraint -> weight rows per tile (0 = heuristic): 128 / 256 for the bf16 tensor-core kernel,
-    128 / 384 for the block-scaled kernel."""
+    128 / 256 / 384 for the block-scaled kernel (256: where a value takes a byte of shared memory, else its own choice)."""
     bn = get_opt_flags_constraints().get("block_n")
     return bn if bn in (128, 256, 384) else 0
 

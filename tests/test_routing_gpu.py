@@ -252,6 +252,20 @@ def test_routing_in_one_cluster(T, E, k, device):
     assert torch.equal(gather.cpu().int(), (col // k).int())
 
 
+@pytest.mark.parametrize("E, k, one", [(64, 1, (257, 1024)), (128, 2, (257, 1024)), (256, 1, (257, 1024)), (8, 1, (1025, 1536)), (8, 2, (1025, 1536)),
+                                       (32, 2, (257, 896)), (128, 4, (257, 896)), (256, 8, (257, 1536))])
+def test_lists_that_one_cluster_routes(E, k, one, device):
+    """Launches of a step on either side of the lines between one cluster and two launches."""
+    lib = _lib.load()
+    for T, n in ((one[0], 1), (one[1], 1), (one[1] + 1, 2)):
+        logits = torch.randn(T, E, device=device)
+        before = lib.moe_launch_count()
+        sp = routing(logits, k)[3]
+        assert lib.moe_launch_count() - before == n, (T, n)
+        vals, indx, bm = oracle.topk_oracle(logits.cpu(), k, True)
+        assert torch.equal(sp.indx.cpu().int(), indx.int())
+
+
 @pytest.mark.parametrize("T, E, k", [(257, 20, 3), (2049, 128, 4), (8193, 200, 6), (8300, 256, 8), (8321, 256, 8), (18176, 32, 1), (18305, 32, 1), (300, 256, 40)])
 def test_routing_in_two_launches(T, E, k, device):
     """Either side of where the blocks that rank also add up the counts (their number and the length of a block's list decide), k that the quad

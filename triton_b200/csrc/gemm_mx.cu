@@ -875,9 +875,9 @@ MxPlan mx_plan(const MoeGemmArgs& a) {
   pl.grid_m = a.slice_sizes ? blocks_bound(a.E, a.M, tb) : cdiv64(a.M, tb);
   // several weight blocks per CTA tile share one token tile (fewer token bytes per weight byte); one block when there
   // would be too few tiles to fill the SMs.  Three of packed weights; two where a value takes a byte of shared memory, of which the ring holds five stages
-  // where it takes three of three: what bounds those forms is the weights in flight per SM, 82 KB against 74, less the stage at work (bf16, 300 and 500
-  // tokens of 128 experts 248 -> 238 and 349 -> 326 us per step, 150 tokens of 32 experts of 4096 x 4096 212 -> 193; e4m3, 64 and 100 tokens
-  // of 32 experts 99.9 -> 92.5 and 103.2 -> 95.6).
+  // where it takes three of three: what bounds those forms is the weights in flight per SM, 82 KB against 74, less the stage at work.  us per step at
+  // boost clocks and (second pair) in a long run under the power limit: bf16, 300 tokens of 128 experts 252 -> 243, 279 -> 278; 500 tokens 348 -> 314, 374 ->
+  // 358; 150 tokens of 32 experts of 4096 x 4096 218 -> 202, 230 -> 223; e4m3, 100 tokens of 32 experts 107 -> 97, 103 -> 97.
   const int wide = pl.f4 ? 3 : 2;
   // (Three of a byte per value are built for the constraint that asks for them alone.)
   pl.mb = a.tile_n == 128 ? 1 : a.tile_n == 384 ? 3 : a.tile_n == 256 && !pl.f4 ? 2 : pl.grid_m * cdiv64(pl.NB, wide) >= (int64_t)moe_sm_count() ? wide : 1;
@@ -1024,8 +1024,9 @@ int moe_gemm_mx_launch(const GemmParams& p_in, const MoeGemmArgs& a, const Token
   q.KT = pl.KT; q.NB = pl.NB; q.stages = pl.stages; q.stage_bytes = pl.stage_bytes; q.acc_bufs = pl.acc_bufs;
   q.grid_m = pl.grid_m;
   // Up to a third of a block of rows per expert, where few experts have several blocks.  What streams through L2 otherwise pushes out code, tokens
-  // and rows: steps of 1, 4, 16 and 300 tokens 36.8 -> 33.0, 58.3 -> 55.3, 71.8 -> 68.7 and 265 -> 253 us; with half a block per expert (64 tokens,
-  // 32 experts) the other blocks of an expert would miss what the first has read, 100.5 -> 103.5.
+  // and rows: us per step of 128 experts, 1 token 34.6 -> 32.7, 4 tokens 56.3 -> 54.0, 64 tokens 161.9 -> 158.4, 300 tokens 285 -> 278 (252 -> 243 at boost
+  // clocks), 16 tokens of 32 experts 73.1 -> 69.6; with half a block per expert (64 tokens, 32 experts) the other blocks of an expert would miss
+  // what the first has read, 100.5 -> 103.5.
   q.once = 3 * a.M <= (int64_t)pl.tb * (a.slice_sizes ? a.E : 1);
   q.hint_m = (uint32_t)(a.slice_sizes && a.ld_block_sched < pl.grid_m ? a.ld_block_sched : pl.grid_m);
   MxMaps w_map;

@@ -1305,14 +1305,22 @@ extern "C" __attribute__((visibility("default"))) size_t moe_route_workspace(int
 //   32 experts, k = 4:   64 tokens 7.4, 6.8;  96  6.3, 7.2;  256  8.8, 9.8, 7.9;  300  -, 7.9, 8.0, 11.9;  1024  -, 9.7, 8.4;  2048  -, 11.3, 8.6, 12.8
 //   8 experts, k = 2:    64 tokens 5.3, 6.0;  256  5.2, 7.6, 6.6;  300  -, 6.5, 6.7, 12.5;  2048  -, 7.4, 7.2, 12.9
 //   256 experts, k = 16: 64 tokens 26.8, 11.7, 36.7;  768  -, 29.7, 39.9;  1536  -, 44.2, 40.5;  2048  -, 56.1, 41.5
+// and (cluster, two launches) of short lists:
+//   k = 1:  8 experts 900 tokens 6.8, 6.7;  1280  6.2, 7.0;  1536  6.3, 6.8;  64 experts 1024  7.2, 7.6;  1280  7.6, 7.6;  128 experts 1024  8.1, 9.1;
+//           1280  9.0, 8.8;  256 experts 1024  9.8, 11.4;  1280  12.0, 11.5
+//   k = 2:  8 experts 900 tokens 7.3, 7.1;  1280  6.6, 7.1;  1536  6.8, 7.1;  32 experts 900  7.6, 7.2;  128 experts 1024  9.4, 9.8;  1280  10.0, 9.4;
+//           256 experts 1024  11.7, 12.2;  1280  13.0, 12.3
 // The small form repeats the whole selection in five blocks, the cluster has an eighth of it in each of eight and two barriers; past 768 to 1024
 // tokens eight SMs are fewer than the selection wants, and two launches are ahead.  With long lists (E k > 1024) the finish of those takes
-// longest and the line lies at 1536.
+// longest and the line lies at 1536.  Lists of one or two picks leave the cluster little to sort: from 64 experts on its line lies at 1024, and the shortest
+// (E k <= 16) go back to it where it has four lanes per token, from 1025 to 1536.  (From 129 to 256 tokens the rule does not follow the table: two launches
+// would be up to 1.8 us ahead with four picks and more, and the cluster's 32 lanes per token take longer there than 16 do at 300.)
 enum { ROUTE_SMALL, ROUTE_CLUSTER, ROUTE_LAUNCHES };
 static int route_form(int64_t T, int E, int k) {
   if (!(k == 1 || k == 2 || k == 4 || k == 8 || k == 16)) return ROUTE_LAUNCHES;
   if (T <= kRouteSmallTokens) return T >= 24 && k >= 4 && (E * k >= 512 || T <= 64) ? ROUTE_CLUSTER : ROUTE_SMALL;
-  return T <= (E * k <= 1024 ? 896 : 1536) ? ROUTE_CLUSTER : ROUTE_LAUNCHES;
+  if (E * k <= 16 && T > 1024) return T <= 1536 ? ROUTE_CLUSTER : ROUTE_LAUNCHES;
+  return T <= (E * k > 1024 ? 1536 : k <= 2 && E >= 64 ? 1024 : 896) ? ROUTE_CLUSTER : ROUTE_LAUNCHES;
 }
 
 static int route_launch(

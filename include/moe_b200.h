@@ -86,7 +86,7 @@ int moe_bitmatrix_metadata(const int16_t* indx, int64_t ld_indx, int64_t T, int 
                            const int32_t* n_rows_dev, int32_t* col_sum, int32_t* col_sorted,
                            int32_t* row_sorted, void* workspace, size_t workspace_bytes, void* stream);
 
-/* The whole routing step of a layer in one launch (up to some 900 tokens) to three: moe_topk_fwd +
+/* The whole routing step of a layer in one launch (up to 896 to 2048 tokens) to three: moe_topk_fwd +
  * moe_bitmatrix_metadata + moe_ragged_metadata (topk.py:106-141 -> tensor.py:202-209 -> ragged_tensor.py:183-210 of the
  * reference, what its test helper `routing` composes, tests/test_distributed.py:203-210) with the expert histogram taken
  * in the top-k pass and the ragged metadata built beside the sort.  Every one of the T rows is valid (no device-side row

@@ -252,18 +252,35 @@ def test_routing_in_one_cluster(T, E, k, device):
     assert torch.equal(gather.cpu().int(), (col // k).int())
 
 
-@pytest.mark.parametrize("E, k, one", [(64, 1, (257, 1024)), (128, 2, (257, 1024)), (256, 1, (257, 1024)), (8, 1, (1025, 1536)), (8, 2, (1025, 1536)),
-                                       (32, 2, (257, 896)), (128, 4, (257, 896)), (256, 8, (257, 1536))])
-def test_lists_that_one_cluster_routes(E, k, one, device):
-    """Launches of a step on either side of the lines between one cluster and two launches."""
+@pytest.mark.parametrize("E, k, line", [(8, 1, 2048), (64, 2, 2048), (32, 4, 2048), (16, 8, 2048), (256, 1, 1536), (256, 2, 1536), (128, 4, 1536), (32, 8, 1536),
+                                        (200, 4, 896), (64, 8, 896), (16, 16, 896), (256, 8, 1536)])
+def test_lists_that_one_cluster_routes(E, k, line, device):
+    """Launches of a call by itself on either side of the line between one cluster and two launches."""
     lib = _lib.load()
-    for T, n in ((one[0], 1), (one[1], 1), (one[1] + 1, 2)):
+    for T, n in ((257, 1), (line, 1), (line + 1, 2)):
         logits = torch.randn(T, E, device=device)
         before = lib.moe_launch_count()
         sp = routing(logits, k)[3]
         assert lib.moe_launch_count() - before == n, (T, n)
         vals, indx, bm = oracle.topk_oracle(logits.cpu(), k, True)
         assert torch.equal(sp.indx.cpu().int(), indx.int())
+
+
+@pytest.mark.parametrize("E, k, one, two", [(64, 1, 1024, 1025), (128, 2, 1024, 1025), (256, 1, 1024, 1025), (8, 1, 896, 897), (8, 2, 1025, 1024), (8, 1, 1536, 1537),
+                                            (32, 2, 896, 897), (128, 4, 896, 897), (16, 8, 896, 897), (256, 8, 1536, 1537)])
+def test_lists_that_one_cluster_routes_in_a_step(E, k, one, two, device):
+    """The same of a layer step: one launch fewer with `one` tokens than with `two`, and the rows of the smaller step with either."""
+    from triton_b200.moe import moe_layer_forward
+    from triton_b200.testing import make_synthetic_layer
+    lib, lw = _lib.load(), make_synthetic_layer(E, 256, 128, device, seed=1, chunk=E, block_scaled=True)
+    x, logits = torch.randn(max(one, two), 256, device=device).bfloat16(), torch.randn(max(one, two), E, device=device)
+    count, rows = [], []
+    for T in (one, two):
+        before = lib.moe_launch_count()
+        rows.append(moe_layer_forward(x[:T], logits[:T], lw, k)[: min(one, two)])
+        count.append(lib.moe_launch_count() - before)
+    assert count[1] - count[0] == 1
+    torch.testing.assert_close(rows[0], rows[1], rtol=2 ** -6, atol=1e-3)
 
 
 @pytest.mark.parametrize("T, E, k", [(257, 20, 3), (2049, 128, 4), (8193, 200, 6), (8300, 256, 8), (8321, 256, 8), (18176, 32, 1), (18305, 32, 1), (300, 256, 40)])

@@ -744,7 +744,7 @@ extern "C" __attribute__((visibility("default"))) int moe_ragged_metadata_remap(
 
 // ---------------------------------------------------------------------------------------------------------
 // moe_route: the whole routing step in one to three launches (the standalone entry points above take more).  Small batches: one launch of five
-// independent blocks (route_small_kernel); up to 896 tokens (1536 with long lists): one launch of a cluster of eight (route_cluster_kernel, both at the end of
+// independent blocks (route_small_kernel); up to 896 tokens (2048 with short lists): one launch of a cluster of eight (route_cluster_kernel, both at the end of
 // this section; rule: route_form).  Others: A, then route_finish_kernel where its blocks are a wave, else B and C.
 //   A  topk_quad_kernel<HIST>   top-k + softmax + bitmatrix row of every token, and the expert histogram of each block
 //      (route_topk_hist_kernel  of 128 tokens (partial[blk][e]) in the same pass over the logits;
@@ -1175,7 +1175,7 @@ __global__ void __launch_bounds__(1024) route_small_kernel(
 
 constexpr int kRouteSmallTokens = 256;
 
-// The whole routing step of a batch of up to 896 tokens (1536 with long lists, see route_form) in one launch of one cluster: eight blocks take an eighth of the tokens each, read
+// The whole routing step of a batch of up to 896 to 2048 tokens (see route_form) in one launch of one cluster: eight blocks take an eighth of the tokens each, read
 // one another's expert counts through distributed shared memory behind a cluster barrier, and rank their own entries on top of
 // them; blocks 3 to 7 build a row of the ragged metadata each.
 
@@ -1296,7 +1296,7 @@ extern "C" __attribute__((visibility("default"))) size_t moe_route_workspace(int
   return (size_t)((2 * nb * E + E) * (int64_t)sizeof(int32_t));
 }
 
-// us per call in a graph (small, cluster, two launches, three launches):
+// us on the device, calls of a graph (small, cluster, two launches, three launches):
 //   128 experts, k = 4:  16 tokens 5.6, 6.4;  32  7.7, 6.5;  64  8.1, 7.0;  256  13.6, 10.0, 10.4;  300  -, 8.5, 10.5, 13.6;  512  -, 10.5, 10.7, 13.6;
 //                        768  -, 10.4, 11.2, 14.1;  1024  -, 12.2, 11.5, 14.2;  1536  -, 13.8, 11.3, 14.4;  2048  -, 16.7, 11.6, 14.4
 //   64 experts, k = 8:   16 tokens 7.4, 7.0;  256  15.5, 13.9, 12.4;  300  -, 10.3, 12.4, 17.1;  768  -, 12.6, 12.9, 17.5;
@@ -1315,10 +1315,15 @@ extern "C" __attribute__((visibility("default"))) size_t moe_route_workspace(int
 // longest and the line lies at 1536.  Lists of one or two picks leave the cluster little to sort: from 64 experts on its line lies at 1024, and the shortest
 // (E k <= 16) go back to it where it has four lanes per token, from 1025 to 1536.  (From 129 to 256 tokens the rule does not follow the table: two launches
 // would be up to 1.8 us ahead with four picks and more, and the cluster's 32 lanes per token take longer there than 16 do at 300.)
+// These are the lines of a layer step, whose products keep the device ahead of the host.  A call by itself takes 12 us of the host with one launch and 14 with two,
+// more than the device has to do up to E k = 512, so there the cluster's lines are at 1536 and 2048 (us per call in a loop, cluster and two launches: 1024
+// tokens of 128 experts, k = 4, 12.4, 14.1; 1536 14.1, 13.9; 1536 of 32 experts, k = 8, 13.4, 14.0; 2048 of 32 experts, k = 4, 12.1, 14.1; but 900 of 64
+// experts, k = 8, 14.9, 13.9; of 200, k = 4, 14.8, 14.0).
 enum { ROUTE_SMALL, ROUTE_CLUSTER, ROUTE_LAUNCHES };
-static int route_form(int64_t T, int E, int k) {
+static int route_form(int64_t T, int E, int k, bool step) {
   if (!(k == 1 || k == 2 || k == 4 || k == 8 || k == 16)) return ROUTE_LAUNCHES;
   if (T <= kRouteSmallTokens) return T >= 24 && k >= 4 && (E * k >= 512 || T <= 64) ? ROUTE_CLUSTER : ROUTE_SMALL;
+  if (!step && k <= 8 && E * k <= (k <= 4 ? 512 : 256)) return T <= (E * k <= 128 ? 2048 : 1536) ? ROUTE_CLUSTER : ROUTE_LAUNCHES;
   if (E * k <= 16 && T > 1024) return T <= 1536 ? ROUTE_CLUSTER : ROUTE_LAUNCHES;
   return T <= (E * k > 1024 ? 1536 : k <= 2 && E >= 64 ? 1024 : 896) ? ROUTE_CLUSTER : ROUTE_LAUNCHES;
 }
@@ -1341,7 +1346,7 @@ static int route_launch(
   MOE_CHECK_ARG(workspace_bytes >= moe_route_workspace(T, E, k), "moe_route: workspace too small (%zu < %zu)", workspace_bytes,
                 moe_route_workspace(T, E, k));
   cudaStream_t st = (cudaStream_t)stream;
-  const int form = route_form(T, E, k);
+  const int form = route_form(T, E, k, out.weight != nullptr);
   if (form == ROUTE_SMALL) {
     const int n = (int)T * k, warps = (n + 31) / 32 < 32 ? (n + 31) / 32 : 32;
     const size_t smem_s = (size_t)(3 * (E + 1) + n) * sizeof(int32_t) + (size_t)(n + warps * E) * sizeof(int16_t);   // < 48 KB

@@ -12,8 +12,8 @@ FUSED_MAX_TOKENS = 1 << 22
 
 
 def route(logits, n_expts_act, apply_softmax=True):
-    """Top-k, expert histogram, expert-major sort and ragged metadata of one batch of logits in one launch (up to some 1500
-    tokens), two or three: -> (ragged_metadata, sparse_logits), the same objects `topk` + `make_ragged_tensor_metadata` return.
+    """Top-k, expert histogram, expert-major sort and ragged metadata of one batch of logits in one launch (up to some 900
+    tokens, 1536 or 2048 with short lists), two or three: -> (ragged_metadata, sparse_logits), the same objects `topk` + `make_ragged_tensor_metadata` return.
     More than 256 experts, more than FUSED_MAX_TOKENS tokens, or logits that are not a plain 2-D tensor take the
     five-launch composition of the separate entry points."""
     return _route(logits, n_expts_act, apply_softmax)[:2]

@@ -288,12 +288,15 @@ struct PackRows {
 // one of the experts (dropped ones are -1)
 struct PickChunk { uint8_t* chunk; int r, lines; };
 __device__ __forceinline__ PickChunk pick_chunk(const GemmParams& p, const PackParams& a, const PackRows& w, int64_t at, int kt, bool split) {
-  const int pick = w.experts[at], e = (unsigned)pick < (unsigned)p.E ? pick : 0, rows = p.slice_sizes[e];
-  const int rr = w.positions[at] - p.slice_offs[e], j = rr / a.tb;
+  // (the loads side by side: with the block's behind the check a step of 4 tokens of 8 experts took 0.4 us longer)
+  const int pick = w.experts[at], m = w.positions[at], e = (unsigned)pick < (unsigned)p.E ? pick : 0;
+  const int rows = p.slice_sizes[e], off = p.slice_offs[e], first = p.block_offs[e];
+  const int rr = m - off, j = rr / a.tb;
   PickChunk c;
   c.r = rr - j * a.tb;
   c.lines = !split ? a.n_mma : a.fit ? chunk_lines(min(a.tb, rows - j * a.tb)) : a.tb;
-  c.chunk = e == pick && rr >= 0 && rr < rows ? a.out + ((int64_t)(p.block_offs[e] + j) * a.KT + kt) * a.chunk_bytes : nullptr;
+  uint8_t* chunk = a.out + ((int64_t)(first + j) * a.KT + kt) * a.chunk_bytes;
+  c.chunk = e == pick && rr >= 0 && rr < rows ? chunk : nullptr;
   return c;
 }
 // `store`(chunk, r, lines) for each pick of token t that has a chunk, by the whole warp

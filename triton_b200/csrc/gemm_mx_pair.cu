@@ -316,8 +316,8 @@ __device__ __forceinline__ int64_t pick_prow(const GemmParams& p, const PairPack
   const int pick = a.experts[t * a.k + j];
   e = (unsigned)pick < (unsigned)p.E ? pick : 0;
   m = a.positions[t * a.k + j];
-  const int off = p.slice_offs[e];
-  return e == pick && m >= off && m < off + p.slice_sizes[e] ? padded_base(e, off) + (m - off) : -1;
+  const int off = p.slice_offs[e], rows = p.slice_sizes[e];
+  return e == pick && m >= off && m < off + rows ? padded_base(e, off) + (m - off) : -1;
 }
 template <bool TILED>
 __global__ void __launch_bounds__(256) mx_pair_pack2_rows_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ PairPackParams a) {

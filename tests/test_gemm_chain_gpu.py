@@ -235,10 +235,10 @@ def test_decode_tokens_by_row_are_those_by_position(block, e4m3, rows, k, depth,
     assert torch.equal(by_position, by_row) and bool(by_row.abs().sum() > 0)
 
 
-# k steps in one part, two and four; an infinity in the first part, the last, or both
-@pytest.mark.parametrize("depth", [896, 1056, 1952, 2080])
-def test_pair_tokens_in_parts_are_those_by_row(depth, device):
-    p = Passes(1184, 2, depth, 256, device)                    # eight rows for each of 148 SMs: by row with the positions
+# k steps in one part, two and four; an infinity in the first part, the last, or both; whole blocks from two and a half per SM on
+@pytest.mark.parametrize("depth, rows", [(896, 1184), (1056, 1184), (1952, 1184), (2080, 1184), (2080, 2920), (2080, 2928), (1056, 4000)])
+def test_pair_tokens_in_parts_are_those_by_row(depth, rows, device):
+    p = Passes(rows, 2, depth, 256, device)                    # 1184, eight rows for each of 148 SMs: from there on by row with the positions
     p.x[3, 5] = p.x[40, depth - 1] = p.x[77, depth // 2] = float("inf")
     p.x[77, 0] = float("-inf")
     by_position, by_row = p.run(False, b"gemm_mx_pair_kernel"), p.run(True, b"gemm_mx_pair_kernel")

@@ -1077,9 +1077,11 @@ int moe_gemm_mx_pair_launch(const GemmParams& p_in, const MoeGemmArgs& a, const 
                                 pl.terms == 1 ? 0 : (size_t)PACK_TOKENS * a.x_k * sizeof(int64_t), st, p, pk));
     } else {
       auto pack = pl.terms == 1 ? mx_pair_pack1_kernel : tiled ? mx_pair_pack2_kernel<true> : mx_pair_pack2_kernel<false>;
-      // Blocks of 16 rows in parts of a turn or two of their threads (32 experts of 2880 x 5760, 256 tokens: 146.3 us per step whole, 144.9 in two
-      // parts, 144.1 in four; 512 deep, four k steps: 29.4 whole, 30.1 in four).
-      if (pl.terms == 2) pk.parts = pl.KT >= 16 ? 4 : pl.KT >= 8 ? 2 : 1;
+      // Blocks of 16 rows in parts of a turn or two of their threads, where whole ones are less than the three that an SM holds (512 deep, four k
+      // steps: 29.4 us whole, 30.1 in four).  us of a product of 1024 columns with its pass, whole and in parts: 32 experts, 2880 deep, 1024 rows (95 blocks) 34.9, 23.9;
+      // 2400 (182) 40.0, 31.9; 4800 (331) 54.9, 51.6; 9600 (631) 78.4, 79.1; 16000 (1031) 113, 116; 64000 432, 478; 1440 deep, 4800 rows 34.3, 34.2; 7200 (481) 38.1,
+      // 39.8; 32000 118, 124; 128 experts, 1440 deep, 2400 rows (278) 44.4, 42.1; 4800 (427) 48.2, 49.3.
+      if (pl.terms == 2 && 2 * blocks16 <= 5 * (int64_t)moe_sm_count()) pk.parts = pl.KT >= 16 ? 4 : pl.KT >= 8 ? 2 : 1;
       MOE_CHECK_CUDA(launch_pdl(pack, dim3((unsigned)(blocks16 * pk.parts)), dim3(256), 0, st, p, pk));
     }
     MOE_CHECK_LAUNCH();

@@ -93,7 +93,6 @@ struct PairPackParams {
   int64_t prows;
   uint8_t* xq; uint8_t* xs;
   uint32_t* done;
-  int parts;                     // blocks (1, 2 or 4) that share the groups of 16 rows; each has its bytes of the rows' words
   const int32_t* positions; const int16_t* experts;      // [rows_x, k]: where the rows of x go (NULL: gather says)
   int k;
   TokenOut out;                  // the product's rows are the next one's tokens: those computed here go there too
@@ -273,13 +272,15 @@ __device__ __noinline__ uint32_t exact_rows(const GemmParams& p, const PairPackP
 // TILED: k inside eight in the order of the default weight tiles (0, 2, 4, 6, 1, 3, 5, 7).  A thread takes a whole group of 32 k:
 // no exchange between lanes, 64 bytes in, a 32-byte sector out per term.  With eight k per lane and four lanes to a group, 65536
 // rows of 2880 took 153 us and 4800 rows 20.3, so 141 and 16.8.
-template <bool TILED>
-__global__ void __launch_bounds__(256, 3) mx_pair_pack2_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ PairPackParams a) {
+// PARTS: blocks (1, 2 or 4) that share the groups of 16 rows, each with its bytes of the rows' words.  (A constant: divided by at run time, and with the
+// registers of three blocks per SM for whole ones too, a product of 64 experts of 736 x 1440 took 0.8 us of 22 longer.)
+template <bool TILED, int PARTS>
+__global__ void __launch_bounds__(256, PARTS == 1 ? 1 : 3) mx_pair_pack2_kernel(const __grid_constant__ GemmParams p, const __grid_constant__ PairPackParams a) {
   pdl_begin();
   int e; int64_t row0, prow0; int rows;
-  const int part = (int)(blockIdx.x & (unsigned)(a.parts - 1));
-  if (!pack_block(p, blockIdx.x / (unsigned)a.parts, e, row0, rows, prow0)) return;
-  const int kt0 = part * a.KT / a.parts, G = ((part + 1) * a.KT / a.parts - kt0) * 4;      // groups of this part's k steps
+  const int part = (int)(blockIdx.x % PARTS);
+  if (!pack_block(p, blockIdx.x / PARTS, e, row0, rows, prow0)) return;
+  const int kt0 = part * a.KT / PARTS, G = ((part + 1) * a.KT / PARTS - kt0) * 4;      // groups of this part's k steps
   bool beyond = false;
   for (int t = threadIdx.x; t < rows * G; t += 256) {
     const int r = t / G, g = kt0 * 4 + t - r * G;
@@ -300,10 +301,15 @@ __global__ void __launch_bounds__(256, 3) mx_pair_pack2_kernel(const __grid_cons
   if ((int)threadIdx.x < rows) {
     uint32_t* word = a.done + prow0 + threadIdx.x;
     const uint32_t bit = (done >> threadIdx.x) & 1u;
-    if (a.parts == 1) *word = bit;
-    else if (a.parts == 2) ((uint16_t*)word)[part] = (uint16_t)bit;
+    if constexpr (PARTS == 1) *word = bit;
+    else if constexpr (PARTS == 2) ((uint16_t*)word)[part] = (uint16_t)bit;
     else ((uint8_t*)word)[part] = (uint8_t)bit;
   }
+}
+
+template <bool TILED>
+auto pack2_in_parts(int parts) {
+  return parts == 4 ? mx_pair_pack2_kernel<TILED, 4> : parts == 2 ? mx_pair_pack2_kernel<TILED, 2> : mx_pair_pack2_kernel<TILED, 1>;
 }
 
 // The same with the rows of x in turn, given the positions of every one (positions, experts: k per row): a row that k experts take is read
@@ -1065,7 +1071,6 @@ int moe_gemm_mx_pair_launch(const GemmParams& p_in, const MoeGemmArgs& a, const 
   const bool tiled = a.w_kind == MOE_W_MX4_B200;
   pk.out = out;
   pk.positions = nullptr; pk.experts = nullptr; pk.k = 0;
-  pk.parts = 1;
   if (!packed) {
     // by rows of x where every one of them has its k positions, several (and no more than a block has shared memory for), and their blocks
     // fill the SMs (256 rows, two positions each: 27.6 us per layer step by position, 28.1 by row)
@@ -1076,13 +1081,13 @@ int moe_gemm_mx_pair_launch(const GemmParams& p_in, const MoeGemmArgs& a, const 
       MOE_CHECK_CUDA(launch_pdl(pack, dim3((unsigned)cdiv64(a.rows_x, PACK_TOKENS)), dim3(256),
                                 pl.terms == 1 ? 0 : (size_t)PACK_TOKENS * a.x_k * sizeof(int64_t), st, p, pk));
     } else {
-      auto pack = pl.terms == 1 ? mx_pair_pack1_kernel : tiled ? mx_pair_pack2_kernel<true> : mx_pair_pack2_kernel<false>;
       // Blocks of 16 rows in parts of a turn or two of their threads, where whole ones are less than the three that an SM holds (512 deep, four k
       // steps: 29.4 us whole, 30.1 in four).  us of a product of 1024 columns with its pass, whole and in parts: 32 experts, 2880 deep, 1024 rows (95 blocks) 34.9, 23.9;
       // 2400 (182) 40.0, 31.9; 4800 (331) 54.9, 51.6; 9600 (631) 78.4, 79.1; 16000 (1031) 113, 116; 64000 432, 478; 1440 deep, 4800 rows 34.3, 34.2; 7200 (481) 38.1,
       // 39.8; 32000 118, 124; 128 experts, 1440 deep, 2400 rows (278) 44.4, 42.1; 4800 (427) 48.2, 49.3.
-      if (pl.terms == 2 && 2 * blocks16 <= 5 * (int64_t)moe_sm_count()) pk.parts = pl.KT >= 16 ? 4 : pl.KT >= 8 ? 2 : 1;
-      MOE_CHECK_CUDA(launch_pdl(pack, dim3((unsigned)(blocks16 * pk.parts)), dim3(256), 0, st, p, pk));
+      const int parts = pl.terms == 1 || 2 * blocks16 > 5 * (int64_t)moe_sm_count() ? 1 : pl.KT >= 16 ? 4 : pl.KT >= 8 ? 2 : 1;
+      auto pack = pl.terms == 1 ? mx_pair_pack1_kernel : tiled ? pack2_in_parts<true>(parts) : pack2_in_parts<false>(parts);
+      MOE_CHECK_CUDA(launch_pdl(pack, dim3((unsigned)(blocks16 * parts)), dim3(256), 0, st, p, pk));
     }
     MOE_CHECK_LAUNCH();
   }

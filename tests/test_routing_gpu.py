@@ -106,8 +106,8 @@ def test_expert_sort_at_the_segments_of_its_scan(T, E, k, device):
 
 @pytest.mark.parametrize("T, E, k, n_rows", [(1, 1, 1, None), (7, 3, 2, 5), (9, 256, 1, None), (8192, 256, 4, None), (8193, 256, 4, None),
                                              (10922, 20, 3, 10000), (3000, 33, 5, 0)])
-def test_expert_sort_in_one_cluster(T, E, k, n_rows, device):
-    # up to 32768 entries: eight shares (empty and partial ones), dropped entries and rows past a device-side bound
+def test_expert_sort_in_one_launch(T, E, k, n_rows, device):
+    # up to 32768 entries: whole and partial shares of 1024, dropped entries and rows past a device-side bound
     torch.manual_seed(T + E)
     indx = torch.randint(-1 if E > 3 else 0, E, (T, k)).short()
     bound = None if n_rows is None else torch.tensor([n_rows], dtype=torch.int32, device=device)

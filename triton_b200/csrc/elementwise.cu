@@ -270,7 +270,8 @@ extern "C" __attribute__((visibility("default"))) int moe_swiglu(const void* a, 
 }
 
 // The plain sum over R slots of rows of 16-byte vectors: HBM-bound, so the loads of four slots are under way before the first is added (with one
-// at a time a thread had 16 bytes in flight: the combine of 16384 tokens 104 -> 93 us, of 8192 50 -> 44).  Same order of additions as reduce_kernel.
+// at a time a thread had 16 bytes in flight).  us by itself, before and now, four slots of 2880: 300 tokens 2.6, 2.2; 1200 4.8, 4.4; 4096 18.6, 16.2; 16384 73.3,
+// 74.2; in a prefill step some 104, 93 and, 8192 tokens, 50, 44, which the step's spread under the power limit hides.  Same order of additions as reduce_kernel.
 template <typename TX, typename TY>
 __global__ void __launch_bounds__(256) sum_slots_kernel(const TX* x, int R, uint32_t per_row, uint32_t total, int64_t sx_r, int64_t sx_0, TY* y,
                                                         int64_t sy_0) {

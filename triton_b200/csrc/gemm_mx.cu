@@ -236,10 +236,6 @@ __global__ void __launch_bounds__(256) mx_pack_x_kernel(const GemmParams p, cons
 // Two values at a time by the conversion instructions (round to nearest, ties to the even code; |q| <= 6 but for Inf, which
 // saturates): with compares and selects per value, and a warp reduction under four masks, the pack of 64 tokens for 128 experts
 // took 13.6-14.4 us, so 10.5-11.1.
-// (16 warps over the rows of eight k steps, for a third of the blocks: 2.6 x slower at 64 tokens, the blocks of 16 rows decide;
-// four warps instead of eight: 8 % slower.)  (A warp per (token block, k step, four rows) with the rows' chains side by side, and dead warps grouped into whole
-// CTAs, was tried in place of the loop over rows below: 2.3 x slower.  A row's four-term chain is latency, and four of
-// them in one warp add up where eight warps of a CTA overlap them.)
 __device__ __forceinline__ uint32_t group_max_bits(uint32_t top) {        // over the 8 lanes that hold a group
 #pragma unroll
   for (int o = 1; o <= 4; o <<= 1) top = max(top, __shfl_xor_sync(0xFFFFFFFFu, top, o));
@@ -250,6 +246,11 @@ __device__ __forceinline__ void pack_store4(uint8_t* chunk, int lines, int line,
   *reinterpret_cast<uint16_t*>(chunk + line * 64 + ((g ^ (uint32_t)((line >> 1) & 3)) << 4) + (uint32_t)(lane & 7) * 2u) = (uint16_t)codes;      // a 32-group is one 16-byte piece
   if ((lane & 7) == 0) chunk[lines * 64 + (line & 31) * 16 + (line >> 5) * 4 + (int)g] = (uint8_t)sb;
 }
+// The pass by position, a warp a row at a time.
+// (16 warps over the rows of eight k steps, for a third of the blocks: 2.6 x slower at 64 tokens, the blocks of 16 rows decide;
+// four warps instead of eight: 8 % slower.)  (A warp per (token block, k step, four rows) with the rows' chains side by side, and dead warps grouped into whole
+// CTAs, was tried in place of the loop over rows below: 2.3 x slower.  A row's four-term chain is latency, and four of
+// them in one warp add up where eight warps of a CTA overlap them.)
 __global__ void __launch_bounds__(256) mx_pack_x4_kernel(const GemmParams p, const PackParams a) {
   pdl_begin();
   const int64_t slot = blockIdx.x;

@@ -142,6 +142,7 @@ __device__ __forceinline__ void elect_tile_3d(uint32_t dst, const CUtensorMap* t
       "l"(tmap), "r"(x), "r"(y), "r"(z), "r"(bar)
       : "memory");
 }
+// the same with a cache policy
 __device__ __forceinline__ void elect_tile_3d_hint(uint32_t dst, const CUtensorMap* tmap, int x, int y, int z, uint32_t bar, uint64_t policy) {
   asm volatile(
       "{\n\t.reg .pred q;\n\telect.sync _|q, 0xFFFFFFFF;\n\t"
@@ -149,7 +150,6 @@ __device__ __forceinline__ void elect_tile_3d_hint(uint32_t dst, const CUtensorM
       "l"(tmap), "r"(x), "r"(y), "r"(z), "r"(bar), "l"(policy)
       : "memory");
 }
-// the same with a cache policy
 __device__ __forceinline__ void elect_bulk_g2s_hint(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar, uint64_t policy) {
   asm volatile(
       "{\n\t.reg .pred q;\n\telect.sync _|q, 0xFFFFFFFF;\n\t"

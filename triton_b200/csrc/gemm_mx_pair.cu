@@ -1008,6 +1008,7 @@ int launch_mx_pair_ty(const GemmParams& p, const PairParams& q, const MoeGemmArg
 //   bf16   128 experts of 2880 x 5760:  20 rows 429, 452; 377, 357.  24 rows 449, 437; 436, 391
 //          32 experts of the same:  20 rows 109, 131; 123, 129.  25 rows 118, 134; 133, 131.  30 rows 135, 138; 141, 136.  40 rows 172, 143; 164, 149
 //          64 experts of 1440 x 2880:  20 rows 86, 96; 81, 88.  25 rows 84, 95; 94, 94.  32 rows 101, 98; 102, 97
+//          a product of 64 experts of 736 x 1440:  20 rows 26, 23; 29, 23.  24 rows 28, 24; 34, 25
 //   e4m3   128 experts of 2880 x 5760:  16 rows 359, 397; 307, 287.  20 rows 361, 396; 338, 295.  24 rows 376, 406; 377, 314
 //          32 experts of the same:  16 rows 102, 129; 100, 121.  25 rows 110, 131; 122, 127.  32 rows 130, 133; 135, 132
 //          64 experts of 1440 x 2880:  16 rows 77, 91; 75, 80.  25 rows 79, 91; 87, 89
